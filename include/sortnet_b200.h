@@ -124,10 +124,18 @@ int snb_inf_dist_forward_noalloc(const float* x, const float* w, int B, int CO, 
                                  int HW, float* y, int* pos, void* stream);
 int snb_inf_dist_forward_noalloc_max_outputs(void);
 
+/* Scratch with which the `_ws` entry points below evaluate a problem in the pruned form (the exact results, but
+ * only the columns of w that can matter are looked at per row): tensors = 1 for a point value, 2 for a box, 3 for both
+ * (snb_layer_bound_forward_ws); K = 1, or the sort neuron's K; words = 1 when positions are wanted; column_lists = 1 with
+ * kept-column lists.  0 when the problem is too small or too wide for it.  Fewer bytes (or NULL) select the dense kernels. */
+size_t snb_prune_scratch_bytes(int tensors, int K, int words, int B, int CO, int CI, int W_CO, int W_CI,
+                               int column_lists);
+
 /* Same y without pos, unmasked.  Replaces inf_dist::forward_nograd (norm_dist.h:22-23;
  * inf_dist_cuda.cu:277-304). */
 int snb_inf_dist_forward_nograd(const float* x, const float* w, int B, int CO, int CI, int G,
                                 int HW, float* y, void* stream);
+int snb_inf_dist_forward_nograd_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y, void* workspace, size_t workspace_bytes, void* stream);
 
 /* grad_input[b, idx] += s * grad_output[b,j] with (idx, s) decoded from pos.
  * Replaces inf_dist::backward_input (norm_dist.h:27-28; inf_dist_cuda.cu:325-336). */
@@ -189,6 +197,7 @@ int snb_norm_dist_backward_input_weight(const float* grad_output, const float* x
 int snb_bound_inf_dist_forward_nograd(const float* xl, const float* xu, const float* w, int B,
                                       int CO, int CI, int G, int HW, float* yl, float* yu,
                                       void* stream);
+int snb_bound_inf_dist_forward_nograd_ws(const float* xl, const float* xu, const float* w, int B, int CO, int CI, int G, int HW, float* yl, float* yu, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Same bounds plus the words of the coordinates that set them: c | (bit 31 when w - xL > xU - w);
  * posL = 0xffffffff when the lower bound stayed at its floor (no gradient), posU defaults to 0.
@@ -196,6 +205,7 @@ int snb_bound_inf_dist_forward_nograd(const float* xl, const float* xu, const fl
 int snb_bound_inf_dist_forward(const float* xl, const float* xu, const float* w, int B, int CO,
                                int CI, int G, int HW, float* yl, float* yu, int* posl, int* posu,
                                void* stream);
+int snb_bound_inf_dist_forward_ws(const float* xl, const float* xu, const float* w, int B, int CO, int CI, int G, int HW, float* yl, float* yu, int* posl, int* posu, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Sparse backward of the bounds.  Replaces bound_inf_dist::backward_input and
  * ::backward_input_weight (norm_dist.h:39-44; bound_inf_dist_cuda.cu:362-383). */
@@ -214,17 +224,20 @@ int snb_bound_inf_dist_backward_input_weight(const float* grad_yl, const float* 
  * sort_neuron.cu:403-435). */
 int snb_sort_neuron_forward_nograd(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
                                    float* y, float q, int K, void* stream);
+int snb_sort_neuron_forward_nograd_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y, float q, int K, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Same value plus pos [K, B, CO, HW]: word of the r-th largest element (index | bit 31 when
  * x - w < 0); of equal values the later index ranks higher; unfilled ranks hold word 0.
  * Replaces sort_neuron::forward (norm_dist.h:50-51; sort_neuron.cu:453-485). */
 int snb_sort_neuron_forward(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
                             float* y, int* pos, float q, int K, void* stream);
+int snb_sort_neuron_forward_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y, int* pos, float q, int K, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Interval bounds of the sort neuron over the box [xL, xU].
  * Replaces bound_sort_neuron_forward_cuda (norm_dist.h:58-59; sort_neuron.cu:502-534). */
 int snb_bound_sort_neuron_forward(const float* xl, const float* xu, const float* w, int B, int CO, int CI,
                                   int G, int HW, float* yl, float* yu, float q, int K, void* stream);
+int snb_bound_sort_neuron_forward_ws(const float* xl, const float* xu, const float* w, int B, int CO, int CI, int G, int HW, float* yl, float* yu, float q, int K, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Sparse backward through the K recorded positions.  Replaces sort_neuron::backward_input and
  * ::backward_input_weight (norm_dist.h:52-56; sort_neuron.cu:536-562). */
@@ -315,6 +328,7 @@ int snb_layer_backward(const float* grad_out, const float* x, const float* w, co
 int snb_layer_bound_forward(const float* x, const float* xl, const float* xu, const float* w, int B, int CO, int CI,
                             const float* running_mean, const float* bias, float* y, float* yl, float* yu,
                             void* stream);
+int snb_layer_bound_forward_ws(const float* x, const float* xl, const float* xu, const float* w, int B, int CO, int CI, const float* running_mean, const float* bias, float* y, float* yl, float* yu, void* workspace, size_t workspace_bytes, void* stream);
 
 /* xl = max(x - eps, down), xu = min(x + eps, up) over n values: the input box of the certification
  * forward for scalar bounds.  Replaces ell_inf_models.py:35-36. */

@@ -34,6 +34,14 @@ SIGNATURES = {
     "snb_bound_sort_neuron_forward": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P],
     "snb_sort_neuron_backward_input": [_P, _P, _I, _I, _I, _I, _I, _P, _F, _I, _P],
     "snb_sort_neuron_backward_input_weight": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P],
+    "snb_inf_dist_forward_nograd_ws": [_P, _P, _I, _I, _I, _I, _I, _P, _P, ctypes.c_size_t, _P],
+    "snb_bound_inf_dist_forward_nograd_ws": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, ctypes.c_size_t, _P],
+    "snb_bound_inf_dist_forward_ws": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, ctypes.c_size_t, _P],
+    "snb_sort_neuron_forward_nograd_ws": [_P, _P, _I, _I, _I, _I, _I, _P, _F, _I, _P, ctypes.c_size_t, _P],
+    "snb_sort_neuron_forward_ws": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P, ctypes.c_size_t, _P],
+    "snb_bound_sort_neuron_forward_ws": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P, ctypes.c_size_t, _P],
+    "snb_layer_bound_forward_ws": [_P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P],
+    "snb_prune_scratch_bytes": [_I, _I, _I, _I, _I, _I, _I, _I, _I],     # returns size_t
     "snb_mean_shift_stats": [_P, _P, _I, _I, _I, _P, _P, _F, _P],
     "snb_mean_shift_apply": [_P, _P, _P, _I, _I, _P, _P],
     "snb_sample_mask": [_P, _I, _I, _I, ctypes.c_ulonglong, _P],
@@ -93,6 +101,7 @@ def load(build_if_missing: bool = False):
     lib.snb_inf_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     lib.snb_inf_dist_forward_sorted_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
     lib.snb_inf_dist_forward_sorted_workspace_bytes.restype = ctypes.c_size_t
+    lib.snb_prune_scratch_bytes.restype = ctypes.c_size_t
     lib.snb_norm_dist_forward_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_float]
     lib.snb_norm_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     _lib = lib

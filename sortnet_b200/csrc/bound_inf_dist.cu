@@ -12,6 +12,7 @@
 #include "tile.cuh"
 #include "launch.h"
 #include "general_shapes.h"
+#include "prune.cuh"
 
 namespace snb {
 
@@ -359,13 +360,27 @@ static int check_bound(const void* xl, const void* xu, const void* w, const void
     return SNB_OK;
 }
 
-extern "C" int snb_bound_inf_dist_forward_nograd(const float* xl, const float* xu, const float* w,
-                                                 int B, int CO, int CI, int G, int HW, float* yl,
-                                                 float* yu, void* stream) {
+static PruneProblem box_problem(const float* xl, const float* xu, const float* w, int B, int CO, int CI, float* yl,
+                                float* yu, int* posl, int* posu) {
+    PruneProblem p;
+    p.xl = xl, p.xu = xu, p.w = w, p.yl = yl, p.yu = yu, p.posl = posl, p.posu = posu;
+    p.B = B, p.CO = p.W_CO = CO, p.CI = p.W_CI = CI;
+    return p;
+}
+
+// workspace: snb_prune_scratch_bytes(2, 1, 0, ...) bytes or null
+extern "C" int snb_bound_inf_dist_forward_nograd_ws(const float* xl, const float* xu, const float* w, int B, int CO,
+                                                    int CI, int G, int HW, float* yl, float* yu, void* workspace,
+                                                    size_t workspace_bytes, void* stream) {
     if (G != 1 || HW != 1)
         return general_bound_forward(xl, xu, w, B, CO, CI, G, HW, yl, yu, nullptr, nullptr, (cudaStream_t)stream);
     int rc = check_bound(xl, xu, w, yl, yu, B, CO, CI, G, HW);
     if (rc) return rc;
+    const PruneProblem pp = box_problem(xl, xu, w, B, CO, CI, yl, yu, nullptr, nullptr);
+    if (prune_fits(pp, workspace, workspace_bytes)) {
+        SNB_CUDA(prune_forward(pp, workspace, (cudaStream_t)stream));
+        return SNB_OK;
+    }
     BoundParams p{xl, xu, w, yl, yu, nullptr, nullptr, B, CO, CI, 0, 0, 0};
     const bool vec = (CI % 4 == 0) && aligned16(xl) && aligned16(xu) && aligned16(w);
     cudaStream_t st = (cudaStream_t)stream;
@@ -392,9 +407,15 @@ extern "C" int snb_bound_inf_dist_forward_nograd(const float* xl, const float* x
     return SNB_OK;
 }
 
-extern "C" int snb_bound_inf_dist_forward(const float* xl, const float* xu, const float* w, int B,
-                                          int CO, int CI, int G, int HW, float* yl, float* yu,
-                                          int* posl, int* posu, void* stream) {
+extern "C" int snb_bound_inf_dist_forward_nograd(const float* xl, const float* xu, const float* w, int B, int CO, int CI,
+                                                 int G, int HW, float* yl, float* yu, void* stream) {
+    return snb_bound_inf_dist_forward_nograd_ws(xl, xu, w, B, CO, CI, G, HW, yl, yu, nullptr, 0, stream);
+}
+
+// workspace: snb_prune_scratch_bytes(2, 1, 1, ...) bytes or null
+extern "C" int snb_bound_inf_dist_forward_ws(const float* xl, const float* xu, const float* w, int B, int CO, int CI,
+                                             int G, int HW, float* yl, float* yu, int* posl, int* posu, void* workspace,
+                                             size_t workspace_bytes, void* stream) {
     if (G != 1 || HW != 1) {
         if (!posl || !posu) return SNB_ERR_NULL_POINTER;
         return general_bound_forward(xl, xu, w, B, CO, CI, G, HW, yl, yu, posl, posu, (cudaStream_t)stream);
@@ -402,6 +423,11 @@ extern "C" int snb_bound_inf_dist_forward(const float* xl, const float* xu, cons
     int rc = check_bound(xl, xu, w, yl, yu, B, CO, CI, G, HW);
     if (rc) return rc;
     if (!posl || !posu) return SNB_ERR_NULL_POINTER;
+    const PruneProblem pp = box_problem(xl, xu, w, B, CO, CI, yl, yu, posl, posu);
+    if (prune_fits(pp, workspace, workspace_bytes)) {
+        SNB_CUDA(prune_forward(pp, workspace, (cudaStream_t)stream));
+        return SNB_OK;
+    }
     BoundParams p{xl, xu, w, yl, yu, posl, posu, B, CO, CI, 0, 0, 0};
     const bool vec = (CI % 4 == 0) && aligned16(xl) && aligned16(xu) && aligned16(w);
     dim3 grid((B + 63) / 64, (CO + 63) / 64);
@@ -418,6 +444,11 @@ extern "C" int snb_bound_inf_dist_forward(const float* xl, const float* xu, cons
     else bound_fwd_pos_kernel<false><<<grid, 256, SMEM, (cudaStream_t)stream>>>(p);
     SNB_CUDA(cudaGetLastError());
     return SNB_OK;
+}
+
+extern "C" int snb_bound_inf_dist_forward(const float* xl, const float* xu, const float* w, int B, int CO, int CI, int G,
+                                          int HW, float* yl, float* yu, int* posl, int* posu, void* stream) {
+    return snb_bound_inf_dist_forward_ws(xl, xu, w, B, CO, CI, G, HW, yl, yu, posl, posu, nullptr, 0, stream);
 }
 
 static int bound_backward(const float* gl, const float* gu, const int* posl, const int* posu, int B,

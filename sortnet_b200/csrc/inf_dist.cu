@@ -16,6 +16,7 @@
 #include "tile.cuh"
 #include "launch.h"
 #include "general_shapes.h"
+#include "prune.cuh"
 
 namespace snb {
 
@@ -530,13 +531,22 @@ static int check_fwd(const void* x, const void* w, const void* y, int B, int CO,
 
 static int inf_forward_impl(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
                             float* y, int* pos, const int* ci, const int* co, int W_CO, int W_CI,
-                            unsigned long long* keys, cudaStream_t st) {
+                            void* ws, size_t ws_bytes, cudaStream_t st) {
     if (G != 1 || HW != 1)
         return general_inf_forward(x, w, B, CO, CI, G, HW, y, pos, ci, co, W_CO, W_CI, st);
     int rc = check_fwd(x, w, y, B, CO, CI, G, HW, W_CO, W_CI, ci, co);
     if (rc) return rc;
     if (!pos) return SNB_ERR_NULL_POINTER;
     if ((CI + CHUNK_TILES * BK - 1) / (CHUNK_TILES * BK) >= 0xffff) return SNB_ERR_TOO_LARGE;
+    PruneProblem pp;
+    pp.x = x, pp.w = w, pp.ci = ci, pp.co = co, pp.y = y, pp.pos = pos;
+    pp.B = B, pp.CO = CO, pp.CI = CI, pp.W_CO = W_CO, pp.W_CI = W_CI;
+    if (prune_fits(pp, ws, ws_bytes)) {
+        SNB_CUDA(prune_forward(pp, ws, st));
+        return SNB_OK;
+    }
+    unsigned long long* keys = ws && ws_bytes >= sizeof(unsigned long long) * (size_t)B * (size_t)CO
+                                   ? (unsigned long long*)ws : nullptr;
     InfFwdParams p{x, w, y, pos, ci, co, B, CO, CI, W_CI};
     bool split = false;
     SNB_CUDA(dispatch_fwd<true>(p, keys, &split, st));
@@ -547,7 +557,7 @@ static int inf_forward_impl(const float* x, const float* w, int B, int CO, int C
 extern "C" int snb_inf_dist_forward(const float* x, const float* w, int B, int CO, int CI, int G,
                                     int HW, float* y, int* pos, const int* w_index_ci,
                                     const int* w_index_co, int W_CO, int W_CI, void* stream) {
-    return inf_forward_impl(x, w, B, CO, CI, G, HW, y, pos, w_index_ci, w_index_co, W_CO, W_CI, nullptr,
+    return inf_forward_impl(x, w, B, CO, CI, G, HW, y, pos, w_index_ci, w_index_co, W_CO, W_CI, nullptr, 0,
                             (cudaStream_t)stream);
 }
 
@@ -559,13 +569,9 @@ extern "C" int snb_inf_dist_forward_ws(const float* x, const float* w, int B, in
                                        int HW, float* y, int* pos, const int* w_index_ci,
                                        const int* w_index_co, int W_CO, int W_CI, void* workspace,
                                        size_t workspace_bytes, void* stream) {
-    unsigned long long* keys = nullptr;
-    if (workspace) {
-        if (reinterpret_cast<uintptr_t>(workspace) & 7u) return SNB_ERR_ALIGNMENT;
-        if (workspace_bytes >= snb_inf_dist_forward_workspace_bytes(B, CO)) keys = (unsigned long long*)workspace;
-    }
-    return inf_forward_impl(x, w, B, CO, CI, G, HW, y, pos, w_index_ci, w_index_co, W_CO, W_CI, keys,
-                            (cudaStream_t)stream);
+    if (reinterpret_cast<uintptr_t>(workspace) & 7u) return SNB_ERR_ALIGNMENT;
+    return inf_forward_impl(x, w, B, CO, CI, G, HW, y, pos, w_index_ci, w_index_co, W_CO, W_CI, workspace,
+                            workspace_bytes, (cudaStream_t)stream);
 }
 
 // Workspace of the ascending-list form: merge keys [B * CO] u64, then the full-width input
@@ -595,6 +601,10 @@ extern "C" int snb_inf_dist_forward_sorted_ws(const float* x, const float* w, in
                 !(reinterpret_cast<uintptr_t>(workspace) & 15u) &&
                 workspace_bytes >= snb_inf_dist_forward_sorted_workspace_bytes(B, CO, W_CI) &&
                 (long long)B * W_CI < (1ll << 31);
+    PruneProblem pp;
+    pp.x = x, pp.w = w, pp.ci = w_index_ci, pp.co = w_index_co, pp.y = y, pp.pos = pos;
+    pp.B = B, pp.CO = CO, pp.CI = CI, pp.W_CO = W_CO, pp.W_CI = W_CI;
+    if (fast && prune_fits(pp, workspace, workspace_bytes)) fast = false;   // the general entry point prunes
     // computing the dropped columns too must cost less than the vector copies save
     if (fast && w_index_ci && (long long)CI * 4 < (long long)W_CI * 3) fast = false;
     if (fast && !w_index_ci && !aligned16(x)) fast = false;
@@ -623,17 +633,29 @@ extern "C" int snb_inf_dist_forward_sorted_ws(const float* x, const float* w, in
     return SNB_OK;
 }
 
-extern "C" int snb_inf_dist_forward_nograd(const float* x, const float* w, int B, int CO, int CI,
-                                           int G, int HW, float* y, void* stream) {
+// workspace: snb_prune_scratch_bytes(1, 1, 0, ...) bytes or null
+extern "C" int snb_inf_dist_forward_nograd_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
+                                              float* y, void* workspace, size_t workspace_bytes, void* stream) {
     if (G != 1 || HW != 1)
         return general_inf_forward(x, w, B, CO, CI, G, HW, y, nullptr, nullptr, nullptr, CO, CI,
                                    (cudaStream_t)stream);
     int rc = check_fwd(x, w, y, B, CO, CI, G, HW, CO, CI, nullptr, nullptr);
     if (rc) return rc;
+    PruneProblem pp;
+    pp.x = x, pp.w = w, pp.y = y, pp.B = B, pp.CO = pp.W_CO = CO, pp.CI = pp.W_CI = CI;
+    if (prune_fits(pp, workspace, workspace_bytes)) {
+        SNB_CUDA(prune_forward(pp, workspace, (cudaStream_t)stream));
+        return SNB_OK;
+    }
     InfFwdParams p{x, w, y, nullptr, nullptr, nullptr, B, CO, CI, CI};
     bool split = false;
     SNB_CUDA(dispatch_fwd<false>(p, nullptr, &split, (cudaStream_t)stream));
     return SNB_OK;
+}
+
+extern "C" int snb_inf_dist_forward_nograd(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y,
+                                           void* stream) {
+    return snb_inf_dist_forward_nograd_ws(x, w, B, CO, CI, G, HW, y, nullptr, 0, stream);
 }
 
 // ---- entry point that allocates nothing ----------------------------------------------------
@@ -672,7 +694,7 @@ extern "C" int snb_inf_dist_forward_noalloc(const float* x, const float* w, int 
     // The launcher zero-fills the keys it is going to merge into (cudaMemsetAsync on `stream`)
     // before the kernel runs, so what an earlier call left in the array does not matter.
     return inf_forward_impl(x, w, B, CO, CI, G, HW, y, pos, nullptr, nullptr, CO, CI, keys,
-                            (cudaStream_t)stream);
+                            sizeof(unsigned long long) * (size_t)B * CO, (cudaStream_t)stream);
 }
 
 extern "C" int snb_inf_dist_forward_noalloc_max_outputs(void) { return SNB_NOALLOC_MAX_OUTPUTS; }

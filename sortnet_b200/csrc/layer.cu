@@ -12,6 +12,7 @@
 #include "../../include/sortnet_b200.h"
 #include "common.cuh"
 #include "launch.h"
+#include "prune.cuh"
 
 namespace snb {
 
@@ -247,7 +248,7 @@ extern "C" int snb_layer_forward(const float* x, const float* w, int B, int CO, 
             rc = snb_inf_dist_forward_sorted_ws(x, w, B, CO, CI, 1, 1, y_dist, pos, w_index_ci, w_index_co, W_CO, W_CI,
                                                 workspace, workspace_bytes, stream);
         else if (!w_index_ci && !w_index_co)
-            rc = snb_inf_dist_forward_nograd(x, w, B, CO, CI, 1, 1, y_dist, stream);
+            rc = snb_inf_dist_forward_nograd_ws(x, w, B, CO, CI, 1, 1, y_dist, workspace, workspace_bytes, stream);
         else
             return SNB_ERR_NULL_POINTER;      // masked forward always records positions
     } else {
@@ -305,21 +306,29 @@ extern "C" int snb_layer_backward(const float* grad_out, const float* x, const f
                                                  W_CO, W_CI, stream);
 }
 
-extern "C" int snb_layer_bound_forward(const float* x, const float* xl, const float* xu, const float* w, int B, int CO,
-                                       int CI, const float* running_mean, const float* bias, float* y, float* yl,
-                                       float* yu, void* stream) {
+// workspace: snb_prune_scratch_bytes(1, 2 or 3 tensors, 1, 0, ...) bytes or null
+extern "C" int snb_layer_bound_forward_ws(const float* x, const float* xl, const float* xu, const float* w, int B, int CO,
+                                          int CI, const float* running_mean, const float* bias, float* y, float* yl,
+                                          float* yu, void* workspace, size_t workspace_bytes, void* stream) {
     if (!w || (!x && !xl)) return SNB_ERR_NULL_POINTER;
     int rc = check2d(B, CO, CI);
     if (rc) return rc;
-    if (x) {
-        if (!y) return SNB_ERR_NULL_POINTER;
-        rc = snb_inf_dist_forward_nograd(x, w, B, CO, CI, 1, 1, y, stream);
-        if (rc) return rc;
-    }
-    if (xl) {
-        if (!xu || !yl || !yu) return SNB_ERR_NULL_POINTER;
-        rc = snb_bound_inf_dist_forward_nograd(xl, xu, w, B, CO, CI, 1, 1, yl, yu, stream);
-        if (rc) return rc;
+    if ((x && !y) || (xl && (!xu || !yl || !yu))) return SNB_ERR_NULL_POINTER;
+    if ((long long)CO * CI >= (1ll << 31)) return SNB_ERR_TOO_LARGE;
+    PruneProblem pp;
+    pp.x = x, pp.xl = xl, pp.xu = xu, pp.w = w, pp.y = y, pp.yl = yl, pp.yu = yu;
+    pp.B = B, pp.CO = pp.W_CO = CO, pp.CI = pp.W_CI = CI;
+    if (prune_fits(pp, workspace, workspace_bytes)) {
+        SNB_CUDA(prune_forward(pp, workspace, (cudaStream_t)stream));
+    } else {
+        if (x) {
+            rc = snb_inf_dist_forward_nograd(x, w, B, CO, CI, 1, 1, y, stream);
+            if (rc) return rc;
+        }
+        if (xl) {
+            rc = snb_bound_inf_dist_forward_nograd(xl, xu, w, B, CO, CI, 1, 1, yl, yu, stream);
+            if (rc) return rc;
+        }
     }
     if (running_mean || bias) {
         const size_t n = (size_t)B * CO;
@@ -329,6 +338,12 @@ extern "C" int snb_layer_bound_forward(const float* x, const float* xl, const fl
         SNB_CUDA(cudaGetLastError());
     }
     return SNB_OK;
+}
+
+extern "C" int snb_layer_bound_forward(const float* x, const float* xl, const float* xu, const float* w, int B, int CO,
+                                       int CI, const float* running_mean, const float* bias, float* y, float* yl,
+                                       float* yu, void* stream) {
+    return snb_layer_bound_forward_ws(x, xl, xu, w, B, CO, CI, running_mean, bias, y, yl, yu, nullptr, 0, stream);
 }
 
 extern "C" int snb_input_box(const float* x, float eps, float down, float up, long long n, float* xl, float* xu,

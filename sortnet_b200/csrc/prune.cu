@@ -1,0 +1,1172 @@
+// Pruned evaluation of the max-type distance operators: see prune.cuh for the method.
+//
+// What bounds it: the one read of W (prune_filter, HBM).  For 512 x 5120 x 5120 a dense max-plus
+// kernel issues 13.4 G subtract / max pairs; here about 40 columns per output row survive the
+// filter and about 12 of them are looked at, 1/400 of the pairs.
+#include "prune.cuh"
+
+namespace snb {
+
+namespace {
+
+constexpr int PAD = 8;              // lists are padded to a multiple of this
+constexpr int STEP = 4;             // list entries per bound ub
+constexpr int MAX_COLUMNS = 12288;  // widest row the filter takes: 512 threads x 6 x 4
+constexpr int BUCKETS = 32;
+
+struct PruneArgs {
+    PruneProblem p;
+    int S, NX, m, lcap;
+    unsigned* fail_count;
+    unsigned* hi;                   // order-preserving codes of max(x), max(-x) per column; 0 = no value
+    unsigned* nlo;
+    float* xt;                      // [S][W_CI][NX][32]
+    int* inv;                       // [S][W_CI] full column -> compact position (with ci)
+    int* cnt;                       // [W_CO] list length, -1: no list
+    float* tau;                     // [W_CO]
+    float* ub;                      // [W_CO][lcap / STEP] largest U from this step of the list on
+    int2* cand;                     // [W_CO][lcap] (column, bits of w)
+    int4* fail;                     // units (sub-batch, first output, mask of outputs) left to prune_fix
+};
+
+__device__ __forceinline__ unsigned order_code(float f) {
+    const unsigned b = __float_as_uint(f);
+    return f != f ? 0u : ((b & 0x80000000u) ? ~b : (b | 0x80000000u));
+}
+__device__ __forceinline__ float decode(unsigned e) {   // 0 -> NaN
+    return __uint_as_float((e & 0x80000000u) ? (e ^ 0x80000000u) : ~e);
+}
+
+// ---- transpose + column ranges ----------------------------------------------------------------
+// CTA = 32 rows (one sub-batch) x 64 compact columns.  Bound by the traffic of x and xt and by launch latency.
+template <int NX>
+__global__ void __launch_bounds__(256) prune_prep(const PruneArgs a) {
+    __shared__ float tile[NX][32][65];
+    const PruneProblem& p = a.p;
+    const int s = blockIdx.y, c0 = blockIdx.x * 64, tid = threadIdx.x;
+    const float nan = __int_as_float(0x7fc00000);
+    const int col = tid & 63, r0 = tid >> 6;
+    const bool cok = c0 + col < p.CI;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int r = r0 + 4 * i, b = s * 32 + r;
+        const bool ok = cok && b < p.B;
+        const size_t o = (size_t)b * p.CI + c0 + col;
+        if (NX != 2) tile[0][r][col] = ok ? p.x[o] : nan;
+        if (NX >= 2) {
+            float l = ok ? p.xl[o] : nan, u = ok ? p.xu[o] : nan;
+            if (l > u) l = u = (l + u) * 0.5f;               // inverted interval -> its midpoint
+            tile[NX - 2][r][col] = l;
+            tile[NX - 1][r][col] = u;
+        }
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int lc = warp + 8 * k;
+        if (c0 + lc >= p.CI) break;
+        const int c = p.ci ? p.ci[(size_t)s * p.CI + c0 + lc] : c0 + lc;
+        unsigned hi = 0u, nlo = 0u;
+#pragma unroll
+        for (int t = 0; t < NX; t++) {
+            const float v = tile[t][lane][lc];
+            a.xt[(((size_t)s * p.W_CI + c) * NX + t) * 32 + lane] = v;
+            hi = max(hi, order_code(v));
+            nlo = max(nlo, order_code(-v));
+        }
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        nlo = __reduce_max_sync(0xffffffffu, nlo);
+        if (lane == 0) {
+            atomicMax(a.hi + c, hi);
+            atomicMax(a.nlo + c, nlo);
+            if (p.ci) a.inv[(size_t)s * p.W_CI + c] = c0 + lc;
+        }
+    }
+}
+
+// ---- candidate lists --------------------------------------------------------------------------
+// Named barriers: a subset of the CTA's warps, or producers that only arrive and consumers that wait.
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+enum { BAR_FILTER = 1, BAR_FULL = 2, BAR_EMPTY = 4 };
+
+// Persistent CTA: FT filter threads + R ordering warps.  A thread owns NIT x 4 columns; it keeps their centre and
+// radius in registers and copies its part of the next rows of W ahead with cp.async (its own shared memory: no barrier
+// for the data).  Per step of R rows:
+//   sweep 1   the largest |w - mid| - rad of every thread; the m-th largest of the warps' best is the threshold;
+//   sweep 2   every column with |w - mid| + rad at or above it goes into the row's list;
+// and the ordering warps sort the lists of the step before meanwhile (two list buffers).  Both sweeps read W from
+// shared memory, HBM is read once.
+// The centre form is rounded, so the sweep tests against thr (1 - 2^-19): with rad rounded up, a column it
+// leaves out has |fl(x - w)| < thr (1 - 2^-19)(1 + 2^-21) < thr = tau for every row.
+template <int R, int NIT, int FT, int STAGES, bool VEC>
+__global__ void __launch_bounds__(FT + 32 * R) prune_filter(const PruneArgs a) {
+    constexpr int WARPS = FT / 32, TOP = 32 / WARPS, ALL = FT + 32 * R;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    const PruneProblem& p = a.p;
+    const int C = p.W_CI, lcap = a.lcap, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float4* stage = reinterpret_cast<float4*>(dyn);                                  // [STAGES][R][NIT][FT]
+    int2* lists = reinterpret_cast<int2*>(stage + STAGES * R * NIT * FT);            // [2][R][lcap] (column, w)
+    float* sorted = reinterpret_cast<float*>(lists + 2 * R * lcap);                  // [R][2][lcap] U as found, ordered
+    __shared__ unsigned top[2][R][32];
+    __shared__ float thr[2][R];
+    __shared__ int n_found[2][R];
+    __shared__ int hist[R][BUCKETS];
+    const int steps = (p.W_CO + R - 1) / R;
+    const float nan = __int_as_float(0x7fc00000);
+    if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
+    __syncthreads();
+
+    if (tid < FT) {
+        auto column = [&](int it, int e) { return it * 4 * FT + (VEC ? tid * 4 + e : e * FT + tid); };
+        float mid[NIT][4], rad[NIT][4];
+#pragma unroll
+        for (int it = 0; it < NIT; it++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int c = column(it, e);
+                const float hi = decode(c < C ? a.hi[c] : 0u), lo = -decode(c < C ? a.nlo[c] : 0u);
+                if (isinf(hi) || isinf(lo)) {
+                    mid[it][e] = 0.f;
+                    rad[it][e] = INFINITY;                   // always a candidate
+                } else {
+                    mid[it][e] = 0.5f * lo + 0.5f * hi;      // NaN without any value: never a candidate
+                    rad[it][e] = fmaxf(hi - mid[it][e], mid[it][e] - lo) * (1.0f + 0x1p-22f);
+                }
+            }
+        auto fetch = [&](int step, int st) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int j = step * R + r;
+#pragma unroll
+                for (int it = 0; it < NIT; it++) {
+                    float4* dst = stage + ((st * R + r) * NIT + it) * FT + tid;
+                    if (VEC) {
+                        const int c = column(it, 0);
+                        const bool ok = j < p.W_CO && c < C;
+                        cp_async16(smem_u32(dst), ok ? p.w + (size_t)j * C + c : p.w, ok ? 16 : 0);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int c = column(it, e);
+                            const bool ok = j < p.W_CO && c < C;
+                            cp_async4(smem_u32(reinterpret_cast<float*>(dst) + e), ok ? p.w + (size_t)j * C + c : p.w, ok ? 4 : 0);
+                        }
+                    }
+                }
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < STAGES; k++) {
+            const int step = blockIdx.x + k * gridDim.x;
+            if (step < steps) fetch(step, k);
+            cp_async_commit();
+        }
+        int i = 0, st = 0;
+        for (int step = blockIdx.x; step < steps; step += gridDim.x, i++) {
+            const int buf = i & 1;
+            cp_async_wait<STAGES - 1>();
+            const float4* rows = stage + st * R * NIT * FT + tid;
+            float best[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                best[r] = 0.f;
+#pragma unroll
+                for (int it = 0; it < NIT; it++) {
+                    const float4 w = rows[(r * NIT + it) * FT];
+                    best[r] = max3(best[r], fabsf(w.x - mid[it][0]) - rad[it][0], fabsf(w.y - mid[it][1]) - rad[it][1]);
+                    best[r] = max3(best[r], fabsf(w.z - mid[it][2]) - rad[it][2], fabsf(w.w - mid[it][3]) - rad[it][3]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                unsigned mine = __float_as_uint(best[r]);    // non-negative: integer order = float order
+                if (a.m == 1) {
+                    mine = __reduce_max_sync(0xffffffffu, mine);
+                    if (lane < TOP) top[buf][r][warp * TOP + lane] = lane == 0 ? mine : 0u;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < TOP; k++) {
+                        const unsigned mx = __reduce_max_sync(0xffffffffu, mine);
+                        const unsigned who = __ballot_sync(0xffffffffu, mine == mx);
+                        if (lane == __ffs(who) - 1) {
+                            top[buf][r][warp * TOP + k] = mx;
+                            mine = 0u;
+                        }
+                    }
+                }
+            }
+            if (i >= 2) bar_sync(BAR_EMPTY + buf, ALL);      // the ordering warps are done with this list buffer
+            bar_sync(BAR_FILTER, FT);
+            if (warp < R) {
+                unsigned v = top[buf][warp][lane], kth;
+                if (a.m == 1) {
+                    kth = __reduce_max_sync(0xffffffffu, v);
+                } else {
+                    int rank = 0;
+#pragma unroll
+                    for (int k = 0; k < 32; k++) {
+                        const unsigned o = __shfl_sync(0xffffffffu, v, k);
+                        rank += o > v || (o == v && k < lane);
+                    }
+                    kth = __reduce_max_sync(0xffffffffu, rank == a.m - 1 ? v : 0u);
+                }
+                if (lane == 0) thr[buf][warp] = __uint_as_float(kth) * (1.0f - 0x1p-21f);
+            }
+            bar_sync(BAR_FILTER, FT);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float t = thr[buf][r] * (1.0f - 0x1p-19f);
+                unsigned hit = 0u;
+#pragma unroll
+                for (int it = 0; it < NIT; it++) {
+                    const float4 w = rows[(r * NIT + it) * FT];
+                    if (fabsf(w.x - mid[it][0]) + rad[it][0] >= t) hit |= 1u << (4 * it);
+                    if (fabsf(w.y - mid[it][1]) + rad[it][1] >= t) hit |= 2u << (4 * it);
+                    if (fabsf(w.z - mid[it][2]) + rad[it][2] >= t) hit |= 4u << (4 * it);
+                    if (fabsf(w.w - mid[it][3]) + rad[it][3] >= t) hit |= 8u << (4 * it);
+                }
+                const int mine = __popc(hit);
+                if (!__any_sync(0xffffffffu, mine != 0)) continue;
+                int incl = mine;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += o;
+                }
+                int base = 0;
+                if (lane == 31) base = atomicAdd(&n_found[buf][r], incl);
+                int at = __shfl_sync(0xffffffffu, base, 31) + incl - mine;
+                while (hit) {
+                    const int k = __ffs(hit) - 1;
+                    hit &= hit - 1;
+                    if (at < lcap)
+                        lists[(buf * R + r) * lcap + at] =
+                            make_int2(column(k >> 2, k & 3), reinterpret_cast<const int*>(rows + (r * NIT + (k >> 2)) * FT)[k & 3]);
+                    at++;
+                }
+            }
+            bar_arrive(BAR_FULL + buf, ALL);
+            const int next = step + STAGES * (int)gridDim.x;
+            if (next < steps) fetch(next, st);
+            cp_async_commit();
+            st = st + 1 == STAGES ? 0 : st + 1;
+        }
+        cp_async_wait<0>();
+        return;
+    }
+
+    // ordering warps: list r of every step, by U, largest first, in BUCKETS steps of U
+    const int r = warp - WARPS;
+    float* u_in = sorted + 2 * r * lcap;
+    float* u_out = u_in + lcap;
+    int i = 0;
+    for (int step = blockIdx.x; step < steps; step += gridDim.x, i++) {
+        const int buf = i & 1, j = step * R + r;
+        bar_sync(BAR_FULL + buf, ALL);
+        const int2* c_in = lists + (buf * R + r) * lcap;
+        const int n = n_found[buf][r];
+        const float t = thr[buf][r];
+        if (j < p.W_CO && n <= lcap) {
+            float umax = 0.f;
+            for (int k = lane; k < n; k += 32) {
+                const int2 e = c_in[k];
+                const float hi = decode(a.hi[e.x]), lo = -decode(a.nlo[e.x]), w = __int_as_float(e.y);
+                const float u = fmaxf(hi - w, w - lo);       // exact: rounding is monotone
+                u_in[k] = u;
+                umax = fmaxf(umax, u);
+            }
+            umax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(umax)));
+            const float scale = umax > t ? (BUCKETS - 0.01f) / (umax - t) : 0.f;
+            auto bucket = [&](float u) { return min(BUCKETS - 1, max(0, (int)((umax - u) * scale))); };
+            hist[r][lane] = 0;
+            __syncwarp();
+            for (int k = lane; k < n; k += 32) atomicAdd(&hist[r][bucket(u_in[k])], 1);
+            __syncwarp();
+            {
+                const int h = hist[r][lane];
+                int incl = h;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += o;
+                }
+                hist[r][lane] = incl - h;
+            }
+            __syncwarp();
+            int2* c_out = a.cand + (size_t)j * lcap;
+            const int padded = (n + PAD - 1) / PAD * PAD;
+            for (int k = lane; k < n; k += 32) {
+                const float u = u_in[k];
+                const int at = atomicAdd(&hist[r][bucket(u)], 1);
+                u_out[at] = u;
+                c_out[at] = c_in[k];
+            }
+            for (int k = n + lane; k < padded; k += 32) {
+                u_out[k] = 0.f;
+                c_out[k] = make_int2(c_in[0].x, __float_as_int(nan));   // w = NaN: changes nothing
+            }
+            __syncwarp();
+            // ub[b]: no entry of step b or later has a larger U
+            const int nb = padded / STEP;
+            float tail = 0.f;
+            for (int base = (nb - 1) / 32 * 32; base >= 0; base -= 32) {
+                const int b = base + lane;
+                float v = 0.f;
+                if (b < nb)
+                    for (int e = 0; e < STEP; e++) v = fmaxf(v, u_out[b * STEP + e]);
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const float o = __shfl_down_sync(0xffffffffu, v, d);
+                    if (lane + d < 32) v = fmaxf(v, o);
+                }
+                v = fmaxf(v, tail);
+                if (b < nb) a.ub[(size_t)j * (lcap / STEP) + b] = v;
+                tail = __shfl_sync(0xffffffffu, v, 0);
+            }
+        }
+        if (lane == 0) {
+            if (j < p.W_CO) {
+                a.cnt[j] = n <= lcap ? n : -1;
+                a.tau[j] = t;
+            }
+            n_found[buf][r] = 0;
+        }
+        __syncwarp();
+        if (step + 2 * (int)gridDim.x < steps) bar_arrive(BAR_EMPTY + buf, ALL);
+    }
+}
+
+// ---- one column against the 32 rows of a warp ----------------------------------------------------
+// Argmax word of the reference: position | sign bit of (x - w); the lowest position wins a tie, whatever
+// the order in which the columns come.
+__device__ __forceinline__ void take_word(float v, uint32_t idx, bool negative, float& acc, uint32_t& word) {
+    if (v > acc || (v == acc && word != SNB_NO_GRAD_ID && idx < (word & ~SNB_SIGN_BIT))) {
+        acc = v;
+        word = idx | (negative ? SNB_SIGN_BIT : 0u);
+    }
+}
+
+// Running result of one output (K = 1): plain maxima, or maxima with their words.
+template <int NX, bool TRACK>
+struct MaxState {
+    float acc[NX];
+    uint32_t word[TRACK ? NX : 1];
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int t = 0; t < NX; t++) acc[t] = SNB_EPS;
+        if (TRACK) {
+            word[0] = NX == 2 ? SNB_NO_GRAD_ID : 0u;         // lower bound: no gradient until it leaves its floor
+            if (NX == 2) word[NX - 1] = 0u;
+        }
+    }
+    // v: the row's values of this column (x | l, u | x, l, u)
+    __device__ __forceinline__ void add(const float (&v)[NX], float w, uint32_t idx) {
+        if (NX != 2) {
+            const float t = v[0] - w;
+            if (TRACK) take_word(fabsf(t), idx, t < 0.f, acc[0], word[0]);
+            else acc[0] = fmaxf(acc[0], fabsf(t));
+        }
+        if (NX >= 2) {
+            const float t1 = w - v[NX - 2], t2 = v[NX - 1] - w;
+            if (TRACK) {
+                const bool second = !(t1 <= t2);
+                take_word(fmaxf(-t1, -t2), idx, second, acc[NX - 2], word[0]);
+                take_word(fmaxf(t1, t2), idx, second, acc[NX - 1], word[TRACK ? NX - 1 : 0]);
+            } else {
+                acc[NX - 2] = max3(acc[NX - 2], -t1, -t2);
+                acc[NX - 1] = max3(acc[NX - 1], t1, t2);
+            }
+        }
+    }
+    __device__ __forceinline__ float worst() const {
+        float m = acc[0];
+#pragma unroll
+        for (int t = 1; t < NX; t++) m = fminf(m, acc[t]);
+        return m;
+    }
+};
+
+// The KMAX largest values of one output, ascending; slots above the number of values seen stay 0.
+template <int KMAX>
+struct TopList {
+    float v[KMAX];
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int s = 0; s < KMAX; s++) v[s] = 0.f;
+    }
+    // warp-uniform branch: a value that beats no row's weakest slot changes nothing
+    __device__ __forceinline__ void add(float d) {
+        if (__any_sync(0xffffffffu, d > v[0])) {
+            const float e = d == d ? d : 0.f;                // a NaN must not move the list
+#pragma unroll
+            for (int s = 0; s < KMAX - 1; s++) v[s] = fmaxf(v[s], fminf(v[s + 1], e));
+            v[KMAX - 1] = fmaxf(v[KMAX - 1], e);
+        }
+    }
+    __device__ __forceinline__ float kth(int K) const {
+        float r = v[0];
+#pragma unroll
+        for (int s = 1; s < KMAX; s++)
+            if (s == KMAX - K) r = v[s];
+        return r;
+    }
+    // (eps0 + sum_r q (1-q)^r v_r) / (1 - (1-q)^K), largest first, in the reference's order of operations
+    __device__ __forceinline__ float combine(int K, float q, float eps0) const {
+        float ans = eps0, c = 1.0f;
+#pragma unroll
+        for (int r = 0; r < KMAX; r++)
+            if (r < K) {
+                ans += v[KMAX - 1 - r] * c * q;
+                c *= 1 - q;
+            }
+        return ans / (1 - c);
+    }
+};
+
+template <int NX, int KMAX>
+struct SortState {
+    TopList<KMAX> top[NX];
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int t = 0; t < NX; t++) top[t].init();
+    }
+    __device__ __forceinline__ void add(const float (&v)[NX], float w, uint32_t) {
+        if (NX != 2) top[0].add(fabsf(v[0] - w));
+        if (NX >= 2) {
+            const float t1 = w - v[NX - 2], t2 = v[NX - 1] - w;
+            top[NX - 2].add(fmaxf(-t1, -t2));
+            top[NX - 1].add(fmaxf(t1, t2));
+        }
+    }
+    __device__ __forceinline__ float worst(int K) const {
+        float m = top[0].kth(K);
+#pragma unroll
+        for (int t = 1; t < NX; t++) m = fminf(m, top[t].kth(K));
+        return m;
+    }
+    // the lower bound's list holds the mirrored values: -combine(-1e-10, -v) = combine(1e-10, v)
+    __device__ __forceinline__ float result(int t, int K, float q) const { return top[t].combine(K, q, SNB_EPS); }
+};
+
+// Positions of the K largest values, given a lower bound `floor_` of the K-th: columns must come in
+// ascending order.  A value enters when it beats the weakest entry and passes every entry that it is >=
+// to (the later of two equal columns ranks higher), the reference's bubble rule.
+template <int KMAX>
+struct PosList {
+    float v[KMAX];
+    uint32_t word[KMAX];
+    float seed;
+    __device__ __forceinline__ void init(float floor_) {
+#pragma unroll
+        for (int s = 0; s < KMAX; s++) v[s] = 0.f, word[s] = 0u;
+        seed = floor_ > 0.f ? __int_as_float(__float_as_int(floor_) - 1) : 0.f;
+    }
+    // entries KMAX - K .. KMAX - 1 are in use
+    __device__ __forceinline__ void add(float t, uint32_t c, int K) {
+        const float d = fabsf(t);
+        if (!__any_sync(0xffffffffu, d > seed)) return;
+        float weakest = v[0];
+#pragma unroll
+        for (int s = 1; s < KMAX; s++)
+            if (s == KMAX - K) weakest = v[s];
+        const bool enter = d > seed && d > weakest;
+        const uint32_t wd = c | (t >= 0.f ? 0u : SNB_SIGN_BIT);
+#pragma unroll
+        for (int s = 0; s < KMAX; s++) {
+            if (s < KMAX - K) continue;
+            const bool here = enter && (s == KMAX - K || d >= v[s]);
+            const bool above = s + 1 < KMAX && enter && d >= v[s + 1 < KMAX ? s + 1 : s];
+            v[s] = above ? v[s + 1 < KMAX ? s + 1 : s] : (here ? d : v[s]);
+            word[s] = above ? word[s + 1 < KMAX ? s + 1 : s] : (here ? wd : word[s]);
+        }
+    }
+};
+
+// ---- list walks -----------------------------------------------------------------------------------
+// CTA = 32 outputs of one sub-batch, eight lanes per output, four rows per lane (one 16-byte load of xt per tensor and
+// column): a warp walks four lists side by side.  A step is STEP columns; the entries of the next step are fetched
+// while this one's columns are on their way; a walk ends when the largest U left is below the results of all 32 rows.
+// Bound by the latency of the two dependent loads (list, column) and by the columns' traffic from L2.
+// TRACK keeps the list entry that set each maximum; the word is made from it at the end.  An equal value met
+// on the way (rare) sends the warp over the list once more for the lowest position.
+template <int NX, bool TRACK>
+__global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
+    constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
+    constexpr int WORDS = TRACK ? NX : 0;
+    __shared__ float tile[NV + WORDS][32][33];
+    __shared__ unsigned failed;
+    const PruneProblem& p = a.p;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l = lane & 7;
+    const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, slot = warp * 4 + g, n = n0 + slot;
+    const float4* xt = reinterpret_cast<const float4*>(a.xt + (size_t)s * C * NX * 32) + l;
+    if (tid == 0) failed = 0u;
+    __syncthreads();
+    const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
+    const int cnt = n < p.CO ? a.cnt[j] : 0;
+    const float tau = a.tau[j];
+    const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
+    const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
+    const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
+
+    float acc[NV][4];
+    int at[TRACK ? NV : 1][TRACK ? 4 : 1];
+    bool tied = false;
+#pragma unroll
+    for (int t = 0; t < NV; t++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            acc[t][q] = q < live ? SNB_EPS : INFINITY;       // rows past the batch never hold a walk up
+            if (TRACK) at[TRACK ? t : 0][TRACK ? q : 0] = -1;
+        }
+    auto worst = [&]() {
+        float m = acc[0][0];
+#pragma unroll
+        for (int t = 0; t < NV; t++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) m = fminf(m, acc[t][q]);
+        return m;
+    };
+    // the row's values for column value(s) x and weight w
+    auto values = [&](const float (&x)[NX], float w, float (&v)[NV]) {
+        if (NX != 2) v[0] = fabsf(x[0] - w);
+        if (NX >= 2) {
+            const float t1 = w - x[NX - 2], t2 = x[NX - 1] - w;
+            v[NV - 2] = fmaxf(-t1, -t2);
+            v[NV - 1] = fmaxf(t1, t2);
+        }
+    };
+    bool active = cnt > 0;
+    int4 e01 = make_int4(0, 0, 0, 0), e23 = e01;
+    float left = 0.f;
+    if (active) e01 = list[0], e23 = list[1];
+    for (int b = 0;; b++) {
+        if (b > 0) {
+            const unsigned over = __ballot_sync(0xffffffffu, worst() > left);
+            active = active && b * STEP < cnt && ((over >> (8 * g)) & 0xffu) != 0xffu;
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        if (active) {
+            const int c[STEP] = {e01.x, e01.z, e23.x, e23.z};
+            const float w[STEP] = {__int_as_float(e01.y), __int_as_float(e01.w), __int_as_float(e23.y), __int_as_float(e23.w)};
+            float4 x[STEP][NX];
+#pragma unroll
+            for (int e = 0; e < STEP; e++)
+#pragma unroll
+                for (int t = 0; t < NX; t++) x[e][t] = xt[((size_t)c[e] * NX + t) * 8];
+            if ((b + 1) * STEP < cnt) {
+                e01 = list[2 * b + 2];
+                e23 = list[2 * b + 3];
+                left = ub[b + 1];
+            }
+#pragma unroll
+            for (int e = 0; e < STEP; e++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float xq[NX], v[NV];
+#pragma unroll
+                    for (int t = 0; t < NX; t++) xq[t] = q == 0 ? x[e][t].x : q == 1 ? x[e][t].y : q == 2 ? x[e][t].z : x[e][t].w;
+                    values(xq, w[e], v);
+#pragma unroll
+                    for (int t = 0; t < NV; t++) {
+                        if (TRACK) {
+                            int& k = at[TRACK ? t : 0][TRACK ? q : 0];
+                            if (v[t] == acc[t][q]) tied = tied || k >= 0;
+                            if (v[t] > acc[t][q]) k = b * STEP + e;
+                        }
+                        acc[t][q] = fmaxf(acc[t][q], v[t]);
+                    }
+                }
+        }
+    }
+    const unsigned good = __ballot_sync(0xffffffffu, worst() >= tau);
+    if (l == 0 && n < p.CO && (cnt < 0 || ((good >> (8 * g)) & 0xffu) != 0xffu)) atomicOr(&failed, 1u << slot);
+#pragma unroll
+    for (int t = 0; t < NV; t++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) tile[t][4 * l + q][slot] = acc[t][q];
+    if (TRACK) {
+        const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
+        const int2* entries = a.cand + (size_t)j * a.lcap;
+        const float* xs = reinterpret_cast<const float*>(xt);
+        uint32_t word[TRACK ? NV : 1][4];
+        // word of the entry k for row q
+        auto make_word = [&](int t, int q, int k) {
+            const int2 e = entries[k];
+            const uint32_t idx = (uint32_t)(inv ? inv[e.x] : e.x);
+            const float w = __int_as_float(e.y);
+            const float x0 = xs[(size_t)e.x * NX * 32 + q];
+            if (NX == 1) return idx | (x0 - w < 0.f ? SNB_SIGN_BIT : 0u);
+            const float x1 = xs[((size_t)e.x * NX + NX - 1) * 32 + q];
+            return idx | (w - x0 <= x1 - w ? 0u : SNB_SIGN_BIT);
+        };
+#pragma unroll
+        for (int t = 0; t < NV; t++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int k = at[TRACK ? t : 0][TRACK ? q : 0];
+                word[TRACK ? t : 0][q] = k >= 0 ? make_word(t, q, k) : (NX == 2 && t == 0) ? SNB_NO_GRAD_ID : 0u;
+            }
+        if (tied) {
+#pragma unroll 1
+            for (int k = 0; k < cnt; k++) {
+                const int2 e = entries[k];
+                for (int q = 0; q < live; q++) {
+                    float xq[NX], v[NV];
+#pragma unroll
+                    for (int t = 0; t < NX; t++) xq[t] = xs[((size_t)e.x * NX + t) * 32 + q];
+                    values(xq, __int_as_float(e.y), v);
+#pragma unroll
+                    for (int t = 0; t < NV; t++)
+#pragma unroll
+                        for (int r = 0; r < 4; r++)
+                            if (r == q && at[TRACK ? t : 0][TRACK ? r : 0] >= 0 && v[t] == acc[t][r]) {
+                                const uint32_t other = make_word(t, q, k);
+                                uint32_t& wd = word[TRACK ? t : 0][r];
+                                if ((other & ~SNB_SIGN_BIT) < (wd & ~SNB_SIGN_BIT)) wd = other;
+                            }
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < NV; t++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) tile[NV + (TRACK ? t : 0)][4 * l + q][slot] = __uint_as_float(word[TRACK ? t : 0][q]);
+    }
+    __syncthreads();
+    float* outs[NV + WORDS];
+    if (NX != 2) outs[0] = p.y;
+    if (NX >= 2) outs[NX - 2] = p.yl, outs[NX - 1] = p.yu;
+    if (TRACK && NX == 1) outs[1] = reinterpret_cast<float*>(p.pos);
+    if (TRACK && NX == 2) outs[NX] = reinterpret_cast<float*>(p.posl), outs[NX + WORDS - 1] = reinterpret_cast<float*>(p.posu);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int r = warp + 8 * k, b = s * 32 + r, no = n0 + lane;
+        if (b >= p.B || no >= p.CO) continue;
+#pragma unroll
+        for (int t = 0; t < NV + WORDS; t++) outs[t][(size_t)b * p.CO + no] = tile[t][r][lane];
+    }
+    if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
+}
+
+// Positions of one output whose K-th largest value is shared by several columns in some row: the entries of
+// the list in ascending column order through PosList (rare; 32 lanes pick the next column together).
+template <int KMAX>
+__device__ __noinline__ void ordered_positions(const int2* entries, int cnt, const float* xt, float least, int K,
+                                               float (*words)[32][33], int slot) {
+    const int lane = threadIdx.x & 31;
+    PosList<KMAX> pl;
+    pl.init(least);
+    int last = -1;
+    for (;;) {
+        uint32_t next = 0xffffffffu;                         // (column << 9 | entry) of the lowest column above `last`
+        for (int k = lane; k < cnt; k += 32) {
+            const int c = entries[k].x;
+            if (c > last) next = min(next, (uint32_t)c << 9 | (uint32_t)k);
+        }
+        next = __reduce_min_sync(0xffffffffu, next);
+        if (next == 0xffffffffu) break;
+        const int2 e = entries[next & 511u];
+        last = e.x;
+        pl.add(xt[(size_t)e.x * 32] - __int_as_float(e.y), (uint32_t)e.x, K);
+    }
+#pragma unroll
+    for (int k = 0; k < KMAX; k++)
+        if (k < K) words[k][lane][slot] = __uint_as_float(pl.word[KMAX - 1 - k]);
+}
+
+// The sort neuron over the same lists, one warp per output, lane = row; POS: the K positions too.  Bound by the
+// issue rate of the insertion chains.  With the values known, a second walk finds the positions: the rank of an
+// element among a row's K largest is the number of larger values in the row's list, and of equal values the later column
+// comes first.  Only where more columns share the K-th value than there is room for does the order of insertion
+// decide (ordered_positions).
+template <int NX, int KMAX, bool POS>
+__global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
+    constexpr uint32_t EMPTY = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(dyn);   // [NX] values, then [K] words
+    __shared__ unsigned failed;
+    const PruneProblem& p = a.p;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, K = p.K;
+    const bool live = s * 32 + lane < p.B;
+    const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
+    if (tid == 0) failed = 0u;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 0; i < 4; i++) {
+        const int slot = warp * 4 + i, j = n0 + slot;
+        if (j >= p.CO) break;
+        const int cnt = a.cnt[j];
+        const float tau = a.tau[j];
+        const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
+        const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
+        SortState<NX, KMAX> st;
+        st.init();
+        int k = 0;                                           // entries seen
+        for (; k < cnt; k += PAD) {
+            if (k >= K) {
+                const float left = ub[k / STEP];
+                if (__all_sync(0xffffffffu, !live || st.worst(K) > left)) break;
+            }
+            float w[PAD], v[PAD][NX];
+#pragma unroll
+            for (int e = 0; e < PAD / 2; e++) {
+                const int4 two = list[k / 2 + e];
+                w[2 * e] = __int_as_float(two.y);
+                w[2 * e + 1] = __int_as_float(two.w);
+#pragma unroll
+                for (int t = 0; t < NX; t++) {
+                    v[2 * e][t] = xt[((size_t)two.x * NX + t) * 32];
+                    v[2 * e + 1][t] = xt[((size_t)two.z * NX + t) * 32];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < PAD; e++) st.add(v[e], w[e], 0u);
+        }
+        const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || st.worst(K) >= tau);
+        if (!good && lane == 0) atomicOr(&failed, 1u << slot);
+#pragma unroll
+        for (int t = 0; t < NX; t++) tile[t][lane][slot] = st.result(t, K, p.q);
+        if (POS && good) {
+            const float least = st.top[0].kth(K);
+            bool crowded = false;
+            for (int r = 0; r < K; r++) tile[NX + r][lane][slot] = __uint_as_float(EMPTY);
+            for (int k2 = 0; k2 < k; k2 += PAD) {
+                int c[PAD];
+                float w[PAD], v[PAD];
+#pragma unroll
+                for (int e = 0; e < PAD / 2; e++) {
+                    const int4 two = list[k2 / 2 + e];
+                    c[2 * e] = two.x;
+                    w[2 * e] = __int_as_float(two.y);
+                    c[2 * e + 1] = two.z;
+                    w[2 * e + 1] = __int_as_float(two.w);
+                    v[2 * e] = xt[(size_t)two.x * 32];
+                    v[2 * e + 1] = xt[(size_t)two.z * 32];
+                }
+#pragma unroll
+                for (int e = 0; e < PAD; e++) {
+                    const float t = v[e] - w[e], d = fabsf(t);
+                    const bool hit = d >= least && d > 0.f;
+                    if (!__any_sync(0xffffffffu, hit)) continue;
+                    int rank = 0;
+#pragma unroll
+                    for (int r = 0; r < KMAX; r++) rank += st.top[0].v[r] > d;
+                    if (hit) {
+                        uint32_t word = (uint32_t)c[e] | (t >= 0.f ? 0u : SNB_SIGN_BIT);
+                        for (; rank < K; rank++) {           // past equal values of later columns
+                            const uint32_t other = __float_as_uint(tile[NX + rank][lane][slot]);
+                            if (other == EMPTY || (other & ~SNB_SIGN_BIT) < (word & ~SNB_SIGN_BIT)) {
+                                tile[NX + rank][lane][slot] = __uint_as_float(word);
+                                word = other;
+                            }
+                            if (word == EMPTY) break;
+                        }
+                        crowded = crowded || rank == K;
+                    }
+                }
+            }
+            if (__any_sync(0xffffffffu, live && crowded))
+                ordered_positions<KMAX>(a.cand + (size_t)j * a.lcap, cnt, xt, live ? least : 0.f, K, tile + NX, slot);
+        }
+    }
+    __syncthreads();
+    float* outs[NX];
+    if (NX != 2) outs[0] = p.y;
+    if (NX >= 2) outs[NX - 2] = p.yl, outs[NX - 1] = p.yu;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int r = warp + 8 * k, b = s * 32 + r, n = n0 + lane;
+        if (b >= p.B || n >= p.CO) continue;
+#pragma unroll
+        for (int t = 0; t < NX; t++) outs[t][(size_t)b * p.CO + n] = tile[t][r][lane];
+        if (POS)
+            for (int t = 0; t < K; t++) {
+                const uint32_t word = __float_as_uint(tile[NX + t][r][lane]);
+                p.pos[((size_t)t * p.B + b) * p.CO + n] = word == EMPTY ? 0 : (int)word;   // fewer than K values above 0
+            }
+    }
+    if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
+}
+
+// ---- outputs whose list was not enough ------------------------------------------------------------
+// Persistent CTAs over the recorded units (32 outputs of one sub-batch, a mask of those to redo).  A few
+// outputs: the eight warps share the columns of one output.  Many: warp = four outputs side by side over all
+// columns, xt staged in shared memory for the eight warps, W read along rows by uniform 16-byte loads; that is the dense
+// evaluation of unprunable data, bound by the issue rate of subtract and max like any max-plus product.
+constexpr int FIX_K = 32;           // columns per stage
+constexpr int FIX_FEW = 4;
+
+template <int NX>
+__device__ __forceinline__ void fix_stage(const float* xt_s, float* sm, int k0, int C) {
+    const int n = min(FIX_K, C - k0) * NX * 8;               // 16-byte pieces; the columns of a sub-batch are contiguous
+    const float* src = xt_s + (size_t)k0 * NX * 32;
+    for (int k = threadIdx.x; k < n; k += 256) cp_async16(smem_u32(sm + k * 4), src + k * 4, 16);
+}
+
+template <int NX, bool TRACK>
+__global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
+    __shared__ __align__(16) float sm[2][FIX_K * NX * 32];
+    const PruneProblem& p = a.p;
+    const int count = (int)*a.fail_count;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = p.W_CI;
+    for (int unit = blockIdx.x; unit < count; unit += gridDim.x) {
+        const int4 f = a.fail[unit];
+        const int s = f.x, n0 = f.y;
+        const unsigned mask = (unsigned)f.z;
+        const float* xs = a.xt + (size_t)s * C * NX * 32;
+        const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
+        const int b = s * 32 + lane;
+        auto store = [&](const MaxState<NX, TRACK>& st, int n) {
+            if (b >= p.B) return;
+            const size_t o = (size_t)b * p.CO + n;
+            if (NX != 2) p.y[o] = st.acc[0];
+            if (NX >= 2) p.yl[o] = st.acc[NX - 2], p.yu[o] = st.acc[NX - 1];
+            if (TRACK && NX == 1) p.pos[o] = (int)st.word[0];
+            if (TRACK && NX == 2) p.posl[o] = (int)st.word[0], p.posu[o] = (int)st.word[TRACK ? NX - 1 : 0];
+        };
+        if (__popc(mask) <= FIX_FEW) {
+            unsigned todo = mask;
+            while (todo) {
+                const int n = n0 + __ffs(todo) - 1;
+                todo &= todo - 1;
+                const float* wr = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
+                MaxState<NX, TRACK> st;
+                st.init();
+                for (int c0 = warp * 8; c0 < C; c0 += 64) {
+                    float v[8][NX], w[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        const int c = min(c0 + e, C - 1);            // a repeated column changes nothing
+                        w[e] = wr[c];
+#pragma unroll
+                        for (int t = 0; t < NX; t++) v[e][t] = xs[((size_t)c * NX + t) * 32 + lane];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        const int c = min(c0 + e, C - 1);
+                        st.add(v[e], w[e], TRACK ? (uint32_t)(inv ? inv[c] : c) : 0u);
+                    }
+                }
+                float* part = &sm[0][0];                             // [8 warps][NX (+ NX words)][32]
+                constexpr int PER = (TRACK ? 2 : 1) * NX;
+                static_assert(8 * PER * 32 <= 2 * FIX_K * NX * 32, "partial results fit the stages");
+                __syncthreads();
+#pragma unroll
+                for (int t = 0; t < NX; t++) {
+                    part[(warp * PER + t) * 32 + lane] = st.acc[t];
+                    if (TRACK) part[(warp * PER + NX + t) * 32 + lane] = __uint_as_float(st.word[TRACK ? t : 0]);
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    for (int k = 1; k < 8; k++)
+#pragma unroll
+                        for (int t = 0; t < NX; t++) {
+                            const float v = part[(k * PER + t) * 32 + lane];
+                            if (TRACK) {
+                                const uint32_t wd = __float_as_uint(part[(k * PER + NX + t) * 32 + lane]);
+                                if (wd != SNB_NO_GRAD_ID)
+                                    take_word(v, wd & ~SNB_SIGN_BIT, (wd & SNB_SIGN_BIT) != 0, st.acc[t], st.word[TRACK ? t : 0]);
+                            } else {
+                                st.acc[t] = fmaxf(st.acc[t], v);
+                            }
+                        }
+                    store(st, n);
+                }
+            }
+            __syncthreads();
+            continue;
+        }
+        MaxState<NX, TRACK> st[4];
+        const float* wr[4];
+        const bool vec = (C % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.w) & 15u) == 0);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int n = min(n0 + warp * 4 + i, p.CO - 1);
+            wr[i] = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
+            st[i].init();
+        }
+        fix_stage<NX>(xs, sm[0], 0, C);
+        cp_async_commit();
+        for (int k0 = 0, cur = 0; k0 < C; k0 += FIX_K, cur ^= 1) {
+            cp_async_wait<0>();
+            __syncthreads();
+            if (k0 + FIX_K < C) fix_stage<NX>(xs, sm[cur ^ 1], k0 + FIX_K, C);
+            cp_async_commit();
+            const int kn = min(FIX_K, C - k0);
+            for (int k = 0; k < kn; k += 4) {
+                float w[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (vec) {
+                        const float4 q = __ldg(reinterpret_cast<const float4*>(wr[i] + k0 + k));
+                        w[i][0] = q.x; w[i][1] = q.y; w[i][2] = q.z; w[i][3] = q.w;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) w[i][e] = __ldg(wr[i] + min(k0 + k + e, C - 1));
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    if (k + e >= kn) break;
+                    float v[NX];
+#pragma unroll
+                    for (int t = 0; t < NX; t++) v[t] = sm[cur][((k + e) * NX + t) * 32 + lane];
+                    const uint32_t idx = TRACK ? (uint32_t)(inv ? inv[k0 + k + e] : k0 + k + e) : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) st[i].add(v, w[i][e], idx);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int slot = warp * 4 + i;
+            if ((mask >> slot) & 1u) store(st[i], n0 + slot);
+        }
+        __syncthreads();
+    }
+}
+
+template <int NX, int KMAX, bool POS>
+__global__ void __launch_bounds__(256) prune_fix_sort(const PruneArgs a) {
+    __shared__ __align__(16) float sm[2][FIX_K * NX * 32];
+    const PruneProblem& p = a.p;
+    const int count = (int)*a.fail_count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = p.W_CI, K = p.K;
+    for (int unit = blockIdx.x; unit < count; unit += gridDim.x) {
+        const int4 f = a.fail[unit];
+        const int s = f.x, n0 = f.y, b = s * 32 + lane;
+        const unsigned mask = (unsigned)f.z;
+        const float* xs = a.xt + (size_t)s * C * NX * 32;
+        for (int i = 0; i < 4; i++) {
+            const int slot = warp + 8 * i;                          // the CTA's warps do eight outputs at a time
+            if (((mask >> (8 * i)) & 0xffu) == 0u) continue;
+            const bool mine = (mask >> slot) & 1u;
+            const int n = min(n0 + slot, p.CO - 1);
+            const float* wr = p.w + (size_t)n * C;
+            const size_t o = (size_t)b * p.CO + n;
+            auto sweep = [&](auto&& body) {
+                __syncthreads();
+                fix_stage<NX>(xs, sm[0], 0, C);
+                cp_async_commit();
+                for (int k0 = 0, cur = 0; k0 < C; k0 += FIX_K, cur ^= 1) {
+                    cp_async_wait<0>();
+                    __syncthreads();
+                    if (k0 + FIX_K < C) fix_stage<NX>(xs, sm[cur ^ 1], k0 + FIX_K, C);
+                    cp_async_commit();
+                    if (!mine) continue;
+                    const int kn = min(FIX_K, C - k0);
+                    const float wl = lane < kn ? wr[k0 + lane] : 0.f;
+                    for (int k = 0; k < kn; k++) {
+                        float v[NX];
+#pragma unroll
+                        for (int t = 0; t < NX; t++) v[t] = sm[cur][(k * NX + t) * 32 + lane];
+                        body(v, __shfl_sync(0xffffffffu, wl, k), (uint32_t)(k0 + k));
+                    }
+                }
+            };
+            SortState<NX, KMAX> st;
+            st.init();
+            sweep([&](const float(&v)[NX], float w, uint32_t c) { st.add(v, w, c); });
+            if (mine && b < p.B) {
+                if (NX != 2) p.y[o] = st.result(0, K, p.q);
+                if (NX >= 2) p.yl[o] = st.result(NX - 2, K, p.q), p.yu[o] = st.result(NX - 1, K, p.q);
+            }
+            if constexpr (POS) {
+                PosList<KMAX> pl;
+                pl.init(st.top[0].kth(K));
+                sweep([&](const float(&v)[NX], float w, uint32_t c) { pl.add(v[0] - w, c, K); });
+                if (mine && b < p.B) {
+#pragma unroll
+                    for (int k = 0; k < KMAX; k++)
+                        if (k < K) p.pos[((size_t)k * p.B + b) * p.CO + n] = (int)pl.word[KMAX - 1 - k];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+
+int tensors(const PruneProblem& p) { return (p.x ? 1 : 0) + (p.xl ? 2 : 0); }
+bool with_words(const PruneProblem& p) { return p.pos || p.posl; }
+
+// How many columns must reach the threshold.  Without masks K: the K-th largest value of every row then
+// reaches it by construction.  With column lists the m columns may all be missing from a sub-batch's list; m is chosen so
+// that this happens to about one output in 10^7 for random lists, and such outputs go to prune_fix.
+int threshold_rank(const PruneProblem& p) {
+    int m = p.K;
+    if (p.ci) {
+        const double gone = 1.0 - (double)p.CI / p.W_CI;
+        m = 1;
+        for (double all = gone; all > 1e-7 && m < 16; all *= gone) m++;
+    }
+    return m;
+}
+// List capacity: N(0,1)-like weights leave 35 columns on average for the maximum, 180 for ten values, 230 for rank 14.
+int list_capacity(const PruneProblem& p) {
+    const int m = threshold_rank(p);
+    const int want = m <= 2 ? 192 : 512;
+    const int c = (p.W_CI + PAD - 1) / PAD * PAD;
+    return c < want ? c : want;
+}
+
+size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
+    const size_t S = (p.B + 31) / 32, NX = tensors(p), lcap = list_capacity(p), C = p.W_CI, J = p.W_CO;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char* at = base + off;
+        off += up256(bytes);
+        return at;
+    };
+    char* zeroed = take(64 + 2 * up256(sizeof(unsigned) * C));    // counter and ranges: one memset
+    char* xt = take(sizeof(float) * S * C * NX * 32);
+    char* inv = take(p.ci ? sizeof(int) * S * C : 0);
+    char* cnt = take(sizeof(int) * J);
+    char* tau = take(sizeof(float) * J);
+    char* ub = take(sizeof(float) * J * (lcap / STEP));
+    char* cand = take(sizeof(int2) * J * lcap);
+    char* fail = take(sizeof(int4) * S * ((p.CO + 31) / 32));
+    if (a) {
+        a->p = p;
+        a->S = (int)S;
+        a->NX = (int)NX;
+        a->m = threshold_rank(p);
+        a->lcap = (int)lcap;
+        a->fail_count = reinterpret_cast<unsigned*>(zeroed);
+        a->hi = reinterpret_cast<unsigned*>(zeroed + 64);
+        a->nlo = reinterpret_cast<unsigned*>(zeroed + 64 + up256(sizeof(unsigned) * C));
+        a->xt = reinterpret_cast<float*>(xt);
+        a->inv = p.ci ? reinterpret_cast<int*>(inv) : nullptr;
+        a->cnt = reinterpret_cast<int*>(cnt);
+        a->tau = reinterpret_cast<float*>(tau);
+        a->ub = reinterpret_cast<float*>(ub);
+        a->cand = reinterpret_cast<int2*>(cand);
+        a->fail = reinterpret_cast<int4*>(fail);
+    }
+    return off;
+}
+
+template <auto KERN>
+cudaError_t set_smem(int bytes) {
+    static std::atomic<int> configured[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (bytes <= 48 * 1024 || configured[dev & 63].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) configured[dev & 63].store(bytes, std::memory_order_release);
+    return e;
+}
+
+// Persistent grid: as many CTAs as fit (the shared memory of the stages limits them to two per SM for wide rows).
+template <int R, int NIT, int FT, int STAGES, bool VEC>
+cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
+    const int smem = STAGES * R * NIT * FT * 16 + R * a.lcap * (2 * (int)sizeof(int2) + 2 * (int)sizeof(float));
+    cudaError_t e = set_smem<prune_filter<R, NIT, FT, STAGES, VEC>>(smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_filter<R, NIT, FT, STAGES, VEC>, FT + 32 * R, smem);
+    if (e != cudaSuccess) return e;
+    const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
+    prune_filter<R, NIT, FT, STAGES, VEC><<<steps < slots ? steps : slots, FT + 32 * R, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <bool VEC>
+cudaError_t filter(const PruneArgs& a, cudaStream_t st) {
+    const int C = a.p.W_CI;
+    if (C <= 1024) return launch_filter<4, 1, 256, 2, VEC>(a, st);
+    if (C <= 2048) return launch_filter<2, 2, 256, 2, VEC>(a, st);
+    if (C <= 3072) return launch_filter<2, 3, 256, 2, VEC>(a, st);
+    if (C <= 4096) return launch_filter<2, 4, 256, 2, VEC>(a, st);
+    if (C <= 5120) return launch_filter<2, 5, 256, 2, VEC>(a, st);
+    if (C <= 6144) return launch_filter<1, 6, 256, 2, VEC>(a, st);
+    if (C <= 8192) return launch_filter<1, 4, 512, 2, VEC>(a, st);
+    return launch_filter<1, 6, 512, 2, VEC>(a, st);
+}
+
+template <int NX, bool TRACK>
+cudaError_t run_max(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st) {
+    prune_max<NX, TRACK><<<grid, 256, 0, st>>>(a);
+    prune_fix_max<NX, TRACK><<<fix_grid, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <int NX, int KMAX, bool POS>
+cudaError_t run_sort(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st) {
+    const int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
+    cudaError_t e = set_smem<prune_sort<NX, KMAX, POS>>(smem);
+    if (e != cudaSuccess) return e;
+    prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
+    prune_fix_sort<NX, KMAX, POS><<<fix_grid, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+bool prune_applies(const PruneProblem& p) {
+    if (p.W_CI > MAX_COLUMNS) return false;
+    if (p.ci && 5ll * p.CI < 2ll * p.W_CI) return false;
+    if ((p.B + 31) / 32 > 65535) return false;
+    // the pruned form costs 20 to 30 us however small the problem; the dense kernels need that long at
+    const long long least = p.K > 1 ? 1ll << 20 : p.xl ? 4ll << 20 : 12ll << 20;
+    return (long long)p.B * p.CO * p.W_CI >= least && p.W_CI >= 128;
+}
+
+size_t prune_workspace_bytes(const PruneProblem& p) { return layout(p, nullptr, nullptr); }
+
+cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
+    PruneArgs a{};
+    layout(p, static_cast<char*>(ws), &a);
+    const size_t C = p.W_CI;
+    cudaError_t e = cudaMemsetAsync(a.fail_count, 0, 64 + 2 * up256(sizeof(unsigned) * C), st);
+    if (e != cudaSuccess) return e;
+    // all bits set is a NaN: the dropped columns
+    if (p.ci && (e = cudaMemsetAsync(a.xt, 0xff, sizeof(float) * a.S * C * a.NX * 32, st)) != cudaSuccess) return e;
+    const dim3 pg((p.CI + 63) / 64, a.S);
+    if (a.NX == 1) prune_prep<1><<<pg, 256, 0, st>>>(a);
+    else if (a.NX == 2) prune_prep<2><<<pg, 256, 0, st>>>(a);
+    else prune_prep<3><<<pg, 256, 0, st>>>(a);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = (C % 4 == 0) && aligned16(p.w) ? filter<true>(a, st) : filter<false>(a, st);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((p.CO + 31) / 32, a.S);
+    const int fg = sm_count() * 2;
+    if (p.K == 1) {
+        const bool track = with_words(p);
+        if (a.NX == 1) return track ? run_max<1, true>(a, grid, fg, st) : run_max<1, false>(a, grid, fg, st);
+        if (a.NX == 2) return track ? run_max<2, true>(a, grid, fg, st) : run_max<2, false>(a, grid, fg, st);
+        return run_max<3, false>(a, grid, fg, st);
+    }
+    if (p.K <= 10) {
+        if (a.NX == 1) return p.pos ? run_sort<1, 10, true>(a, grid, fg, st) : run_sort<1, 10, false>(a, grid, fg, st);
+        return a.NX == 2 ? run_sort<2, 10, false>(a, grid, fg, st) : run_sort<3, 10, false>(a, grid, fg, st);
+    }
+    if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, grid, fg, st) : run_sort<1, 25, false>(a, grid, fg, st);
+    return run_sort<2, 25, false>(a, grid, fg, st);
+}
+
+}  // namespace snb
+
+// Scratch with which the `_ws` entry points evaluate a problem in the pruned form: tensors = 1 (point value),
+// 2 (box) or 3 (both), K = 1 or the sort neuron's size, words = positions wanted, column_lists = kept-column
+// lists given.  0: the problem is too small or too wide for it, the entry points then need no (other) scratch.
+extern "C" size_t snb_prune_scratch_bytes(int tensors, int K, int words, int B, int CO, int CI, int W_CO, int W_CI,
+                                          int column_lists) {
+    if (B <= 0 || CO <= 0 || CI <= 0 || W_CO <= 0 || W_CI <= 0 || tensors < 1 || tensors > 3) return 0;
+    static const float some = 0.f;
+    static const int none = 0;
+    snb::PruneProblem p;
+    p.x = tensors != 2 ? &some : nullptr;
+    p.xl = tensors != 1 ? &some : nullptr;
+    p.ci = column_lists ? &none : nullptr;
+    static int word = 0;
+    p.pos = words ? &word : nullptr;
+    p.B = B, p.CO = CO, p.CI = CI, p.W_CO = W_CO, p.W_CI = W_CI, p.K = K;
+    return snb::prune_applies(p) ? snb::prune_workspace_bytes(p) : 0;
+}

@@ -1,0 +1,55 @@
+// Exact pruned evaluation of the max-type distance operators (l-infinity values, positions, interval
+// bounds, sort neurons): only the columns of W that can matter are looked at per row of the batch.
+//
+// max_c |x[b,c] - w[j,c]| over thousands of columns is decided by a handful of them.  With lo[c] and
+// hi[c] the smallest and largest value of column c of the input over the batch,
+//     L[j,c] = max(lo - w, w - hi, 0)  <=  |x[b,c] - w[j,c]|  <=  U[j,c] = max(hi - w, w - lo)
+// holds for every row b, in rounded fp32 arithmetic too (rounding is monotone).  A column whose U lies
+// below a threshold tau that the result reaches cannot be the maximum, nor tie with it.  Steps:
+//   prune_prep     transposes the input to xt[sub-batch][column][tensor][32 rows] (NaN where a column
+//                  was dropped or a row does not exist: NaN never enters a maximum) and collects lo / hi;
+//   prune_filter   reads W once: per row j the threshold tau (the m-th largest L among disjoint
+//                  groups of columns) and the list of columns with U >= tau, largest U first;
+//   prune_max / prune_sort   one warp per (sub-batch, output), lane = row: walks the list until no
+//                  remaining U can change any row, and CHECKS that every row's result (its K-th
+//                  largest value for the sort neuron) reaches tau.  Outputs that do not are recorded;
+//   prune_fix      evaluates the recorded outputs over all columns.
+// The result is exact whatever the data: the thresholds only decide how many columns are read.  Data
+// that cannot be pruned (rows of W whose entries all have about the same distance to the input)
+// ends in prune_fix, a dense kernel.
+#pragma once
+#include "common.cuh"
+#include "launch.h"
+
+namespace snb {
+
+struct PruneProblem {
+    // inputs: x [B, CI] (compact over ci when given) and / or the ends of a box xl, xu [B, W_CI]
+    const float* x = nullptr;
+    const float* xl = nullptr;
+    const float* xu = nullptr;
+    const float* w = nullptr;   // [W_CO, W_CI]
+    const int* ci = nullptr;    // [S, CI] kept columns per sub-batch, or null
+    const int* co = nullptr;    // [S, CO] kept rows of W per sub-batch, or null
+    int B = 0, CO = 0, CI = 0, W_CO = 0, W_CI = 0;
+    // outputs [B, CO]; positions optional
+    float* y = nullptr;
+    float* yl = nullptr;
+    float* yu = nullptr;
+    int* pos = nullptr;         // x: argmax words ([K][B][CO] for the sort neuron)
+    int* posl = nullptr;        // box: words of both bounds
+    int* posu = nullptr;
+    int K = 1;                  // 1: maximum; 2..25: sort neuron of that many values
+    float q = 0.f;
+};
+
+// Whether the pruned evaluation is the faster one for this problem (sizes only), and its scratch.
+bool prune_applies(const PruneProblem& p);
+size_t prune_workspace_bytes(const PruneProblem& p);
+// ws: prune_workspace_bytes(p) bytes, 16-byte aligned.
+cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st);
+inline bool prune_fits(const PruneProblem& p, const void* ws, size_t ws_bytes) {
+    return ws && aligned16(ws) && prune_applies(p) && ws_bytes >= prune_workspace_bytes(p);
+}
+
+}  // namespace snb

@@ -12,6 +12,7 @@
 #include "tile.cuh"
 #include "launch.h"
 #include "general_shapes.h"
+#include "prune.cuh"
 
 namespace snb {
 
@@ -512,20 +513,42 @@ static int check_sort(const void* x, const void* w, const void* y, int B, int CO
     return SNB_OK;
 }
 
-extern "C" int snb_sort_neuron_forward_nograd(const float* x, const float* w, int B, int CO, int CI, int G,
-                                              int HW, float* y, float q, int K, void* stream) {
+// Runs the pruned form when the scratch (snb_prune_scratch_bytes) allows it; *done tells.
+static int pruned_sort(const float* x, const float* xl, const float* xu, const float* w, int B, int CO, int CI, float* y,
+                       float* yl, float* yu, int* pos, float q, int K, void* ws, size_t ws_bytes, cudaStream_t st, bool* done) {
+    PruneProblem p;
+    p.x = x, p.xl = xl, p.xu = xu, p.w = w, p.y = y, p.yl = yl, p.yu = yu, p.pos = pos, p.K = K, p.q = q;
+    p.B = B, p.CO = p.W_CO = CO, p.CI = p.W_CI = CI;
+    *done = prune_fits(p, ws, ws_bytes);
+    if (*done) SNB_CUDA(prune_forward(p, ws, st));
+    return SNB_OK;
+}
+
+extern "C" int snb_sort_neuron_forward_nograd_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
+                                                 float* y, float q, int K, void* workspace, size_t workspace_bytes,
+                                                 void* stream) {
     if ((G != 1 || HW != 1) && q > 0.f && q < 1.f)
         return general_sort_forward(x, w, B, CO, CI, G, HW, y, nullptr, q, K, (cudaStream_t)stream);
     int rc = check_sort(x, w, y, B, CO, CI, G, HW, q, K);
     if (rc) return rc;
+    bool done = false;
+    rc = pruned_sort(x, nullptr, nullptr, w, B, CO, CI, y, nullptr, nullptr, nullptr, q, K, workspace, workspace_bytes,
+                     (cudaStream_t)stream, &done);
+    if (rc || done) return rc;
     SortParams p{x, x, w, y, nullptr, nullptr, B, CO, CI, K, q};
     SNB_CUDA(K <= 10 ? launch_sort_fwd<10, false>(p, (cudaStream_t)stream)
                      : launch_sort_fwd<25, false>(p, (cudaStream_t)stream));
     return SNB_OK;
 }
 
-extern "C" int snb_sort_neuron_forward(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
-                                       float* y, int* pos, float q, int K, void* stream) {
+extern "C" int snb_sort_neuron_forward_nograd(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
+                                              float* y, float q, int K, void* stream) {
+    return snb_sort_neuron_forward_nograd_ws(x, w, B, CO, CI, G, HW, y, q, K, nullptr, 0, stream);
+}
+
+extern "C" int snb_sort_neuron_forward_ws(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y,
+                                          int* pos, float q, int K, void* workspace, size_t workspace_bytes,
+                                          void* stream) {
     if ((G != 1 || HW != 1) && q > 0.f && q < 1.f) {
         if (!pos) return SNB_ERR_NULL_POINTER;
         return general_sort_forward(x, w, B, CO, CI, G, HW, y, pos, q, K, (cudaStream_t)stream);
@@ -533,6 +556,10 @@ extern "C" int snb_sort_neuron_forward(const float* x, const float* w, int B, in
     int rc = check_sort(x, w, y, B, CO, CI, G, HW, q, K);
     if (rc) return rc;
     if (!pos) return SNB_ERR_NULL_POINTER;
+    bool done = false;
+    rc = pruned_sort(x, nullptr, nullptr, w, B, CO, CI, y, nullptr, nullptr, pos, q, K, workspace, workspace_bytes,
+                     (cudaStream_t)stream, &done);
+    if (rc || done) return rc;
     SortParams p{x, x, w, y, nullptr, pos, B, CO, CI, K, q};
     dim3 grid((B + SP_ROWS - 1) / SP_ROWS, (CO + SP_COLS - 1) / SP_COLS);
     if (K <= 16) sort_fwd_pos_half_kernel<<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p);
@@ -541,18 +568,32 @@ extern "C" int snb_sort_neuron_forward(const float* x, const float* w, int B, in
     return SNB_OK;
 }
 
-extern "C" int snb_bound_sort_neuron_forward(const float* xl, const float* xu, const float* w, int B, int CO,
-                                             int CI, int G, int HW, float* yl, float* yu, float q, int K,
-                                             void* stream) {
+extern "C" int snb_sort_neuron_forward(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y,
+                                       int* pos, float q, int K, void* stream) {
+    return snb_sort_neuron_forward_ws(x, w, B, CO, CI, G, HW, y, pos, q, K, nullptr, 0, stream);
+}
+
+extern "C" int snb_bound_sort_neuron_forward_ws(const float* xl, const float* xu, const float* w, int B, int CO, int CI,
+                                                int G, int HW, float* yl, float* yu, float q, int K, void* workspace,
+                                                size_t workspace_bytes, void* stream) {
     if ((G != 1 || HW != 1) && q > 0.f && q < 1.f)
         return general_sort_bound_forward(xl, xu, w, B, CO, CI, G, HW, yl, yu, q, K, (cudaStream_t)stream);
     int rc = check_sort(xl, w, yl, B, CO, CI, G, HW, q, K);
     if (rc) return rc;
     if (!xu || !yu) return SNB_ERR_NULL_POINTER;
+    bool done = false;
+    rc = pruned_sort(nullptr, xl, xu, w, B, CO, CI, nullptr, yl, yu, nullptr, q, K, workspace, workspace_bytes,
+                     (cudaStream_t)stream, &done);
+    if (rc || done) return rc;
     SortParams p{xl, xu, w, yl, yu, nullptr, B, CO, CI, K, q};
     SNB_CUDA(K <= 10 ? launch_sort_fwd<10, true>(p, (cudaStream_t)stream)
                      : launch_sort_fwd<25, true>(p, (cudaStream_t)stream));
     return SNB_OK;
+}
+
+extern "C" int snb_bound_sort_neuron_forward(const float* xl, const float* xu, const float* w, int B, int CO, int CI,
+                                             int G, int HW, float* yl, float* yu, float q, int K, void* stream) {
+    return snb_bound_sort_neuron_forward_ws(xl, xu, w, B, CO, CI, G, HW, yl, yu, q, K, nullptr, 0, stream);
 }
 
 static int sort_backward(const float* g, const int* pos, int B, int CO, int CI, int G, int HW, float* gx,

@@ -69,18 +69,23 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+def _area(ws):
+    """(pointer, bytes) of a scratch tensor of 8-byte elements; (None, 0) without one."""
+    return (None, 0) if ws is None or ws.numel() == 0 else (ws.data_ptr(), ws.numel() * 8)
+
+
 def _dims(x, out):
     return x.size(0), out.size(1), x.size(1), x.size(2)
 
 
 # Kernels launched by each C entry point (memsets are not counted).
 _KERNELS = {
-    "snb_inf_dist_forward": 2, "snb_inf_dist_forward_ws": 2, "snb_inf_dist_forward_sorted_ws": 3, "snb_inf_dist_forward_nograd": 1, "snb_inf_dist_backward_input": 1,
+    "snb_inf_dist_forward": 2, "snb_inf_dist_forward_ws": 2, "snb_inf_dist_forward_sorted_ws": 3, "snb_inf_dist_forward_nograd_ws": 1, "snb_inf_dist_backward_input": 1,
     "snb_inf_dist_backward_input_weight": 1, "snb_norm_dist_forward": 1, "snb_norm_dist_forward_ws": 2, "snb_norm_dist_backward_input": 1,
-    "snb_norm_dist_backward_input_weight": 1, "snb_bound_inf_dist_forward_nograd": 1,
-    "snb_bound_inf_dist_forward": 1, "snb_bound_inf_dist_backward_input": 1,
+    "snb_norm_dist_backward_input_weight": 1, "snb_bound_inf_dist_forward_nograd_ws": 1,
+    "snb_bound_inf_dist_forward_ws": 1, "snb_bound_inf_dist_backward_input": 1,
     "snb_bound_inf_dist_backward_input_weight": 1, "snb_mean_shift_stats": 1, "snb_mean_shift_apply": 1, "snb_sample_mask": 1, "snb_sample_mask_batch": 1,
-    "snb_sort_neuron_forward_nograd": 1, "snb_sort_neuron_forward": 1, "snb_bound_sort_neuron_forward": 1,
+    "snb_sort_neuron_forward_nograd_ws": 1, "snb_sort_neuron_forward_ws": 1, "snb_bound_sort_neuron_forward_ws": 1,
     "snb_sort_neuron_backward_input": 1, "snb_sort_neuron_backward_input_weight": 1,
 }
 
@@ -138,6 +143,14 @@ def _same_device(*ts):
     return dev
 
 
+def _scratch(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists, dev, at_least=0):
+    """Scratch for a forward call, taken from PyTorch's caching allocator (stream-ordered, no device
+    synchronisation): what the pruned evaluation asks for (snb_prune_scratch_bytes), or `at_least` bytes;
+    an empty tensor when neither needs any."""
+    nbytes = max(_lib.load().snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists), at_least)
+    return torch.empty((nbytes + 7) // 8, dtype=torch.int64, device=dev)
+
+
 def inf_dist_forward(input, weight, output, pos, G, w_index_ci=None, w_index_co=None):
     """core/cuda/norm_dist.cpp:131-147."""
     _check(input, "input"); _check(weight, "weight"); _check(output, "output")
@@ -149,12 +162,13 @@ def inf_dist_forward(input, weight, output, pos, G, w_index_ci=None, w_index_co=
     if output.size(0) != B or pos.shape != output.shape:
         raise RuntimeError("output / pos shape mismatch")
     dev = _same_device(input, weight, output, pos, w_index_ci, w_index_co)
-    # scratch for the k-split merge of (value, position) pairs: 8 bytes per output, taken from
-    # PyTorch's caching allocator (stream-ordered, no device synchronisation)
-    ws = torch.empty(B * CO, dtype=torch.int64, device=dev)
+    # pruned form, or 8 bytes per output for the k-split merge of (value, position) pairs
+    flat = G == 1 and HW == 1
+    ws = _scratch(1, 1, 1, B, CO, CI, weight.size(0), weight.size(1), int(w_index_ci is not None), dev, 8 * B * CO) \
+        if flat else torch.empty(0, dtype=torch.int64, device=dev)
     _call(dev, input, "snb_inf_dist_forward_ws", (B, CO, CI),
           _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), _ptr(pos), _ptr(w_index_ci),
-          _ptr(w_index_co), weight.size(0), weight.size(1) * G, ws.data_ptr(), ws.numel() * 8)
+          _ptr(w_index_co), weight.size(0), weight.size(1) * G, *_area(ws))
 
 
 def inf_dist_forward_sorted(input, weight, output, pos, w_index_ci=None, w_index_co=None):
@@ -174,11 +188,11 @@ def inf_dist_forward_sorted(input, weight, output, pos, w_index_ci=None, w_index
         for t, name, channels in ((w_index_ci, "w_index_ci", weight.size(1)), (w_index_co, "w_index_co", weight.size(0))):
             if t is not None and not check_index_lists(t, channels, name):
                 raise RuntimeError("%s is not in ascending order: use inf_dist_forward" % name)
-    nbytes = _lib.load().snb_inf_dist_forward_sorted_workspace_bytes(B, CO, weight.size(1))
-    ws = torch.empty((nbytes + 7) // 8, dtype=torch.int64, device=dev)
+    ws = _scratch(1, 1, 1, B, CO, CI, weight.size(0), weight.size(1), int(w_index_ci is not None), dev,
+                  _lib.load().snb_inf_dist_forward_sorted_workspace_bytes(B, CO, weight.size(1)))
     _call(dev, input, "snb_inf_dist_forward_sorted_ws", (B, CO, CI),
           _ptr(input), _ptr(weight), B, CO, CI, 1, HW, _ptr(output), _ptr(pos), _ptr(w_index_ci),
-          _ptr(w_index_co), weight.size(0), weight.size(1), ws.data_ptr(), ws.numel() * 8)
+          _ptr(w_index_co), weight.size(0), weight.size(1), *_area(ws))
 
 
 def inf_dist_forward_nograd(input, weight, output, G):
@@ -188,8 +202,9 @@ def inf_dist_forward_nograd(input, weight, output, G):
     if weight.size(0) != CO or weight.size(1) * G != CI or output.size(0) != B:
         raise RuntimeError("shape mismatch between input, weight and output")
     dev = _same_device(input, weight, output)
-    _call(dev, input, "snb_inf_dist_forward_nograd", (B, CO, CI),
-          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output))
+    ws = _scratch(1, 1, 0, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, input, "snb_inf_dist_forward_nograd_ws", (B, CO, CI),
+          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), *_area(ws))
 
 
 def inf_dist_backward_input(grad_output, pos, grad_input, G):
@@ -290,8 +305,9 @@ def bound_inf_dist_forward_nograd(inputL, inputU, weight, outputL, outputU, G):
             or weight.size(1) * G != CI:
         raise RuntimeError("shape mismatch")
     dev = _same_device(inputL, inputU, weight, outputL, outputU)
-    _call(dev, inputL, "snb_bound_inf_dist_forward_nograd", (B, CO, CI),
-          _ptr(inputL), _ptr(inputU), _ptr(weight), B, CO, CI, G, HW, _ptr(outputL), _ptr(outputU))
+    ws = _scratch(2, 1, 0, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, inputL, "snb_bound_inf_dist_forward_nograd_ws", (B, CO, CI),
+          _ptr(inputL), _ptr(inputU), _ptr(weight), B, CO, CI, G, HW, _ptr(outputL), _ptr(outputU), *_area(ws))
 
 
 def bound_inf_dist_forward(inputL, inputU, weight, outputL, outputU, posL, posU, G):
@@ -305,9 +321,10 @@ def bound_inf_dist_forward(inputL, inputU, weight, outputL, outputU, posL, posU,
             or weight.size(1) * G != CI or posL.shape != outputL.shape or posU.shape != outputL.shape:
         raise RuntimeError("shape mismatch")
     dev = _same_device(inputL, inputU, weight, outputL, outputU, posL, posU)
-    _call(dev, inputL, "snb_bound_inf_dist_forward", (B, CO, CI),
+    ws = _scratch(2, 1, 1, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, inputL, "snb_bound_inf_dist_forward_ws", (B, CO, CI),
           _ptr(inputL), _ptr(inputU), _ptr(weight), B, CO, CI, G, HW, _ptr(outputL), _ptr(outputU),
-          _ptr(posL), _ptr(posU))
+          _ptr(posL), _ptr(posU), *_area(ws))
 
 
 def bound_inf_dist_backward_input(grad_outputL, grad_outputU, posL, posU, grad_inputL, grad_inputU, G):
@@ -346,8 +363,9 @@ def sort_neuron_forward(input, weight, output, pos, G, q, K):
     if weight.size(0) != CO or weight.size(1) * G != CI or tuple(pos.shape) != (K, B, CO, HW):
         raise RuntimeError("shape mismatch")
     dev = _same_device(input, weight, output, pos)
-    _call(dev, input, "snb_sort_neuron_forward", (B, CO, CI),
-          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), _ptr(pos), float(q), int(K))
+    ws = _scratch(1, int(K), 1, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, input, "snb_sort_neuron_forward_ws", (B, CO, CI),
+          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), _ptr(pos), float(q), int(K), *_area(ws))
 
 
 def bound_sort_neuron_forward(inputL, inputU, weight, outputL, outputU, G, q, K):
@@ -360,9 +378,10 @@ def bound_sort_neuron_forward(inputL, inputU, weight, outputL, outputU, G, q, K)
             or weight.size(1) * G != CI:
         raise RuntimeError("shape mismatch")
     dev = _same_device(inputL, inputU, weight, outputL, outputU)
-    _call(dev, inputL, "snb_bound_sort_neuron_forward", (B, CO, CI),
+    ws = _scratch(2, int(K), 0, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, inputL, "snb_bound_sort_neuron_forward_ws", (B, CO, CI),
           _ptr(inputL), _ptr(inputU), _ptr(weight), B, CO, CI, G, HW, _ptr(outputL), _ptr(outputU),
-          float(q), int(K))
+          float(q), int(K), *_area(ws))
 
 
 def sort_neuron_forward_nograd(input, weight, output, G, q, K):
@@ -372,8 +391,9 @@ def sort_neuron_forward_nograd(input, weight, output, G, q, K):
     if weight.size(0) != CO or weight.size(1) * G != CI:
         raise RuntimeError("shape mismatch")
     dev = _same_device(input, weight, output)
-    _call(dev, input, "snb_sort_neuron_forward_nograd", (B, CO, CI),
-          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), float(q), int(K))
+    ws = _scratch(1, int(K), 0, B, CO, CI, CO, CI, 0, dev) if G == 1 and HW == 1 else None
+    _call(dev, input, "snb_sort_neuron_forward_nograd_ws", (B, CO, CI),
+          _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), float(q), int(K), *_area(ws))
 
 
 def sort_neuron_backward_input(grad_output, pos, grad_input, G, q, K):
@@ -463,7 +483,7 @@ def sample_masks_into(outs, channels, seeds):
 
 # ---- whole layers and the model head (one C call each; G = 1, HW = 1, 2-D tensors) ---------------
 
-_LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward": 4, "snb_layer_bound_forward": 3, "snb_input_box": 1,
+_LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward": 4, "snb_layer_bound_forward_ws": 3, "snb_input_box": 1,
                   "snb_margin_loss": 2, "snb_certified_fraction": 2}
 
 
@@ -521,9 +541,10 @@ def layer_bound_forward(x, xl, xu, weight, running_mean, bias, y, yl, yu):
     some = x if x is not None else xl
     B, CI = some.shape
     CO = weight.size(0)
-    _layer_call("snb_layer_bound_forward", (B, CO, CI), some,
+    ws = _scratch((x is not None) + 2 * (xl is not None), 1, 0, B, CO, CI, CO, CI, 0, some.device)
+    _layer_call("snb_layer_bound_forward_ws", (B, CO, CI), some,
                 _ptr(x), _ptr(xl), _ptr(xu), weight.data_ptr(), B, CO, CI, _ptr(running_mean), _ptr(bias), _ptr(y),
-                _ptr(yl), _ptr(yu))
+                _ptr(yl), _ptr(yu), *_area(ws))
 
 
 def input_box(x, eps, down, up, xl, xu):

@@ -1,0 +1,142 @@
+"""Pruned evaluation of the max-type operators (csrc/prune.cu) against the CPU oracle: bit-exact values,
+positions and bound words, whatever the data.  Every shape here is large enough for it
+(snb_prune_scratch_bytes > 0)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from gpu_util import col3, dev, host, idx3, make_masks, rel
+
+pytestmark = pytest.mark.gpu
+EPS = np.float32(1e-10)
+
+
+def operands(kind, rng, B, CI, CO):
+    if kind == "normal":                 # what the layers hold: a handful of columns per row survive
+        return rng.random((B, CI), dtype=np.float32), rng.standard_normal((CO, CI)).astype(np.float32)
+    if kind == "ties":                   # quantised: many columns share the maximum
+        return ((rng.integers(0, 4, (B, CI)) / 4).astype(np.float32),
+                (rng.standard_normal((CO, CI)) * 2).round().astype(np.float32) / 2)
+    if kind == "flat":                   # nothing can be pruned: every output is left to the dense kernel
+        return ((rng.random((B, CI)) * 2 - 1).astype(np.float32), (0.01 * rng.random((CO, CI))).astype(np.float32))
+    assert kind == "mixed"               # some rows of W flat, NaN and infinities among the rest
+    x, w = rng.standard_normal((B, CI)).astype(np.float32), rng.standard_normal((CO, CI)).astype(np.float32)
+    w[::7] *= 0.001
+    x[3, 5], x[1, 9], w[2, 4], w[8, 11], w[11] = np.nan, np.inf, np.nan, -np.inf, np.nan
+    return x, w
+
+
+def uses_pruning(tensors, K, words, B, CO, CI, W_CO, W_CI, lists):
+    from sortnet_b200 import _lib
+    return _lib.load().snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, lists) > 0
+
+
+# widths: one step of the filter up to its widest row, odd ones, tile edges; ragged rows and outputs
+SHAPES = [(70, 1024, 1000), (33, 1025, 1101), (128, 784, 520), (32, 5120, 257), (40, 6147, 200), (31, 12288, 130),
+          (300, 130, 1033), (5, 8192, 1024)]
+
+
+@pytest.mark.parametrize("B,CI,CO", SHAPES)
+@pytest.mark.parametrize("kind", ["normal", "ties", "flat", "mixed"])
+def test_distance_and_words(B, CI, CO, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    assert uses_pruning(1, 1, 1, B, CO, CI, CO, CI, 0)
+    x, w = operands(kind, np.random.default_rng(B + CI), B, CI, CO)
+    y_o, pos_o = oracle.inf_dist_forward(x, w)
+    y, pos = torch.full((B, CO, 1), 7.0, device="cuda"), torch.full((B, CO, 1), 7, device="cuda", dtype=torch.int32)
+    C.inf_dist_forward(col3(x), dev(w), y, pos, 1)
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+    yn = torch.full((B, CO, 1), 7.0, device="cuda")
+    C.inf_dist_forward_nograd(col3(x), dev(w), yn, 1)
+    assert np.array_equal(host(yn), y_o)
+
+
+@pytest.mark.parametrize("B,CI,CO,keep", [(70, 1024, 1100, 0.9), (160, 1030, 460, 0.7), (33, 2049, 1900, 0.5),
+                                          (96, 5120, 200, 0.95)])
+@pytest.mark.parametrize("which", ["both", "ci", "co"])
+@pytest.mark.parametrize("kind", ["normal", "ties", "flat"])
+@pytest.mark.parametrize("ascending", [True, False])
+def test_masked_distance(B, CI, CO, keep, which, kind, ascending):
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(B + CI + CO)
+    ci = make_masks(rng, B, CI, keep) if which in ("both", "ci") else None
+    co = make_masks(rng, B, CO, keep) if which in ("both", "co") else None
+    if not ascending:
+        ci, co = (None if m is None else rng.permuted(m, axis=1) for m in (ci, co))
+    x, w = operands(kind, rng, B, CI, CO)
+    x = np.ascontiguousarray(x[:, :ci.shape[1]]) if ci is not None else x
+    n_out = co.shape[1] if co is not None else CO
+    assert uses_pruning(1, 1, 1, B, n_out, x.shape[1], CO, CI, int(ci is not None))
+    y_o, pos_o = oracle.inf_dist_forward(x, w, ci, co)
+    y = torch.empty(B, n_out, 1, device="cuda")
+    pos = torch.empty(B, n_out, 1, device="cuda", dtype=torch.int32)
+    entry = C.inf_dist_forward_sorted if ascending else lambda a, b, c, d, i, o: C.inf_dist_forward(a, b, c, d, 1, i, o)
+    entry(col3(x), dev(w), y, pos, idx3(ci), idx3(co))
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+
+
+def test_lists_that_miss_the_largest_weights():
+    """The kept columns are those with the smallest weights: every output is found wanting and redone."""
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(5)
+    B, CI, CO = 64, 1024, 600
+    x, w = operands("normal", rng, B, CI, CO)
+    w[:, CI // 2:] *= 100
+    ci = np.tile(np.arange(CI // 2, dtype=np.int32), (2, 1))
+    x = np.ascontiguousarray(x[:, :CI // 2])
+    y_o, pos_o = oracle.inf_dist_forward(x, w, ci, None)
+    y, pos = torch.empty(B, CO, 1, device="cuda"), torch.empty(B, CO, 1, device="cuda", dtype=torch.int32)
+    C.inf_dist_forward_sorted(col3(x), dev(w), y, pos, idx3(ci), None)
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+
+
+@pytest.mark.parametrize("B,CI,CO", SHAPES[:6])
+@pytest.mark.parametrize("kind", ["normal", "ties", "flat", "mixed"])
+def test_interval_bounds(B, CI, CO, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(B * 3 + CI)
+    assert uses_pruning(2, 1, 1, B, CO, CI, CO, CI, 0) and uses_pruning(3, 1, 0, B, CO, CI, CO, CI, 0)
+    x, w = operands(kind, rng, B, CI, CO)
+    half = np.float32(0.25) if kind == "ties" else np.float32(0.03)
+    xl, xu = (x - half).astype(np.float32), (x + half).astype(np.float32)
+    flip = rng.random((B, CI)) < 0.01                       # inverted intervals are repaired to their midpoint
+    xl[flip], xu[flip] = xu[flip], xl[flip]
+    yl_o, yu_o, pl_o, pu_o = oracle.bound_inf_dist_forward(xl, xu, w)
+    XL, XU, W = col3(xl), col3(xu), dev(w)
+    yl, yu = torch.empty(B, CO, 1, device="cuda"), torch.empty(B, CO, 1, device="cuda")
+    C.bound_inf_dist_forward_nograd(XL, XU, W, yl, yu, 1)
+    assert np.array_equal(host(yl), yl_o) and np.array_equal(host(yu), yu_o)
+    pl, pu = torch.empty_like(yl, dtype=torch.int32), torch.empty_like(yl, dtype=torch.int32)
+    yl.fill_(7), yu.fill_(7)
+    C.bound_inf_dist_forward(XL, XU, W, yl, yu, pl, pu, 1)
+    assert np.array_equal(host(yl), yl_o) and np.array_equal(host(yu), yu_o)
+    assert np.array_equal(host(pl), pl_o) and np.array_equal(host(pu), pu_o)
+    # point value and box in one pass; the point may lie outside the box
+    y3 = [torch.empty(B, CO, device="cuda") for _ in range(3)]
+    xp = (x + np.float32(0.1)).astype(np.float32)
+    C.layer_bound_forward(dev(xp), XL.squeeze(-1), XU.squeeze(-1), W, None, None, *y3)
+    y_o, _ = oracle.inf_dist_forward(xp, w)
+    assert all(np.array_equal(a.cpu().numpy(), b) for a, b in zip(y3, (y_o, yl_o, yu_o)))
+
+
+@pytest.mark.parametrize("B,CI,CO", [(70, 1024, 1000), (33, 1025, 1101), (32, 5120, 257)])
+@pytest.mark.parametrize("q,K", [(0.75, 10), (0.5, 4), (0.85, 25), (0.6, 17)])
+@pytest.mark.parametrize("kind", ["normal", "ties", "flat"])
+def test_sort_neuron(B, CI, CO, q, K, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    assert uses_pruning(1, K, 1, B, CO, CI, CO, CI, 0)
+    x, w = operands(kind, np.random.default_rng(B + CI), B, CI, CO)
+    y_o, pos_o = oracle.sort_forward(x, w, q, K)
+    X, W = col3(x), dev(w)
+    y = torch.empty(B, CO, 1, device="cuda")
+    C.sort_neuron_forward_nograd(X, W, y, 1, q, K)
+    assert rel(host(y), y_o) < 2e-6
+    y2, pos = torch.empty_like(y), torch.empty(K, B, CO, 1, device="cuda", dtype=torch.int32)
+    C.sort_neuron_forward(X, W, y2, pos, 1, q, K)
+    assert np.array_equal(host(y2), host(y)) and np.array_equal(pos.squeeze(-1).cpu().numpy(), pos_o)
+    xl, xu = (x - np.float32(0.03)).astype(np.float32), (x + np.float32(0.03)).astype(np.float32)
+    yl_o, yu_o = oracle.sort_bound_forward(xl, xu, w, q, K)
+    yl, yu = torch.empty_like(y), torch.empty_like(y)
+    C.bound_sort_neuron_forward(col3(xl), col3(xu), W, yl, yu, 1, q, K)
+    assert rel(host(yl), yl_o) < 2e-6 and rel(host(yu), yu_o) < 2e-6
