@@ -91,28 +91,29 @@ __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("ba
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 enum { BAR_FILTER = 1, BAR_FULL = 2, BAR_EMPTY = 4 };
 
-// Persistent CTA: FT filter threads + R ordering warps.  A thread owns NIT x 4 columns; it keeps their centre and
+// Persistent CTA: FT filter threads + 2 R ordering warps.  A thread owns NIT x 4 columns; it keeps their centre and
 // radius in registers and copies its part of the next rows of W ahead with cp.async (its own shared memory: no barrier
 // for the data).  Per step of R rows:
 //   sweep 1   the largest |w - mid| - rad of every thread; the m-th largest of the warps' best is the threshold;
 //   sweep 2   every column with |w - mid| + rad at or above it goes into the row's list;
-// and the ordering warps sort the lists of the step before meanwhile (two list buffers).  Both sweeps read W from
-// shared memory, HBM is read once.
+// and the ordering warps sort the lists of the steps before meanwhile: two list buffers, each with R warps of its own,
+// which so have the time of two steps (a list of 230 entries takes one warp longer than a step).  Both sweeps read
+// W from shared memory, HBM is read once.
 // The centre form is rounded, so the sweep tests against thr (1 - 2^-19): with rad rounded up, a column it
 // leaves out has |fl(x - w)| < thr (1 - 2^-19)(1 + 2^-21) < thr = tau for every row.
 template <int R, int NIT, int FT, int STAGES, bool VEC>
-__global__ void __launch_bounds__(FT + 32 * R) prune_filter(const PruneArgs a) {
-    constexpr int WARPS = FT / 32, TOP = 32 / WARPS, ALL = FT + 32 * R;
+__global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
+    constexpr int WARPS = FT / 32, TOP = 32 / WARPS, ALL = FT + 32 * R;   // ALL: the filter and one buffer's ordering warps
     extern __shared__ __align__(16) unsigned char dyn[];
     const PruneProblem& p = a.p;
     const int C = p.W_CI, lcap = a.lcap, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float4* stage = reinterpret_cast<float4*>(dyn);                                  // [STAGES][R][NIT][FT]
     int2* lists = reinterpret_cast<int2*>(stage + STAGES * R * NIT * FT);            // [2][R][lcap] (column, w)
-    float* sorted = reinterpret_cast<float*>(lists + 2 * R * lcap);                  // [R][2][lcap] U as found, ordered
+    float* bounds = reinterpret_cast<float*>(lists + 2 * R * lcap);                  // [2 R][lcap] U, then [lcap / STEP] of steps
     __shared__ unsigned top[2][R][32];
     __shared__ float thr[2][R];
     __shared__ int n_found[2][R];
-    __shared__ int hist[R][BUCKETS];
+    __shared__ int hist[2 * R][BUCKETS];
     const int steps = (p.W_CO + R - 1) / R;
     const float nan = __int_as_float(0x7fc00000);
     if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
@@ -257,69 +258,78 @@ __global__ void __launch_bounds__(FT + 32 * R) prune_filter(const PruneArgs a) {
         return;
     }
 
-    // ordering warps: list r of every step, by U, largest first, in BUCKETS steps of U
-    const int r = warp - WARPS;
-    float* u_in = sorted + 2 * r * lcap;
-    float* u_out = u_in + lcap;
-    int i = 0;
-    for (int step = blockIdx.x; step < steps; step += gridDim.x, i++) {
-        const int buf = i & 1, j = step * R + r;
+    // ordering warps: list r of every other step, by U, largest first, in BUCKETS steps of U
+    const int o = warp - WARPS, r = o % R, buf = o / R;
+    float* u_in = bounds + o * (lcap + lcap / STEP);
+    unsigned* u_step = reinterpret_cast<unsigned*>(u_in + lcap);                     // largest U of each step of four
+    const int2* c_in = lists + (buf * R + r) * lcap;
+    for (int step = blockIdx.x + buf * (int)gridDim.x; step < steps; step += 2 * (int)gridDim.x) {
+        const int j = step * R + r;
         bar_sync(BAR_FULL + buf, ALL);
-        const int2* c_in = lists + (buf * R + r) * lcap;
         const int n = n_found[buf][r];
         const float t = thr[buf][r];
         if (j < p.W_CO && n <= lcap) {
             float umax = 0.f;
-            for (int k = lane; k < n; k += 32) {
-                const int2 e = c_in[k];
-                const float hi = decode(a.hi[e.x]), lo = -decode(a.nlo[e.x]), w = __int_as_float(e.y);
-                const float u = fmaxf(hi - w, w - lo);       // exact: rounding is monotone
-                u_in[k] = u;
-                umax = fmaxf(umax, u);
+            for (int k0 = 0; k0 < n; k0 += 128) {            // four entries per lane: their loads overlap
+                int2 e[4];
+                unsigned h[4], l[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int k = k0 + 32 * q + lane;
+                    e[q] = k < n ? c_in[k] : make_int2(0, __float_as_int(nan));
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) h[q] = a.hi[e[q].x], l[q] = a.nlo[e[q].x];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int k = k0 + 32 * q + lane;
+                    const float w = __int_as_float(e[q].y);
+                    const float u = fmaxf(decode(h[q]) - w, w + decode(l[q]));     // exact: rounding is monotone
+                    if (k < n) {
+                        u_in[k] = u;
+                        umax = fmaxf(umax, u);
+                    }
+                }
             }
             umax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(umax)));
             const float scale = umax > t ? (BUCKETS - 0.01f) / (umax - t) : 0.f;
             auto bucket = [&](float u) { return min(BUCKETS - 1, max(0, (int)((umax - u) * scale))); };
-            hist[r][lane] = 0;
+            const int padded = (n + PAD - 1) / PAD * PAD;
+            hist[o][lane] = 0;
+            for (int k = lane; k < padded / STEP; k += 32) u_step[k] = 0u;
             __syncwarp();
-            for (int k = lane; k < n; k += 32) atomicAdd(&hist[r][bucket(u_in[k])], 1);
+            for (int k = lane; k < n; k += 32) atomicAdd(&hist[o][bucket(u_in[k])], 1);
             __syncwarp();
             {
-                const int h = hist[r][lane];
+                const int h = hist[o][lane];
                 int incl = h;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
-                    const int o = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += o;
+                    const int below = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += below;
                 }
-                hist[r][lane] = incl - h;
+                hist[o][lane] = incl - h;
             }
             __syncwarp();
             int2* c_out = a.cand + (size_t)j * lcap;
-            const int padded = (n + PAD - 1) / PAD * PAD;
             for (int k = lane; k < n; k += 32) {
                 const float u = u_in[k];
-                const int at = atomicAdd(&hist[r][bucket(u)], 1);
-                u_out[at] = u;
+                const int at = atomicAdd(&hist[o][bucket(u)], 1);
+                atomicMax(&u_step[at / STEP], __float_as_uint(u));
                 c_out[at] = c_in[k];
             }
-            for (int k = n + lane; k < padded; k += 32) {
-                u_out[k] = 0.f;
-                c_out[k] = make_int2(c_in[0].x, __float_as_int(nan));   // w = NaN: changes nothing
-            }
+            if (n + lane < padded) c_out[n + lane] = make_int2(c_in[0].x, __float_as_int(nan));   // w = NaN: changes nothing
             __syncwarp();
             // ub[b]: no entry of step b or later has a larger U
             const int nb = padded / STEP;
             float tail = 0.f;
             for (int base = (nb - 1) / 32 * 32; base >= 0; base -= 32) {
                 const int b = base + lane;
-                float v = 0.f;
-                if (b < nb)
-                    for (int e = 0; e < STEP; e++) v = fmaxf(v, u_out[b * STEP + e]);
+                float v = b < nb ? __uint_as_float(u_step[b]) : 0.f;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
-                    const float o = __shfl_down_sync(0xffffffffu, v, d);
-                    if (lane + d < 32) v = fmaxf(v, o);
+                    const float after = __shfl_down_sync(0xffffffffu, v, d);
+                    if (lane + d < 32) v = fmaxf(v, after);
                 }
                 v = fmaxf(v, tail);
                 if (b < nb) a.ub[(size_t)j * (lcap / STEP) + b] = v;
@@ -489,8 +499,8 @@ struct PosList {
 // column): a warp walks four lists side by side.  A step is STEP columns; the entries of the next step are fetched
 // while this one's columns are on their way; a walk ends when the largest U left is below the results of all 32 rows.
 // Bound by the latency of the two dependent loads (list, column) and by the columns' traffic from L2.
-// TRACK keeps the list entry that set each maximum; the word is made from it at the end.  An equal value met
-// on the way (rare) sends the warp over the list once more for the lowest position.
+// TRACK keeps, per row, the step that set the maximum; the word is made at the end from the step's columns.  A
+// later step that only equals the maximum (rare) sends the lane over the list once more for the lowest position.
 template <int NX, bool TRACK>
 __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
@@ -511,8 +521,8 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
 
     float acc[NV][4];
-    int at[TRACK ? NV : 1][TRACK ? 4 : 1];
-    bool tied = false;
+    int at[TRACK ? NV : 1][TRACK ? 4 : 1];                   // step of the maximum, -1: at its floor
+    unsigned tied = 0u;                                      // bit t * 4 + q: another step reaches the same value
 #pragma unroll
     for (int t = 0; t < NV; t++)
 #pragma unroll
@@ -540,6 +550,7 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     bool active = cnt > 0;
     int4 e01 = make_int4(0, 0, 0, 0), e23 = e01;
     float left = 0.f;
+    int walked = 0;
     if (active) e01 = list[0], e23 = list[1];
     for (int b = 0;; b++) {
         if (b > 0) {
@@ -561,23 +572,31 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
                 left = ub[b + 1];
             }
 #pragma unroll
-            for (int e = 0; e < STEP; e++)
+            for (int q = 0; q < 4; q++) {
+                float v[STEP][NV];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float xq[NX], v[NV];
+                for (int e = 0; e < STEP; e++) {
+                    float xq[NX];
 #pragma unroll
                     for (int t = 0; t < NX; t++) xq[t] = q == 0 ? x[e][t].x : q == 1 ? x[e][t].y : q == 2 ? x[e][t].z : x[e][t].w;
-                    values(xq, w[e], v);
+                    values(xq, w[e], v[e]);
+                }
 #pragma unroll
-                    for (int t = 0; t < NV; t++) {
-                        if (TRACK) {
-                            int& k = at[TRACK ? t : 0][TRACK ? q : 0];
-                            if (v[t] == acc[t][q]) tied = tied || k >= 0;
-                            if (v[t] > acc[t][q]) k = b * STEP + e;
+                for (int t = 0; t < NV; t++) {
+                    if (TRACK) {
+                        const float m = fmaxf(max3(v[0][t], v[1][t], v[2][t]), v[3][t]);
+                        if (m == acc[t][q]) tied |= 1u << (t * 4 + q);
+                        if (m > acc[t][q]) {
+                            at[TRACK ? t : 0][TRACK ? q : 0] = b;
+                            tied &= ~(1u << (t * 4 + q));
                         }
-                        acc[t][q] = fmaxf(acc[t][q], v[t]);
+                        acc[t][q] = fmaxf(acc[t][q], m);
+                    } else {
+                        acc[t][q] = max3(max3(acc[t][q], v[0][t], v[1][t]), v[2][t], v[3][t]);
                     }
                 }
+            }
+            walked = b + 1;
         }
     }
     const unsigned good = __ballot_sync(0xffffffffu, worst() >= tau);
@@ -588,47 +607,44 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
         for (int q = 0; q < 4; q++) tile[t][4 * l + q][slot] = acc[t][q];
     if (TRACK) {
         const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
-        const int2* entries = a.cand + (size_t)j * a.lcap;
         const float* xs = reinterpret_cast<const float*>(xt);
-        uint32_t word[TRACK ? NV : 1][4];
-        // word of the entry k for row q
-        auto make_word = [&](int t, int q, int k) {
-            const int2 e = entries[k];
-            const uint32_t idx = (uint32_t)(inv ? inv[e.x] : e.x);
-            const float w = __int_as_float(e.y);
-            const float x0 = xs[(size_t)e.x * NX * 32 + q];
-            if (NX == 1) return idx | (x0 - w < 0.f ? SNB_SIGN_BIT : 0u);
-            const float x1 = xs[((size_t)e.x * NX + NX - 1) * 32 + q];
-            return idx | (w - x0 <= x1 - w ? 0u : SNB_SIGN_BIT);
+        // lowest position among the entries of step k whose value for row q is `want`
+        auto step_word = [&](int t, int q, int k, float want, uint32_t word) {
+            const int4 a01 = list[2 * k], a23 = list[2 * k + 1];
+            const int c[STEP] = {a01.x, a01.z, a23.x, a23.z};
+            const float w[STEP] = {__int_as_float(a01.y), __int_as_float(a01.w), __int_as_float(a23.y), __int_as_float(a23.w)};
+            float xq[STEP][NX];
+            int idx[STEP];
+#pragma unroll
+            for (int e = 0; e < STEP; e++) {
+                idx[e] = inv ? inv[c[e]] : c[e];
+#pragma unroll
+                for (int u = 0; u < NX; u++) xq[e][u] = xs[((size_t)c[e] * NX + u) * 32 + q];
+            }
+#pragma unroll
+            for (int e = 0; e < STEP; e++) {
+                float v[NV];
+                values(xq[e], w[e], v);
+                bool negative = xq[e][0] - w[e] < 0.f;
+                if (NX == 2) negative = !(w[e] - xq[e][0] <= xq[e][NX - 1] - w[e]);
+                if (v[t] == want && (uint32_t)idx[e] < (word & ~SNB_SIGN_BIT)) word = (uint32_t)idx[e] | (negative ? SNB_SIGN_BIT : 0u);
+            }
+            return word;
         };
+        uint32_t word[TRACK ? NV : 1][4];
 #pragma unroll
         for (int t = 0; t < NV; t++)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int k = at[TRACK ? t : 0][TRACK ? q : 0];
-                word[TRACK ? t : 0][q] = k >= 0 ? make_word(t, q, k) : (NX == 2 && t == 0) ? SNB_NO_GRAD_ID : 0u;
-            }
-        if (tied) {
-#pragma unroll 1
-            for (int k = 0; k < cnt; k++) {
-                const int2 e = entries[k];
-                for (int q = 0; q < live; q++) {
-                    float xq[NX], v[NV];
-#pragma unroll
-                    for (int t = 0; t < NX; t++) xq[t] = xs[((size_t)e.x * NX + t) * 32 + q];
-                    values(xq, __int_as_float(e.y), v);
-#pragma unroll
-                    for (int t = 0; t < NV; t++)
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-                            if (r == q && at[TRACK ? t : 0][TRACK ? r : 0] >= 0 && v[t] == acc[t][r]) {
-                                const uint32_t other = make_word(t, q, k);
-                                uint32_t& wd = word[TRACK ? t : 0][r];
-                                if ((other & ~SNB_SIGN_BIT) < (wd & ~SNB_SIGN_BIT)) wd = other;
-                            }
+                uint32_t wd = (NX == 2 && t == 0) ? SNB_NO_GRAD_ID : 0u;
+                if (k >= 0) {
+                    wd = step_word(t, q, k, acc[t][q], 0x7fffffffu);
+                    if ((tied >> (t * 4 + q)) & 1u)
+                        for (int k2 = 0; k2 < walked; k2++) wd = step_word(t, q, k2, acc[t][q], wd);
                 }
+                word[TRACK ? t : 0][q] = wd;
             }
-        }
 #pragma unroll
         for (int t = 0; t < NV; t++)
 #pragma unroll
@@ -1066,14 +1082,14 @@ cudaError_t set_smem(int bytes) {
 // Persistent grid: as many CTAs as fit (the shared memory of the stages limits them to two per SM for wide rows).
 template <int R, int NIT, int FT, int STAGES, bool VEC>
 cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
-    const int smem = STAGES * R * NIT * FT * 16 + R * a.lcap * (2 * (int)sizeof(int2) + 2 * (int)sizeof(float));
+    const int smem = STAGES * R * NIT * FT * 16 + R * (a.lcap * (2 * (int)sizeof(int2) + 2 * (int)sizeof(float)) + a.lcap / STEP * 2 * (int)sizeof(float));
     cudaError_t e = set_smem<prune_filter<R, NIT, FT, STAGES, VEC>>(smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_filter<R, NIT, FT, STAGES, VEC>, FT + 32 * R, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_filter<R, NIT, FT, STAGES, VEC>, FT + 64 * R, smem);
     if (e != cudaSuccess) return e;
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
-    prune_filter<R, NIT, FT, STAGES, VEC><<<steps < slots ? steps : slots, FT + 32 * R, smem, st>>>(a);
+    prune_filter<R, NIT, FT, STAGES, VEC><<<steps < slots ? steps : slots, FT + 64 * R, smem, st>>>(a);
     return cudaGetLastError();
 }
 
