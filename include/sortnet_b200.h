@@ -124,6 +124,43 @@ int snb_inf_dist_forward_noalloc(const float* x, const float* w, int B, int CO, 
                                  int HW, float* y, int* pos, void* stream);
 int snb_inf_dist_forward_noalloc_max_outputs(void);
 
+/* ---- a whole SortNet-MLP per call (G == 1, HW == 1) --------------------------------------------
+ * Layer k of the net: w [out, in], optional bias [out] (added after the mean shift), optional running_mean [out]
+ * (training: updated in place with `momentum`; evaluation: subtracted), the kept channels of its output as ascending
+ * int32 lists kept_list [S, kept] (training of a sort-neuron estimate; NULL keeps all), and for the evaluation
+ * pass K = 1 (l-inf distance) or the size of its sort neuron with ratio q.  Same arithmetic, layer by layer, as
+ * snb_layer_forward / snb_layer_backward / snb_layer_bound_forward and the sort-neuron entry points; activations move
+ * between the layers in the form the pruned evaluation reads.  No counterpart in the reference (there: a chain of Python
+ * calls, ell_inf_models.py:34-50, main.py:357-364). */
+typedef struct {
+    const float* w;
+    const float* bias;
+    float* running_mean;
+    const int* kept_list;
+    int in, out, kept, K;
+    float momentum, q;
+} snb_mlp_layer;
+
+/* 1 when the calls below take these layers at B rows and are the faster way. */
+int snb_mlp_applies(const snb_mlp_layer* layers, int depth, int B);
+/* Bytes of `saved` (forward to backward) and of the scratch areas. */
+size_t snb_mlp_saved_bytes(const snb_mlp_layer* layers, int depth, int B);
+size_t snb_mlp_scratch_bytes(const snb_mlp_layer* layers, int depth, int B, int tensors, int training);
+size_t snb_mlp_backward_scratch_bytes(const snb_mlp_layer* layers, int depth, int B);
+/* p = infinity training pass: hidden layers with batch mean shift, head with bias, then snb_margin_loss on its
+ * outputs.  saved and scratch 256-byte aligned.  launches (host, optional): kernels launched. */
+int snb_mlp_train_forward(const snb_mlp_layer* layers, int depth, const float* x, int B, const long long* targets, float eps,
+                          float clip, float lam, float scale, void* saved, void* scratch, float* loss, int* launches,
+                          void* stream);
+int snb_mlp_train_backward(const snb_mlp_layer* layers, int depth, int B, const float* grad_loss, const void* saved,
+                           void* scratch, float* const* grad_w, float* grad_bias, float* grad_x, int* launches, void* stream);
+/* Evaluation pass: tensors = 1 (y) or 3 (y and the bounds of a box: xl, xu, or [max(x - box_eps, down), min(x + box_eps, up)]
+ * when they are NULL); score / margin [B, classes] optional. */
+int snb_mlp_eval_forward(const snb_mlp_layer* layers, int depth, const float* x, const float* xl, const float* xu, int B,
+                         int tensors, float box_eps, float down, float up, void* scratch, float* y, float* yl, float* yu,
+                         const long long* targets, float inv_two_eps, float scale, float* score, float* margin, int* launches,
+                         void* stream);
+
 /* Scratch with which the `_ws` entry points below evaluate a problem in the pruned form (the exact results, but
  * only the columns of w that can matter are looked at per row): tensors = 1 for a point value, 2 for a box, 3 for both
  * (snb_layer_bound_forward_ws); K = 1, or the sort neuron's K; words = 1 when positions are wanted; column_lists = 1 with

@@ -55,6 +55,14 @@ SIGNATURES = {
     "snb_input_box": [_P, _F, _F, _F, ctypes.c_longlong, _P, _P, _P],
     "snb_margin_loss": [_P, _P, _I, _I, _F, _F, _F, _F, _P, _P, _P, _P, _P],
     "snb_certified_fraction": [_P, _P, _P, _I, _I, _P, _P, _P],
+    # the three *_bytes return size_t
+    "snb_mlp_applies": [_P, _I, _I],
+    "snb_mlp_saved_bytes": [_P, _I, _I],
+    "snb_mlp_scratch_bytes": [_P, _I, _I, _I, _I],
+    "snb_mlp_backward_scratch_bytes": [_P, _I, _I],
+    "snb_mlp_train_forward": [_P, _I, _P, _I, _P, _F, _F, _F, _F, _P, _P, _P, _P, _P],
+    "snb_mlp_train_backward": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P],
+    "snb_mlp_eval_forward": [_P, _I, _P, _P, _P, _I, _I, _F, _F, _F, _P, _P, _P, _P, _P, _F, _F, _P, _P, _P, _P],
     "snb_peer_barrier": [_P, _I, _I, ctypes.c_uint, ctypes.c_ulonglong, _P, _P],
     "snb_peer_signal": [_P, _I, _I, ctypes.c_uint, _P],
     "snb_peer_wait": [_P, _I, _I, ctypes.c_uint, ctypes.c_ulonglong, _P, _P],
@@ -101,7 +109,8 @@ def load(build_if_missing: bool = False):
     lib.snb_inf_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     lib.snb_inf_dist_forward_sorted_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
     lib.snb_inf_dist_forward_sorted_workspace_bytes.restype = ctypes.c_size_t
-    lib.snb_prune_scratch_bytes.restype = ctypes.c_size_t
+    for name in ("snb_prune_scratch_bytes", "snb_mlp_saved_bytes", "snb_mlp_scratch_bytes", "snb_mlp_backward_scratch_bytes"):
+        getattr(lib, name).restype = ctypes.c_size_t
     lib.snb_norm_dist_forward_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_float]
     lib.snb_norm_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     _lib = lib

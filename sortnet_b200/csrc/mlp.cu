@@ -1,0 +1,522 @@
+// A whole SortNet-MLP in one call per direction: the p = infinity training pass (masked forward, margin and mixture loss,
+// sparse backward) and the evaluation pass (point value and interval bounds, l-inf or sort neuron per layer).
+//
+// The layers are those of layer.cu, with the same arithmetic in the same order; what differs is what moves
+// between them.  Activations stay in the form in which the pruned evaluation reads its input (prune.cuh:
+// [sub-batch][channel][32 rows], full width, NaN in dropped channels), so a layer is filter + walk (+ redo of rejected outputs)
+// + one pass that takes the batch mean off; nothing is gathered through index lists.  The backward works on full-width rows
+// too: per layer one pass that centres the gradient and one launch that builds grad_x row by row (batch rows) and grad_w
+// row by row (outputs) in shared memory, so grad_w is written once, whole, instead of zero-filled and hit with one atomic per
+// (row, output).  For six layers the host issues 28 + 12 launches from C instead of some 100 from Python.
+#include "../../include/sortnet_b200.h"
+#include "prune.cuh"
+
+namespace snb {
+namespace {
+
+// Index lists [S][count] of the hidden layers -> flags [S][channels], one CTA per list.
+constexpr int MAX_DEPTH = 16;
+struct KeepJobs {
+    const int* list[MAX_DEPTH];
+    unsigned char* flags[MAX_DEPTH];
+    int count[MAX_DEPTH], channels[MAX_DEPTH];
+};
+__global__ void __launch_bounds__(256) keep_flags_kernel(const KeepJobs jobs) {
+    const int* list = nullptr;
+    unsigned char* flags = nullptr;
+    int count = 0, channels = 0;
+#pragma unroll
+    for (int j = 0; j < MAX_DEPTH; j++)                      // compile-time indices keep the table in the parameter bank
+        if (j == (int)blockIdx.y) list = jobs.list[j], flags = jobs.flags[j], count = jobs.count[j], channels = jobs.channels[j];
+    if (!list) return;
+    const int s = blockIdx.x;
+    unsigned char* f = flags + (size_t)s * channels;
+    for (int c = threadIdx.x; c < channels; c += 256) f[c] = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < count; k += 256) f[list[(size_t)s * count + k]] = 1;
+}
+
+// Training mean shift in the chain form: the batch mean of every channel from the sub-batches' row sums (in the order of
+// mean_shift_stats_kernel, bit for bit), running mean, y - mean in place, and the column ranges of the result.
+// CTA = 16 channels, lane = row.  Bound by the latency of its two dependent reads (sums, then y from L2), so all of a
+// CTA's sums are fetched at once and eight rows of y per warp are in flight.
+constexpr int SHIFT_C = 16, SHIFT_S = 64;                    // sub-batches whose sums fit shared memory
+__global__ void __launch_bounds__(256) chain_shift_kernel(float* __restrict__ yt, const float* __restrict__ part,
+                                                          const unsigned char* __restrict__ keep, int B, int S, int C,
+                                                          float* __restrict__ running_mean, float momentum,
+                                                          float* __restrict__ rows_kept, unsigned* __restrict__ hi_out,
+                                                          unsigned* __restrict__ nlo_out) {
+    __shared__ float sums[SHIFT_S][SHIFT_C];                 // NaN: dropped
+    __shared__ float mean[SHIFT_C];
+    __shared__ unsigned hi[SHIFT_C], nlo[SHIFT_C];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = blockIdx.x * SHIFT_C, n = min(SHIFT_C, C - c0);
+    const int cx = tid & (SHIFT_C - 1), c = c0 + cx;
+    auto fetch = [&](int s) {
+        const bool kept = cx < n && (!keep || keep[(size_t)s * C + c]);
+        return kept ? part[(size_t)s * C + c] : __int_as_float(0x7fc00000);
+    };
+    for (int s = tid / SHIFT_C; s < min(S, SHIFT_S); s += 256 / SHIFT_C) sums[s][cx] = fetch(s);
+    __syncthreads();
+    if (tid < SHIFT_C) {
+        hi[tid] = nlo[tid] = 0u;
+        float t = 0.f, cnt = 0.f;
+        for (int k = 0; k < 16; k++) {
+            float sum = 0.f;
+            for (int s = k; s < S; s += 16) {
+                const float v = s < SHIFT_S ? sums[s][cx] : fetch(s);
+                if (v == v) {
+                    sum += v;
+                    cnt += (float)(min(B, s * 32 + 32) - s * 32);
+                }
+            }
+            t += sum;
+        }
+        const float m = t / fmaxf(cnt, 1e-10f);
+        mean[tid] = m;
+        if (tid < n) {
+            rows_kept[c] = cnt;
+            if (running_mean) running_mean[c] = running_mean[c] * (1.0f - momentum) + momentum * m;
+        }
+    }
+    __syncthreads();
+    const int items = S * SHIFT_C;                           // (sub-batch, channel) rows of 32
+    for (int i0 = warp; i0 < items; i0 += 64) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = i0 + 8 * u, ch = i % SHIFT_C;
+            v[u] = i < items && ch < n ? yt[((size_t)(i / SHIFT_C) * C + c0 + ch) * 32 + lane] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = i0 + 8 * u, ch = i % SHIFT_C;
+            if (i >= items || ch >= n) continue;
+            const float y = v[u] - mean[ch];
+            yt[((size_t)(i / SHIFT_C) * C + c0 + ch) * 32 + lane] = y;
+            const unsigned h = __reduce_max_sync(0xffffffffu, order_code(y)), l = __reduce_max_sync(0xffffffffu, order_code(-y));
+            if (lane == 0) {
+                atomicMax(&hi[ch], h);
+                atomicMax(&nlo[ch], l);
+            }
+        }
+    }
+    __syncthreads();
+    if (tid < n) hi_out[c] = hi[tid], nlo_out[c] = nlo[tid];
+}
+
+// Gradient of a layer's outputs g [B][C] (times *scale): centred when rows_kept is given (the backward of the mean
+// shift: minus the mean over the rows that kept the channel; g is 0 where a channel was dropped), written back
+// row by row and transposed to gt [S][C][32]; column sums on request (bias gradient).
+// CTA = 32 channels, warp = row of every sub-batch, whose values stay in registers between the two sweeps (up to
+// CENTER_S sub-batches, then they are read again).  Bound by latency and L2 traffic.
+constexpr int CENTER_S = 16;
+__global__ void __launch_bounds__(1024) chain_center_kernel(const float* g, const float* __restrict__ scale,
+                                                            const float* __restrict__ rows_kept, int B, int S, int C,
+                                                            float* g_out, float* __restrict__ gt, float* __restrict__ col_sum) {
+    __shared__ float tile[2][32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    const float f = scale ? *scale : 1.f;
+    auto fetch = [&](int s) {
+        const int b = s * 32 + warp;
+        return b < B && c < C ? g[(size_t)b * C + c] * f : 0.f;
+    };
+    float v[CENTER_S], sum = 0.f, mean = 0.f;
+#pragma unroll
+    for (int s = 0; s < CENTER_S; s++) v[s] = s < S ? fetch(s) : 0.f;
+    if (rows_kept || col_sum) {
+#pragma unroll
+        for (int s = 0; s < CENTER_S; s++) sum += v[s];
+        for (int s = CENTER_S; s < S; s++) sum += fetch(s);
+        tile[0][warp][lane] = sum;
+        __syncthreads();
+        sum = tile[0][lane][warp];                           // the sums of channel `warp`
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == 0) tile[1][0][warp] = sum;
+        __syncthreads();
+        sum = tile[1][0][lane];
+        if (col_sum && warp == 0 && c < C) col_sum[c] = sum;
+        if (rows_kept && c < C) mean = sum / fmaxf(rows_kept[c], 1e-10f);
+        __syncthreads();
+    }
+    const int ch = blockIdx.x * 32 + warp;
+    auto put = [&](int s, float x) {
+        const int b = s * 32 + warp;
+        x -= mean;
+        if (b < B && c < C) g_out[(size_t)b * C + c] = x;
+        tile[s & 1][warp][lane] = x;
+        __syncthreads();                                     // the other buffer's readers are past their previous barrier
+        if (ch < C) gt[((size_t)s * C + ch) * 32 + lane] = tile[s & 1][lane][warp];
+    };
+#pragma unroll
+    for (int s = 0; s < CENTER_S; s++)
+        if (s < S) put(s, v[s]);
+    for (int s = CENTER_S; s < S; s++) put(s, fetch(s));
+}
+
+// Sparse l-inf backward of one layer.  CTAs 0 .. gx_rows - 1: row b of grad_x; the others: row j of grad_w.  Both are
+// accumulated in shared memory and written whole.  The rows of one sub-batch share a handful of argmax columns of W row j, so
+// a warp adds up per distinct column before it touches shared memory (32 lanes on few addresses otherwise retry
+// one by one: 61 instead of 27 us for 512 x 5120 x 5120).  Bound by the write of grad_w (HBM).
+__global__ void __launch_bounds__(256) chain_bwd_kernel(const float* __restrict__ g, const float* __restrict__ gt,
+                                                        const int* __restrict__ pos, const int* __restrict__ post, int B, int S,
+                                                        int CO, int CI, int gx_rows, float* __restrict__ gx,
+                                                        float* __restrict__ gw) {
+    extern __shared__ __align__(16) float row[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool vec = (CI & 3) == 0 && ((reinterpret_cast<uintptr_t>(gx) | reinterpret_cast<uintptr_t>(gw)) & 15u) == 0;
+    for (int c = tid; c < (CI + 3) / 4; c += 256) reinterpret_cast<float4*>(row)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    float* dst;
+    if ((int)blockIdx.x < gx_rows) {
+        const int b = blockIdx.x;
+        dst = gx + (size_t)b * CI;
+        for (int j0 = tid; j0 < CO; j0 += 1024) {
+            uint32_t word[4];
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int j = j0 + 256 * u;
+                word[u] = j < CO ? (uint32_t)pos[(size_t)b * CO + j] : SNB_NO_GRAD_ID;
+                v[u] = j < CO ? g[(size_t)b * CO + j] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (word[u] != SNB_NO_GRAD_ID) atomicAdd(row + (word[u] & ~SNB_SIGN_BIT), (word[u] & SNB_SIGN_BIT) ? -v[u] : v[u]);
+        }
+    } else {
+        const int j = blockIdx.x - gx_rows;
+        dst = gw + (size_t)j * CI;
+        for (int s = tid >> 5; s < S; s += 8) {
+            const size_t o = ((size_t)s * CO + j) * 32 + lane;
+            const uint32_t word = (uint32_t)post[o];
+            const uint32_t col = word == SNB_NO_GRAD_ID ? SNB_NO_GRAD_ID : (word & ~SNB_SIGN_BIT);
+            const float v = (word & SNB_SIGN_BIT) ? gt[o] : -gt[o];
+            unsigned todo = __ballot_sync(0xffffffffu, col != SNB_NO_GRAD_ID);
+            while (todo) {
+                const uint32_t one = __shfl_sync(0xffffffffu, col, __ffs(todo) - 1);
+                const bool mine = col == one;
+                todo &= ~__ballot_sync(0xffffffffu, mine);
+                float sum = mine ? v : 0.f;
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+                if (lane == 0) atomicAdd(row + one, sum);
+            }
+        }
+    }
+    __syncthreads();
+    if (vec)
+        for (int c = tid; c < CI / 4; c += 256) __stcs(reinterpret_cast<float4*>(dst) + c, reinterpret_cast<float4*>(row)[c]);
+    else
+        for (int c = tid; c < CI; c += 256) dst[c] = row[c];
+}
+
+// Scores and margins of the evaluation pass from the head's outputs (ell_inf_models.py:45-50): score = -y * scale,
+// margin[b, c] = ((-yl[b, c]) - (-yu[b, t])) / (2 eps), 0 at the target.
+__global__ void __launch_bounds__(256) scores_kernel(const float* __restrict__ y, const float* __restrict__ yl,
+                                                     const float* __restrict__ yu, const long long* __restrict__ target, int B,
+                                                     int K, float inv_two_eps, float scale, float* __restrict__ score,
+                                                     float* __restrict__ margin) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= B * K) return;
+    const int b = i / K, c = i % K, t = (int)target[b];
+    score[i] = -y[i] * scale;
+    margin[i] = c == t ? 0.f * inv_two_eps : (-yl[i] - -yu[(size_t)b * K + t]) * inv_two_eps;
+}
+
+size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+struct Cursor {
+    char* base;
+    size_t off = 0;
+    template <class T>
+    T* take(size_t n) {
+        char* at = base + off;
+        off += up256(sizeof(T) * n);
+        return reinterpret_cast<T*>(at);
+    }
+};
+
+// What the backward needs from the forward.
+struct Saved {
+    unsigned char* keep[MAX_DEPTH];
+    int* pos[MAX_DEPTH];
+    int* post[MAX_DEPTH];
+    float* rows_kept[MAX_DEPTH];
+    float* grad_d;
+};
+size_t saved_layout(const snb_mlp_layer* l, int depth, int B, char* base, Saved* out) {
+    const size_t S = (B + 31) / 32;
+    Cursor at{base};
+    Saved v{};
+    for (int k = 0; k < depth; k++) {
+        const size_t C = l[k].out;
+        v.keep[k] = at.take<unsigned char>(l[k].kept_list ? S * C : 0);
+        v.pos[k] = at.take<int>((size_t)B * C);
+        v.post[k] = at.take<int>(S * C * 32);
+        v.rows_kept[k] = at.take<float>(C);
+    }
+    v.grad_d = at.take<float>((size_t)B * l[depth - 1].out);
+    if (out) *out = v;
+    return at.off;
+}
+
+int widest(const snb_mlp_layer* l, int depth) {
+    int c = l[0].in;
+    for (int k = 0; k < depth; k++) c = l[k].out > c ? l[k].out : c;
+    return c;
+}
+
+PruneProblem layer_problem(const snb_mlp_layer* l, int k, int B, int tensors) {
+    static const float some = 0.f;
+    PruneProblem p;
+    if (tensors != 2) p.x = &some;
+    if (tensors != 1) p.xl = p.xu = &some;
+    p.w = l[k].w;
+    p.B = B, p.CO = p.W_CO = l[k].out, p.CI = p.W_CI = l[k].in;
+    p.K = l[k].K, p.q = l[k].q;
+    if (k > 0 && l[k - 1].kept_list) p.kept = l[k - 1].kept, p.kept_list = l[k - 1].kept_list;
+    return p;
+}
+
+struct Scratch {
+    char* zeroed;                  // fail counters and input ranges of every layer, one memset
+    size_t zero_bytes;
+    unsigned* fail[MAX_DEPTH];
+    unsigned* hi[MAX_DEPTH];       // ranges of layer k's input
+    unsigned* nlo[MAX_DEPTH];
+    float* xt[2];
+    float* part;
+    float* d;
+    float* row_loss;
+    char* prune;
+};
+size_t scratch_layout(const snb_mlp_layer* l, int depth, int B, int tensors, bool training, char* base, Scratch* out) {
+    const size_t S = (B + 31) / 32, W = widest(l, depth);
+    Cursor at{base};
+    Scratch v{};
+    v.zeroed = base;
+    for (int k = 0; k < depth; k++) {
+        v.fail[k] = at.take<unsigned>(1);
+        v.hi[k] = at.take<unsigned>(l[k].in);
+        v.nlo[k] = at.take<unsigned>(l[k].in);
+    }
+    v.zero_bytes = at.off;
+    for (int i = 0; i < 2; i++) v.xt[i] = at.take<float>(S * W * tensors * 32);
+    v.part = at.take<float>(training ? S * W : 0);
+    v.d = at.take<float>((size_t)tensors * B * l[depth - 1].out);
+    v.row_loss = at.take<float>(B);
+    size_t most = 0;
+    static const float some = 0.f;
+    static unsigned none = 0;
+    static int word = 0;
+    for (int k = 0; k < depth; k++) {
+        PruneProblem p = layer_problem(l, k, B, tensors);
+        p.xt = &some, p.hi = p.nlo = &none, p.fail_count = &none;
+        if (training) p.pos = &word;
+        const size_t n = prune_workspace_bytes(p);
+        most = n > most ? n : most;
+    }
+    v.prune = at.take<char>(most);
+    if (out) *out = v;
+    return at.off;
+}
+
+int check_layers(const snb_mlp_layer* l, int depth, int B) {
+    if (!l) return SNB_ERR_NULL_POINTER;
+    if (depth < 1 || B <= 0) return SNB_ERR_BAD_SHAPE;
+    if (depth > MAX_DEPTH) return SNB_ERR_UNSUPPORTED;
+    for (int k = 0; k < depth; k++) {
+        if (l[k].in <= 0 || l[k].out <= 0 || (k > 0 && l[k].in != l[k - 1].out)) return SNB_ERR_BAD_SHAPE;
+        if (l[k].kept_list && (l[k].kept <= 0 || l[k].kept > l[k].out)) return SNB_ERR_BAD_SHAPE;
+        if (l[k].K < 1 || l[k].K > 25 || l[k].K > l[k].in) return SNB_ERR_UNSUPPORTED;
+        if ((long long)l[k].in * l[k].out >= (1ll << 31) || (long long)B * l[k].in >= (1ll << 31) ||
+            (long long)B * l[k].out >= (1ll << 31))
+            return SNB_ERR_TOO_LARGE;
+    }
+    return SNB_OK;
+}
+
+}  // namespace
+}  // namespace snb
+
+using namespace snb;
+
+// 1 when the calls below take these layers: rows of W within the filter's width, and enough work that the pruned
+// form is the faster one (the sizes at which the single-layer entry points change over, for the net as a whole).
+extern "C" int snb_mlp_applies(const snb_mlp_layer* l, int depth, int B) {
+    if (check_layers(l, depth, B) != SNB_OK || (B + 31) / 32 > 65535) return 0;
+    long long work = 0;
+    for (int k = 0; k < depth; k++) {
+        if (l[k].in > 12288 || l[k].in < 64) return 0;
+        work += (long long)B * l[k].in * l[k].out;
+    }
+    return work >= (16ll << 20) * depth;
+}
+
+extern "C" size_t snb_mlp_saved_bytes(const snb_mlp_layer* l, int depth, int B) {
+    return check_layers(l, depth, B) == SNB_OK ? saved_layout(l, depth, B, nullptr, nullptr) : 0;
+}
+extern "C" size_t snb_mlp_scratch_bytes(const snb_mlp_layer* l, int depth, int B, int tensors, int training) {
+    return check_layers(l, depth, B) == SNB_OK ? scratch_layout(l, depth, B, tensors, training != 0, nullptr, nullptr) : 0;
+}
+// backward: two gradients row by row and one transposed
+extern "C" size_t snb_mlp_backward_scratch_bytes(const snb_mlp_layer* l, int depth, int B) {
+    if (check_layers(l, depth, B) != SNB_OK) return 0;
+    const size_t W = widest(l, depth), S = (B + 31) / 32;
+    return 2 * up256(sizeof(float) * B * W) + up256(sizeof(float) * S * 32 * W);
+}
+
+extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const float* x, int B, const long long* targets, float eps,
+                                     float clip, float lam, float scale, void* saved, void* scratch, float* loss, int* launches,
+                                     void* stream) {
+    int rc = check_layers(l, depth, B);
+    if (rc) return rc;
+    if (!x || !targets || !saved || !scratch || !loss) return SNB_ERR_NULL_POINTER;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int S = (B + 31) / 32;
+    Saved sv;
+    Scratch sc;
+    saved_layout(l, depth, B, static_cast<char*>(saved), &sv);
+    scratch_layout(l, depth, B, 1, true, static_cast<char*>(scratch), &sc);
+    int count = 0;
+    SNB_CUDA(cudaMemsetAsync(sc.zeroed, 0, sc.zero_bytes, st));
+    KeepJobs jobs{};
+    int masked = 0;
+    for (int k = 0; k < depth; k++)
+        if (l[k].kept_list) {
+            jobs.list[masked] = l[k].kept_list, jobs.flags[masked] = sv.keep[k];
+            jobs.count[masked] = l[k].kept, jobs.channels[masked] = l[k].out;
+            masked++;
+        }
+    if (masked) {
+        keep_flags_kernel<<<dim3(S, masked), 256, 0, st>>>(jobs);
+        SNB_CUDA(cudaGetLastError());
+        count++;
+    }
+    PrunePrep prep;
+    prep.x = x, prep.B = B, prep.CI = prep.W_CI = l[0].in;
+    prep.xt = sc.xt[0], prep.hi = sc.hi[0], prep.nlo = sc.nlo[0];
+    SNB_CUDA(prune_prepare(prep, st));
+    count++;
+    for (int k = 0; k < depth; k++) {
+        const bool head = k == depth - 1;
+        const int C = l[k].out;
+        PruneProblem p = layer_problem(l, k, B, 1);
+        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.fail_count = sc.fail[k];
+        p.pos = sv.pos[k], p.post = sv.post[k];
+        p.keep = l[k].kept_list ? sv.keep[k] : nullptr;
+        if (head) {
+            p.y = sc.d;
+            p.bias = l[k].bias;
+        } else {
+            p.yt = sc.xt[(k + 1) & 1];
+            p.part = sc.part;
+        }
+        SNB_CUDA(prune_forward(p, sc.prune, st));
+        count += 3;
+        if (!head) {
+            chain_shift_kernel<<<(C + SHIFT_C - 1) / SHIFT_C, 256, 0, st>>>(p.yt, p.part, p.keep, B, S, C, l[k].running_mean, l[k].momentum,
+                                                              sv.rows_kept[k], sc.hi[k + 1], sc.nlo[k + 1]);
+            SNB_CUDA(cudaGetLastError());
+            count++;
+        }
+    }
+    rc = snb_margin_loss(sc.d, targets, B, l[depth - 1].out, eps, clip, lam, scale, nullptr, sc.row_loss, loss, sv.grad_d, stream);
+    if (rc) return rc;
+    if (launches) *launches = count + 2;
+    return SNB_OK;
+}
+
+// grad_w [depth] (entries may be null), grad_bias of the head and grad_x [B, in] optional; grad_loss: device scalar.
+extern "C" int snb_mlp_train_backward(const snb_mlp_layer* l, int depth, int B, const float* grad_loss, const void* saved,
+                                      void* scratch, float* const* grad_w, float* grad_bias, float* grad_x, int* launches,
+                                      void* stream) {
+    int rc = check_layers(l, depth, B);
+    if (rc) return rc;
+    if (!grad_loss || !saved || !scratch || !grad_w) return SNB_ERR_NULL_POINTER;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int S = (B + 31) / 32, W = widest(l, depth);
+    Saved sv;
+    saved_layout(l, depth, B, const_cast<char*>(static_cast<const char*>(saved)), &sv);
+    Cursor at{static_cast<char*>(scratch)};
+    float* rows[2] = {at.take<float>((size_t)B * W), at.take<float>((size_t)B * W)};
+    float* gt = at.take<float>((size_t)S * 32 * W);
+    static std::atomic<int> configured[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int most = (W + 3) / 4 * 16;
+    if (most > 48 * 1024 && configured[dev & 63].load(std::memory_order_acquire) < most) {
+        SNB_CUDA(cudaFuncSetAttribute(chain_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        configured[dev & 63].store(most, std::memory_order_release);
+    }
+    int lowest = 0;                                          // deepest layer that anybody wants a gradient from
+    while (!grad_x && lowest < depth && !grad_w[lowest]) lowest++;
+    if (lowest == depth && grad_bias) lowest = depth - 1;
+    int count = 0;
+    const float* g = sv.grad_d;
+    for (int k = depth - 1; k >= lowest; k--) {
+        const bool head = k == depth - 1;
+        const int C = l[k].out, CI = l[k].in;
+        float* centred = rows[0];
+        chain_center_kernel<<<(C + 31) / 32, 1024, 0, st>>>(g, head ? grad_loss : nullptr, head ? nullptr : sv.rows_kept[k], B, S, C,
+                                                           centred, gt, head ? grad_bias : nullptr);
+        SNB_CUDA(cudaGetLastError());
+        count++;
+        float* gx = k > lowest ? rows[1] : (k == 0 ? grad_x : nullptr);
+        const int nx = gx ? B : 0, nw = grad_w[k] ? C : 0;
+        if (nx + nw > 0) {
+            chain_bwd_kernel<<<nx + nw, 256, (CI + 3) / 4 * 16, st>>>(centred, gt, sv.pos[k], sv.post[k], B, S, C, CI, nx, gx,
+                                                                      grad_w[k]);
+            SNB_CUDA(cudaGetLastError());
+            count++;
+        }
+        g = rows[1];
+    }
+    if (launches) *launches = count;
+    return SNB_OK;
+}
+
+// Evaluation pass.  tensors = 1: y only; 3: y, yl, yu for the box xl, xu, or (xl null) [max(x - eps, down), min(x + eps, up)].
+// y, yl, yu [B, classes] are the head's outputs; score / margin optional (tensors = 3, targets given).
+extern "C" int snb_mlp_eval_forward(const snb_mlp_layer* l, int depth, const float* x, const float* xl, const float* xu, int B,
+                                    int tensors, float box_eps, float down, float up, void* scratch, float* y, float* yl,
+                                    float* yu, const long long* targets, float inv_two_eps, float scale, float* score,
+                                    float* margin, int* launches, void* stream) {
+    int rc = check_layers(l, depth, B);
+    if (rc) return rc;
+    if (!x || !scratch || !y || (tensors == 3 && (!yl || !yu)) || ((xl != nullptr) != (xu != nullptr))) return SNB_ERR_NULL_POINTER;
+    if (tensors != 1 && tensors != 3) return SNB_ERR_UNSUPPORTED;
+    if (score && (tensors != 3 || !targets || !margin)) return SNB_ERR_NULL_POINTER;
+    cudaStream_t st = (cudaStream_t)stream;
+    Scratch sc;
+    scratch_layout(l, depth, B, tensors, false, static_cast<char*>(scratch), &sc);
+    int count = 0;
+    SNB_CUDA(cudaMemsetAsync(sc.zeroed, 0, sc.zero_bytes, st));
+    PrunePrep prep;
+    prep.x = x, prep.B = B, prep.CI = prep.W_CI = l[0].in;
+    if (tensors == 3) prep.xl = xl, prep.xu = xu, prep.box = !xl, prep.eps = box_eps, prep.down = down, prep.up = up;
+    prep.xt = sc.xt[0], prep.hi = sc.hi[0], prep.nlo = sc.nlo[0];
+    SNB_CUDA(prune_prepare(prep, st));
+    for (int k = 0; k < depth; k++) {
+        PruneProblem p = layer_problem(l, k, B, tensors);
+        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.fail_count = sc.fail[k];
+        p.mean = l[k].running_mean, p.bias = l[k].bias;
+        if (k == depth - 1) {
+            p.y = y;
+            if (tensors == 3) p.yl = yl, p.yu = yu;
+        } else {
+            p.yt = sc.xt[(k + 1) & 1], p.yhi = sc.hi[k + 1], p.ynlo = sc.nlo[k + 1];
+        }
+        SNB_CUDA(prune_forward(p, sc.prune, st));
+        count += 3;
+    }
+    if (score) {
+        const int n = B * l[depth - 1].out;
+        scores_kernel<<<(n + 255) / 256, 256, 0, st>>>(y, yl, yu, targets, B, l[depth - 1].out, inv_two_eps, scale, score, margin);
+        SNB_CUDA(cudaGetLastError());
+        count++;
+    }
+    if (launches) *launches = count + 1;
+    return SNB_OK;
+}

@@ -18,9 +18,9 @@ struct PruneArgs {
     PruneProblem p;
     int S, NX, m, lcap;
     unsigned* fail_count;
-    unsigned* hi;                   // order-preserving codes of max(x), max(-x) per column; 0 = no value
-    unsigned* nlo;
-    float* xt;                      // [S][W_CI][NX][32]
+    const unsigned* hi;             // order codes of max(x), max(-x) per column; 0 = no value
+    const unsigned* nlo;
+    const float* xt;                // [S][W_CI][NX][32]
     int* inv;                       // [S][W_CI] full column -> compact position (with ci)
     int* cnt;                       // [W_CO] list length, -1: no list
     float* tau;                     // [W_CO]
@@ -29,20 +29,11 @@ struct PruneArgs {
     int4* fail;                     // units (sub-batch, first output, mask of outputs) left to prune_fix
 };
 
-__device__ __forceinline__ unsigned order_code(float f) {
-    const unsigned b = __float_as_uint(f);
-    return f != f ? 0u : ((b & 0x80000000u) ? ~b : (b | 0x80000000u));
-}
-__device__ __forceinline__ float decode(unsigned e) {   // 0 -> NaN
-    return __uint_as_float((e & 0x80000000u) ? (e ^ 0x80000000u) : ~e);
-}
-
 // ---- transpose + column ranges ----------------------------------------------------------------
 // CTA = 32 rows (one sub-batch) x 64 compact columns.  Bound by the traffic of x and xt and by launch latency.
 template <int NX>
-__global__ void __launch_bounds__(256) prune_prep(const PruneArgs a) {
+__global__ void __launch_bounds__(256) prune_prep(const PrunePrep p) {
     __shared__ float tile[NX][32][65];
-    const PruneProblem& p = a.p;
     const int s = blockIdx.y, c0 = blockIdx.x * 64, tid = threadIdx.x;
     const float nan = __int_as_float(0x7fc00000);
     const int col = tid & 63, r0 = tid >> 6;
@@ -52,9 +43,17 @@ __global__ void __launch_bounds__(256) prune_prep(const PruneArgs a) {
         const int r = r0 + 4 * i, b = s * 32 + r;
         const bool ok = cok && b < p.B;
         const size_t o = (size_t)b * p.CI + c0 + col;
-        if (NX != 2) tile[0][r][col] = ok ? p.x[o] : nan;
+        float x = nan;
+        if (NX != 2) tile[0][r][col] = x = ok ? p.x[o] : nan;
         if (NX >= 2) {
-            float l = ok ? p.xl[o] : nan, u = ok ? p.xu[o] : nan;
+            float l = nan, u = nan;
+            if (NX == 3 && p.box) {
+                l = x == x ? fmaxf(x - p.eps, p.down) : x;
+                u = x == x ? fminf(x + p.eps, p.up) : x;
+            } else if (ok) {
+                l = p.xl[o];
+                u = p.xu[o];
+            }
             if (l > u) l = u = (l + u) * 0.5f;               // inverted interval -> its midpoint
             tile[NX - 2][r][col] = l;
             tile[NX - 1][r][col] = u;
@@ -71,16 +70,16 @@ __global__ void __launch_bounds__(256) prune_prep(const PruneArgs a) {
 #pragma unroll
         for (int t = 0; t < NX; t++) {
             const float v = tile[t][lane][lc];
-            a.xt[(((size_t)s * p.W_CI + c) * NX + t) * 32 + lane] = v;
+            p.xt[(((size_t)s * p.W_CI + c) * NX + t) * 32 + lane] = v;
             hi = max(hi, order_code(v));
             nlo = max(nlo, order_code(-v));
         }
         hi = __reduce_max_sync(0xffffffffu, hi);
         nlo = __reduce_max_sync(0xffffffffu, nlo);
         if (lane == 0) {
-            atomicMax(a.hi + c, hi);
-            atomicMax(a.nlo + c, nlo);
-            if (p.ci) a.inv[(size_t)s * p.W_CI + c] = c0 + lc;
+            atomicMax(p.hi + c, hi);
+            atomicMax(p.nlo + c, nlo);
+            if (p.ci) p.inv[(size_t)s * p.W_CI + c] = c0 + lc;
         }
     }
 }
@@ -363,11 +362,11 @@ template <int NX, bool TRACK>
 struct MaxState {
     float acc[NX];
     uint32_t word[TRACK ? NX : 1];
-    __device__ __forceinline__ void init() {
+    __device__ __forceinline__ void init(uint32_t floor_word) {
 #pragma unroll
         for (int t = 0; t < NX; t++) acc[t] = SNB_EPS;
         if (TRACK) {
-            word[0] = NX == 2 ? SNB_NO_GRAD_ID : 0u;         // lower bound: no gradient until it leaves its floor
+            word[0] = NX == 2 ? SNB_NO_GRAD_ID : floor_word; // lower bound: no gradient until it leaves its floor
             if (NX == 2) word[NX - 1] = 0u;
         }
     }
@@ -406,20 +405,30 @@ struct TopList {
 #pragma unroll
         for (int s = 0; s < KMAX; s++) v[s] = 0.f;
     }
-    // warp-uniform branch: a value that beats no row's weakest slot changes nothing
+    // Warp-uniform branches: a value that beats no row's weakest slot changes nothing, and one that beats no row's
+    // slot HALF only moves the slots below it (the lists are walked largest first, so that is the later entries' lot).
     __device__ __forceinline__ void add(float d) {
+        constexpr int HALF = KMAX / 2;
         if (__any_sync(0xffffffffu, d > v[0])) {
             const float e = d == d ? d : 0.f;                // a NaN must not move the list
+            if (__any_sync(0xffffffffu, d > v[HALF])) {
 #pragma unroll
-            for (int s = 0; s < KMAX - 1; s++) v[s] = fmaxf(v[s], fminf(v[s + 1], e));
-            v[KMAX - 1] = fmaxf(v[KMAX - 1], e);
+                for (int s = 0; s < KMAX - 1; s++) v[s] = fmaxf(v[s], fminf(v[s + 1], e));
+                v[KMAX - 1] = fmaxf(v[KMAX - 1], e);
+            } else {
+#pragma unroll
+                for (int s = 0; s < HALF - 1; s++) v[s] = fmaxf(v[s], fminf(v[s + 1], e));
+                v[HALF - 1] = fmaxf(v[HALF - 1], e);
+            }
         }
     }
+    // v[KMAX - K], as a minimum over an ascending tail: an index that is not a constant would move the list to local memory
     __device__ __forceinline__ float kth(int K) const {
-        float r = v[0];
+        if (K == KMAX) return v[0];
+        float r = v[KMAX - 1];
 #pragma unroll
-        for (int s = 1; s < KMAX; s++)
-            if (s == KMAX - K) r = v[s];
+        for (int s = 0; s < KMAX - 1; s++)
+            if (s >= KMAX - K) r = fminf(r, v[s]);
         return r;
     }
     // (eps0 + sum_r q (1-q)^r v_r) / (1 - (1-q)^K), largest first, in the reference's order of operations
@@ -477,10 +486,10 @@ struct PosList {
     __device__ __forceinline__ void add(float t, uint32_t c, int K) {
         const float d = fabsf(t);
         if (!__any_sync(0xffffffffu, d > seed)) return;
-        float weakest = v[0];
+        float weakest = v[KMAX - 1];
 #pragma unroll
-        for (int s = 1; s < KMAX; s++)
-            if (s == KMAX - K) weakest = v[s];
+        for (int s = 0; s < KMAX - 1; s++)
+            if (s >= KMAX - K) weakest = fminf(weakest, v[s]);
         const bool enter = d > seed && d > weakest;
         const uint32_t wd = c | (t >= 0.f ? 0u : SNB_SIGN_BIT);
 #pragma unroll
@@ -493,6 +502,82 @@ struct PosList {
         }
     }
 };
+
+// ---- results of 32 outputs / of one output ---------------------------------------------------------
+template <int NV>
+__device__ __forceinline__ float shifted(const PruneProblem& p, float v, int j) {
+    if (p.mean) v = v - p.mean[j];
+    if (p.bias) v = v + p.bias[j];
+    return v;
+}
+
+// One output of a sub-batch in the chain form, lane = row.
+template <int NV>
+__device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, const float (&v)[NV], uint32_t word) {
+    const int lane = threadIdx.x & 31;
+    const bool live = s * 32 + lane < p.B, kept = !p.keep || p.keep[(size_t)s * p.CO + j];
+    if (p.yt) {
+        unsigned hi = 0u, nlo = 0u;
+#pragma unroll
+        for (int t = 0; t < NV; t++) {
+            const float o = live && kept ? shifted<NV>(p, v[t], j) : __int_as_float(0x7fc00000);
+            p.yt[(((size_t)s * p.CO + j) * NV + t) * 32 + lane] = o;
+            hi = max(hi, order_code(o));
+            nlo = max(nlo, order_code(-o));
+        }
+        if (p.yhi) {
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            nlo = __reduce_max_sync(0xffffffffu, nlo);
+            if (lane == 0) {
+                atomicMax(p.yhi + j, hi);
+                atomicMax(p.ynlo + j, nlo);
+            }
+        }
+    }
+    if (p.post) p.post[((size_t)s * p.CO + j) * 32 + lane] = live && kept ? (int)word : (int)SNB_NO_GRAD_ID;
+}
+
+// 32 outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
+template <int NX, int NV, int NW>
+__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* outs[NV];
+    if (NX != 2) outs[0] = p.y;
+    if (NX >= 2) outs[NV - 2] = p.yl, outs[NV - 1] = p.yu;
+    const int no = n0 + lane;
+    const bool kept = no < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + no]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int r = warp + 8 * k, b = s * 32 + r;
+        if (b >= p.B || no >= p.CO) continue;
+        const size_t o = (size_t)b * p.CO + no;
+#pragma unroll
+        for (int t = 0; t < NV; t++)
+            if (outs[t]) outs[t][o] = shifted<NV>(p, tile[t][r][lane], no);
+        if (NW == 1 && NX == 1) p.pos[o] = kept ? __float_as_int(tile[NV][r][lane]) : (int)SNB_NO_GRAD_ID;
+        if (NW == 2) {
+            p.posl[o] = __float_as_int(tile[NV][r][lane]);
+            p.posu[o] = __float_as_int(tile[NV + NW - 1][r][lane]);
+        }
+    }
+    if (p.yt || p.post) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int slot = warp * 4 + i;
+            if (n0 + slot >= p.CO) break;
+            float v[NV];
+#pragma unroll
+            for (int t = 0; t < NV; t++) v[t] = tile[t][lane][slot];
+            emit_chain<NV>(p, s, n0 + slot, v, NW > 0 ? __float_as_uint(tile[NW > 0 ? NV : 0][lane][slot]) : 0u);
+        }
+    }
+    if (p.part && warp == 0 && no < p.CO) {
+        float sum = 0.f;
+        const int rows = min(32, p.B - s * 32);
+        for (int r = 0; r < rows; r++) sum += tile[0][r][lane];
+        p.part[(size_t)s * p.CO + no] = kept ? sum : 0.f;
+    }
+}
 
 // ---- list walks -----------------------------------------------------------------------------------
 // CTA = 32 outputs of one sub-batch, eight lanes per output, four rows per lane (one 16-byte load of xt per tensor and
@@ -514,7 +599,8 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     if (tid == 0) failed = 0u;
     __syncthreads();
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
-    const int cnt = n < p.CO ? a.cnt[j] : 0;
+    const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
+    const int cnt = wanted ? a.cnt[j] : 0;
     const float tau = a.tau[j];
     const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
     const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
@@ -600,7 +686,7 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
         }
     }
     const unsigned good = __ballot_sync(0xffffffffu, worst() >= tau);
-    if (l == 0 && n < p.CO && (cnt < 0 || ((good >> (8 * g)) & 0xffu) != 0xffu)) atomicOr(&failed, 1u << slot);
+    if (l == 0 && wanted && (cnt < 0 || ((good >> (8 * g)) & 0xffu) != 0xffu)) atomicOr(&failed, 1u << slot);
 #pragma unroll
     for (int t = 0; t < NV; t++)
 #pragma unroll
@@ -631,13 +717,14 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
             }
             return word;
         };
+        const uint32_t floor_word = p.kept_list ? (uint32_t)p.kept_list[(size_t)s * p.kept] : 0u;
         uint32_t word[TRACK ? NV : 1][4];
 #pragma unroll
         for (int t = 0; t < NV; t++)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int k = at[TRACK ? t : 0][TRACK ? q : 0];
-                uint32_t wd = (NX == 2 && t == 0) ? SNB_NO_GRAD_ID : 0u;
+                uint32_t wd = (NX == 2 && t == 0) ? SNB_NO_GRAD_ID : floor_word;
                 if (k >= 0) {
                     wd = step_word(t, q, k, acc[t][q], 0x7fffffffu);
                     if ((tied >> (t * 4 + q)) & 1u)
@@ -651,18 +738,7 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
             for (int q = 0; q < 4; q++) tile[NV + (TRACK ? t : 0)][4 * l + q][slot] = __uint_as_float(word[TRACK ? t : 0][q]);
     }
     __syncthreads();
-    float* outs[NV + WORDS];
-    if (NX != 2) outs[0] = p.y;
-    if (NX >= 2) outs[NX - 2] = p.yl, outs[NX - 1] = p.yu;
-    if (TRACK && NX == 1) outs[1] = reinterpret_cast<float*>(p.pos);
-    if (TRACK && NX == 2) outs[NX] = reinterpret_cast<float*>(p.posl), outs[NX + WORDS - 1] = reinterpret_cast<float*>(p.posu);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int r = warp + 8 * k, b = s * 32 + r, no = n0 + lane;
-        if (b >= p.B || no >= p.CO) continue;
-#pragma unroll
-        for (int t = 0; t < NV + WORDS; t++) outs[t][(size_t)b * p.CO + no] = tile[t][r][lane];
-    }
+    emit_tile<NX, NV, WORDS>(p, tile, s, n0);
     if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
 }
 
@@ -700,6 +776,7 @@ __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, con
 template <int NX, int KMAX, bool POS>
 __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
+    constexpr int WALK = STEP;                               // entries per step: all insertion chains of a step are unrolled
     extern __shared__ __align__(16) unsigned char dyn[];
     float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(dyn);   // [NX] values, then [K] words
     __shared__ unsigned failed;
@@ -721,14 +798,14 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
         SortState<NX, KMAX> st;
         st.init();
         int k = 0;                                           // entries seen
-        for (; k < cnt; k += PAD) {
+        for (; k < cnt; k += WALK) {
             if (k >= K) {
                 const float left = ub[k / STEP];
                 if (__all_sync(0xffffffffu, !live || st.worst(K) > left)) break;
             }
-            float w[PAD], v[PAD][NX];
+            float w[WALK], v[WALK][NX];
 #pragma unroll
-            for (int e = 0; e < PAD / 2; e++) {
+            for (int e = 0; e < WALK / 2; e++) {
                 const int4 two = list[k / 2 + e];
                 w[2 * e] = __int_as_float(two.y);
                 w[2 * e + 1] = __int_as_float(two.w);
@@ -739,7 +816,7 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
                 }
             }
 #pragma unroll
-            for (int e = 0; e < PAD; e++) st.add(v[e], w[e], 0u);
+            for (int e = 0; e < WALK; e++) st.add(v[e], w[e], 0u);
         }
         const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || st.worst(K) >= tau);
         if (!good && lane == 0) atomicOr(&failed, 1u << slot);
@@ -789,20 +866,17 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
         }
     }
     __syncthreads();
-    float* outs[NX];
-    if (NX != 2) outs[0] = p.y;
-    if (NX >= 2) outs[NX - 2] = p.yl, outs[NX - 1] = p.yu;
+    emit_tile<NX, NX, 0>(p, tile, s, n0);
+    if (POS) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int r = warp + 8 * k, b = s * 32 + r, n = n0 + lane;
-        if (b >= p.B || n >= p.CO) continue;
-#pragma unroll
-        for (int t = 0; t < NX; t++) outs[t][(size_t)b * p.CO + n] = tile[t][r][lane];
-        if (POS)
+        for (int k = 0; k < 4; k++) {
+            const int r = warp + 8 * k, b = s * 32 + r, n = n0 + lane;
+            if (b >= p.B || n >= p.CO) continue;
             for (int t = 0; t < K; t++) {
                 const uint32_t word = __float_as_uint(tile[NX + t][r][lane]);
                 p.pos[((size_t)t * p.B + b) * p.CO + n] = word == EMPTY ? 0 : (int)word;   // fewer than K values above 0
             }
+        }
     }
     if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
 }
@@ -835,11 +909,18 @@ __global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
         const float* xs = a.xt + (size_t)s * C * NX * 32;
         const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
         const int b = s * 32 + lane;
-        auto store = [&](const MaxState<NX, TRACK>& st, int n) {
+        const uint32_t floor_word = p.kept_list ? (uint32_t)p.kept_list[(size_t)s * p.kept] : 0u;
+        auto store = [&](const MaxState<NX, TRACK>& st, int n) {          // all lanes of a warp
+            if (p.yt || p.post) emit_chain<NX>(p, s, n, st.acc, TRACK ? st.word[0] : 0u);
+            if (p.part) {
+                float sum = 0.f;
+                for (int r = 0; r < min(32, p.B - s * 32); r++) sum += __shfl_sync(0xffffffffu, st.acc[0], r);
+                if (lane == 0) p.part[(size_t)s * p.CO + n] = sum;
+            }
             if (b >= p.B) return;
             const size_t o = (size_t)b * p.CO + n;
-            if (NX != 2) p.y[o] = st.acc[0];
-            if (NX >= 2) p.yl[o] = st.acc[NX - 2], p.yu[o] = st.acc[NX - 1];
+            if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, st.acc[0], n);
+            if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, st.acc[NX - 2], n), p.yu[o] = shifted<NX>(p, st.acc[NX - 1], n);
             if (TRACK && NX == 1) p.pos[o] = (int)st.word[0];
             if (TRACK && NX == 2) p.posl[o] = (int)st.word[0], p.posu[o] = (int)st.word[TRACK ? NX - 1 : 0];
         };
@@ -850,7 +931,7 @@ __global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
                 todo &= todo - 1;
                 const float* wr = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
                 MaxState<NX, TRACK> st;
-                st.init();
+                st.init(floor_word);
                 for (int c0 = warp * 8; c0 < C; c0 += 64) {
                     float v[8][NX], w[8];
 #pragma unroll
@@ -902,7 +983,7 @@ __global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
         for (int i = 0; i < 4; i++) {
             const int n = min(n0 + warp * 4 + i, p.CO - 1);
             wr[i] = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
-            st[i].init();
+            st[i].init(floor_word);
         }
         fix_stage<NX>(xs, sm[0], 0, C);
         cp_async_commit();
@@ -986,9 +1067,15 @@ __global__ void __launch_bounds__(256) prune_fix_sort(const PruneArgs a) {
             SortState<NX, KMAX> st;
             st.init();
             sweep([&](const float(&v)[NX], float w, uint32_t c) { st.add(v, w, c); });
-            if (mine && b < p.B) {
-                if (NX != 2) p.y[o] = st.result(0, K, p.q);
-                if (NX >= 2) p.yl[o] = st.result(NX - 2, K, p.q), p.yu[o] = st.result(NX - 1, K, p.q);
+            if (mine) {
+                float v[NX];
+#pragma unroll
+                for (int t = 0; t < NX; t++) v[t] = st.result(t, K, p.q);
+                if (p.yt) emit_chain<NX>(p, s, n, v, 0u);
+                if (b < p.B) {
+                    if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, v[0], n);
+                    if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, v[NX - 2], n), p.yu[o] = shifted<NX>(p, v[NX - 1], n);
+                }
             }
             if constexpr (POS) {
                 PosList<KMAX> pl;
@@ -1015,10 +1102,11 @@ bool with_words(const PruneProblem& p) { return p.pos || p.posl; }
 // that this happens to about one output in 10^7 for random lists, and such outputs go to prune_fix.
 int threshold_rank(const PruneProblem& p) {
     int m = p.K;
-    if (p.ci) {
-        const double gone = 1.0 - (double)p.CI / p.W_CI;
+    if (p.ci || p.kept) {
+        const double gone = 1.0 - (double)(p.kept ? p.kept : p.CI) / p.W_CI;
         m = 1;
         for (double all = gone; all > 1e-7 && m < 16; all *= gone) m++;
+        if (m < p.K) m = p.K;
     }
     return m;
 }
@@ -1040,8 +1128,9 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
         off += up256(bytes);
         return at;
     };
-    char* zeroed = take(64 + 2 * up256(sizeof(unsigned) * C));    // counter and ranges: one memset
-    char* xt = take(sizeof(float) * S * C * NX * 32);
+    const bool given = p.xt != nullptr;
+    char* zeroed = take(64 + (given ? 0 : 2 * up256(sizeof(unsigned) * C)));    // counter and ranges: one memset
+    char* xt = take(given ? 0 : sizeof(float) * S * C * NX * 32);
     char* inv = take(p.ci ? sizeof(int) * S * C : 0);
     char* cnt = take(sizeof(int) * J);
     char* tau = take(sizeof(float) * J);
@@ -1054,10 +1143,10 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
         a->NX = (int)NX;
         a->m = threshold_rank(p);
         a->lcap = (int)lcap;
-        a->fail_count = reinterpret_cast<unsigned*>(zeroed);
-        a->hi = reinterpret_cast<unsigned*>(zeroed + 64);
-        a->nlo = reinterpret_cast<unsigned*>(zeroed + 64 + up256(sizeof(unsigned) * C));
-        a->xt = reinterpret_cast<float*>(xt);
+        a->fail_count = p.fail_count ? p.fail_count : reinterpret_cast<unsigned*>(zeroed);
+        a->hi = given ? p.hi : reinterpret_cast<unsigned*>(zeroed + 64);
+        a->nlo = given ? p.nlo : reinterpret_cast<unsigned*>(zeroed + 64 + up256(sizeof(unsigned) * C));
+        a->xt = given ? p.xt : reinterpret_cast<float*>(xt);
         a->inv = p.ci ? reinterpret_cast<int*>(inv) : nullptr;
         a->cnt = reinterpret_cast<int*>(cnt);
         a->tau = reinterpret_cast<float*>(tau);
@@ -1136,19 +1225,30 @@ bool prune_applies(const PruneProblem& p) {
 
 size_t prune_workspace_bytes(const PruneProblem& p) { return layout(p, nullptr, nullptr); }
 
+cudaError_t prune_prepare(const PrunePrep& q, cudaStream_t st) {
+    const dim3 grid((q.CI + 63) / 64, (q.B + 31) / 32);
+    if (!q.x) prune_prep<2><<<grid, 256, 0, st>>>(q);
+    else if (q.box || q.xl) prune_prep<3><<<grid, 256, 0, st>>>(q);
+    else prune_prep<1><<<grid, 256, 0, st>>>(q);
+    return cudaGetLastError();
+}
+
 cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
     PruneArgs a{};
     layout(p, static_cast<char*>(ws), &a);
     const size_t C = p.W_CI;
-    cudaError_t e = cudaMemsetAsync(a.fail_count, 0, 64 + 2 * up256(sizeof(unsigned) * C), st);
+    cudaError_t e = cudaSuccess;
+    if (!p.fail_count) e = cudaMemsetAsync(a.fail_count, 0, 64 + (p.xt ? 0 : 2 * up256(sizeof(unsigned) * C)), st);
     if (e != cudaSuccess) return e;
-    // all bits set is a NaN: the dropped columns
-    if (p.ci && (e = cudaMemsetAsync(a.xt, 0xff, sizeof(float) * a.S * C * a.NX * 32, st)) != cudaSuccess) return e;
-    const dim3 pg((p.CI + 63) / 64, a.S);
-    if (a.NX == 1) prune_prep<1><<<pg, 256, 0, st>>>(a);
-    else if (a.NX == 2) prune_prep<2><<<pg, 256, 0, st>>>(a);
-    else prune_prep<3><<<pg, 256, 0, st>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (!p.xt) {
+        // all bits set is a NaN: the dropped columns
+        float* xt = const_cast<float*>(a.xt);
+        if (p.ci && (e = cudaMemsetAsync(xt, 0xff, sizeof(float) * a.S * C * a.NX * 32, st)) != cudaSuccess) return e;
+        PrunePrep q;
+        q.x = p.x, q.xl = p.xl, q.xu = p.xu, q.ci = p.ci, q.inv = a.inv, q.B = p.B, q.CI = p.CI, q.W_CI = p.W_CI;
+        q.xt = xt, q.hi = const_cast<unsigned*>(a.hi), q.nlo = const_cast<unsigned*>(a.nlo);
+        if ((e = prune_prepare(q, st)) != cudaSuccess) return e;
+    }
     e = (C % 4 == 0) && aligned16(p.w) ? filter<true>(a, st) : filter<false>(a, st);
     if (e != cudaSuccess) return e;
     const dim3 grid((p.CO + 31) / 32, a.S);
@@ -1164,7 +1264,7 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
         return a.NX == 2 ? run_sort<2, 10, false>(a, grid, fg, st) : run_sort<3, 10, false>(a, grid, fg, st);
     }
     if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, grid, fg, st) : run_sort<1, 25, false>(a, grid, fg, st);
-    return run_sort<2, 25, false>(a, grid, fg, st);
+    return a.NX == 2 ? run_sort<2, 25, false>(a, grid, fg, st) : run_sort<3, 25, false>(a, grid, fg, st);
 }
 
 }  // namespace snb

@@ -41,7 +41,53 @@ struct PruneProblem {
     int* posu = nullptr;
     int K = 1;                  // 1: maximum; 2..25: sort neuron of that many values
     float q = 0.f;
+
+    // Chain form (csrc/mlp.cu): one layer hands its result to the next without a row-major copy in between.
+    // Input: xt [S][W_CI][tensors][32] and the order codes of its column ranges, as prune_prep leaves them (x, xl, xu
+    // then only say which tensors there are; ci and co are null); kept = columns that every sub-batch holds.
+    const float* xt = nullptr;
+    const unsigned* hi = nullptr;
+    const unsigned* nlo = nullptr;
+    int kept = 0;
+    // Output: yt [S][CO][tensors][32], NaN in rows past the batch and in outputs that `keep` [S][CO] drops; ranges
+    // (zeroed before), sums over the rows of a sub-batch in row order [S][CO], words [S][CO][32] and in pos [B][CO]
+    // (SNB_NO_GRAD_ID where dropped).  y = (y - mean[j]) + bias[j] before it is written anywhere (either may be null).
+    float* yt = nullptr;
+    unsigned* yhi = nullptr;
+    unsigned* ynlo = nullptr;
+    float* part = nullptr;
+    int* post = nullptr;
+    const unsigned char* keep = nullptr;
+    const float* mean = nullptr;
+    const float* bias = nullptr;
+    unsigned* fail_count = nullptr;     // a zeroed counter of the caller's, or null: one in the workspace
+    const int* kept_list = nullptr;     // [S][kept] kept columns: the first one is the position of an output at its floor
 };
+
+// Transposes x (or x and the box [max(x - eps, down), min(x + eps, up)], or given box ends) to the chain form.
+struct PrunePrep {
+    const float* x = nullptr;
+    const float* xl = nullptr;
+    const float* xu = nullptr;
+    const int* ci = nullptr;
+    int* inv = nullptr;
+    int B = 0, CI = 0, W_CI = 0;
+    bool box = false;           // make xl, xu from x
+    float eps = 0.f, down = 0.f, up = 0.f;
+    float* xt = nullptr;
+    unsigned* hi = nullptr;     // zeroed before
+    unsigned* nlo = nullptr;
+};
+cudaError_t prune_prepare(const PrunePrep& q, cudaStream_t st);
+
+// Order-preserving codes of floats; 0 stands for "no value" (NaN).
+__device__ __forceinline__ unsigned order_code(float f) {
+    const unsigned b = __float_as_uint(f);
+    return f != f ? 0u : ((b & 0x80000000u) ? ~b : (b | 0x80000000u));
+}
+__device__ __forceinline__ float decode(unsigned e) {   // 0 -> NaN
+    return __uint_as_float((e & 0x80000000u) ? (e ^ 0x80000000u) : ~e);
+}
 
 // Whether the pruned evaluation is the faster one for this problem (sizes only), and its scratch.
 bool prune_applies(const PruneProblem& p);

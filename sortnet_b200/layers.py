@@ -424,6 +424,33 @@ class SortMLPModel(nn.Module):
             masks[k] = sample_mask(sub, 1, l.in_features, l.keep_rate, device, count=max(int(c), 1))
         return masks
 
+    def _plan(self, masks=None, sort_eval=False):
+        """Layer table for the whole-net calls (norm_dist_cuda.MlpPlan), or None when the stack is not the
+        one built here (hidden layers with a mean shift and no bias, a head without mean shift, p = inf)."""
+        rows, last = [], len(self.fc_dist) - 1
+        for k, l in enumerate(self.fc_dist):
+            shift = l.mean_shift
+            if not math.isinf(l.p) or (shift is None) != (k == last) or (k < last and l.bias is not None):
+                return None
+            if shift is not None and (shift.affine or shift.training != l.training):
+                return None
+            K, q = 1, 0.0
+            if sort_eval and not ops._sort_is_plain_max(l.weight, l.dropout, 10):
+                K, q = min(l.in_features, 10), l.dropout
+            kept = _as_index32(masks[k]) if masks is not None and k < last else None
+            rows.append((l.weight, l.bias, None if shift is None else shift.running_mean,
+                         0.0 if shift is None else shift.momentum, kept, K, q))
+        return _C.MlpPlan(rows)
+
+    def _eval_plan(self, x, sort_eval):
+        """The plan for an evaluation pass without gradients on x [B, pixels], or None."""
+        if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist):
+            return None
+        if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
+            return None
+        plan = self._plan(sort_eval=sort_eval)
+        return plan if plan is not None and plan.applies(x.size(0)) else None
+
     @torch.no_grad()
     def certified_margin(self, x, targets, eps, up, down, sort_eval=None, after_layer=None):
         """Evaluation-mode interval-bound pass over the box [x - eps, x + eps] clipped to
@@ -457,7 +484,10 @@ class SortMLPModel(nn.Module):
             else:
                 lower = torch.maximum(x - eps, torch.as_tensor(down, device=x.device))
                 upper = torch.minimum(x + eps, torch.as_tensor(up, device=x.device))
-            for k, layer in enumerate(self.fc_dist):
+            plan = self._eval_plan(x, sort_eval) if after_layer is None else None
+            if plan is not None:
+                _, lower, upper, _, _ = _C.mlp_eval_forward(plan, x.contiguous(), (lower.contiguous(), upper.contiguous()))
+            for k, layer in enumerate(self.fc_dist if plan is None else ()):
                 assert math.isinf(layer.p)
                 x, lower, upper = layer(x, lower, upper, sort_eval=sort_eval and layer.keep_rate != 1.0)
                 if after_layer is not None:
@@ -478,7 +508,17 @@ class SortMLPModel(nn.Module):
         """Training forward followed by the reference's `mixture` loss (main.py:357-364) on the
         margin of ell_inf_models.py:45-50: mean_b max_c clamp(margin, 0, clip) + lam * cross_entropy.
         Same value and gradients as `forward(x, targets, eps)` followed by that loss in PyTorch
-        ops; the head (margin, loss and its gradient) runs as one kernel."""
+        ops; the head (margin, loss and its gradient) runs as one kernel, and at p = inf the whole pass is
+        one library call per direction (ops.MlpMixtureLossF)."""
+        x = x.reshape(x.size(0), -1)
+        if FUSED_LAYERS and self.training and x.is_cuda and x.dtype == torch.float32 and torch.is_grad_enabled() \
+                and not isinstance(self.scalar, torch.Tensor) and all(math.isinf(l.p) for l in self.fc_dist):
+            if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
+                masks = self.draw_masks(x.size(0), x.device)
+            plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)
+            if plan is not None and plan.applies(x.size(0)) and any(t.requires_grad for t in (x, *plan.weights)):
+                return ops.MlpMixtureLossF.apply(x.contiguous(), targets.contiguous(), eps, clip, lam, float(self.scalar), plan,
+                                                 plan.head_bias, *plan.weights)
         d = self._distances(x, masks)
         if FUSED_LAYERS and d.is_cuda and not isinstance(self.scalar, torch.Tensor):
             return ops.margin_loss(d, targets, eps, clip, lam, float(self.scalar))
@@ -514,6 +554,25 @@ class SortMLPModel(nn.Module):
     def forward(self, x=None, targets=None, eps=0, up=None, down=None, masks=None):
         x = x.reshape(x.size(0), -1)
         lower = upper = None
+        plan = self._eval_plan(x, any(l.keep_rate != 1.0 for l in self.fc_dist))
+        if plan is not None:
+            x = x.contiguous()
+            if up is None or down is None:
+                y = _C.mlp_eval_forward(plan, x)[0]
+                return -y * self.scalar if targets is None else self._scores(y, None, None, targets, eps)
+            if isinstance(up, (int, float)) and isinstance(down, (int, float)):
+                box = (eps, down, up)
+            else:
+                up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
+                box = (torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down).contiguous(),
+                       torch.minimum(x + eps, up.reshape(1, -1) if up.dim() else up).contiguous())
+            number = not isinstance(self.scalar, torch.Tensor)
+            y, lower, upper, score, margin = _C.mlp_eval_forward(
+                plan, x, box, targets.contiguous() if targets is not None and number else None, 2 * eps,
+                float(self.scalar) if number else 1.0)
+            if targets is None:
+                return -y * self.scalar
+            return (score, margin) if number else self._scores(y, lower, upper, targets, eps)
         if up is not None and down is not None and self._certifying():
             up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
             lower = torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down)

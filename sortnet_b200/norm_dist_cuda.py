@@ -567,6 +567,88 @@ def certified_fraction(yl, yu, targets, row_flag, fraction):
                 row_flag.data_ptr(), fraction.data_ptr())
 
 
+# ---- a whole SortNet-MLP per call -----------------------------------------------------------------
+
+
+class MlpLayer(ctypes.Structure):
+    """snb_mlp_layer of include/sortnet_b200.h."""
+    _fields_ = [("w", ctypes.c_void_p), ("bias", ctypes.c_void_p), ("running_mean", ctypes.c_void_p),
+                ("kept_list", ctypes.c_void_p), ("n_in", ctypes.c_int), ("n_out", ctypes.c_int), ("kept", ctypes.c_int),
+                ("K", ctypes.c_int), ("momentum", ctypes.c_float), ("q", ctypes.c_float)]
+
+
+class MlpPlan:
+    """The layer table of one call, with the tensors it points to."""
+
+    def __init__(self, rows):
+        """rows: (weight, bias, running_mean, momentum, kept list [S, 1, count] or None, K, q) per layer."""
+        self.depth = len(rows)
+        self.weights = [r[0] for r in rows]
+        self.head_bias = rows[-1][1]
+        self.keep = rows
+        self.table = (MlpLayer * self.depth)(*[
+            MlpLayer(w.data_ptr(), _ptr(b), _ptr(rm), _ptr(kept), w.size(1), w.size(0), 0 if kept is None else kept.size(2),
+                     K, mom, q) for w, b, rm, mom, kept, K, q in rows])
+
+    def applies(self, B):
+        return _timeline is None and bool(_lib.load().snb_mlp_applies(self.table, self.depth, B))
+
+
+def _mlp_call(entry, ref, *args):
+    """Runs a snb_mlp_* entry point with the device of `ref` current; counts what it launched."""
+    global launch_count
+    dev, fn, n = ref.device, getattr(_lib.load(), entry), ctypes.c_int(0)
+    if torch.cuda.current_device() == dev.index:
+        rc = fn(*args, ctypes.byref(n), torch.cuda.current_stream(dev).cuda_stream)
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, ctypes.byref(n), torch.cuda.current_stream(dev).cuda_stream)
+    if rc:
+        _lib.check(rc, entry[4:])
+    launch_count += n.value
+
+
+def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):
+    """snb_mlp_train_forward: (loss, saved); x [B, in] fp32, targets [B] int64."""
+    B, lib = x.size(0), _lib.load()
+    saved = torch.empty(lib.snb_mlp_saved_bytes(plan.table, plan.depth, B), device=x.device, dtype=torch.uint8)
+    scratch = torch.empty(lib.snb_mlp_scratch_bytes(plan.table, plan.depth, B, 1, 1), device=x.device, dtype=torch.uint8)
+    loss = torch.empty((), device=x.device, dtype=torch.float32)
+    _mlp_call("snb_mlp_train_forward", x, plan.table, plan.depth, x.data_ptr(), B, targets.data_ptr(), float(eps), float(clip),
+              float(lam), float(scale), saved.data_ptr(), scratch.data_ptr(), loss.data_ptr())
+    return loss, saved
+
+
+def mlp_train_backward(plan, B, grad_loss, saved, grad_w, grad_bias, grad_x):
+    """snb_mlp_train_backward; grad_w: one tensor or None per layer."""
+    scratch = torch.empty(_lib.load().snb_mlp_backward_scratch_bytes(plan.table, plan.depth, B), device=saved.device,
+                          dtype=torch.uint8)
+    ptrs = (ctypes.c_void_p * plan.depth)(*[_ptr(g) for g in grad_w])
+    _mlp_call("snb_mlp_train_backward", saved, plan.table, plan.depth, B, grad_loss.data_ptr(), saved.data_ptr(),
+              scratch.data_ptr(), ptrs, _ptr(grad_bias), _ptr(grad_x))
+
+
+def mlp_eval_forward(plan, x, box=None, targets=None, two_eps=1.0, scale=1.0):
+    """snb_mlp_eval_forward.  box: None, (xl, xu) tensors [B, in], or (eps, down, up) numbers.  Returns
+    (y, yl, yu, score, margin); the last four None without a box, the last two None without targets."""
+    B, K, dev = x.size(0), plan.weights[-1].size(0), x.device
+    tensors = 1 if box is None else 3
+    scratch = torch.empty(_lib.load().snb_mlp_scratch_bytes(plan.table, plan.depth, B, tensors, 0), device=dev, dtype=torch.uint8)
+    y = torch.empty(B, K, device=dev, dtype=torch.float32)
+    yl = yu = score = margin = None
+    if tensors == 3:
+        yl, yu = torch.empty_like(y), torch.empty_like(y)
+        if targets is not None:
+            score, margin = torch.empty_like(y), torch.empty_like(y)
+    ends = box if tensors == 3 and len(box) == 2 else (None, None)
+    numbers = tuple(float(v) for v in box) if tensors == 3 and len(box) == 3 else (0.0, 0.0, 0.0)
+    inverse = float("inf") if two_eps == 0 else 1.0 / two_eps
+    _mlp_call("snb_mlp_eval_forward", x, plan.table, plan.depth, x.data_ptr(), _ptr(ends[0]), _ptr(ends[1]), B, tensors, *numbers,
+              scratch.data_ptr(), y.data_ptr(), _ptr(yl), _ptr(yu), None if score is None else targets.data_ptr(), inverse,
+              float(scale), _ptr(score), _ptr(margin))
+    return y, yl, yu, score, margin
+
+
 def install():
     """Registers this module under the name the reference's operator layer imports."""
     sys.modules["norm_dist_cuda"] = sys.modules[__name__]

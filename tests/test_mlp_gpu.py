@@ -1,0 +1,100 @@
+"""Whole-net calls (csrc/mlp.cu) against the same net taken layer by layer: the forward is the same arithmetic in the
+same order (bit-identical), gradients are fp32 sums in another order (1e-5 of the largest entry, as elsewhere)."""
+import pytest
+import torch
+
+from gpu_util import rel
+
+pytestmark = pytest.mark.gpu
+
+
+def nets(depth, width, dims, classes, keep, **kw):
+    from sortnet_b200.layers import SortMLPModel
+    torch.manual_seed(1)
+    a = SortMLPModel(depth=depth, width=width, input_dim=dims, num_classes=classes, dropout=keep, **kw).cuda()
+    b = SortMLPModel(depth=depth, width=width, input_dim=dims, num_classes=classes, dropout=keep, **kw).cuda()
+    b.load_state_dict(a.state_dict())
+    return a, b
+
+
+def layer_by_layer(fn):
+    from sortnet_b200 import layers
+    layers.FUSED_LAYERS = False
+    try:
+        return fn()
+    finally:
+        layers.FUSED_LAYERS = True
+
+
+# ragged rows and widths, one and several sub-batches, more than 16 of them, odd class counts
+CASES = [(70, 4, 700, (3, 17, 17), 10, 0.8), (33, 5, 1280, (1, 28, 28), 200, 0.9), (300, 4, 515, (3, 15, 15), 7, 1.0),
+         (545, 4, 385, (1, 20, 20), 10, 0.7), (32, 4, 1024, (3, 32, 32), 10, 0.5)]
+
+
+@pytest.mark.parametrize("B,depth,width,dims,classes,keep", CASES)
+@pytest.mark.parametrize("flat", [False, True])
+def test_training_pass(B, depth, width, dims, classes, keep, flat):
+    """flat: activations hardly differ from the weights' spread, so that outputs are left to the dense kernel."""
+    a, b = nets(depth, width, dims, classes, keep, std=0.02 if flat else 1.0)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.rand(B, *dims, device="cuda", generator=g)
+    t = torch.randint(0, classes, (B,), device="cuda", generator=g)
+    from sortnet_b200 import norm_dist_cuda as C
+    plan = a._plan(None)
+    assert plan.applies(B)
+    out = []
+    for net, run in ((a, lambda f: f()), (b, layer_by_layer)):
+        net.train()
+        xi = x.clone().requires_grad_()
+        torch.manual_seed(7)
+        loss = run(lambda: net.mixture_loss(xi, t, 0.05))
+        run(lambda: (2 * loss).backward())
+        out.append([loss.detach(), xi.grad] + [p.grad for p in net.parameters()])
+        out[-1] += [l.mean_shift.running_mean for l in net.fc_dist[:-1]]
+    n = len(list(a.parameters()))
+    assert abs(float(out[0][0]) - float(out[1][0])) <= 2e-6 * max(1.0, abs(float(out[1][0])))
+    for u, v in zip(out[0][1:2 + n], out[1][1:2 + n]):
+        assert rel(u.cpu().numpy(), v.cpu().numpy()) < 1e-5
+    for u, v in zip(out[0][2 + n:], out[1][2 + n:]):
+        assert torch.equal(u, v)
+
+
+def test_training_pass_with_sinks_and_frozen_layers():
+    from sortnet_b200.optim import FlatAdamW
+    a, b = nets(4, 700, (3, 17, 17), 10, 0.8)
+    for net in (a, b):
+        net.fc_dist[0].weight.requires_grad_(False)
+        net.fc_dist[2].weight.requires_grad_(False)
+    x = torch.rand(70, 3, 17, 17, device="cuda")
+    t = torch.randint(0, 10, (70,), device="cuda")
+    opt = FlatAdamW(a)
+    for k in range(2):                      # the second backward of a step adds
+        torch.manual_seed(k)
+        a.mixture_loss(x, t, 0.05).backward()
+        torch.manual_seed(k)
+        layer_by_layer(lambda: b.mixture_loss(x, t, 0.05).backward())
+    opt.gather_grads()
+    for p, q in zip(a.parameters(), b.parameters()):
+        if p.requires_grad:
+            assert rel(p.grad_sink.cpu().numpy(), q.grad.cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("B,depth,width,dims,classes,keep", CASES)
+@pytest.mark.parametrize("flat", [False, True])
+def test_evaluation_pass(B, depth, width, dims, classes, keep, flat):
+    a, _ = nets(depth, width, dims, classes, keep, std=0.02 if flat else 1.0)
+    x = torch.rand(B, *dims, device="cuda")
+    t = torch.randint(0, classes, (B,), device="cuda")
+    from sortnet_b200.layers import update_running_means
+    update_running_means(a, [x])
+    a.eval()
+    assert a._plan(None).applies(B)
+    pixels = x.view(B, -1).size(1)
+    box = (torch.rand(pixels, device="cuda") * 0.1 + 0.9, torch.rand(pixels, device="cuda") * 0.1)
+    with torch.no_grad():
+        for run in (lambda: a(x), lambda: a(x, t, 0.02), lambda: a(x, t, 0.02, up=1.0, down=0.0),
+                    lambda: a(x, t, 0.02, up=box[0], down=box[1]), lambda: a.certified_margin(x, t, 0.02, 1.0, 0.0),
+                    lambda: a.certified_margin(x, t, 0.02, 1.0, 0.0, sort_eval=False)):
+            got, want = run(), layer_by_layer(run)
+            for u, v in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
+                assert torch.equal(u, v)
