@@ -124,6 +124,14 @@ int snb_inf_dist_forward_noalloc(const float* x, const float* w, int B, int CO, 
                                  int HW, float* y, int* pos, void* stream);
 int snb_inf_dist_forward_noalloc_max_outputs(void);
 
+/* Patches of x [B, C, H, W] -> out [B, C kh kw, oh ow] (zero padding), its transpose (the sum of g's patches onto the
+ * image), and the lists of the (channel, position) plane: index [S, G, kept] of within-group channels ->
+ * out [S, G kept hw] with entries channel * hw + position.  Replace torch.nn.functional.unfold and the index arithmetic
+ * around MeanShiftDropout (core/models/norm_dist.py:130-164, bound_basic_module.py:123-157). */
+int snb_unfold(const float* x, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil, float* out, void* stream);
+int snb_fold(const float* g, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil, float* gx, void* stream);
+int snb_plane_index(const int* index, int S, int G, int kept, int channels, int hw, int* out, void* stream);
+
 /* ---- a whole SortNet-MLP per call (G == 1, HW == 1) --------------------------------------------
  * Layer k of the net: w [out, in], optional bias [out] (added after the mean shift), optional running_mean [out]
  * (training: updated in place with `momentum`; evaluation: subtracted), the kept channels of its output as ascending

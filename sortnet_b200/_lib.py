@@ -55,6 +55,9 @@ SIGNATURES = {
     "snb_input_box": [_P, _F, _F, _F, ctypes.c_longlong, _P, _P, _P],
     "snb_margin_loss": [_P, _P, _I, _I, _F, _F, _F, _F, _P, _P, _P, _P, _P],
     "snb_certified_fraction": [_P, _P, _P, _I, _I, _P, _P, _P],
+    "snb_unfold": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "snb_fold": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "snb_plane_index": [_P, _I, _I, _I, _I, _I, _P, _P],
     # the three *_bytes return size_t
     "snb_mlp_applies": [_P, _I, _I],
     "snb_mlp_saved_bytes": [_P, _I, _I],
@@ -115,6 +118,23 @@ def load(build_if_missing: bool = False):
     lib.snb_norm_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     _lib = lib
     return lib
+
+
+_ops = None
+
+
+def ops():
+    """The native operator layer (_ops.so, csrc/ops_ext.cpp), bound to the library; raises if it is not built."""
+    global _ops
+    if _ops is None:
+        load()
+        try:
+            from . import _ops as module
+        except ImportError as exc:
+            raise SortnetB200Error("_ops.so is not built (run `python -m sortnet_b200.build`): %s" % exc) from exc
+        module.init(LIB_PATH)
+        _ops = module
+    return _ops
 
 
 def check(status: int, what: str):

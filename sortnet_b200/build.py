@@ -1,4 +1,5 @@
-"""Builds libsortnet_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libsortnet_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and _ops.so, the PyTorch
+module of csrc/ops_ext.cpp, with the host compiler.
 
     python -m sortnet_b200.build [--force]
 
@@ -16,6 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libsortnet_b200.so")
+OPS = os.path.join(HERE, "_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -44,8 +46,32 @@ def _compile(src, obj, verbose):
     return r.stderr
 
 
+def build_ops(force: bool = False) -> str:
+    """The native operator layer: one C++ file against PyTorch's headers, no CUDA code."""
+    src = os.path.join(CSRC, "ops_ext.cpp")
+    newest = max(os.path.getmtime(src), _newest_header())
+    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest:
+        return OPS
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_ops", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for inc in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
+        cmd += ["-isystem", inc]
+    lib = os.path.join(base, "lib")
+    cmd += [src, "-o", OPS, "-L" + lib, "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for %s:\n%s" % (src, r.stderr))
+    return OPS
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
+    ops_job = concurrent.futures.ThreadPoolExecutor(max_workers=1).submit(build_ops, force)
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     hdr = _newest_header()
     jobs, objs = [], []
@@ -62,6 +88,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if jobs or not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(o) for o in objs):
         cmd = [_nvcc(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB] + objs
         subprocess.check_call(cmd)
+    ops_job.result()
     return LIB
 
 

@@ -143,6 +143,7 @@ int make_geo(int B, int CO, int CI, int G, int HW, int W_CO, Geo* q) {
     return SNB_OK;
 }
 
+size_t most(size_t a, size_t b) { return a > b ? a : b; }
 size_t words(const Geo& q, int C, int K = 1) { return sizeof(uint32_t) * (size_t)q.G * K * q.Bp * C; }
 
 cudaError_t pack(const void* src, void* dst, const Geo& q, int C, int K, uint32_t fill, cudaStream_t st) {
@@ -185,6 +186,7 @@ int general_inf_forward(const float* x, const float* w, int B, int CO, int CI, i
     size_t op = pos ? a.reserve(words(q, COg)) : 0;
     size_t oci = ci ? a.reserve(mask_bytes(q, CIg)) : 0, oco = co ? a.reserve(mask_bytes(q, COg)) : 0;
     size_t ws_bytes = pos ? snb_inf_dist_forward_workspace_bytes(q.Bp, COg) : 0;
+    ws_bytes = most(ws_bytes, snb_prune_scratch_bytes(1, 1, pos != nullptr, q.Bp, COg, CIg, W_COg, W_CIg, ci != nullptr));
     size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xp = a.at<float>(ox), *yp = a.at<float>(oy);
@@ -198,8 +200,8 @@ int general_inf_forward(const float* x, const float* w, int B, int CO, int CI, i
         int rc = pos ? snb_inf_dist_forward_ws(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1, grp(yp, q, g, COg),
                                                grp(pp, q, g, COg), mgrp(cip, q, g, CIg), mgrp(cop, q, g, COg),
                                                W_COg, W_CIg, a.at<void>(ows), ws_bytes, st)
-                     : snb_inf_dist_forward_nograd(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1,
-                                                   grp(yp, q, g, COg), st);
+                     : snb_inf_dist_forward_nograd_ws(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1, grp(yp, q, g, COg),
+                                                      a.at<void>(ows), ws_bytes, st);
         if (rc) return rc;
     }
     SNB_CUDA(unpack(yp, y, q, COg, 1, st));
@@ -311,6 +313,8 @@ int general_bound_forward(const float* xl, const float* xu, const float* w, int 
     size_t oxl = a.reserve(words(q, CIg)), oxu = a.reserve(words(q, CIg));
     size_t oyl = a.reserve(words(q, COg)), oyu = a.reserve(words(q, COg));
     size_t opl = posl ? a.reserve(words(q, COg)) : 0, opu = posl ? a.reserve(words(q, COg)) : 0;
+    const size_t ws_bytes = snb_prune_scratch_bytes(2, 1, posl != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xlp = a.at<float>(oxl), *xup = a.at<float>(oxu), *ylp = a.at<float>(oyl), *yup = a.at<float>(oyu);
     int *plp = posl ? a.at<int>(opl) : nullptr, *pup = posl ? a.at<int>(opu) : nullptr;
@@ -318,11 +322,12 @@ int general_bound_forward(const float* xl, const float* xu, const float* w, int 
     SNB_CUDA(pack(xu, xup, q, CIg, 1, 0u, st));
     for (int g = 0; g < G; g++) {
         const float* wg = w + (size_t)g * COg * CIg;
-        int rc = posl ? snb_bound_inf_dist_forward(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1,
-                                                   grp(ylp, q, g, COg), grp(yup, q, g, COg), grp(plp, q, g, COg),
-                                                   grp(pup, q, g, COg), st)
-                      : snb_bound_inf_dist_forward_nograd(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), wg, q.Bp, COg,
-                                                          CIg, 1, 1, grp(ylp, q, g, COg), grp(yup, q, g, COg), st);
+        int rc = posl ? snb_bound_inf_dist_forward_ws(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1,
+                                                      grp(ylp, q, g, COg), grp(yup, q, g, COg), grp(plp, q, g, COg),
+                                                      grp(pup, q, g, COg), a.at<void>(ows), ws_bytes, st)
+                      : snb_bound_inf_dist_forward_nograd_ws(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1,
+                                                             grp(ylp, q, g, COg), grp(yup, q, g, COg), a.at<void>(ows), ws_bytes,
+                                                             st);
         if (rc) return rc;
     }
     SNB_CUDA(unpack(ylp, yl, q, COg, 1, st));
@@ -376,16 +381,18 @@ int general_sort_forward(const float* x, const float* w, int B, int CO, int CI, 
     Arena a(st);
     size_t ox = a.reserve(words(q, CIg)), oy = a.reserve(words(q, COg));
     size_t op = pos ? a.reserve(words(q, COg, K)) : 0;
+    const size_t ws_bytes = snb_prune_scratch_bytes(1, K, pos != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xp = a.at<float>(ox), *yp = a.at<float>(oy);
     int* pp = pos ? a.at<int>(op) : nullptr;
     SNB_CUDA(pack(x, xp, q, CIg, 1, 0u, st));
     for (int g = 0; g < G; g++) {
         const float* wg = w + (size_t)g * COg * CIg;
-        int rc = pos ? snb_sort_neuron_forward(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1, grp(yp, q, g, COg),
-                                               grp(pp, q, g, COg, K), qq, K, st)
-                     : snb_sort_neuron_forward_nograd(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1,
-                                                      grp(yp, q, g, COg), qq, K, st);
+        int rc = pos ? snb_sort_neuron_forward_ws(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1, grp(yp, q, g, COg),
+                                                  grp(pp, q, g, COg, K), qq, K, a.at<void>(ows), ws_bytes, st)
+                     : snb_sort_neuron_forward_nograd_ws(grp(xp, q, g, CIg), wg, q.Bp, COg, CIg, 1, 1, grp(yp, q, g, COg), qq, K,
+                                                         a.at<void>(ows), ws_bytes, st);
         if (rc) return rc;
     }
     SNB_CUDA(unpack(yp, y, q, COg, 1, st));
@@ -402,14 +409,16 @@ int general_sort_bound_forward(const float* xl, const float* xu, const float* w,
     Arena a(st);
     size_t oxl = a.reserve(words(q, CIg)), oxu = a.reserve(words(q, CIg));
     size_t oyl = a.reserve(words(q, COg)), oyu = a.reserve(words(q, COg));
+    const size_t ws_bytes = snb_prune_scratch_bytes(2, K, 0, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xlp = a.at<float>(oxl), *xup = a.at<float>(oxu), *ylp = a.at<float>(oyl), *yup = a.at<float>(oyu);
     SNB_CUDA(pack(xl, xlp, q, CIg, 1, 0u, st));
     SNB_CUDA(pack(xu, xup, q, CIg, 1, 0u, st));
     for (int g = 0; g < G; g++) {
-        int rc = snb_bound_sort_neuron_forward(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), w + (size_t)g * COg * CIg,
-                                               q.Bp, COg, CIg, 1, 1, grp(ylp, q, g, COg), grp(yup, q, g, COg), qq, K,
-                                               st);
+        int rc = snb_bound_sort_neuron_forward_ws(grp(xlp, q, g, CIg), grp(xup, q, g, CIg), w + (size_t)g * COg * CIg,
+                                                  q.Bp, COg, CIg, 1, 1, grp(ylp, q, g, COg), grp(yup, q, g, COg), qq, K,
+                                                  a.at<void>(ows), ws_bytes, st);
         if (rc) return rc;
     }
     SNB_CUDA(unpack(ylp, yl, q, COg, 1, st));

@@ -1,0 +1,376 @@
+// Native form of the operator layer (ops.py): argument checks, output allocation, the library call and the autograd node of
+// norm_dist, norm_dist_dropout, sort_neuron and bound_inf_dist in C++.  The Python classes of ops.py do the same
+// steps at about four times the host time (a small layer's forward, backward and bounds: 310 us per pass against
+// kernels of 30 us); they stay for what needs Python: gradient sinks, the profile, index-list validation.
+//
+// The library is reached through function pointers (init), so this module links against PyTorch only.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <cmath>
+
+#include "../../include/sortnet_b200.h"
+
+namespace {
+
+using at::Tensor;
+using c10::optional;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+struct Api {
+    decltype(&snb_inf_dist_forward_ws) inf_forward;
+    decltype(&snb_inf_dist_forward_sorted_ws) inf_forward_sorted;
+    decltype(&snb_inf_dist_forward_sorted_workspace_bytes) inf_sorted_bytes;
+    decltype(&snb_inf_dist_forward_nograd_ws) inf_forward_nograd;
+    decltype(&snb_inf_dist_backward_input) inf_backward_x;
+    decltype(&snb_inf_dist_backward_input_weight) inf_backward_xw;
+    decltype(&snb_norm_dist_forward_ws) lp_forward;
+    decltype(&snb_norm_dist_backward_input) lp_backward_x;
+    decltype(&snb_norm_dist_backward_input_weight) lp_backward_xw;
+    decltype(&snb_bound_inf_dist_forward_nograd_ws) bound_forward_nograd;
+    decltype(&snb_bound_inf_dist_forward_ws) bound_forward;
+    decltype(&snb_bound_inf_dist_backward_input) bound_backward_x;
+    decltype(&snb_bound_inf_dist_backward_input_weight) bound_backward_xw;
+    decltype(&snb_sort_neuron_forward_nograd_ws) sort_forward_nograd;
+    decltype(&snb_sort_neuron_forward_ws) sort_forward;
+    decltype(&snb_sort_neuron_backward_input) sort_backward_x;
+    decltype(&snb_sort_neuron_backward_input_weight) sort_backward_xw;
+    decltype(&snb_bound_sort_neuron_forward_ws) bound_sort_forward;
+    decltype(&snb_prune_scratch_bytes) scratch_bytes;
+    decltype(&snb_status_string) status_string;
+    decltype(&snb_last_cuda_error) last_cuda_error;
+} api;
+std::atomic<long> launches{0};
+
+void init(const std::string& path) {
+    void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+    TORCH_CHECK(h, "cannot load ", path, ": ", dlerror());
+    auto get = [&](auto& f, const char* name) {
+        f = reinterpret_cast<std::decay_t<decltype(f)>>(dlsym(h, name));
+        TORCH_CHECK(f, path, " has no ", name);
+    };
+    get(api.inf_forward, "snb_inf_dist_forward_ws");
+    get(api.inf_forward_sorted, "snb_inf_dist_forward_sorted_ws");
+    get(api.inf_sorted_bytes, "snb_inf_dist_forward_sorted_workspace_bytes");
+    get(api.inf_forward_nograd, "snb_inf_dist_forward_nograd_ws");
+    get(api.inf_backward_x, "snb_inf_dist_backward_input");
+    get(api.inf_backward_xw, "snb_inf_dist_backward_input_weight");
+    get(api.lp_forward, "snb_norm_dist_forward_ws");
+    get(api.lp_backward_x, "snb_norm_dist_backward_input");
+    get(api.lp_backward_xw, "snb_norm_dist_backward_input_weight");
+    get(api.bound_forward_nograd, "snb_bound_inf_dist_forward_nograd_ws");
+    get(api.bound_forward, "snb_bound_inf_dist_forward_ws");
+    get(api.bound_backward_x, "snb_bound_inf_dist_backward_input");
+    get(api.bound_backward_xw, "snb_bound_inf_dist_backward_input_weight");
+    get(api.sort_forward_nograd, "snb_sort_neuron_forward_nograd_ws");
+    get(api.sort_forward, "snb_sort_neuron_forward_ws");
+    get(api.sort_backward_x, "snb_sort_neuron_backward_input");
+    get(api.sort_backward_xw, "snb_sort_neuron_backward_input_weight");
+    get(api.bound_sort_forward, "snb_bound_sort_neuron_forward_ws");
+    get(api.scratch_bytes, "snb_prune_scratch_bytes");
+    get(api.status_string, "snb_status_string");
+    get(api.last_cuda_error, "snb_last_cuda_error");
+}
+
+void check(const Tensor& t, const char* name, at::ScalarType type = at::kFloat) {
+    TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
+    TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
+    TORCH_CHECK(t.scalar_type() == type, name, " must have dtype ", type, ", got ", t.scalar_type());
+}
+void check_input(const Tensor& x, const Tensor& w, const char* name = "input") {
+    check(x, name);
+    check(w, "weight");
+    TORCH_CHECK(x.dim() == 3 && w.dim() == 2, name, " must have shape [B, C, HW] and weight [CO, CI / groups]");
+    TORCH_CHECK(x.device() == w.device(), "all tensors must be on the same device");
+}
+void check_list(const optional<Tensor>& t, const char* name, int64_t B, int64_t G, int64_t width, const Tensor& x) {
+    if (!t.has_value()) return;
+    check(*t, name, at::kInt);
+    TORCH_CHECK(t->dim() == 3 && t->size(0) == (B + 31) / 32 && t->size(1) == G && t->size(2) * G == width, name,
+                " must have shape [", (B + 31) / 32, ", ", G, ", ", width / std::max<int64_t>(G, 1), "], got ", t->sizes());
+    TORCH_CHECK(t->device() == x.device(), "all tensors must be on the same device");
+}
+const int* list_ptr(const optional<Tensor>& t) { return t.has_value() ? t->data_ptr<int>() : nullptr; }
+
+void done(int rc, const char* what, int kernels) {
+    if (rc) {
+        TORCH_CHECK(rc != SNB_STATUS_CUDA, what, " failed: ", api.status_string(rc), ": ", api.last_cuda_error(), " (status ", rc, ")");
+        TORCH_CHECK(false, what, " failed: ", api.status_string(rc), " (status ", rc, ")");
+    }
+    launches.fetch_add(kernels, std::memory_order_relaxed);
+}
+
+// Scratch of a forward call from PyTorch's caching allocator (stream-ordered).
+struct Area {
+    Tensor t;
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    Area(const Tensor& like, int tensors, int K, int words, int64_t B, int64_t CO, int64_t CI, int64_t W_CO, int64_t W_CI, bool lists,
+         bool flat, size_t at_least = 0) {
+        bytes = flat ? api.scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, lists) : 0;
+        bytes = std::max(bytes, at_least);
+        if (bytes) {
+            t = at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
+            ptr = t.data_ptr();
+        }
+    }
+};
+
+struct Call {
+    c10::cuda::OptionalCUDAGuard guard;
+    cudaStream_t stream;
+    explicit Call(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
+};
+
+// ---- distance --------------------------------------------------------------------------------------
+struct DistOut {
+    Tensor y, pos;
+};
+DistOut dist_forward(const Tensor& x, const Tensor& w, const optional<Tensor>& ci, const optional<Tensor>& co, int64_t G, double p,
+                     bool record, bool ascending) {
+    check_input(x, w);
+    const int64_t B = x.size(0), CI = x.size(1), HW = x.size(2);
+    const int64_t CO = co.has_value() ? co->size(-1) * G : w.size(0);
+    check_list(ci, "w_index_ci", B, G, CI, x);
+    check_list(co, "w_index_co", B, G, CO, x);
+    Call call(x);
+    DistOut out;
+    out.y = at::empty({B, CO, HW}, x.options());
+    const bool flat = G == 1 && HW == 1;
+    const int64_t W_CO = w.size(0), W_CI = w.size(1);
+    if (std::isinf(p)) {
+        if (!record) {
+            Area ws(x, 1, 1, 0, B, CO, CI, CO, CI, false, flat);
+            done(api.inf_forward_nograd(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), ws.ptr,
+                                        ws.bytes, call.stream), "inf_dist_forward_nograd", 1);
+            return out;
+        }
+        out.pos = at::empty({B, CO, HW}, x.options().dtype(at::kInt));
+        const bool sorted = ascending && flat && (ci.has_value() || co.has_value());
+        Area ws(x, 1, 1, 1, B, CO, CI, W_CO, W_CI, ci.has_value(), flat,
+                !flat ? 0 : sorted ? api.inf_sorted_bytes(B, CO, W_CI) : sizeof(int64_t) * (size_t)(B * CO));
+        auto f = sorted ? api.inf_forward_sorted : api.inf_forward;
+        done(f(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), out.pos.data_ptr<int>(),
+               list_ptr(ci), list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "inf_dist_forward", 2);
+        return out;
+    }
+    Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false, p > 10 ? sizeof(float) * (size_t)(B * CO * HW) : 0);
+    done(api.lp_forward(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), (float)p, list_ptr(ci),
+                        list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "norm_dist_forward", p > 10 ? 3 : 2);
+    return out;
+}
+
+struct DistFn : public torch::autograd::Function<DistFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const optional<Tensor>& ci, const optional<Tensor>& co,
+                          int64_t G, double p, bool ascending) {
+        DistOut out = dist_forward(x, w, ci, co, G, p, true, ascending);
+        ctx->saved_data["p"] = p;
+        ctx->saved_data["G"] = G;
+        if (ci.has_value()) ctx->saved_data["ci"] = *ci;
+        if (co.has_value()) ctx->saved_data["co"] = *co;
+        ctx->save_for_backward({x, w, std::isinf(p) ? out.pos : out.y});
+        return out.y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0], &w = saved[1], &third = saved[2];
+        const double p = ctx->saved_data["p"].toDouble();
+        const int64_t G = ctx->saved_data["G"].toInt();
+        optional<Tensor> ci, co;
+        if (ctx->saved_data.count("ci")) ci = ctx->saved_data["ci"].toTensor();
+        if (ctx->saved_data.count("co")) co = ctx->saved_data["co"].toTensor();
+        const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+        variable_list out(7);
+        if (!need_x && !need_w) return out;
+        Call call(x);
+        const Tensor g = grads[0].contiguous();
+        check(g, "grad_output");
+        const int64_t B = g.size(0), CO = g.size(1), HW = g.size(2), CI = x.size(1);
+        Tensor gx = at::empty_like(x), gw = need_w ? at::empty_like(w) : Tensor();
+        const float* gp = g.data_ptr<float>();
+        if (std::isinf(p)) {
+            if (need_w)
+                done(api.inf_backward_xw(gp, third.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), gw.data_ptr<float>(),
+                                         list_ptr(ci), list_ptr(co), w.size(0), w.size(1) * G, call.stream),
+                     "inf_dist_backward_input_weight", 1);
+            else
+                done(api.inf_backward_x(gp, third.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), call.stream),
+                     "inf_dist_backward_input", 1);
+        } else if (need_w) {
+            done(api.lp_backward_xw(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
+                                    gx.data_ptr<float>(), gw.data_ptr<float>(), (float)p, list_ptr(ci), list_ptr(co), w.size(0),
+                                    w.size(1) * G, call.stream), "norm_dist_backward_input_weight", 1);
+        } else {
+            done(api.lp_backward_x(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
+                                   gx.data_ptr<float>(), (float)p, list_ptr(ci), list_ptr(co), w.size(0), w.size(1) * G, call.stream),
+                 "norm_dist_backward_input", 1);
+        }
+        if (need_x) out[0] = gx;
+        out[1] = gw;
+        return out;
+    }
+};
+
+// record: some operand wants a gradient (always true for the masked operator, as in the Python form)
+Tensor dist(const Tensor& x, const Tensor& w, const optional<Tensor>& ci, const optional<Tensor>& co, int64_t G, double p, bool record,
+            bool ascending) {
+    if (!std::isinf(p)) TORCH_CHECK(p > 0, "p must be positive");
+    const bool graph = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
+    if (!graph) return dist_forward(x, w, ci, co, G, p, record, ascending).y;
+    return DistFn::apply(x, w, ci, co, G, p, ascending);
+}
+
+// ---- sort neuron -----------------------------------------------------------------------------------
+Tensor sort_forward(const Tensor& x, const Tensor& w, int64_t G, double q, int64_t K, Tensor* pos) {
+    check_input(x, w);
+    const int64_t B = x.size(0), CI = x.size(1), HW = x.size(2), CO = w.size(0);
+    TORCH_CHECK(w.size(1) * G == CI, "shape mismatch");
+    Call call(x);
+    Tensor y = at::empty({B, CO, HW}, x.options());
+    Area ws(x, 1, K, pos != nullptr, B, CO, CI, CO, CI, false, G == 1 && HW == 1);
+    if (pos) {
+        *pos = at::empty({K, B, CO, HW}, x.options().dtype(at::kInt));
+        done(api.sort_forward(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, y.data_ptr<float>(), pos->data_ptr<int>(),
+                              (float)q, K, ws.ptr, ws.bytes, call.stream), "sort_neuron_forward", 1);
+    } else {
+        done(api.sort_forward_nograd(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, y.data_ptr<float>(), (float)q, K,
+                                     ws.ptr, ws.bytes, call.stream), "sort_neuron_forward_nograd", 1);
+    }
+    return y;
+}
+
+struct SortFn : public torch::autograd::Function<SortFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, int64_t G, double q, int64_t K) {
+        Tensor pos, y = sort_forward(x, w, G, q, K, &pos);
+        ctx->saved_data["G"] = G;
+        ctx->saved_data["q"] = q;
+        ctx->saved_data["K"] = K;
+        ctx->save_for_backward({x, w, pos});
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0], &w = saved[1], &pos = saved[2];
+        const int64_t G = ctx->saved_data["G"].toInt(), K = ctx->saved_data["K"].toInt();
+        const float q = (float)ctx->saved_data["q"].toDouble();
+        const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+        variable_list out(5);
+        if (!need_x && !need_w) return out;
+        Call call(x);
+        const Tensor g = grads[0].contiguous();
+        check(g, "grad_output");
+        const int64_t B = g.size(0), CO = g.size(1), HW = g.size(2), CI = x.size(1);
+        Tensor gx = at::empty_like(x), gw = need_w ? at::empty_like(w) : Tensor();
+        if (need_w)
+            done(api.sort_backward_xw(g.data_ptr<float>(), pos.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(),
+                                      gw.data_ptr<float>(), q, K, call.stream), "sort_neuron_backward_input_weight", 1);
+        else
+            done(api.sort_backward_x(g.data_ptr<float>(), pos.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), q, K,
+                                     call.stream), "sort_neuron_backward_input", 1);
+        if (need_x) out[0] = gx;
+        out[1] = gw;
+        return out;
+    }
+};
+
+Tensor sort_neuron(const Tensor& x, const Tensor& w, int64_t G, double q, int64_t K) {
+    if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad())) return SortFn::apply(x, w, G, q, K);
+    return sort_forward(x, w, G, q, K, nullptr);
+}
+
+// ---- interval bounds -------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor> bound_forward(const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G, Tensor* words) {
+    check_input(xl, w, "inputL");
+    check_input(xu, w, "inputU");
+    const int64_t B = xl.size(0), CI = xl.size(1), HW = xl.size(2), CO = w.size(0);
+    TORCH_CHECK(xl.sizes() == xu.sizes() && w.size(1) * G == CI, "shape mismatch");
+    Call call(xl);
+    Tensor yl = at::empty({B, CO, HW}, xl.options()), yu = at::empty({B, CO, HW}, xl.options());
+    Area ws(xl, 2, 1, words != nullptr, B, CO, CI, CO, CI, false, G == 1 && HW == 1);
+    if (words) {
+        *words = at::empty({2, B, CO, HW}, xl.options().dtype(at::kInt));
+        int* lw = words->data_ptr<int>();
+        done(api.bound_forward(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, yl.data_ptr<float>(),
+                               yu.data_ptr<float>(), lw, lw + B * CO * HW, ws.ptr, ws.bytes, call.stream), "bound_inf_dist_forward", 1);
+    } else {
+        done(api.bound_forward_nograd(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW,
+                                      yl.data_ptr<float>(), yu.data_ptr<float>(), ws.ptr, ws.bytes, call.stream),
+             "bound_inf_dist_forward_nograd", 1);
+    }
+    return {yl, yu};
+}
+
+struct BoundFn : public torch::autograd::Function<BoundFn> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G) {
+        Tensor words;
+        auto [yl, yu] = bound_forward(xl, xu, w, G, &words);
+        ctx->saved_data["G"] = G;
+        ctx->save_for_backward({xl, xu, w, words});
+        return {yl, yu};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &xl = saved[0], &w = saved[2], &words = saved[3];
+        const int64_t G = ctx->saved_data["G"].toInt();
+        const bool need_l = ctx->needs_input_grad(0), need_u = ctx->needs_input_grad(1), need_w = ctx->needs_input_grad(2);
+        variable_list out(4);
+        Call call(xl);
+        const int64_t B = words.size(1), CO = words.size(2), HW = words.size(3), CI = xl.size(1);
+        Tensor g[2];
+        for (int k = 0; k < 2; k++) {
+            g[k] = grads[k].defined() ? grads[k].contiguous() : at::zeros({B, CO, HW}, xl.options());
+            check(g[k], "grad_output");
+        }
+        const bool run = need_w || (need_l && need_u);      // one end of the box alone gets zeros, as in the Python form
+        Tensor gl = run ? at::empty_like(xl) : at::zeros_like(xl), gu = run ? at::empty_like(xl) : at::zeros_like(xl);
+        Tensor gw = need_w ? at::empty_like(w) : Tensor();
+        const int* lw = words.data_ptr<int>();
+        const float *pl = g[0].data_ptr<float>(), *pu = g[1].data_ptr<float>();
+        if (need_w)
+            done(api.bound_backward_xw(pl, pu, lw, lw + B * CO * HW, B, CO, CI, G, HW, gl.data_ptr<float>(), gu.data_ptr<float>(),
+                                       gw.data_ptr<float>(), call.stream), "bound_inf_dist_backward_input_weight", 1);
+        else if (run)
+            done(api.bound_backward_x(pl, pu, lw, lw + B * CO * HW, B, CO, CI, G, HW, gl.data_ptr<float>(), gu.data_ptr<float>(),
+                                      call.stream), "bound_inf_dist_backward_input", 1);
+        if (need_l) out[0] = gl;
+        if (need_u) out[1] = gu;
+        out[2] = gw;
+        return out;
+    }
+};
+
+std::tuple<Tensor, Tensor> bound_inf_dist(const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G) {
+    if (at::GradMode::is_enabled() && (xl.requires_grad() || xu.requires_grad() || w.requires_grad())) {
+        auto y = BoundFn::apply(xl, xu, w, G);
+        return {y[0], y[1]};
+    }
+    return bound_forward(xl, xu, w, G, nullptr);
+}
+
+std::tuple<Tensor, Tensor> bound_sort_neuron(const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G, double q, int64_t K) {
+    check_input(xl, w, "inputL");
+    check_input(xu, w, "inputU");
+    const int64_t B = xl.size(0), CI = xl.size(1), HW = xl.size(2), CO = w.size(0);
+    TORCH_CHECK(xl.sizes() == xu.sizes() && w.size(1) * G == CI, "shape mismatch");
+    Call call(xl);
+    Tensor yl = at::empty({B, CO, HW}, xl.options()), yu = at::empty({B, CO, HW}, xl.options());
+    Area ws(xl, 2, K, 0, B, CO, CI, CO, CI, false, G == 1 && HW == 1);
+    done(api.bound_sort_forward(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, yl.data_ptr<float>(),
+                                yu.data_ptr<float>(), (float)q, K, ws.ptr, ws.bytes, call.stream), "bound_sort_neuron_forward", 1);
+    return {yl, yu};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("init", &init);
+    m.def("dist", &dist);
+    m.def("sort_neuron", &sort_neuron);
+    m.def("bound_inf_dist", &bound_inf_dist);
+    m.def("bound_sort_neuron", &bound_sort_neuron);
+    m.def("launches", [] { return launches.load(); });
+}

@@ -77,10 +77,30 @@ def _plane_index(index, channels, hw):
     [S, 1, n] int32 form the mean-shift kernels take; None stays None."""
     if index is None:
         return None
+    if index.is_cuda and index.dtype == torch.int32:
+        return _C.plane_index(index.contiguous(), channels, hw)
     glob = _global_index(index, channels)
     if hw > 1:
         glob = (glob.unsqueeze(-1) * hw + torch.arange(hw, device=glob.device)).reshape(glob.size(0), -1)
     return glob.int().unsqueeze(1).contiguous()
+
+
+def _per_position(mean, hw):
+    """mean [C] -> [C * hw], every entry hw times."""
+    return mean if hw == 1 else mean.unsqueeze(1).expand(-1, hw).reshape(-1)
+
+
+class _UnfoldF(torch.autograd.Function):
+    """Patches of an image batch in one launch per direction."""
+
+    @staticmethod
+    def forward(ctx, x, kernel, stride, padding, dilation):
+        ctx.args = (x.shape, kernel, stride, padding, dilation)
+        return _C.unfold(x.contiguous(), kernel, stride, padding, dilation)
+
+    @staticmethod
+    def backward(ctx, grad):
+        return (_C.fold(grad.contiguous(), *ctx.args), None, None, None, None)
 
 
 class _MeanShiftPlaneF(torch.autograd.Function):
@@ -98,7 +118,7 @@ class _MeanShiftPlaneF(torch.autograd.Function):
         _C.mean_shift_stats(flat, plane_index, per_pos, None, 0.0)
         mean = per_pos.view(channels, hw).mean(dim=1)
         y = torch.empty_like(flat)
-        _C.mean_shift_apply(flat, mean.repeat_interleave(hw), plane_index, y)
+        _C.mean_shift_apply(flat, _per_position(mean, hw), plane_index, y)
         ctx.plane_index, ctx.channels = plane_index, channels
         ctx.mark_non_differentiable(mean)
         return y.view(x.shape), mean
@@ -111,7 +131,7 @@ class _MeanShiftPlaneF(torch.autograd.Function):
         _C.mean_shift_stats(flat, ctx.plane_index, per_pos, None, 0.0)
         gmean = per_pos.view(ctx.channels, hw).mean(dim=1)
         grad_x = torch.empty_like(flat)
-        _C.mean_shift_apply(flat, gmean.repeat_interleave(hw), ctx.plane_index, grad_x)
+        _C.mean_shift_apply(flat, _per_position(gmean, hw), ctx.plane_index, grad_x)
         return grad_x.view(grad_y.shape), None, None
 
 
@@ -178,8 +198,8 @@ class MeanShiftDropout(nn.Module):
         else:
             mean = self.running_mean if self.bias is None else self.running_mean - self.bias.detach()
             x_done, todo = None, (x, lower, upper)
-        if plane and hw > 1:
-            mean = mean.repeat_interleave(hw)
+        if plane:
+            mean = _per_position(mean, hw)
         outs = []
         for z in todo:
             if z is None:
@@ -337,6 +357,8 @@ class NormDistConv(nn.Module):
             return None
         if self.kernel_size == (1, 1) and self.stride == 1 and self.padding == 0:
             return z.reshape(z.size(0), z.size(1), -1).contiguous()
+        if z.is_cuda and z.dtype == torch.float32 and all(isinstance(v, int) for v in (self.dilation, self.padding, self.stride)):
+            return _UnfoldF.apply(z, self.kernel_size, self.stride, self.padding, self.dilation)
         return F.unfold(z, self.kernel_size, self.dilation, self.padding, self.stride).contiguous()
 
     def forward(self, x=None, lower=None, upper=None, mask_in=None, mask_out=None, sort_eval=False):
@@ -408,14 +430,15 @@ class SortMLPModel(nn.Module):
         # are drawn from the host generator (a few thousand uniforms) instead of on the device, which
         # would cost a device synchronisation per step and stop the host from queueing kernels
         # ahead of the GPU.
-        counts = [int((torch.rand(l.in_features) < l.keep_rate).sum()) for _, l in todo]
+        # One draw for all layers: the generator gives the same numbers as one draw per layer.
+        uniform = torch.rand(sum(l.in_features for _, l in todo)).split([l.in_features for _, l in todo])
+        counts = [int((u < l.keep_rate).sum()) for u, (_, l) in zip(uniform, todo)]
         device = torch.device(device)
         if device.type == "cuda" and 1 < len(todo) <= 16:
             # all layers' lists in one launch; counts, seeds and lists are those of the per-layer calls
-            outs, seeds = [], []
+            outs, seeds = [], torch.randint(0, 2 ** 62, (len(todo),)).tolist()
             for (k, l), c in zip(todo, counts):
                 c = min(max(int(c), 1), l.in_features)
-                seeds.append(int(torch.randint(0, 2 ** 62, (1,))))
                 outs.append(torch.empty(sub, 1, c, dtype=torch.int32, device=device))
                 masks[k] = outs[-1]
             _C.sample_masks_into(outs, [l.in_features for _, l in todo], seeds)

@@ -17,6 +17,7 @@ unmodified `core/norm_dist.py` (`import norm_dist_cuda as _C`) runs on these ker
 import ctypes
 import os
 import sys
+import types
 
 import torch
 
@@ -84,18 +85,37 @@ _KERNELS = {
     "snb_inf_dist_backward_input_weight": 1, "snb_norm_dist_forward": 1, "snb_norm_dist_forward_ws": 2, "snb_norm_dist_backward_input": 1,
     "snb_norm_dist_backward_input_weight": 1, "snb_bound_inf_dist_forward_nograd_ws": 1,
     "snb_bound_inf_dist_forward_ws": 1, "snb_bound_inf_dist_backward_input": 1,
-    "snb_bound_inf_dist_backward_input_weight": 1, "snb_mean_shift_stats": 1, "snb_mean_shift_apply": 1, "snb_sample_mask": 1, "snb_sample_mask_batch": 1,
+    "snb_bound_inf_dist_backward_input_weight": 1, "snb_unfold": 1, "snb_fold": 1, "snb_plane_index": 1, "snb_mean_shift_stats": 1, "snb_mean_shift_apply": 1, "snb_sample_mask": 1, "snb_sample_mask_batch": 1,
     "snb_sort_neuron_forward_nograd_ws": 1, "snb_sort_neuron_forward_ws": 1, "snb_bound_sort_neuron_forward_ws": 1,
     "snb_sort_neuron_backward_input": 1, "snb_sort_neuron_backward_input_weight": 1,
 }
 
-launch_count = 0          # kernels launched through this module since import / reset_counters()
+_launched = 0             # kernels launched from Python since import / reset_counters()
+_native_base = 0          # the native operator layer's count at the last reset
 _timeline = None          # when profiling: list of (entry point, work tag, start event, end event)
 
 
+class _Module(types.ModuleType):
+    """`launch_count`: kernels launched since import / reset_counters(), by this module and by the native
+    operator layer; assignable (callers that launch through the library themselves add to it)."""
+
+    @property
+    def launch_count(self):
+        return _launched + (_lib._ops.launches() - _native_base if _lib._ops is not None else 0)
+
+    @launch_count.setter
+    def launch_count(self, value):
+        global _launched
+        _launched += value - self.launch_count
+
+
+sys.modules[__name__].__class__ = _Module
+
+
 def reset_counters():
-    global launch_count
-    launch_count = 0
+    global _launched, _native_base
+    _launched = 0
+    _native_base = _lib._ops.launches() if _lib._ops is not None else 0
 
 
 def start_profile():
@@ -115,24 +135,32 @@ def stop_profile():
     return out
 
 
+def _stream(dev):
+    """Handle of the current stream of `dev`."""
+    return torch._C._cuda_getCurrentRawStream(dev.index)
+
+
 def _call(dev, ref_tensor, entry, tag, *args):
     """Runs C entry point `entry` with `dev` current, on the current stream of that device."""
-    global launch_count
-    lib = _lib.load()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev)
-        if _timeline is not None:
-            e0 = torch.cuda.Event(enable_timing=True)
-            e1 = torch.cuda.Event(enable_timing=True)
-            e0.record(stream)
-        rc = getattr(lib, entry)(*args, stream.cuda_stream)
-        if _timeline is not None:
-            e1.record(stream)
-            _timeline.append((entry, tag, e0, e1))
+    global _launched
+    fn = getattr(_lib.load(), entry)
+    if _timeline is None and torch.cuda.current_device() == dev.index:
+        rc = fn(*args, _stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            stream = torch.cuda.current_stream(dev)
+            if _timeline is not None:
+                e0 = torch.cuda.Event(enable_timing=True)
+                e1 = torch.cuda.Event(enable_timing=True)
+                e0.record(stream)
+            rc = fn(*args, stream.cuda_stream)
+            if _timeline is not None:
+                e1.record(stream)
+                _timeline.append((entry, tag, e0, e1))
     _lib.check(rc, entry[4:])
-    launch_count += _KERNELS[entry]
+    _launched += _KERNELS[entry]
     if entry in ("snb_norm_dist_forward", "snb_norm_dist_forward_ws") and args[8] > 10.0:
-        launch_count += 1      # the l-inf pass that supplies the normaliser
+        _launched += 1      # the l-inf pass that supplies the normaliser
 
 
 def _same_device(*ts):
@@ -481,6 +509,34 @@ def sample_masks_into(outs, channels, seeds):
           n, ptrs, chans, counts, seed_arr, lists)
 
 
+def unfold(x, kernel, stride, padding, dilation):
+    """torch.nn.functional.unfold for x [B, C, H, W] in one launch -> [B, C kh kw, oh ow]."""
+    _check(x, "x")
+    B, C, H, W = x.shape
+    oh, ow = ((n + 2 * padding - dilation * (k - 1) - 1) // stride + 1 for n, k in zip((H, W), kernel))
+    out = torch.empty(B, C * kernel[0] * kernel[1], max(oh, 0) * max(ow, 0), device=x.device, dtype=torch.float32)
+    _call(x.device, x, "snb_unfold", (B, C), x.data_ptr(), B, C, H, W, kernel[0], kernel[1], stride, padding, dilation, out.data_ptr())
+    return out
+
+
+def fold(g, shape, kernel, stride, padding, dilation):
+    """The transpose of unfold: g [B, C kh kw, oh ow] -> `shape` [B, C, H, W]."""
+    _check(g, "g")
+    B, C, H, W = shape
+    out = torch.empty(shape, device=g.device, dtype=torch.float32)
+    _call(g.device, g, "snb_fold", (B, C), g.data_ptr(), B, C, H, W, kernel[0], kernel[1], stride, padding, dilation, out.data_ptr())
+    return out
+
+
+def plane_index(index, channels, hw):
+    """Lists of the (channel, position) plane: index [S, G, kept] -> [S, 1, G kept hw] int32."""
+    _check(index, "index", torch.int32)
+    S, G, kept = index.shape
+    out = torch.empty(S, 1, G * kept * hw, device=index.device, dtype=torch.int32)
+    _call(index.device, index, "snb_plane_index", (S, G), index.data_ptr(), S, G, kept, channels, hw, out.data_ptr())
+    return out
+
+
 # ---- whole layers and the model head (one C call each; G = 1, HW = 1, 2-D tensors) ---------------
 
 _LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward": 4, "snb_layer_bound_forward_ws": 3, "snb_input_box": 1,
@@ -491,19 +547,19 @@ def _layer_call(entry, tag, ref, *args):
     """Lean variant of _call for the layer-level entry points: the callers in ops.py / layers.py own
     every tensor they pass (fresh allocations of the right shape and dtype), so only the device is
     looked after here."""
-    global launch_count
+    global _launched
     if _timeline is not None:
         return _call(ref.device, ref, entry, tag, *args)
     dev = ref.device
     fn = getattr(_lib.load(), entry)
     if torch.cuda.current_device() == dev.index:
-        rc = fn(*args, torch.cuda.current_stream(dev).cuda_stream)
+        rc = fn(*args, _stream(dev))
     else:
         with torch.cuda.device(dev):
-            rc = fn(*args, torch.cuda.current_stream(dev).cuda_stream)
+            rc = fn(*args, _stream(dev))
     if rc:
         _lib.check(rc, entry[4:])
-    launch_count += _LAYER_KERNELS[entry]
+    _launched += _LAYER_KERNELS[entry]
 
 
 _KERNELS.update(_LAYER_KERNELS)
@@ -596,16 +652,16 @@ class MlpPlan:
 
 def _mlp_call(entry, ref, *args):
     """Runs a snb_mlp_* entry point with the device of `ref` current; counts what it launched."""
-    global launch_count
+    global _launched
     dev, fn, n = ref.device, getattr(_lib.load(), entry), ctypes.c_int(0)
     if torch.cuda.current_device() == dev.index:
-        rc = fn(*args, ctypes.byref(n), torch.cuda.current_stream(dev).cuda_stream)
+        rc = fn(*args, ctypes.byref(n), _stream(dev))
     else:
         with torch.cuda.device(dev):
-            rc = fn(*args, ctypes.byref(n), torch.cuda.current_stream(dev).cuda_stream)
+            rc = fn(*args, ctypes.byref(n), _stream(dev))
     if rc:
         _lib.check(rc, entry[4:])
-    launch_count += n.value
+    _launched += n.value
 
 
 def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):

@@ -1,0 +1,105 @@
+"""The native operator layer (csrc/ops_ext.cpp) against the Python classes of ops.py: same kernels, so values and
+words agree bit for bit and gradients to the order of their atomics."""
+import pytest
+import torch
+
+from gpu_util import rel
+
+pytestmark = pytest.mark.gpu
+INF = float("inf")
+
+
+def both(fn):
+    """(native, Python) results of fn()."""
+    from sortnet_b200 import ops
+    native = fn()
+    keep, ops._native = ops._native, lambda w: False
+    try:
+        return native, fn()
+    finally:
+        ops._native = keep
+
+
+def operands(B, CI, CO, HW=1, groups=1, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.rand(B, CI, HW, device="cuda", generator=g, requires_grad=True)
+    w = torch.randn(CO, CI // groups, device="cuda", generator=g, requires_grad=True)
+    return x, w, torch.randn(B, CO, HW, device="cuda", generator=g)
+
+
+def compare(a, b):
+    """1e-5 as for all gradients here: a finite p sums its outputs in run-dependent order (a few 2^-24), and the
+    backward raises ratios of them to the power p - 1 (30 at most)."""
+    assert len(a) == len(b)
+    for u, v in zip(a, b):
+        assert (u is None) == (v is None)
+        if u is not None:
+            assert u.shape == v.shape and rel(u.detach().cpu().numpy(), v.detach().cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("p", [INF, 1.0, 8.0, 31.6])
+@pytest.mark.parametrize("shape", [(9, 97, 33, 1, 1), (40, 12, 18, 4, 3), (70, 1024, 400, 1, 1)])
+@pytest.mark.parametrize("needs", ["xw", "x", "w", ""])
+def test_distance(p, shape, needs):
+    from sortnet_b200 import ops
+    B, CI, CO, HW, G = shape
+    x, w, gy = operands(B, CI, CO, HW, G)
+    x.requires_grad_("x" in needs), w.requires_grad_("w" in needs)
+
+    def run():
+        y = ops.norm_dist(x, w, p, G)
+        wanted = [t for t in (x, w) if t.requires_grad]
+        return [y] + (list(torch.autograd.grad(y, wanted, gy)) if wanted else [])
+    compare(*both(run))
+
+
+@pytest.mark.parametrize("p", [INF, 3.0])
+@pytest.mark.parametrize("ascending", [False, True])
+def test_masked_distance(p, ascending):
+    from sortnet_b200 import ops
+    from sortnet_b200.layers import sample_mask
+    x, w, _ = operands(70, 300, 200)
+    ci, co = sample_mask(3, 1, 300, 0.8, "cuda"), sample_mask(3, 1, 200, 0.9, "cuda")
+    x = x.detach()[:, :ci.size(2)].contiguous().requires_grad_()
+    gy = torch.randn(70, co.size(2), 1, device="cuda")
+    op = ops.norm_dist_dropout_ascending if ascending else ops.norm_dist_dropout
+
+    def run():
+        y = op(x, w, ci, co, p)
+        return [y, *torch.autograd.grad(y, (x, w), gy)]
+    compare(*both(run))
+
+
+@pytest.mark.parametrize("shape", [(40, 30, 20, 1, 1), (33, 12, 18, 4, 3)])
+def test_sort_neuron_and_bounds(shape):
+    from sortnet_b200 import ops
+    B, CI, CO, HW, G = shape
+    x, w, gy = operands(B, CI, CO, HW, G)
+    lo, hi = (x.detach() - 0.1).requires_grad_(), (x.detach() + 0.1).requires_grad_()
+
+    def run():
+        y = ops.sort_neuron(x, w, G, q=0.8, truncate=4)
+        yl, yu = ops.bound_inf_dist(lo, hi, w, G)
+        out = [y, yl, yu, *torch.autograd.grad(y, (x, w), gy)]
+        out += torch.autograd.grad((yl, yu), (lo, hi, w), (gy, 2 * gy), retain_graph=True)
+        out += torch.autograd.grad(yu, (lo, hi), gy)            # only one of the two outputs is used
+        with torch.no_grad():
+            return out + [*ops.bound_sort_neuron(lo, hi, w, G, q=0.8, truncate=4), ops.sort_neuron(x, w, G, q=0.8)]
+    compare(*both(run))
+
+
+def test_errors_and_counter():
+    from sortnet_b200 import norm_dist_cuda as C, ops
+    x, w, _ = operands(8, 16, 5)
+    C.reset_counters()
+    y = ops.norm_dist(x, w, INF)
+    y.sum().backward()
+    assert C.launch_count >= 2
+    with pytest.raises(RuntimeError):
+        ops.norm_dist(x.detach().cpu(), w, INF)
+    with pytest.raises(RuntimeError):
+        ops.norm_dist(x.double(), w, INF)
+    with pytest.raises(RuntimeError):
+        ops.norm_dist(x.transpose(0, 1).transpose(0, 1)[::2], w, INF)   # not contiguous
+    with pytest.raises(AssertionError):
+        ops.norm_dist(x, w[:, :8], INF)
