@@ -527,7 +527,7 @@ def lp_blocks(job, peak_gflops, sm_mhz):
             roof = {"bound": "xu (special-function unit)", "peak": round(xu_peak, 1), "unit": "G transcendental/s",
                     "peak_source": "16 per clock per SM x %d SMs x %s MHz (median SM clock of this run)" % (sms, sm_mhz),
                     "ops_per_element": 2.0, "p": 31.6}
-            for entry, key in (("snb_norm_dist_forward_ws", "forward"), ("snb_norm_dist_backward_input_weight", "backward")):
+            for entry, key in (("snb_norm_dist_forward_ws", "forward"), ("snb_norm_dist_backward_ws", "backward")):
                 ks = kernel_stats(tl, entry)
                 if ks is None:
                     continue

@@ -234,6 +234,17 @@ int snb_norm_dist_backward_input_weight(const float* grad_output, const float* x
                                         const int* w_index_ci, const int* w_index_co, int W_CO,
                                         int W_CI, void* stream);
 
+/* Both backward forms with caller-provided scratch (grad_weight may be NULL), and the scratch with which the l-p entry
+ * points evaluate only the terms that can matter (p > 10 and large enough problems, G == 1 and HW == 1): terms below
+ * 2^-40 of the largest of their sum are left out, which fp32 sums cannot show.  snb_norm_dist_scratch_bytes: bytes for
+ * snb_norm_dist_forward_ws (backward = 0; never less than snb_norm_dist_forward_workspace_bytes) or snb_norm_dist_backward_ws
+ * (backward = 1; 0: the call needs none); column_lists = 1 when w_index_ci is given.  16-byte aligned, any content on
+ * entry.  With less workspace, or NULL, the dense kernels run.  No counterpart in the reference. */
+size_t snb_norm_dist_scratch_bytes(int backward, int B, int CO, int CI, int W_CO, int W_CI, float p, int column_lists);
+int snb_norm_dist_backward_ws(const float* grad_output, const float* x, const float* w, const float* y, int B, int CO, int CI,
+                              int G, int HW, float* grad_input, float* grad_weight, float p, const int* w_index_ci,
+                              const int* w_index_co, int W_CO, int W_CI, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- interval bounds through an l-infinity layer ------------------------------------------- */
 
 /* yL = -min(-1e-10, min_c min(w - xL, xU - w)), yU = max(1e-10, max_c max(w - xL, xU - w)); an
@@ -364,6 +375,11 @@ int snb_layer_backward(const float* grad_out, const float* x, const float* w, co
                        int B, int CO, int CI, float p, const int* w_index_ci, const int* w_index_co, int W_CO,
                        int W_CI, int mean_shift, float* mean, float* grad_centred, float* grad_bias, float* grad_x,
                        float* grad_w, void* stream);
+/* The same with scratch for the distance backward of a finite p (snb_norm_dist_scratch_bytes(1, ...); may be NULL). */
+int snb_layer_backward_ws(const float* grad_out, const float* x, const float* w, const float* y_dist, const int* pos,
+                          int B, int CO, int CI, float p, const int* w_index_ci, const int* w_index_co, int W_CO,
+                          int W_CI, int mean_shift, float* mean, float* grad_centred, float* grad_bias, float* grad_x,
+                          float* grad_w, void* workspace, size_t workspace_bytes, void* stream);
 
 /* One layer of the evaluation-mode l-inf interval-bound pass: y = l-inf distance of the point value x
  * (x may be NULL), (yl, yu) = interval bounds of the box (xl, xu) (may be NULL), then running_mean

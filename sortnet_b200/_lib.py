@@ -25,6 +25,8 @@ SIGNATURES = {
     "snb_norm_dist_forward_ws": [_P, _P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, ctypes.c_size_t, _P],
     "snb_norm_dist_backward_input": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P],
     "snb_norm_dist_backward_input_weight": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _P, _P, _I, _I, _P],
+    "snb_norm_dist_backward_ws": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _P, _P, _I, _I, _P, ctypes.c_size_t, _P],
+    "snb_norm_dist_scratch_bytes": [_I, _I, _I, _I, _I, _I, _F, _I],     # returns size_t
     "snb_bound_inf_dist_forward_nograd": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P],
     "snb_bound_inf_dist_forward": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
     "snb_bound_inf_dist_backward_input": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P],
@@ -51,6 +53,7 @@ SIGNATURES = {
     "snb_dp_adamw_step": [_P, _P, _P, _P, _I, _I, ctypes.c_longlong, ctypes.c_longlong, _F, _F, _F, _F, _F, _I, _P],
     "snb_layer_forward": [_P, _P, _I, _I, _I, _F, _P, _P, _I, _I, _P, _P, _P, ctypes.c_size_t, _P, _F, _P, _P, _P, _P],
     "snb_layer_backward": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P],
+    "snb_layer_backward_ws": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P],
     "snb_layer_bound_forward": [_P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P],
     "snb_input_box": [_P, _F, _F, _F, ctypes.c_longlong, _P, _P, _P],
     "snb_margin_loss": [_P, _P, _I, _I, _F, _F, _F, _F, _P, _P, _P, _P, _P],
@@ -112,7 +115,7 @@ def load(build_if_missing: bool = False):
     lib.snb_inf_dist_forward_workspace_bytes.restype = ctypes.c_size_t
     lib.snb_inf_dist_forward_sorted_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
     lib.snb_inf_dist_forward_sorted_workspace_bytes.restype = ctypes.c_size_t
-    for name in ("snb_prune_scratch_bytes", "snb_mlp_saved_bytes", "snb_mlp_scratch_bytes", "snb_mlp_backward_scratch_bytes"):
+    for name in ("snb_prune_scratch_bytes", "snb_norm_dist_scratch_bytes", "snb_mlp_saved_bytes", "snb_mlp_scratch_bytes", "snb_mlp_backward_scratch_bytes"):
         getattr(lib, name).restype = ctypes.c_size_t
     lib.snb_norm_dist_forward_workspace_bytes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_float]
     lib.snb_norm_dist_forward_workspace_bytes.restype = ctypes.c_size_t

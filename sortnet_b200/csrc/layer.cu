@@ -270,11 +270,11 @@ extern "C" int snb_layer_forward(const float* x, const float* w, int B, int CO, 
     return SNB_OK;
 }
 
-extern "C" int snb_layer_backward(const float* grad_out, const float* x, const float* w, const float* y_dist,
-                                  const int* pos, int B, int CO, int CI, float p, const int* w_index_ci,
-                                  const int* w_index_co, int W_CO, int W_CI, int mean_shift, float* mean,
-                                  float* grad_centred, float* grad_bias, float* grad_x, float* grad_w,
-                                  void* stream) {
+extern "C" int snb_layer_backward_ws(const float* grad_out, const float* x, const float* w, const float* y_dist,
+                                     const int* pos, int B, int CO, int CI, float p, const int* w_index_ci,
+                                     const int* w_index_co, int W_CO, int W_CI, int mean_shift, float* mean,
+                                     float* grad_centred, float* grad_bias, float* grad_x, float* grad_w, void* workspace,
+                                     size_t workspace_bytes, void* stream) {
     if (!grad_out) return SNB_ERR_NULL_POINTER;
     int rc = check2d(B, CO, CI);
     if (rc) return rc;
@@ -300,10 +300,16 @@ extern "C" int snb_layer_backward(const float* grad_out, const float* x, const f
                                                            w_index_co, W_CO, W_CI, stream)
                       : snb_inf_dist_backward_input(g, pos, B, CO, CI, 1, 1, grad_x, stream);
     }
-    return grad_w ? snb_norm_dist_backward_input_weight(g, x, w, y_dist, B, CO, CI, 1, 1, grad_x, grad_w, p,
-                                                        w_index_ci, w_index_co, W_CO, W_CI, stream)
-                  : snb_norm_dist_backward_input(g, x, w, y_dist, B, CO, CI, 1, 1, grad_x, p, w_index_ci, w_index_co,
-                                                 W_CO, W_CI, stream);
+    return snb_norm_dist_backward_ws(g, x, w, y_dist, B, CO, CI, 1, 1, grad_x, grad_w, p, w_index_ci, w_index_co, W_CO, W_CI,
+                                     workspace, workspace_bytes, stream);
+}
+
+extern "C" int snb_layer_backward(const float* grad_out, const float* x, const float* w, const float* y_dist, const int* pos,
+                                  int B, int CO, int CI, float p, const int* w_index_ci, const int* w_index_co, int W_CO,
+                                  int W_CI, int mean_shift, float* mean, float* grad_centred, float* grad_bias, float* grad_x,
+                                  float* grad_w, void* stream) {
+    return snb_layer_backward_ws(grad_out, x, w, y_dist, pos, B, CO, CI, p, w_index_ci, w_index_co, W_CO, W_CI, mean_shift, mean,
+                                 grad_centred, grad_bias, grad_x, grad_w, nullptr, 0, stream);
 }
 
 // workspace: snb_prune_scratch_bytes(1, 2 or 3 tensors, 1, 0, ...) bytes or null

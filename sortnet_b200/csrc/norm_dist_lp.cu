@@ -17,6 +17,8 @@
 // amplification of the logarithm's error at the level of the fp32 rounding of r itself.
 #include <float.h>
 #include "tile.cuh"
+#include "lp_math.cuh"
+#include "lp_skip.h"
 #include "launch.h"
 #include "general_shapes.h"
 
@@ -25,45 +27,6 @@ namespace snb {
 // defined in inf_dist.cu: y = max(1e-10, max_c |x - w|) with optional index lists, no argmax
 cudaError_t inf_forward_values(const float* x, const float* w, float* y, const int* ci, const int* co,
                                int B, int CO, int CI, int W_CI, cudaStream_t st);
-
-// Special-function-unit exp2 / log2.  The .ftz forms skip the denormal fix-up code: a denormal
-// argument of log2 reads as 0 (its power is 0 to fp32 anyway) and results below 2^-126 flush to 0.
-__device__ __forceinline__ float ex2_approx(float z) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
-    return r;
-}
-__device__ __forceinline__ float lg2_approx(float a) {
-    float r;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-    return r;
-}
-
-// log2(a) by a degree-8 series in d = a - 1 (exact subtraction), for |d| <= 0.125.  The hardware
-// approximation has an absolute error of 2^-22, i.e. no relative accuracy near a = 1; the series
-// keeps the relative error of log2 at fp32 level there, so that a^e for large e is as accurate as
-// the fp32 rounding of a allows.
-__device__ __forceinline__ float log2_series(float a) {
-    const float d = a - 1.0f;
-    float s = fmaf(d, -0.125f, 1.0f / 7.0f);
-    s = fmaf(d, s, -1.0f / 6.0f);
-    s = fmaf(d, s, 0.2f);
-    s = fmaf(d, s, -0.25f);
-    s = fmaf(d, s, 1.0f / 3.0f);
-    s = fmaf(d, s, -0.5f);
-    s = fmaf(d, s, 1.0f);
-    return d * 1.4426950408889634f * s;
-}
-__device__ __forceinline__ bool near_one(float a) { return fabsf(a - 1.0f) <= 0.125f; }
-
-// a^e for a >= 0, accurate per value (used once per output and in the backward).
-__device__ __forceinline__ float pow_pos(float a, float e) {
-    return ex2_approx(e * (near_one(a) ? log2_series(a) : lg2_approx(a)));
-}
-// a^e where only the *sum* of many such terms matters (forward): the absolute error of the
-// hardware log2 perturbs the sum by ~1.7e-7 * e relative, and the e-th root taken afterwards
-// divides that by e.
-__device__ __forceinline__ float pow_pos_sum(float a, float e) { return ex2_approx(e * lg2_approx(a)); }
 
 // |r|^IP for integer IP (multiply chain) or |r|^e for IP < 0; forward terms.
 template <int IP>
@@ -578,7 +541,7 @@ using namespace snb;
 
 static int lp_forward_impl(const float* x, const float* w, int B, int CO, int CI, int G, int HW, float* y,
                            float p, const int* w_index_ci, const int* w_index_co, int W_CO, int W_CI,
-                           float* scratch, cudaStream_t st) {
+                           void* ws, size_t ws_bytes, cudaStream_t st) {
     if (!(p > 0) || isinf(p)) return SNB_ERR_UNSUPPORTED;
     if (G != 1 || HW != 1)
         return general_lp_forward(x, w, B, CO, CI, G, HW, y, p, w_index_ci, w_index_co, W_CO, W_CI, st);
@@ -590,6 +553,13 @@ static int lp_forward_impl(const float* x, const float* w, int B, int CO, int CI
         return SNB_ERR_TOO_LARGE;
     LpFwdParams q{x, w, y, nullptr, w_index_ci, w_index_co, B, CO, CI, W_CI, p, 0};
     if (p > 10.0f) {
+        const LpProblem sparse{x, w, w_index_ci, w_index_co, B, CO, CI, W_CO, W_CI, p};
+        const size_t need = lp_skip_forward_bytes(sparse);
+        if (ws && need && ws_bytes >= need) {
+            SNB_CUDA(lp_skip_forward(sparse, y, ws, st));
+            return SNB_OK;
+        }
+        float* scratch = ws && ws_bytes >= sizeof(float) * (size_t)B * CO ? static_cast<float*>(ws) : nullptr;
         // the maxima go to the scratch array when there is one (y is then free to collect partial
         // sums from CTAs that share a tile), else into y itself
         float* maxima = scratch ? scratch : y;
@@ -616,7 +586,7 @@ extern "C" int snb_norm_dist_forward(const float* x, const float* w, int B, int 
                                      int HW, float* y, float p, const int* w_index_ci,
                                      const int* w_index_co, int W_CO, int W_CI, void* stream) {
     return lp_forward_impl(x, w, B, CO, CI, G, HW, y, p, w_index_ci, w_index_co, W_CO, W_CI, nullptr,
-                           (cudaStream_t)stream);
+                           0, (cudaStream_t)stream);
 }
 
 extern "C" size_t snb_norm_dist_forward_workspace_bytes(int B, int CO, float p) {
@@ -627,18 +597,24 @@ extern "C" int snb_norm_dist_forward_ws(const float* x, const float* w, int B, i
                                         int HW, float* y, float p, const int* w_index_ci,
                                         const int* w_index_co, int W_CO, int W_CI, void* workspace,
                                         size_t workspace_bytes, void* stream) {
-    float* scratch = nullptr;
-    if (workspace && p > 10.0f) {
-        if (reinterpret_cast<uintptr_t>(workspace) & 15u) return SNB_ERR_ALIGNMENT;
-        if (workspace_bytes >= snb_norm_dist_forward_workspace_bytes(B, CO, p)) scratch = (float*)workspace;
-    }
-    return lp_forward_impl(x, w, B, CO, CI, G, HW, y, p, w_index_ci, w_index_co, W_CO, W_CI, scratch,
+    if (workspace && p > 10.0f && !aligned16(workspace)) return SNB_ERR_ALIGNMENT;
+    return lp_forward_impl(x, w, B, CO, CI, G, HW, y, p, w_index_ci, w_index_co, W_CO, W_CI, workspace, workspace_bytes,
                            (cudaStream_t)stream);
+}
+
+extern "C" size_t snb_norm_dist_scratch_bytes(int backward, int B, int CO, int CI, int W_CO, int W_CI, float p, int column_lists) {
+    if (B <= 0 || CO <= 0 || CI <= 0 || W_CO <= 0 || W_CI <= 0 || !(p > 0) || isinf(p)) return 0;
+    static const int none = 0;
+    static const float some = 0.f;
+    const LpProblem sparse{&some, &some, column_lists ? &none : nullptr, nullptr, B, CO, CI, W_CO, W_CI, p};
+    if (backward) return lp_skip_backward_bytes(sparse);
+    const size_t need = lp_skip_forward_bytes(sparse), least = snb_norm_dist_forward_workspace_bytes(B, CO, p);
+    return need > least ? need : least;
 }
 
 static int lp_backward(const float* g, const float* x, const float* w, const float* y, int B, int CO,
                        int CI, int G, int HW, float* gx, float* gw, float p, const int* ci,
-                       const int* co, int W_CO, int W_CI, cudaStream_t st) {
+                       const int* co, int W_CO, int W_CI, void* ws, size_t ws_bytes, cudaStream_t st) {
     if (!(p > 0) || isinf(p)) return SNB_ERR_UNSUPPORTED;
     if (G != 1 || HW != 1)
         return general_lp_backward(g, x, w, y, B, CO, CI, G, HW, gx, gw, p, ci, co, W_CO, W_CI, st);
@@ -648,6 +624,12 @@ static int lp_backward(const float* g, const float* x, const float* w, const flo
     if ((long long)W_CO * W_CI >= (1ll << 31) || (long long)B * CO >= (1ll << 31) || (long long)B * CI >= (1ll << 31))
         return SNB_ERR_TOO_LARGE;
     if (gw) SNB_CUDA(cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)W_CO * W_CI, st));
+    const LpProblem sparse{x, w, ci, co, B, CO, CI, W_CO, W_CI, p};
+    const size_t need = lp_skip_backward_bytes(sparse);
+    if (ws && need && ws_bytes >= need) {
+        SNB_CUDA(lp_skip_backward(sparse, g, y, gx, gw, ws, st));
+        return SNB_OK;
+    }
     LpBwdParams q{g, x, w, y, gx, gw, ci, co, B, CO, CI, W_CI, p - 1.0f};
     switch (integer_power(p - 1.0f)) {
         case 0: SNB_CUDA(launch_lp_bwd<0>(q, st)); break;
@@ -672,7 +654,7 @@ extern "C" int snb_norm_dist_backward_input(const float* grad_output, const floa
                                             float* grad_input, float p, const int* w_index_ci,
                                             const int* w_index_co, int W_CO, int W_CI, void* stream) {
     return lp_backward(grad_output, x, w, y, B, CO, CI, G, HW, grad_input, nullptr, p, w_index_ci,
-                       w_index_co, W_CO, W_CI, (cudaStream_t)stream);
+                       w_index_co, W_CO, W_CI, nullptr, 0, (cudaStream_t)stream);
 }
 
 extern "C" int snb_norm_dist_backward_input_weight(const float* grad_output, const float* x,
@@ -683,5 +665,14 @@ extern "C" int snb_norm_dist_backward_input_weight(const float* grad_output, con
                                                    void* stream) {
     if (!grad_weight) return SNB_ERR_NULL_POINTER;
     return lp_backward(grad_output, x, w, y, B, CO, CI, G, HW, grad_input, grad_weight, p, w_index_ci,
-                       w_index_co, W_CO, W_CI, (cudaStream_t)stream);
+                       w_index_co, W_CO, W_CI, nullptr, 0, (cudaStream_t)stream);
+}
+
+extern "C" int snb_norm_dist_backward_ws(const float* grad_output, const float* x, const float* w, const float* y, int B, int CO,
+                                         int CI, int G, int HW, float* grad_input, float* grad_weight, float p,
+                                         const int* w_index_ci, const int* w_index_co, int W_CO, int W_CI, void* workspace,
+                                         size_t workspace_bytes, void* stream) {
+    if (workspace && !aligned16(workspace)) return SNB_ERR_ALIGNMENT;
+    return lp_backward(grad_output, x, w, y, B, CO, CI, G, HW, grad_input, grad_weight, p, w_index_ci, w_index_co, W_CO, W_CI,
+                       workspace, workspace_bytes, (cudaStream_t)stream);
 }

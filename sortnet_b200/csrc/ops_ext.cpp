@@ -29,8 +29,8 @@ struct Api {
     decltype(&snb_inf_dist_backward_input) inf_backward_x;
     decltype(&snb_inf_dist_backward_input_weight) inf_backward_xw;
     decltype(&snb_norm_dist_forward_ws) lp_forward;
-    decltype(&snb_norm_dist_backward_input) lp_backward_x;
-    decltype(&snb_norm_dist_backward_input_weight) lp_backward_xw;
+    decltype(&snb_norm_dist_backward_ws) lp_backward;
+    decltype(&snb_norm_dist_scratch_bytes) lp_bytes;
     decltype(&snb_bound_inf_dist_forward_nograd_ws) bound_forward_nograd;
     decltype(&snb_bound_inf_dist_forward_ws) bound_forward;
     decltype(&snb_bound_inf_dist_backward_input) bound_backward_x;
@@ -60,8 +60,8 @@ void init(const std::string& path) {
     get(api.inf_backward_x, "snb_inf_dist_backward_input");
     get(api.inf_backward_xw, "snb_inf_dist_backward_input_weight");
     get(api.lp_forward, "snb_norm_dist_forward_ws");
-    get(api.lp_backward_x, "snb_norm_dist_backward_input");
-    get(api.lp_backward_xw, "snb_norm_dist_backward_input_weight");
+    get(api.lp_backward, "snb_norm_dist_backward_ws");
+    get(api.lp_bytes, "snb_norm_dist_scratch_bytes");
     get(api.bound_forward_nograd, "snb_bound_inf_dist_forward_nograd_ws");
     get(api.bound_forward, "snb_bound_inf_dist_forward_ws");
     get(api.bound_backward_x, "snb_bound_inf_dist_backward_input");
@@ -158,7 +158,7 @@ DistOut dist_forward(const Tensor& x, const Tensor& w, const optional<Tensor>& c
                list_ptr(ci), list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "inf_dist_forward", 2);
         return out;
     }
-    Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false, p > 10 ? sizeof(float) * (size_t)(B * CO * HW) : 0);
+    Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false, flat ? api.lp_bytes(0, B, CO, CI, W_CO, W_CI, (float)p, ci.has_value()) : 0);
     done(api.lp_forward(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), (float)p, list_ptr(ci),
                         list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "norm_dist_forward", p > 10 ? 3 : 2);
     return out;
@@ -200,14 +200,14 @@ struct DistFn : public torch::autograd::Function<DistFn> {
             else
                 done(api.inf_backward_x(gp, third.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), call.stream),
                      "inf_dist_backward_input", 1);
-        } else if (need_w) {
-            done(api.lp_backward_xw(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
-                                    gx.data_ptr<float>(), gw.data_ptr<float>(), (float)p, list_ptr(ci), list_ptr(co), w.size(0),
-                                    w.size(1) * G, call.stream), "norm_dist_backward_input_weight", 1);
         } else {
-            done(api.lp_backward_x(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
-                                   gx.data_ptr<float>(), (float)p, list_ptr(ci), list_ptr(co), w.size(0), w.size(1) * G, call.stream),
-                 "norm_dist_backward_input", 1);
+            const int64_t W_CO = w.size(0), W_CI = w.size(1);
+            Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false,
+                    G == 1 && HW == 1 ? api.lp_bytes(1, B, CO, CI, W_CO, W_CI, (float)p, ci.has_value()) : 0);
+            done(api.lp_backward(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
+                                 gx.data_ptr<float>(), need_w ? gw.data_ptr<float>() : nullptr, (float)p, list_ptr(ci), list_ptr(co),
+                                 W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream),
+                 need_w ? "norm_dist_backward_input_weight" : "norm_dist_backward_input", 1);
         }
         if (need_x) out[0] = gx;
         out[1] = gw;

@@ -82,8 +82,8 @@ def _dims(x, out):
 # Kernels launched by each C entry point (memsets are not counted).
 _KERNELS = {
     "snb_inf_dist_forward": 2, "snb_inf_dist_forward_ws": 2, "snb_inf_dist_forward_sorted_ws": 3, "snb_inf_dist_forward_nograd_ws": 1, "snb_inf_dist_backward_input": 1,
-    "snb_inf_dist_backward_input_weight": 1, "snb_norm_dist_forward": 1, "snb_norm_dist_forward_ws": 2, "snb_norm_dist_backward_input": 1,
-    "snb_norm_dist_backward_input_weight": 1, "snb_bound_inf_dist_forward_nograd_ws": 1,
+    "snb_inf_dist_backward_input_weight": 1, "snb_norm_dist_forward": 1, "snb_norm_dist_forward_ws": 2, "snb_norm_dist_backward_ws": 1,
+    "snb_bound_inf_dist_forward_nograd_ws": 1,
     "snb_bound_inf_dist_forward_ws": 1, "snb_bound_inf_dist_backward_input": 1,
     "snb_bound_inf_dist_backward_input_weight": 1, "snb_unfold": 1, "snb_fold": 1, "snb_plane_index": 1, "snb_mean_shift_stats": 1, "snb_mean_shift_apply": 1, "snb_sample_mask": 1, "snb_sample_mask_batch": 1,
     "snb_sort_neuron_forward_nograd_ws": 1, "snb_sort_neuron_forward_ws": 1, "snb_bound_sort_neuron_forward_ws": 1,
@@ -177,6 +177,12 @@ def _scratch(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists, dev, at_lea
     an empty tensor when neither needs any."""
     nbytes = max(_lib.load().snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists), at_least)
     return torch.empty((nbytes + 7) // 8, dtype=torch.int64, device=dev)
+
+
+def _lp_scratch(backward, B, CO, CI, W_CO, W_CI, p, ci, dev):
+    """The same for the l-p entry points (snb_norm_dist_scratch_bytes); None when they need none."""
+    nbytes = _lib.load().snb_norm_dist_scratch_bytes(backward, B, CO, CI, W_CO, W_CI, p, int(ci is not None))
+    return torch.empty((nbytes + 7) // 8, dtype=torch.int64, device=dev) if nbytes else None
 
 
 def inf_dist_forward(input, weight, output, pos, G, w_index_ci=None, w_index_co=None):
@@ -276,13 +282,10 @@ def norm_dist_forward(input, weight, output, G, p, w_index_ci=None, w_index_co=N
     _check(input, "input"); _check(weight, "weight"); _check(output, "output")
     B, CO, CI, HW = _lp_common(input, weight, output, w_index_ci, w_index_co, G)
     dev = _same_device(input, weight, output, w_index_ci, w_index_co)
-    # p > 10: scratch for the maxima (4 bytes per output) from PyTorch's caching allocator, so that
-    # the kernel may share output tiles between thread blocks
-    ws = torch.empty(B * CO * HW if p > 10 else 0, dtype=torch.float32, device=dev)
+    ws = _lp_scratch(0, B, CO, CI, weight.size(0), weight.size(1), p, w_index_ci, dev) if G == 1 and HW == 1 else None
     _call(dev, input, "snb_norm_dist_forward_ws", (B, CO, CI),
           _ptr(input), _ptr(weight), B, CO, CI, G, HW, _ptr(output), float(p), _ptr(w_index_ci),
-          _ptr(w_index_co), weight.size(0), weight.size(1) * G, ws.data_ptr() if ws.numel() else None,
-          ws.numel() * 4)
+          _ptr(w_index_co), weight.size(0), weight.size(1) * G, *_area(ws))
 
 
 def norm_dist_forward_with_max(input, weight, max_output, output, G, p, w_index_ci=None, w_index_co=None):
@@ -294,6 +297,13 @@ def norm_dist_forward_with_max(input, weight, max_output, output, G, p, w_index_
     norm_dist_forward(input, weight, output, G, p, w_index_ci, w_index_co)
 
 
+def _lp_backward(dev, grad_output, input, weight, output, grad_input, grad_weight, B, CO, CI, HW, G, p, ci, co):
+    ws = _lp_scratch(1, B, CO, CI, weight.size(0), weight.size(1), p, ci, dev) if G == 1 and HW == 1 else None
+    _call(dev, input, "snb_norm_dist_backward_ws", (B, CO, CI),
+          _ptr(grad_output), _ptr(input), _ptr(weight), _ptr(output), B, CO, CI, G, HW, _ptr(grad_input),
+          _ptr(grad_weight), float(p), _ptr(ci), _ptr(co), weight.size(0), weight.size(1) * G, *_area(ws))
+
+
 def norm_dist_backward_input(grad_output, input, weight, output, grad_input, G, p,
                              w_index_ci=None, w_index_co=None):
     """core/cuda/norm_dist.cpp:87-106."""
@@ -302,9 +312,7 @@ def norm_dist_backward_input(grad_output, input, weight, output, grad_input, G, 
         _check(t, n)
     B, CO, CI, HW = _lp_common(input, weight, output, w_index_ci, w_index_co, G)
     dev = _same_device(grad_output, input, weight, output, grad_input, w_index_ci, w_index_co)
-    _call(dev, input, "snb_norm_dist_backward_input", (B, CO, CI),
-          _ptr(grad_output), _ptr(input), _ptr(weight), _ptr(output), B, CO, CI, G, HW, _ptr(grad_input),
-          float(p), _ptr(w_index_ci), _ptr(w_index_co), weight.size(0), weight.size(1) * G)
+    _lp_backward(dev, grad_output, input, weight, output, grad_input, None, B, CO, CI, HW, G, p, w_index_ci, w_index_co)
 
 
 def norm_dist_backward_input_weight(grad_output, input, weight, output, grad_input, grad_weight, G, p,
@@ -317,10 +325,8 @@ def norm_dist_backward_input_weight(grad_output, input, weight, output, grad_inp
     if grad_weight.shape != weight.shape:
         raise RuntimeError("grad_weight must have the shape of weight")
     dev = _same_device(grad_output, input, weight, output, grad_input, grad_weight, w_index_ci, w_index_co)
-    _call(dev, input, "snb_norm_dist_backward_input_weight", (B, CO, CI),
-          _ptr(grad_output), _ptr(input), _ptr(weight), _ptr(output), B, CO, CI, G, HW, _ptr(grad_input),
-          _ptr(grad_weight), float(p), _ptr(w_index_ci), _ptr(w_index_co), weight.size(0),
-          weight.size(1) * G)
+    _lp_backward(dev, grad_output, input, weight, output, grad_input, grad_weight, B, CO, CI, HW, G, p, w_index_ci,
+                 w_index_co)
 
 
 def bound_inf_dist_forward_nograd(inputL, inputU, weight, outputL, outputU, G):
@@ -539,7 +545,7 @@ def plane_index(index, channels, hw):
 
 # ---- whole layers and the model head (one C call each; G = 1, HW = 1, 2-D tensors) ---------------
 
-_LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward": 4, "snb_layer_bound_forward_ws": 3, "snb_input_box": 1,
+_LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward_ws": 4, "snb_layer_bound_forward_ws": 3, "snb_input_box": 1,
                   "snb_margin_loss": 2, "snb_certified_fraction": 2}
 
 
@@ -581,15 +587,18 @@ def layer_forward(x, weight, p, w_index_ci, w_index_co, y_dist, pos, workspace, 
 
 def layer_backward(grad_out, x, weight, y_dist, pos, p, w_index_ci, w_index_co, mean_shift, mean, grad_centred,
                    grad_bias, grad_x, grad_w):
-    """snb_layer_backward on 2-D tensors (see layer_forward); grad_x [B, CI'] or None, grad_w like
+    """snb_layer_backward_ws on 2-D tensors (see layer_forward); grad_x [B, CI'] or None, grad_w like
     weight or None, grad_bias [W_CO] or None; mean [W_CO] and grad_centred [B, CO'] are scratch for
     the mean-shift part."""
     B, CO = grad_out.shape
     CI = x.size(1)
-    _layer_call("snb_layer_backward", (B, CO, CI), grad_out,
+    ws = None
+    if p < float("inf") and grad_x is not None:
+        ws = _lp_scratch(1, B, CO, CI, weight.size(0), weight.size(1), p, w_index_ci, grad_out.device)
+    _layer_call("snb_layer_backward_ws", (B, CO, CI), grad_out,
                 grad_out.data_ptr(), x.data_ptr(), weight.data_ptr(), _ptr(y_dist), _ptr(pos), B, CO, CI, float(p),
                 _ptr(w_index_ci), _ptr(w_index_co), weight.size(0), weight.size(1), 1 if mean_shift else 0,
-                _ptr(mean), _ptr(grad_centred), _ptr(grad_bias), _ptr(grad_x), _ptr(grad_w))
+                _ptr(mean), _ptr(grad_centred), _ptr(grad_bias), _ptr(grad_x), _ptr(grad_w), *_area(ws))
 
 
 def layer_bound_forward(x, xl, xu, weight, running_mean, bias, y, yl, yu):
