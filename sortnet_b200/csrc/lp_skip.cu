@@ -118,6 +118,13 @@ struct Slabs {
     long long total;                        // sub-batches * chunks * outer
 };
 
+// Results of a lane's tests as bits, one instruction each: the sign of `value` (set: a miss; an arithmetic NaN has none)
+// comes in from below.  512 x 3840 x 3840, p = 1000, against compare and select: 0.60 -> 0.58 and 0.46 -> 0.42 ms.
+constexpr unsigned ALL_MISS = 0xffffffffu;
+__device__ __forceinline__ unsigned shift_in_sign(unsigned bits, float value) {
+    return __funnelshift_l(__float_as_uint(value), bits, 1);
+}
+
 // A warp's queue of passed pairs (inner index in the slab, weight).
 struct PairQueue {
     int2* q;
@@ -128,16 +135,16 @@ struct PairQueue {
         if (hit) q[n + __popc(b & ((1u << (threadIdx.x & 31)) - 1u))] = make_int2(k, __float_as_int(w));
         n += __popc(b);
     }
-    // The pairs k + lane + 32 i (bit i of `hits`) of a scan step, those past the end of the slab excepted; whenever 16
-    // are there they are evaluated.
+    // The pairs k + lane + 32 i of a scan step that are no misses, those past the end of the slab excepted; whenever 16 are
+    // there they are evaluated.
     template <typename F>
-    __device__ __forceinline__ void take(unsigned hits, int k, int end, const float (&w)[SCAN / 32], F&& evaluate) {
+    __device__ __forceinline__ void take(unsigned misses, int k, int end, const float (&w)[SCAN / 32], F&& evaluate) {
         const int lane = threadIdx.x & 31;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
 #pragma unroll
             for (int i = h * (SCAN / 64); i < (h + 1) * (SCAN / 64); i++)
-                push((hits >> i & 1u) && k + lane + 32 * i < end, k + lane + 32 * i, w[i]);
+                push(!(misses >> (SCAN / 32 - 1 - i) & 1u) && k + lane + 32 * i < end, k + lane + 32 * i, w[i]);
             __syncwarp();
             if (n < 16) continue;
             int done = 0;
@@ -230,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) skip_maxima(const ForwardArgs a) {
                 }
             };
             for (int k = 0; k < n; k += SCAN) {
-                float w[SCAN / 32], up[SCAN / 32], best = low;
+                float w[SCAN / 32], up[SCAN / 32], down[SCAN / 32], best = low;
 #pragma unroll
                 for (int i = 0; i < SCAN / 32; i++) w[i] = wr[col[k + lane + 32 * i]];
 #pragma unroll
@@ -238,14 +245,16 @@ __global__ void __launch_bounds__(THREADS, 1) skip_maxima(const ForwardArgs a) {
                     const float2 c = mr[k + lane + 32 * i];
                     const float d = fabsf(w[i] - c.x);
                     up[i] = d + c.y;
-                    best = fmaxf(best, d - c.y);
+                    down[i] = d - c.y;
                 }
+#pragma unroll
+                for (int i = 0; i < SCAN / 32; i += 2) best = max3(best, down[i], down[i + 1]);
                 low = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(best)));     // never negative
                 const float thr = low * (1.0f - 0x1p-19f);      // the bounds are rounded
-                unsigned hits = 0u;
+                unsigned misses = ALL_MISS;
 #pragma unroll
-                for (int i = 0; i < SCAN / 32; i++) hits |= up[i] < thr ? 0u : 1u << i;
-                if (__any_sync(0xffffffffu, hits != 0u)) queue.take(hits, k, n, w, evaluate);
+                for (int i = 0; i < SCAN / 32; i++) misses = shift_in_sign(misses, up[i] - thr);
+                if (__any_sync(0xffffffffu, misses != ALL_MISS)) queue.take(misses, k, n, w, evaluate);
             }
             queue.finish(evaluate);
 #pragma unroll
@@ -264,7 +273,7 @@ __global__ void __launch_bounds__(THREADS, 1) skip_maxima(const ForwardArgs a) {
 // Per warp: an output; its lanes test 256 columns at a time against the row of W and queue those that pass; 16 queued
 // columns are then evaluated together, four groups of eight lanes x four rows (one 16-byte read of x per lane and column).
 // Bound by the special-function unit where many columns pass, by the scan of W where few do.  512 x 3840 x 3840 (inputs
-// N(0, 0.2), maxima included): p = 31.6 4.27 -> 1.28 ms, p = 1000 2.08 -> 0.60 ms.
+// N(0, 0.2), maxima included): p = 31.6 4.26 -> 1.26 ms, p = 1000 2.07 -> 0.58 ms.
 __global__ void __launch_bounds__(THREADS, 1) skip_forward(const ForwardArgs a) {
     extern __shared__ __align__(16) unsigned char dyn[];
     const int padded = up_to(a.sl.chunk, SCAN);
@@ -323,15 +332,15 @@ __global__ void __launch_bounds__(THREADS, 1) skip_forward(const ForwardArgs a) 
             };
             for (int k = 0; k < n; k += SCAN) {
                 float w[SCAN / 32];
-                unsigned hits = 0u;
+                unsigned misses = ALL_MISS;
 #pragma unroll
                 for (int i = 0; i < SCAN / 32; i++) w[i] = wr[col[k + lane + 32 * i]];
 #pragma unroll
                 for (int i = 0; i < SCAN / 32; i++) {
                     const float2 c = mr[k + lane + 32 * i];
-                    hits |= fabsf(w[i] - c.x) + c.y < thr ? 0u : 1u << i;
+                    misses = shift_in_sign(misses, (fabsf(w[i] - c.x) + c.y) - thr);
                 }
-                if (__any_sync(0xffffffffu, hits != 0u)) queue.take(hits, k, n, w, evaluate);
+                if (__any_sync(0xffffffffu, misses != ALL_MISS)) queue.take(misses, k, n, w, evaluate);
             }
             queue.finish(evaluate);
             const float total = sum_groups(acc, lane);
@@ -382,7 +391,7 @@ struct BackwardArgs {
 // the column of W.  Of 16 queued outputs every group evaluates four; the sums over the rows go to grad_w with one reduction
 // per pair, grad_x stays in registers for the length of the slab.  FINE as in lp_bwd_kernel: ratios near 1 take the
 // series and the remainder of the rounded product.  Bounds as in the forward; 512 x 3840 x 3840: p = 31.6 4.23 -> 1.48 ms,
-// p = 1000 2.63 -> 0.46 ms.  A slab of 32 warps of 64 registers beat 16 of 128 (p = 31.6: 1.60 ms).
+// p = 1000 2.64 -> 0.42 ms.  A slab of 32 warps of 64 registers beat 16 of 128 (p = 31.6: 1.60 ms).
 template <bool FINE>
 __global__ void __launch_bounds__(THREADS, 1) skip_backward(const BackwardArgs a) {
     constexpr int E = FINE ? 2 : 4;                                         // pairs per group at a time: what 64 registers hold
@@ -494,14 +503,14 @@ __global__ void __launch_bounds__(THREADS, 1) skip_backward(const BackwardArgs a
             };
             for (int k = 0; k < n; k += SCAN) {
                 float w[SCAN / 32];
-                unsigned hits = 0u;
+                unsigned misses = ALL_MISS;
 #pragma unroll
                 for (int i = 0; i < SCAN / 32; i++) w[i] = wr[row[k + lane + 32 * i]];
 #pragma unroll
                 for (int i = 0; i < SCAN / 32; i++) {
-                    hits |= (fabsf(w[i] - mr.x) + mr.y) * most[k + lane + 32 * i] < a.cut ? 0u : 1u << i;
+                    misses = shift_in_sign(misses, fmaf(fabsf(w[i] - mr.x) + mr.y, most[k + lane + 32 * i], -a.cut));
                 }
-                if (__any_sync(0xffffffffu, hits != 0u)) queue.take(hits, k, n, w, evaluate);
+                if (__any_sync(0xffffffffu, misses != ALL_MISS)) queue.take(misses, k, n, w, evaluate);
             }
             queue.finish(evaluate);
             const float total = sum_groups(acc, lane);
@@ -559,7 +568,7 @@ cudaError_t launch(void (*kern)(Args), const Args& a, int smem, cudaStream_t st)
 }
 
 // Sizes and exponents from which the sparse form is the faster one (B200, dense -> sparse; 512 x 3840 x 3840 of masked
-// 5120 x 5120: p = 10.5 4.26 -> 3.91 and 4.23 -> 3.84 ms, p = 31.6 4.26 -> 1.28 and 4.23 -> 1.48 ms).  Below 64 M terms the
+// 5120 x 5120: p = 10.5 4.26 -> 3.91 and 4.23 -> 3.84 ms, p = 31.6 4.26 -> 1.26 and 4.23 -> 1.47 ms).  Below 64 M terms the
 // passes around the kernels decide: 128 x 784 x 300, p = 10.5 0.083 -> 0.091 and 0.036 -> 0.056 ms; p = 16 0.083 -> 0.079 and
 // 0.036 -> 0.055 ms; p = 100 0.089 -> 0.042 and 0.056 -> 0.039 ms.
 bool applies(const LpProblem& q, float small_p) {
