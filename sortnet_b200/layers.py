@@ -534,8 +534,9 @@ class SortMLPModel(nn.Module):
         ops; the head (margin, loss and its gradient) runs as one kernel, and at p = inf the whole pass is
         one library call per direction (ops.MlpMixtureLossF)."""
         x = x.reshape(x.size(0), -1)
-        if FUSED_LAYERS and self.training and x.is_cuda and x.dtype == torch.float32 and torch.is_grad_enabled() \
-                and not isinstance(self.scalar, torch.Tensor) and all(math.isinf(l.p) for l in self.fc_dist):
+        if FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32 and torch.is_grad_enabled() \
+                and not isinstance(self.scalar, torch.Tensor) and all(math.isinf(l.p) for l in self.fc_dist) \
+                and all(m.training for m in self.modules()):     # a layer in evaluation mode keeps its statistics
             if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
                 masks = self.draw_masks(x.size(0), x.device)
             plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)

@@ -1,0 +1,53 @@
+"""When the whole-net calls (csrc/mlp.cu) stand in for the layers: never where the layers would do something else."""
+import pytest
+import torch
+
+from gpu_util import rel
+from test_mlp_gpu import nets
+
+pytestmark = pytest.mark.gpu
+
+
+def by_layers(fn):
+    """fn() without the whole-net calls: layer by layer, as at sizes where they do not apply."""
+    from sortnet_b200 import norm_dist_cuda as C
+    keep, C.MlpPlan.applies = C.MlpPlan.applies, lambda self, *a: False
+    try:
+        return fn()
+    finally:
+        C.MlpPlan.applies = keep
+
+
+def batch(B=70, dims=(3, 17, 17), classes=10, seed=3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.rand(B, *dims, device="cuda", generator=g), torch.randint(0, classes, (B,), device="cuda", generator=g)
+
+
+def step(net, x, t, **kw):
+    torch.manual_seed(7)
+    loss = net.mixture_loss(x, t, 0.05, **kw)
+    loss.backward()
+    return loss.detach()
+
+
+def same_step(a, b, x, t, **kw):
+    """Loss, gradients and running means of a step with the whole-net calls allowed and without them."""
+    la, lb = step(a, x, t, **kw), by_layers(lambda: step(b, x, t, **kw))
+    assert abs(float(la) - float(lb)) <= 2e-6 * max(1.0, abs(float(lb)))
+    for p, q in zip(a.parameters(), b.parameters()):
+        assert (p.grad is None) == (q.grad is None)
+        assert p.grad is None or rel(p.grad.cpu().numpy(), q.grad.cpu().numpy()) < 1e-5
+    for u, v in zip(a.buffers(), b.buffers()):
+        assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("keep", [0.8, 1.0])
+def test_layer_in_evaluation_mode_during_training(keep):
+    """A layer with frozen statistics subtracts its running mean and leaves it alone, whatever the batch size."""
+    a, b = nets(4, 700, (3, 17, 17), 10, keep)
+    for net in (a, b):
+        net.train()
+        net.fc_dist[1].mean_shift.running_mean.fill_(2.0)
+        net.fc_dist[1].eval()
+    same_step(a, b, *batch())
+    assert bool((a.fc_dist[1].mean_shift.running_mean == 2.0).all())
