@@ -469,8 +469,8 @@ class SortMLPModel(nn.Module):
         """The plan for an evaluation pass without gradients on x [B, pixels], or None."""
         if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist):
             return None
-        if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
-            return None
+        if torch.is_grad_enabled() and (self.training or x.requires_grad or any(p.requires_grad for p in self.parameters())):
+            return None                      # a model in training mode draws masks, whatever its layers do
         plan = self._plan(sort_eval=sort_eval)
         return plan if plan is not None and plan.applies(x.size(0)) else None
 

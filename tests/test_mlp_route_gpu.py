@@ -51,3 +51,17 @@ def test_layer_in_evaluation_mode_during_training(keep):
         net.fc_dist[1].eval()
     same_step(a, b, *batch())
     assert bool((a.fc_dist[1].mean_shift.running_mean == 2.0).all())
+
+
+def test_model_in_training_mode_with_layers_in_evaluation_mode():
+    """Sub-sampling follows the model's own flag: masks are drawn although every layer evaluates."""
+    a, b = nets(4, 700, (3, 17, 17), 10, 0.8)
+    x, _ = batch()
+    for net in (a, b):
+        net.requires_grad_(False).train()
+        for l in net.fc_dist:
+            l.eval()
+    torch.manual_seed(7)
+    got = a(x)
+    torch.manual_seed(7)
+    assert torch.equal(got, by_layers(lambda: b(x)))
