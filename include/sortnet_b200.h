@@ -163,7 +163,7 @@ int snb_mlp_train_forward(const snb_mlp_layer* layers, int depth, const float* x
 int snb_mlp_train_backward(const snb_mlp_layer* layers, int depth, int B, const float* grad_loss, const void* saved,
                            void* scratch, float* const* grad_w, float* grad_bias, float* grad_x, int* launches, void* stream);
 /* Evaluation pass: tensors = 1 (y) or 3 (y and the bounds of a box: xl, xu, or [max(x - box_eps, down), min(x + box_eps, up)]
- * when they are NULL); score / margin [B, classes] optional. */
+ * when they are NULL); score / margin [B, classes] optional (a label outside [0, classes): NaN margins in its row). */
 int snb_mlp_eval_forward(const snb_mlp_layer* layers, int depth, const float* x, const float* xl, const float* xu, int B,
                          int tensors, float box_eps, float down, float up, void* scratch, float* y, float* yl, float* yu,
                          const long long* targets, float inv_two_eps, float scale, float* score, float* margin, int* launches,

@@ -212,16 +212,18 @@ __global__ void __launch_bounds__(256) chain_bwd_kernel(const float* __restrict_
 }
 
 // Scores and margins of the evaluation pass from the head's outputs (ell_inf_models.py:45-50): score = -y * scale,
-// margin[b, c] = ((-yl[b, c]) - (-yu[b, t])) / (2 eps), 0 at the target.
+// margin[b, c] = ((-yl[b, c]) - (-yu[b, t])) / (2 eps), 0 at the target.  A label outside [0, K) gives NaN.
 __global__ void __launch_bounds__(256) scores_kernel(const float* __restrict__ y, const float* __restrict__ yl,
                                                      const float* __restrict__ yu, const long long* __restrict__ target, int B,
                                                      int K, float inv_two_eps, float scale, float* __restrict__ score,
                                                      float* __restrict__ margin) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= B * K) return;
-    const int b = i / K, c = i % K, t = (int)target[b];
+    const int b = i / K, c = i % K;
+    const long long t = target[b];
     score[i] = -y[i] * scale;
-    margin[i] = c == t ? 0.f * inv_two_eps : (-yl[i] - -yu[(size_t)b * K + t]) * inv_two_eps;
+    if (t < 0 || t >= K) margin[i] = __int_as_float(0x7fc00000);
+    else margin[i] = c == t ? 0.f * inv_two_eps : (-yl[i] - -yu[(size_t)b * K + t]) * inv_two_eps;
 }
 
 size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }

@@ -590,13 +590,13 @@ class SortMLPModel(nn.Module):
                 up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
                 box = (torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down).contiguous(),
                        torch.minimum(x + eps, up.reshape(1, -1) if up.dim() else up).contiguous())
-            number = not isinstance(self.scalar, torch.Tensor)
-            y, lower, upper, score, margin = _C.mlp_eval_forward(
-                plan, x, box, targets.contiguous() if targets is not None and number else None, 2 * eps,
-                float(self.scalar) if number else 1.0)
+            # targets of another kind are left to _scores, which knows what to accept and what to refuse
+            head = targets is not None and not isinstance(self.scalar, torch.Tensor) and _C.targets_fit(targets, x)
+            y, lower, upper, score, margin = _C.mlp_eval_forward(plan, x, box, targets.contiguous() if head else None, 2 * eps,
+                                                                 float(self.scalar) if head else 1.0)
             if targets is None:
                 return -y * self.scalar
-            return (score, margin) if number else self._scores(y, lower, upper, targets, eps)
+            return (score, margin) if head else self._scores(y, lower, upper, targets, eps)
         if up is not None and down is not None and self._certifying():
             up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
             lower = torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down)

@@ -673,8 +673,20 @@ def _mlp_call(entry, ref, *args):
     _launched += n.value
 
 
+def targets_fit(targets, x):
+    """Whether `targets` is what the kernels read: one int64 label per row of x, on its device."""
+    return targets.dtype == torch.int64 and targets.device == x.device and targets.numel() == x.size(0)
+
+
+def _check_targets(targets, x):
+    if not targets_fit(targets, x) or not targets.is_contiguous():
+        raise RuntimeError("targets must be %d contiguous int64 labels on %s, got %s %s on %s"
+                           % (x.size(0), x.device, tuple(targets.shape), targets.dtype, targets.device))
+
+
 def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):
     """snb_mlp_train_forward: (loss, saved); x [B, in] fp32, targets [B] int64."""
+    _check_targets(targets, x)
     B, lib = x.size(0), _lib.load()
     saved = torch.empty(lib.snb_mlp_saved_bytes(plan.table, plan.depth, B), device=x.device, dtype=torch.uint8)
     scratch = torch.empty(lib.snb_mlp_scratch_bytes(plan.table, plan.depth, B, 1, 1), device=x.device, dtype=torch.uint8)
@@ -695,7 +707,10 @@ def mlp_train_backward(plan, B, grad_loss, saved, grad_w, grad_bias, grad_x):
 
 def mlp_eval_forward(plan, x, box=None, targets=None, two_eps=1.0, scale=1.0):
     """snb_mlp_eval_forward.  box: None, (xl, xu) tensors [B, in], or (eps, down, up) numbers.  Returns
-    (y, yl, yu, score, margin); the last four None without a box, the last two None without targets."""
+    (y, yl, yu, score, margin); the last four None without a box, the last two None without targets.  A label outside
+    [0, classes) makes its row's margins NaN."""
+    if targets is not None:
+        _check_targets(targets, x)
     B, K, dev = x.size(0), plan.weights[-1].size(0), x.device
     tensors = 1 if box is None else 3
     scratch = torch.empty(_lib.load().snb_mlp_scratch_bytes(plan.table, plan.depth, B, tensors, 0), device=dev, dtype=torch.uint8)

@@ -87,6 +87,18 @@ def test_tensor_checks_raise_on_cpu_tensors():
         C.bound_inf_dist_forward_nograd(x, x, w, y, y, 1)
 
 
+def test_whole_net_calls_refuse_other_targets():
+    """Labels are read as int64 on the device: nothing else gets as far as a launch."""
+    from sortnet_b200 import norm_dist_cuda as C
+    x = torch.rand(4, 8)
+    C._check_targets(torch.tensor([0, 1, 2, 3]), x)
+    for bad in (torch.zeros(4, dtype=torch.int32), torch.zeros(3, dtype=torch.int64), torch.zeros(8, dtype=torch.int64)[::2],
+                torch.zeros(4, dtype=torch.int64, device="meta"), torch.zeros(4)):
+        for call in (lambda: C.mlp_train_forward(None, x, bad, 0.1, 1.0, 0.1, 1.0), lambda: C.mlp_eval_forward(None, x, None, bad)):
+            with pytest.raises(RuntimeError, match="targets"):
+                call()
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops

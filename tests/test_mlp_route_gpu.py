@@ -65,3 +65,36 @@ def test_model_in_training_mode_with_layers_in_evaluation_mode():
     got = a(x)
     torch.manual_seed(7)
     assert torch.equal(got, by_layers(lambda: b(x)))
+
+
+def evaluating(keep=0.8, scalar=False):
+    a, _ = nets(4, 700, (3, 17, 17), 10, keep, scalar=scalar)
+    return a.eval()
+
+
+def test_labels_out_of_range_give_nan_margins():
+    """As the last row and inside: no other row's bounds are read for them."""
+    a, (x, t) = evaluating(), batch()
+    with torch.no_grad():
+        score, margin = a(x, t, 0.02, up=1.0, down=0.0)
+        for row, label in ((0, -1), (5, 10), (69, 2 ** 40), (31, -(2 ** 62))):
+            t[row] = label
+        s2, m2 = a(x, t, 0.02, up=1.0, down=0.0)
+    bad = torch.tensor([0, 5, 31, 69], device="cuda")
+    good = torch.ones(70, dtype=torch.bool, device="cuda").index_fill_(0, bad, False)
+    assert torch.equal(score, s2) and torch.equal(margin[good], m2[good]) and bool(m2[bad].isnan().all())
+
+
+def test_other_targets_are_refused():
+    a, (x, t) = evaluating(), batch()
+    with torch.no_grad():
+        for bad in (t.int(), t.cpu(), t[:60]):
+            with pytest.raises((RuntimeError, IndexError)):
+                a(x, bad, 0.02, up=1.0, down=0.0)
+        want = a(x, t, 0.02, up=1.0, down=0.0)
+        got = a(x, t.view(-1, 1), 0.02, up=1.0, down=0.0)
+    assert torch.equal(want[1], got[1])
+    a.train()
+    for bad in (t.int(), t[:60]):
+        with pytest.raises(RuntimeError):
+            a.mixture_loss(x, bad, 0.02)
