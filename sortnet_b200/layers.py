@@ -575,6 +575,13 @@ class SortMLPModel(nn.Module):
         margin = margin.scatter(1, targets.view(-1, 1), 0)
         return score * self.scalar, margin / (2 * eps)
 
+    @staticmethod
+    def _box(x, eps, up, down):
+        """[max(x - eps, down), min(x + eps, up)]; up and down are numbers or values per pixel."""
+        up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
+        return (torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down),
+                torch.minimum(x + eps, up.reshape(1, -1) if up.dim() else up))
+
     def forward(self, x=None, targets=None, eps=0, up=None, down=None, masks=None):
         x = x.reshape(x.size(0), -1)
         lower = upper = None
@@ -584,23 +591,20 @@ class SortMLPModel(nn.Module):
             if up is None or down is None:
                 y = _C.mlp_eval_forward(plan, x)[0]
                 return -y * self.scalar if targets is None else self._scores(y, None, None, targets, eps)
-            if isinstance(up, (int, float)) and isinstance(down, (int, float)):
+            number = isinstance(eps, (int, float))          # else a tensor, perhaps with a value per row
+            if number and isinstance(up, (int, float)) and isinstance(down, (int, float)):
                 box = (eps, down, up)
             else:
-                up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
-                box = (torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down).contiguous(),
-                       torch.minimum(x + eps, up.reshape(1, -1) if up.dim() else up).contiguous())
+                box = tuple(z.contiguous() for z in self._box(x, eps, up, down))
             # targets of another kind are left to _scores, which knows what to accept and what to refuse
-            head = targets is not None and not isinstance(self.scalar, torch.Tensor) and _C.targets_fit(targets, x)
-            y, lower, upper, score, margin = _C.mlp_eval_forward(plan, x, box, targets.contiguous() if head else None, 2 * eps,
-                                                                 float(self.scalar) if head else 1.0)
+            head = targets is not None and number and not isinstance(self.scalar, torch.Tensor) and _C.targets_fit(targets, x)
+            y, lower, upper, score, margin = _C.mlp_eval_forward(plan, x, box, targets.contiguous() if head else None,
+                                                                 2 * eps if head else 1.0, float(self.scalar) if head else 1.0)
             if targets is None:
                 return -y * self.scalar
             return (score, margin) if head else self._scores(y, lower, upper, targets, eps)
         if up is not None and down is not None and self._certifying():
-            up, down = (torch.as_tensor(z, device=x.device, dtype=x.dtype) for z in (up, down))
-            lower = torch.maximum(x - eps, down.reshape(1, -1) if down.dim() else down)
-            upper = torch.minimum(x + eps, up.reshape(1, -1) if up.dim() else up)
+            lower, upper = self._box(x, eps, up, down)
         out = self._distances(x, masks, lower, upper)
         if lower is not None:
             x, lower, upper = out

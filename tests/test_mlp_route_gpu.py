@@ -98,3 +98,16 @@ def test_other_targets_are_refused():
     for bad in (t.int(), t[:60]):
         with pytest.raises(RuntimeError):
             a.mixture_loss(x, bad, 0.02)
+
+
+@pytest.mark.parametrize("keep", [0.8, 1.0])
+@pytest.mark.parametrize("limits", ["numbers", "pixels"])
+@pytest.mark.parametrize("eps", ["row", "one", "zero-dim"])
+def test_eps_as_a_tensor(keep, limits, eps):
+    a, (x, t) = evaluating(keep), batch()
+    eps = {"row": 0.05 * torch.rand(70, 1, device="cuda") + 0.01, "one": torch.full((1,), 0.02, device="cuda"),
+           "zero-dim": torch.tensor(0.02)}[eps]
+    box = (1.0, 0.0) if limits == "numbers" else (torch.ones(867, device="cuda"), torch.zeros(867, device="cuda"))
+    with torch.no_grad():
+        got, want = (run(lambda: a(x, t, eps, up=box[0], down=box[1])) for run in (lambda f: f(), by_layers))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
