@@ -33,7 +33,10 @@ __global__ void __launch_bounds__(256) keep_flags_kernel(const KeepJobs jobs) {
     unsigned char* f = flags + (size_t)s * channels;
     for (int c = threadIdx.x; c < channels; c += 256) f[c] = 0;
     __syncthreads();
-    for (int k = threadIdx.x; k < count; k += 256) f[list[(size_t)s * count + k]] = 1;
+    for (int k = threadIdx.x; k < count; k += 256) {
+        const int c = list[(size_t)s * count + k];
+        if ((unsigned)c < (unsigned)channels) f[c] = 1;      // the lists are the caller's: an entry out of range keeps nothing
+    }
 }
 
 // Training mean shift in the chain form: the batch mean of every channel from the sub-batches' row sums (in the order of

@@ -503,6 +503,11 @@ struct PosList {
     }
 };
 
+// Position of an output at its floor: the first kept column (never one outside W, whatever the list holds).
+__device__ __forceinline__ uint32_t first_kept(const PruneProblem& p, int s) {
+    return p.kept_list ? min((uint32_t)p.kept_list[(size_t)s * p.kept], (uint32_t)p.W_CI - 1u) : 0u;
+}
+
 // ---- results of 32 outputs / of one output ---------------------------------------------------------
 template <int NV>
 __device__ __forceinline__ float shifted(const PruneProblem& p, float v, int j) {
@@ -717,7 +722,7 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
             }
             return word;
         };
-        const uint32_t floor_word = p.kept_list ? (uint32_t)p.kept_list[(size_t)s * p.kept] : 0u;
+        const uint32_t floor_word = first_kept(p, s);
         uint32_t word[TRACK ? NV : 1][4];
 #pragma unroll
         for (int t = 0; t < NV; t++)
@@ -909,7 +914,7 @@ __global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
         const float* xs = a.xt + (size_t)s * C * NX * 32;
         const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
         const int b = s * 32 + lane;
-        const uint32_t floor_word = p.kept_list ? (uint32_t)p.kept_list[(size_t)s * p.kept] : 0u;
+        const uint32_t floor_word = first_kept(p, s);
         auto store = [&](const MaxState<NX, TRACK>& st, int n) {          // all lanes of a warp
             if (p.yt || p.post) emit_chain<NX>(p, s, n, st.acc, TRACK ? st.word[0] : 0u);
             if (p.part) {

@@ -460,7 +460,7 @@ class SortMLPModel(nn.Module):
             K, q = 1, 0.0
             if sort_eval and not ops._sort_is_plain_max(l.weight, l.dropout, 10):
                 K, q = min(l.in_features, 10), l.dropout
-            kept = _as_index32(masks[k]) if masks is not None and k < last else None
+            kept = _as_index32(masks[k]) if masks is not None and k < min(last, len(masks)) else None
             rows.append((l.weight, l.bias, None if shift is None else shift.running_mean,
                          0.0 if shift is None else shift.momentum, kept, K, q))
         return _C.MlpPlan(rows)
@@ -472,7 +472,7 @@ class SortMLPModel(nn.Module):
         if torch.is_grad_enabled() and (self.training or x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return None                      # a model in training mode draws masks, whatever its layers do
         plan = self._plan(sort_eval=sort_eval)
-        return plan if plan is not None and plan.applies(x.size(0)) else None
+        return plan if plan is not None and plan.takes(x) and plan.applies(x.size(0)) else None
 
     @torch.no_grad()
     def certified_margin(self, x, targets, eps, up, down, sort_eval=None, after_layer=None):
@@ -507,9 +507,9 @@ class SortMLPModel(nn.Module):
             else:
                 lower = torch.maximum(x - eps, torch.as_tensor(down, device=x.device))
                 upper = torch.minimum(x + eps, torch.as_tensor(up, device=x.device))
-            plan = self._eval_plan(x, sort_eval) if after_layer is None else None
+            plan = self._eval_plan(x, sort_eval) if after_layer is None and _C.box_fits((lower, upper), x) else None
             if plan is not None:
-                _, lower, upper, _, _ = _C.mlp_eval_forward(plan, x.contiguous(), (lower.contiguous(), upper.contiguous()))
+                _, lower, upper, _, _ = _C.mlp_eval_forward(plan, x.contiguous(), (lower, upper))
             for k, layer in enumerate(self.fc_dist if plan is None else ()):
                 assert math.isinf(layer.p)
                 x, lower, upper = layer(x, lower, upper, sort_eval=sort_eval and layer.keep_rate != 1.0)
@@ -540,7 +540,7 @@ class SortMLPModel(nn.Module):
             if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
                 masks = self.draw_masks(x.size(0), x.device)
             plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)
-            if plan is not None and plan.applies(x.size(0)) and any(t.requires_grad for t in (x, *plan.weights)):
+            if plan is not None and plan.takes(x) and plan.applies(x.size(0)) and any(t.requires_grad for t in (x, *plan.weights)):
                 return ops.MlpMixtureLossF.apply(x.contiguous(), targets.contiguous(), eps, clip, lam, float(self.scalar), plan,
                                                  plan.head_bias, *plan.weights)
         d = self._distances(x, masks)
@@ -584,27 +584,24 @@ class SortMLPModel(nn.Module):
 
     def forward(self, x=None, targets=None, eps=0, up=None, down=None, masks=None):
         x = x.reshape(x.size(0), -1)
-        lower = upper = None
+        lower = upper = box = None
+        number = isinstance(eps, (int, float))              # else a tensor, perhaps with a value per row
         plan = self._eval_plan(x, any(l.keep_rate != 1.0 for l in self.fc_dist))
-        if plan is not None:
-            x = x.contiguous()
-            if up is None or down is None:
-                y = _C.mlp_eval_forward(plan, x)[0]
-                return -y * self.scalar if targets is None else self._scores(y, None, None, targets, eps)
-            number = isinstance(eps, (int, float))          # else a tensor, perhaps with a value per row
-            if number and isinstance(up, (int, float)) and isinstance(down, (int, float)):
+        if up is not None and down is not None and self._certifying():
+            if plan is not None and number and isinstance(up, (int, float)) and isinstance(down, (int, float)):
                 box = (eps, down, up)
             else:
-                box = tuple(z.contiguous() for z in self._box(x, eps, up, down))
+                lower, upper = box = self._box(x, eps, up, down)
+                plan = plan if _C.box_fits(box, x) else None
+        if plan is not None:
             # targets of another kind are left to _scores, which knows what to accept and what to refuse
-            head = targets is not None and number and not isinstance(self.scalar, torch.Tensor) and _C.targets_fit(targets, x)
-            y, lower, upper, score, margin = _C.mlp_eval_forward(plan, x, box, targets.contiguous() if head else None,
+            head = box is not None and targets is not None and number and not isinstance(self.scalar, torch.Tensor) \
+                and _C.targets_fit(targets, x)
+            y, lower, upper, score, margin = _C.mlp_eval_forward(plan, x.contiguous(), box, targets.contiguous() if head else None,
                                                                  2 * eps if head else 1.0, float(self.scalar) if head else 1.0)
             if targets is None:
                 return -y * self.scalar
             return (score, margin) if head else self._scores(y, lower, upper, targets, eps)
-        if up is not None and down is not None and self._certifying():
-            lower, upper = self._box(x, eps, up, down)
         out = self._distances(x, masks, lower, upper)
         if lower is not None:
             x, lower, upper = out

@@ -652,8 +652,25 @@ class MlpPlan:
         self.head_bias = rows[-1][1]
         self.keep = rows
         self.table = (MlpLayer * self.depth)(*[
-            MlpLayer(w.data_ptr(), _ptr(b), _ptr(rm), _ptr(kept), w.size(1), w.size(0), 0 if kept is None else kept.size(2),
+            MlpLayer(w.data_ptr(), _ptr(b), _ptr(rm), _ptr(kept), w.size(-1), w.size(0), 0 if kept is None else kept.size(-1),
                      K, mom, q) for w, b, rm, mom, kept, K, q in rows])
+
+    def takes(self, x):
+        """Whether every tensor is what the kernels read through its pointer: fp32 (int32 lists), contiguous, on the
+        device of x [B, in], of the shapes of a chain of layers."""
+        B, width = x.shape
+        for w, bias, mean, _, kept, _, _ in self.keep:
+            if w.dim() != 2 or w.size(1) != width:
+                return False
+            width = w.size(0)
+            fits = [(w, tuple(w.shape), torch.float32)]
+            fits += [(t, (width,), torch.float32) for t in (bias, mean) if t is not None]
+            if kept is not None:
+                fits.append((kept, ((B + _SUB_BATCH - 1) // _SUB_BATCH, 1, kept.size(-1)), torch.int32))
+            if any(t.device != x.device or t.dtype != dtype or tuple(t.shape) != shape or not t.is_contiguous()
+                   for t, shape, dtype in fits):
+                return False
+        return True
 
     def applies(self, B):
         return _timeline is None and bool(_lib.load().snb_mlp_applies(self.table, self.depth, B))
@@ -678,6 +695,11 @@ def targets_fit(targets, x):
     return targets.dtype == torch.int64 and targets.device == x.device and targets.numel() == x.size(0)
 
 
+def box_fits(box, x):
+    """Whether both ends of a box are what the kernels read: fp32 tensors like x [B, in] on its device."""
+    return all(z.dtype == torch.float32 and z.device == x.device and z.shape == x.shape for z in box)
+
+
 def _check_targets(targets, x):
     if not targets_fit(targets, x) or not targets.is_contiguous():
         raise RuntimeError("targets must be %d contiguous int64 labels on %s, got %s %s on %s"
@@ -687,6 +709,10 @@ def _check_targets(targets, x):
 def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):
     """snb_mlp_train_forward: (loss, saved); x [B, in] fp32, targets [B] int64."""
     _check_targets(targets, x)
+    if DEBUG_INDEX_CHECKS:
+        for w, _, _, _, kept, _, _ in plan.keep:
+            if kept is not None and not check_index_lists(kept, w.size(0), "mask"):
+                raise RuntimeError("mask is not in ascending order")
     B, lib = x.size(0), _lib.load()
     saved = torch.empty(lib.snb_mlp_saved_bytes(plan.table, plan.depth, B), device=x.device, dtype=torch.uint8)
     scratch = torch.empty(lib.snb_mlp_scratch_bytes(plan.table, plan.depth, B, 1, 1), device=x.device, dtype=torch.uint8)
@@ -720,7 +746,11 @@ def mlp_eval_forward(plan, x, box=None, targets=None, two_eps=1.0, scale=1.0):
         yl, yu = torch.empty_like(y), torch.empty_like(y)
         if targets is not None:
             score, margin = torch.empty_like(y), torch.empty_like(y)
-    ends = box if tensors == 3 and len(box) == 2 else (None, None)
+    ends = (None, None)
+    if tensors == 3 and len(box) == 2:
+        if not box_fits(box, x):
+            raise RuntimeError("the ends of the box must be float32 tensors of shape %s on %s" % (tuple(x.shape), x.device))
+        ends = tuple(z.contiguous() for z in box)
     numbers = tuple(float(v) for v in box) if tensors == 3 and len(box) == 3 else (0.0, 0.0, 0.0)
     inverse = float("inf") if two_eps == 0 else 1.0 / two_eps
     _mlp_call("snb_mlp_eval_forward", x, plan.table, plan.depth, x.data_ptr(), _ptr(ends[0]), _ptr(ends[1]), B, tensors, *numbers,

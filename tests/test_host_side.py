@@ -99,6 +99,31 @@ def test_whole_net_calls_refuse_other_targets():
                 call()
 
 
+def test_whole_net_plan_takes_only_what_the_kernels_read():
+    """Anything else is left to the layers, which refuse it or know what to do with it."""
+    from sortnet_b200 import norm_dist_cuda as C
+    x = torch.rand(40, 12)
+
+    def rows():
+        lists = torch.zeros(2, 1, 5, dtype=torch.int32)
+        return [[torch.rand(8, 12), None, torch.zeros(8), 0.1, lists, 1, 0.0], [torch.rand(3, 8), torch.zeros(3), None, 0.0, None, 1, 0.0]]
+
+    assert C.MlpPlan(rows()).takes(x)
+    assert not C.MlpPlan(rows()).takes(x[:, :11]) and not C.MlpPlan(rows()).takes(torch.rand(70, 12))
+    for layer, field, bad in ((0, 0, torch.rand(8, 12).double()), (0, 0, torch.rand(12, 8).t()), (0, 0, torch.rand(8, 11)),
+                              (1, 0, torch.rand(3, 9)), (0, 2, torch.zeros(7)), (1, 1, torch.zeros(3).half()),
+                              (0, 4, torch.zeros(1, 1, 5, dtype=torch.int32)), (0, 4, torch.zeros(2, 2, 5, dtype=torch.int32)),
+                              (0, 4, torch.zeros(2, 1, 5, dtype=torch.int64)), (0, 4, torch.zeros(2, 5, dtype=torch.int32))):
+        table = rows()
+        table[layer][field] = bad
+        assert not C.MlpPlan(table).takes(x), (layer, field)
+    assert C.box_fits((x, x), x)
+    for bad in (x.double(), x[:, :11], x.unsqueeze(0)):
+        assert not C.box_fits((x, bad), x)
+        with pytest.raises(RuntimeError, match="box"):
+            C.mlp_eval_forward(C.MlpPlan(rows()), x, (x, bad))
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops

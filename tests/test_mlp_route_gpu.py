@@ -111,3 +111,23 @@ def test_eps_as_a_tensor(keep, limits, eps):
     with torch.no_grad():
         got, want = (run(lambda: a(x, t, eps, up=box[0], down=box[1])) for run in (lambda f: f(), by_layers))
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_masks_of_the_caller(monkeypatch):
+    """Entries outside the layer keep nothing and are written nowhere; with index checks on they are refused, as
+    lists in another order are; lists of another shape go to the layers, which refuse them."""
+    from sortnet_b200 import norm_dist_cuda as C
+    a, b = nets(4, 700, (3, 17, 17), 10, 0.8)
+    x, t = batch()
+    masks = a.draw_masks(70, "cuda")
+    shorter = [m[..., :-1].contiguous() for m in masks]
+    for m in masks:
+        m[0, 0, -1], m[1, 0, -1], m[2, 0, -1] = 700, 2 ** 30, -1
+    out = [net.mixture_loss(x, t, 0.05, masks=m).detach() for net, m in ((a, masks), (b, shorter))]
+    assert torch.equal(*out)
+    good = a.draw_masks(70, "cuda")
+    monkeypatch.setattr(C, "DEBUG_INDEX_CHECKS", True)
+    a.mixture_loss(x, t, 0.05, masks=good)
+    for bad in (masks, [m.flip(-1).contiguous() for m in good]):
+        with pytest.raises(RuntimeError):
+            a.mixture_loss(x, t, 0.05, masks=bad)
