@@ -22,6 +22,7 @@ import math
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules import module as _module
 
 from . import norm_dist_cuda as _C
 from . import ops
@@ -391,6 +392,15 @@ class NormDistConv(nn.Module):
             self.bias is not None, self.dropout)
 
 
+def _is_plain(module, cls):
+    """Whether calling `module` is calling cls.forward and nothing else: no hooks, no override."""
+    own = module.__dict__
+    return type(module).forward is cls.forward and "forward" not in own and not any(own[name] for name in _HOOKS)
+
+
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+
+
 class SortMLPModel(nn.Module):
     """depth norm-distance layers: pixels -> width -> ... -> width -> num_classes.
 
@@ -449,8 +459,14 @@ class SortMLPModel(nn.Module):
 
     def _plan(self, masks=None, sort_eval=False):
         """Layer table for the whole-net calls (norm_dist_cuda.MlpPlan), or None when the stack is not the
-        one built here (hidden layers with a mean shift and no bias, a head without mean shift, p = inf)."""
+        one built here (hidden layers with a mean shift and no bias, a head without mean shift, p = inf) or somebody
+        wants the layers called one by one (hooks, methods of a subclass)."""
         rows, last = [], len(self.fc_dist) - 1
+        if any(getattr(type(self), name) is not getattr(SortMLPModel, name) for name in ("_distances", "_scores", "_certifying")) \
+                or any(getattr(_module, "_global" + name) for name in _HOOKS) \
+                or not all(_is_plain(l, NormDist) and (l.mean_shift is None or _is_plain(l.mean_shift, MeanShiftDropout))
+                           for l in self.fc_dist):
+            return None
         for k, l in enumerate(self.fc_dist):
             shift = l.mean_shift
             if not math.isinf(l.p) or (shift is None) != (k == last) or (k < last and l.bias is not None):

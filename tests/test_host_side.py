@@ -124,6 +124,44 @@ def test_whole_net_plan_takes_only_what_the_kernels_read():
             C.mlp_eval_forward(C.MlpPlan(rows()), x, (x, bad))
 
 
+def test_hooks_and_overrides_keep_the_layers():
+    """No whole-net plan for a net whose layers somebody wants called."""
+    from sortnet_b200 import layers
+
+    def net(p=float("inf")):
+        m = layers.SortMLPModel(depth=3, width=16, input_dim=(1, 3, 3), num_classes=3, dropout=0.9)
+        m.set_p(p)
+        return m
+
+    class Loud(layers.NormDist):
+        def forward(self, *args, **kw):
+            return super().forward(*args, **kw)
+
+    class Other(layers.SortMLPModel):
+        def _distances(self, *args, **kw):
+            return super()._distances(*args, **kw)
+
+    assert net()._plan() is not None and net(8.0)._plan() is None
+    for register in ("register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook",
+                     "register_full_backward_pre_hook"):
+        for pick in (lambda m: m.fc_dist[1], lambda m: m.fc_dist[2], lambda m: m.fc_dist[0].mean_shift):
+            m = net()
+            handle = getattr(pick(m), register)(lambda *a: None)
+            assert m._plan() is None, register
+            handle.remove()
+            assert m._plan() is not None
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert net()._plan() is None
+    handle.remove()
+    m = net()
+    m.fc_dist[1].__class__ = Loud
+    assert m._plan() is None
+    m = net()
+    m.fc_dist[1].forward = m.fc_dist[1].forward
+    assert m._plan() is None
+    assert Other(depth=3, width=16, input_dim=(1, 3, 3), num_classes=3)._plan() is None
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops

@@ -131,3 +131,16 @@ def test_masks_of_the_caller(monkeypatch):
     for bad in (masks, [m.flip(-1).contiguous() for m in good]):
         with pytest.raises(RuntimeError):
             a.mixture_loss(x, t, 0.05, masks=bad)
+
+
+def test_hooks_of_layers_are_called():
+    a, (x, t) = nets(4, 700, (3, 17, 17), 10, 0.8)[0], batch()
+    seen = []
+    for k, l in enumerate(a.fc_dist):
+        l.register_forward_hook(lambda m, i, o, k=k: seen.append(k))
+    a.mixture_loss(x, t, 0.05).backward()
+    a.eval()
+    with torch.no_grad():
+        a(x, t, 0.02, up=1.0, down=0.0)
+        a.certified_margin(x, t, 0.02, 1.0, 0.0)
+    assert seen == 3 * [0, 1, 2, 3]
