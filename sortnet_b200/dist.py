@@ -4,8 +4,9 @@ The reference wraps its model in torch DistributedDataParallel (main.py:402), i.
 all-reduce(mean) of every parameter gradient per step.  Here each parameter's gradient is
 all-reduced as soon as autograd has finished accumulating it (a post-accumulate hook), on
 NCCL's own stream, so the exchange of layer k overlaps the backward kernels of layers
-k-1 ... 1; the wide layers' gradients are 60-400 MB each, large enough to run at NVLink
-bandwidth without bucketing.  `finish()` waits for the outstanding reductions and turns the
+k-1 ... 1 (SortMLPModel.mixture_loss takes the layers one by one for parameters with such hooks:
+its whole-net call would hand over all gradients after the last kernel); the wide layers' gradients
+are 60-400 MB each, large enough to run at NVLink bandwidth without bucketing.  `finish()` waits for the outstanding reductions and turns the
 sums into means.  Ranks only ever touch their own memory; NCCL does the transport.
 """
 import torch

@@ -556,7 +556,10 @@ class SortMLPModel(nn.Module):
             if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
                 masks = self.draw_masks(x.size(0), x.device)
             plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)
-            if plan is not None and plan.takes(x) and plan.applies(x.size(0)) and any(t.requires_grad for t in (x, *plan.weights)):
+            # post-accumulate hooks (dist.GradientAllReduce) get a layer's gradient while earlier layers still run: by layers
+            early = any(p._post_accumulate_grad_hooks for p in self.parameters())
+            if plan is not None and not early and plan.takes(x) and plan.applies(x.size(0)) \
+                    and any(t.requires_grad for t in (x, *plan.weights)):
                 return ops.MlpMixtureLossF.apply(x.contiguous(), targets.contiguous(), eps, clip, lam, float(self.scalar), plan,
                                                  plan.head_bias, *plan.weights)
         d = self._distances(x, masks)

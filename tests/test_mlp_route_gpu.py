@@ -144,3 +144,21 @@ def test_hooks_of_layers_are_called():
         a(x, t, 0.02, up=1.0, down=0.0)
         a.certified_margin(x, t, 0.02, 1.0, 0.0)
     assert seen == 3 * [0, 1, 2, 3]
+
+
+def test_gradients_arrive_layer_by_layer_for_post_accumulate_hooks(monkeypatch):
+    """What dist.GradientAllReduce overlaps its exchange with: when the hook of a layer fires, the backward of the layer
+    before it has not been queued yet."""
+    from sortnet_b200 import norm_dist_cuda as C
+    a, b = nets(4, 700, (3, 17, 17), 10, 0.8)
+    x, t = batch()
+    log, call = [], C._layer_call
+    monkeypatch.setattr(C, "_layer_call", lambda entry, *args: (log.append(entry), call(entry, *args)))
+    for k, l in enumerate(a.fc_dist):
+        l.weight.register_post_accumulate_grad_hook(lambda p, k=k: log.append(k))
+    step(a, x, t)
+    events = [e for e in log if not isinstance(e, str) or "backward" in e]
+    assert events == [e for k in (3, 2, 1, 0) for e in ("snb_layer_backward_ws", k)]
+    by_layers(lambda: step(b, x, t))
+    for p, q in zip(a.parameters(), b.parameters()):
+        assert rel(p.grad.cpu().numpy(), q.grad.cpu().numpy()) < 1e-5
