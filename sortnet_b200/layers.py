@@ -78,7 +78,7 @@ def _plane_index(index, channels, hw):
     [S, 1, n] int32 form the mean-shift kernels take; None stays None."""
     if index is None:
         return None
-    if index.is_cuda and index.dtype == torch.int32:
+    if index.is_cuda and index.dtype == torch.int32 and not ops.tracing():
         return _C.plane_index(index.contiguous(), channels, hw)
     glob = _global_index(index, channels)
     if hw > 1:
@@ -483,7 +483,7 @@ class SortMLPModel(nn.Module):
 
     def _eval_plan(self, x, sort_eval):
         """The plan for an evaluation pass without gradients on x [B, pixels], or None."""
-        if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist):
+        if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist) or ops.tracing():
             return None
         if torch.is_grad_enabled() and (self.training or x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return None                      # a model in training mode draws masks, whatever its layers do

@@ -162,6 +162,23 @@ def test_hooks_and_overrides_keep_the_layers():
     assert Other(depth=3, width=16, input_dim=(1, 3, 3), num_classes=3)._plan() is None
 
 
+class CudaWeight:
+    """As far as ops._native looks at a weight."""
+    is_cuda = True
+
+
+def test_native_operators_stand_back_while_tracing():
+    from sortnet_b200 import ops
+    seen = []
+
+    def f(x):
+        seen.append(ops._native(CudaWeight()))
+        return x + 1
+    f(torch.ones(1))
+    torch.jit.trace(f, (torch.ones(1),), check_trace=False)
+    assert seen == [True, False]
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops

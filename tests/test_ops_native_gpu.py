@@ -103,3 +103,27 @@ def test_errors_and_counter():
         ops.norm_dist(x.transpose(0, 1).transpose(0, 1)[::2], w, INF)   # not contiguous
     with pytest.raises(AssertionError):
         ops.norm_dist(x, w[:, :8], INF)
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("grad", [False, True])
+def test_traced_calls_replay(grad):
+    """torch.jit.trace records the operators and replays them on other inputs."""
+    from sortnet_b200 import layers, ops
+    x, w, _ = operands(40, 12, 18)
+    x2, w2, _ = operands(40, 12, 18, seed=1)
+    for t in (x, w, x2, w2):
+        t.requires_grad_(grad)
+    calls = [lambda a, b: ops.norm_dist(a, b, INF), lambda a, b: ops.norm_dist(a, b, 3.0),
+             lambda a, b: ops.sort_neuron(a, b, q=0.8, truncate=4), lambda a, b: ops.bound_inf_dist(a, a + 0.1, b)[1]]
+    for f in calls:
+        traced = torch.jit.trace(f, (x, w), check_trace=False)
+        spoil = torch.full((40, 18, 1), 7.0, device="cuda")      # what an allocation that nobody fills finds
+        del spoil
+        assert torch.allclose(traced(x2, w2), f(x2, w2), rtol=1e-6)
+    index = layers.sample_mask(3, 2, 9, 0.8, "cuda", count=6)
+    other = layers.sample_mask(3, 2, 9, 0.8, "cuda", count=6)
+    traced = torch.jit.trace(lambda i: layers._plane_index(i, 18, 4), (index,), check_trace=False)
+    spoil = torch.full((3, 1, 48), 7, dtype=torch.int32, device="cuda")
+    del spoil
+    assert torch.equal(traced(other), layers._plane_index(other, 18, 4))
