@@ -483,7 +483,8 @@ class SortMLPModel(nn.Module):
 
     def _eval_plan(self, x, sort_eval):
         """The plan for an evaluation pass without gradients on x [B, pixels], or None."""
-        if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist) or ops.tracing():
+        if not (FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32) or any(l.training for l in self.fc_dist) \
+                or ops.tracing() or ops.forward_mode():
             return None
         if torch.is_grad_enabled() and (self.training or x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return None                      # a model in training mode draws masks, whatever its layers do
@@ -552,7 +553,7 @@ class SortMLPModel(nn.Module):
         x = x.reshape(x.size(0), -1)
         if FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32 and torch.is_grad_enabled() \
                 and not isinstance(self.scalar, torch.Tensor) and all(math.isinf(l.p) for l in self.fc_dist) \
-                and all(m.training for m in self.modules()):     # a layer in evaluation mode keeps its statistics
+                and not ops.tracing() and all(m.training for m in self.modules()):     # a layer in evaluation mode keeps its statistics
             if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
                 masks = self.draw_masks(x.size(0), x.device)
             plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)

@@ -179,6 +179,15 @@ def test_native_operators_stand_back_while_tracing():
     assert seen == [True, False]
 
 
+def test_native_operators_stand_back_in_forward_mode():
+    from torch.autograd import forward_ad
+    from sortnet_b200 import ops
+    assert ops._native(CudaWeight())
+    with forward_ad.dual_level():
+        assert not ops._native(CudaWeight())
+    assert ops._native(CudaWeight())
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops

@@ -127,3 +127,19 @@ def test_traced_calls_replay(grad):
     spoil = torch.full((3, 1, 48), 7, dtype=torch.int32, device="cuda")
     del spoil
     assert torch.equal(traced(other), layers._plane_index(other, 18, 4))
+
+
+def test_dual_tensors_are_refused():
+    """There is no forward-mode derivative; a result without a tangent would read as a zero one."""
+    from torch.autograd import forward_ad
+    from sortnet_b200 import ops
+    x, w, _ = operands(40, 12, 18)
+    x, w = x.detach(), w.detach()
+    with forward_ad.dual_level():
+        dual = forward_ad.make_dual(x, torch.ones_like(x))
+        for call in (lambda: ops.norm_dist(dual, w, INF), lambda: ops.norm_dist(dual, w, 3.0),
+                     lambda: ops.sort_neuron(dual, w, q=0.8, truncate=4), lambda: ops.bound_inf_dist(dual, dual, w),
+                     lambda: ops.norm_dist_dropout(dual, w, None, None, INF)):
+            with pytest.raises(RuntimeError, match="jvp"):
+                call()
+    assert ops.norm_dist(x, w, INF).shape == (40, 18, 1)
