@@ -84,7 +84,9 @@ void check(const Tensor& t, const char* name, at::ScalarType type = at::kFloat) 
 void check_input(const Tensor& x, const Tensor& w, const char* name = "input") {
     check(x, name);
     check(w, "weight");
-    TORCH_CHECK(x.dim() == 3 && w.dim() == 2, name, " must have shape [B, C, HW] and weight [CO, CI / groups]");
+    // further axes of size 1 are fine
+    TORCH_CHECK(x.dim() >= 3 && x.numel() == x.size(0) * x.size(1) * x.size(2) && w.dim() >= 2 && w.numel() == w.size(0) * w.size(1), name,
+                " must have shape [B, C, HW] and weight [CO, CI / groups]");
     TORCH_CHECK(x.device() == w.device(), "all tensors must be on the same device");
 }
 void check_list(const optional<Tensor>& t, const char* name, int64_t B, int64_t G, int64_t width, const Tensor& x) {

@@ -143,3 +143,17 @@ def test_dual_tensors_are_refused():
             with pytest.raises(RuntimeError, match="jvp"):
                 call()
     assert ops.norm_dist(x, w, INF).shape == (40, 18, 1)
+
+
+def test_further_axes_of_size_one():
+    """A 1 x 1 convolution's weight [CO, CI, 1, 1] and inputs [B, C, HW, 1]: gradients have the operands' shapes."""
+    from sortnet_b200 import ops
+    x, w, gy = operands(40, 12, 18, HW=4)
+    x4, w4 = x.detach().unsqueeze(-1).requires_grad_(), w.detach()[..., None, None].requires_grad_()
+    for call in (lambda a, b: ops.norm_dist(a, b, INF), lambda a, b: ops.norm_dist(a, b, 3.0),
+                 lambda a, b: ops.bound_inf_dist(a, a + 0.1, b)[1]):
+        def run(a=x4, b=w4):
+            y = call(a, b)
+            return [y, *torch.autograd.grad(y, (a, b), gy)]
+        compare(*both(run))
+        compare([t.reshape(-1) for t in run()], [t.reshape(-1) for t in run(x, w)])
