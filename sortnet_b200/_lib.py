@@ -135,7 +135,7 @@ def ops():
             from . import _ops as module
         except ImportError as exc:
             raise SortnetB200Error("_ops.so is not built (run `python -m sortnet_b200.build`): %s" % exc) from exc
-        module.init(LIB_PATH)
+        module.init(LIB_PATH, SortnetB200Error)
         _ops = module
     return _ops
 

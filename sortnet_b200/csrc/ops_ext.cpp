@@ -11,6 +11,8 @@
 
 #include <atomic>
 #include <cmath>
+#include <stdexcept>
+#include <string>
 
 #include "../../include/sortnet_b200.h"
 
@@ -46,7 +48,14 @@ struct Api {
 } api;
 std::atomic<long> launches{0};
 
-void init(const std::string& path) {
+// A status code of the library: arrives in Python as the exception class that _lib.check raises.
+struct LibraryError : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+PyObject* library_error = PyExc_RuntimeError;
+
+void init(const std::string& path, py::object error_class) {
+    library_error = error_class.release().ptr();             // kept for the life of the process
     void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
     TORCH_CHECK(h, "cannot load ", path, ": ", dlerror());
     auto get = [&](auto& f, const char* name) {
@@ -100,8 +109,9 @@ const int* list_ptr(const optional<Tensor>& t) { return t.has_value() ? t->data_
 
 void done(int rc, const char* what, int kernels) {
     if (rc) {
-        TORCH_CHECK(rc != SNB_STATUS_CUDA, what, " failed: ", api.status_string(rc), ": ", api.last_cuda_error(), " (status ", rc, ")");
-        TORCH_CHECK(false, what, " failed: ", api.status_string(rc), " (status ", rc, ")");
+        std::string why = api.status_string(rc);
+        if (rc == SNB_STATUS_CUDA) why += std::string(": ") + api.last_cuda_error();
+        throw LibraryError(std::string(what) + " failed: " + why + " (status " + std::to_string(rc) + ")");
     }
     launches.fetch_add(kernels, std::memory_order_relaxed);
 }
@@ -369,6 +379,13 @@ std::tuple<Tensor, Tensor> bound_sort_neuron(const Tensor& xl, const Tensor& xu,
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    py::register_exception_translator([](std::exception_ptr p) {
+        try {
+            if (p) std::rethrow_exception(p);
+        } catch (const LibraryError& e) {
+            PyErr_SetString(library_error, e.what());
+        }
+    });
     m.def("init", &init);
     m.def("dist", &dist);
     m.def("sort_neuron", &sort_neuron);

@@ -157,3 +157,20 @@ def test_further_axes_of_size_one():
             return [y, *torch.autograd.grad(y, (a, b), gy)]
         compare(*both(run))
         compare([t.reshape(-1) for t in run()], [t.reshape(-1) for t in run(x, w)])
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_status_codes_arrive_as_the_library_error(grad):
+    from sortnet_b200 import _lib, ops
+    x, w, _ = operands(8, 40, 5)
+    x.requires_grad_(grad), w.requires_grad_(grad)
+    for got in both_errors(lambda: ops.sort_neuron(x, w, q=0.8, truncate=30)):      # more values than the kernels take
+        assert type(got) is _lib.SortnetB200Error and "status 3" in str(got)
+
+
+def both_errors(fn):
+    def caught():
+        with pytest.raises(Exception) as info:
+            fn()
+        return info.value
+    return both(caught)
