@@ -447,14 +447,11 @@ extern "C" int snb_mlp_train_backward(const snb_mlp_layer* l, int depth, int B, 
     Cursor at{static_cast<char*>(scratch)};
     float* rows[2] = {at.take<float>((size_t)B * W), at.take<float>((size_t)B * W)};
     float* gt = at.take<float>((size_t)S * 32 * W);
-    static std::atomic<int> configured[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int most = (W + 3) / 4 * 16;
-    if (most > 48 * 1024 && configured[dev & 63].load(std::memory_order_acquire) < most) {
-        SNB_CUDA(cudaFuncSetAttribute(chain_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        configured[dev & 63].store(most, std::memory_order_release);
-    }
+    int most = 0;                                            // shared memory of the widest row of W
+    for (int k = 0; k < depth; k++) most = l[k].in > most ? l[k].in : most;
+    most = (most + 3) / 4 * 16;
+    if (most > MOST_SMEM) return SNB_ERR_UNSUPPORTED;
+    if (most > 48 * 1024) SNB_CUDA(allow_smem<chain_bwd_kernel, MOST_SMEM>());
     int lowest = 0;                                          // deepest layer that anybody wants a gradient from
     while (!grad_x && lowest < depth && !grad_w[lowest]) lowest++;
     if (lowest == depth && grad_bias) lowest = depth - 1;

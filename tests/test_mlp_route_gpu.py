@@ -166,3 +166,9 @@ def test_gradients_arrive_layer_by_layer_for_post_accumulate_hooks(monkeypatch):
     by_layers(lambda: step(b, x, t))
     for p, q in zip(a.parameters(), b.parameters()):
         assert rel(p.grad.cpu().numpy(), q.grad.cpu().numpy()) < 1e-5
+
+
+def test_head_wider_than_shared_memory():
+    """The backward's shared memory follows the layers' inputs; 60 000 classes are no more than 60 000 rows."""
+    a, b = nets(4, 512, (1, 16, 16), 60000, 0.8)
+    same_step(a, b, *batch(33, (1, 16, 16), 60000))
