@@ -26,7 +26,7 @@ namespace {
 constexpr int WARPS = 32, THREADS = WARPS * 32;
 constexpr int SCAN = 256;                   // pairs that a warp tests per step of its scan: eight loads of W in flight per lane
 constexpr int QUEUE = 160;                  // passed pairs of a warp: at most 15 left over + 128 new ones
-constexpr int SMEM = 227 * 1024;
+constexpr int SMEM = MOST_SMEM;
 constexpr float CUT_LOG2 = -40.0f;          // backward: terms below 2^CUT_LOG2 of the largest are left out
 
 __host__ __device__ constexpr int up_to(int n, int m) { return (n + m - 1) / m * m; }
@@ -557,13 +557,12 @@ int slab_bytes(const Slabs& sl, int entry, int test) {
     return (sl.chunk + 1) * entry + up_to(sl.chunk, SCAN) * test + WARPS * QUEUE * (int)sizeof(int2);
 }
 
-template <typename Args>
-cudaError_t launch(void (*kern)(Args), const Args& a, int smem, cudaStream_t st) {
-    // per device and small: set on every launch rather than remembered
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+template <auto KERN, typename Args>
+cudaError_t launch(const Args& a, int smem, cudaStream_t st) {
+    cudaError_t e = allow_smem<KERN, SMEM>();
     if (e != cudaSuccess) return e;
     const long long sms = sm_count(), want = (a.sl.total + WARPS - 1) / WARPS;
-    kern<<<(unsigned)(want < sms ? want : sms), THREADS, smem, st>>>(a);
+    KERN<<<(unsigned)(want < sms ? want : sms), THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -640,8 +639,8 @@ cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, cudaStream_t
     // maxima and sums lie side by side
     if (a.sl.chunks > 1 && (e = cudaMemsetAsync(a.mt, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - (char*)a.mt, st)) != cudaSuccess) return e;
     skip_columns<<<dim3((q.CI + 63) / 64, S), 256, 0, st>>>(q.x, q.B, q.CI, const_cast<float*>(a.xt), const_cast<float2*>(a.range));
-    if ((e = launch(skip_maxima, a, smem, st)) != cudaSuccess) return e;
-    if ((e = launch(skip_forward, a, smem, st)) != cudaSuccess) return e;
+    if ((e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
+    if ((e = launch<skip_forward>(a, smem, st)) != cudaSuccess) return e;
     skip_finish<<<dim3((q.CO + 63) / 64, S), 256, 0, st>>>(a.sum, a.mt, q.B, q.CO, q.p, y);
     return cudaGetLastError();
 }
@@ -658,7 +657,7 @@ cudaError_t lp_skip_backward(const LpProblem& q, const float* g, const float* y,
     skip_transpose<<<dim3((q.W_CI + 63) / 64, (q.W_CO + 63) / 64), 256, 0, st>>>(q.w, q.W_CO, q.W_CI, const_cast<float*>(a.wt));
     if (a.sl.chunks > 1 && (e = cudaMemsetAsync(a.gxt, 0, sizeof(float) * S * q.CI * 32, st)) != cudaSuccess) return e;
     const int smem = slab_bytes(a.sl, 256, 8);
-    if ((e = fine ? launch(skip_backward<true>, a, smem, st) : launch(skip_backward<false>, a, smem, st)) != cudaSuccess) return e;
+    if ((e = fine ? launch<skip_backward<true>>(a, smem, st) : launch<skip_backward<false>>(a, smem, st)) != cudaSuccess) return e;
     skip_rows<<<dim3((q.CI + 63) / 64, S), 256, 0, st>>>(a.gxt, q.B, q.CI, gx);
     return cudaGetLastError();
 }

@@ -13,6 +13,7 @@ constexpr int PAD = 8;              // lists are padded to a multiple of this
 constexpr int STEP = 4;             // list entries per bound ub
 constexpr int MAX_COLUMNS = 12288;  // widest row the filter takes: 512 threads x 6 x 4
 constexpr int BUCKETS = 32;
+constexpr int LONG_LIST = 512;       // most entries of a list
 
 struct PruneArgs {
     PruneProblem p;
@@ -1118,7 +1119,7 @@ int threshold_rank(const PruneProblem& p) {
 // List capacity: N(0,1)-like weights leave 35 columns on average for the maximum, 180 for ten values, 230 for rank 14.
 int list_capacity(const PruneProblem& p) {
     const int m = threshold_rank(p);
-    const int want = m <= 2 ? 192 : 512;
+    const int want = m <= 2 ? 192 : LONG_LIST;
     const int c = (p.W_CI + PAD - 1) / PAD * PAD;
     return c < want ? c : want;
 }
@@ -1162,22 +1163,14 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
     return off;
 }
 
-template <auto KERN>
-cudaError_t set_smem(int bytes) {
-    static std::atomic<int> configured[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (bytes <= 48 * 1024 || configured[dev & 63].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) configured[dev & 63].store(bytes, std::memory_order_release);
-    return e;
-}
-
 // Persistent grid: as many CTAs as fit (the shared memory of the stages limits them to two per SM for wide rows).
 template <int R, int NIT, int FT, int STAGES, bool VEC>
 cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
-    const int smem = STAGES * R * NIT * FT * 16 + R * (a.lcap * (2 * (int)sizeof(int2) + 2 * (int)sizeof(float)) + a.lcap / STEP * 2 * (int)sizeof(float));
-    cudaError_t e = set_smem<prune_filter<R, NIT, FT, STAGES, VEC>>(smem);
+    constexpr auto bytes = [](int lcap) {
+        return STAGES * R * NIT * FT * 16 + R * (lcap * (2 * (int)sizeof(int2) + 2 * (int)sizeof(float)) + lcap / STEP * 2 * (int)sizeof(float));
+    };
+    const int smem = bytes(a.lcap);
+    cudaError_t e = allow_smem<prune_filter<R, NIT, FT, STAGES, VEC>, bytes(LONG_LIST)>();
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_filter<R, NIT, FT, STAGES, VEC>, FT + 64 * R, smem);
@@ -1209,8 +1202,8 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st
 
 template <int NX, int KMAX, bool POS>
 cudaError_t run_sort(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st) {
-    const int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
-    cudaError_t e = set_smem<prune_sort<NX, KMAX, POS>>(smem);
+    constexpr int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
+    cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS>, smem>();
     if (e != cudaSuccess) return e;
     prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
     prune_fix_sort<NX, KMAX, POS><<<fix_grid, 256, 0, st>>>(a);

@@ -125,3 +125,26 @@ def test_values_that_are_no_numbers(p):
         ok = a.isfinite() & b.isfinite()
         assert p >= 49 or torch.equal(a.isfinite(), b.isfinite())
         assert not ok.any() or near(b[ok], a[ok]) < TOL
+
+
+def test_host_threads_with_different_sizes():
+    """Launches of the same kernel with more and with less shared memory from several threads."""
+    import threading
+    jobs = [(inputs(32, CI, CO, 1.0, CI), 60.0) for CI, CO in ((1344, 1600), (400, 1100), (3100, 705), (257, 1700))]
+    want = [calls(*args, p)[0] for args, p in jobs]
+    failures = []
+
+    def work(args, p, y_o):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(100):
+                    y, _, _ = calls(*args, p)
+                    torch.cuda.current_stream().synchronize()
+                    if near(y, y_o) > 1e-6:                         # sums in another order
+                        failures.append("values")
+        except Exception as exc:
+            failures.append(repr(exc))
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(args, p, y)) for (args, p), y in zip(jobs, want)]
+    [t.start() for t in threads], [t.join() for t in threads]
+    assert not failures, failures[:3]
