@@ -28,6 +28,7 @@ constexpr int SCAN = 256;                   // pairs that a warp tests per step 
 constexpr int QUEUE = 160;                  // passed pairs of a warp: at most 15 left over + 128 new ones
 constexpr int SMEM = MOST_SMEM;
 constexpr float CUT_LOG2 = -40.0f;          // backward: terms below 2^CUT_LOG2 of the largest are left out
+constexpr float CUT_MOST = 1.0f - 0x1p-19f; // a cut above this (p of 10^7 and more) would lie within the rounding of the tests
 
 __host__ __device__ constexpr int up_to(int n, int m) { return (n + m - 1) / m * m; }
 
@@ -600,7 +601,7 @@ size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a) {
         a->sl = slabs((int)S, q.CI, q.CO, 128, 12);
         a->B = q.B, a->CO = q.CO, a->CI = q.CI, a->W_CI = q.W_CI;
         // what is left out changes y by less than CI cut^p / p = 2^-27 of it
-        a->p = q.p, a->cut = exp2f(-(27.0f + log2f((float)q.CI / q.p)) / q.p);
+        a->p = q.p, a->cut = fminf(exp2f(-(27.0f + log2f((float)q.CI / q.p)) / q.p), CUT_MOST);
     }
     return at.off;
 }
@@ -618,7 +619,7 @@ size_t backward_layout(const LpProblem& q, char* base, BackwardArgs* a) {
         a->wt = wt, a->ci = q.ci, a->co = q.co, a->xt = xt, a->range = range, a->gr = gr, a->most = most, a->gxt = gxt;
         a->sl = slabs((int)S, q.CO, q.CI, 256, 8);
         a->B = q.B, a->CO = q.CO, a->CI = q.CI, a->W_CO = q.W_CO, a->W_CI = q.W_CI;
-        a->pm1 = q.p - 1.0f, a->cut = exp2f(CUT_LOG2 / (q.p - 1.0f));
+        a->pm1 = q.p - 1.0f, a->cut = fminf(exp2f(CUT_LOG2 / (q.p - 1.0f)), CUT_MOST);
     }
     return at.off;
 }

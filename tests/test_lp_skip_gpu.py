@@ -148,3 +148,19 @@ def test_host_threads_with_different_sizes():
     threads = [threading.Thread(target=work, args=(args, p, y)) for (args, p), y in zip(jobs, want)]
     [t.start() for t in threads], [t.join() for t in threads]
     assert not failures, failures[:3]
+
+
+@pytest.mark.parametrize("p", [1e6, 1e8, 3e8, 6e8])
+@pytest.mark.parametrize("shape", [(64, 1400, 800), (512, 300, 300)])
+@pytest.mark.parametrize("narrow", [False, True])
+def test_huge_finite_p(p, shape, narrow):
+    """y is the maximum up to CI^(1/p), of which nothing is left in fp32.  Up to p = 7e8 the rounding of |t| / M (1 - 2^-23 at
+    worst, to the power p above 2^-126) leaves a sum that is not zero, in the dense kernel as here.  narrow: rows that hardly
+    differ, so that the range of a column is no wider than the rounding of the test."""
+    x, w, g, ci, co = inputs(*shape, 1.0, 11)
+    if narrow:
+        x = x[:1] + 2e-7 * x
+    y, _, _ = calls(x, w, g, ci, co, p)
+    dense, _, _ = calls(x, w, g, ci, co, p, sparse=False)
+    top = (x[:, None, :] - w[None]).abs().amax(-1)
+    assert near(y, dense) < 1e-6 and float(((y - top).abs() / top).max()) < 1e-5
