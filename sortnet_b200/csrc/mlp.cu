@@ -287,7 +287,7 @@ PruneProblem layer_problem(const snb_mlp_layer* l, int k, int B, int tensors) {
 struct Scratch {
     char* zeroed;                  // fail counters and input ranges of every layer, one memset
     size_t zero_bytes;
-    unsigned* fail[MAX_DEPTH];
+    unsigned* counters[MAX_DEPTH];
     unsigned* hi[MAX_DEPTH];       // ranges of layer k's input
     unsigned* nlo[MAX_DEPTH];
     float* xt[2];
@@ -302,7 +302,7 @@ size_t scratch_layout(const snb_mlp_layer* l, int depth, int B, int tensors, boo
     Scratch v{};
     v.zeroed = base;
     for (int k = 0; k < depth; k++) {
-        v.fail[k] = at.take<unsigned>(1);
+        v.counters[k] = at.take<unsigned>(4);
         v.hi[k] = at.take<unsigned>(l[k].in);
         v.nlo[k] = at.take<unsigned>(l[k].in);
     }
@@ -317,7 +317,7 @@ size_t scratch_layout(const snb_mlp_layer* l, int depth, int B, int tensors, boo
     static int word = 0;
     for (int k = 0; k < depth; k++) {
         PruneProblem p = layer_problem(l, k, B, tensors);
-        p.xt = &some, p.hi = p.nlo = &none, p.fail_count = &none;
+        p.xt = &some, p.hi = p.nlo = &none, p.counters = &none;
         if (training) p.pos = &word;
         const size_t n = prune_workspace_bytes(p);
         most = n > most ? n : most;
@@ -408,9 +408,9 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
         const bool head = k == depth - 1;
         const int C = l[k].out;
         PruneProblem p = layer_problem(l, k, B, 1);
-        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.fail_count = sc.fail[k];
+        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.counters = sc.counters[k];
         p.pos = sv.pos[k], p.post = sv.post[k];
-        p.keep = l[k].kept_list ? sv.keep[k] : nullptr;
+        if (l[k].kept_list) p.keep = sv.keep[k], p.out_list = l[k].kept_list, p.out_kept = l[k].kept;
         if (head) {
             p.y = sc.d;
             p.bias = l[k].bias;
@@ -502,7 +502,7 @@ extern "C" int snb_mlp_eval_forward(const snb_mlp_layer* l, int depth, const flo
     SNB_CUDA(prune_prepare(prep, st));
     for (int k = 0; k < depth; k++) {
         PruneProblem p = layer_problem(l, k, B, tensors);
-        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.fail_count = sc.fail[k];
+        p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.counters = sc.counters[k];
         p.mean = l[k].running_mean, p.bias = l[k].bias;
         if (k == depth - 1) {
             p.y = y;

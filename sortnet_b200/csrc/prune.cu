@@ -18,7 +18,7 @@ constexpr int LONG_LIST = 512;       // most entries of a list
 struct PruneArgs {
     PruneProblem p;
     int S, NX, m, lcap;
-    unsigned* fail_count;
+    unsigned* counters;             // [FAILED], [OVERFLOWED], [GENERAL]
     const unsigned* hi;             // order codes of max(x), max(-x) per column; 0 = no value
     const unsigned* nlo;
     const float* xt;                // [S][W_CI][NX][32]
@@ -27,8 +27,23 @@ struct PruneArgs {
     float* tau;                     // [W_CO]
     float* ub;                      // [W_CO][lcap / STEP] largest U from this step of the list on
     int2* cand;                     // [W_CO][lcap] (column, bits of w)
-    int4* fail;                     // units (sub-batch, first output, mask of outputs) left to prune_fix
+    int4* fail;                     // units (sub-batch, first output, mask of outputs) left to prune_redo
+    // used when the layer is evaluated as a whole (dense_mode)
+    int ldr;                        // W_CI up to a multiple of 4
+    float* xr;                      // [tensors][S][32][ldr] the rows of xt, NaN past the last column
+    char* partial;                  // [results][S][CO][32] maxima, or keys (value, chunk of columns)
+    unsigned* tile_done;            // [S][blocks of 128 outputs] k-tiles merged
 };
+
+// Outputs left over by the walks; rows of W whose list overflowed; column lists that are not strictly ascending.
+enum { FAILED = 0, OVERFLOWED = 1, GENERAL = 2 };
+
+// Above this share of overflowed lists the layer is evaluated as a whole.  One output by itself costs about 12 times
+// its part of the whole (512 x 5120 x 5120 with positions).
+constexpr int DENSE_SHARE = 32;
+__device__ __forceinline__ bool dense_mode(const PruneArgs& a) {
+    return (a.p.ci && a.counters[GENERAL] != 0u) || (long long)a.counters[OVERFLOWED] * DENSE_SHARE > a.p.W_CO;
+}
 
 // ---- transpose + column ranges ----------------------------------------------------------------
 // CTA = 32 rows (one sub-batch) x 64 compact columns.  Bound by the traffic of x and xt and by launch latency.
@@ -66,7 +81,16 @@ __global__ void __launch_bounds__(256) prune_prep(const PrunePrep p) {
     for (int k = 0; k < 8; k++) {
         const int lc = warp + 8 * k;
         if (c0 + lc >= p.CI) break;
-        const int c = p.ci ? p.ci[(size_t)s * p.CI + c0 + lc] : c0 + lc;
+        int c = c0 + lc;
+        if (p.ci) {
+            const int* at = p.ci + (size_t)s * p.CI + c0 + lc;
+            c = *at;
+            const bool last = c0 + lc + 1 == p.CI;
+            if ((unsigned)c >= (unsigned)p.W_CI || (!last && at[1] <= c)) {  // not for the column order: see prune_redo.cuh
+                if (lane == 0) *p.general = 1u;
+                continue;
+            }
+        }
         unsigned hi = 0u, nlo = 0u;
 #pragma unroll
         for (int t = 0; t < NX; t++) {
@@ -116,6 +140,7 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
     __shared__ int hist[2 * R][BUCKETS];
     const int steps = (p.W_CO + R - 1) / R;
     const float nan = __int_as_float(0x7fc00000);
+    if (p.ci && a.counters[GENERAL] != 0u) return;           // no list will be walked
     if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
     __syncthreads();
 
@@ -340,6 +365,7 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
             if (j < p.W_CO) {
                 a.cnt[j] = n <= lcap ? n : -1;
                 a.tau[j] = t;
+                if (n > lcap) atomicAdd(a.counters + OVERFLOWED, 1u);
             }
             n_found[buf][r] = 0;
         }
@@ -545,7 +571,7 @@ __device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, 
 
 // 32 outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
 template <int NX, int NV, int NW>
-__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0) {
+__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0, unsigned skip = 0u) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* outs[NV];
     if (NX != 2) outs[0] = p.y;
@@ -571,6 +597,7 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
         for (int i = 0; i < 4; i++) {
             const int slot = warp * 4 + i;
             if (n0 + slot >= p.CO) break;
+            if ((skip >> slot) & 1u) continue;               // its values would widen the ranges
             float v[NV];
 #pragma unroll
             for (int t = 0; t < NV; t++) v[t] = tile[t][lane][slot];
@@ -585,6 +612,50 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
     }
 }
 
+// ---- a layer that will be evaluated as a whole ------------------------------------------------------
+// What prune_redo needs, shared out over the CTAs (s, n0) of the walk it replaces: the rows of x side by side again, empty
+// partial results (`bytes` per value; 0: none are kept), and the outputs that `keep` drops.  256 threads.
+template <int NX>
+__device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, int bytes) {
+    const PruneProblem& p = a.p;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = p.W_CI;
+    const float nan = __int_as_float(0x7fc00000);
+    if (!p.ci || a.counters[GENERAL] == 0u) {
+        const int pieces = (C + 7) / 8;
+        for (int k = (int)((long long)pieces * blockIdx.x / gridDim.x) + warp; k < (long long)pieces * (blockIdx.x + 1) / gridDim.x; k += 8)
+#pragma unroll
+            for (int t = 0; t < NX; t++) {
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int c = 8 * k + e;
+                    v[e] = c < C ? a.xt[(((size_t)s * C + c) * NX + t) * 32 + lane] : nan;
+                }
+                float4* dst = reinterpret_cast<float4*>(a.xr + ((size_t)(t * a.S + s) * 32 + lane) * a.ldr + 8 * k);
+                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                if (8 * k + 4 < a.ldr) dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+    }
+    if (bytes) {
+        const int quads = min(32, p.CO - n0) * 32 * bytes / 16;
+#pragma unroll
+        for (int t = 0; t < NX; t++) {
+            int4* part = reinterpret_cast<int4*>(a.partial + ((size_t)(t * a.S + s) * p.CO + n0) * 32 * bytes);
+            for (int k = tid; k < quads; k += 256) part[k] = make_int4(0, 0, 0, 0);
+        }
+        if (tid == 0 && n0 % 128 == 0) a.tile_done[(size_t)s * ((p.CO + 127) / 128) + n0 / 128] = 0u;
+    }
+    if (!p.keep) return;
+    for (int i = 0; i < 4; i++) {
+        const int n = n0 + warp * 4 + i, b = s * 32 + lane;
+        if (n >= p.CO || p.keep[(size_t)s * p.CO + n]) continue;
+        const float v[NX] = {};
+        emit_chain<NX>(p, s, n, v, 0u);
+        if (b < p.B && p.pos) p.pos[(size_t)b * p.CO + n] = (int)SNB_NO_GRAD_ID;
+        if (p.part && lane == 0) p.part[(size_t)s * p.CO + n] = 0.f;
+    }
+}
+
 // ---- list walks -----------------------------------------------------------------------------------
 // CTA = 32 outputs of one sub-batch, eight lanes per output, four rows per lane (one 16-byte load of xt per tensor and
 // column): a warp walks four lists side by side.  A step is STEP columns; the entries of the next step are fetched
@@ -593,7 +664,7 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
 // TRACK keeps, per row, the step that set the maximum; the word is made at the end from the step's columns.  A
 // later step that only equals the maximum (rare) sends the lane over the list once more for the lowest position.
 template <int NX, bool TRACK>
-__global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
+__global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneArgs a) {
     constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
     constexpr int WORDS = TRACK ? NX : 0;
     __shared__ float tile[NV + WORDS][32][33];
@@ -602,8 +673,7 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l = lane & 7;
     const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, slot = warp * 4 + g, n = n0 + slot;
     const float4* xt = reinterpret_cast<const float4*>(a.xt + (size_t)s * C * NX * 32) + l;
-    if (tid == 0) failed = 0u;
-    __syncthreads();
+    const bool dense = dense_mode(a);                        // its load and those of the list's head are in flight together
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
     const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
     const int cnt = wanted ? a.cnt[j] : 0;
@@ -611,6 +681,12 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
     const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
     const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
     const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
+    if (dense) {
+        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
+        return;
+    }
+    if (tid == 0) failed = 0u;
+    __syncthreads();
 
     float acc[NV][4];
     int at[TRACK ? NV : 1][TRACK ? 4 : 1];                   // step of the maximum, -1: at its floor
@@ -744,8 +820,8 @@ __global__ void __launch_bounds__(256) prune_max(const PruneArgs a) {
             for (int q = 0; q < 4; q++) tile[NV + (TRACK ? t : 0)][4 * l + q][slot] = __uint_as_float(word[TRACK ? t : 0][q]);
     }
     __syncthreads();
-    emit_tile<NX, NV, WORDS>(p, tile, s, n0);
-    if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
+    emit_tile<NX, NV, WORDS>(p, tile, s, n0, failed);
+    if (tid == 0 && failed) a.fail[atomicAdd(a.counters + FAILED, 1u)] = make_int4(s, n0, (int)failed, 0);
 }
 
 // Positions of one output whose K-th largest value is shared by several columns in some row: the entries of
@@ -780,7 +856,7 @@ __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, con
 // comes first.  Only where more columns share the K-th value than there is room for does the order of insertion
 // decide (ordered_positions).
 template <int NX, int KMAX, bool POS>
-__global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
+__global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
     constexpr int WALK = STEP;                               // entries per step: all insertion chains of a step are unrolled
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -791,6 +867,10 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
     const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, K = p.K;
     const bool live = s * 32 + lane < p.B;
     const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
+    if (dense_mode(a)) {
+        dense_prepare<NX>(a, s, n0, 0);
+        return;
+    }
     if (tid == 0) failed = 0u;
     __syncthreads();
 #pragma unroll 1
@@ -872,7 +952,7 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
         }
     }
     __syncthreads();
-    emit_tile<NX, NX, 0>(p, tile, s, n0);
+    emit_tile<NX, NX, 0>(p, tile, s, n0, failed);
     if (POS) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -884,219 +964,17 @@ __global__ void __launch_bounds__(256) prune_sort(const PruneArgs a) {
             }
         }
     }
-    if (tid == 0 && failed) a.fail[atomicAdd(a.fail_count, 1u)] = make_int4(s, n0, (int)failed, 0);
+    if (tid == 0 && failed) a.fail[atomicAdd(a.counters + FAILED, 1u)] = make_int4(s, n0, (int)failed, 0);
 }
 
-// ---- outputs whose list was not enough ------------------------------------------------------------
-// Persistent CTAs over the recorded units (32 outputs of one sub-batch, a mask of those to redo).  A few
-// outputs: the eight warps share the columns of one output.  Many: warp = four outputs side by side over all
-// columns, xt staged in shared memory for the eight warps, W read along rows by uniform 16-byte loads; that is the dense
-// evaluation of unprunable data, bound by the issue rate of subtract and max like any max-plus product.
-constexpr int FIX_K = 32;           // columns per stage
-constexpr int FIX_FEW = 4;
+}  // namespace
+}  // namespace snb
 
-template <int NX>
-__device__ __forceinline__ void fix_stage(const float* xt_s, float* sm, int k0, int C) {
-    const int n = min(FIX_K, C - k0) * NX * 8;               // 16-byte pieces; the columns of a sub-batch are contiguous
-    const float* src = xt_s + (size_t)k0 * NX * 32;
-    for (int k = threadIdx.x; k < n; k += 256) cp_async16(smem_u32(sm + k * 4), src + k * 4, 16);
-}
+#include "prune_redo.cuh"
 
-template <int NX, bool TRACK>
-__global__ void __launch_bounds__(256) prune_fix_max(const PruneArgs a) {
-    __shared__ __align__(16) float sm[2][FIX_K * NX * 32];
-    const PruneProblem& p = a.p;
-    const int count = (int)*a.fail_count;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = p.W_CI;
-    for (int unit = blockIdx.x; unit < count; unit += gridDim.x) {
-        const int4 f = a.fail[unit];
-        const int s = f.x, n0 = f.y;
-        const unsigned mask = (unsigned)f.z;
-        const float* xs = a.xt + (size_t)s * C * NX * 32;
-        const int* inv = p.ci ? a.inv + (size_t)s * C : nullptr;
-        const int b = s * 32 + lane;
-        const uint32_t floor_word = first_kept(p, s);
-        auto store = [&](const MaxState<NX, TRACK>& st, int n) {          // all lanes of a warp
-            if (p.yt || p.post) emit_chain<NX>(p, s, n, st.acc, TRACK ? st.word[0] : 0u);
-            if (p.part) {
-                float sum = 0.f;
-                for (int r = 0; r < min(32, p.B - s * 32); r++) sum += __shfl_sync(0xffffffffu, st.acc[0], r);
-                if (lane == 0) p.part[(size_t)s * p.CO + n] = sum;
-            }
-            if (b >= p.B) return;
-            const size_t o = (size_t)b * p.CO + n;
-            if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, st.acc[0], n);
-            if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, st.acc[NX - 2], n), p.yu[o] = shifted<NX>(p, st.acc[NX - 1], n);
-            if (TRACK && NX == 1) p.pos[o] = (int)st.word[0];
-            if (TRACK && NX == 2) p.posl[o] = (int)st.word[0], p.posu[o] = (int)st.word[TRACK ? NX - 1 : 0];
-        };
-        if (__popc(mask) <= FIX_FEW) {
-            unsigned todo = mask;
-            while (todo) {
-                const int n = n0 + __ffs(todo) - 1;
-                todo &= todo - 1;
-                const float* wr = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
-                MaxState<NX, TRACK> st;
-                st.init(floor_word);
-                for (int c0 = warp * 8; c0 < C; c0 += 64) {
-                    float v[8][NX], w[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        const int c = min(c0 + e, C - 1);            // a repeated column changes nothing
-                        w[e] = wr[c];
-#pragma unroll
-                        for (int t = 0; t < NX; t++) v[e][t] = xs[((size_t)c * NX + t) * 32 + lane];
-                    }
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        const int c = min(c0 + e, C - 1);
-                        st.add(v[e], w[e], TRACK ? (uint32_t)(inv ? inv[c] : c) : 0u);
-                    }
-                }
-                float* part = &sm[0][0];                             // [8 warps][NX (+ NX words)][32]
-                constexpr int PER = (TRACK ? 2 : 1) * NX;
-                static_assert(8 * PER * 32 <= 2 * FIX_K * NX * 32, "partial results fit the stages");
-                __syncthreads();
-#pragma unroll
-                for (int t = 0; t < NX; t++) {
-                    part[(warp * PER + t) * 32 + lane] = st.acc[t];
-                    if (TRACK) part[(warp * PER + NX + t) * 32 + lane] = __uint_as_float(st.word[TRACK ? t : 0]);
-                }
-                __syncthreads();
-                if (warp == 0) {
-                    for (int k = 1; k < 8; k++)
-#pragma unroll
-                        for (int t = 0; t < NX; t++) {
-                            const float v = part[(k * PER + t) * 32 + lane];
-                            if (TRACK) {
-                                const uint32_t wd = __float_as_uint(part[(k * PER + NX + t) * 32 + lane]);
-                                if (wd != SNB_NO_GRAD_ID)
-                                    take_word(v, wd & ~SNB_SIGN_BIT, (wd & SNB_SIGN_BIT) != 0, st.acc[t], st.word[TRACK ? t : 0]);
-                            } else {
-                                st.acc[t] = fmaxf(st.acc[t], v);
-                            }
-                        }
-                    store(st, n);
-                }
-            }
-            __syncthreads();
-            continue;
-        }
-        MaxState<NX, TRACK> st[4];
-        const float* wr[4];
-        const bool vec = (C % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.w) & 15u) == 0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int n = min(n0 + warp * 4 + i, p.CO - 1);
-            wr[i] = p.w + (size_t)(p.co ? p.co[(size_t)s * p.CO + n] : n) * C;
-            st[i].init(floor_word);
-        }
-        fix_stage<NX>(xs, sm[0], 0, C);
-        cp_async_commit();
-        for (int k0 = 0, cur = 0; k0 < C; k0 += FIX_K, cur ^= 1) {
-            cp_async_wait<0>();
-            __syncthreads();
-            if (k0 + FIX_K < C) fix_stage<NX>(xs, sm[cur ^ 1], k0 + FIX_K, C);
-            cp_async_commit();
-            const int kn = min(FIX_K, C - k0);
-            for (int k = 0; k < kn; k += 4) {
-                float w[4][4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (vec) {
-                        const float4 q = __ldg(reinterpret_cast<const float4*>(wr[i] + k0 + k));
-                        w[i][0] = q.x; w[i][1] = q.y; w[i][2] = q.z; w[i][3] = q.w;
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; e++) w[i][e] = __ldg(wr[i] + min(k0 + k + e, C - 1));
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    if (k + e >= kn) break;
-                    float v[NX];
-#pragma unroll
-                    for (int t = 0; t < NX; t++) v[t] = sm[cur][((k + e) * NX + t) * 32 + lane];
-                    const uint32_t idx = TRACK ? (uint32_t)(inv ? inv[k0 + k + e] : k0 + k + e) : 0u;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) st[i].add(v, w[i][e], idx);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int slot = warp * 4 + i;
-            if ((mask >> slot) & 1u) store(st[i], n0 + slot);
-        }
-        __syncthreads();
-    }
-}
+namespace snb {
 
-template <int NX, int KMAX, bool POS>
-__global__ void __launch_bounds__(256) prune_fix_sort(const PruneArgs a) {
-    __shared__ __align__(16) float sm[2][FIX_K * NX * 32];
-    const PruneProblem& p = a.p;
-    const int count = (int)*a.fail_count;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = p.W_CI, K = p.K;
-    for (int unit = blockIdx.x; unit < count; unit += gridDim.x) {
-        const int4 f = a.fail[unit];
-        const int s = f.x, n0 = f.y, b = s * 32 + lane;
-        const unsigned mask = (unsigned)f.z;
-        const float* xs = a.xt + (size_t)s * C * NX * 32;
-        for (int i = 0; i < 4; i++) {
-            const int slot = warp + 8 * i;                          // the CTA's warps do eight outputs at a time
-            if (((mask >> (8 * i)) & 0xffu) == 0u) continue;
-            const bool mine = (mask >> slot) & 1u;
-            const int n = min(n0 + slot, p.CO - 1);
-            const float* wr = p.w + (size_t)n * C;
-            const size_t o = (size_t)b * p.CO + n;
-            auto sweep = [&](auto&& body) {
-                __syncthreads();
-                fix_stage<NX>(xs, sm[0], 0, C);
-                cp_async_commit();
-                for (int k0 = 0, cur = 0; k0 < C; k0 += FIX_K, cur ^= 1) {
-                    cp_async_wait<0>();
-                    __syncthreads();
-                    if (k0 + FIX_K < C) fix_stage<NX>(xs, sm[cur ^ 1], k0 + FIX_K, C);
-                    cp_async_commit();
-                    if (!mine) continue;
-                    const int kn = min(FIX_K, C - k0);
-                    const float wl = lane < kn ? wr[k0 + lane] : 0.f;
-                    for (int k = 0; k < kn; k++) {
-                        float v[NX];
-#pragma unroll
-                        for (int t = 0; t < NX; t++) v[t] = sm[cur][(k * NX + t) * 32 + lane];
-                        body(v, __shfl_sync(0xffffffffu, wl, k), (uint32_t)(k0 + k));
-                    }
-                }
-            };
-            SortState<NX, KMAX> st;
-            st.init();
-            sweep([&](const float(&v)[NX], float w, uint32_t c) { st.add(v, w, c); });
-            if (mine) {
-                float v[NX];
-#pragma unroll
-                for (int t = 0; t < NX; t++) v[t] = st.result(t, K, p.q);
-                if (p.yt) emit_chain<NX>(p, s, n, v, 0u);
-                if (b < p.B) {
-                    if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, v[0], n);
-                    if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, v[NX - 2], n), p.yu[o] = shifted<NX>(p, v[NX - 1], n);
-                }
-            }
-            if constexpr (POS) {
-                PosList<KMAX> pl;
-                pl.init(st.top[0].kth(K));
-                sweep([&](const float(&v)[NX], float w, uint32_t c) { pl.add(v[0] - w, c, K); });
-                if (mine && b < p.B) {
-#pragma unroll
-                    for (int k = 0; k < KMAX; k++)
-                        if (k < K) p.pos[((size_t)k * p.B + b) * p.CO + n] = (int)pl.word[KMAX - 1 - k];
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
+namespace {
 
 // ---- host side ----------------------------------------------------------------------------------
 
@@ -1105,7 +983,7 @@ bool with_words(const PruneProblem& p) { return p.pos || p.posl; }
 
 // How many columns must reach the threshold.  Without masks K: the K-th largest value of every row then
 // reaches it by construction.  With column lists the m columns may all be missing from a sub-batch's list; m is chosen so
-// that this happens to about one output in 10^7 for random lists, and such outputs go to prune_fix.
+// that this happens to about one output in 10^7 for random lists, and such outputs go to prune_redo.
 int threshold_rank(const PruneProblem& p) {
     int m = p.K;
     if (p.ci || p.kept) {
@@ -1135,7 +1013,7 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
         return at;
     };
     const bool given = p.xt != nullptr;
-    char* zeroed = take(64 + (given ? 0 : 2 * up256(sizeof(unsigned) * C)));    // counter and ranges: one memset
+    char* zeroed = take(64 + (given ? 0 : 2 * up256(sizeof(unsigned) * C)));    // counters and ranges: one memset
     char* xt = take(given ? 0 : sizeof(float) * S * C * NX * 32);
     char* inv = take(p.ci ? sizeof(int) * S * C : 0);
     char* cnt = take(sizeof(int) * J);
@@ -1143,13 +1021,21 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
     char* ub = take(sizeof(float) * J * (lcap / STEP));
     char* cand = take(sizeof(int2) * J * lcap);
     char* fail = take(sizeof(int4) * S * ((p.CO + 31) / 32));
+    const size_t ldr = (C + 3) / 4 * 4;
+    char* xr = take(sizeof(float) * NX * S * 32 * ldr);
+    char* partial = take(p.K > 1 ? 0 : (with_words(p) ? 8 : 4) * NX * S * p.CO * 32);
+    char* tile_done = take(p.K > 1 ? 0 : sizeof(unsigned) * S * ((p.CO + 127) / 128));
     if (a) {
+        a->ldr = (int)ldr;
+        a->xr = reinterpret_cast<float*>(xr);
+        a->partial = partial;
+        a->tile_done = reinterpret_cast<unsigned*>(tile_done);
         a->p = p;
         a->S = (int)S;
         a->NX = (int)NX;
         a->m = threshold_rank(p);
         a->lcap = (int)lcap;
-        a->fail_count = p.fail_count ? p.fail_count : reinterpret_cast<unsigned*>(zeroed);
+        a->counters = p.counters ? p.counters : reinterpret_cast<unsigned*>(zeroed);
         a->hi = given ? p.hi : reinterpret_cast<unsigned*>(zeroed + 64);
         a->nlo = given ? p.nlo : reinterpret_cast<unsigned*>(zeroed + 64 + up256(sizeof(unsigned) * C));
         a->xt = given ? p.xt : reinterpret_cast<float*>(xt);
@@ -1193,20 +1079,38 @@ cudaError_t filter(const PruneArgs& a, cudaStream_t st) {
     return launch_filter<1, 6, 512, 2, VEC>(a, st);
 }
 
+// As many CTAs of the redo kernel as fit: with nothing to redo they read a few counters and end.
+template <auto KERN>
+cudaError_t redo_grid(int threads, int smem, int* grid) {
+    int per_sm = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, threads, smem);
+    *grid = sm_count() * (per_sm > 0 ? per_sm : 1);
+    return e;
+}
+
 template <int NX, bool TRACK>
-cudaError_t run_max(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st) {
+cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
+    constexpr int smem = redo_max_smem<NX, TRACK>();
+    cudaError_t e = allow_smem<prune_redo_max<NX, TRACK>, smem>();
+    if (e != cudaSuccess) return e;
+    int redo = 0;
+    if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
     prune_max<NX, TRACK><<<grid, 256, 0, st>>>(a);
-    prune_fix_max<NX, TRACK><<<fix_grid, 256, 0, st>>>(a);
+    prune_redo_max<NX, TRACK><<<redo, REDO_THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
 
 template <int NX, int KMAX, bool POS>
-cudaError_t run_sort(const PruneArgs& a, dim3 grid, int fix_grid, cudaStream_t st) {
+cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     constexpr int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
     cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS>, smem>();
     if (e != cudaSuccess) return e;
+    constexpr int again = redo_sort_smem<KMAX, POS>();
+    if ((e = allow_smem<prune_redo_sort<NX, KMAX, POS>, again>()) != cudaSuccess) return e;
+    int redo = 0;
+    if ((e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, again, &redo)) != cudaSuccess) return e;
     prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
-    prune_fix_sort<NX, KMAX, POS><<<fix_grid, 256, 0, st>>>(a);
+    prune_redo_sort<NX, KMAX, POS><<<redo, 256, again, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1236,7 +1140,7 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
     layout(p, static_cast<char*>(ws), &a);
     const size_t C = p.W_CI;
     cudaError_t e = cudaSuccess;
-    if (!p.fail_count) e = cudaMemsetAsync(a.fail_count, 0, 64 + (p.xt ? 0 : 2 * up256(sizeof(unsigned) * C)), st);
+    if (!p.counters) e = cudaMemsetAsync(a.counters, 0, 64 + (p.xt ? 0 : 2 * up256(sizeof(unsigned) * C)), st);
     if (e != cudaSuccess) return e;
     if (!p.xt) {
         // all bits set is a NaN: the dropped columns
@@ -1244,25 +1148,24 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
         if (p.ci && (e = cudaMemsetAsync(xt, 0xff, sizeof(float) * a.S * C * a.NX * 32, st)) != cudaSuccess) return e;
         PrunePrep q;
         q.x = p.x, q.xl = p.xl, q.xu = p.xu, q.ci = p.ci, q.inv = a.inv, q.B = p.B, q.CI = p.CI, q.W_CI = p.W_CI;
-        q.xt = xt, q.hi = const_cast<unsigned*>(a.hi), q.nlo = const_cast<unsigned*>(a.nlo);
+        q.xt = xt, q.hi = const_cast<unsigned*>(a.hi), q.nlo = const_cast<unsigned*>(a.nlo), q.general = a.counters + GENERAL;
         if ((e = prune_prepare(q, st)) != cudaSuccess) return e;
     }
     e = (C % 4 == 0) && aligned16(p.w) ? filter<true>(a, st) : filter<false>(a, st);
     if (e != cudaSuccess) return e;
     const dim3 grid((p.CO + 31) / 32, a.S);
-    const int fg = sm_count() * 2;
     if (p.K == 1) {
         const bool track = with_words(p);
-        if (a.NX == 1) return track ? run_max<1, true>(a, grid, fg, st) : run_max<1, false>(a, grid, fg, st);
-        if (a.NX == 2) return track ? run_max<2, true>(a, grid, fg, st) : run_max<2, false>(a, grid, fg, st);
-        return run_max<3, false>(a, grid, fg, st);
+        if (a.NX == 1) return track ? run_max<1, true>(a, grid, st) : run_max<1, false>(a, grid, st);
+        if (a.NX == 2) return track ? run_max<2, true>(a, grid, st) : run_max<2, false>(a, grid, st);
+        return run_max<3, false>(a, grid, st);
     }
     if (p.K <= 10) {
-        if (a.NX == 1) return p.pos ? run_sort<1, 10, true>(a, grid, fg, st) : run_sort<1, 10, false>(a, grid, fg, st);
-        return a.NX == 2 ? run_sort<2, 10, false>(a, grid, fg, st) : run_sort<3, 10, false>(a, grid, fg, st);
+        if (a.NX == 1) return p.pos ? run_sort<1, 10, true>(a, grid, st) : run_sort<1, 10, false>(a, grid, st);
+        return a.NX == 2 ? run_sort<2, 10, false>(a, grid, st) : run_sort<3, 10, false>(a, grid, st);
     }
-    if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, grid, fg, st) : run_sort<1, 25, false>(a, grid, fg, st);
-    return a.NX == 2 ? run_sort<2, 25, false>(a, grid, fg, st) : run_sort<3, 25, false>(a, grid, fg, st);
+    if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, grid, st) : run_sort<1, 25, false>(a, grid, st);
+    return a.NX == 2 ? run_sort<2, 25, false>(a, grid, st) : run_sort<3, 25, false>(a, grid, st);
 }
 
 }  // namespace snb

@@ -13,10 +13,10 @@
 //   prune_max / prune_sort   one warp per (sub-batch, output), lane = row: walks the list until no
 //                  remaining U can change any row, and CHECKS that every row's result (its K-th
 //                  largest value for the sort neuron) reaches tau.  Outputs that do not are recorded;
-//   prune_fix      evaluates the recorded outputs over all columns.
-// The result is exact whatever the data: the thresholds only decide how many columns are read.  Data
-// that cannot be pruned (rows of W whose entries all have about the same distance to the input)
-// ends in prune_fix, a dense kernel.
+//   prune_redo     evaluates the recorded outputs over all columns.
+// The result is exact whatever the data: the thresholds only decide how many columns are read.  Where
+// too many lists overflow (inputs spread as wide as the weights), nothing is walked and prune_redo evaluates
+// the layer as a whole with register tiles.
 #pragma once
 #include "common.cuh"
 #include "launch.h"
@@ -58,9 +58,11 @@ struct PruneProblem {
     float* part = nullptr;
     int* post = nullptr;
     const unsigned char* keep = nullptr;
+    const int* out_list = nullptr;      // [S][out_kept] the outputs that `keep` keeps (null without `keep`)
+    int out_kept = 0;
     const float* mean = nullptr;
     const float* bias = nullptr;
-    unsigned* fail_count = nullptr;     // a zeroed counter of the caller's, or null: one in the workspace
+    unsigned* counters = nullptr;       // four zeroed counters of the caller's, or null: those in the workspace
     const int* kept_list = nullptr;     // [S][kept] kept columns: the first one is the position of an output at its floor
 };
 
@@ -77,6 +79,7 @@ struct PrunePrep {
     float* xt = nullptr;
     unsigned* hi = nullptr;     // zeroed before
     unsigned* nlo = nullptr;
+    unsigned* general = nullptr;    // with ci: set to 1 when a list is not strictly ascending or leaves [0, W_CI)
 };
 cudaError_t prune_prepare(const PrunePrep& q, cudaStream_t st);
 
