@@ -38,11 +38,8 @@ struct PruneArgs {
 // Outputs left over by the walks; rows of W whose list overflowed; column lists that are not strictly ascending.
 enum { FAILED = 0, OVERFLOWED = 1, GENERAL = 2 };
 
-// Above this share of overflowed lists the layer is evaluated as a whole.  One output by itself costs about 12 times
-// its part of the whole (512 x 5120 x 5120 with positions).
-constexpr int DENSE_SHARE = 32;
 __device__ __forceinline__ bool dense_mode(const PruneArgs& a) {
-    return (a.p.ci && a.counters[GENERAL] != 0u) || (long long)a.counters[OVERFLOWED] * DENSE_SHARE > a.p.W_CO;
+    return (a.p.ci && a.counters[GENERAL] != 0u) || prune_gives_up(a.counters[OVERFLOWED], a.p.W_CO);
 }
 
 // ---- transpose + column ranges ----------------------------------------------------------------
@@ -673,7 +670,10 @@ __global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneAr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l = lane & 7;
     const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, slot = warp * 4 + g, n = n0 + slot;
     const float4* xt = reinterpret_cast<const float4*>(a.xt + (size_t)s * C * NX * 32) + l;
-    const bool dense = dense_mode(a);                        // its load and those of the list's head are in flight together
+    if (dense_mode(a)) {
+        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
+        return;
+    }
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
     const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
     const int cnt = wanted ? a.cnt[j] : 0;
@@ -681,10 +681,6 @@ __global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneAr
     const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
     const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
     const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
-    if (dense) {
-        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
-        return;
-    }
     if (tid == 0) failed = 0u;
     __syncthreads();
 
@@ -868,7 +864,7 @@ __global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneA
     const bool live = s * 32 + lane < p.B;
     const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
     if (dense_mode(a)) {
-        dense_prepare<NX>(a, s, n0, 0);
+        if (!POS) dense_prepare<NX>(a, s, n0, 0);            // positions: sort_positions_if reads the rows as they came
         return;
     }
     if (tid == 0) failed = 0u;
@@ -1105,13 +1101,12 @@ cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     constexpr int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
     cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS>, smem>();
     if (e != cudaSuccess) return e;
-    constexpr int again = redo_sort_smem<KMAX, POS>();
-    if ((e = allow_smem<prune_redo_sort<NX, KMAX, POS>, again>()) != cudaSuccess) return e;
     int redo = 0;
-    if ((e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, again, &redo)) != cudaSuccess) return e;
+    if ((e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo)) != cudaSuccess) return e;
     prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
-    prune_redo_sort<NX, KMAX, POS><<<redo, 256, again, st>>>(a);
-    return cudaGetLastError();
+    prune_redo_sort<NX, KMAX, POS><<<redo, 256, 0, st>>>(a);
+    if ((e = cudaGetLastError()) != cudaSuccess || !POS) return e;
+    return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
 }
 
 }  // namespace

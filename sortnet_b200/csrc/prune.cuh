@@ -92,6 +92,13 @@ __device__ __forceinline__ float decode(unsigned e) {   // 0 -> NaN
     return __uint_as_float((e & 0x80000000u) ? (e ^ 0x80000000u) : ~e);
 }
 
+// Above 1 / 32 of overflowed lists the layer is evaluated as a whole: one output by itself costs about 12 times its part
+// of the whole (512 x 5120 x 5120 with positions).
+__host__ __device__ __forceinline__ bool prune_gives_up(unsigned overflowed, int W_CO) { return (long long)overflowed * 32 > W_CO; }
+
+// y and pos of a sort neuron by the kernels of sort_neuron.cu if the layer is to be evaluated as a whole, nothing otherwise.
+cudaError_t sort_positions_if(const PruneProblem& p, const unsigned* overflowed, cudaStream_t st);
+
 // Whether the pruned evaluation is the faster one for this problem (sizes only), and its scratch.
 bool prune_applies(const PruneProblem& p);
 size_t prune_workspace_bytes(const PruneProblem& p);

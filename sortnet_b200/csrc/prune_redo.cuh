@@ -7,6 +7,8 @@
 // over all CTAs along (tile, k-tile) pairs.  Column lists that are not strictly ascending take that way too, in the order
 // of the list: position, not column, decides their ties, and a column may come twice.
 #pragma once
+#include <type_traits>
+
 #include "tile.cuh"
 
 namespace snb {
@@ -112,99 +114,168 @@ __device__ __forceinline__ void* part_of(const PruneArgs& a, int t) {
     return a.partial + (size_t)t * a.S * a.p.CO * 32 * (TRACK ? 8 : 4);
 }
 
-// Words and stores of 128 outputs whose partial results are complete, 32 at a time through shared memory `sm`.  Warp = eight of
-// the 32 outputs, lane = row; the words of an output: the chunks of its rows are read once more, a lane per column, for as many
-// rows at once as registers allow (the loads are all this waits for).
-template <int NX, bool TRACK>
-__device__ __noinline__ void dense_emit(const PruneArgs& a, const DenseLayer& d, int s, int block, float* sm) {
-    constexpr int SLOTS = 32 / (REDO_THREADS / 32), AHEAD = NX == 1 ? 32 : 16, NW = TRACK ? NX : 0;
-    const PruneProblem& p = a.p;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = p.W_CI, rows = min(32, p.B - s * 32);
-    const int* inv = p.ci && !d.gather ? a.inv + (size_t)s * C : nullptr;
-    const int* list = d.gather ? p.ci + (size_t)s * p.CI : nullptr;
-    float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(sm);           // [NX values, NW words][row][output]
-    const int stride = d.gather ? p.CI : a.ldr, last = d.K - 1;
-    const float* xs[NX];
+// Words of PAIR neighbouring outputs (tensor t) from the chunks of their rows: in `words` the low halves of the keys (0: at
+// the floor) are replaced by place in the chunk | sign.
+template <int NX>
+struct Rescan {
+    const float* xs[NX];            // rows of the sub-batch
+    int stride, rows, last;         // last: the last column
+    const int* list;                // columns of W, or null
+    template <int T>
+    __device__ __forceinline__ static bool holds(float x, float u, float w, float want, bool* negative) {
+        if (NX == 1) {
+            *negative = x - w < 0.f;
+            return fabsf(x - w) == want;
+        }
+        const float t1 = w - x, t2 = u - w;
+        *negative = !(t1 <= t2);
+        return (T == 0 ? fmaxf(-t1, -t2) : fmaxf(t1, t2)) == want;
+    }
+    // four lanes per row, eight columns each by 16-byte loads: rows 8 e + lane / 4 of SETS e at a time
+    template <int T, int PAIR, int SETS>
+    __device__ __forceinline__ void vectors(const float* const (&wr)[PAIR], const float (&value)[PAIR], uint32_t (&low)[PAIR]) const {
+        const int lane = threadIdx.x & 31;
+        uint32_t found[PAIR];
 #pragma unroll
-    for (int u = 0; u < NX; u++) xs[u] = d.gather ? p.x + (size_t)s * 32 * p.CI : a.xr + (size_t)(u * a.S + s) * 32 * a.ldr;
-    for (int base = block * 128; base < min(d.N, block * 128 + 128); base += 32) {
-        __syncthreads();
-        float v[SLOTS][NX];
-        unsigned low[TRACK ? SLOTS : 1][TRACK ? NX : 1];
-#pragma unroll
-        for (int i = 0; i < SLOTS; i++)
-#pragma unroll
-            for (int t = 0; t < NX; t++) {
-                const size_t at = ((size_t)s * p.CO + min(base + warp * SLOTS + i, d.N - 1)) * 32 + lane;
-                if (TRACK) {
-                    const unsigned long long key = __ldcg(static_cast<const unsigned long long*>(part_of<TRACK>(a, t)) + at);
-                    v[i][t] = __uint_as_float((unsigned)(key >> 32));
-                    low[TRACK ? i : 0][TRACK ? t : 0] = (unsigned)key;
-                } else {
-                    v[i][t] = __ldcg(static_cast<const float*>(part_of<TRACK>(a, t)) + at);
-                }
-            }
-#pragma unroll
-        for (int i = 0; i < SLOTS; i++)
-#pragma unroll
-            for (int t = 0; t < NX; t++) tile[t][lane][warp * SLOTS + i] = v[i][t];
-        if (TRACK) {
+        for (int o = 0; o < PAIR; o++) found[o] = 0u;
 #pragma unroll 1
-            for (int i = 0; i < SLOTS; i++) {
-                const int n = base + warp * SLOTS + i;
-                if (n >= d.N) break;
-                const float* wr = p.w + (size_t)dense_row(p, s, dense_output(p, s, n)) * C;
-#pragma unroll 1
-                for (int t = 0; t < NX; t++) {
-                    unsigned lw = low[0][0];
+        for (int e0 = 0; e0 < 4; e0 += SETS) {
+            float4 x[PAIR][SETS][NX][2], w[PAIR][SETS][2];
+            int at[PAIR][SETS][2];
 #pragma unroll
-                    for (int k = 0; k < SLOTS; k++)
+            for (int o = 0; o < PAIR; o++)
+#pragma unroll
+                for (int e = 0; e < SETS; e++) {
+                    const int r = 8 * (e0 + e) + (lane >> 2);
+                    const unsigned q = __shfl_sync(0xffffffffu, low[o], r);
+                    const int c = (q ? (int)(0xffffffffu - q) * 32 : 0) + 8 * (lane & 3);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        at[o][e][h] = min(c + 4 * h, last - 3);      // past the end: the last columns once more
+                        w[o][e][h] = *reinterpret_cast<const float4*>(wr[o] + at[o][e][h]);
 #pragma unroll
                         for (int u = 0; u < NX; u++)
-                            if (k == i && u == t) lw = low[TRACK ? k : 0][TRACK ? u : 0];
-                    const float value = tile[t][lane][warp * SLOTS + i];
-                    uint32_t wd = NX == 1 ? first_kept(p, s) : t == 0 ? SNB_NO_GRAD_ID : 0u;      // at its floor
-                    auto rescan = [&](auto column) {
-#pragma unroll 1
-                        for (int r0 = 0; r0 < rows; r0 += AHEAD) {
-                            float x[AHEAD][NX], w[AHEAD];
-#pragma unroll
-                            for (int e = 0; e < AHEAD; e++) {        // past the end: the last column once more
-                                const unsigned q = __shfl_sync(0xffffffffu, lw, r0 + e);
-                                const int c = min(q ? (int)(0xffffffffu - q) * 32 + lane : 0, last);
-                                w[e] = wr[column(c)];
-#pragma unroll
-                                for (int u = 0; u < NX; u++) x[e][u] = xs[u][(size_t)min(r0 + e, rows - 1) * stride + c];
-                            }
-#pragma unroll
-                            for (int e = 0; e < AHEAD; e++) {
-                                const float want = __shfl_sync(0xffffffffu, value, r0 + e);
-                                float got;
-                                bool negative;
-                                if (NX == 1) {
-                                    got = fabsf(x[e][0] - w[e]);
-                                    negative = x[e][0] - w[e] < 0.f;
-                                } else {
-                                    const float t1 = w[e] - x[e][0], t2 = x[e][NX - 1] - w[e];
-                                    got = t == 0 ? fmaxf(-t1, -t2) : fmaxf(t1, t2);
-                                    negative = !(t1 <= t2);
-                                }
-                                const unsigned hits = __ballot_sync(0xffffffffu, got == want);
-                                const unsigned signs = __ballot_sync(0xffffffffu, negative);
-                                const int k = __ffs(hits) - 1;
-                                const uint32_t here = (uint32_t)k | ((signs >> (k & 31)) & 1u ? SNB_SIGN_BIT : 0u);
-                                if (lane == r0 + e && lw) wd = here;
-                            }
-                        }
-                    };
-                    if (list) rescan([&](int c) { return list[c]; });
-                    else rescan([](int c) { return c; });
-                    if (lw) {                                // place in the chunk -> position
-                        const int col = (int)(0xffffffffu - lw) * 32 + (int)(wd & 31u);
-                        wd = (uint32_t)(inv ? inv[min(col, last)] : col) | (wd & SNB_SIGN_BIT);
+                            x[o][e][u][h] = *reinterpret_cast<const float4*>(xs[u] + (size_t)min(r, rows - 1) * stride + at[o][e][h]);
                     }
-                    tile[NX + (TRACK ? t : 0)][lane][warp * SLOTS + i] = __uint_as_float(wd);
                 }
+#pragma unroll
+            for (int o = 0; o < PAIR; o++)
+#pragma unroll
+                for (int e = 0; e < SETS; e++) {
+                    const float want = __shfl_sync(0xffffffffu, value[o], 8 * (e0 + e) + (lane >> 2));
+                    unsigned best = 0xffffffffu;                     // column << 1 | negative
+#pragma unroll
+                    for (int k = 7; k >= 0; k--) {
+                        auto of = [&](const float4& v) { return (k & 3) == 0 ? v.x : (k & 3) == 1 ? v.y : (k & 3) == 2 ? v.z : v.w; };
+                        bool negative;
+                        if (holds<T>(of(x[o][e][0][k >> 2]), of(x[o][e][NX - 1][k >> 2]), of(w[o][e][k >> 2]), want, &negative))
+                            best = (unsigned)(at[o][e][k >> 2] + (k & 3)) << 1 | (negative ? 1u : 0u);
+                    }
+                    best = min(best, __shfl_xor_sync(0xffffffffu, best, 1));
+                    best = min(best, __shfl_xor_sync(0xffffffffu, best, 2));
+                    best = __shfl_sync(0xffffffffu, best, 4 * (lane & 7));
+                    if ((lane >> 3) == e0 + e) found[o] = ((best >> 1) & 31u) | (best & 1u ? SNB_SIGN_BIT : 0u);
+                }
+        }
+#pragma unroll
+        for (int o = 0; o < PAIR; o++) low[o] = found[o];
+    }
+    // a lane per column, AHEAD rows at a time
+    template <int T, int AHEAD>
+    __device__ __forceinline__ uint32_t columns(const float* wr, float value, uint32_t low) const {
+        const int lane = threadIdx.x & 31;
+        uint32_t found = 0u;
+#pragma unroll 1
+        for (int r0 = 0; r0 < rows; r0 += AHEAD) {
+            float x[AHEAD][NX], w[AHEAD];
+#pragma unroll
+            for (int e = 0; e < AHEAD; e++) {                        // past the end: the last column once more
+                const unsigned q = __shfl_sync(0xffffffffu, low, r0 + e);
+                const int c = min(q ? (int)(0xffffffffu - q) * 32 + lane : 0, last);
+                w[e] = wr[list ? list[c] : c];
+#pragma unroll
+                for (int u = 0; u < NX; u++) x[e][u] = xs[u][(size_t)min(r0 + e, rows - 1) * stride + c];
+            }
+#pragma unroll
+            for (int e = 0; e < AHEAD; e++) {
+                bool negative;
+                const bool hit = holds<T>(x[e][0], x[e][NX - 1], w[e], __shfl_sync(0xffffffffu, value, r0 + e), &negative);
+                const unsigned hits = __ballot_sync(0xffffffffu, hit), signs = __ballot_sync(0xffffffffu, negative);
+                const int k = (__ffs(hits) - 1) & 31;
+                if (lane == r0 + e) found = (uint32_t)k | ((signs >> k) & 1u ? SNB_SIGN_BIT : 0u);
+            }
+        }
+        return found;
+    }
+};
+
+// Words and stores of 128 outputs whose partial results are complete, 32 at a time through shared memory `sm`.  Warp = eight of
+// the 32 outputs, lane = row; the words of an output: the chunks of its rows are read once more, by four lanes per row where
+// 16-byte loads are allowed, else by a lane per column.  Bound by the loads in flight (512 x 5120 x 5120: a lane per column
+// 0.6 ms, four lanes per row 0.25 ms on top of 0.84).
+template <int NX, bool TRACK>
+__device__ __noinline__ void dense_emit(const PruneArgs& a, const DenseLayer& d, int s, int block, float* sm) {
+    constexpr int SLOTS = 32 / (REDO_THREADS / 32), NW = TRACK ? NX : 0;
+    const PruneProblem& p = a.p;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = p.W_CI, rows = min(32, p.B - s * 32);
+    float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(sm);           // [NX values, NW words][row][output]
+    for (int base = block * 128; base < min(d.N, block * 128 + 128); base += 32) {
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < NX; t++)
+#pragma unroll
+            for (int i = 0; i < SLOTS; i++) {
+                const int slot = warp * SLOTS + i;
+                const size_t at = ((size_t)s * p.CO + min(base + slot, d.N - 1)) * 32 + lane;
+                if (TRACK) {
+                    const unsigned long long key = __ldcg(static_cast<const unsigned long long*>(part_of<TRACK>(a, t)) + at);
+                    tile[t][lane][slot] = __uint_as_float((unsigned)(key >> 32));
+                    tile[NX + t][lane][slot] = __uint_as_float((unsigned)key);
+                } else {
+                    tile[t][lane][slot] = __ldcg(static_cast<const float*>(part_of<TRACK>(a, t)) + at);
+                }
+            }
+        if constexpr (TRACK) {
+            constexpr int PAIR = NX == 1 ? 2 : 1;
+            const int* inv = p.ci && !d.gather ? a.inv + (size_t)s * C : nullptr;
+            Rescan<NX> scan;
+            scan.stride = d.gather ? p.CI : a.ldr, scan.rows = rows, scan.last = d.K - 1;
+            scan.list = d.gather ? p.ci + (size_t)s * p.CI : nullptr;
+#pragma unroll
+            for (int u = 0; u < NX; u++)
+                scan.xs[u] = d.gather ? p.x + (size_t)s * 32 * p.CI : a.xr + (size_t)(u * a.S + s) * 32 * a.ldr;
+            auto words = [&](auto which, int i) {            // of the outputs i, i + 1 of the warp
+                constexpr int T = decltype(which)::value;
+                const float* wr[PAIR];
+                float value[PAIR];
+                uint32_t low[PAIR], place[PAIR];
+#pragma unroll
+                for (int o = 0; o < PAIR; o++) {
+                    const int slot = warp * SLOTS + i + o;
+                    wr[o] = p.w + (size_t)dense_row(p, s, dense_output(p, s, min(base + slot, d.N - 1))) * C;
+                    value[o] = tile[T][lane][slot];
+                    place[o] = low[o] = __float_as_uint(tile[NX + T][lane][slot]);
+                }
+                if (d.vec) {
+                    scan.template vectors<T, PAIR, NX == 1 ? 4 : 2>(wr, value, place);
+                } else {
+#pragma unroll
+                    for (int o = 0; o < PAIR; o++) place[o] = scan.template columns<T, 16>(wr[o], value[o], place[o]);
+                }
+#pragma unroll
+                for (int o = 0; o < PAIR; o++) {
+                    uint32_t word = NX == 1 ? first_kept(p, s) : T == 0 ? SNB_NO_GRAD_ID : 0u;       // at its floor
+                    if (low[o]) {
+                        const int col = min((int)(0xffffffffu - low[o]) * 32 + (int)(place[o] & 31u), d.K - 1);
+                        word = (uint32_t)(inv ? inv[col] : col) | (place[o] & SNB_SIGN_BIT);
+                    }
+                    tile[NX + T][lane][warp * SLOTS + i + o] = __uint_as_float(word);
+                }
+            };
+#pragma unroll 1
+            for (int i = 0; i < SLOTS; i += PAIR) {
+                words(std::integral_constant<int, 0>(), i);
+                if constexpr (NX == 2) words(std::integral_constant<int, 1>(), i);
             }
         }
         __syncthreads();
@@ -614,15 +685,14 @@ __global__ void __launch_bounds__(REDO_THREADS, 2) prune_redo_max(const __grid_c
 
 // ---- sort neurons ------------------------------------------------------------------------------------
 // A whole layer: unit = 32 rows x 32 outputs, thread 2 x 2 (rows ty + 16 i, outputs tx + 16 j) with its lists in registers.
-// Bound by the insertion chains.  Values of the point first, then of the box, then (POS) a second sweep for the positions:
-// with the K-th value known few columns are looked at.
+// Bound by the insertion chains.  Values of the point first, then of the box.
 template <int NT>
 __device__ __forceinline__ void sort_stage(const PruneArgs& a, float* dst, int s, int t, int kt) {
     stage_dense_vec<32, NT>(dst, a.xr + (size_t)t * a.S * 32 * a.ldr, s * 32, a.S * 32, a.ldr, kt * BK, a.ldr, threadIdx.x);
 }
 
-// body(column, x of two rows x four columns [, u], w of two outputs x four columns) over all columns in order; rows of xr in
-// tensor t0 (and t0 + 1).  Past the last column the operands are NaN or all zero: neither enters a list.
+// body(x of two rows [, u], w of two outputs) for every column; rows of xr in tensor t0 (and t0 + 1).  Past the last column the
+// operands are NaN or all zero: neither enters a list.
 template <bool BOX, typename F>
 __device__ __forceinline__ void sort_sweep(const PruneArgs& a, float* sm, int s, int n0, int t0, F&& body) {
     constexpr int NT = 256, TILE = 2 * 32 * LDS;
@@ -647,41 +717,31 @@ __device__ __forceinline__ void sort_sweep(const PruneArgs& a, float* sm, int s,
         const float* xr = sm + (kt & 1) * 32 * LDS + ty * LDS;
         const float* wr = sm + 2 * TILE + (kt & 1) * 32 * LDS + tx * LDS;
 #pragma unroll 1
-        for (int k = 0; k < BK; k += 4) {
-            float4 x[2], u[2], w[2];
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                x[i] = *reinterpret_cast<const float4*>(xr + 16 * i * LDS + k);
-                if (BOX) u[i] = *reinterpret_cast<const float4*>(xr + TILE + 16 * i * LDS + k);
-                w[i] = *reinterpret_cast<const float4*>(wr + 16 * i * LDS + k);
-            }
-            body(kt * BK + k, x, u, w);
+        for (int k = 0; k < BK; k++) {
+            const float x[2] = {xr[k], xr[16 * LDS + k]}, w[2] = {wr[k], wr[16 * LDS + k]};
+            const float u[2] = {BOX ? xr[TILE + k] : 0.f, BOX ? xr[TILE + 16 * LDS + k] : 0.f};
+            body(x, u, w);
         }
     }
 }
-__device__ __forceinline__ void minus4(float (&d)[4], const float4& a, const float4& b) {
-    d[0] = a.x - b.x, d[1] = a.y - b.y, d[2] = a.z - b.z, d[3] = a.w - b.w;
-}
-// four values for a list: one vote for all of them rules most of them out
+// The insertion of TopList::add without its second vote: the columns come in no order, so values land all over the list.
 template <int KMAX>
-__device__ __forceinline__ void add4(TopList<KMAX>& top, const float (&d)[4]) {
-    if (!__any_sync(0xffffffffu, fmaxf(max3(d[0], d[1], d[2]), d[3]) > top.v[0])) return;
+__device__ __forceinline__ void add_any(TopList<KMAX>& top, float d) {
+    if (!__any_sync(0xffffffffu, d > top.v[0])) return;
+    d = fmaxf(d, 0.f);                                       // a NaN must not move the list
 #pragma unroll
-    for (int e = 0; e < 4; e++) top.add(d[e]);
+    for (int k = 0; k < KMAX - 1; k++) top.v[k] = fmaxf(top.v[k], fminf(top.v[k + 1], d));
+    top.v[KMAX - 1] = fmaxf(top.v[KMAX - 1], d);
 }
 
 constexpr int SORT_STAGES = 3 * 2 * 32 * LDS;                // floats: two stages of x (or l), u, W
-template <int KMAX, bool POS>
-constexpr int redo_sort_smem() { return (SORT_STAGES + (POS ? KMAX * 32 * 33 : 0)) * (int)sizeof(float); }
 
-template <int NX, int KMAX, bool POS>
+template <int NX, int KMAX>
 __device__ void dense_sort(const PruneArgs& a, float* sm) {
     const PruneProblem& p = a.p;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4, K = p.K;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, K = p.K;
     static_assert(NX * 32 * 33 <= SORT_STAGES, "results fit the stages");
     float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(sm);
-    float(*words)[32][33] = reinterpret_cast<float(*)[32][33]>(sm + SORT_STAGES);            // POS: [K][row][output]
-    constexpr uint32_t EMPTY = 0xffffffffu;
     const int tiles_n = (p.CO + 31) / 32;
     for (int unit = blockIdx.x; unit < a.S * tiles_n; unit += gridDim.x) {
         const int s = unit % a.S, n0 = unit / a.S * 32;
@@ -690,100 +750,23 @@ __device__ void dense_sort(const PruneArgs& a, float* sm) {
             TopList<KMAX> top[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) top[i].init();
-            sort_sweep<false>(a, sm, s, n0, 0, [&](int, const float4(&x)[2], const float4(&)[2], const float4(&w)[2]) {
+            sort_sweep<false>(a, sm, s, n0, 0, [&](const float(&x)[2], const float(&)[2], const float(&w)[2]) {
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float d[4];
-                    minus4(d, x[i >> 1], w[i & 1]);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) d[e] = fabsf(d[e]);
-                    add4(top[i], d);
-                }
+                for (int i = 0; i < 4; i++) add_any(top[i], fabsf(x[i >> 1] - w[i & 1]));
             });
 #pragma unroll
             for (int i = 0; i < 4; i++) result[0][i] = top[i].combine(K, p.q, SNB_EPS);
-            if constexpr (POS) {
-                // the rank of an element is the number of larger values in its list, and of equal values the later column
-                // comes first, as in prune_sort; pairs in which more columns share the K-th value than there is
-                // room for take the order of insertion (PosList)
-                float seed[4];
-                bool crowded = false;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float least = top[i].kth(K);
-                    seed[i] = least > 0.f ? __int_as_float(__float_as_int(least) - 1) : 0.f;
-                    for (int r = 0; r < K; r++) words[r][ty + 16 * (i >> 1)][tx + 16 * (i & 1)] = __uint_as_float(EMPTY);
-                }
-                sort_sweep<false>(a, sm, s, n0, 0, [&](int c, const float4(&x)[2], const float4(&)[2], const float4(&w)[2]) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float t[4];
-                        minus4(t, x[i >> 1], w[i & 1]);
-                        if (!__any_sync(0xffffffffu, max3abs(max3abs(t[0], t[1], t[2]), t[3], t[3]) > seed[i])) continue;
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float v = fabsf(t[e]);
-                            if (!(v > seed[i])) continue;
-                            int rank = 0;
-#pragma unroll
-                            for (int r = 0; r < KMAX; r++) rank += top[i].v[r] > v;
-                            uint32_t word = (uint32_t)(c + e) | (t[e] >= 0.f ? 0u : SNB_SIGN_BIT);
-                            for (; rank < K; rank++) {       // past equal values of later columns
-                                float& at = words[rank][ty + 16 * (i >> 1)][tx + 16 * (i & 1)];
-                                const uint32_t other = __float_as_uint(at);
-                                if (other == EMPTY || (other & ~SNB_SIGN_BIT) < (word & ~SNB_SIGN_BIT)) {
-                                    at = __uint_as_float(word);
-                                    word = other;
-                                }
-                                if (word == EMPTY) break;
-                            }
-                            crowded = crowded || rank == K;
-                        }
-                    }
-                });
-                if (__syncthreads_or(crowded)) {             // rare
-#pragma unroll 1
-                    for (int g = 0; g < 4; g++) {
-                        PosList<KMAX> pl;
-                        pl.init(0.f);
-                        pl.seed = g == 0 ? seed[0] : g == 1 ? seed[1] : g == 2 ? seed[2] : seed[3];
-                        sort_sweep<false>(a, sm, s, n0, 0, [&](int c, const float4(&x)[2], const float4(&)[2], const float4(&w)[2]) {
-                            float t[4];
-                            minus4(t, g & 2 ? x[1] : x[0], g & 1 ? w[1] : w[0]);
-#pragma unroll
-                            for (int e = 0; e < 4; e++) pl.add(t[e], (uint32_t)(c + e), K);
-                        });
-#pragma unroll
-                        for (int k = 0; k < KMAX; k++)
-                            if (k < K) words[k][ty + 8 * (g & 2)][tx + 16 * (g & 1)] = __uint_as_float(pl.word[KMAX - 1 - k]);
-                    }
-                    __syncthreads();
-                }
-                for (int r = warp; r < min(32, p.B - s * 32); r += 8) {
-                    if (n0 + lane >= p.CO) continue;
-                    for (int t = 0; t < K; t++) {
-                        const uint32_t word = __float_as_uint(words[t][r][lane]);
-                        p.pos[((size_t)t * p.B + s * 32 + r) * p.CO + n0 + lane] = word == EMPTY ? 0 : (int)word;
-                    }
-                }
-            }
         }
         if constexpr (NX >= 2) {
             TopList<KMAX> low[4], high[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) low[i].init(), high[i].init();
-            sort_sweep<true>(a, sm, s, n0, NX - 2, [&](int, const float4(&x)[2], const float4(&u)[2], const float4(&w)[2]) {
+            sort_sweep<true>(a, sm, s, n0, NX - 2, [&](const float(&x)[2], const float(&u)[2], const float(&w)[2]) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    float t1[4], t2[4], d[4];
-                    minus4(t1, w[i & 1], x[i >> 1]);
-                    minus4(t2, u[i >> 1], w[i & 1]);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) d[e] = fmaxf(-t1[e], -t2[e]);
-                    add4(low[i], d);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) d[e] = fmaxf(t1[e], t2[e]);
-                    add4(high[i], d);
+                    const float t1 = w[i & 1] - x[i >> 1], t2 = u[i >> 1] - w[i & 1];
+                    add_any(low[i], fmaxf(-t1, -t2));
+                    add_any(high[i], fmaxf(t1, t2));
                 }
             });
 #pragma unroll
@@ -804,10 +787,9 @@ __device__ void dense_sort(const PruneArgs& a, float* sm) {
 
 template <int NX, int KMAX, bool POS>
 __global__ void __launch_bounds__(256, KMAX > 10 ? 1 : (NX == 1 && !POS ? 4 : 2)) prune_redo_sort(const __grid_constant__ PruneArgs a) {
-    extern __shared__ __align__(16) float redo_smem[];
-    float* const sm = redo_smem;
+    __shared__ __align__(16) float sm[SORT_STAGES];
     if (dense_mode(a)) {
-        dense_sort<NX, KMAX, POS>(a, sm);
+        if constexpr (!POS) dense_sort<NX, KMAX>(a, sm);    // POS: sort_positions_if
         return;
     }
     constexpr int STAGE = FIX_K * NX * 32;

@@ -225,11 +225,11 @@ __device__ __forceinline__ void sp_stage(const SortParams& p, float (*xs)[SP_KT]
     }
 }
 
-__global__ void __launch_bounds__(SP_THREADS, 4) sort_fwd_pos_kernel(const SortParams p) {
+__device__ __forceinline__ void sort_pos_tile(const SortParams& p, int tile_m, int tile_n) {
     __shared__ __align__(16) float xs[2][SP_ROWS][SP_KT];
     __shared__ __align__(16) float ws[2][SP_COLS][SP_KT];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = blockIdx.x * SP_ROWS, n0 = blockIdx.y * SP_COLS;
+    const int m0 = tile_m * SP_ROWS, n0 = tile_n * SP_COLS;
     const int K = p.K;
     const int nk = (p.CI + SP_KT - 1) / SP_KT;
 
@@ -322,11 +322,11 @@ __global__ void __launch_bounds__(SP_THREADS, 4) sort_fwd_pos_kernel(const SortP
 // list only to be pushed out again are never inserted.  Elements >= T0 meet exactly the
 // comparisons they meet in the unseeded scan (anything below T0 in the list loses to them either
 // way), so values, positions and the tie rules are unchanged.
-__global__ void __launch_bounds__(SP_THREADS, 4) sort_fwd_pos_half_kernel(const SortParams p) {
+__device__ __forceinline__ void sort_pos_half_tile(const SortParams& p, int tile_m, int tile_n) {
     __shared__ __align__(16) float xs[2][SP_ROWS][SP_KT];
     __shared__ __align__(16) float ws[2][SP_COLS][SP_KT];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4, hl = lane & 15;
-    const int m0 = blockIdx.x * SP_ROWS, n0 = blockIdx.y * SP_COLS;
+    const int m0 = tile_m * SP_ROWS, n0 = tile_n * SP_COLS;
     const int K = p.K;
     const int nk = (p.CI + SP_KT - 1) / SP_KT;
 
@@ -449,6 +449,34 @@ __global__ void __launch_bounds__(SP_THREADS, 4) sort_fwd_pos_half_kernel(const 
     }
 }
 
+// One tile per CTA; IF: persistent CTAs over all tiles when the pruned form gives up (as a rule it does not, and the grid has
+// to be small because it ends at once).
+template <bool HALF, bool IF>
+__global__ void __launch_bounds__(SP_THREADS, 4) sort_fwd_pos(const SortParams p, const unsigned* overflowed) {
+    auto tile = [&](int m, int n) {
+        if (HALF) sort_pos_half_tile(p, m, n);
+        else sort_pos_tile(p, m, n);
+    };
+    if (!IF) {
+        tile(blockIdx.x, blockIdx.y);
+        return;
+    }
+    if (!prune_gives_up(*overflowed, p.CO)) return;
+    const int tiles_m = (p.B + SP_ROWS - 1) / SP_ROWS, tiles_n = (p.CO + SP_COLS - 1) / SP_COLS;
+    for (long long t = blockIdx.x; t < (long long)tiles_m * tiles_n; t += gridDim.x) {
+        __syncthreads();                                     // the previous tile's readers are done with the stages
+        tile((int)(t % tiles_m), (int)(t / tiles_m));
+    }
+}
+
+cudaError_t sort_positions_if(const PruneProblem& q, const unsigned* overflowed, cudaStream_t st) {
+    const SortParams p{q.x, q.x, q.w, q.y, nullptr, q.pos, q.B, q.CO, q.CI, q.K, q.q};
+    const int grid = 4 * sm_count();
+    if (q.K <= 16) sort_fwd_pos<true, true><<<grid, SP_THREADS, 0, st>>>(p, overflowed);
+    else sort_fwd_pos<false, true><<<grid, SP_THREADS, 0, st>>>(p, overflowed);
+    return cudaGetLastError();
+}
+
 // Sparse backward: one CTA per batch row, grad_x of the row accumulated in shared memory.
 __global__ void __launch_bounds__(256) sort_bwd_kernel(const float* __restrict__ g, const int* __restrict__ pos,
                                                        int B, int CO, int CI, int K, float q, float c0,
@@ -562,8 +590,8 @@ extern "C" int snb_sort_neuron_forward_ws(const float* x, const float* w, int B,
     if (rc || done) return rc;
     SortParams p{x, x, w, y, nullptr, pos, B, CO, CI, K, q};
     dim3 grid((B + SP_ROWS - 1) / SP_ROWS, (CO + SP_COLS - 1) / SP_COLS);
-    if (K <= 16) sort_fwd_pos_half_kernel<<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p);
-    else sort_fwd_pos_kernel<<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p);
+    if (K <= 16) sort_fwd_pos<true, false><<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p, nullptr);
+    else sort_fwd_pos<false, false><<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p, nullptr);
     SNB_CUDA(cudaGetLastError());
     return SNB_OK;
 }
