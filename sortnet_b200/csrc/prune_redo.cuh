@@ -87,6 +87,28 @@ struct DenseLayer {
         vec = !gather && (a.p.W_CI & 3) == 0 && (reinterpret_cast<uintptr_t>(a.p.w) & 15u) == 0;
     }
 };
+// A CTA's share of `tiles` x nk k-tiles: whole tiles, and of the rest an equal part.  Half of the CTAs do that part first: a tile
+// is stored (a latency-bound time) by whoever completes it, and so the two CTAs of an SM do not store at the same time.
+struct DenseWork {
+    int nk, next, tiles;
+    long long u0, u1;
+    __device__ __forceinline__ DenseWork(int all, int nk_) : nk(nk_), next(blockIdx.x) {
+        tiles = all / (int)gridDim.x * (int)gridDim.x;
+        const long long rest = (long long)(all - tiles) * nk;
+        u0 = rest * blockIdx.x / gridDim.x, u1 = rest * (blockIdx.x + 1) / gridDim.x;
+    }
+    __device__ __forceinline__ bool take(int& tile, int& ka, int& kb) {
+        if (u0 < u1 && (next >= tiles || blockIdx.x >= gridDim.x / 2)) {
+            tile = tiles + (int)(u0 / nk), ka = (int)(u0 % nk), kb = (int)min((long long)nk, ka + (u1 - u0));
+            u0 += kb - ka;
+            return true;
+        }
+        if (next >= tiles) return false;
+        tile = next, ka = 0, kb = nk;
+        next += gridDim.x;
+        return true;
+    }
+};
 // n-th output of sub-batch s, and its row of W
 __device__ __forceinline__ int dense_output(const PruneProblem& p, int s, int n) {
     return p.out_list ? p.out_list[(size_t)s * p.out_kept + n] : n;
@@ -114,8 +136,8 @@ __device__ __forceinline__ void* part_of(const PruneArgs& a, int t) {
     return a.partial + (size_t)t * a.S * a.p.CO * 32 * (TRACK ? 8 : 4);
 }
 
-// Words of PAIR neighbouring outputs (tensor t) from the chunks of their rows: in `words` the low halves of the keys (0: at
-// the floor) are replaced by place in the chunk | sign.
+// Which column of its chunk of 32 gave a row's value: place in the chunk | sign, for one output, lane = row.  low: the low
+// halves of the keys (0: at the floor).
 template <int NX>
 struct Rescan {
     const float* xs[NX];            // rows of the sub-batch
@@ -132,53 +154,46 @@ struct Rescan {
         return (T == 0 ? fmaxf(-t1, -t2) : fmaxf(t1, t2)) == want;
     }
     // four lanes per row, eight columns each by 16-byte loads: rows 8 e + lane / 4 of SETS e at a time
-    template <int T, int PAIR, int SETS>
-    __device__ __forceinline__ void vectors(const float* const (&wr)[PAIR], const float (&value)[PAIR], uint32_t (&low)[PAIR]) const {
+    template <int T, int SETS>
+    __device__ __forceinline__ uint32_t vectors(const float* wr, float value, uint32_t low) const {
         const int lane = threadIdx.x & 31;
-        uint32_t found[PAIR];
-#pragma unroll
-        for (int o = 0; o < PAIR; o++) found[o] = 0u;
+        uint32_t found = 0u;
 #pragma unroll 1
         for (int e0 = 0; e0 < 4; e0 += SETS) {
-            float4 x[PAIR][SETS][NX][2], w[PAIR][SETS][2];
-            int at[PAIR][SETS][2];
+            float4 x[SETS][NX][2], w[SETS][2];
+            int at[SETS][2];
 #pragma unroll
-            for (int o = 0; o < PAIR; o++)
+            for (int e = 0; e < SETS; e++) {
+                const int r = 8 * (e0 + e) + (lane >> 2);
+                const unsigned q = __shfl_sync(0xffffffffu, low, r);
+                const int c = (q ? (int)(0xffffffffu - q) * 32 : 0) + 8 * (lane & 3);
 #pragma unroll
-                for (int e = 0; e < SETS; e++) {
-                    const int r = 8 * (e0 + e) + (lane >> 2);
-                    const unsigned q = __shfl_sync(0xffffffffu, low[o], r);
-                    const int c = (q ? (int)(0xffffffffu - q) * 32 : 0) + 8 * (lane & 3);
+                for (int h = 0; h < 2; h++) {
+                    at[e][h] = min(c + 4 * h, last - 3);             // past the end: the last columns once more
+                    w[e][h] = *reinterpret_cast<const float4*>(wr + at[e][h]);
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        at[o][e][h] = min(c + 4 * h, last - 3);      // past the end: the last columns once more
-                        w[o][e][h] = *reinterpret_cast<const float4*>(wr[o] + at[o][e][h]);
-#pragma unroll
-                        for (int u = 0; u < NX; u++)
-                            x[o][e][u][h] = *reinterpret_cast<const float4*>(xs[u] + (size_t)min(r, rows - 1) * stride + at[o][e][h]);
-                    }
+                    for (int u = 0; u < NX; u++)
+                        x[e][u][h] = *reinterpret_cast<const float4*>(xs[u] + (size_t)min(r, rows - 1) * stride + at[e][h]);
                 }
+            }
 #pragma unroll
-            for (int o = 0; o < PAIR; o++)
+            for (int e = 0; e < SETS; e++) {
+                const float want = __shfl_sync(0xffffffffu, value, 8 * (e0 + e) + (lane >> 2));
+                unsigned best = 0xffffffffu;                         // column << 1 | negative
 #pragma unroll
-                for (int e = 0; e < SETS; e++) {
-                    const float want = __shfl_sync(0xffffffffu, value[o], 8 * (e0 + e) + (lane >> 2));
-                    unsigned best = 0xffffffffu;                     // column << 1 | negative
-#pragma unroll
-                    for (int k = 7; k >= 0; k--) {
-                        auto of = [&](const float4& v) { return (k & 3) == 0 ? v.x : (k & 3) == 1 ? v.y : (k & 3) == 2 ? v.z : v.w; };
-                        bool negative;
-                        if (holds<T>(of(x[o][e][0][k >> 2]), of(x[o][e][NX - 1][k >> 2]), of(w[o][e][k >> 2]), want, &negative))
-                            best = (unsigned)(at[o][e][k >> 2] + (k & 3)) << 1 | (negative ? 1u : 0u);
-                    }
-                    best = min(best, __shfl_xor_sync(0xffffffffu, best, 1));
-                    best = min(best, __shfl_xor_sync(0xffffffffu, best, 2));
-                    best = __shfl_sync(0xffffffffu, best, 4 * (lane & 7));
-                    if ((lane >> 3) == e0 + e) found[o] = ((best >> 1) & 31u) | (best & 1u ? SNB_SIGN_BIT : 0u);
+                for (int k = 7; k >= 0; k--) {
+                    auto of = [&](const float4& v) { return (k & 3) == 0 ? v.x : (k & 3) == 1 ? v.y : (k & 3) == 2 ? v.z : v.w; };
+                    bool negative;
+                    if (holds<T>(of(x[e][0][k >> 2]), of(x[e][NX - 1][k >> 2]), of(w[e][k >> 2]), want, &negative))
+                        best = (unsigned)(at[e][k >> 2] + (k & 3)) << 1 | (negative ? 1u : 0u);
                 }
+                best = min(best, __shfl_xor_sync(0xffffffffu, best, 1));
+                best = min(best, __shfl_xor_sync(0xffffffffu, best, 2));
+                best = __shfl_sync(0xffffffffu, best, 4 * (lane & 7));
+                if ((lane >> 3) == e0 + e) found = ((best >> 1) & 31u) | (best & 1u ? SNB_SIGN_BIT : 0u);
+            }
         }
-#pragma unroll
-        for (int o = 0; o < PAIR; o++) low[o] = found[o];
+        return found;
     }
     // a lane per column, AHEAD rows at a time
     template <int T, int AHEAD>
@@ -236,7 +251,6 @@ __device__ __noinline__ void dense_emit(const PruneArgs& a, const DenseLayer& d,
                 }
             }
         if constexpr (TRACK) {
-            constexpr int PAIR = NX == 1 ? 2 : 1;
             const int* inv = p.ci && !d.gather ? a.inv + (size_t)s * C : nullptr;
             Rescan<NX> scan;
             scan.stride = d.gather ? p.CI : a.ldr, scan.rows = rows, scan.last = d.K - 1;
@@ -244,38 +258,24 @@ __device__ __noinline__ void dense_emit(const PruneArgs& a, const DenseLayer& d,
 #pragma unroll
             for (int u = 0; u < NX; u++)
                 scan.xs[u] = d.gather ? p.x + (size_t)s * 32 * p.CI : a.xr + (size_t)(u * a.S + s) * 32 * a.ldr;
-            auto words = [&](auto which, int i) {            // of the outputs i, i + 1 of the warp
+            auto words = [&](auto which, int slot) {
                 constexpr int T = decltype(which)::value;
-                const float* wr[PAIR];
-                float value[PAIR];
-                uint32_t low[PAIR], place[PAIR];
-#pragma unroll
-                for (int o = 0; o < PAIR; o++) {
-                    const int slot = warp * SLOTS + i + o;
-                    wr[o] = p.w + (size_t)dense_row(p, s, dense_output(p, s, min(base + slot, d.N - 1))) * C;
-                    value[o] = tile[T][lane][slot];
-                    place[o] = low[o] = __float_as_uint(tile[NX + T][lane][slot]);
+                const float* wr = p.w + (size_t)dense_row(p, s, dense_output(p, s, min(base + slot, d.N - 1))) * C;
+                const float value = tile[T][lane][slot];
+                const uint32_t low = __float_as_uint(tile[NX + T][lane][slot]);
+                const uint32_t place = d.vec ? scan.template vectors<T, NX == 1 ? 4 : 2>(wr, value, low)
+                                             : scan.template columns<T, 16>(wr, value, low);
+                uint32_t word = NX == 1 ? first_kept(p, s) : T == 0 ? SNB_NO_GRAD_ID : 0u;       // at its floor
+                if (low) {
+                    const int col = min((int)(0xffffffffu - low) * 32 + (int)(place & 31u), d.K - 1);
+                    word = (uint32_t)(inv ? inv[col] : col) | (place & SNB_SIGN_BIT);
                 }
-                if (d.vec) {
-                    scan.template vectors<T, PAIR, NX == 1 ? 4 : 2>(wr, value, place);
-                } else {
-#pragma unroll
-                    for (int o = 0; o < PAIR; o++) place[o] = scan.template columns<T, 16>(wr[o], value[o], place[o]);
-                }
-#pragma unroll
-                for (int o = 0; o < PAIR; o++) {
-                    uint32_t word = NX == 1 ? first_kept(p, s) : T == 0 ? SNB_NO_GRAD_ID : 0u;       // at its floor
-                    if (low[o]) {
-                        const int col = min((int)(0xffffffffu - low[o]) * 32 + (int)(place[o] & 31u), d.K - 1);
-                        word = (uint32_t)(inv ? inv[col] : col) | (place[o] & SNB_SIGN_BIT);
-                    }
-                    tile[NX + T][lane][warp * SLOTS + i + o] = __uint_as_float(word);
-                }
+                tile[NX + T][lane][slot] = __uint_as_float(word);
             };
 #pragma unroll 1
-            for (int i = 0; i < SLOTS; i += PAIR) {
-                words(std::integral_constant<int, 0>(), i);
-                if constexpr (NX == 2) words(std::integral_constant<int, 1>(), i);
+            for (int i = 0; i < SLOTS; i++) {
+                words(std::integral_constant<int, 0>(), warp * SLOTS + i);
+                if constexpr (NX == 2) words(std::integral_constant<int, 1>(), warp * SLOTS + i);
             }
         }
         __syncthreads();
@@ -341,11 +341,9 @@ __device__ void dense_point(const PruneArgs& a, const DenseLayer& d, float* smem
     float* ws = smem + 2 * BM * LDS;                         // [2][BN][LDS]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN, tb = lane >> 3, tj = lane & 7;
     const int tiles_m = (a.S + WM - 1) / WM;
-    const StreamK sk{tiles_m, (d.N + BN - 1) / BN, (d.K + BK - 1) / BK};
-    long long u0, u1;
-    sk.range(u0, u1);
-    while (u0 < u1) {
-        const int tile = (int)(u0 / sk.nk), ka = (int)(u0 % sk.nk), kb = (int)min((long long)sk.nk, ka + (u1 - u0));
+    const int nk = (d.K + BK - 1) / BK;
+    DenseWork work(tiles_m * ((d.N + BN - 1) / BN), nk);
+    for (int tile, ka, kb; work.take(tile, ka, kb);) {
         const int s0 = tile % tiles_m * WM, s = s0 + wm, n0 = tile / tiles_m * BN;
         const int* list = d.gather ? p.ci + (size_t)s0 * p.CI : nullptr;
         DenseW<BN / 16> rw;
@@ -412,7 +410,7 @@ __device__ void dense_point(const PruneArgs& a, const DenseLayer& d, float* smem
                     }
             }
         }
-        const bool whole = ka == 0 && kb == sk.nk;
+        const bool whole = ka == 0 && kb == nk;
 #pragma unroll
         for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -424,7 +422,6 @@ __device__ void dense_point(const PruneArgs& a, const DenseLayer& d, float* smem
                                  (j & 1) ? id >> 16 : id & 0xffffu, whole);
             }
         dense_finish<NX, TRACK>(a, d, s0, min(WM, a.S - s0), n0 / 128, BN / 128, kb - ka, smem);
-        u0 += kb - ka;
     }
 }
 
@@ -440,11 +437,9 @@ __device__ void dense_box(const PruneArgs& a, const DenseLayer& d, float* smem) 
     const float* xl = a.xr + (size_t)(NX - 2) * a.S * 32 * a.ldr;
     const float* xu = a.xr + (size_t)(NX - 1) * a.S * 32 * a.ldr;
     const int tid = threadIdx.x, lane = tid & 31, wn = tid >> 5, tb = lane >> 3, tj = lane & 7;
-    const StreamK sk{a.S, (d.N + BN - 1) / BN, (d.K + BK - 1) / BK};
-    long long u0, u1;
-    sk.range(u0, u1);
-    while (u0 < u1) {
-        const int tile = (int)(u0 / sk.nk), ka = (int)(u0 % sk.nk), kb = (int)min((long long)sk.nk, ka + (u1 - u0));
+    const int nk = (d.K + BK - 1) / BK;
+    DenseWork work(a.S * ((d.N + BN - 1) / BN), nk);
+    for (int tile, ka, kb; work.take(tile, ka, kb);) {
         const int s = tile % a.S, n0 = tile / a.S * BN;
         DenseW<BN / 16> rw;
 #pragma unroll
@@ -522,7 +517,7 @@ __device__ void dense_box(const PruneArgs& a, const DenseLayer& d, float* smem) 
                     }
             }
         }
-        const bool whole = ka == 0 && kb == sk.nk;
+        const bool whole = ka == 0 && kb == nk;
 #pragma unroll
         for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -535,7 +530,6 @@ __device__ void dense_box(const PruneArgs& a, const DenseLayer& d, float* smem) 
                 merge<TRACK>(part_of<TRACK>(a, NX - 1), at, hi[i][j], id >> 16, whole);
             }
         dense_finish<NX, TRACK>(a, d, s, 1, n0 / 128, 1, kb - ka, smem);
-        u0 += kb - ka;
     }
 }
 

@@ -150,12 +150,12 @@ def test_host_threads_with_different_sizes():
     assert not failures, failures[:3]
 
 
-@pytest.mark.parametrize("p", [1e6, 1e8, 3e8, 6e8])
+@pytest.mark.parametrize("p", [1e6, 1e8, 3e8])
 @pytest.mark.parametrize("shape", [(64, 1400, 800), (512, 300, 300)])
 @pytest.mark.parametrize("narrow", [False, True])
 def test_huge_finite_p(p, shape, narrow):
-    """y is the maximum up to CI^(1/p), of which nothing is left in fp32.  Up to p = 7e8 the rounding of |t| / M (1 - 2^-23 at
-    worst, to the power p above 2^-126) leaves a sum that is not zero, in the dense kernel as here.  narrow: rows that hardly
+    """y is the maximum up to CI^(1/p), of which nothing is left in fp32.  At p = 3e8 the rounding of |t| / M and of
+    its logarithm (2^-22, to the power p above 2^-126) leaves a sum that is not zero, in the dense kernel as here.  narrow: rows that hardly
     differ, so that the range of a column is no wider than the rounding of the test."""
     x, w, g, ci, co = inputs(*shape, 1.0, 11)
     if narrow:
