@@ -48,12 +48,15 @@ def _compile(src, obj, verbose):
 
 def build_ops(force: bool = False) -> str:
     """The native operator layer: one C++ file against PyTorch's headers, no CUDA code."""
-    src = os.path.join(CSRC, "ops_ext.cpp")
-    newest = max(os.path.getmtime(src), _newest_header())
-    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest:
-        return OPS
     import sysconfig
     import torch
+    src = os.path.join(CSRC, "ops_ext.cpp")
+    newest = max(os.path.getmtime(src), _newest_header())
+    stamp = os.path.join(OBJ, "ops_built_for")               # the module is bound to one PyTorch and one Python
+    target = "%s %s %s" % (torch.__version__, sysconfig.get_config_var("SOABI"), torch._C._GLIBCXX_USE_CXX11_ABI)
+    built_for = open(stamp).read() if os.path.exists(stamp) else ""
+    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest and built_for == target:
+        return OPS
     base = os.path.dirname(torch.__file__)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_ops", "-DTORCH_API_INCLUDE_EXTENSION_H",
@@ -66,6 +69,9 @@ def build_ops(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed for %s:\n%s" % (src, r.stderr))
+    os.makedirs(OBJ, exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(target)
     return OPS
 
 

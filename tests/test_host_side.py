@@ -44,6 +44,29 @@ def test_loader_signatures_cover_the_header(built_lib):
     assert lib.snb_inf_dist_forward_sorted_workspace_bytes(33, 3, 8) == 800 + 4 * 33 * 8 + 4 * 2 * 8   # 792 rounded up to 16
 
 
+def test_operator_module_follows_the_installed_torch(built_lib, monkeypatch):
+    """_ops.so is rebuilt for another PyTorch, whatever the modification times say."""
+    import subprocess
+    from sortnet_b200 import build
+    calls = []
+
+    def compiler(cmd, **kw):
+        calls.append(cmd[0])
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+    monkeypatch.setattr(build.subprocess, "run", compiler)
+    build.build_ops()
+    assert calls == []
+    stamp = os.path.join(build.OBJ, "ops_built_for")
+    was = open(stamp).read()
+    try:
+        monkeypatch.setattr(torch, "__version__", "0.0.0")
+        build.build_ops()
+        assert calls == ["g++"]
+    finally:
+        with open(stamp, "w") as f:
+            f.write(was)
+
+
 def test_status_codes_without_gpu(built_lib):
     # argument checks run before any CUDA call
     from sortnet_b200 import _lib
