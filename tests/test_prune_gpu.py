@@ -140,3 +140,90 @@ def test_sort_neuron(B, CI, CO, q, K, kind):
     yl, yu = torch.empty_like(y), torch.empty_like(y)
     C.bound_sort_neuron_forward(col3(xl), col3(xu), W, yl, yu, 1, q, K)
     assert rel(host(yl), yl_o) < 2e-6 and rel(host(yu), yu_o) < 2e-6
+
+
+def half_prunable(kind, rng, B, CI, CO):
+    """Rows of W whose list overflows: single ones (below the share at which the layer is evaluated as a whole), a block
+    of neighbours, and all of them, on inputs as wide as the weights and with NaN, infinities and ties."""
+    x, w = rng.random((B, CI), dtype=np.float32), rng.standard_normal((CO, CI)).astype(np.float32)
+    if kind == "single":
+        w[::64] *= 0.001
+    elif kind == "block":
+        w[40:40 + CO // 40] *= 0.001
+    else:
+        x = (0.5 * rng.standard_normal((B, CI))).astype(np.float32)
+        if kind == "wide ties":
+            x, w = (x * 4).round() / 4, (w * 2).round() / 2
+        else:
+            x[3, 5], x[1, 9], x[0], w[2, 4], w[8, 11], w[11] = np.nan, np.inf, 0.25, np.nan, -np.inf, 0.25
+    return x.astype(np.float32), w
+
+
+# columns around the tiles' steps (32) and the rows' alignment (4), outputs around their tiles (64, 128, 256), one and more sub-batches
+@pytest.mark.parametrize("B,CI,CO", [(33, 1024, 1100), (64, 1028, 1000), (70, 1025, 1000), (31, 1503, 1281), (100, 4100, 321)])
+@pytest.mark.parametrize("kind", ["single", "block", "wide", "wide ties"])
+def test_lists_that_overflow(B, CI, CO, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    assert uses_pruning(1, 1, 1, B, CO, CI, CO, CI, 0) and uses_pruning(1, 10, 1, B, CO, CI, CO, CI, 0)
+    x, w = half_prunable(kind, np.random.default_rng(B + CI), B, CI, CO)
+    y_o, pos_o = oracle.inf_dist_forward(x, w)
+    X, W = col3(x), dev(w)
+    y, pos = torch.full((B, CO, 1), 7.0, device="cuda"), torch.full((B, CO, 1), 7, device="cuda", dtype=torch.int32)
+    C.inf_dist_forward(X, W, y, pos, 1)
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+    C.inf_dist_forward_nograd(X, W, y.fill_(7), 1)
+    assert np.array_equal(host(y), y_o)
+    xl, xu = (x - np.float32(0.05)).astype(np.float32), (x + np.float32(0.05)).astype(np.float32)
+    yl_o, yu_o, pl_o, pu_o = oracle.bound_inf_dist_forward(xl, xu, w)
+    XL, XU = col3(xl), col3(xu)
+    yl, yu, pl, pu = (torch.empty_like(y), torch.empty_like(y), torch.empty_like(pos), torch.empty_like(pos))
+    C.bound_inf_dist_forward(XL, XU, W, yl, yu, pl, pu, 1)
+    assert all(np.array_equal(host(a), b) for a, b in zip((yl, yu, pl, pu), (yl_o, yu_o, pl_o, pu_o)))
+    y3 = [torch.empty(B, CO, device="cuda") for _ in range(3)]
+    C.layer_bound_forward(X.squeeze(-1), XL.squeeze(-1), XU.squeeze(-1), W, None, None, *y3)
+    assert all(np.array_equal(a.cpu().numpy(), b) for a, b in zip(y3, (y_o, yl_o, yu_o)))
+    if kind == "wide":
+        return                                              # the oracle's sort is not defined on NaN
+    ys, ps = torch.empty_like(y), torch.empty(10, B, CO, 1, device="cuda", dtype=torch.int32)
+    ys_o, ps_o = oracle.sort_forward(x, w, 0.75, 10)
+    C.sort_neuron_forward(X, W, ys, ps, 1, 0.75, 10)
+    assert rel(host(ys), ys_o) < 2e-6 and np.array_equal(ps.squeeze(-1).cpu().numpy(), ps_o)
+    C.sort_neuron_forward_nograd(X, W, ys.fill_(7), 1, 0.75, 10)
+    assert rel(host(ys), ys_o) < 2e-6
+    yl_o, yu_o = oracle.sort_bound_forward(xl, xu, w, 0.75, 10)
+    C.bound_sort_neuron_forward(XL, XU, W, yl, yu, 1, 0.75, 10)
+    assert rel(host(yl), yl_o) < 2e-6 and rel(host(yu), yu_o) < 2e-6
+
+
+@pytest.mark.parametrize("which", ["both", "ci"])
+@pytest.mark.parametrize("kind", ["wide", "wide ties", "single"])
+def test_masked_lists_that_overflow(which, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(4)
+    B, CI, CO = 97, 1030, 700
+    ci, co = make_masks(rng, B, CI, 0.8), make_masks(rng, B, CO, 0.8) if which == "both" else None
+    x, w = half_prunable(kind, rng, B, CI, CO)
+    x = np.ascontiguousarray(x[:, :ci.shape[1]])
+    n_out = CO if co is None else co.shape[1]
+    y_o, pos_o = oracle.inf_dist_forward(x, w, ci, co)
+    for entry in (C.inf_dist_forward_sorted, lambda a, b, c, d, i, o: C.inf_dist_forward(a, b, c, d, 1, i, o)):
+        y, pos = torch.empty(B, n_out, 1, device="cuda"), torch.empty(B, n_out, 1, device="cuda", dtype=torch.int32)
+        entry(col3(x), dev(w), y, pos, idx3(ci), idx3(co))
+        assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+
+
+@pytest.mark.parametrize("kind", ["normal", "ties", "flat"])
+def test_columns_that_come_twice(kind):
+    """A list may name a column more than once, each with inputs of its own."""
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(6)
+    B, CI, CO = 70, 1024, 1000
+    x, w = operands(kind, rng, B, CI, CO)
+    ci = rng.integers(0, CI, (3, 900)).astype(np.int32)
+    ci[1] = np.sort(rng.permutation(CI)[:900])              # one of the sub-batches has a list like any other
+    x = np.ascontiguousarray(x[:, :900])
+    assert uses_pruning(1, 1, 1, B, CO, 900, CO, CI, 1)
+    y_o, pos_o = oracle.inf_dist_forward(x, w, ci, None)
+    y, pos = torch.empty(B, CO, 1, device="cuda"), torch.empty(B, CO, 1, device="cuda", dtype=torch.int32)
+    C.inf_dist_forward(col3(x), dev(w), y, pos, 1, idx3(ci), None)
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
