@@ -54,6 +54,8 @@ extern "C" {
 const char* snb_status_string(int status);
 const char* snb_last_cuda_error(void);
 int snb_version(void);
+/* Kernels launched by this process through the library so far (copies and memsets are not counted), all host threads. */
+long long snb_launch_count(void);
 
 /* 1 if a bounded device-side wait (the mbarrier waits of the TMA-staged kernels) ever gave up on the
  * current device, 0 if not, -1 on a CUDA error; synchronises the device.  No counterpart in the

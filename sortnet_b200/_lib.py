@@ -73,6 +73,7 @@ SIGNATURES = {
     "snb_peer_signal": [_P, _I, _I, ctypes.c_uint, _P],
     "snb_peer_wait": [_P, _I, _I, ctypes.c_uint, ctypes.c_ulonglong, _P, _P],
     "snb_check_index_lists": [_P, _I, _I, _I, ctypes.POINTER(ctypes.c_int), _P],
+    "snb_launch_count": [],                                              # returns long long
     "snb_probe_fp32": [_P, _I, ctypes.POINTER(ctypes.c_double), _P],
 }
 
@@ -105,6 +106,7 @@ def load(build_if_missing: bool = False):
     lib.snb_last_cuda_error.restype = ctypes.c_char_p
     lib.snb_version.argtypes = []
     lib.snb_version.restype = ctypes.c_int
+    lib.snb_launch_count.restype = ctypes.c_longlong
     lib.snb_trim_scratch.argtypes = []
     lib.snb_trim_scratch.restype = ctypes.c_int
     lib.snb_device_wait_failed.argtypes = []

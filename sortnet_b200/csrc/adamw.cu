@@ -124,7 +124,7 @@ extern "C" int snb_adamw_reduce_step(const float* w_src, float* w_dst, const voi
         SNB_REDUCE_CASE(16)
     }
 #undef SNB_REDUCE_CASE
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -141,6 +141,6 @@ extern "C" int snb_adamw_step(float* w, const float* g, float* m, float* v, long
         reinterpret_cast<float4*>(w), reinterpret_cast<const float4*>(g), reinterpret_cast<float4*>(m),
         reinterpret_cast<float4*>(v), (size_t)n / 4, 1.0f - lr * weight_decay, beta1, beta2, step_size,
         inv_sqrt_bc2, eps, grad_scale);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

@@ -334,7 +334,7 @@ static cudaError_t launch_bound(BoundParams p, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     kern<<<(unsigned)grid, NT, SMEM, st>>>(p);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace snb
@@ -442,7 +442,7 @@ extern "C" int snb_bound_inf_dist_forward_ws(const float* xl, const float* xu, c
     }
     if (vec) bound_fwd_pos_kernel<true><<<grid, 256, SMEM, (cudaStream_t)stream>>>(p);
     else bound_fwd_pos_kernel<false><<<grid, 256, SMEM, (cudaStream_t)stream>>>(p);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -467,7 +467,7 @@ static int bound_backward(const float* gl, const float* gu, const int* posl, con
     }
     bound_bwd_kernel<<<B, 256, use_smem ? 2 * CI * sizeof(float) : 0, st>>>(gl, gu, posl, posu, CO, CI,
                                                                          gxl, gxu, gw, use_smem);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 

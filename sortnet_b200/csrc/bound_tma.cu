@@ -265,7 +265,7 @@ cudaError_t bound_forward_tma(const float* xl, const float* xu, const float* w, 
         if (e != cudaSuccess) return e;
     }
     bound_fwd_tma_kernel<<<(unsigned)grid, TMA_NT, TMA_SMEM, st>>>(ml, mu, mw, p);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace snb

@@ -108,6 +108,6 @@ extern "C" int snb_dp_adamw_step(const void* const* grad_ptrs, void* const* para
         SNB_DP_CASE(14) SNB_DP_CASE(15) SNB_DP_CASE(16)
     }
 #undef SNB_DP_CASE
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

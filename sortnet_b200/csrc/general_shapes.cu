@@ -149,17 +149,17 @@ size_t words(const Geo& q, int C, int K = 1) { return sizeof(uint32_t) * (size_t
 cudaError_t pack(const void* src, void* dst, const Geo& q, int C, int K, uint32_t fill, cudaStream_t st) {
     long long n = (long long)q.G * K * q.Bp * C;
     pack_rows_kernel<<<grid_for(n), 256, 0, st>>>((const uint32_t*)src, (uint32_t*)dst, q, C, K, fill, n);
-    return cudaGetLastError();
+    return launched();
 }
 cudaError_t unpack(const void* src, void* dst, const Geo& q, int C, int K, cudaStream_t st) {
     long long n = (long long)K * q.B * q.G * C * q.HW;
     unpack_rows_kernel<<<grid_for(n), 256, 0, st>>>((const uint32_t*)src, (uint32_t*)dst, q, C, K, n);
-    return cudaGetLastError();
+    return launched();
 }
 cudaError_t expand(const int* m, int* mp, const Geo& q, int C, cudaStream_t st) {
     long long n = (long long)q.G * q.S * q.HW * C;
     expand_mask_kernel<<<grid_for(n), 256, 0, st>>>(m, mp, q, C, n);
-    return cudaGetLastError();
+    return launched();
 }
 size_t mask_bytes(const Geo& q, int C) { return sizeof(int) * (size_t)q.G * q.S * q.HW * C; }
 // Group g of a packed matrix / an expanded mask / the weights.

@@ -193,7 +193,7 @@ static cudaError_t launch_resolve(const InfFwdParams& p, const unsigned long lon
         if (vec) inf_resolve_kernel<false><<<grid, 256, 0, st>>>(p, nullptr);
         else inf_resolve_lists_kernel<false><<<lists_grid, 256, 0, st>>>(p, nullptr);
     }
-    return cudaGetLastError();
+    return launched();
 }
 
 // Sparse backward: one CTA per batch row.  grad_x of the row is accumulated in shared
@@ -480,7 +480,7 @@ static cudaError_t launch_sk(InfSkParams p, bool* split, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     kern<<<(unsigned)grid, NT, SMEM, st>>>(p);
-    return cudaGetLastError();
+    return launched();
 }
 
 // *split tells whether tiles were shared between CTAs; for TRACK that means the result is in
@@ -621,7 +621,7 @@ extern "C" int snb_inf_dist_forward_sorted_ws(const float* x, const float* w, in
         float* xw = reinterpret_cast<float*>(static_cast<char*>(workspace) + sorted_ws_input_offset(B, CO));
         int* inv_w = reinterpret_cast<int*>(xw + (size_t)B * W_CI);
         expand_rows_kernel<<<B, 256, 0, st>>>(x, w_index_ci, B, CI, W_CI, xw, inv_w);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
         xin = xw;
         inv = inv_w;
     }
@@ -718,7 +718,7 @@ static int inf_backward(const float* g, const int* pos, int B, int CO, int CI, i
         dim3 grid((CO + 255) / 256, B);
         inf_bwd_wide_kernel<<<grid, 256, 0, st>>>(g, pos, B, CO, CI, gx, gw, ci, co, W_CI);
     }
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 

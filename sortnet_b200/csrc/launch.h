@@ -11,6 +11,9 @@ namespace snb {
 // Records the last CUDA runtime error seen by an entry point of this thread.
 void set_last_cuda_error(cudaError_t e);
 
+// Called after every launch (or n of them): counts them (snb_launch_count) and returns the launch error, if any.
+cudaError_t launched(int n = 1);
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

@@ -265,7 +265,7 @@ extern "C" int snb_layer_forward(const float* x, const float* w, int B, int CO, 
         dim3 grid((CO + 255) / 256, (B + SNB_SUB_BATCH - 1) / SNB_SUB_BATCH);
         shift_bias_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(y_dist, shift ? mean : nullptr, bias, w_index_co, B,
                                                                   CO, out);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
     }
     return SNB_OK;
 }
@@ -281,7 +281,7 @@ extern "C" int snb_layer_backward_ws(const float* grad_out, const float* x, cons
     cudaStream_t st = (cudaStream_t)stream;
     if (grad_bias) {
         column_sum_kernel<<<(W_CO + 15) / 16, 256, 0, st>>>(grad_out, w_index_co, B, CO, W_CO, grad_bias);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
     }
     const float* g = grad_out;
     if (mean_shift) {
@@ -341,7 +341,7 @@ extern "C" int snb_layer_bound_forward_ws(const float* x, const float* xl, const
         const int blocks = (int)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368);
         shift_bias3_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(x ? y : nullptr, xl ? yl : nullptr,
                                                                      xl ? yu : nullptr, running_mean, bias, B, CO);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
     }
     return SNB_OK;
 }
@@ -358,7 +358,7 @@ extern "C" int snb_input_box(const float* x, float eps, float down, float up, lo
     if (n <= 0) return SNB_ERR_BAD_SHAPE;
     const int blocks = (int)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368);
     input_box_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(x, eps, down, up, (size_t)n, xl, xu);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -369,9 +369,9 @@ extern "C" int snb_margin_loss(const float* d, const long long* target, int B, i
     cudaStream_t st = (cudaStream_t)stream;
     margin_loss_kernel<<<(B + 7) / 8, 256, 0, st>>>(d, target, B, K, eps, 2.0f * eps, clip, lam, scale, margin, row_loss,
                                                     grad_d);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     mean_rows_kernel<<<1, 256, 0, st>>>(row_loss, B, loss);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -381,8 +381,8 @@ extern "C" int snb_certified_fraction(const float* yl, const float* yu, const lo
     if (B <= 0 || K <= 0) return SNB_ERR_BAD_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     certified_rows_kernel<<<(B + 7) / 8, 256, 0, st>>>(yl, yu, target, B, K, row_flag);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     mean_rows_kernel<<<1, 256, 0, st>>>(row_flag, B, fraction);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

@@ -564,7 +564,7 @@ cudaError_t launch(const Args& a, int smem, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const long long sms = sm_count(), want = (a.sl.total + WARPS - 1) / WARPS;
     KERN<<<(unsigned)(want < sms ? want : sms), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launched();
 }
 
 // Sizes and exponents from which the sparse form is the faster one (B200, dense -> sparse; 512 x 3840 x 3840 of masked
@@ -643,7 +643,7 @@ cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, cudaStream_t
     if ((e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
     if ((e = launch<skip_forward>(a, smem, st)) != cudaSuccess) return e;
     skip_finish<<<dim3((q.CO + 63) / 64, S), 256, 0, st>>>(a.sum, a.mt, q.B, q.CO, q.p, y);
-    return cudaGetLastError();
+    return launched(2);
 }
 
 cudaError_t lp_skip_backward(const LpProblem& q, const float* g, const float* y, float* gx, float* gw, void* ws, cudaStream_t st) {
@@ -660,7 +660,7 @@ cudaError_t lp_skip_backward(const LpProblem& q, const float* g, const float* y,
     const int smem = slab_bytes(a.sl, 256, 8);
     if ((e = fine ? launch<skip_backward<true>>(a, smem, st) : launch<skip_backward<false>>(a, smem, st)) != cudaSuccess) return e;
     skip_rows<<<dim3((q.CI + 63) / 64, S), 256, 0, st>>>(a.gxt, q.B, q.CI, gx);
-    return cudaGetLastError();
+    return launched(4);
 }
 
 }  // namespace snb

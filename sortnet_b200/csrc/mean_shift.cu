@@ -94,7 +94,7 @@ extern "C" int snb_mean_shift_stats(const float* x, const int* index, int B, int
     if ((long long)B * C >= (1ll << 31)) return SNB_ERR_TOO_LARGE;
     mean_shift_stats_kernel<<<(C_full + 15) / 16, 256, 0, (cudaStream_t)stream>>>(
         x, index, B, C, C_full, mean, running_mean, momentum);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -105,6 +105,6 @@ extern "C" int snb_mean_shift_apply(const float* x, const float* mean, const int
     if ((long long)B * C >= (1ll << 31)) return SNB_ERR_TOO_LARGE;
     dim3 grid((C + 255) / 256, (B + SNB_SUB_BATCH - 1) / SNB_SUB_BATCH);
     mean_shift_apply_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(x, mean, index, B, C, y);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

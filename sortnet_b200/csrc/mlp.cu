@@ -396,7 +396,7 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
         }
     if (masked) {
         keep_flags_kernel<<<dim3(S, masked), 256, 0, st>>>(jobs);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
         count++;
     }
     PrunePrep prep;
@@ -423,7 +423,7 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
         if (!head) {
             chain_shift_kernel<<<(C + SHIFT_C - 1) / SHIFT_C, 256, 0, st>>>(p.yt, p.part, p.keep, B, S, C, l[k].running_mean, l[k].momentum,
                                                               sv.rows_kept[k], sc.hi[k + 1], sc.nlo[k + 1]);
-            SNB_CUDA(cudaGetLastError());
+            SNB_CUDA(launched());
             count++;
         }
     }
@@ -463,14 +463,14 @@ extern "C" int snb_mlp_train_backward(const snb_mlp_layer* l, int depth, int B, 
         float* centred = rows[0];
         chain_center_kernel<<<(C + 31) / 32, 1024, 0, st>>>(g, head ? grad_loss : nullptr, head ? nullptr : sv.rows_kept[k], B, S, C,
                                                            centred, gt, head ? grad_bias : nullptr);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
         count++;
         float* gx = k > lowest ? rows[1] : (k == 0 ? grad_x : nullptr);
         const int nx = gx ? B : 0, nw = grad_w[k] ? C : 0;
         if (nx + nw > 0) {
             chain_bwd_kernel<<<nx + nw, 256, (CI + 3) / 4 * 16, st>>>(centred, gt, sv.pos[k], sv.post[k], B, S, C, CI, nx, gx,
                                                                       grad_w[k]);
-            SNB_CUDA(cudaGetLastError());
+            SNB_CUDA(launched());
             count++;
         }
         g = rows[1];
@@ -516,7 +516,7 @@ extern "C" int snb_mlp_eval_forward(const snb_mlp_layer* l, int depth, const flo
     if (score) {
         const int n = B * l[depth - 1].out;
         scores_kernel<<<(n + 255) / 256, 256, 0, st>>>(y, yl, yu, targets, B, l[depth - 1].out, inv_two_eps, scale, score, margin);
-        SNB_CUDA(cudaGetLastError());
+        SNB_CUDA(launched());
         count++;
     }
     if (launches) *launches = count + 1;

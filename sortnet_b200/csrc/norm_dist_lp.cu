@@ -490,7 +490,7 @@ static cudaError_t launch_lp_bwd(const LpBwdParams& q, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(q.gx, 0, sizeof(float) * (size_t)q.B * q.CI, st);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)(total < slots ? total : slots), NT, SMEM, st>>>(q);
-    return cudaGetLastError();
+    return launched();
 }
 
 // p.m == nullptr with NORM: the maxima are in y and no scratch is available -> one CTA per tile,
@@ -521,7 +521,7 @@ static cudaError_t launch_lp_fwd(LpFwdParams p, cudaStream_t st) {
     if (NORM && p.m == nullptr) p.m = p.y;
     if (p.direct) {
         kern<<<(unsigned)tiles, WN * 32, SMEM, st>>>(p);
-        return cudaGetLastError();
+        return launched();
     }
     const size_t n = (size_t)p.B * p.CO;
     cudaError_t e = cudaMemsetAsync(p.y, 0, sizeof(float) * n, st);
@@ -529,7 +529,7 @@ static cudaError_t launch_lp_fwd(LpFwdParams p, cudaStream_t st) {
     const long long units = tiles * ((p.CI + BK - 1) / BK);
     kern<<<(unsigned)(units < slots ? units : slots), WN * 32, SMEM, st>>>(p);
     lp_finish_kernel<<<sm_count() * 4, 256, 0, st>>>(p.y, NORM ? p.m : nullptr, (long long)n, 1.0f / p.p);
-    return cudaGetLastError();
+    return launched(2);
 }
 
 template <int IP, bool NORM>
@@ -654,7 +654,6 @@ static int lp_backward(const float* g, const float* x, const float* w, const flo
             else SNB_CUDA((launch_lp_bwd<-1, false>(q, st)));
             break;
     }
-    SNB_CUDA(cudaGetLastError());
     return SNB_OK;
 }
 

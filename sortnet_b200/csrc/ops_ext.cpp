@@ -9,7 +9,6 @@
 #include <dlfcn.h>
 #include <torch/extension.h>
 
-#include <atomic>
 #include <cmath>
 #include <stdexcept>
 #include <string>
@@ -46,8 +45,6 @@ struct Api {
     decltype(&snb_status_string) status_string;
     decltype(&snb_last_cuda_error) last_cuda_error;
 } api;
-std::atomic<long> launches{0};
-
 // A status code of the library: arrives in Python as the exception class that _lib.check raises.
 struct LibraryError : std::runtime_error {
     using std::runtime_error::runtime_error;
@@ -107,13 +104,12 @@ void check_list(const optional<Tensor>& t, const char* name, int64_t B, int64_t 
 }
 const int* list_ptr(const optional<Tensor>& t) { return t.has_value() ? t->data_ptr<int>() : nullptr; }
 
-void done(int rc, const char* what, int kernels) {
+void done(int rc, const char* what) {
     if (rc) {
         std::string why = api.status_string(rc);
         if (rc == SNB_STATUS_CUDA) why += std::string(": ") + api.last_cuda_error();
         throw LibraryError(std::string(what) + " failed: " + why + " (status " + std::to_string(rc) + ")");
     }
-    launches.fetch_add(kernels, std::memory_order_relaxed);
 }
 
 // Scratch of a forward call from PyTorch's caching allocator (stream-ordered).
@@ -158,7 +154,7 @@ DistOut dist_forward(const Tensor& x, const Tensor& w, const optional<Tensor>& c
         if (!record) {
             Area ws(x, 1, 1, 0, B, CO, CI, CO, CI, false, flat);
             done(api.inf_forward_nograd(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), ws.ptr,
-                                        ws.bytes, call.stream), "inf_dist_forward_nograd", 1);
+                                        ws.bytes, call.stream), "inf_dist_forward_nograd");
             return out;
         }
         out.pos = at::empty({B, CO, HW}, x.options().dtype(at::kInt));
@@ -167,12 +163,12 @@ DistOut dist_forward(const Tensor& x, const Tensor& w, const optional<Tensor>& c
                 !flat ? 0 : sorted ? api.inf_sorted_bytes(B, CO, W_CI) : sizeof(int64_t) * (size_t)(B * CO));
         auto f = sorted ? api.inf_forward_sorted : api.inf_forward;
         done(f(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), out.pos.data_ptr<int>(),
-               list_ptr(ci), list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "inf_dist_forward", 2);
+               list_ptr(ci), list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "inf_dist_forward");
         return out;
     }
     Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false, flat ? api.lp_bytes(0, B, CO, CI, W_CO, W_CI, (float)p, ci.has_value()) : 0);
     done(api.lp_forward(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, out.y.data_ptr<float>(), (float)p, list_ptr(ci),
-                        list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "norm_dist_forward", p > 10 ? 3 : 2);
+                        list_ptr(co), W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream), "norm_dist_forward");
     return out;
 }
 
@@ -208,10 +204,10 @@ struct DistFn : public torch::autograd::Function<DistFn> {
             if (need_w)
                 done(api.inf_backward_xw(gp, third.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), gw.data_ptr<float>(),
                                          list_ptr(ci), list_ptr(co), w.size(0), w.size(1) * G, call.stream),
-                     "inf_dist_backward_input_weight", 1);
+                     "inf_dist_backward_input_weight");
             else
                 done(api.inf_backward_x(gp, third.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), call.stream),
-                     "inf_dist_backward_input", 1);
+                     "inf_dist_backward_input");
         } else {
             const int64_t W_CO = w.size(0), W_CI = w.size(1);
             Area ws(x, 1, 1, 0, B, CO, CI, W_CO, W_CI, false, false,
@@ -219,7 +215,7 @@ struct DistFn : public torch::autograd::Function<DistFn> {
             done(api.lp_backward(gp, x.data_ptr<float>(), w.data_ptr<float>(), third.data_ptr<float>(), B, CO, CI, G, HW,
                                  gx.data_ptr<float>(), need_w ? gw.data_ptr<float>() : nullptr, (float)p, list_ptr(ci), list_ptr(co),
                                  W_CO, W_CI * G, ws.ptr, ws.bytes, call.stream),
-                 need_w ? "norm_dist_backward_input_weight" : "norm_dist_backward_input", 1);
+                 need_w ? "norm_dist_backward_input_weight" : "norm_dist_backward_input");
         }
         if (need_x) out[0] = gx;
         out[1] = gw;
@@ -247,10 +243,10 @@ Tensor sort_forward(const Tensor& x, const Tensor& w, int64_t G, double q, int64
     if (pos) {
         *pos = at::empty({K, B, CO, HW}, x.options().dtype(at::kInt));
         done(api.sort_forward(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, y.data_ptr<float>(), pos->data_ptr<int>(),
-                              (float)q, K, ws.ptr, ws.bytes, call.stream), "sort_neuron_forward", 1);
+                              (float)q, K, ws.ptr, ws.bytes, call.stream), "sort_neuron_forward");
     } else {
         done(api.sort_forward_nograd(x.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, y.data_ptr<float>(), (float)q, K,
-                                     ws.ptr, ws.bytes, call.stream), "sort_neuron_forward_nograd", 1);
+                                     ws.ptr, ws.bytes, call.stream), "sort_neuron_forward_nograd");
     }
     return y;
 }
@@ -279,10 +275,10 @@ struct SortFn : public torch::autograd::Function<SortFn> {
         Tensor gx = at::empty_like(x), gw = need_w ? at::empty_like(w) : Tensor();
         if (need_w)
             done(api.sort_backward_xw(g.data_ptr<float>(), pos.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(),
-                                      gw.data_ptr<float>(), q, K, call.stream), "sort_neuron_backward_input_weight", 1);
+                                      gw.data_ptr<float>(), q, K, call.stream), "sort_neuron_backward_input_weight");
         else
             done(api.sort_backward_x(g.data_ptr<float>(), pos.data_ptr<int>(), B, CO, CI, G, HW, gx.data_ptr<float>(), q, K,
-                                     call.stream), "sort_neuron_backward_input", 1);
+                                     call.stream), "sort_neuron_backward_input");
         if (need_x) out[0] = gx;
         out[1] = gw;
         return out;
@@ -307,11 +303,11 @@ std::tuple<Tensor, Tensor> bound_forward(const Tensor& xl, const Tensor& xu, con
         *words = at::empty({2, B, CO, HW}, xl.options().dtype(at::kInt));
         int* lw = words->data_ptr<int>();
         done(api.bound_forward(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, yl.data_ptr<float>(),
-                               yu.data_ptr<float>(), lw, lw + B * CO * HW, ws.ptr, ws.bytes, call.stream), "bound_inf_dist_forward", 1);
+                               yu.data_ptr<float>(), lw, lw + B * CO * HW, ws.ptr, ws.bytes, call.stream), "bound_inf_dist_forward");
     } else {
         done(api.bound_forward_nograd(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW,
                                       yl.data_ptr<float>(), yu.data_ptr<float>(), ws.ptr, ws.bytes, call.stream),
-             "bound_inf_dist_forward_nograd", 1);
+             "bound_inf_dist_forward_nograd");
     }
     return {yl, yu};
 }
@@ -344,10 +340,10 @@ struct BoundFn : public torch::autograd::Function<BoundFn> {
         const float *pl = g[0].data_ptr<float>(), *pu = g[1].data_ptr<float>();
         if (need_w)
             done(api.bound_backward_xw(pl, pu, lw, lw + B * CO * HW, B, CO, CI, G, HW, gl.data_ptr<float>(), gu.data_ptr<float>(),
-                                       gw.data_ptr<float>(), call.stream), "bound_inf_dist_backward_input_weight", 1);
+                                       gw.data_ptr<float>(), call.stream), "bound_inf_dist_backward_input_weight");
         else if (run)
             done(api.bound_backward_x(pl, pu, lw, lw + B * CO * HW, B, CO, CI, G, HW, gl.data_ptr<float>(), gu.data_ptr<float>(),
-                                      call.stream), "bound_inf_dist_backward_input", 1);
+                                      call.stream), "bound_inf_dist_backward_input");
         if (need_l) out[0] = gl;
         if (need_u) out[1] = gu;
         out[2] = gw;
@@ -372,7 +368,7 @@ std::tuple<Tensor, Tensor> bound_sort_neuron(const Tensor& xl, const Tensor& xu,
     Tensor yl = at::empty({B, CO, HW}, xl.options()), yu = at::empty({B, CO, HW}, xl.options());
     Area ws(xl, 2, K, 0, B, CO, CI, CO, CI, false, G == 1 && HW == 1);
     done(api.bound_sort_forward(xl.data_ptr<float>(), xu.data_ptr<float>(), w.data_ptr<float>(), B, CO, CI, G, HW, yl.data_ptr<float>(),
-                                yu.data_ptr<float>(), (float)q, K, ws.ptr, ws.bytes, call.stream), "bound_sort_neuron_forward", 1);
+                                yu.data_ptr<float>(), (float)q, K, ws.ptr, ws.bytes, call.stream), "bound_sort_neuron_forward");
     return {yl, yu};
 }
 
@@ -391,5 +387,4 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sort_neuron", &sort_neuron);
     m.def("bound_inf_dist", &bound_inf_dist);
     m.def("bound_sort_neuron", &bound_sort_neuron);
-    m.def("launches", [] { return launches.load(); });
 }

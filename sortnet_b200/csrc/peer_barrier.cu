@@ -84,7 +84,7 @@ static int launch_peer(void* const* flag_ptrs, int rank, int world, unsigned int
     }
     if (world == 1) return SNB_OK;
     peer_barrier_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(fp, rank, world, epoch, timeout_ns, status, what);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 

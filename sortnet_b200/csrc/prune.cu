@@ -1059,7 +1059,7 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
     prune_filter<R, NIT, FT, STAGES, VEC><<<steps < slots ? steps : slots, FT + 64 * R, smem, st>>>(a);
-    return cudaGetLastError();
+    return launched();
 }
 
 template <bool VEC>
@@ -1093,7 +1093,7 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
     prune_max<NX, TRACK><<<grid, 256, 0, st>>>(a);
     prune_redo_max<NX, TRACK><<<redo, REDO_THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launched(2);
 }
 
 template <int NX, int KMAX, bool POS>
@@ -1105,7 +1105,7 @@ cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     if ((e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo)) != cudaSuccess) return e;
     prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
     prune_redo_sort<NX, KMAX, POS><<<redo, 256, 0, st>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess || !POS) return e;
+    if ((e = launched(2)) != cudaSuccess || !POS) return e;
     return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
 }
 
@@ -1127,7 +1127,7 @@ cudaError_t prune_prepare(const PrunePrep& q, cudaStream_t st) {
     if (!q.x) prune_prep<2><<<grid, 256, 0, st>>>(q);
     else if (q.box || q.xl) prune_prep<3><<<grid, 256, 0, st>>>(q);
     else prune_prep<1><<<grid, 256, 0, st>>>(q);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {

@@ -8,6 +8,13 @@ static thread_local cudaError_t g_last = cudaSuccess;
 
 void set_last_cuda_error(cudaError_t e) { g_last = e; }
 
+static std::atomic<long long> g_launched{0};
+
+cudaError_t launched(int n) {
+    g_launched.fetch_add(n, std::memory_order_relaxed);
+    return cudaGetLastError();
+}
+
 int sm_count() {
     static std::atomic<int> cached[64];
     int dev = 0;
@@ -40,5 +47,7 @@ extern "C" const char* snb_status_string(int status) {
 }
 
 extern "C" const char* snb_last_cuda_error(void) { return cudaGetErrorString(snb::g_last); }
+
+extern "C" long long snb_launch_count(void) { return snb::g_launched.load(std::memory_order_relaxed); }
 
 extern "C" int snb_version(void) { return 100; }

@@ -202,7 +202,7 @@ extern "C" int snb_check_index_lists(const int* index, int lists, int count, int
     const long long n = (long long)lists * count;
     const int blocks = (int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
     check_index_kernel<<<blocks, 256, 0, st>>>(index, n, count, channels);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     SNB_CUDA(cudaMemcpyFromSymbolAsync(&bits, snb_index_check_bits, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
     SNB_CUDA(cudaStreamSynchronize(st));
     if (flags) *flags = bits;
@@ -245,7 +245,7 @@ extern "C" int snb_sample_mask_batch(int jobs, int* const* outs, const int* chan
     int rc = configure_sampler();
     if (rc) return rc;
     sample_mask_batch_kernel<<<jobs * lists, SM_THREADS, smem, (cudaStream_t)stream>>>(table, lists);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -259,6 +259,6 @@ extern "C" int snb_sample_mask(int* out, int lists, int channels, int count, uns
     if (rc) return rc;
     sample_mask_kernel<<<lists, SM_THREADS, smem, (cudaStream_t)stream>>>(out, channels, count, (uint32_t)seed,
                                                                          (uint32_t)(seed >> 32));
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

@@ -474,7 +474,7 @@ cudaError_t sort_positions_if(const PruneProblem& q, const unsigned* overflowed,
     const int grid = 4 * sm_count();
     if (q.K <= 16) sort_fwd_pos<true, true><<<grid, SP_THREADS, 0, st>>>(p, overflowed);
     else sort_fwd_pos<false, true><<<grid, SP_THREADS, 0, st>>>(p, overflowed);
-    return cudaGetLastError();
+    return launched();
 }
 
 // Sparse backward: one CTA per batch row, grad_x of the row accumulated in shared memory.
@@ -524,7 +524,7 @@ static cudaError_t launch_sort_fwd(const SortParams& p, cudaStream_t st) {
     }
     dim3 grid((p.B + BM - 1) / BM, (p.CO + BN - 1) / BN);
     kern<<<grid, 256, SMEM, st>>>(p);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace snb
@@ -592,7 +592,7 @@ extern "C" int snb_sort_neuron_forward_ws(const float* x, const float* w, int B,
     dim3 grid((B + SP_ROWS - 1) / SP_ROWS, (CO + SP_COLS - 1) / SP_COLS);
     if (K <= 16) sort_fwd_pos<true, false><<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p, nullptr);
     else sort_fwd_pos<false, false><<<grid, SP_THREADS, 0, (cudaStream_t)stream>>>(p, nullptr);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -638,7 +638,7 @@ static int sort_backward(const float* g, const int* pos, int B, int CO, int CI, 
     float n = powf(1 - q, (float)K);
     n = 1.0f + n / (1.0f - n);
     sort_bwd_kernel<<<B, 256, use_smem ? CI * sizeof(float) : 0, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 

@@ -77,7 +77,7 @@ extern "C" int snb_unfold(const float* x, int B, int C, int H, int W, int kh, in
     if (int rc = make_patch_geo(B, C, H, W, kh, kw, stride, pad, dil, &q)) return rc;
     const long long n = (long long)B * C * kh * kw * q.oh * q.ow;
     unfold_kernel<<<patch_blocks(n), 256, 0, (cudaStream_t)stream>>>(x, out, q, n);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -88,7 +88,7 @@ extern "C" int snb_fold(const float* g, int B, int C, int H, int W, int kh, int 
     if (int rc = make_patch_geo(B, C, H, W, kh, kw, stride, pad, dil, &q)) return rc;
     const long long n = (long long)B * C * H * W;
     fold_kernel<<<patch_blocks(n), 256, 0, (cudaStream_t)stream>>>(g, gx, q, n);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }
 
@@ -97,6 +97,6 @@ extern "C" int snb_plane_index(const int* index, int S, int G, int kept, int cha
     if (S <= 0 || G <= 0 || kept <= 0 || hw <= 0 || channels <= 0 || channels % G) return SNB_ERR_BAD_SHAPE;
     const long long n = (long long)S * G * kept * hw;
     plane_index_kernel<<<patch_blocks(n), 256, 0, (cudaStream_t)stream>>>(index, G, kept, channels / G, hw, out, n);
-    SNB_CUDA(cudaGetLastError());
+    SNB_CUDA(launched());
     return SNB_OK;
 }

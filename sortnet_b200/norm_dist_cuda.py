@@ -79,43 +79,30 @@ def _dims(x, out):
     return x.size(0), out.size(1), x.size(1), x.size(2)
 
 
-# Kernels launched by each C entry point (memsets are not counted).
-_KERNELS = {
-    "snb_inf_dist_forward": 2, "snb_inf_dist_forward_ws": 2, "snb_inf_dist_forward_sorted_ws": 3, "snb_inf_dist_forward_nograd_ws": 1, "snb_inf_dist_backward_input": 1,
-    "snb_inf_dist_backward_input_weight": 1, "snb_norm_dist_forward": 1, "snb_norm_dist_forward_ws": 2, "snb_norm_dist_backward_ws": 1,
-    "snb_bound_inf_dist_forward_nograd_ws": 1,
-    "snb_bound_inf_dist_forward_ws": 1, "snb_bound_inf_dist_backward_input": 1,
-    "snb_bound_inf_dist_backward_input_weight": 1, "snb_unfold": 1, "snb_fold": 1, "snb_plane_index": 1, "snb_mean_shift_stats": 1, "snb_mean_shift_apply": 1, "snb_sample_mask": 1, "snb_sample_mask_batch": 1,
-    "snb_sort_neuron_forward_nograd_ws": 1, "snb_sort_neuron_forward_ws": 1, "snb_bound_sort_neuron_forward_ws": 1,
-    "snb_sort_neuron_backward_input": 1, "snb_sort_neuron_backward_input_weight": 1,
-}
-
-_launched = 0             # kernels launched from Python since import / reset_counters()
-_native_base = 0          # the native operator layer's count at the last reset
+_counted_from = 0         # the library's launch counter at the last reset
 _timeline = None          # when profiling: list of (entry point, work tag, start event, end event)
 
 
 class _Module(types.ModuleType):
-    """`launch_count`: kernels launched since import / reset_counters(), by this module and by the native
-    operator layer; assignable (callers that launch through the library themselves add to it)."""
+    """`launch_count`: kernels launched through the library since import / reset_counters(), whoever called it
+    (snb_launch_count); assignable."""
 
     @property
     def launch_count(self):
-        return _launched + (_lib._ops.launches() - _native_base if _lib._ops is not None else 0)
+        return _lib.load().snb_launch_count() - _counted_from
 
     @launch_count.setter
     def launch_count(self, value):
-        global _launched
-        _launched += value - self.launch_count
+        global _counted_from
+        _counted_from = _lib.load().snb_launch_count() - value
 
 
 sys.modules[__name__].__class__ = _Module
 
 
 def reset_counters():
-    global _launched, _native_base
-    _launched = 0
-    _native_base = _lib._ops.launches() if _lib._ops is not None else 0
+    global _counted_from
+    _counted_from = _lib.load().snb_launch_count()
 
 
 def start_profile():
@@ -142,7 +129,6 @@ def _stream(dev):
 
 def _call(dev, ref_tensor, entry, tag, *args):
     """Runs C entry point `entry` with `dev` current, on the current stream of that device."""
-    global _launched
     fn = getattr(_lib.load(), entry)
     if _timeline is None and torch.cuda.current_device() == dev.index:
         rc = fn(*args, _stream(dev))
@@ -158,9 +144,6 @@ def _call(dev, ref_tensor, entry, tag, *args):
                 e1.record(stream)
                 _timeline.append((entry, tag, e0, e1))
     _lib.check(rc, entry[4:])
-    _launched += _KERNELS[entry]
-    if entry in ("snb_norm_dist_forward", "snb_norm_dist_forward_ws") and args[8] > 10.0:
-        _launched += 1      # the l-inf pass that supplies the normaliser
 
 
 def _same_device(*ts):
@@ -545,15 +528,10 @@ def plane_index(index, channels, hw):
 
 # ---- whole layers and the model head (one C call each; G = 1, HW = 1, 2-D tensors) ---------------
 
-_LAYER_KERNELS = {"snb_layer_forward": 4, "snb_layer_backward_ws": 4, "snb_layer_bound_forward_ws": 3, "snb_input_box": 1,
-                  "snb_margin_loss": 2, "snb_certified_fraction": 2}
-
-
 def _layer_call(entry, tag, ref, *args):
     """Lean variant of _call for the layer-level entry points: the callers in ops.py / layers.py own
     every tensor they pass (fresh allocations of the right shape and dtype), so only the device is
     looked after here."""
-    global _launched
     if _timeline is not None:
         return _call(ref.device, ref, entry, tag, *args)
     dev = ref.device
@@ -565,10 +543,6 @@ def _layer_call(entry, tag, ref, *args):
             rc = fn(*args, _stream(dev))
     if rc:
         _lib.check(rc, entry[4:])
-    _launched += _LAYER_KERNELS[entry]
-
-
-_KERNELS.update(_LAYER_KERNELS)
 
 
 def layer_forward(x, weight, p, w_index_ci, w_index_co, y_dist, pos, workspace, running_mean, momentum, mean, bias,
@@ -677,17 +651,15 @@ class MlpPlan:
 
 
 def _mlp_call(entry, ref, *args):
-    """Runs a snb_mlp_* entry point with the device of `ref` current; counts what it launched."""
-    global _launched
-    dev, fn, n = ref.device, getattr(_lib.load(), entry), ctypes.c_int(0)
+    """Runs a snb_mlp_* entry point with the device of `ref` current."""
+    dev, fn = ref.device, getattr(_lib.load(), entry)
     if torch.cuda.current_device() == dev.index:
-        rc = fn(*args, ctypes.byref(n), _stream(dev))
+        rc = fn(*args, None, _stream(dev))
     else:
         with torch.cuda.device(dev):
-            rc = fn(*args, ctypes.byref(n), _stream(dev))
+            rc = fn(*args, None, _stream(dev))
     if rc:
         _lib.check(rc, entry[4:])
-    _launched += n.value
 
 
 def targets_fit(targets, x):

@@ -16,7 +16,6 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
-from . import norm_dist_cuda as _C
 
 # Only plain peer loads, stores and copies are used here: keep symmetric memory off the NVLink
 # multicast objects (a rank that dies while bound to one disturbs its peers' GPUs).
@@ -171,7 +170,6 @@ class FlatAdamW:
         if rc != 0:
             self._failed = "peer barrier could not be launched"
         _lib.check(rc, "peer_barrier")
-        _C.launch_count += 1
 
     def check(self):
         """Raises if a barrier of an earlier step gave up on a peer (reads a pinned host word, no
@@ -189,7 +187,6 @@ class FlatAdamW:
         if rc != 0:
             self._failed = "peer signal could not be launched"
         _lib.check(rc, "peer_signal")
-        _C.launch_count += 1
         return self._epoch
 
     def _wait(self, epoch, stream):
@@ -198,7 +195,6 @@ class FlatAdamW:
         if rc != 0:
             self._failed = "peer wait could not be launched"
         _lib.check(rc, "peer_wait")
-        _C.launch_count += 1
 
     def begin_exchange(self):
         """Opens the gradient exchange behind everything that is on the current stream now (the
@@ -278,7 +274,6 @@ class FlatAdamW:
                 if rc != 0:
                     self._failed = "the shard update could not be launched"
                 _lib.check(rc, "adamw_reduce_step")
-                _C.launch_count += 1
             self._updated.record(main)
             self._side.wait_event(self._updated)
             with torch.cuda.stream(self._side):
@@ -381,7 +376,6 @@ class FlatAdamW:
                 if rc != 0:
                     self._failed = "the fused exchange kernel could not be launched"
                 _lib.check(rc, "dp_adamw_step")
-                _C.launch_count += 1
                 # ... and every rank's new parameters have landed here before the next forward
                 self._barrier(stream)
             self._grads_consumed()
@@ -393,5 +387,4 @@ class FlatAdamW:
                 float(self.betas[1]), float(self.eps), float(self.weight_decay), self.step_count,
                 1.0 / self.world, torch.cuda.current_stream(dev).cuda_stream)
         _lib.check(rc, "adamw_step")
-        _C.launch_count += 1
         self._grads_consumed()

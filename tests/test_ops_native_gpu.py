@@ -174,3 +174,41 @@ def both_errors(fn):
             fn()
         return info.value
     return both(caught)
+
+
+def test_launch_count_is_what_the_device_ran():
+    """snb_launch_count against the profiler's list, over entry points of every kind."""
+    from torch.profiler import ProfilerActivity, profile
+    from sortnet_b200 import layers, norm_dist_cuda as C, ops
+    from sortnet_b200.optim import FlatAdamW
+    x, w, gy = operands(70, 1024, 1000)
+    small, ws, gs = operands(9, 40, 20)
+    model = layers.SortMLPModel(depth=4, width=700, input_dim=(3, 17, 17), num_classes=10, dropout=0.8).cuda().train()
+    images, labels = torch.rand(70, 3, 17, 17, device="cuda"), torch.randint(0, 10, (70,), device="cuda")
+    opt = FlatAdamW(model)
+
+    def work():
+        for a, b, g in ((x, w, gy), (small, ws, gs)):
+            for p in (INF, 3.0, 60.0):
+                torch.autograd.grad(ops.norm_dist(a, b, p), (a, b), g)
+            torch.autograd.grad(ops.sort_neuron(a, b, q=0.8), (a, b), g)
+            torch.autograd.grad(ops.bound_inf_dist(a, a, b)[0], (a, b), g)
+            ops.bound_sort_neuron(a.detach(), a.detach(), b.detach(), q=0.8)
+        for p in (INF, 3.0):
+            model.set_p(p)
+            model.mixture_loss(images, labels, 0.05).backward()
+            opt.step()
+        model.set_p(INF)
+        with torch.no_grad():
+            model.eval()(images, labels, 0.02, up=1.0, down=0.0)
+            model.train()
+
+    work()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        C.reset_counters()
+        work()
+        torch.cuda.synchronize()
+        counted = C.launch_count
+    ours = [e.name for e in prof.events() if e.device_type.name == "CUDA" and "snb::" in e.name]
+    assert len(ours) > 60 and counted == len(ours), (counted, len(ours))
