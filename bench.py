@@ -12,9 +12,10 @@ with the CIFAR-10 shapes ([512, 3, 32, 32] uniform in [0, 1), labels uniform in 
 weights N(0, 1); the per-GPU batch is fixed as N grows (weak scaling).
 
 Prints one JSON line (rank 0).  `value` is samples/s with inputs resident in HBM; `e2e` is the
-same step fed from pinned host memory with the loss read back every step; `roofline` is the
-dominant kernel's FP32 fraction, its time taken from CUDA events around its launches in a short
-separate pass (the headline regions run without those events); `cpu_baseline` is the
+same step fed from pinned host memory with the loss read back every step; `roofline` sets the bytes
+that the entry point with the largest share of the step must move, over its time, against the
+measured copy bandwidth (CUDA events around its calls in a short separate pass; the headline
+regions run without those events); `cpu_baseline` is the
 reference's PyTorch way of computing the same step timed on this host's cores.  Secondary
 blocks (never the headline): `gpu_comparator` (the same step through the reference's own model
 code and CUDA kernels compiled for sm_100a, when oracle/_ref holds them), `configs[0]`,
@@ -57,17 +58,6 @@ ADAM = dict(lr=0.02, betas=(0.9, 0.99), eps=1e-10, weight_decay=0.0)
 # loading, first-launch set-up) seconds apart on a busy host; a rank that is really gone still ends
 # the run with an error instead of a hang
 PEER_WAIT_S = 30.0
-
-# dram__bytes_read.sum + dram__bytes_write.sum per launch from the ncu captures summarised under
-# profiles/ (bound_fwd_kernel_64x256_512x5120x5120.md; inf_fwd_sk_kernel_masked_512x4619x4596.md,
-# all kernels of the entry point), at the shapes of the widest layers of the headline workload.
-NCU_DRAM_BYTES_PER_LAUNCH = {
-    "snb_bound_inf_dist_forward_nograd": 302.8e6,
-    "snb_inf_dist_forward_ws": 262.2e6,
-    "snb_inf_dist_forward_sorted_ws": 266.2e6,
-    "snb_inf_dist_forward_nograd": 203.9e6,       # inf_fwd_sk_kernel_dense_512x5120x5120.md
-}
-
 
 # adamw_kernel: 480.0 MB read + 302.2-304.4 MB written per launch on 30 M parameters (ncu, the capture
 # of profiles/adamw_kernel_30m_parameters.md; the last writes are still in L2 when the kernel ends);
@@ -450,10 +440,6 @@ def fp32_peak_gflops(dev):
     return best * 1e-9
 
 
-PEAK_SOURCE = ("FFMA probe timed in this run (2 flops per FMA); MEASURED_PEAKS.json has no FP32 figure; nominal "
-               "148 SM x 128 lanes x 2 x 1.965 GHz = 74.5 TFLOP/s")
-
-
 def kernel_stats(timeline, entry):
     """Launches of `entry` on the widest layers (mask sizes differ a little from step to step, so
     every shape within 10 % of the largest counts): a representative shape, the mean time per
@@ -472,8 +458,9 @@ def kernel_stats(timeline, entry):
 
 def profiled_pass(job, steps, **kw):
     """A few steps with a CUDA-event pair around every entry-point call: {(entry, shape): [ms]}.
-    The layers are run operator by operator here (the same kernels in the same order as the
-    one-call-per-layer path of the headline regions), so that every kernel gets its own events."""
+    The layers are run operator by operator here (the same evaluation as in the whole-net calls of
+    the headline regions, csrc/mlp.cu, with a pass between the layers instead of the chain form), so
+    that every entry point gets its own events."""
     from sortnet_b200 import layers, norm_dist_cuda as C
     layers.FUSED_LAYERS = False
     try:
@@ -485,35 +472,65 @@ def profiled_pass(job, steps, **kw):
         layers.FUSED_LAYERS = True
 
 
-def roofline_blocks(timeline, peak_gflops):
+def measured_hbm():
+    """(GB/s, source): the measured copy bandwidth of this pool's B200s."""
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            return float(json.load(f)["hbm_gbs"]), "MEASURED_PEAKS.json hbm_gbs (STREAM-style copy)"
+    except Exception:
+        return 6650.0, "fallback 6.65 TB/s (MEASURED_PEAKS.json absent)"
+
+
+# Words of 4 bytes that a call cannot do without, per (rows B, outputs CO, inputs CI) and the full weight matrix W: the pruned
+# and sparse forms look at few of the (row, output, input) terms, so it is the bytes that bound them from below.
+MUST_MOVE = {
+    "snb_bound_inf_dist_forward_nograd_ws": lambda B, CO, CI, W: W + 2 * B * CI + 2 * B * CO,
+    "snb_inf_dist_forward_sorted_ws": lambda B, CO, CI, W: W + B * CI + 2 * B * CO,
+    "snb_inf_dist_forward_ws": lambda B, CO, CI, W: W + B * CI + 2 * B * CO,
+    "snb_inf_dist_forward_nograd_ws": lambda B, CO, CI, W: W + B * CI + B * CO,
+    "snb_inf_dist_backward_input_weight": lambda B, CO, CI, W: W + 2 * B * CO + B * CI,
+    "snb_norm_dist_forward_ws": lambda B, CO, CI, W: W + B * CI + B * CO,
+    "snb_norm_dist_backward_ws": lambda B, CO, CI, W: 2 * W + 2 * B * CI + 2 * B * CO,
+}
+
+
+def bytes_roof(timeline, entry, width):
+    """Bytes that `entry` must move on the widest layers over the time it takes, against the copy bandwidth."""
+    ks = kernel_stats(timeline, entry)
+    if ks is None:
+        return None
+    (b_, co_, ci_), mean_ms, _ = ks
+    nbytes = 4 * MUST_MOVE[entry](b_, co_, ci_, width * width)
+    peak, source = measured_hbm()
+    achieved = nbytes / (mean_ms * 1e-3) * 1e-9
+    return {"bound": "hbm", "kernel": entry[4:], "shape_B_CO_CI": [b_, co_, ci_], "algorithmic_bytes": nbytes,
+            "ms_per_launch": round(mean_ms, 4), "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+            "frac": round(achieved / peak, 4), "traffic": None, "peak_source": source}
+
+
+def roofline_blocks(timeline, width, expected):
+    """Shares of the entry points in the profiled steps, and the roofline of those in `expected`; an entry that is not there
+    or does better than memory allows is a mistake of this file and says so."""
     by_entry = {}
     for (entry, tag), v in timeline.items():
         by_entry[entry] = by_entry.get(entry, 0.0) + sum(v)
     total = sum(by_entry.values())
     shares = {k[4:]: round(v / total, 4) for k, v in sorted(by_entry.items(), key=lambda kv: -kv[1])}
     roofs = {}
-    for entry, ops_per_elem in (("snb_bound_inf_dist_forward_nograd", 6.0), ("snb_inf_dist_forward_sorted_ws", 2.0),
-                                ("snb_inf_dist_forward_ws", 2.0), ("snb_inf_dist_forward_nograd", 2.0)):
-        ks = kernel_stats(timeline, entry)
-        if ks is None:
-            continue
-        (b_, co_, ci_), mean_ms, mean_elems = ks
-        achieved = ops_per_elem * mean_elems / (mean_ms * 1e-3) * 1e-9
-        roofs[entry] = {
-            "bound": "fp32", "kernel": entry[4:], "shape_B_CO_CI": [b_, co_, ci_],
-            "ops_per_element": ops_per_elem, "ms_per_launch": round(mean_ms, 4),
-            "achieved": round(achieved, 1), "peak": round(peak_gflops, 1), "unit": "GFLOP/s",
-            "frac": round(achieved / peak_gflops, 4), "traffic": NCU_DRAM_BYTES_PER_LAUNCH.get(entry),
-            "peak_source": PEAK_SOURCE,
-        }
-    dominant = max(roofs.values(), key=lambda r: by_entry.get("snb_" + r["kernel"], 0.0)) if roofs else None
+    for entry in expected:
+        roof = bytes_roof(timeline, entry, width)
+        roofs[entry] = roof if roof is not None else {"kernel": entry[4:], "error": "not among the profiled calls"}
+        if roof is not None and roof["frac"] > 1.0:
+            roof["error"] = "more than the copy bandwidth: the byte count or the timing is wrong"
+    timed_roofs = [r for r in roofs.values() if "frac" in r]
+    dominant = max(timed_roofs, key=lambda r: by_entry.get("snb_" + r["kernel"], 0.0)) if timed_roofs else None
     return shares, roofs, dominant, total
 
 
-def lp_blocks(job, peak_gflops, sm_mhz):
+def lp_blocks(job):
     """The p-annealed phases of the recipe (p = 8, then a general p) on the headline model: one masked
     training step without the bound pass, device-timed over 10 steps, plus the generic-p kernels
-    against the special-function-unit roof (2 transcendentals per element; 16 per clock per SM)."""
+    against the bytes that they must move."""
     import torch
     out, roof = {}, None
     for p_val in (8.0, 31.6):
@@ -522,20 +539,10 @@ def lp_blocks(job, peak_gflops, sm_mhz):
         out["p=%g" % p_val] = {"ms_per_step": round(ms, 3), "samples_per_s": round(job.B / (ms * 1e-3), 1), "steps": 10}
         if p_val == 31.6:
             tl = profiled_pass(job, 2, bounds=False)
-            sms = torch.cuda.get_device_properties(job.dev).multi_processor_count
-            xu_peak = 16.0 * sms * (sm_mhz or 1965.0) * 1e6 * 1e-9          # G transcendentals / s
-            roof = {"bound": "xu (special-function unit)", "peak": round(xu_peak, 1), "unit": "G transcendental/s",
-                    "peak_source": "16 per clock per SM x %d SMs x %s MHz (median SM clock of this run)" % (sms, sm_mhz),
-                    "ops_per_element": 2.0, "p": 31.6}
-            for entry, key in (("snb_norm_dist_forward_ws", "forward"), ("snb_norm_dist_backward_ws", "backward")):
-                ks = kernel_stats(tl, entry)
-                if ks is None:
-                    continue
-                shape, mean_ms, elems = ks
-                ach = 2.0 * elems / (mean_ms * 1e-3) * 1e-9
-                roof[key] = {"shape_B_CO_CI": list(shape), "ms_per_launch": round(mean_ms, 4),
-                             "achieved": round(ach, 1), "frac": round(ach / xu_peak, 4)}
-            roof["note"] = "the forward's time includes the l-inf pass that supplies the normaliser and the root kernel"
+            _, roof, _, _ = roofline_blocks(tl, job.cfg["width"], ("snb_norm_dist_forward_ws", "snb_norm_dist_backward_ws"))
+            roof = {"p": 31.6, "forward": roof["snb_norm_dist_forward_ws"], "backward": roof["snb_norm_dist_backward_ws"],
+                    "note": "evaluated are the terms that can matter; the special-function unit bounds those (75 % busy, "
+                            "profiles/lp_skip_kernels.md).  The forward's time includes the maxima that supply the normaliser"}
     job.model.set_p(INF)
     return out, roof
 
@@ -545,13 +552,7 @@ def hbm_block(job):
     against the measured copy bandwidth of this pool's B200s."""
     import torch
     opt = job.opt
-    hbm_peak, hbm_src = 6650.0, "fallback 6.65 TB/s (MEASURED_PEAKS.json absent)"
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            hbm_peak = float(json.load(f)["hbm_gbs"])
-            hbm_src = "MEASURED_PEAKS.json hbm_gbs (STREAM-style copy)"
-    except Exception:
-        pass
+    hbm_peak, hbm_src = measured_hbm()
     def one_step():
         opt.set_flat_grad()                    # keep the gradients of the last backward: the step then
         opt.step()                             # is the update kernel alone, as inside a training step
@@ -572,7 +573,7 @@ def hbm_block(job):
             "peak_source": hbm_src}
 
 
-def single_layer_block(dev, peak_gflops):
+def single_layer_block(dev):
     """one l-inf layer, x [128, 784], W [5120, 784], box [x - 0.3, x + 0.3] clipped to
     [0, 1]: forward with argmax words, sparse backward, interval bounds, each device-timed.  The
     weights rotate through 9 copies (145 MB) so that no launch finds its operands in L2."""
@@ -600,16 +601,14 @@ def single_layer_block(dev, peak_gflops):
         torch.cuda.synchronize()
         return a.elapsed_time(b) / iters
 
-    E = B * CI * CO
     t_f = timed(lambda w: C.inf_dist_forward(x, w, y, pos, 1))
     t_b = timed(lambda w: C.inf_dist_backward_input_weight(gy, pos, gx, gw, 1))
     t_i = timed(lambda w: C.bound_inf_dist_forward_nograd(xl, xu, w, yl, yu, 1))
-    frac = lambda ops, ms: round(ops * E / (ms * 1e-3) * 1e-9 / peak_gflops, 4)
-    bwd_bytes = 8 * B * CO + 4 * B * CI + 4 * CO * CI      # g + pos read, grad_x written, grad_w zero-filled
+    gbs = lambda entry, ms: round(4 * MUST_MOVE[entry](B, CO, CI, CO * CI) / (ms * 1e-3) * 1e-9, 1)
     return {"workload": "configs[0]: single l-inf layer 128 x 784 -> 5120, fwd + argmax, sparse bwd, interval bounds",
-            "forward_ms": round(t_f, 4), "forward_frac_fp32": frac(2.0, t_f),
-            "backward_ms": round(t_b, 4), "backward_gbs": round(bwd_bytes / (t_b * 1e-3) * 1e-9, 1),
-            "bounds_ms": round(t_i, 4), "bounds_frac_fp32": frac(6.0, t_i),
+            "forward_ms": round(t_f, 4), "forward_gbs": gbs("snb_inf_dist_forward_ws", t_f),
+            "backward_ms": round(t_b, 4), "backward_gbs": gbs("snb_inf_dist_backward_input_weight", t_b),
+            "bounds_ms": round(t_i, 4), "bounds_gbs": gbs("snb_bound_inf_dist_forward_nograd_ws", t_i),
             "samples_per_s": round(B / ((t_f + t_b + t_i) * 1e-3), 1), "l2": "weights rotate through 145 MB"}
 
 
@@ -937,17 +936,22 @@ def run_gpu_arm(args):
             "clocks": clocks,
         }
         if timeline:
-            shares, roofs, dominant, total_kernel_ms = roofline_blocks(timeline, peak_gflops)
-            line.update({"roofline": dominant, "roofline_linf_forward": roofs.get("snb_inf_dist_forward_sorted_ws") or roofs.get("snb_inf_dist_forward_ws"),
-                         "roofline_linf_point_forward": roofs.get("snb_inf_dist_forward_nograd"),
+            shares, roofs, dominant, total_kernel_ms = roofline_blocks(
+                timeline, HEADLINE["width"], ("snb_inf_dist_forward_sorted_ws", "snb_inf_dist_forward_nograd_ws",
+                                              "snb_bound_inf_dist_forward_nograd_ws", "snb_inf_dist_backward_input_weight"))
+            line.update({"roofline": dominant, "roofline_linf_forward": roofs["snb_inf_dist_forward_sorted_ws"],
+                         "roofline_linf_point_forward": roofs["snb_inf_dist_forward_nograd_ws"],
+                         "roofline_interval_bounds": roofs["snb_bound_inf_dist_forward_nograd_ws"],
+                         "roofline_linf_backward": roofs["snb_inf_dist_backward_input_weight"],
+                         "fp32_probe_gflops": round(peak_gflops, 1),
                          "kernel_time_share": shares, "kernel_ms_per_step": round(total_kernel_ms / 3, 3),
                          "kernel_time_source": "3 extra steps, run operator by operator with a CUDA-event pair around "
-                                               "every entry-point call; the headline regions run one library call "
-                                               "per layer without those events"})
+                                               "every entry-point call; the headline regions run the whole net in "
+                                               "one library call per direction without those events"})
         line.update(extra)
         if world == 1 and not args.no_extras:
             line["roofline_hbm"] = hbm_block(job)
-            lp, lp_roof = lp_blocks(job, peak_gflops, clocks.get("sm_mhz"))
+            lp, lp_roof = lp_blocks(job)
             line["lp_training_step"] = lp
             if lp_roof:
                 line["roofline_lp"] = lp_roof
@@ -960,7 +964,7 @@ def run_gpu_arm(args):
                 cmp_block["speedup"] = round(cmp_block["ms_per_step"] / ms, 3)
             line["gpu_comparator"] = cmp_block
             job.release()
-            line["configs[0]"] = single_layer_block(dev, peak_gflops)
+            line["configs[0]"] = single_layer_block(dev)
             line["configs[2]"] = config_step_block(2, dev)
             line["configs[3]"] = config_step_block(3, dev)
         if world == 1 and not args.no_cpu_baseline:
