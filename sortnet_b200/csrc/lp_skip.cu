@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) skip_transpose(const float* __restrict__ 
 // ---- slabs ------------------------------------------------------------------------------------------
 // A slab is one sub-batch x one chunk of the inner index (columns in the forward, outputs in the backward), in shared
 // memory.  The pairs (slab, outer index) form one sequence, cut into gridDim.x equal ranges; within a slab the warps of
-// the CTA take every 16th outer index and need no barrier.
+// the CTA take every 32nd outer index and need no barrier.
 struct Slabs {
     int inner, outer, chunk, chunks;
     long long total;                        // sub-batches * chunks * outer
@@ -388,7 +388,7 @@ struct BackwardArgs {
     float pm1, cut;
 };
 
-// Per warp: a column, with its 32 values of x and their range in registers; its lanes test 128 outputs at a time against
+// Per warp: a column, with its 32 values of x and their range in registers; its lanes test 256 outputs at a time against
 // the column of W.  Of 16 queued outputs every group evaluates four; the sums over the rows go to grad_w with one reduction
 // per pair, grad_x stays in registers for the length of the slab.  FINE as in lp_bwd_kernel: ratios near 1 take the
 // series and the remainder of the rounded product.  Bounds as in the forward; 512 x 3840 x 3840: p = 31.6 4.23 -> 1.48 ms,

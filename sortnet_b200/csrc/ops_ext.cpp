@@ -12,6 +12,8 @@
 #include <cmath>
 #include <stdexcept>
 #include <string>
+#include <tuple>
+#include <vector>
 
 #include "../../include/sortnet_b200.h"
 
@@ -372,6 +374,25 @@ std::tuple<Tensor, Tensor> bound_sort_neuron(const Tensor& xl, const Tensor& xu,
     return {yl, yu};
 }
 
+// ---- whole nets ------------------------------------------------------------------------------------
+// Whether every tensor of a layer table is what the kernels read through its pointer: fp32 (int32 lists), contiguous, on the
+// device of x [B, in], of the shapes of a chain of layers.  rows: (weight, bias, running mean, kept list) per layer.
+using Row = std::tuple<Tensor, optional<Tensor>, optional<Tensor>, optional<Tensor>>;
+bool mlp_takes(const Tensor& x, const std::vector<Row>& rows) {
+    if (x.dim() != 2) return false;
+    const int64_t subs = (x.size(0) + 31) / 32;
+    int64_t width = x.size(1);
+    auto plain = [&](const Tensor& t, at::ScalarType type) { return t.device() == x.device() && t.scalar_type() == type && t.is_contiguous(); };
+    for (const auto& [w, bias, mean, kept] : rows) {
+        if (w.dim() != 2 || w.size(1) != width || !plain(w, at::kFloat)) return false;
+        width = w.size(0);
+        for (const auto* t : {&bias, &mean})
+            if (t->has_value() && ((*t)->dim() != 1 || (*t)->size(0) != width || !plain(**t, at::kFloat))) return false;
+        if (kept.has_value() && (kept->dim() != 3 || kept->size(0) != subs || kept->size(1) != 1 || !plain(*kept, at::kInt))) return false;
+    }
+    return true;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -387,4 +408,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sort_neuron", &sort_neuron);
     m.def("bound_inf_dist", &bound_inf_dist);
     m.def("bound_sort_neuron", &bound_sort_neuron);
+    m.def("mlp_takes", &mlp_takes);
 }

@@ -22,7 +22,7 @@ struct PruneArgs {
     const unsigned* hi;             // order codes of max(x), max(-x) per column; 0 = no value
     const unsigned* nlo;
     const float* xt;                // [S][W_CI][NX][32]
-    int* inv;                       // [S][W_CI] full column -> compact position (with ci)
+    int* inv;                       // [S][W_CI] full column -> compact position, -1 where dropped (with ci)
     int* cnt;                       // [W_CO] list length, -1: no list
     float* tau;                     // [W_CO]
     float* ub;                      // [W_CO][lcap / STEP] largest U from this step of the list on
@@ -35,11 +35,13 @@ struct PruneArgs {
     unsigned* tile_done;            // [S][blocks of 128 outputs] k-tiles merged
 };
 
-// Outputs left over by the walks; rows of W whose list overflowed; column lists that are not strictly ascending.
+// Outputs left over by the walks; rows of W whose list overflowed; what the column lists are not: in ascending order, or (the
+// transposed input has one place per column) without an entry that comes twice.
 enum { FAILED = 0, OVERFLOWED = 1, GENERAL = 2 };
+constexpr unsigned LIST_ORDER = 1u, LIST_TWICE = 2u;
 
 __device__ __forceinline__ bool dense_mode(const PruneArgs& a) {
-    return (a.p.ci && a.counters[GENERAL] != 0u) || prune_gives_up(a.counters[OVERFLOWED], a.p.W_CO);
+    return (a.p.ci && (a.counters[GENERAL] & LIST_TWICE)) || prune_gives_up(a.counters[OVERFLOWED], a.p.W_CO);
 }
 
 // ---- transpose + column ranges ----------------------------------------------------------------
@@ -82,11 +84,11 @@ __global__ void __launch_bounds__(256) prune_prep(const PrunePrep p) {
         if (p.ci) {
             const int* at = p.ci + (size_t)s * p.CI + c0 + lc;
             c = *at;
-            const bool last = c0 + lc + 1 == p.CI;
-            if ((unsigned)c >= (unsigned)p.W_CI || (!last && at[1] <= c)) {  // not for the column order: see prune_redo.cuh
-                if (lane == 0) *p.general = 1u;
+            if ((unsigned)c >= (unsigned)p.W_CI) {           // the list is the caller's; nothing is written for such an entry
+                if (lane == 0) atomicOr(p.general, LIST_ORDER | LIST_TWICE);
                 continue;
             }
+            if (lane == 0 && c0 + lc + 1 < p.CI && at[1] <= c) atomicOr(p.general, LIST_ORDER);
         }
         unsigned hi = 0u, nlo = 0u;
 #pragma unroll
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(256) prune_prep(const PrunePrep p) {
         if (lane == 0) {
             atomicMax(p.hi + c, hi);
             atomicMax(p.nlo + c, nlo);
-            if (p.ci) p.inv[(size_t)s * p.W_CI + c] = c0 + lc;
+            if (p.ci && atomicExch(p.inv + (size_t)s * p.W_CI + c, c0 + lc) != -1) atomicOr(p.general, LIST_ORDER | LIST_TWICE);
         }
     }
 }
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
     __shared__ int hist[2 * R][BUCKETS];
     const int steps = (p.W_CO + R - 1) / R;
     const float nan = __int_as_float(0x7fc00000);
-    if (p.ci && a.counters[GENERAL] != 0u) return;           // no list will be walked
+    if (p.ci && (a.counters[GENERAL] & LIST_TWICE)) return;  // no list will be walked
     if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
     __syncthreads();
 
@@ -1138,9 +1140,9 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
     if (!p.counters) e = cudaMemsetAsync(a.counters, 0, 64 + (p.xt ? 0 : 2 * up256(sizeof(unsigned) * C)), st);
     if (e != cudaSuccess) return e;
     if (!p.xt) {
-        // all bits set is a NaN: the dropped columns
+        // all bits set is a NaN (the dropped columns) and a -1 (inv, which lies behind xt)
         float* xt = const_cast<float*>(a.xt);
-        if (p.ci && (e = cudaMemsetAsync(xt, 0xff, sizeof(float) * a.S * C * a.NX * 32, st)) != cudaSuccess) return e;
+        if (p.ci && (e = cudaMemsetAsync(xt, 0xff, (char*)(a.inv + a.S * C) - (char*)xt, st)) != cudaSuccess) return e;
         PrunePrep q;
         q.x = p.x, q.xl = p.xl, q.xu = p.xu, q.ci = p.ci, q.inv = a.inv, q.B = p.B, q.CI = p.CI, q.W_CI = p.W_CI;
         q.xt = xt, q.hi = const_cast<unsigned*>(a.hi), q.nlo = const_cast<unsigned*>(a.nlo), q.general = a.counters + GENERAL;

@@ -72,14 +72,14 @@ struct PrunePrep {
     const float* xl = nullptr;
     const float* xu = nullptr;
     const int* ci = nullptr;
-    int* inv = nullptr;
+    int* inv = nullptr;         // with ci: -1 before
     int B = 0, CI = 0, W_CI = 0;
     bool box = false;           // make xl, xu from x
     float eps = 0.f, down = 0.f, up = 0.f;
     float* xt = nullptr;
     unsigned* hi = nullptr;     // zeroed before
     unsigned* nlo = nullptr;
-    unsigned* general = nullptr;    // with ci: set to 1 when a list is not strictly ascending or leaves [0, W_CI)
+    unsigned* general = nullptr;    // with ci: flags of what its lists are not (zeroed before)
 };
 cudaError_t prune_prepare(const PrunePrep& q, cudaStream_t st);
 

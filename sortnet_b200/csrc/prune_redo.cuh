@@ -3,9 +3,9 @@
 // Two cases.  A few outputs here and there (a mask that took all the columns of a threshold, a row of W unlike the
 // others): prune_max / prune_sort record them, and they are evaluated one by one.  Or the data cannot be pruned at all (inputs
 // spread as wide as the weights: every column can matter): prune_filter counts the rows of W whose list overflowed, and above
-// 1 / DENSE_SHARE of them nothing is walked; the whole layer is evaluated by register tiles like those of inf_dist.cu, split
-// over all CTAs along (tile, k-tile) pairs.  Column lists that are not strictly ascending take that way too, in the order
-// of the list: position, not column, decides their ties, and a column may come twice.
+// a share of them (prune_gives_up) nothing is walked; the whole layer is evaluated by register tiles like those of inf_dist.cu,
+// split over all CTAs along (tile, k-tile) pairs.  Columns come in the order of W, or, where lists are in another order (position,
+// not column, decides their ties), in that of the list; a list that names a column twice is always evaluated like that.
 #pragma once
 #include <type_traits>
 

@@ -395,7 +395,13 @@ class NormDistConv(nn.Module):
 def _is_plain(module, cls):
     """Whether calling `module` is calling cls.forward and nothing else: no hooks, no override."""
     own = module.__dict__
-    return type(module).forward is cls.forward and "forward" not in own and not any(own[name] for name in _HOOKS)
+    return (type(module).forward is cls.forward and "forward" not in own
+            and not (own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"]))
+
+
+def _own_methods(cls):
+    """Whether the model's layer loop is SortMLPModel's."""
+    return cls is SortMLPModel or all(getattr(cls, name) is getattr(SortMLPModel, name) for name in ("_distances", "_scores", "_certifying"))
 
 
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
@@ -462,16 +468,13 @@ class SortMLPModel(nn.Module):
         one built here (hidden layers with a mean shift and no bias, a head without mean shift, p = inf) or somebody
         wants the layers called one by one (hooks, methods of a subclass)."""
         rows, last = [], len(self.fc_dist) - 1
-        if any(getattr(type(self), name) is not getattr(SortMLPModel, name) for name in ("_distances", "_scores", "_certifying")) \
-                or any(getattr(_module, "_global" + name) for name in _HOOKS) \
-                or not all(_is_plain(l, NormDist) and (l.mean_shift is None or _is_plain(l.mean_shift, MeanShiftDropout))
-                           for l in self.fc_dist):
+        if not _own_methods(type(self)) or any(getattr(_module, "_global" + name) for name in _HOOKS):
             return None
         for k, l in enumerate(self.fc_dist):
             shift = l.mean_shift
-            if not math.isinf(l.p) or (shift is None) != (k == last) or (k < last and l.bias is not None):
+            if not math.isinf(l.p) or (shift is None) != (k == last) or (k < last and l.bias is not None) or not _is_plain(l, NormDist):
                 return None
-            if shift is not None and (shift.affine or shift.training != l.training):
+            if shift is not None and (shift.affine or shift.training != l.training or not _is_plain(shift, MeanShiftDropout)):
                 return None
             K, q = 1, 0.0
             if sort_eval and not ops._sort_is_plain_max(l.weight, l.dropout, 10):
@@ -489,7 +492,7 @@ class SortMLPModel(nn.Module):
         if torch.is_grad_enabled() and (self.training or x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return None                      # a model in training mode draws masks, whatever its layers do
         plan = self._plan(sort_eval=sort_eval)
-        return plan if plan is not None and plan.takes(x) and plan.applies(x.size(0)) else None
+        return plan if plan is not None and plan.applies(x.size(0)) and plan.takes(x) else None
 
     @torch.no_grad()
     def certified_margin(self, x, targets, eps, up, down, sort_eval=None, after_layer=None):
@@ -553,14 +556,13 @@ class SortMLPModel(nn.Module):
         x = x.reshape(x.size(0), -1)
         if FUSED_LAYERS and x.is_cuda and x.dtype == torch.float32 and torch.is_grad_enabled() \
                 and not isinstance(self.scalar, torch.Tensor) and all(math.isinf(l.p) for l in self.fc_dist) \
-                and not ops.tracing() and all(m.training for m in self.modules()):     # a layer in evaluation mode keeps its statistics
+                and self.training and all(l.training for l in self.fc_dist) and not ops.tracing():   # one in evaluation keeps its statistics
             if masks is None and any(l.keep_rate != 1.0 for l in self.fc_dist):
                 masks = self.draw_masks(x.size(0), x.device)
             plan = self._plan(masks if any(l.keep_rate != 1.0 for l in self.fc_dist) else None)
             # post-accumulate hooks (dist.GradientAllReduce) get a layer's gradient while earlier layers still run: by layers
-            early = any(p._post_accumulate_grad_hooks for p in self.parameters())
-            if plan is not None and not early and plan.takes(x) and plan.applies(x.size(0)) \
-                    and any(t.requires_grad for t in (x, *plan.weights)):
+            if plan is not None and any(t.requires_grad for t in (x, *plan.weights)) and plan.applies(x.size(0)) and plan.takes(x) \
+                    and not any(p._post_accumulate_grad_hooks for p in (*plan.weights, plan.head_bias) if p is not None):
                 return ops.MlpMixtureLossF.apply(x.contiguous(), targets.contiguous(), eps, clip, lam, float(self.scalar), plan,
                                                  plan.head_bias, *plan.weights)
         d = self._distances(x, masks)

@@ -630,21 +630,8 @@ class MlpPlan:
                      K, mom, q) for w, b, rm, mom, kept, K, q in rows])
 
     def takes(self, x):
-        """Whether every tensor is what the kernels read through its pointer: fp32 (int32 lists), contiguous, on the
-        device of x [B, in], of the shapes of a chain of layers."""
-        B, width = x.shape
-        for w, bias, mean, _, kept, _, _ in self.keep:
-            if w.dim() != 2 or w.size(1) != width:
-                return False
-            width = w.size(0)
-            fits = [(w, tuple(w.shape), torch.float32)]
-            fits += [(t, (width,), torch.float32) for t in (bias, mean) if t is not None]
-            if kept is not None:
-                fits.append((kept, ((B + _SUB_BATCH - 1) // _SUB_BATCH, 1, kept.size(-1)), torch.int32))
-            if any(t.device != x.device or t.dtype != dtype or tuple(t.shape) != shape or not t.is_contiguous()
-                   for t, shape, dtype in fits):
-                return False
-        return True
+        """Whether every tensor is what the kernels read through its pointer (csrc/ops_ext.cpp, mlp_takes)."""
+        return _lib.ops().mlp_takes(x, [(r[0], r[1], r[2], r[4]) for r in self.keep])
 
     def applies(self, B):
         return _timeline is None and bool(_lib.load().snb_mlp_applies(self.table, self.depth, B))

@@ -197,16 +197,19 @@ def test_lists_that_overflow(B, CI, CO, kind):
 
 @pytest.mark.parametrize("which", ["both", "ci"])
 @pytest.mark.parametrize("kind", ["wide", "wide ties", "single"])
-def test_masked_lists_that_overflow(which, kind):
+@pytest.mark.parametrize("ascending", [True, False])
+def test_masked_lists_that_overflow(which, kind, ascending):
     from sortnet_b200 import norm_dist_cuda as C
     rng = np.random.default_rng(4)
     B, CI, CO = 97, 1030, 700
     ci, co = make_masks(rng, B, CI, 0.8), make_masks(rng, B, CO, 0.8) if which == "both" else None
+    ci = ci if ascending else rng.permuted(ci, axis=1)
     x, w = half_prunable(kind, rng, B, CI, CO)
     x = np.ascontiguousarray(x[:, :ci.shape[1]])
     n_out = CO if co is None else co.shape[1]
     y_o, pos_o = oracle.inf_dist_forward(x, w, ci, co)
-    for entry in (C.inf_dist_forward_sorted, lambda a, b, c, d, i, o: C.inf_dist_forward(a, b, c, d, 1, i, o)):
+    entries = [lambda a, b, c, d, i, o: C.inf_dist_forward(a, b, c, d, 1, i, o)] + ([C.inf_dist_forward_sorted] if ascending else [])
+    for entry in entries:
         y, pos = torch.empty(B, n_out, 1, device="cuda"), torch.empty(B, n_out, 1, device="cuda", dtype=torch.int32)
         entry(col3(x), dev(w), y, pos, idx3(ci), idx3(co))
         assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
