@@ -573,7 +573,8 @@ cudaError_t launch(const Args& a, int smem, cudaStream_t st) {
 // 0.036 -> 0.055 ms; p = 100 0.089 -> 0.042 and 0.056 -> 0.039 ms.
 bool applies(const LpProblem& q, float small_p) {
     const long long terms = (long long)q.B * q.CO * q.CI;
-    return q.p > 10.0f && terms >= (q.p >= small_p ? 12ll << 20 : 64ll << 20) && q.CI >= 128 && q.CO >= 128 && (q.B + 31) / 32 <= 65535;
+    return q.p > 10.0f && terms >= (q.p >= small_p ? 12ll << 20 : 64ll << 20) && q.CI >= 128 && q.CO >= 128 && (q.B + 31) / 32 <= 65535 &&
+           (q.W_CO + 63) / 64 <= 65535;                     // grid limits of the passes around the kernels
 }
 bool forward_applies(const LpProblem& q) { return applies(q, 16.0f); }
 bool backward_applies(const LpProblem& q) { return applies(q, 48.0f); }

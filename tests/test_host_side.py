@@ -211,6 +211,19 @@ def test_native_operators_stand_back_in_forward_mode():
     assert ops._native(CudaWeight())
 
 
+def test_forms_with_scratch_stay_within_their_limits(built_lib):
+    """Millions of outputs: no sparse form beyond its grids, no pruned form whose lists outgrow the card."""
+    from sortnet_b200 import _lib
+    lib = _lib.load()
+    for outputs, sparse in ((4_000_000, True), (5_000_000, False)):
+        assert (lib.snb_norm_dist_scratch_bytes(1, 32, outputs, 128, outputs, 128, 100.0, 0) > 0) == sparse
+        dense = lib.snb_norm_dist_forward_workspace_bytes(32, outputs, 100.0)
+        assert (lib.snb_norm_dist_scratch_bytes(0, 32, outputs, 128, outputs, 128, 100.0, 0) > dense) == sparse
+    for outputs, pruned in ((1_000_000, True), (10_000_000, False)):
+        assert (lib.snb_prune_scratch_bytes(1, 1, 1, 32, outputs, 128, outputs, 128, 0) > 0) == pruned
+    assert lib.snb_prune_scratch_bytes(3, 10, 0, 512, 5120, 5120, 5120, 5120, 0) > 0
+
+
 def test_operator_layer_signatures_match_the_reference():
     import inspect
     from sortnet_b200 import ops
