@@ -13,6 +13,7 @@ constexpr int PAD = 8;              // lists are padded to a multiple of this
 constexpr int STEP = 4;             // list entries per bound ub
 constexpr int MAX_COLUMNS = 12288;  // widest row the filter takes: 512 threads x 6 x 4
 constexpr int BUCKETS = 32;
+constexpr size_t MOST_SCRATCH = (size_t)4 << 30;   // with millions of outputs the lists would take more than W itself
 constexpr int LONG_LIST = 512;       // most entries of a list
 
 struct PruneArgs {
@@ -42,6 +43,13 @@ constexpr unsigned LIST_ORDER = 1u, LIST_TWICE = 2u;
 
 __device__ __forceinline__ bool dense_mode(const PruneArgs& a) {
     return (a.p.ci && (a.counters[GENERAL] & LIST_TWICE)) || prune_gives_up(a.counters[OVERFLOWED], a.p.W_CO);
+}
+
+// A load that stays where it is written.
+__device__ __forceinline__ unsigned load_now(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
 // ---- transpose + column ranges ----------------------------------------------------------------
@@ -544,7 +552,7 @@ __device__ __forceinline__ float shifted(const PruneProblem& p, float v, int j) 
 
 // One output of a sub-batch in the chain form, lane = row.
 template <int NV>
-__device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, const float (&v)[NV], uint32_t word) {
+__device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, const float (&v)[NV], uint32_t word, bool final = true) {
     const int lane = threadIdx.x & 31;
     const bool live = s * 32 + lane < p.B, kept = !p.keep || p.keep[(size_t)s * p.CO + j];
     if (p.yt) {
@@ -556,7 +564,7 @@ __device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, 
             hi = max(hi, order_code(o));
             nlo = max(nlo, order_code(-o));
         }
-        if (p.yhi) {
+        if (p.yhi && final) {                                // values that will be done again would widen the ranges
             hi = __reduce_max_sync(0xffffffffu, hi);
             nlo = __reduce_max_sync(0xffffffffu, nlo);
             if (lane == 0) {
@@ -570,7 +578,7 @@ __device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, 
 
 // 32 outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
 template <int NX, int NV, int NW>
-__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0, unsigned skip = 0u) {
+__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0, unsigned again = 0u) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* outs[NV];
     if (NX != 2) outs[0] = p.y;
@@ -596,11 +604,10 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
         for (int i = 0; i < 4; i++) {
             const int slot = warp * 4 + i;
             if (n0 + slot >= p.CO) break;
-            if ((skip >> slot) & 1u) continue;               // its values would widen the ranges
             float v[NV];
 #pragma unroll
             for (int t = 0; t < NV; t++) v[t] = tile[t][lane][slot];
-            emit_chain<NV>(p, s, n0 + slot, v, NW > 0 ? __float_as_uint(tile[NW > 0 ? NV : 0][lane][slot]) : 0u);
+            emit_chain<NV>(p, s, n0 + slot, v, NW > 0 ? __float_as_uint(tile[NW > 0 ? NV : 0][lane][slot]) : 0u, !((again >> slot) & 1u));
         }
     }
     if (p.part && warp == 0 && no < p.CO) {
@@ -663,7 +670,7 @@ __device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, in
 // TRACK keeps, per row, the step that set the maximum; the word is made at the end from the step's columns.  A
 // later step that only equals the maximum (rare) sends the lane over the list once more for the lowest position.
 template <int NX, bool TRACK>
-__global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneArgs a) {
+__global__ void __launch_bounds__(256, NX == 1 && !TRACK ? 6 : NX == 2 && TRACK ? 3 : 4) prune_max(const __grid_constant__ PruneArgs a) {
     constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
     constexpr int WORDS = TRACK ? NX : 0;
     __shared__ float tile[NV + WORDS][32][33];
@@ -672,10 +679,7 @@ __global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneAr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l = lane & 7;
     const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, slot = warp * 4 + g, n = n0 + slot;
     const float4* xt = reinterpret_cast<const float4*>(a.xt + (size_t)s * C * NX * 32) + l;
-    if (dense_mode(a)) {
-        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
-        return;
-    }
+    const unsigned overflowed = load_now(a.counters + OVERFLOWED), general = p.ci ? load_now(a.counters + GENERAL) : 0u;
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
     const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
     const int cnt = wanted ? a.cnt[j] : 0;
@@ -683,8 +687,6 @@ __global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneAr
     const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
     const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
     const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
-    if (tid == 0) failed = 0u;
-    __syncthreads();
 
     float acc[NV][4];
     int at[TRACK ? NV : 1][TRACK ? 4 : 1];                   // step of the maximum, -1: at its floor
@@ -718,6 +720,13 @@ __global__ void __launch_bounds__(256) prune_max(const __grid_constant__ PruneAr
     float left = 0.f;
     int walked = 0;
     if (active) e01 = list[0], e23 = list[1];
+    // looked at only here, so that it is on its way together with the head of the list
+    if ((general & LIST_TWICE) || prune_gives_up(overflowed, p.W_CO)) {
+        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
+        return;
+    }
+    if (tid == 0) failed = 0u;
+    __syncthreads();
     for (int b = 0;; b++) {
         if (b > 0) {
             const unsigned over = __ballot_sync(0xffffffffu, worst() > left);
@@ -1119,7 +1128,8 @@ bool prune_applies(const PruneProblem& p) {
     if ((p.B + 31) / 32 > 65535) return false;
     // the pruned form costs 20 to 30 us however small the problem; the dense kernels need that long at
     const long long least = p.K > 1 ? 1ll << 20 : p.xl ? 4ll << 20 : 12ll << 20;
-    return (long long)p.B * p.CO * p.W_CI >= least && p.W_CI >= 128;
+    if ((long long)p.B * p.CO * p.W_CI < least || p.W_CI < 128) return false;
+    return layout(p, nullptr, nullptr) <= MOST_SCRATCH;
 }
 
 size_t prune_workspace_bytes(const PruneProblem& p) { return layout(p, nullptr, nullptr); }
