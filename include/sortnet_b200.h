@@ -177,6 +177,8 @@ int snb_mlp_eval_forward(const snb_mlp_layer* layers, int depth, const float* x,
  * kept-column lists.  0 when the problem is too small or too wide for it.  Fewer bytes (or NULL) select the dense kernels. */
 size_t snb_prune_scratch_bytes(int tensors, int K, int words, int B, int CO, int CI, int W_CO, int W_CI,
                                int column_lists);
+/* 1 when that form is the faster one at these sizes (for data that can be pruned); callers pass no scratch otherwise. */
+int snb_prune_pays(int tensors, int K, int words, int B, int CO, int W_CI);
 
 /* Same y without pos, unmasked.  Replaces inf_dist::forward_nograd (norm_dist.h:22-23;
  * inf_dist_cuda.cu:277-304). */

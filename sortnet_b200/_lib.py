@@ -43,6 +43,7 @@ SIGNATURES = {
     "snb_sort_neuron_forward_ws": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P, ctypes.c_size_t, _P],
     "snb_bound_sort_neuron_forward_ws": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _I, _P, ctypes.c_size_t, _P],
     "snb_layer_bound_forward_ws": [_P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P],
+    "snb_prune_pays": [_I, _I, _I, _I, _I, _I],
     "snb_prune_scratch_bytes": [_I, _I, _I, _I, _I, _I, _I, _I, _I],     # returns size_t
     "snb_mean_shift_stats": [_P, _P, _I, _I, _I, _P, _P, _F, _P],
     "snb_mean_shift_apply": [_P, _P, _P, _I, _I, _P, _P],

@@ -144,6 +144,9 @@ int make_geo(int B, int CO, int CI, int G, int HW, int W_CO, Geo* q) {
 }
 
 size_t most(size_t a, size_t b) { return a > b ? a : b; }
+size_t prune_bytes(int tensors, int K, int words, int B, int CO, int CI, int W_CO, int W_CI, int lists) {
+    return snb_prune_pays(tensors, K, words, B, CO, W_CI) ? snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, lists) : 0;
+}
 size_t words(const Geo& q, int C, int K = 1) { return sizeof(uint32_t) * (size_t)q.G * K * q.Bp * C; }
 
 cudaError_t pack(const void* src, void* dst, const Geo& q, int C, int K, uint32_t fill, cudaStream_t st) {
@@ -186,7 +189,7 @@ int general_inf_forward(const float* x, const float* w, int B, int CO, int CI, i
     size_t op = pos ? a.reserve(words(q, COg)) : 0;
     size_t oci = ci ? a.reserve(mask_bytes(q, CIg)) : 0, oco = co ? a.reserve(mask_bytes(q, COg)) : 0;
     size_t ws_bytes = pos ? snb_inf_dist_forward_workspace_bytes(q.Bp, COg) : 0;
-    ws_bytes = most(ws_bytes, snb_prune_scratch_bytes(1, 1, pos != nullptr, q.Bp, COg, CIg, W_COg, W_CIg, ci != nullptr));
+    ws_bytes = most(ws_bytes, prune_bytes(1, 1, pos != nullptr, q.Bp, COg, CIg, W_COg, W_CIg, ci != nullptr));
     size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xp = a.at<float>(ox), *yp = a.at<float>(oy);
@@ -313,7 +316,7 @@ int general_bound_forward(const float* xl, const float* xu, const float* w, int 
     size_t oxl = a.reserve(words(q, CIg)), oxu = a.reserve(words(q, CIg));
     size_t oyl = a.reserve(words(q, COg)), oyu = a.reserve(words(q, COg));
     size_t opl = posl ? a.reserve(words(q, COg)) : 0, opu = posl ? a.reserve(words(q, COg)) : 0;
-    const size_t ws_bytes = snb_prune_scratch_bytes(2, 1, posl != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ws_bytes = prune_bytes(2, 1, posl != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
     const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xlp = a.at<float>(oxl), *xup = a.at<float>(oxu), *ylp = a.at<float>(oyl), *yup = a.at<float>(oyu);
@@ -381,7 +384,7 @@ int general_sort_forward(const float* x, const float* w, int B, int CO, int CI, 
     Arena a(st);
     size_t ox = a.reserve(words(q, CIg)), oy = a.reserve(words(q, COg));
     size_t op = pos ? a.reserve(words(q, COg, K)) : 0;
-    const size_t ws_bytes = snb_prune_scratch_bytes(1, K, pos != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ws_bytes = prune_bytes(1, K, pos != nullptr, q.Bp, COg, CIg, COg, CIg, 0);
     const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xp = a.at<float>(ox), *yp = a.at<float>(oy);
@@ -409,7 +412,7 @@ int general_sort_bound_forward(const float* xl, const float* xu, const float* w,
     Arena a(st);
     size_t oxl = a.reserve(words(q, CIg)), oxu = a.reserve(words(q, CIg));
     size_t oyl = a.reserve(words(q, COg)), oyu = a.reserve(words(q, COg));
-    const size_t ws_bytes = snb_prune_scratch_bytes(2, K, 0, q.Bp, COg, CIg, COg, CIg, 0);
+    const size_t ws_bytes = prune_bytes(2, K, 0, q.Bp, COg, CIg, COg, CIg, 0);
     const size_t ows = a.reserve(ws_bytes);
     SNB_CUDA(a.commit());
     float *xlp = a.at<float>(oxl), *xup = a.at<float>(oxu), *ylp = a.at<float>(oyl), *yup = a.at<float>(oyu);

@@ -347,8 +347,9 @@ int check_layers(const snb_mlp_layer* l, int depth, int B) {
 
 using namespace snb;
 
-// 1 when the calls below take these layers: rows of W within the filter's width, and enough work that the pruned
-// form is the faster one (the sizes at which the single-layer entry points change over, for the net as a whole).
+// 1 when the calls below take these layers: rows of W within the filter's width, and enough work that nothing is lost on small
+// nets.  Wall time of five-layer MNIST nets on a B200, by layers / whole: training 945 / 653 us at 3 M terms per layer, 1093 / 539 at 25 M,
+// 1200 / 596 at 50 M; certification 693 / 272, 889 / 331, 911 / 346.
 extern "C" int snb_mlp_applies(const snb_mlp_layer* l, int depth, int B) {
     if (check_layers(l, depth, B) != SNB_OK || (B + 31) / 32 > 65535) return 0;
     long long work = 0;

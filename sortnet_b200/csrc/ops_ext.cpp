@@ -44,6 +44,7 @@ struct Api {
     decltype(&snb_sort_neuron_backward_input_weight) sort_backward_xw;
     decltype(&snb_bound_sort_neuron_forward_ws) bound_sort_forward;
     decltype(&snb_prune_scratch_bytes) scratch_bytes;
+    decltype(&snb_prune_pays) pays;
     decltype(&snb_status_string) status_string;
     decltype(&snb_last_cuda_error) last_cuda_error;
 } api;
@@ -80,6 +81,7 @@ void init(const std::string& path, py::object error_class) {
     get(api.sort_backward_xw, "snb_sort_neuron_backward_input_weight");
     get(api.bound_sort_forward, "snb_bound_sort_neuron_forward_ws");
     get(api.scratch_bytes, "snb_prune_scratch_bytes");
+    get(api.pays, "snb_prune_pays");
     get(api.status_string, "snb_status_string");
     get(api.last_cuda_error, "snb_last_cuda_error");
 }
@@ -121,7 +123,7 @@ struct Area {
     size_t bytes = 0;
     Area(const Tensor& like, int tensors, int K, int words, int64_t B, int64_t CO, int64_t CI, int64_t W_CO, int64_t W_CI, bool lists,
          bool flat, size_t at_least = 0) {
-        bytes = flat ? api.scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, lists) : 0;
+        bytes = flat && api.pays(tensors, K, words, B, CO, W_CI) ? api.scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, lists) : 0;
         bytes = std::max(bytes, at_least);
         if (bytes) {
             t = at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));

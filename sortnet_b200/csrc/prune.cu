@@ -1126,7 +1126,7 @@ bool prune_applies(const PruneProblem& p) {
     if (p.W_CI > MAX_COLUMNS) return false;
     if (p.ci && 5ll * p.CI < 2ll * p.W_CI) return false;
     if ((p.B + 31) / 32 > 65535) return false;
-    // the pruned form costs 20 to 30 us however small the problem; the dense kernels need that long at
+    // below these sizes it cannot pay; where it does is up to the caller (snb_prune_pays)
     const long long least = p.K > 1 ? 1ll << 20 : p.xl ? 4ll << 20 : 12ll << 20;
     if ((long long)p.B * p.CO * p.W_CI < least || p.W_CI < 128) return false;
     return layout(p, nullptr, nullptr) <= MOST_SCRATCH;
@@ -1176,6 +1176,17 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
 }
 
 }  // namespace snb
+
+// Whether the pruned form is the faster one for data that can be pruned (inputs in [0, 1], N(0, 1) weights).  B200, one call
+// inside a graph, dense / pruned: values 9.0 / 17.1 us at 32 M terms, 12.2 / 17.9 at 64 M, 16.1 / 17.8 at 128 M, 42 / 20 at 512 M; with
+// positions 12.7 / 16.8 at 32 M, 16.1 / 16.7 at 64 M, 22.3 / 17.4 at 128 M; bounds 18.0 / 18.1 at 2 M, 17.7 / 16.4 at 4 M,
+// 24.0 / 18.4 at 32 M; ten largest 97 / 44 at 1 M.  It takes five launches however small the problem.
+extern "C" int snb_prune_pays(int tensors, int K, int words, int B, int CO, int W_CI) {
+    const long long terms = (long long)B * CO * W_CI;
+    if (K > 1) return terms >= 1ll << 20;
+    if (tensors != 1) return terms >= 4ll << 20;
+    return terms >= (words ? 80ll << 20 : 160ll << 20);
+}
 
 // Scratch with which the `_ws` entry points evaluate a problem in the pruned form: tensors = 1 (point value),
 // 2 (box) or 3 (both), K = 1 or the sort neuron's size, words = positions wanted, column_lists = kept-column

@@ -99,7 +99,7 @@ __host__ __device__ __forceinline__ bool prune_gives_up(unsigned overflowed, int
 // y and pos of a sort neuron by the kernels of sort_neuron.cu if the layer is to be evaluated as a whole, nothing otherwise.
 cudaError_t sort_positions_if(const PruneProblem& p, const unsigned* overflowed, cudaStream_t st);
 
-// Whether the pruned evaluation is the faster one for this problem (sizes only), and its scratch.
+// Whether the pruned evaluation takes this problem (sizes only), and its scratch.
 bool prune_applies(const PruneProblem& p);
 size_t prune_workspace_bytes(const PruneProblem& p);
 // ws: prune_workspace_bytes(p) bytes, 16-byte aligned.

@@ -154,11 +154,18 @@ def _same_device(*ts):
     return dev
 
 
+def _prune_pays(tensors, K, words, B, CO, W_CI):
+    """Whether to ask for the pruned evaluation at these sizes."""
+    return _lib.load().snb_prune_pays(tensors, K, words, B, CO, W_CI)
+
+
 def _scratch(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists, dev, at_least=0):
     """Scratch for a forward call, taken from PyTorch's caching allocator (stream-ordered, no device
-    synchronisation): what the pruned evaluation asks for (snb_prune_scratch_bytes), or `at_least` bytes;
-    an empty tensor when neither needs any."""
-    nbytes = max(_lib.load().snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists), at_least)
+    synchronisation): what the pruned evaluation asks for (snb_prune_scratch_bytes) where it is the faster
+    one, or `at_least` bytes; an empty tensor when neither needs any."""
+    nbytes = at_least
+    if _prune_pays(tensors, K, words, B, CO, W_CI):
+        nbytes = max(_lib.load().snb_prune_scratch_bytes(tensors, K, words, B, CO, CI, W_CO, W_CI, column_lists), at_least)
     return torch.empty((nbytes + 7) // 8, dtype=torch.int64, device=dev)
 
 

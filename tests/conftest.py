@@ -37,3 +37,11 @@ def golden():
         with np.load(os.path.join(GOLDEN, name + ".npz")) as z:
             return {k: z[k] for k in z.files}
     return load
+
+
+@pytest.fixture(autouse=True)
+def pruned_form_at_every_size(request, monkeypatch):
+    """The tests of the pruned form use shapes at its edges, below the sizes from which the wrappers ask for it."""
+    if request.module.__name__ == "test_prune_gpu":
+        from sortnet_b200 import norm_dist_cuda
+        monkeypatch.setattr(norm_dist_cuda, "_prune_pays", lambda *sizes: True)
