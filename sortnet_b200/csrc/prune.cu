@@ -1179,13 +1179,14 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
 
 // Whether the pruned form is the faster one for data that can be pruned (inputs in [0, 1], N(0, 1) weights).  B200, one call
 // inside a graph, dense / pruned: values 9.0 / 17.1 us at 32 M terms, 12.2 / 17.9 at 64 M, 16.1 / 17.8 at 128 M, 42 / 20 at 512 M; with
-// positions 12.7 / 16.8 at 32 M, 16.1 / 16.7 at 64 M, 22.3 / 17.4 at 128 M; bounds 18.0 / 18.1 at 2 M, 17.7 / 16.4 at 4 M,
+// positions 12.7 / 16.8 at 32 M, 16.1 / 16.7 at 64 M, 22.3 / 17.4 at 128 M, the same with ascending lists 15.7 / 24.9 at 29 M, 19.2 / 25.7 at
+// 58 M, 26.3 / 26.0 at 115 M, 39.6 / 27.0 at 230 M; bounds 18.0 / 18.1 at 2 M, 17.7 / 16.4 at 4 M,
 // 24.0 / 18.4 at 32 M; ten largest 97 / 44 at 1 M.  It takes five launches however small the problem.
 extern "C" int snb_prune_pays(int tensors, int K, int words, int B, int CO, int W_CI) {
     const long long terms = (long long)B * CO * W_CI;
     if (K > 1) return terms >= 1ll << 20;
     if (tensors != 1) return terms >= 4ll << 20;
-    return terms >= (words ? 80ll << 20 : 160ll << 20);
+    return terms >= (words ? 96ll << 20 : 160ll << 20);
 }
 
 // Scratch with which the `_ws` entry points evaluate a problem in the pruned form: tensors = 1 (point value),
