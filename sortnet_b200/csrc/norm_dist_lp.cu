@@ -11,13 +11,14 @@
 //
 // The reference reaches the p > 10 value with an online running maximum that may lag the true
 // maximum by 1e-6 relative; here M is the exact maximum, computed first by the l-infinity
-// kernel into y, so the result is the exact-math value up to fp32 rounding.  Integer p in
-// [1, 8] uses multiply chains (as the reference does), any other p uses ex2(p * log2 r) on the
-// special-function unit with a series for log2 near r = 1 (log2_rel), which keeps the p-fold
+// kernel into y, so the result is the exact-math value up to fp32 rounding.  Whole p in
+// [1, 8] uses multiply chains (as the reference does; lp_power.cu), any other p uses ex2(p * log2 r)
+// on the special-function unit with a series for log2 near r = 1 (log2_series), which keeps the p-fold
 // amplification of the logarithm's error at the level of the fp32 rounding of r itself.
 #include <float.h>
 #include "tile.cuh"
 #include "lp_math.cuh"
+#include "lp_dense.h"
 #include "lp_skip.h"
 #include "launch.h"
 #include "general_shapes.h"
@@ -28,55 +29,12 @@ namespace snb {
 cudaError_t inf_forward_values(const float* x, const float* w, float* y, const int* ci, const int* co,
                                int B, int CO, int CI, int W_CI, cudaStream_t st);
 
-// |r|^IP for integer IP (multiply chain) or |r|^e for IP < 0; forward terms.
-template <int IP>
-__device__ __forceinline__ float pow_abs(float r, float e) {
-    if (IP == 0) return 1.0f;
-    if (IP == 1) return fabsf(r);
-    if (IP == 2) return r * r;
-    if (IP == 3) return fabsf(r) * r * r;
-    if (IP == 4) { float a = r * r; return a * a; }
-    if (IP == 5) { float a = r * r; return fabsf(r) * a * a; }
-    if (IP == 6) { float a = r * r; return a * a * a; }
-    if (IP == 7) { float a = r * r; return fabsf(r) * a * a * a; }
-    if (IP == 8) { float a = r * r; a = a * a; return a * a; }
-    return pow_pos_sum(fabsf(r), e);
-}
-
-// sgn(r) * |r|^IP; backward terms.
-template <int IP>
-__device__ __forceinline__ float pow_signed(float r, float e) {
-    if (IP == 0) return r >= 0 ? 1.0f : -1.0f;
-    if (IP == 1) return r;
-    if (IP == 2) return fabsf(r) * r;
-    if (IP == 3) return r * r * r;
-    if (IP == 4) { float a = r * r; return fabsf(r) * r * a; }
-    if (IP == 5) { float a = r * r; return a * a * r; }
-    if (IP == 6) { float a = r * r; return fabsf(r) * r * a * a; }
-    if (IP == 7) { float a = r * r; return a * a * a * r; }
-    return copysignf(pow_pos(fabsf(r), e), r);
-}
-
-struct LpFwdParams {
-    const float* x;
-    const float* w;
-    float* y;
-    const float* m;  // NORMALISED: the maxima M (may be y itself when direct)
-    const int* ci;
-    const int* co;
-    int B, CO, CI, W_CI;
-    float p;
-    int direct;      // 1: one CTA per output tile, finished in the kernel; 0: shared tiles, lp_finish_kernel follows
-};
-
-enum { MODE_VEC = 0, MODE_SCALAR = 1, MODE_GATHER = 2 };
-
 // 32 x (64 * WN) output tiles (one sub-batch of rows), 8x8 outputs per thread.  The (tile, k-tile)
 // pairs of the whole problem form one sequence that is cut into gridDim.x equal ranges (see
 // StreamK), so all SMs stay busy whatever the shape and the mask sizes.  With `direct` the grid
 // has one CTA per tile and each CTA turns its sums into distances itself; otherwise every range
 // adds its partial sums into the zero-filled y with atomics and lp_finish_kernel takes the root.
-template <int WN, int MODE, int IP, bool NORMALISED>
+template <int WN, int MODE, bool NORMALISED>
 __global__ void __launch_bounds__(WN * 32) lp_fwd_kernel(const LpFwdParams p) {
     constexpr int BM = 32, BN = 64 * WN, NT = WN * 32;
     extern __shared__ __align__(16) float smem[];
@@ -130,7 +88,7 @@ __global__ void __launch_bounds__(WN * 32) lp_fwd_kernel(const LpFwdParams p) {
                 const float mx = (m < p.B && n < p.CO) ? p.m[(size_t)m * p.CO + n] : 1.0f;
                 rm[i][j] = 1.0f / mx;
                 // the (EPS / M)^p seed term, once per output
-                if (kt_begin == 0) acc[i][j] = pow_abs<IP>(SNB_EPS * rm[i][j], p.p);
+                if (kt_begin == 0) acc[i][j] = pow_pos_sum(SNB_EPS * rm[i][j], p.p);
             }
         }
 
@@ -173,14 +131,14 @@ __global__ void __launch_bounds__(WN * 32) lp_fwd_kernel(const LpFwdParams p) {
                     if (use_skip && __all_sync(0xffffffffu, big < skip_below)) continue;
 #pragma unroll
                     for (int j = 0; j < 8; j++) {
-                        acc[i][j] += pow_abs<IP>(a0[j], p.p);
-                        acc[i][j] += pow_abs<IP>(a1[j], p.p);
+                        acc[i][j] += pow_pos_sum(a0[j], p.p);
+                        acc[i][j] += pow_pos_sum(a1[j], p.p);
                     }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 8; j++) {
-                        acc[i][j] += pow_abs<IP>(xf[i].x - wf[j].x, p.p);
-                        acc[i][j] += pow_abs<IP>(xf[i].y - wf[j].y, p.p);
+                        acc[i][j] += pow_pos_sum(fabsf(xf[i].x - wf[j].x), p.p);
+                        acc[i][j] += pow_pos_sum(fabsf(xf[i].y - wf[j].y), p.p);
                     }
                 }
             }
@@ -218,19 +176,6 @@ __global__ void lp_finish_kernel(float* __restrict__ y, const float* __restrict_
     }
 }
 
-struct LpBwdParams {
-    const float* g;
-    const float* x;
-    const float* w;
-    const float* y;
-    float* gx;
-    float* gw;  // may be null: grad_x only
-    const int* ci;
-    const int* co;
-    int B, CO, CI, W_CI;
-    float pm1;  // p - 1
-};
-
 // Work unit: one 32-row sub-batch x NT compact input columns x one tile of 32 outputs j.  The units
 // of the whole problem form one sequence (sub-batch, column tile, j tile) that is cut into
 // gridDim.x equal ranges, so every CTA does the same amount of work whatever the shape; a range
@@ -245,13 +190,12 @@ constexpr int LPB_JT = 32;
 // are two vector loads (all lanes of a warp that share tb read the same words: broadcast)
 constexpr int LPB_GLD = 36;
 
-// FINE (general exponent only): the two warp votes per 16-term batch ("all terms negligible",
-// "some ratio near 1 -> accurate log2 series").  They pay from p - 1 >= 40: below that no term is
-// negligible and the hardware log2's absolute error of 2^-22, multiplied by p - 1, stays under
-// 7e-6 of a term; without the votes nothing separates the batches and the compiler overlaps
-// their log2 / exp2 chains.
-template <int IP, int NT, bool FINE>
-__global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdParams p) {
+// FINE: the two warp votes per 16-term batch ("all terms negligible", "some ratio near 1 -> accurate
+// log2 series").  They pay from p - 1 >= 40: below that no term is negligible and the hardware
+// log2's absolute error of 2^-22, multiplied by p - 1, stays under 7e-6 of a term; without the
+// votes nothing separates the batches and the compiler overlaps their log2 / exp2 chains.
+template <int NT, bool FINE>
+__global__ void __launch_bounds__(NT, 4) lp_bwd_kernel(const LpBwdParams p) {
     constexpr int LPB_WLD = NT + 4;  // floats per W-tile row (+4: keeps 16-byte alignment, shifts banks)
     extern __shared__ __align__(16) float smem[];
     float* wt = smem;                                   // [2][JT][WLD]
@@ -266,7 +210,7 @@ __global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdP
     const long long u_end = total * (blockIdx.x + 1) / gridDim.x;
     // |u|^(p-1) < 2^-40 for a whole warp: the terms are dropped (the largest terms are ~1)
     const bool use_skip = p.pm1 >= 48.0f;
-    const float skip_below = IP < 0 ? exp2f(-40.0f / fmaxf(p.pm1, 1e-3f)) : 0.f;
+    const float skip_below = exp2f(-40.0f / fmaxf(p.pm1, 1e-3f));
 
   while (u < u_end) {
     const int unit = (int)(u / ntiles), t_begin = (int)(u % ntiles);
@@ -289,14 +233,12 @@ __global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdP
         }
 
     const int mycol = tb == 0 ? col[0] : tb == 1 ? col[1] : tb == 2 ? col[2] : col[3];
-    // Element r of this thread in the 32 x 32 (g, y) tiles.  Integer exponents: a warp takes eight neighbouring j of four rows,
-    // whole sectors in memory and 32 different banks in shared memory (consecutive j alone hit 8 banks; 512 x 3840 x 3840,
-    // p = 2: 1.77 -> 1.69 ms, p = 5: 2.36 -> 2.25, p = 8: 2.64 -> 2.61).  For a general exponent the special-function unit
-    // hides the conflicts and consecutive j are the better reads (p = 9.5: 4.22 ms, 4.29 with the other order).
+    // Element r of this thread in the 32 x 32 (g, y) tiles: consecutive j, the better reads; the special-function unit hides
+    // the bank conflicts of the writes (p = 9.5: 4.22 ms, 4.29 in an order without them).
     auto element = [&](int r, int& jj, int& bb) {
         const int e = tid + NT * r;
-        jj = IP >= 0 ? (e & 7) + 8 * ((e >> 5) & 3) : e & 31;
-        bb = IP >= 0 ? ((e >> 3) & 3) + 4 * (e >> 7) : e >> 5;
+        jj = e & 31;
+        bb = e >> 5;
     };
     // this thread stages rows jj = tb, tb + 4, ... of the W tile (its own four columns) and its elements of the (g, y) tiles
     auto stage = [&](int t, int st) {
@@ -342,13 +284,10 @@ __global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdP
             const float v = yt[o];
             const float ry = v > 0.f ? 1.0f / v : 0.f;
             yt[o] = ry;
-            // integer exponents: g * (|t| / y)^IP = (g / y^IP) * |t|^IP, so the division by y is
-            // folded into g once per (row, output) instead of once per term
-            if (IP >= 0) gt[o] *= pow_abs<IP>(ry, 0.f);
             // large general exponents: 1 / y = ry * (1 + e) with e = 1 - y * ry known exactly (one
             // fma); (1 + e)^(p-1) = 1 + (p-1) e to first order goes into g, so that the rounding of
             // the reciprocal is not amplified by the exponent in every term
-            if (IP < 0 && FINE) gt[o] = fmaf(gt[o], p.pm1 * fmaf(-v, ry, 1.0f), gt[o]);
+            if (FINE) gt[o] = fmaf(gt[o], p.pm1 * fmaf(-v, ry, 1.0f), gt[o]);
         }
         __syncthreads();
         const int j0 = t * LPB_JT;
@@ -364,25 +303,12 @@ __global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdP
                 const float4 ga = g4[0], gb = g4[1];
                 gp[0] = ga.x; gp[1] = ga.y; gp[2] = ga.z; gp[3] = ga.w;
                 gp[4] = gb.x; gp[5] = gb.y; gp[6] = gb.z; gp[7] = gb.w;
-                if (IP < 0) {
-                    const float4 ya = y4[0], yb = y4[1];
-                    yp[0] = ya.x; yp[1] = ya.y; yp[2] = ya.z; yp[3] = ya.w;
-                    yp[4] = yb.x; yp[5] = yb.y; yp[6] = yb.z; yp[7] = yb.w;
-                }
+                const float4 ya = y4[0], yb = y4[1];
+                yp[0] = ya.x; yp[1] = ya.y; yp[2] = ya.z; yp[3] = ya.w;
+                yp[4] = yb.x; yp[5] = yb.y; yp[6] = yb.z; yp[7] = yb.w;
             }
-            if (IP >= 0) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float gv = gp[i];   // already divided by y^IP
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float ps = pow_signed<IP>(xv[i][k] - wv[k], p.pm1);
-                        gx[i][k] = fmaf(gv, ps, gx[i][k]);
-                        gwp[k] = fmaf(gv, ps, gwp[k]);
-                    }
-                }
-            } else {
-                // general exponent: 16 terms at a time so that their log2 / exp2 chains overlap;
+            {
+                // 16 terms at a time so that their log2 / exp2 chains overlap;
                 // one vote per batch for "all negligible" and one for "some ratio is near 1".
                 // |t| <= max_c |t| <= y, so a ratio is near 1 exactly when it is >= 0.875 and the
                 // largest ratio of the batch answers both questions.
@@ -467,7 +393,7 @@ __global__ void __launch_bounds__(NT, IP < 0 ? 4 : 3) lp_bwd_kernel(const LpBwdP
 
 // One CTA per resident slot (SMs x CTAs per SM by the occupancy calculator), each with an equal
 // share of the work units; grad_x is zero-filled first because partial ranges add into it.
-template <int IP, bool FINE = true>
+template <bool FINE>
 static cudaError_t launch_lp_bwd(const LpBwdParams& q, cudaStream_t st) {
     constexpr int NT = 128;
     constexpr int SMEM = (2 * LPB_JT * (NT + 4) + 2 * 2 * LPB_JT * LPB_GLD) * (int)sizeof(float);
@@ -476,7 +402,7 @@ static cudaError_t launch_lp_bwd(const LpBwdParams& q, cudaStream_t st) {
     cudaGetDevice(&dev);
     std::atomic<int>& slot = cached[dev & 63];
     int cps = slot.load(std::memory_order_acquire);
-    auto kern = lp_bwd_kernel<IP, NT, FINE>;
+    auto kern = lp_bwd_kernel<NT, FINE>;
     if (cps == 0) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         int occ = 0;
@@ -495,11 +421,11 @@ static cudaError_t launch_lp_bwd(const LpBwdParams& q, cudaStream_t st) {
 
 // p.m == nullptr with NORM: the maxima are in y and no scratch is available -> one CTA per tile,
 // finished in the kernel.  Otherwise equal (tile, k-tile) ranges over all resident CTA slots.
-template <int WN, int MODE, int IP, bool NORM>
+template <int WN, int MODE, bool NORM>
 static cudaError_t launch_lp_fwd(LpFwdParams p, cudaStream_t st) {
     constexpr int BN = 64 * WN;
     constexpr int SMEM = 2 * (32 + BN) * LDS * (int)sizeof(float);
-    auto kern = lp_fwd_kernel<WN, MODE, IP, NORM>;
+    auto kern = lp_fwd_kernel<WN, MODE, NORM>;
     static std::atomic<int> cached[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -528,20 +454,23 @@ static cudaError_t launch_lp_fwd(LpFwdParams p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const long long units = tiles * ((p.CI + BK - 1) / BK);
     kern<<<(unsigned)(units < slots ? units : slots), WN * 32, SMEM, st>>>(p);
-    lp_finish_kernel<<<sm_count() * 4, 256, 0, st>>>(p.y, NORM ? p.m : nullptr, (long long)n, 1.0f / p.p);
-    return launched(2);
+    if ((e = launched()) != cudaSuccess) return e;
+    return lp_finish(p.y, NORM ? p.m : nullptr, (long long)n, p.p, st);
 }
 
-template <int IP, bool NORM>
+template <bool NORM>
 static cudaError_t dispatch_lp_mode(const LpFwdParams& p, cudaStream_t st) {
-    if (p.ci || p.co) return launch_lp_fwd<4, MODE_GATHER, IP, NORM>(p, st);
+    if (p.ci || p.co) return launch_lp_fwd<4, MODE_GATHER, NORM>(p, st);
     const bool vec = (p.CI % 4 == 0) && (p.W_CI % 4 == 0) && aligned16(p.x) && aligned16(p.w);
-    return vec ? launch_lp_fwd<4, MODE_VEC, IP, NORM>(p, st) : launch_lp_fwd<4, MODE_SCALAR, IP, NORM>(p, st);
+    return vec ? launch_lp_fwd<4, MODE_VEC, NORM>(p, st) : launch_lp_fwd<4, MODE_SCALAR, NORM>(p, st);
 }
 
-static int integer_power(float p) {
-    const int ip = (int)p;
-    return (p == (float)ip && ip >= 0 && ip <= 8) ? ip : -1;
+// The exponents of the multiply chains (lp_power.cu).
+static bool whole(float p, int most) { return p >= 0.f && p <= (float)most && p == (float)(int)p; }
+
+cudaError_t lp_finish(float* y, const float* m, long long n, float p, cudaStream_t st) {
+    lp_finish_kernel<<<sm_count() * 4, 256, 0, st>>>(y, m, n, 1.0f / p);
+    return launched();
 }
 
 }  // namespace snb
@@ -574,20 +503,10 @@ static int lp_forward_impl(const float* x, const float* w, int B, int CO, int CI
         float* maxima = scratch ? scratch : y;
         SNB_CUDA(inf_forward_values(x, w, maxima, w_index_ci, w_index_co, B, CO, CI, W_CI, st));
         q.m = scratch;
-        SNB_CUDA(dispatch_lp_mode<-1, true>(q, st));
+        SNB_CUDA(dispatch_lp_mode<true>(q, st));
         return SNB_OK;
     }
-    switch (integer_power(p)) {
-        case 1: SNB_CUDA(dispatch_lp_mode<1, false>(q, st)); break;
-        case 2: SNB_CUDA(dispatch_lp_mode<2, false>(q, st)); break;
-        case 3: SNB_CUDA(dispatch_lp_mode<3, false>(q, st)); break;
-        case 4: SNB_CUDA(dispatch_lp_mode<4, false>(q, st)); break;
-        case 5: SNB_CUDA(dispatch_lp_mode<5, false>(q, st)); break;
-        case 6: SNB_CUDA(dispatch_lp_mode<6, false>(q, st)); break;
-        case 7: SNB_CUDA(dispatch_lp_mode<7, false>(q, st)); break;
-        case 8: SNB_CUDA(dispatch_lp_mode<8, false>(q, st)); break;
-        default: SNB_CUDA(dispatch_lp_mode<-1, false>(q, st)); break;
-    }
+    SNB_CUDA(whole(p, 8) ? lp_power_forward(q, st) : dispatch_lp_mode<false>(q, st));
     return SNB_OK;
 }
 
@@ -640,20 +559,9 @@ static int lp_backward(const float* g, const float* x, const float* w, const flo
         return SNB_OK;
     }
     LpBwdParams q{g, x, w, y, gx, gw, ci, co, B, CO, CI, W_CI, p - 1.0f};
-    switch (integer_power(p - 1.0f)) {
-        case 0: SNB_CUDA(launch_lp_bwd<0>(q, st)); break;
-        case 1: SNB_CUDA(launch_lp_bwd<1>(q, st)); break;
-        case 2: SNB_CUDA(launch_lp_bwd<2>(q, st)); break;
-        case 3: SNB_CUDA(launch_lp_bwd<3>(q, st)); break;
-        case 4: SNB_CUDA(launch_lp_bwd<4>(q, st)); break;
-        case 5: SNB_CUDA(launch_lp_bwd<5>(q, st)); break;
-        case 6: SNB_CUDA(launch_lp_bwd<6>(q, st)); break;
-        case 7: SNB_CUDA(launch_lp_bwd<7>(q, st)); break;
-        default:
-            if (p - 1.0f >= 40.0f) SNB_CUDA((launch_lp_bwd<-1, true>(q, st)));
-            else SNB_CUDA((launch_lp_bwd<-1, false>(q, st)));
-            break;
-    }
+    if (whole(q.pm1, 7)) SNB_CUDA(lp_power_backward(q, st));
+    else if (q.pm1 >= 40.0f) SNB_CUDA(launch_lp_bwd<true>(q, st));
+    else SNB_CUDA(launch_lp_bwd<false>(q, st));
     return SNB_OK;
 }
 

@@ -96,6 +96,22 @@ def test_masked_vs_oracle(p, which):
     assert rel(gx, gx_o) < TOL and rel(gw, gw_o) < TOL
 
 
+@pytest.mark.parametrize("p", [1.0, 2.0, 3.0, 5.0, 8.0])
+@pytest.mark.parametrize("B,CI,CO", [(1, 1, 1), (33, 127, 8), (32, 128, 9), (65, 129, 33), (31, 260, 71)])
+def test_whole_p_at_tile_edges(p, B, CI, CO):
+    """Remainders of the multiply-chain kernels: rows of a sub-batch, columns of a 128-wide block (16- and 4-byte copies), outputs of
+    a group of eight and of a tile of 32 or 128.  The bars of the file: 1e-5 per output, 1e-5 of the largest gradient."""
+    rng = np.random.default_rng(int(p) + CI)
+    x = rng.random((B, CI), dtype=np.float32)
+    w = rng.standard_normal((CO, CI)).astype(np.float32)
+    y = run_fwd(x, w, p)
+    assert rel_each(y, oracle.norm_dist_forward(x, w, p)) < TOL
+    g = rng.standard_normal((B, CO)).astype(np.float32)
+    gx_o, gw_o = oracle.norm_dist_backward(g, x, w, y, p)
+    gx, gw = run_bwd(g, x, w, y, p)
+    assert rel(gx, gx_o) < TOL and rel(gw, gw_o) < TOL
+
+
 def test_degenerate_rows():
     # identical x and w row: p <= 10 gives FLT_MIN^(1/p), p > 10 gives 1e-10 (the seed term)
     x = np.full((3, 16), 0.25, np.float32)
