@@ -4,10 +4,9 @@
 // The layers are those of layer.cu, with the same arithmetic in the same order; what differs is what moves
 // between them.  Activations stay in the form in which the pruned evaluation reads its input (prune.cuh:
 // [sub-batch][channel][32 rows], full width, NaN in dropped channels), so a layer is filter + walk (+ redo of rejected outputs)
-// + one pass that takes the batch mean off; nothing is gathered through index lists.  The backward works on full-width rows
-// too: per layer one pass that centres the gradient and one launch that builds grad_x row by row (batch rows) and grad_w
-// row by row (outputs) in shared memory, so grad_w is written once, whole, instead of zero-filled and hit with one atomic per
-// (row, output).  For six layers the host issues 28 + 12 launches from C instead of some 100 from Python.
+// + one pass that takes the batch mean off; nothing is gathered through index lists.  The backward keeps that form: one launch
+// per layer adds to the gradient of the layer below, makes grad_w (rows cleared and added to in place) and takes the mean shift's
+// backward on the way.  The host issues the launches of a whole direction from C.
 #include "../../include/sortnet_b200.h"
 #include "prune.cuh"
 
@@ -107,111 +106,119 @@ __global__ void __launch_bounds__(256) chain_shift_kernel(float* __restrict__ yt
     if (tid < n) hi_out[c] = hi[tid], nlo_out[c] = nlo[tid];
 }
 
-// Gradient of a layer's outputs g [B][C] (times *scale): centred when rows_kept is given (the backward of the mean
-// shift: minus the mean over the rows that kept the channel; g is 0 where a channel was dropped), written back
-// row by row and transposed to gt [S][C][32]; column sums on request (bias gradient).
-// CTA = 32 channels, warp = row of every sub-batch, whose values stay in registers between the two sweeps (up to
-// CENTER_S sub-batches, then they are read again).  Bound by latency and L2 traffic.
-constexpr int CENTER_S = 16;
-__global__ void __launch_bounds__(1024) chain_center_kernel(const float* g, const float* __restrict__ scale,
-                                                            const float* __restrict__ rows_kept, int B, int S, int C,
-                                                            float* g_out, float* __restrict__ gt, float* __restrict__ col_sum) {
+// Gradient of the head's outputs: g [B][C] * *scale -> gt [S][C][32], and its column sums (the bias gradient).
+// CTA = 32 channels, warp = row of every sub-batch.  Bound by latency.
+__global__ void __launch_bounds__(1024) head_gradient_kernel(const float* __restrict__ g, const float* __restrict__ scale, int B,
+                                                             int S, int C, float* __restrict__ gt, float* __restrict__ col_sum) {
     __shared__ float tile[2][32][33];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
-    const float f = scale ? *scale : 1.f;
-    auto fetch = [&](int s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, ch = blockIdx.x * 32 + warp;
+    const float f = *scale;
+    float sum = 0.f;
+    for (int s = 0; s < S; s++) {
         const int b = s * 32 + warp;
-        return b < B && c < C ? g[(size_t)b * C + c] * f : 0.f;
-    };
-    float v[CENTER_S], sum = 0.f, mean = 0.f;
-#pragma unroll
-    for (int s = 0; s < CENTER_S; s++) v[s] = s < S ? fetch(s) : 0.f;
-    if (rows_kept || col_sum) {
-#pragma unroll
-        for (int s = 0; s < CENTER_S; s++) sum += v[s];
-        for (int s = CENTER_S; s < S; s++) sum += fetch(s);
-        tile[0][warp][lane] = sum;
-        __syncthreads();
-        sum = tile[0][lane][warp];                           // the sums of channel `warp`
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        if (lane == 0) tile[1][0][warp] = sum;
-        __syncthreads();
-        sum = tile[1][0][lane];
-        if (col_sum && warp == 0 && c < C) col_sum[c] = sum;
-        if (rows_kept && c < C) mean = sum / fmaxf(rows_kept[c], 1e-10f);
-        __syncthreads();
-    }
-    const int ch = blockIdx.x * 32 + warp;
-    auto put = [&](int s, float x) {
-        const int b = s * 32 + warp;
-        x -= mean;
-        if (b < B && c < C) g_out[(size_t)b * C + c] = x;
+        const float x = b < B && c < C ? g[(size_t)b * C + c] * f : 0.f;
+        sum += x;
         tile[s & 1][warp][lane] = x;
         __syncthreads();                                     // the other buffer's readers are past their previous barrier
         if (ch < C) gt[((size_t)s * C + ch) * 32 + lane] = tile[s & 1][lane][warp];
-    };
+    }
+    if (!col_sum) return;
+    __syncthreads();
+    tile[0][warp][lane] = sum;
+    __syncthreads();
+    sum = tile[0][lane][warp];                               // the sums of channel `warp`
 #pragma unroll
-    for (int s = 0; s < CENTER_S; s++)
-        if (s < S) put(s, v[s]);
-    for (int s = CENTER_S; s < S; s++) put(s, fetch(s));
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0 && ch < C) col_sum[ch] = sum;
 }
 
-// Sparse l-inf backward of one layer.  CTAs 0 .. gx_rows - 1: row b of grad_x; the others: row j of grad_w.  Both are
-// accumulated in shared memory and written whole.  The rows of one sub-batch share a handful of argmax columns of W row j, so
-// a warp adds up per distinct column before it touches shared memory (32 lanes on few addresses otherwise retry
-// one by one: 61 instead of 27 us for 512 x 5120 x 5120).  Bound by the write of grad_w (HBM).
-__global__ void __launch_bounds__(256) chain_bwd_kernel(const float* __restrict__ g, const float* __restrict__ gt,
-                                                        const int* __restrict__ pos, const int* __restrict__ post, int B, int S,
-                                                        int CO, int CI, int gx_rows, float* __restrict__ gx,
-                                                        float* __restrict__ gw) {
-    extern __shared__ __align__(16) float row[];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const bool vec = (CI & 3) == 0 && ((reinterpret_cast<uintptr_t>(gx) | reinterpret_cast<uintptr_t>(gw)) & 15u) == 0;
-    for (int c = tid; c < (CI + 3) / 4; c += 256) reinterpret_cast<float4*>(row)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    float* dst;
-    if ((int)blockIdx.x < gx_rows) {
-        const int b = blockIdx.x;
-        dst = gx + (size_t)b * CI;
-        for (int j0 = tid; j0 < CO; j0 += 1024) {
-            uint32_t word[4];
-            float v[4];
+// Sparse l-inf backward of one layer, gradients in the form [sub-batch][channel][32 rows] like the words: two warps per output j,
+// lane = row, up to CHAIN_S sub-batches at a time in registers.  The backward of the mean shift is taken on the way: g minus its mean
+// over the rows that kept output j (g is 0 where it was dropped; rows_kept null: the head).  grad_x is added to the zeroed
+// gradient of the layer below by reductions in L2, one per row, whose addresses share sectors (the rows of a sub-batch share a handful of
+// argmax columns).  The row of grad_w is cleared by plain stores, and behind a barrier the few columns that occur get their sums over
+// the rows, each column's over all sub-batches of the warp before it leaves it.  512 x 5120 x 5120: 31 us, bound by latency and the
+// write of grad_w (16 us); the former kernels (grad_x in shared memory by a CTA per row, rows of grad_w too, the mean in a pass of
+// its own) took 37 + 20 us.
+constexpr int CHAIN_THREADS = 256, CHAIN_ROWS = CHAIN_THREADS / 64, CHAIN_S = 8;
+struct ChainBwd {
+    const float* gt;            // [S][CO][32]
+    const int* post;            // [S][CO][32]
+    const float* rows_kept;     // [CO] or null
+    int S, CO, CI;
+    float* gxt;                 // [S][CI][32], zeroed before, or null
+    float* gx;                  // instead of gxt: [B][CI], zeroed before
+    float* gw;                  // [CO][CI], or null
+};
+__global__ void __launch_bounds__(CHAIN_THREADS) chain_bwd_kernel(const ChainBwd a) {
+    __shared__ float sums[CHAIN_ROWS][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp >> 1, half = warp & 1, t64 = threadIdx.x & 63;
+    const int j = (int)blockIdx.x * CHAIN_ROWS + group, CO = a.CO, CI = a.CI, S = a.S;
+    if (j >= CO) return;
+    const int each = min(CHAIN_S, (S + 1) / 2);              // sub-batches per warp and turn
+    uint32_t word[CHAIN_S];
+    float v[CHAIN_S];
+    auto fetch = [&](int s0) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = j0 + 256 * u;
-                word[u] = j < CO ? (uint32_t)pos[(size_t)b * CO + j] : SNB_NO_GRAD_ID;
-                v[u] = j < CO ? g[(size_t)b * CO + j] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (word[u] != SNB_NO_GRAD_ID) atomicAdd(row + (word[u] & ~SNB_SIGN_BIT), (word[u] & SNB_SIGN_BIT) ? -v[u] : v[u]);
+        for (int u = 0; u < CHAIN_S; u++) {
+            const bool ok = u < each && s0 + u < S;
+            const size_t o = ((size_t)(ok ? s0 + u : 0) * CO + j) * 32 + lane;
+            word[u] = ok ? (uint32_t)a.post[o] : SNB_NO_GRAD_ID;
+            v[u] = ok ? a.gt[o] : 0.f;
         }
-    } else {
-        const int j = blockIdx.x - gx_rows;
-        dst = gw + (size_t)j * CI;
-        for (int s = tid >> 5; s < S; s += 8) {
-            const size_t o = ((size_t)s * CO + j) * 32 + lane;
-            const uint32_t word = (uint32_t)post[o];
-            const uint32_t col = word == SNB_NO_GRAD_ID ? SNB_NO_GRAD_ID : (word & ~SNB_SIGN_BIT);
-            const float v = (word & SNB_SIGN_BIT) ? gt[o] : -gt[o];
-            unsigned todo = __ballot_sync(0xffffffffu, col != SNB_NO_GRAD_ID);
-            while (todo) {
-                const uint32_t one = __shfl_sync(0xffffffffu, col, __ffs(todo) - 1);
-                const bool mine = col == one;
-                todo &= ~__ballot_sync(0xffffffffu, mine);
-                float sum = mine ? v : 0.f;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-                if (lane == 0) atomicAdd(row + one, sum);
-            }
-        }
+    };
+    float sum = 0.f;
+    if (a.rows_kept)
+        for (int s = 2 * each + half * each; s < S; s += 2 * each)                   // the turns after the first one
+            for (int u = 0; u < each && s + u < S; u++) sum += a.gt[((size_t)(s + u) * CO + j) * 32 + lane];
+    fetch(half * each);
+    float* dst = a.gw + (size_t)j * CI;
+    if (a.gw) {
+        if ((CI & 3) == 0 && (reinterpret_cast<uintptr_t>(a.gw) & 15u) == 0)
+            for (int c = t64; c < CI / 4; c += 64) reinterpret_cast<float4*>(dst)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        else
+            for (int c = t64; c < CI; c += 64) dst[c] = 0.f;
     }
-    __syncthreads();
-    if (vec)
-        for (int c = tid; c < CI / 4; c += 256) __stcs(reinterpret_cast<float4*>(dst) + c, reinterpret_cast<float4*>(row)[c]);
-    else
-        for (int c = tid; c < CI; c += 256) dst[c] = row[c];
+#pragma unroll
+    for (int u = 0; u < CHAIN_S; u++) sum += v[u];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0) sums[group][half] = sum;
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + group) : "memory");                    // sums, and the row of grad_w is cleared
+    const float mean = a.rows_kept ? (sums[group][0] + sums[group][1]) / fmaxf(a.rows_kept[j], 1e-10f) : 0.f;
+    for (int s0 = half * each;;) {
+#pragma unroll
+        for (int u = 0; u < CHAIN_S; u++) {
+            if (word[u] == SNB_NO_GRAD_ID) continue;
+            v[u] = (word[u] & SNB_SIGN_BIT) ? v[u] - mean : mean - v[u];             // into grad_w; grad_x gets the opposite
+            word[u] &= ~SNB_SIGN_BIT;
+            if (a.gxt) atomicAdd(a.gxt + ((size_t)(s0 + u) * CI + word[u]) * 32 + lane, -v[u]);
+            else if (a.gx) atomicAdd(a.gx + (size_t)((s0 + u) * 32 + lane) * CI + word[u], -v[u]);
+        }
+        if (a.gw) {
+#pragma unroll
+            for (int u = 0; u < CHAIN_S; u++) {
+                unsigned todo = __ballot_sync(0xffffffffu, word[u] != SNB_NO_GRAD_ID);
+                while (todo) {
+                    const uint32_t one = __shfl_sync(0xffffffffu, word[u], __ffs(todo) - 1);
+                    float part = 0.f;
+#pragma unroll
+                    for (int k = u; k < CHAIN_S; k++)
+                        if (word[k] == one) {
+                            part += v[k];
+                            word[k] = SNB_NO_GRAD_ID;
+                        }
+                    todo = __ballot_sync(0xffffffffu, word[u] != SNB_NO_GRAD_ID);
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+                    if (lane == 0) atomicAdd(dst + one, part);
+                }
+            }
+        }
+        s0 += 2 * each;
+        if (s0 >= S) break;
+        fetch(s0);
+    }
 }
 
 // Scores and margins of the evaluation pass from the head's outputs (ell_inf_models.py:45-50): score = -y * scale,
@@ -245,7 +252,6 @@ struct Cursor {
 // What the backward needs from the forward.
 struct Saved {
     unsigned char* keep[MAX_DEPTH];
-    int* pos[MAX_DEPTH];
     int* post[MAX_DEPTH];
     float* rows_kept[MAX_DEPTH];
     float* grad_d;
@@ -257,7 +263,6 @@ size_t saved_layout(const snb_mlp_layer* l, int depth, int B, char* base, Saved*
     for (int k = 0; k < depth; k++) {
         const size_t C = l[k].out;
         v.keep[k] = at.take<unsigned char>(l[k].kept_list ? S * C : 0);
-        v.pos[k] = at.take<int>((size_t)B * C);
         v.post[k] = at.take<int>(S * C * 32);
         v.rows_kept[k] = at.take<float>(C);
     }
@@ -318,7 +323,7 @@ size_t scratch_layout(const snb_mlp_layer* l, int depth, int B, int tensors, boo
     for (int k = 0; k < depth; k++) {
         PruneProblem p = layer_problem(l, k, B, tensors);
         p.xt = &some, p.hi = p.nlo = &none, p.counters = &none;
-        if (training) p.pos = &word;
+        if (training) p.post = &word;
         const size_t n = prune_workspace_bytes(p);
         most = n > most ? n : most;
     }
@@ -366,11 +371,12 @@ extern "C" size_t snb_mlp_saved_bytes(const snb_mlp_layer* l, int depth, int B) 
 extern "C" size_t snb_mlp_scratch_bytes(const snb_mlp_layer* l, int depth, int B, int tensors, int training) {
     return check_layers(l, depth, B) == SNB_OK ? scratch_layout(l, depth, B, tensors, training != 0, nullptr, nullptr) : 0;
 }
-// backward: two gradients row by row and one transposed
+// backward: the gradients of all layers' outputs
 extern "C" size_t snb_mlp_backward_scratch_bytes(const snb_mlp_layer* l, int depth, int B) {
     if (check_layers(l, depth, B) != SNB_OK) return 0;
-    const size_t W = widest(l, depth), S = (B + 31) / 32;
-    return 2 * up256(sizeof(float) * B * W) + up256(sizeof(float) * S * 32 * W);
+    size_t n = 0;
+    for (int k = 0; k < depth; k++) n += up256(sizeof(float) * (size_t)((B + 31) / 32) * 32 * l[k].out);
+    return n;
 }
 
 extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const float* x, int B, const long long* targets, float eps,
@@ -410,7 +416,7 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
         const int C = l[k].out;
         PruneProblem p = layer_problem(l, k, B, 1);
         p.xt = sc.xt[k & 1], p.hi = sc.hi[k], p.nlo = sc.nlo[k], p.counters = sc.counters[k];
-        p.pos = sv.pos[k], p.post = sv.post[k];
+        p.post = sv.post[k];
         if (l[k].kept_list) p.keep = sv.keep[k], p.out_list = l[k].kept_list, p.out_kept = l[k].kept;
         if (head) {
             p.y = sc.d;
@@ -442,39 +448,37 @@ extern "C" int snb_mlp_train_backward(const snb_mlp_layer* l, int depth, int B, 
     if (rc) return rc;
     if (!grad_loss || !saved || !scratch || !grad_w) return SNB_ERR_NULL_POINTER;
     cudaStream_t st = (cudaStream_t)stream;
-    const int S = (B + 31) / 32, W = widest(l, depth);
+    const int S = (B + 31) / 32;
     Saved sv;
     saved_layout(l, depth, B, const_cast<char*>(static_cast<const char*>(saved)), &sv);
     Cursor at{static_cast<char*>(scratch)};
-    float* rows[2] = {at.take<float>((size_t)B * W), at.take<float>((size_t)B * W)};
-    float* gt = at.take<float>((size_t)S * 32 * W);
-    int most = 0;                                            // shared memory of the widest row of W
-    for (int k = 0; k < depth; k++) most = l[k].in > most ? l[k].in : most;
-    most = (most + 3) / 4 * 16;
-    if (most > MOST_SMEM) return SNB_ERR_UNSUPPORTED;
-    if (most > 48 * 1024) SNB_CUDA(allow_smem<chain_bwd_kernel, MOST_SMEM>());
+    float* gt[MAX_DEPTH];
+    for (int k = 0; k < depth; k++) gt[k] = at.take<float>((size_t)S * 32 * l[k].out);
     int lowest = 0;                                          // deepest layer that anybody wants a gradient from
     while (!grad_x && lowest < depth && !grad_w[lowest]) lowest++;
     if (lowest == depth && grad_bias) lowest = depth - 1;
-    int count = 0;
-    const float* g = sv.grad_d;
+    if (lowest == depth) {
+        if (launches) *launches = 0;
+        return SNB_OK;
+    }
+    const int classes = l[depth - 1].out;
+    if (lowest < depth - 1)
+        SNB_CUDA(cudaMemsetAsync(gt[lowest], 0, (char*)gt[depth - 1] - (char*)gt[lowest], st));
+    if (grad_x) SNB_CUDA(cudaMemsetAsync(grad_x, 0, sizeof(float) * (size_t)B * l[0].in, st));
+    head_gradient_kernel<<<(classes + 31) / 32, 1024, 0, st>>>(sv.grad_d, grad_loss, B, S, classes, gt[depth - 1], grad_bias);
+    SNB_CUDA(launched());
+    int count = 1;
     for (int k = depth - 1; k >= lowest; k--) {
-        const bool head = k == depth - 1;
-        const int C = l[k].out, CI = l[k].in;
-        float* centred = rows[0];
-        chain_center_kernel<<<(C + 31) / 32, 1024, 0, st>>>(g, head ? grad_loss : nullptr, head ? nullptr : sv.rows_kept[k], B, S, C,
-                                                           centred, gt, head ? grad_bias : nullptr);
+        ChainBwd a{};
+        a.gt = gt[k], a.post = sv.post[k], a.rows_kept = k < depth - 1 ? sv.rows_kept[k] : nullptr;
+        a.S = S, a.CO = l[k].out, a.CI = l[k].in;
+        if (k > lowest) a.gxt = gt[k - 1];
+        else if (k == 0) a.gx = grad_x;
+        a.gw = grad_w[k];
+        if (!a.gxt && !a.gx && !a.gw) continue;
+        chain_bwd_kernel<<<(a.CO + CHAIN_ROWS - 1) / CHAIN_ROWS, CHAIN_THREADS, 0, st>>>(a);
         SNB_CUDA(launched());
         count++;
-        float* gx = k > lowest ? rows[1] : (k == 0 ? grad_x : nullptr);
-        const int nx = gx ? B : 0, nw = grad_w[k] ? C : 0;
-        if (nx + nw > 0) {
-            chain_bwd_kernel<<<nx + nw, 256, (CI + 3) / 4 * 16, st>>>(centred, gt, sv.pos[k], sv.post[k], B, S, C, CI, nx, gx,
-                                                                      grad_w[k]);
-            SNB_CUDA(launched());
-            count++;
-        }
-        g = rows[1];
     }
     if (launches) *launches = count;
     return SNB_OK;

@@ -593,7 +593,7 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
 #pragma unroll
         for (int t = 0; t < NV; t++)
             if (outs[t]) outs[t][o] = shifted<NV>(p, tile[t][r][lane], no);
-        if (NW == 1 && NX == 1) p.pos[o] = kept ? __float_as_int(tile[NV][r][lane]) : (int)SNB_NO_GRAD_ID;
+        if (NW == 1 && NX == 1 && p.pos) p.pos[o] = kept ? __float_as_int(tile[NV][r][lane]) : (int)SNB_NO_GRAD_ID;
         if (NW == 2) {
             p.posl[o] = __float_as_int(tile[NV][r][lane]);
             p.posu[o] = __float_as_int(tile[NV + NW - 1][r][lane]);
@@ -986,7 +986,7 @@ namespace {
 // ---- host side ----------------------------------------------------------------------------------
 
 int tensors(const PruneProblem& p) { return (p.x ? 1 : 0) + (p.xl ? 2 : 0); }
-bool with_words(const PruneProblem& p) { return p.pos || p.posl; }
+bool with_words(const PruneProblem& p) { return p.pos || p.posl || p.post; }
 
 // How many columns must reach the threshold.  Without masks K: the K-th largest value of every row then
 // reaches it by construction.  With column lists the m columns may all be missing from a sub-batch's list; m is chosen so

@@ -50,7 +50,7 @@ struct PruneProblem {
     const unsigned* nlo = nullptr;
     int kept = 0;
     // Output: yt [S][CO][tensors][32], NaN in rows past the batch and in outputs that `keep` [S][CO] drops; ranges
-    // (zeroed before), sums over the rows of a sub-batch in row order [S][CO], words [S][CO][32] and in pos [B][CO]
+    // (zeroed before), sums over the rows of a sub-batch in row order [S][CO], words [S][CO][32]
     // (SNB_NO_GRAD_ID where dropped).  y = (y - mean[j]) + bias[j] before it is written anywhere (either may be null).
     float* yt = nullptr;
     unsigned* yhi = nullptr;

@@ -33,7 +33,7 @@ __device__ __forceinline__ void store_output(const PruneProblem& p, int s, int n
     const size_t o = (size_t)b * p.CO + n;
     if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, v[0], n);
     if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, v[NX - 2], n), p.yu[o] = shifted<NX>(p, v[NX - 1], n);
-    if (TRACK && NX == 1) p.pos[o] = (int)word[0];
+    if (TRACK && NX == 1 && p.pos) p.pos[o] = (int)word[0];
     if (TRACK && NX == 2) p.posl[o] = (int)word[0], p.posu[o] = (int)word[TRACK ? NX - 1 : 0];
 }
 
@@ -286,7 +286,7 @@ __device__ __noinline__ void dense_emit(const PruneArgs& a, const DenseLayer& d,
             const size_t o = (size_t)(s * 32 + r) * p.CO + out;
             if (NX != 2 && p.y) p.y[o] = shifted<NX>(p, tile[0][r][lane], out);
             if (NX >= 2 && p.yl) p.yl[o] = shifted<NX>(p, tile[NX - 2][r][lane], out), p.yu[o] = shifted<NX>(p, tile[NX - 1][r][lane], out);
-            if (NW == 1) p.pos[o] = __float_as_int(tile[NX][r][lane]);
+            if (NW == 1 && p.pos) p.pos[o] = __float_as_int(tile[NX][r][lane]);
             if (NW == 2) p.posl[o] = __float_as_int(tile[NX][r][lane]), p.posu[o] = __float_as_int(tile[NX + NW - 1][r][lane]);
         }
         if (p.yt || p.post)                                  // lane = row
