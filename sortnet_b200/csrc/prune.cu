@@ -456,6 +456,35 @@ struct TopList {
             }
         }
     }
+    // Four values at once, none of them NaN or negative: sorted, paired with the four weakest slots (ascending against descending: the
+    // larger of each pair stays, and the slots are a bitonic sequence) and merged.  46 minima and maxima of ten slots against 80
+    // one by one, 26 against 40 where no row's slot HALF is beaten; the votes are per four as well.  Point and box of a
+    // 512 x 5120 x 5120 layer: 300 -> 212 us.
+    template <int N>
+    __device__ __forceinline__ void merge() {                // slots 0 .. N - 1 bitonic -> ascending
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+            for (int s = 0; s < N; s++)
+                if ((s & d) == 0 && s + d < N) {
+                    const float lo = fminf(v[s], v[s + d]), hi = fmaxf(v[s], v[s + d]);
+                    v[s] = lo, v[s + d] = hi;
+                }
+    }
+    __device__ __forceinline__ void add4(float a, float b, float c, float d) {
+        constexpr int HALF = KMAX / 2;
+        const float most = fmaxf(max3(a, b, c), d);
+        if (!__any_sync(0xffffffffu, most > v[0])) return;
+        auto order = [](float& x, float& y) {                // x >= y
+            const float lo = fminf(x, y);
+            x = fmaxf(x, y), y = lo;
+        };
+        order(a, b), order(c, d), order(a, c), order(b, d), order(b, c);
+        const bool high = __any_sync(0xffffffffu, a > v[HALF]);
+        v[0] = fmaxf(v[0], a), v[1] = fmaxf(v[1], b), v[2] = fmaxf(v[2], c), v[3] = fmaxf(v[3], d);
+        if (high) merge<KMAX>();
+        else merge<HALF>();
+    }
     // v[KMAX - K], as a minimum over an ascending tail: an index that is not a constant would move the list to local memory
     __device__ __forceinline__ float kth(int K) const {
         if (K == KMAX) return v[0];
@@ -491,6 +520,26 @@ struct SortState {
             const float t1 = w - v[NX - 2], t2 = v[NX - 1] - w;
             top[NX - 2].add(fmaxf(-t1, -t2));
             top[NX - 1].add(fmaxf(t1, t2));
+        }
+    }
+    // four columns
+    __device__ __forceinline__ void add4(const float (&v)[4][NX], const float (&w)[4]) {
+        float e[4];
+        if (NX != 2) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) e[k] = fmaxf(fabsf(v[k][0] - w[k]), 0.f);        // NaN -> 0
+            top[0].add4(e[0], e[1], e[2], e[3]);
+        }
+        if (NX >= 2) {
+            float u[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float t1 = w[k] - v[k][NX - 2], t2 = v[k][NX - 1] - w[k];
+                e[k] = max3(-t1, -t2, 0.f);
+                u[k] = max3(t1, t2, 0.f);
+            }
+            top[NX - 2].add4(e[0], e[1], e[2], e[3]);
+            top[NX - 1].add4(u[0], u[1], u[2], u[3]);
         }
     }
     __device__ __forceinline__ float worst(int K) const {
@@ -908,8 +957,7 @@ __global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneA
                     v[2 * e + 1][t] = xt[((size_t)two.z * NX + t) * 32];
                 }
             }
-#pragma unroll
-            for (int e = 0; e < WALK; e++) st.add(v[e], w[e], 0u);
+            st.add4(v, w);
         }
         const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || st.worst(K) >= tau);
         if (!good && lane == 0) atomicOr(&failed, 1u << slot);
