@@ -477,27 +477,35 @@ cudaError_t sort_positions_if(const PruneProblem& q, const unsigned* overflowed,
     return launched();
 }
 
-// Sparse backward: one CTA per batch row, grad_x of the row accumulated in shared memory.
-__global__ void __launch_bounds__(256) sort_bwd_kernel(const float* __restrict__ g, const int* __restrict__ pos,
-                                                       int B, int CO, int CI, int K, float q, float c0,
-                                                       float* __restrict__ gx, float* __restrict__ gw,
-                                                       int use_smem) {
+// Sparse backward: one CTA per batch row, grad_x of the row accumulated in shared memory.  Bound by latency: all words of
+// an output are on their way before the first one is used (128 x 5120 x 5120, K = 10: 90 us with one word at a time
+// and 256 threads, 15 us).
+constexpr int SORT_BWD_THREADS = 1024;
+template <int KMAX>
+__global__ void __launch_bounds__(SORT_BWD_THREADS, 1) sort_bwd_kernel(const float* __restrict__ g, const int* __restrict__ pos,
+                                                                       int B, int CO, int CI, int K, float q, float c0,
+                                                                       float* __restrict__ gx, float* __restrict__ gw,
+                                                                       int use_smem) {
     extern __shared__ float row[];
     const int b = blockIdx.x;
     float* acc = use_smem ? row : gx + (size_t)b * CI;
     if (use_smem) {
-        for (int c = threadIdx.x; c < CI; c += blockDim.x) row[c] = 0.f;
+        for (int c = threadIdx.x; c < CI; c += SORT_BWD_THREADS) row[c] = 0.f;
         __syncthreads();
     }
     const size_t plane = (size_t)B * CO;
-    for (int j = threadIdx.x; j < CO; j += blockDim.x) {
+    for (int j = threadIdx.x; j < CO; j += SORT_BWD_THREADS) {
         const size_t o = (size_t)b * CO + j;
+        uint32_t word[KMAX];
+#pragma unroll
+        for (int k = 0; k < KMAX; k++) word[k] = k < K ? (uint32_t)pos[(size_t)k * plane + o] : 0u;
         const float grad = g[o];
         float c = c0;
-        for (int k = 0; k < K; k++) {
-            const uint32_t pw = (uint32_t)pos[(size_t)k * plane + o];
-            const int i = (int)(pw & ~SNB_SIGN_BIT);
-            const float v = ((pw & SNB_SIGN_BIT) ? -grad : grad) * c * q;
+#pragma unroll
+        for (int k = 0; k < KMAX; k++) {
+            if (k >= K) break;
+            const int i = (int)(word[k] & ~SNB_SIGN_BIT);
+            const float v = ((word[k] & SNB_SIGN_BIT) ? -grad : grad) * c * q;
             atomicAdd(acc + i, v);
             if (gw) atomicAdd(gw + (size_t)j * CI + i, -v);
             c *= 1 - q;
@@ -505,7 +513,7 @@ __global__ void __launch_bounds__(256) sort_bwd_kernel(const float* __restrict__
     }
     if (use_smem) {
         __syncthreads();
-        for (int c = threadIdx.x; c < CI; c += blockDim.x) gx[(size_t)b * CI + c] = row[c];
+        for (int c = threadIdx.x; c < CI; c += SORT_BWD_THREADS) gx[(size_t)b * CI + c] = row[c];
     }
 }
 
@@ -637,7 +645,9 @@ static int sort_backward(const float* g, const int* pos, int B, int CO, int CI, 
     if (!use_smem) SNB_CUDA(cudaMemsetAsync(gx, 0, sizeof(float) * (size_t)B * CI, st));
     float n = powf(1 - q, (float)K);
     n = 1.0f + n / (1.0f - n);
-    sort_bwd_kernel<<<B, 256, use_smem ? CI * sizeof(float) : 0, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
+    const size_t smem = use_smem ? CI * sizeof(float) : 0;
+    if (K <= 10) sort_bwd_kernel<10><<<B, SORT_BWD_THREADS, smem, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
+    else sort_bwd_kernel<25><<<B, SORT_BWD_THREADS, smem, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
     SNB_CUDA(launched());
     return SNB_OK;
 }
