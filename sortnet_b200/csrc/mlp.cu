@@ -20,7 +20,7 @@ struct KeepJobs {
     unsigned char* flags[MAX_DEPTH];
     int count[MAX_DEPTH], channels[MAX_DEPTH];
 };
-__global__ void __launch_bounds__(256) keep_flags_kernel(const KeepJobs jobs) {
+__global__ void __launch_bounds__(1024) keep_flags_kernel(const KeepJobs jobs) {
     const int* list = nullptr;
     unsigned char* flags = nullptr;
     int count = 0, channels = 0;
@@ -30,9 +30,10 @@ __global__ void __launch_bounds__(256) keep_flags_kernel(const KeepJobs jobs) {
     if (!list) return;
     const int s = blockIdx.x;
     unsigned char* f = flags + (size_t)s * channels;
-    for (int c = threadIdx.x; c < channels; c += 256) f[c] = 0;
+    for (int c = threadIdx.x; c < channels; c += 1024) f[c] = 0;
     __syncthreads();
-    for (int k = threadIdx.x; k < count; k += 256) {
+#pragma unroll 4
+    for (int k = threadIdx.x; k < count; k += 1024) {
         const int c = list[(size_t)s * count + k];
         if ((unsigned)c < (unsigned)channels) f[c] = 1;      // the lists are the caller's: an entry out of range keeps nothing
     }
@@ -402,7 +403,7 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
             masked++;
         }
     if (masked) {
-        keep_flags_kernel<<<dim3(S, masked), 256, 0, st>>>(jobs);
+        keep_flags_kernel<<<dim3(S, masked), 1024, 0, st>>>(jobs);
         SNB_CUDA(launched());
         count++;
     }
