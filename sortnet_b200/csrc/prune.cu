@@ -625,19 +625,19 @@ __device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, 
     if (p.post) p.post[((size_t)s * p.CO + j) * 32 + lane] = live && kept ? (int)word : (int)SNB_NO_GRAD_ID;
 }
 
-// 32 outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
-template <int NX, int NV, int NW>
+// SLOTS outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
+template <int NX, int NV, int NW, int SLOTS = 32>
 __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0, unsigned again = 0u) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* outs[NV];
     if (NX != 2) outs[0] = p.y;
     if (NX >= 2) outs[NV - 2] = p.yl, outs[NV - 1] = p.yu;
     const int no = n0 + lane;
-    const bool kept = no < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + no]);
+    const bool here = lane < SLOTS && no < p.CO, kept = here && (!p.keep || p.keep[(size_t)s * p.CO + no]);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int r = warp + 8 * k, b = s * 32 + r;
-        if (b >= p.B || no >= p.CO) continue;
+        if (b >= p.B || !here) continue;
         const size_t o = (size_t)b * p.CO + no;
 #pragma unroll
         for (int t = 0; t < NV; t++)
@@ -650,8 +650,8 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
     }
     if (p.yt || p.post) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int slot = warp * 4 + i;
+        for (int i = 0; i < SLOTS / 8; i++) {
+            const int slot = warp * (SLOTS / 8) + i;
             if (n0 + slot >= p.CO) break;
             float v[NV];
 #pragma unroll
@@ -659,7 +659,7 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
             emit_chain<NV>(p, s, n0 + slot, v, NW > 0 ? __float_as_uint(tile[NW > 0 ? NV : 0][lane][slot]) : 0u, !((again >> slot) & 1u));
         }
     }
-    if (p.part && warp == 0 && no < p.CO) {
+    if (p.part && warp == 0 && here) {
         float sum = 0.f;
         const int rows = min(32, p.B - s * 32);
         for (int r = 0; r < rows; r++) sum += tile[0][r][lane];
@@ -671,7 +671,7 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
 // What prune_redo needs, shared out over the CTAs (s, n0) of the walk it replaces: the rows of x side by side again, empty
 // partial results (`bytes` per value; 0: none are kept), and the outputs that `keep` drops.  256 threads.
 template <int NX>
-__device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, int bytes) {
+__device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, int bytes, int slots = 32) {
     const PruneProblem& p = a.p;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = p.W_CI;
     const float nan = __int_as_float(0x7fc00000);
@@ -701,8 +701,8 @@ __device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, in
         if (tid == 0 && n0 % 128 == 0) a.tile_done[(size_t)s * ((p.CO + 127) / 128) + n0 / 128] = 0u;
     }
     if (!p.keep) return;
-    for (int i = 0; i < 4; i++) {
-        const int n = n0 + warp * 4 + i, b = s * 32 + lane;
+    for (int i = 0; i < slots / 8; i++) {
+        const int n = n0 + warp * (slots / 8) + i, b = s * 32 + lane;
         if (n >= p.CO || p.keep[(size_t)s * p.CO + n]) continue;
         const float v[NX] = {};
         emit_chain<NX>(p, s, n, v, 0u);
@@ -907,31 +907,33 @@ __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, con
 }
 
 // The sort neuron over the same lists, one warp per output, lane = row; POS: the K positions too.  Bound by the
-// issue rate of the insertion chains.  With the values known, a second walk finds the positions: the rank of an
-// element among a row's K largest is the number of larger values in the row's list, and of equal values the later column
-// comes first.  Only where more columns share the K-th value than there is room for does the order of insertion
-// decide (ordered_positions).
-template <int NX, int KMAX, bool POS>
-__global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneArgs a) {
+// issue rate of the insertion chains.  With the values known, a second walk collects the columns that reach a row's K-th value, in
+// the order of the list; there are K of them, and the rank of one is the number of larger values in the row's list, of equal
+// values the later column first.  Only where more columns share the K-th value than there is room for does the order of
+// insertion decide (ordered_positions).  Ranking each hit where it is met, in a tile that all lanes wait for: 114 us per
+// 128 x 5120 x 5120 layer against 99.
+template <int NX, int KMAX, bool POS, int SLOTS>
+__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 1) prune_sort(const __grid_constant__ PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
     constexpr int WALK = STEP;                               // entries per step: all insertion chains of a step are unrolled
     extern __shared__ __align__(16) unsigned char dyn[];
     float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(dyn);   // [NX] values, then [K] words
+    float* const found = reinterpret_cast<float*>(dyn) + (NX + (POS ? KMAX : 0)) * 32 * 33;   // POS: [8 warps][KMAX][32]
     __shared__ unsigned failed;
     const PruneProblem& p = a.p;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, K = p.K;
+    const int s = blockIdx.y, n0 = blockIdx.x * SLOTS, C = p.W_CI, K = p.K;
     const bool live = s * 32 + lane < p.B;
     const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
     if (dense_mode(a)) {
-        if (!POS) dense_prepare<NX>(a, s, n0, 0);            // positions: sort_positions_if reads the rows as they came
+        if (!POS) dense_prepare<NX>(a, s, n0, 0, SLOTS);     // positions: sort_positions_if reads the rows as they came
         return;
     }
     if (tid == 0) failed = 0u;
     __syncthreads();
 #pragma unroll 1
-    for (int i = 0; i < 4; i++) {
-        const int slot = warp * 4 + i, j = n0 + slot;
+    for (int i = 0; i < SLOTS / 8; i++) {
+        const int slot = warp * (SLOTS / 8) + i, j = n0 + slot;
         if (j >= p.CO) break;
         const int cnt = a.cnt[j];
         const float tau = a.tau[j];
@@ -940,24 +942,41 @@ __global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneA
         SortState<NX, KMAX> st;
         st.init();
         int k = 0;                                           // entries seen
+        float w[WALK], v[WALK][NX];
+        auto fetch = [&](int at, float (&wv)[WALK], float (&xv)[WALK][NX]) {
+#pragma unroll
+            for (int e = 0; e < WALK / 2; e++) {
+                const int4 two = list[at / 2 + e];
+                wv[2 * e] = __int_as_float(two.y);
+                wv[2 * e + 1] = __int_as_float(two.w);
+#pragma unroll
+                for (int t = 0; t < NX; t++) {
+                    xv[2 * e][t] = xt[((size_t)two.x * NX + t) * 32];
+                    xv[2 * e + 1][t] = xt[((size_t)two.z * NX + t) * 32];
+                }
+            }
+        };
+        // With one tensor the walk waits for its loads: the columns of a step come while the step before is entered.
+        if (NX == 1 && cnt > 0) fetch(0, w, v);
         for (; k < cnt; k += WALK) {
             if (k >= K) {
                 const float left = ub[k / STEP];
                 if (__all_sync(0xffffffffu, !live || st.worst(K) > left)) break;
             }
-            float w[WALK], v[WALK][NX];
+            if (NX == 1) {
+                float w0[WALK], v0[WALK][NX];
 #pragma unroll
-            for (int e = 0; e < WALK / 2; e++) {
-                const int4 two = list[k / 2 + e];
-                w[2 * e] = __int_as_float(two.y);
-                w[2 * e + 1] = __int_as_float(two.w);
+                for (int e = 0; e < WALK; e++) {
+                    w0[e] = w[e];
 #pragma unroll
-                for (int t = 0; t < NX; t++) {
-                    v[2 * e][t] = xt[((size_t)two.x * NX + t) * 32];
-                    v[2 * e + 1][t] = xt[((size_t)two.z * NX + t) * 32];
+                    for (int t = 0; t < NX; t++) v0[e][t] = v[e][t];
                 }
+                if (k + WALK < cnt) fetch(k + WALK, w, v);
+                st.add4(v0, w0);
+            } else {
+                fetch(k, w, v);
+                st.add4(v, w);
             }
-            st.add4(v, w);
         }
         const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || st.worst(K) >= tau);
         if (!good && lane == 0) atomicOr(&failed, 1u << slot);
@@ -965,8 +984,13 @@ __global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneA
         for (int t = 0; t < NX; t++) tile[t][lane][slot] = st.result(t, K, p.q);
         if (POS && good) {
             const float least = st.top[0].kth(K);
-            bool crowded = false;
-            for (int r = 0; r < K; r++) tile[NX + r][lane][slot] = __uint_as_float(EMPTY);
+            float* mine = found + (size_t)warp * KMAX * 32 + lane;   // this row's values in the order of the walk; their words in the tile
+            int hits = 0;
+            bool twice = false;
+#pragma unroll
+            for (int r = 1; r < KMAX; r++)
+                twice = twice || (r > KMAX - K && st.top[0].v[r] > 0.f && st.top[0].v[r] == st.top[0].v[r - 1]);
+            // Entries past k have smaller upper bounds than every row's K-th value: none of them is a hit.
             for (int k2 = 0; k2 < k; k2 += PAD) {
                 int c[PAD];
                 float w[PAD], v[PAD];
@@ -983,36 +1007,44 @@ __global__ void __launch_bounds__(256) prune_sort(const __grid_constant__ PruneA
 #pragma unroll
                 for (int e = 0; e < PAD; e++) {
                     const float t = v[e] - w[e], d = fabsf(t);
-                    const bool hit = d >= least && d > 0.f;
-                    if (!__any_sync(0xffffffffu, hit)) continue;
-                    int rank = 0;
-#pragma unroll
-                    for (int r = 0; r < KMAX; r++) rank += st.top[0].v[r] > d;
-                    if (hit) {
-                        uint32_t word = (uint32_t)c[e] | (t >= 0.f ? 0u : SNB_SIGN_BIT);
-                        for (; rank < K; rank++) {           // past equal values of later columns
-                            const uint32_t other = __float_as_uint(tile[NX + rank][lane][slot]);
-                            if (other == EMPTY || (other & ~SNB_SIGN_BIT) < (word & ~SNB_SIGN_BIT)) {
-                                tile[NX + rank][lane][slot] = __uint_as_float(word);
-                                word = other;
-                            }
-                            if (word == EMPTY) break;
+                    if (d >= least && d > 0.f) {
+                        if (hits < K) {
+                            mine[hits * 32] = d;
+                            tile[NX + hits][lane][slot] = __uint_as_float((uint32_t)c[e] | (t >= 0.f ? 0u : SNB_SIGN_BIT));
                         }
-                        crowded = crowded || rank == K;
+                        hits++;
                     }
                 }
+            }
+            const bool crowded = hits > K;
+            uint32_t word[KMAX];
+#pragma unroll
+            for (int r = 0; r < KMAX; r++) word[r] = r < K && r < hits ? __float_as_uint(tile[NX + r][lane][slot]) : EMPTY;
+            twice = __any_sync(0xffffffffu, twice);
+#pragma unroll
+            for (int i = 0; i < KMAX; i++) {
+                if (i >= K) break;
+                const float d = i < hits ? mine[i * 32] : -1.f;
+                int rank = 0;
+#pragma unroll
+                for (int r = 0; r < KMAX; r++) rank += st.top[0].v[r] > d;
+                if (twice)                                   // of equal values, the later column comes first
+#pragma unroll
+                    for (int r = 0; r < KMAX; r++)
+                        if (r < K && r < hits && i < hits && mine[r * 32] == d && (word[r] & ~SNB_SIGN_BIT) > (word[i] & ~SNB_SIGN_BIT)) rank++;
+                tile[NX + (i < hits ? min(rank, K - 1) : i)][lane][slot] = __uint_as_float(word[i]);
             }
             if (__any_sync(0xffffffffu, live && crowded))
                 ordered_positions<KMAX>(a.cand + (size_t)j * a.lcap, cnt, xt, live ? least : 0.f, K, tile + NX, slot);
         }
     }
     __syncthreads();
-    emit_tile<NX, NX, 0>(p, tile, s, n0, failed);
+    emit_tile<NX, NX, 0, SLOTS>(p, tile, s, n0, failed);
     if (POS) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int r = warp + 8 * k, b = s * 32 + r, n = n0 + lane;
-            if (b >= p.B || n >= p.CO) continue;
+            if (b >= p.B || n >= p.CO || lane >= SLOTS) continue;
             for (int t = 0; t < K; t++) {
                 const uint32_t word = __float_as_uint(tile[NX + t][r][lane]);
                 p.pos[((size_t)t * p.B + b) * p.CO + n] = word == EMPTY ? 0 : (int)word;   // fewer than K values above 0
@@ -1075,7 +1107,7 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
     char* tau = take(sizeof(float) * J);
     char* ub = take(sizeof(float) * J * (lcap / STEP));
     char* cand = take(sizeof(int2) * J * lcap);
-    char* fail = take(sizeof(int4) * S * ((p.CO + 31) / 32));
+    char* fail = take(sizeof(int4) * S * ((p.CO + 31) / 32) * (p.K > 1 ? 4 : 1));      // prune_sort: down to eight outputs per CTA
     const size_t ldr = (C + 3) / 4 * 4;
     char* xr = take(sizeof(float) * NX * S * 32 * ldr);
     char* partial = take(p.K > 1 ? 0 : (with_words(p) ? 8 : 4) * NX * S * p.CO * 32);
@@ -1155,16 +1187,28 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     return launched(2);
 }
 
+template <int NX, int KMAX, bool POS, int SLOTS>
+cudaError_t run_sort_walk(const PruneArgs& a, cudaStream_t st) {
+    constexpr int smem = ((NX + (POS ? KMAX : 0)) * 32 * 33 + (POS ? 8 * KMAX * 32 : 0)) * (int)sizeof(float);
+    const cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS, SLOTS>, smem>();
+    if (e != cudaSuccess) return e;
+    prune_sort<NX, KMAX, POS, SLOTS><<<dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256, smem, st>>>(a);
+    return launched();
+}
+
+// 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves
+// of four CTAs per SM they take eight (128 x 5120 x 5120 with positions, 640 CTAs of 32: 111 -> 99 us; 512 rows for point and
+// box, 2560 CTAs: 211 us with 32, 222 with 8).
 template <int NX, int KMAX, bool POS>
 cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
-    constexpr int smem = (NX + (POS ? KMAX : 0)) * 32 * 33 * (int)sizeof(float);
-    cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS>, smem>();
-    if (e != cudaSuccess) return e;
     int redo = 0;
-    if ((e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo)) != cudaSuccess) return e;
-    prune_sort<NX, KMAX, POS><<<grid, 256, smem, st>>>(a);
+    cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
+    if (e != cudaSuccess) return e;
+    if ((long long)grid.x * grid.y < 12ll * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
+    else e = run_sort_walk<NX, KMAX, POS, 32>(a, st);
+    if (e != cudaSuccess) return e;
     prune_redo_sort<NX, KMAX, POS><<<redo, 256, 0, st>>>(a);
-    if ((e = launched(2)) != cudaSuccess || !POS) return e;
+    if ((e = launched()) != cudaSuccess || !POS) return e;
     return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
 }
 

@@ -159,6 +159,35 @@ def half_prunable(kind, rng, B, CI, CO):
     return x.astype(np.float32), w
 
 
+@pytest.mark.parametrize("off", [-1, 0])
+@pytest.mark.parametrize("kind", ["normal", "ties"])
+@pytest.mark.parametrize("q,K", [(0.75, 10), (0.5, 4)])
+def test_sort_neuron_around_the_split_of_outputs(off, kind, q, K):
+    """Eight outputs per CTA below twelve CTAs of 32 per SM, 32 from there on: both give what 32 rows by themselves give
+    (those are held against the oracle above)."""
+    from sortnet_b200 import norm_dist_cuda as C
+    B, CI = 310, 140
+    tiles = -(-12 * torch.cuda.get_device_properties(0).multi_processor_count // 10) + off
+    CO = 32 * tiles - 27
+    x, w = operands(kind, np.random.default_rng(CO), B, CI, CO)
+    X, W = col3(x), dev(w)
+
+    def run(rows):
+        part, n = X[rows].contiguous(), rows.stop - rows.start
+        y, v = (torch.empty(n, CO, 1, device="cuda") for _ in range(2))
+        pos = torch.empty(K, n, CO, 1, device="cuda", dtype=torch.int32)
+        C.sort_neuron_forward(part, W, y, pos, 1, q, K)
+        C.sort_neuron_forward_nograd(part, W, v, 1, q, K)
+        return torch.stack((y, v)), pos
+
+    Y, P = run(slice(0, B))
+    assert torch.equal(Y[0], Y[1])
+    for b in range(0, B, 32):
+        rows = slice(b, min(b + 32, B))
+        y, p = run(rows)
+        assert torch.equal(y, Y[:, rows]) and torch.equal(p, P[:, rows])
+
+
 # columns around the tiles' steps (32) and the rows' alignment (4), outputs around their tiles (64, 128, 256), one and more sub-batches
 @pytest.mark.parametrize("B,CI,CO", [(33, 1024, 1100), (64, 1028, 1000), (70, 1025, 1000), (31, 1503, 1281), (100, 4100, 321)])
 @pytest.mark.parametrize("kind", ["single", "block", "wide", "wide ties"])
