@@ -447,17 +447,26 @@ class SortMLPModel(nn.Module):
         # would cost a device synchronisation per step and stop the host from queueing kernels
         # ahead of the GPU.
         # One draw for all layers: the generator gives the same numbers as one draw per layer.
-        uniform = torch.rand(sum(l.in_features for _, l in todo)).split([l.in_features for _, l in todo])
-        counts = [int((u < l.keep_rate).sum()) for u, (_, l) in zip(uniform, todo)]
+        widths = [l.in_features for _, l in todo]
+        uniform = torch.rand(sum(widths))
         device = torch.device(device)
-        if device.type == "cuda" and 1 < len(todo) <= 16:
+        batched = device.type == "cuda" and 1 < len(todo) <= 16
+        if batched:
             # all layers' lists in one launch; counts, seeds and lists are those of the per-layer calls
-            outs, seeds = [], torch.randint(0, 2 ** 62, (len(todo),)).tolist()
+            seeds = torch.randint(0, 2 ** 62, (len(todo),))
+            outs = _C.draw_lists(uniform, seeds, widths, [l.keep_rate for _, l in todo], sub, device)
+            if outs is not None:
+                for (k, _), out in zip(todo, outs):
+                    masks[k] = out
+                return masks
+        counts = [int((u < l.keep_rate).sum()) for u, (_, l) in zip(uniform.split(widths), todo)]
+        if batched:
+            outs = []
             for (k, l), c in zip(todo, counts):
                 c = min(max(int(c), 1), l.in_features)
                 outs.append(torch.empty(sub, 1, c, dtype=torch.int32, device=device))
                 masks[k] = outs[-1]
-            _C.sample_masks_into(outs, [l.in_features for _, l in todo], seeds)
+            _C.sample_masks_into(outs, widths, seeds.tolist())
             return masks
         for (k, l), c in zip(todo, counts):
             masks[k] = sample_mask(sub, 1, l.in_features, l.keep_rate, device, count=max(int(c), 1))

@@ -616,15 +616,8 @@ def certified_fraction(yl, yu, targets, row_flag, fraction):
 # ---- a whole SortNet-MLP per call -----------------------------------------------------------------
 
 
-class MlpLayer(ctypes.Structure):
-    """snb_mlp_layer of include/sortnet_b200.h."""
-    _fields_ = [("w", ctypes.c_void_p), ("bias", ctypes.c_void_p), ("running_mean", ctypes.c_void_p),
-                ("kept_list", ctypes.c_void_p), ("n_in", ctypes.c_int), ("n_out", ctypes.c_int), ("kept", ctypes.c_int),
-                ("K", ctypes.c_int), ("momentum", ctypes.c_float), ("q", ctypes.c_float)]
-
-
 class MlpPlan:
-    """The layer table of one call, with the tensors it points to."""
+    """The layer table of one call (csrc/ops_ext.cpp, MlpTable), with the tensors it points to."""
 
     def __init__(self, rows):
         """rows: (weight, bias, running_mean, momentum, kept list [S, 1, count] or None, K, q) per layer."""
@@ -632,16 +625,15 @@ class MlpPlan:
         self.weights = [r[0] for r in rows]
         self.head_bias = rows[-1][1]
         self.keep = rows
-        self.table = (MlpLayer * self.depth)(*[
-            MlpLayer(w.data_ptr(), _ptr(b), _ptr(rm), _ptr(kept), w.size(-1), w.size(0), 0 if kept is None else kept.size(-1),
-                     K, mom, q) for w, b, rm, mom, kept, K, q in rows])
+        self.native = _lib.ops().MlpTable(rows)
+        self.table = self.native.address()           # snb_mlp_layer[depth]
 
     def takes(self, x):
-        """Whether every tensor is what the kernels read through its pointer (csrc/ops_ext.cpp, mlp_takes)."""
-        return _lib.ops().mlp_takes(x, [(r[0], r[1], r[2], r[4]) for r in self.keep])
+        """Whether every tensor is what the kernels read through its pointer."""
+        return self.native.takes(x)
 
     def applies(self, B):
-        return _timeline is None and bool(_lib.load().snb_mlp_applies(self.table, self.depth, B))
+        return _timeline is None and self.native.applies(B)
 
 
 def _mlp_call(entry, ref, *args):
@@ -679,22 +671,20 @@ def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):
         for w, _, _, _, kept, _, _ in plan.keep:
             if kept is not None and not check_index_lists(kept, w.size(0), "mask"):
                 raise RuntimeError("mask is not in ascending order")
-    B, lib = x.size(0), _lib.load()
-    saved = torch.empty(lib.snb_mlp_saved_bytes(plan.table, plan.depth, B), device=x.device, dtype=torch.uint8)
-    scratch = torch.empty(lib.snb_mlp_scratch_bytes(plan.table, plan.depth, B, 1, 1), device=x.device, dtype=torch.uint8)
-    loss = torch.empty((), device=x.device, dtype=torch.float32)
-    _mlp_call("snb_mlp_train_forward", x, plan.table, plan.depth, x.data_ptr(), B, targets.data_ptr(), float(eps), float(clip),
-              float(lam), float(scale), saved.data_ptr(), scratch.data_ptr(), loss.data_ptr())
-    return loss, saved
+    return plan.native.train_forward(x, targets, eps, clip, lam, scale)
 
 
 def mlp_train_backward(plan, B, grad_loss, saved, grad_w, grad_bias, grad_x):
     """snb_mlp_train_backward; grad_w: one tensor or None per layer."""
-    scratch = torch.empty(_lib.load().snb_mlp_backward_scratch_bytes(plan.table, plan.depth, B), device=saved.device,
-                          dtype=torch.uint8)
-    ptrs = (ctypes.c_void_p * plan.depth)(*[_ptr(g) for g in grad_w])
-    _mlp_call("snb_mlp_train_backward", saved, plan.table, plan.depth, B, grad_loss.data_ptr(), saved.data_ptr(),
-              scratch.data_ptr(), ptrs, _ptr(grad_bias), _ptr(grad_x))
+    plan.native.train_backward(B, grad_loss, saved, grad_w, grad_bias, grad_x)
+
+
+def draw_lists(uniform, seeds, channels, keep, subs, device):
+    """One kept-channel list tensor [subs, 1, count] per layer in one launch (csrc/ops_ext.cpp, draw_lists), or None where the
+    Python form has to do it (numbers that are not host floats, a profile that is being taken)."""
+    if _timeline is not None or uniform.device.type != "cpu" or uniform.dtype != torch.float32 or seeds.device.type != "cpu":
+        return None
+    return _lib.ops().draw_lists(uniform, seeds, channels, keep, subs, device)
 
 
 def mlp_eval_forward(plan, x, box=None, targets=None, two_eps=1.0, scale=1.0):

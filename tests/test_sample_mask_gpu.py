@@ -113,6 +113,22 @@ def test_model_masks_are_the_same_through_either_route():
         assert torch.equal(batched[k], single)
 
 
+def test_drawn_lists_keep_the_counts_of_the_comparison():
+    """Rates 0 and 1, and numbers next to a rate that fp32 does not hold: counted as `uniform < rate` counts."""
+    from sortnet_b200 import norm_dist_cuda as C
+    rates, widths = [0.0, 1.0, 0.85, 0.7], [40, 33, 64, 1]
+    u = torch.rand(sum(widths))
+    near = torch.full((20,), 0.85)
+    u[73:93], u[93:113] = near, torch.nextafter(near, torch.zeros(20))
+    seeds = torch.arange(4)
+    lists = C.draw_lists(u, seeds, widths, rates, 3, torch.device("cuda"))
+    counts = [max(int((v < r).sum()), 1) for v, r in zip(u.split(widths), rates)]
+    outs = [torch.empty(3, 1, c, dtype=torch.int32, device="cuda") for c in counts]
+    C.sample_masks_into(outs, widths, seeds.tolist())
+    assert all(torch.equal(a, b) for a, b in zip(lists, outs))
+    assert C.draw_lists(u.double(), seeds, widths, rates, 3, torch.device("cuda")) is None
+
+
 def test_bad_arguments():
     from sortnet_b200 import norm_dist_cuda as C
     out = torch.empty(2, 1, 10, dtype=torch.int32, device="cuda")
