@@ -154,6 +154,61 @@ __global__ void __launch_bounds__(WM* WN * 32) bound_fwd_kernel(const BoundParam
     }
 }
 
+// ---- bounds + argmin/argmax words of small problems: a warp per row and four outputs, a lane per column of 32 -----
+// The same comparisons in the same order per lane; at the end the extreme value, of equal ones the lowest column.  Bound by latency
+// (9 x 97 x 33: 45 us by the tile kernel below, whose one CTA walks the columns alone).
+__global__ void __launch_bounds__(256) bound_small_kernel(const BoundParams p) {
+    const int lane = threadIdx.x & 31, quads = (p.CO + 3) / 4;
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= (long long)p.B * quads) return;
+    const int b = (int)(unit / quads), n0 = (int)(unit % quads) * 4;
+    const float *lr = p.xl + (size_t)b * p.CI, *ur = p.xu + (size_t)b * p.CI;
+    const float* wr[4];
+    float low[4], high[4];                                   // low: minus the smallest, as a maximum from its floor
+    uint32_t pl[4], pu[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        wr[i] = p.w + (size_t)min(n0 + i, p.CO - 1) * p.CI;
+        low[i] = high[i] = SNB_EPS;
+        pl[i] = SNB_NO_GRAD_ID;
+        pu[i] = 0u;
+    }
+#pragma unroll 2
+    for (int c = lane; c < p.CI; c += 32) {
+        float l = lr[c], u = ur[c];
+        if (l > u) l = u = (l + u) * 0.5f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float w = wr[i][c], t1 = w - l, t2 = u - w;
+            const float lo = -fminf(t1, t2), hi = fmaxf(t1, t2);
+            const uint32_t word = (uint32_t)c | (t1 <= t2 ? 0u : SNB_SIGN_BIT);
+            if (lo > low[i]) low[i] = lo, pl[i] = word;
+            if (hi > high[i]) high[i] = hi, pu[i] = word;
+        }
+    }
+    auto extreme = [&](float v, uint32_t word, uint32_t floor_word, float& best) {
+        const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(v));           // not negative: integer order
+        const bool here = __float_as_uint(v) == top && v > SNB_EPS;
+        const unsigned first = __reduce_min_sync(0xffffffffu, here ? word & ~SNB_SIGN_BIT : 0xffffffffu);
+        const unsigned owner = __ballot_sync(0xffffffffu, here && (word & ~SNB_SIGN_BIT) == first);
+        const uint32_t found = __shfl_sync(0xffffffffu, word, owner ? __ffs(owner) - 1 : 0);
+        best = __uint_as_float(top);
+        return owner ? found : floor_word;
+    };
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float yl, yu;
+        const uint32_t wl = extreme(low[i], pl[i], SNB_NO_GRAD_ID, yl), wu = extreme(high[i], pu[i], 0u, yu);
+        if (lane == i && n0 + i < p.CO) {
+            const size_t o = (size_t)b * p.CO + n0 + i;
+            p.yl[o] = yl;
+            p.yu[o] = yu;
+            p.posl[o] = (int)wl;
+            p.posu[o] = (int)wu;
+        }
+    }
+}
+
 // ---- bounds + argmin/argmax words: 4x4 outputs per thread, per-element strict updates ----
 template <bool VEC>
 __global__ void __launch_bounds__(256) bound_fwd_pos_kernel(const BoundParams p) {
@@ -430,6 +485,11 @@ extern "C" int snb_bound_inf_dist_forward_ws(const float* xl, const float* xu, c
     }
     BoundParams p{xl, xu, w, yl, yu, posl, posu, B, CO, CI, 0, 0, 0};
     const bool vec = (CI % 4 == 0) && aligned16(xl) && aligned16(xu) && aligned16(w);
+    if (small_problem(B, CO, CI)) {
+        bound_small_kernel<<<(unsigned)(((long long)B * ((CO + 3) / 4) + 7) / 8), 256, 0, (cudaStream_t)stream>>>(p);
+        SNB_CUDA(launched());
+        return SNB_OK;
+    }
     dim3 grid((B + 63) / 64, (CO + 63) / 64);
     constexpr int SMEM = 2 * 3 * 64 * LDS * (int)sizeof(float);
     static std::atomic<bool> configured[64];

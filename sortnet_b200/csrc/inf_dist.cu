@@ -529,6 +529,55 @@ static int check_fwd(const void* x, const void* w, const void* y, int B, int CO,
     return SNB_OK;
 }
 
+// Small problems: a warp per row and four outputs, a lane per column of 32; values and positions in one launch and without scratch.
+// The lanes' first largest elements meet at the end: the largest value, of equal ones the lowest column, as a scan in
+// ascending order with a strict comparison finds them.  Bound by latency.
+__global__ void __launch_bounds__(256) inf_small_kernel(const InfFwdParams p) {
+    const int lane = threadIdx.x & 31, quads = (p.CO + 3) / 4;
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= (long long)p.B * quads) return;
+    const int b = (int)(unit / quads), n0 = (int)(unit % quads) * 4, s = b / SNB_SUB_BATCH;
+    const int* ci_s = p.ci ? p.ci + (size_t)s * p.CI : nullptr;
+    const int* co_s = p.co ? p.co + (size_t)s * p.CO : nullptr;
+    const float* xr = p.x + (size_t)b * p.CI;
+    const float* wr[4];
+    float acc[4];
+    uint32_t word[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int n = min(n0 + i, p.CO - 1);
+        wr[i] = p.w + (size_t)(co_s ? co_s[n] : n) * p.W_CI;
+        acc[i] = SNB_EPS;
+        word[i] = 0u;
+    }
+#pragma unroll 4
+    for (int k = lane; k < p.CI; k += 32) {
+        const float x = xr[k];
+        const int c = ci_s ? ci_s[k] : k;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float t = x - wr[i][c], v = fabsf(t);
+            if (v > acc[i]) {
+                acc[i] = v;
+                word[i] = (uint32_t)k | (t < 0.f ? SNB_SIGN_BIT : 0u);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(acc[i]));      // not negative: integer order
+        const bool here = __float_as_uint(acc[i]) == top && acc[i] > SNB_EPS;
+        const unsigned first = __reduce_min_sync(0xffffffffu, here ? word[i] & ~SNB_SIGN_BIT : 0xffffffffu);
+        const unsigned owner = __ballot_sync(0xffffffffu, here && (word[i] & ~SNB_SIGN_BIT) == first);
+        const uint32_t found = __shfl_sync(0xffffffffu, word[i], owner ? __ffs(owner) - 1 : 0);
+        if (lane == i && n0 + i < p.CO) {
+            const size_t o = (size_t)b * p.CO + n0 + i;
+            p.y[o] = __uint_as_float(top);
+            p.pos[o] = owner ? (int)found : 0;
+        }
+    }
+}
+
 static int inf_forward_impl(const float* x, const float* w, int B, int CO, int CI, int G, int HW,
                             float* y, int* pos, const int* ci, const int* co, int W_CO, int W_CI,
                             void* ws, size_t ws_bytes, cudaStream_t st) {
@@ -548,6 +597,11 @@ static int inf_forward_impl(const float* x, const float* w, int B, int CO, int C
     unsigned long long* keys = ws && ws_bytes >= sizeof(unsigned long long) * (size_t)B * (size_t)CO
                                    ? (unsigned long long*)ws : nullptr;
     InfFwdParams p{x, w, y, pos, ci, co, B, CO, CI, W_CI};
+    if (CI <= SMALL_COLUMNS && small_problem(B, CO, CI)) {
+        inf_small_kernel<<<(unsigned)(((long long)B * ((CO + 3) / 4) + 7) / 8), 256, 0, st>>>(p);
+        SNB_CUDA(launched());
+        return SNB_OK;
+    }
     bool split = false;
     SNB_CUDA(dispatch_fwd<true>(p, keys, &split, st));
     SNB_CUDA(launch_resolve(p, keys, split, st));

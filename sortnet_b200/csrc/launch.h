@@ -32,6 +32,17 @@ inline cudaError_t allow_smem() {
 }
 constexpr int MOST_SMEM = 227 * 1024;        // what a CTA of sm_100a may have
 
+// Values with positions of small problems by one launch of a warp per row and four outputs, instead of tiles, partial results and a
+// second pass.  B200, launches inside a graph, tiles / warps.  Points: 18.4 / 2.5 us at 9 x 97 x 33, 11.5 / 2.7 at 32 x 256 x 128,
+// 11.7 / 4.5 at 64 x 256 x 256, 11.1 / 6.1 at 16 x 512 x 1024, 12.3 / 7.2 at 32 x 1000 x 250; boxes: 44.2 / 3.1 at 9 x 97 x 33, 82.4 / 5.3
+// at 32 x 256 x 128, 324 / 15 at 9 x 1000 x 200.  The limits: outputs, each of which ends in a reduction over its warp (128 K of them at
+// 64 columns 13.9 / 13.2 and 22.8 / 17.9; 262 K at 8 columns 15.4 / 21.6 and 12.7 / 27.9); terms (12.1 / 9.3 at 64 x 1024 x 256, but 18.0 / 28.1
+// at 512 x 128 x 512); and, for points, whose tiles share long rows out, the columns (4 x 5120 x 64: 12.2 / 19.5, boxes 1602 / 63).
+constexpr long long SMALL_TERMS = 8ll << 20, SMALL_OUTPUTS = 32ll << 10;
+constexpr int SMALL_COLUMNS = 1024;
+
+inline bool small_problem(int B, int CO, int CI) { return (long long)B * CO <= SMALL_OUTPUTS && (long long)B * CO * CI <= SMALL_TERMS; }
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace snb

@@ -97,6 +97,18 @@ def test_inverted_intervals_floors_and_ties():
     assert all(rel(a, b) < 1e-5 for a, b in zip(rb, ob))
 
 
+# quads of outputs, steps of 32 columns, long rows; the last sizes of the small form (8 M terms, 32 K outputs) and the first past them
+@pytest.mark.parametrize("B,CI,CO", [(1, 1, 3), (7, 31, 5), (35, 33, 4), (3, 5121, 30), (2, 5120, 819), (2, 5120, 820), (64, 9, 512), (65, 9, 512)])
+def test_small_problems_with_ties_nan_and_infinities(B, CI, CO):
+    rng = np.random.default_rng(B + CI)
+    xl, xu = ((rng.integers(0, 5, (B, CI)) / 4).astype(np.float32) for _ in range(2))      # about half are inverted
+    w = (rng.integers(-4, 5, (CO, CI)) / 4).astype(np.float32)
+    xl[0] = xu[0] = w[0] = 0.5
+    xl[B // 2, CI // 2], xu[B - 1, CI - 1], w[CO // 2, CI // 3] = np.nan, np.inf, np.nan
+    r, o = run_pos(xl, xu, w), oracle.bound_inf_dist_forward(xl, xu, w)
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(r, o))
+
+
 def test_bounds_enclose_the_point_value():
     from sortnet_b200 import norm_dist_cuda as C
     rng = np.random.default_rng(5)

@@ -77,6 +77,25 @@ def test_unmasked_vs_oracle(B, CI, CO):
     assert rel(gx2, gx_o) < 1e-5
 
 
+# quads of outputs, steps of 32 columns; the last sizes of the small form (1024 columns, 8 M terms, 32 K outputs) and the first past them
+@pytest.mark.parametrize("B,CI,CO", [(1, 1, 3), (7, 31, 5), (35, 33, 4), (3, 1024, 130), (3, 1025, 130), (64, 512, 256), (65, 512, 256),
+                                     (64, 9, 512), (65, 9, 512)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_small_problems_with_ties_nan_and_infinities(B, CI, CO, masked):
+    rng = np.random.default_rng(B + CI)
+    x = (rng.integers(0, 4, (B, CI)) / 4).astype(np.float32)
+    w = ((rng.standard_normal((CO, CI)) * 2).round() / 2).astype(np.float32)
+    w[0] = x[0]                                               # nothing above the floor
+    x[B // 2, CI // 2], w[CO // 2, CI // 3], x[B - 1, CI - 1] = np.nan, np.nan, np.inf
+    ci = co = None
+    if masked:
+        ci, co = make_masks(rng, B, CI, 0.9), make_masks(rng, B, CO, 0.9)
+        x = np.ascontiguousarray(x[:, :ci.shape[1]])
+    y_o, pos_o = oracle.inf_dist_forward(x, w, ci, co)
+    y, pos = run_forward(x, w, ci, co)
+    assert np.array_equal(y, y_o, equal_nan=True) and np.array_equal(pos, pos_o)
+
+
 @pytest.mark.parametrize("B,CI,CO,keep", [(70, 48, 40, 0.8), (96, 300, 520, 0.9), (33, 70, 90, 0.5),
                                           (160, 1030, 260, 0.9), (32, 64, 64, 1.0)])
 @pytest.mark.parametrize("which", ["both", "ci", "co"])
