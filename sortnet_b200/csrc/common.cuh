@@ -70,6 +70,12 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     return d;
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------
+// A kernel launched by launch_next (launch.h) may start while the one before it still runs: nothing that this wrote, and
+// nothing that it may still read, is touched before after_previous().  let_next() allows the next one to start.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- asynchronous global -> shared copies ---------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);

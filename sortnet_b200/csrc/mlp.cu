@@ -44,16 +44,17 @@ __global__ void __launch_bounds__(1024) keep_flags_kernel(const KeepJobs jobs) {
 // CTA = 16 channels, lane = row.  Bound by the latency of its two dependent reads (sums, then y from L2), so all of a
 // CTA's sums are fetched at once and eight rows of y per warp are in flight.
 constexpr int SHIFT_C = 16, SHIFT_S = 64;                    // sub-batches whose sums fit shared memory
-__global__ void __launch_bounds__(256) chain_shift_kernel(float* __restrict__ yt, const float* __restrict__ part,
-                                                          const unsigned char* __restrict__ keep, int B, int S, int C,
-                                                          float* __restrict__ running_mean, float momentum,
-                                                          float* __restrict__ rows_kept, unsigned* __restrict__ hi_out,
-                                                          unsigned* __restrict__ nlo_out) {
+// (No __restrict__: no load may be moved ahead of after_previous().)
+__global__ void __launch_bounds__(256) chain_shift_kernel(float* yt, const float* part, const unsigned char* keep, int B, int S, int C,
+                                                          float* running_mean, float momentum, float* rows_kept, unsigned* hi_out,
+                                                          unsigned* nlo_out) {
     __shared__ float sums[SHIFT_S][SHIFT_C];                 // NaN: dropped
     __shared__ float mean[SHIFT_C];
     __shared__ unsigned hi[SHIFT_C], nlo[SHIFT_C];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = blockIdx.x * SHIFT_C, n = min(SHIFT_C, C - c0);
     const int cx = tid & (SHIFT_C - 1), c = c0 + cx;
+    after_previous();
+    let_next();
     auto fetch = [&](int s) {
         const bool kept = cx < n && (!keep || keep[(size_t)s * C + c]);
         return kept ? part[(size_t)s * C + c] : __int_as_float(0x7fc00000);
@@ -155,6 +156,8 @@ __global__ void __launch_bounds__(CHAIN_THREADS) chain_bwd_kernel(const ChainBwd
     __shared__ float sums[CHAIN_ROWS][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp >> 1, half = warp & 1, t64 = threadIdx.x & 63;
     const int j = (int)blockIdx.x * CHAIN_ROWS + group, CO = a.CO, CI = a.CI, S = a.S;
+    after_previous();
+    let_next();
     if (j >= CO) return;
     const int each = min(CHAIN_S, (S + 1) / 2);              // sub-batches per warp and turn
     uint32_t word[CHAIN_S];
@@ -429,9 +432,8 @@ extern "C" int snb_mlp_train_forward(const snb_mlp_layer* l, int depth, const fl
         SNB_CUDA(prune_forward(p, sc.prune, st));
         count += 3;
         if (!head) {
-            chain_shift_kernel<<<(C + SHIFT_C - 1) / SHIFT_C, 256, 0, st>>>(p.yt, p.part, p.keep, B, S, C, l[k].running_mean, l[k].momentum,
-                                                              sv.rows_kept[k], sc.hi[k + 1], sc.nlo[k + 1]);
-            SNB_CUDA(launched());
+            SNB_CUDA(launch_next(chain_shift_kernel, (C + SHIFT_C - 1) / SHIFT_C, 256, 0, st, p.yt, p.part, p.keep, B, S, C, l[k].running_mean,
+                                 l[k].momentum, sv.rows_kept[k], sc.hi[k + 1], sc.nlo[k + 1]));
             count++;
         }
     }
@@ -477,8 +479,7 @@ extern "C" int snb_mlp_train_backward(const snb_mlp_layer* l, int depth, int B, 
         else if (k == 0) a.gx = grad_x;
         a.gw = grad_w[k];
         if (!a.gxt && !a.gx && !a.gw) continue;
-        chain_bwd_kernel<<<(a.CO + CHAIN_ROWS - 1) / CHAIN_ROWS, CHAIN_THREADS, 0, st>>>(a);
-        SNB_CUDA(launched());
+        SNB_CUDA(launch_next(chain_bwd_kernel, (a.CO + CHAIN_ROWS - 1) / CHAIN_ROWS, CHAIN_THREADS, 0, st, a));
         count++;
     }
     if (launches) *launches = count;

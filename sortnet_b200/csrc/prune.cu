@@ -147,27 +147,15 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
     __shared__ int hist[2 * R][BUCKETS];
     const int steps = (p.W_CO + R - 1) / R;
     const float nan = __int_as_float(0x7fc00000);
-    if (p.ci && (a.counters[GENERAL] & LIST_TWICE)) return;  // no list will be walked
     if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
+    // In a whole-net call the kernel before this one has nothing to do with W, whose first rows are fetched while it ends.
+    const bool ahead = p.xt && !p.ci;
+    if (!ahead) after_previous();
+    if (p.ci && (a.counters[GENERAL] & LIST_TWICE)) return;  // no list will be walked
     __syncthreads();
 
     if (tid < FT) {
         auto column = [&](int it, int e) { return it * 4 * FT + (VEC ? tid * 4 + e : e * FT + tid); };
-        float mid[NIT][4], rad[NIT][4];
-#pragma unroll
-        for (int it = 0; it < NIT; it++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int c = column(it, e);
-                const float hi = decode(c < C ? a.hi[c] : 0u), lo = -decode(c < C ? a.nlo[c] : 0u);
-                if (isinf(hi) || isinf(lo)) {
-                    mid[it][e] = 0.f;
-                    rad[it][e] = INFINITY;                   // always a candidate
-                } else {
-                    mid[it][e] = 0.5f * lo + 0.5f * hi;      // NaN without any value: never a candidate
-                    rad[it][e] = fmaxf(hi - mid[it][e], mid[it][e] - lo) * (1.0f + 0x1p-22f);
-                }
-            }
         auto fetch = [&](int step, int st) {
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -196,6 +184,23 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
             if (step < steps) fetch(step, k);
             cp_async_commit();
         }
+        if (ahead) after_previous();
+        let_next();
+        float mid[NIT][4], rad[NIT][4];
+#pragma unroll
+        for (int it = 0; it < NIT; it++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int c = column(it, e);
+                const float hi = decode(c < C ? a.hi[c] : 0u), lo = -decode(c < C ? a.nlo[c] : 0u);
+                if (isinf(hi) || isinf(lo)) {
+                    mid[it][e] = 0.f;
+                    rad[it][e] = INFINITY;                   // always a candidate
+                } else {
+                    mid[it][e] = 0.5f * lo + 0.5f * hi;      // NaN without any value: never a candidate
+                    rad[it][e] = fmaxf(hi - mid[it][e], mid[it][e] - lo) * (1.0f + 0x1p-22f);
+                }
+            }
         int i = 0, st = 0;
         for (int step = blockIdx.x; step < steps; step += gridDim.x, i++) {
             const int buf = i & 1;
@@ -291,6 +296,8 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
     }
 
     // ordering warps: list r of every other step, by U, largest first, in BUCKETS steps of U
+    if (ahead) after_previous();
+    let_next();
     const int o = warp - WARPS, r = o % R, buf = o / R;
     float* u_in = bounds + o * (lcap + lcap / STEP);
     unsigned* u_step = reinterpret_cast<unsigned*>(u_in + lcap);                     // largest U of each step of four
@@ -728,6 +735,8 @@ __global__ void __launch_bounds__(256, NX == 1 && !TRACK ? 6 : NX == 2 && TRACK 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 3, l = lane & 7;
     const int s = blockIdx.y, n0 = blockIdx.x * 32, C = p.W_CI, slot = warp * 4 + g, n = n0 + slot;
     const float4* xt = reinterpret_cast<const float4*>(a.xt + (size_t)s * C * NX * 32) + l;
+    after_previous();
+    let_next();
     const unsigned overflowed = load_now(a.counters + OVERFLOWED), general = p.ci ? load_now(a.counters + GENERAL) : 0u;
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
     const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
@@ -925,6 +934,8 @@ __global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 1) prune_sort(const __gr
     const int s = blockIdx.y, n0 = blockIdx.x * SLOTS, C = p.W_CI, K = p.K;
     const bool live = s * 32 + lane < p.B;
     const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
+    after_previous();
+    let_next();
     if (dense_mode(a)) {
         if (!POS) dense_prepare<NX>(a, s, n0, 0, SLOTS);     // positions: sort_positions_if reads the rows as they came
         return;
@@ -1149,8 +1160,7 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_filter<R, NIT, FT, STAGES, VEC>, FT + 64 * R, smem);
     if (e != cudaSuccess) return e;
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
-    prune_filter<R, NIT, FT, STAGES, VEC><<<steps < slots ? steps : slots, FT + 64 * R, smem, st>>>(a);
-    return launched();
+    return launch_next(prune_filter<R, NIT, FT, STAGES, VEC>, steps < slots ? steps : slots, FT + 64 * R, smem, st, a);
 }
 
 template <bool VEC>
@@ -1182,9 +1192,8 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     int redo = 0;
     if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
-    prune_max<NX, TRACK><<<grid, 256, 0, st>>>(a);
-    prune_redo_max<NX, TRACK><<<redo, REDO_THREADS, smem, st>>>(a);
-    return launched(2);
+    if ((e = launch_next(prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
+    return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
 }
 
 template <int NX, int KMAX, bool POS, int SLOTS>
@@ -1192,8 +1201,7 @@ cudaError_t run_sort_walk(const PruneArgs& a, cudaStream_t st) {
     constexpr int smem = ((NX + (POS ? KMAX : 0)) * 32 * 33 + (POS ? 8 * KMAX * 32 : 0)) * (int)sizeof(float);
     const cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS, SLOTS>, smem>();
     if (e != cudaSuccess) return e;
-    prune_sort<NX, KMAX, POS, SLOTS><<<dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256, smem, st>>>(a);
-    return launched();
+    return launch_next(prune_sort<NX, KMAX, POS, SLOTS>, dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256, smem, st, a);
 }
 
 // 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves
@@ -1207,8 +1215,7 @@ cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     if ((long long)grid.x * grid.y < 12ll * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
     else e = run_sort_walk<NX, KMAX, POS, 32>(a, st);
     if (e != cudaSuccess) return e;
-    prune_redo_sort<NX, KMAX, POS><<<redo, 256, 0, st>>>(a);
-    if ((e = launched()) != cudaSuccess || !POS) return e;
+    if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;
     return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
 }
 

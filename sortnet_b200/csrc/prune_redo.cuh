@@ -555,6 +555,8 @@ template <int NX, bool TRACK>
 __global__ void __launch_bounds__(REDO_THREADS, 2) prune_redo_max(const __grid_constant__ PruneArgs a) {
     constexpr int WARPS = REDO_THREADS / 32;
     extern __shared__ __align__(16) float redo_smem[];
+    after_previous();
+    let_next();
     if (dense_mode(a)) {
         const DenseLayer d(a);
         if constexpr (NX != 2) {
@@ -782,6 +784,8 @@ __device__ void dense_sort(const PruneArgs& a, float* sm) {
 template <int NX, int KMAX, bool POS>
 __global__ void __launch_bounds__(256, KMAX > 10 ? 1 : (NX == 1 && !POS ? 4 : 2)) prune_redo_sort(const __grid_constant__ PruneArgs a) {
     __shared__ __align__(16) float sm[SORT_STAGES];
+    after_previous();
+    let_next();
     if (dense_mode(a)) {
         if constexpr (!POS) dense_sort<NX, KMAX>(a, sm);    // POS: sort_positions_if
         return;

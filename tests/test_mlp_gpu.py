@@ -98,3 +98,35 @@ def test_evaluation_pass(B, depth, width, dims, classes, keep, flat):
             got, want = run(), layer_by_layer(run)
             for u, v in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
                 assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("flat", [False, True])
+def test_weights_written_right_before_a_pass(flat):
+    """The kernels of a pass may start while the ones before them end, under capture as well: what is written to the weights and
+    to the input ahead of a pass is seen by it, and replays follow one another without waiting."""
+    a, b = nets(4, 700, (3, 17, 17), 10, 1.0, std=0.02 if flat else 1.0)
+    a.eval(), b.eval()
+    x = torch.rand(70, 3, 17, 17, device="cuda")
+    t = torch.randint(0, 10, (70,), device="cuda")
+
+    def step(net, to):
+        for l in net.fc_dist:
+            l.weight.mul_(1.01)
+        to.mul_(0.99)
+        out = net(to, t, 0.02, up=1.0, down=0.0)
+        return out if isinstance(out, tuple) else (out,)
+
+    with torch.no_grad():
+        u, v = x.clone(), x.clone()
+        assert a._plan(None).applies(70)
+        got = [step(a, u) for _ in range(3)]
+        want = [layer_by_layer(lambda: step(b, v)) for _ in range(3)]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            last = step(a, u)
+        for _ in range(3):
+            graph.replay()
+            got.append([o.clone() for o in last])
+            want.append(layer_by_layer(lambda: step(b, v)))
+        for p, q in zip(got, want):
+            assert len(p) == len(q) and all(torch.equal(u, v) for u, v in zip(p, q))
