@@ -509,12 +509,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sort_neuron", &sort_neuron);
     m.def("bound_inf_dist", &bound_inf_dist);
     m.def("bound_sort_neuron", &bound_sort_neuron);
-    m.def("draw_lists", &draw_lists);
+    // A call that issues a whole pass takes long, and as long as the device does once the launch queue is full: other Python
+    // threads run meanwhile.  None of the three touches a Python object.
+    using Unlocked = py::call_guard<py::gil_scoped_release>;
+    m.def("draw_lists", &draw_lists, Unlocked());
     py::class_<MlpTable>(m, "MlpTable")
         .def(py::init<std::vector<Row>>())
         .def("address", &MlpTable::address)
         .def("applies", &MlpTable::applies)
         .def("takes", &MlpTable::takes)
-        .def("train_forward", &MlpTable::train_forward)
-        .def("train_backward", &MlpTable::train_backward);
+        .def("train_forward", &MlpTable::train_forward, Unlocked())
+        .def("train_backward", &MlpTable::train_backward, Unlocked());
 }

@@ -130,3 +130,47 @@ def test_weights_written_right_before_a_pass(flat):
             want.append(layer_by_layer(lambda: step(b, v)))
         for p, q in zip(got, want):
             assert len(p) == len(q) and all(torch.equal(u, v) for u, v in zip(p, q))
+
+
+@pytest.mark.parametrize("what", ["forward", "backward", "lists"])
+def test_other_threads_run_while_a_pass_is_issued(what):
+    """A call that waits for room in the launch queue does not hold the interpreter lock."""
+    import threading
+    import time
+    from sortnet_b200 import norm_dist_cuda as C
+    net, _ = nets(4, 700, (3, 17, 17), 10, 0.8)
+    x, t = torch.rand(70, 867, device="cuda"), torch.randint(0, 10, (70,), device="cuda")
+    plan = net._plan(net.draw_masks(70, x.device))
+    one, grads = torch.ones((), device="cuda"), [torch.empty_like(w) for w in plan.weights]
+    _, saved = C.mlp_train_forward(plan, x, t, 0.05, 1.0, 0.1, 1.0)
+    uniform, seeds = torch.rand(64), torch.zeros(1, dtype=torch.int64)
+    call = {"forward": lambda: C.mlp_train_forward(plan, x, t, 0.05, 1.0, 0.1, 1.0),
+            "backward": lambda: C.mlp_train_backward(plan, 70, one, saved, grads, None, None),
+            "lists": lambda: C.draw_lists(uniform, seeds, [64], [0.5], 3, x.device)}[what]
+    call()
+    torch.cuda.synchronize()
+    ticks, end = [], threading.Event()
+
+    def tick():
+        while not end.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.001)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(10 ** 9)                           # about half a second, behind which the launches pile up
+        slept = torch.cuda.Event()
+        slept.record()
+        began, ended = 0.0, 0.0
+        while not slept.query():
+            t0 = time.perf_counter()
+            call()
+            t1 = time.perf_counter()
+            if t1 - t0 > ended - began:
+                began, ended = t0, t1
+    finally:
+        end.set()
+        thread.join()
+    assert ended - began > 0.05, "no call had to wait"
+    assert sum(began < s < ended for s in ticks) > 100 * (ended - began)
