@@ -638,7 +638,7 @@ __device__ __forceinline__ void emit_chain(const PruneProblem& p, int s, int j, 
 
 // SLOTS outputs from the tile [NV values (+ NW words)][row][output]: row-major arrays and the chain form.
 template <int NX, int NV, int NW, int SLOTS = 32>
-__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][33], int s, int n0, unsigned again = 0u) {
+__device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[32][SLOTS + 1], int s, int n0, unsigned again = 0u) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* outs[NV];
     if (NX != 2) outs[0] = p.y;
@@ -895,9 +895,9 @@ __global__ void __launch_bounds__(256, NX == 1 && !TRACK ? 6 : NX == 2 && TRACK 
 
 // Positions of one output whose K-th largest value is shared by several columns in some row: the entries of
 // the list in ascending column order through PosList (rare; 32 lanes pick the next column together).
-template <int KMAX>
+template <int KMAX, int LD>
 __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, const float* xt, float least, int K,
-                                               float (*words)[32][33], int slot) {
+                                               float (*words)[32][LD], int slot) {
     const int lane = threadIdx.x & 31;
     PosList<KMAX> pl;
     pl.init(least);
@@ -926,12 +926,13 @@ __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, con
 // insertion decide (ordered_positions).  Ranking each hit where it is met, in a tile that all lanes wait for: 114 us per
 // 128 x 5120 x 5120 layer against 99.
 template <int NX, int KMAX, bool POS, int SLOTS>
-__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 1) prune_sort(const __grid_constant__ PruneArgs a) {
+__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : POS ? 2 : 1) prune_sort(const __grid_constant__ PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
     constexpr int WALK = STEP;                               // entries per step: all insertion chains of a step are unrolled
+    constexpr int LD = SLOTS + 1;
     extern __shared__ __align__(16) unsigned char dyn[];
-    float(*tile)[32][33] = reinterpret_cast<float(*)[32][33]>(dyn);   // [NX] values, then [K] words
-    float* const found = reinterpret_cast<float*>(dyn) + (NX + (POS ? KMAX : 0)) * 32 * 33;   // POS: [8 warps][KMAX][32]
+    float(*tile)[32][LD] = reinterpret_cast<float(*)[32][LD]>(dyn);   // [NX] values, then [K] words
+    float* const found = reinterpret_cast<float*>(dyn) + (NX + (POS ? a.p.K : 0)) * 32 * LD;  // POS: [8 warps][K][32]
     __shared__ unsigned failed;
     const PruneProblem& p = a.p;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -999,7 +1000,7 @@ __global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 1) prune_sort(const __gr
         for (int t = 0; t < NX; t++) tile[t][lane][slot] = st.result(t, K, p.q);
         if (POS && good) {
             const float least = st.top[0].kth(K);
-            float* mine = found + (size_t)warp * KMAX * 32 + lane;   // this row's values in the order of the walk; their words in the tile
+            float* mine = found + warp * K * 32 + lane;   // this row's values in the order of the walk; their words in the tile
             int hits = 0;
             bool twice = false;
 #pragma unroll
@@ -1050,7 +1051,7 @@ __global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 1) prune_sort(const __gr
                 tile[NX + (i < hits ? min(rank, K - 1) : i)][lane][slot] = __uint_as_float(word[i]);
             }
             if (__any_sync(0xffffffffu, live && crowded))
-                ordered_positions<KMAX>(a.cand + (size_t)j * a.lcap, cnt, xt, live ? least : 0.f, K, tile + NX, slot);
+                ordered_positions<KMAX, LD>(a.cand + (size_t)j * a.lcap, cnt, xt, live ? least : 0.f, K, tile + NX, slot);
         }
     }
     __syncthreads();
@@ -1200,23 +1201,31 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
 }
 
+template <int NX, bool POS, int SLOTS>
+constexpr int sort_walk_smem(int K) {
+    return ((NX + (POS ? K : 0)) * 32 * (SLOTS + 1) + (POS ? 8 * K * 32 : 0)) * (int)sizeof(float);
+}
 template <int NX, int KMAX, bool POS, int SLOTS>
 cudaError_t run_sort_walk(const PruneArgs& a, cudaStream_t st) {
-    constexpr int smem = ((NX + (POS ? KMAX : 0)) * 32 * 33 + (POS ? 8 * KMAX * 32 : 0)) * (int)sizeof(float);
-    const cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS, SLOTS>, smem>();
+    const cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS, SLOTS>, sort_walk_smem<NX, POS, SLOTS>(KMAX)>();
     if (e != cudaSuccess) return e;
-    return launch_next(prune_sort<NX, KMAX, POS, SLOTS>, dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256, smem, st, a);
+    return launch_next(prune_sort<NX, KMAX, POS, SLOTS>, dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256,
+                       sort_walk_smem<NX, POS, SLOTS>(a.p.K), st, a);
 }
 
-// 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves
-// of four CTAs per SM they take eight (128 x 5120 x 5120 with positions, 640 CTAs of 32: 111 -> 99 us; 512 rows for point and
-// box, 2560 CTAs: 211 us with 32, 222 with 8).
+// 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves of what
+// fits (four CTAs per SM up to ten values, two above: registers) they take eight.  Up to ten values: 128 x 5120 x 5120 with positions,
+// 640 CTAs of 32: 111 us with 32, 99 with 8; 512 rows for point and box, 2560 CTAs: 211 with 32, 222 with 8.  More, with positions, by 32 / 8
+// outputs: 32 x 2048 x 2048 143 / 68 us at K = 17, 128 x 5120 x 5120 536 / 546, 512 x 5120 x 5120 1332 / 1476; past K = 21 the positions of
+// 32 outputs leave room for one CTA: K = 25 at 200 x 2048 x 3000 701 / 577.
 template <int NX, int KMAX, bool POS>
 cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     int redo = 0;
     cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
     if (e != cudaSuccess) return e;
-    if ((long long)grid.x * grid.y < 12ll * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
+    constexpr int FIT = KMAX <= 10 ? 4 : 2;
+    const bool room = FIT * (sort_walk_smem<NX, POS, 32>(a.p.K) + 1152) <= 228 * 1024;       // an SM's; 1 KB per CTA is taken, and its own few words
+    if (!room || (long long)grid.x * grid.y < 3ll * FIT * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
     else e = run_sort_walk<NX, KMAX, POS, 32>(a, st);
     if (e != cudaSuccess) return e;
     if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;

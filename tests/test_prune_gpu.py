@@ -188,6 +188,39 @@ def test_sort_neuron_around_the_split_of_outputs(off, kind, q, K):
         assert torch.equal(y, Y[:, rows]) and torch.equal(p, P[:, rows])
 
 
+@pytest.mark.parametrize("off", [-1, 0])
+@pytest.mark.parametrize("kind", ["normal", "ties"])
+@pytest.mark.parametrize("K", [11, 21, 22, 25])
+def test_sort_neuron_of_many_values_around_the_split_of_outputs(off, kind, K):
+    """The same above ten values: eight outputs per CTA below six CTAs of 32 per SM, and always past K = 21."""
+    from sortnet_b200 import _lib, norm_dist_cuda as C
+    B, CI, q = 100, 200, 0.8
+    CO = 32 * (-(-6 * torch.cuda.get_device_properties(0).multi_processor_count // 4) + off) - 27
+    x, w = operands(kind, np.random.default_rng(CO), B, CI, CO)
+    X, W = col3(x), dev(w)
+    y, v, z = (torch.empty(B, CO, 1, device="cuda") for _ in range(3))
+    pos, want = (torch.empty(K, B, CO, 1, device="cuda", dtype=torch.int32) for _ in range(2))
+    C.sort_neuron_forward(X, W, y, pos, 1, q, K)
+    C.sort_neuron_forward_nograd(X, W, v, 1, q, K)
+    _lib.check(_lib.load().snb_sort_neuron_forward(X.data_ptr(), W.data_ptr(), B, CO, CI, 1, 1, z.data_ptr(), want.data_ptr(), q, K,
+                                                   torch.cuda.current_stream().cuda_stream), "sort_neuron_forward")
+    assert torch.equal(pos, want) and torch.equal(y, v) and rel(host(y), host(z)) < 2e-6
+
+
+def test_positions_of_25_values_where_some_lists_overflow():
+    """Outputs that the walk leaves to prune_redo, among others that it does not: the positions of all are the dense kernel's."""
+    from sortnet_b200 import _lib, norm_dist_cuda as C
+    B, CI, CO, q, K = 70, 5120, 700, 0.75, 25
+    x, w = operands("normal", np.random.default_rng(3), B, CI, CO)
+    X, W = col3(x), dev(w)
+    y, z = (torch.empty(B, CO, 1, device="cuda") for _ in range(2))
+    pos, want = (torch.full((K, B, CO, 1), -1, device="cuda", dtype=torch.int32) for _ in range(2))
+    C.sort_neuron_forward(X, W, y, pos, 1, q, K)
+    _lib.check(_lib.load().snb_sort_neuron_forward(X.data_ptr(), W.data_ptr(), B, CO, CI, 1, 1, z.data_ptr(), want.data_ptr(), q, K,
+                                                   torch.cuda.current_stream().cuda_stream), "sort_neuron_forward")
+    assert torch.equal(pos, want) and rel(host(y), host(z)) < 2e-6
+
+
 # columns around the tiles' steps (32) and the rows' alignment (4), outputs around their tiles (64, 128, 256), one and more sub-batches
 @pytest.mark.parametrize("B,CI,CO", [(33, 1024, 1100), (64, 1028, 1000), (70, 1025, 1000), (31, 1503, 1281), (100, 4100, 321)])
 @pytest.mark.parametrize("kind", ["single", "block", "wide", "wide ties"])
