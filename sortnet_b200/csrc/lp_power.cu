@@ -191,10 +191,12 @@ __global__ void __launch_bounds__(FWD_NT, 3) lp_power_fwd_kernel(const LpFwdPara
 // and a warp's reduction into grad_w covers 32 neighbouring kept columns.  (g, y) of the next 32 outputs are copied to shared memory
 // [j][row] meanwhile; each thread turns the elements that it copied into g / y^(p-1) before the barrier, so that a term is one
 // subtract, the multiply chain and two fmas, and reads them back four rows at a time (all lanes the same words: broadcast).
+// Four CTAs per SM, and three for p = 1, whose selected signs take 168 registers: with 128 it spills (67 x 1000 x 1000 37.0 -> 34.6 us, 16 x
+// 5120 x 5120 227 -> 220, 512 x 2048 x 2048 505 -> 506).
 constexpr int BWD_NT = 128, BWD_JT = 32, BWD_LD = 36, BWD_AHEAD = 8;
 
 template <int IP>
-__global__ void __launch_bounds__(BWD_NT, 4) lp_power_bwd_kernel(const LpBwdParams p) {
+__global__ void __launch_bounds__(BWD_NT, IP == 0 ? 3 : 4) lp_power_bwd_kernel(const LpBwdParams p) {
     constexpr int NT = BWD_NT, JT = BWD_JT, LD = BWD_LD, AHEAD = BWD_AHEAD;
     __shared__ __align__(16) float gt[2][JT * LD], yt[2][JT * LD];
     const int tid = threadIdx.x, lane = tid & 31;
