@@ -45,7 +45,8 @@ inline cudaError_t launch_next(void (*kern)(Params...), dim3 grid, dim3 block, s
     config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem, config.stream = st;
     config.attrs = &attribute, config.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&config, kern, static_cast<Params>(args)...);
-    return e != cudaSuccess ? e : launched();
+    const cudaError_t last = launched();                     // takes a failed launch's error away, so that no later call reports it
+    return e != cudaSuccess ? e : last;
 }
 
 // Values with positions of small problems by one launch of a warp per row and four outputs, instead of tiles, partial results and a

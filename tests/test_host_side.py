@@ -93,6 +93,33 @@ REFERENCE_NAMES = [
 ]
 
 
+FAILED_LAUNCH = """
+#include "launch.h"
+// the runtime keeps the error of a failed call until somebody takes it
+static cudaError_t held = cudaSuccess;
+extern "C" cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return held = cudaErrorInvalidConfiguration; }
+extern "C" cudaError_t cudaGetLastError() {
+    const cudaError_t e = held;
+    held = cudaSuccess;
+    return e;
+}
+cudaError_t snb::launched(int) { return cudaGetLastError(); }
+static void kernel(int) {}
+int main() { return snb::launch_next(kernel, 1, 1, 0, nullptr, 0) != cudaErrorInvalidConfiguration ? 1 : held != cudaSuccess ? 2 : 0; }
+"""
+
+
+def test_failed_launch_is_reported_once(tmp_path):
+    """The next call, which works, must not be refused for it."""
+    import subprocess
+    from sortnet_b200 import build
+    source, program = tmp_path / "failed_launch.cpp", tmp_path / "failed_launch"
+    source.write_text(FAILED_LAUNCH)
+    subprocess.run(["g++", "-std=c++17", "-I", build.CSRC, "-I", os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"),
+                    str(source), "-o", str(program)], check=True)
+    assert subprocess.run([str(program)]).returncode == 0
+
+
 def test_tensor_level_module_has_the_reference_names():
     from sortnet_b200 import norm_dist_cuda as C
     for n in REFERENCE_NAMES:
