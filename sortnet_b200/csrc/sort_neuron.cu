@@ -478,14 +478,18 @@ cudaError_t sort_positions_if(const PruneProblem& q, const unsigned* overflowed,
 }
 
 // Sparse backward: one CTA per batch row, grad_x of the row accumulated in shared memory.  Bound by latency: all words of
-// an output are on their way before the first one is used (128 x 5120 x 5120, K = 10: 90 us with one word at a time
-// and 256 threads, 15 us).
-constexpr int SORT_BWD_THREADS = 1024;
-template <int KMAX>
-__global__ void __launch_bounds__(SORT_BWD_THREADS, 1) sort_bwd_kernel(const float* __restrict__ g, const int* __restrict__ pos,
-                                                                       int B, int CO, int CI, int K, float q, float c0,
-                                                                       float* __restrict__ gx, float* __restrict__ gw,
-                                                                       int use_smem) {
+// an output are on their way before the first one is used (128 x 5120 x 5120, K = 10, grad_x alone: 90 us with one word at a time
+// and 256 threads, 15 us with 1024; with grad_w 142 and 57).
+// Threads of a CTA, by rows x columns x outputs, with grad_w, 256 / 512 / 1024 threads (before: 256, a word at a time); K = 10 if not said:
+//   up to 256 outputs 256, as more have nothing to do: 512 x 5120 x 10 6.3 / 8.2 / 12.7 us (7.8), 4096 x 784 x 100 40 / 42 / 78 (41);
+//   rows that all have an SM to themselves 1024: 128 x 5120 x 5120 63 / 58 / 56 (141);
+//   more rows 512, of which two CTAs fit: 512 x 1024 x 1024 40 / 33 / 35 (41), 512 x 5120 x 5120 194 / 163 / 162 (191); but 256, of which four
+//   do, where a last wave of 512 would leave half of the device idle: 310 x 140 x 1800 54 / 56 / 51 (55), at K = 2 13.1 / 14.3 / 16.5 (14.1), at K = 4
+//   23.7 / 24.9 / 25.1 (23.6). Above ten values that is no gain: 300 x 2048 x 2048 at K = 11 52 / 49 / 54 (51).
+template <int KMAX, int SORT_BWD_THREADS>
+__global__ void __launch_bounds__(SORT_BWD_THREADS, KMAX > 10 ? 1024 / SORT_BWD_THREADS : 1)
+sort_bwd_kernel(const float* __restrict__ g, const int* __restrict__ pos, int B, int CO, int CI, int K, float q, float c0,
+                float* __restrict__ gx, float* __restrict__ gw, int use_smem) {
     extern __shared__ float row[];
     const int b = blockIdx.x;
     float* acc = use_smem ? row : gx + (size_t)b * CI;
@@ -646,9 +650,17 @@ static int sort_backward(const float* g, const int* pos, int B, int CO, int CI, 
     float n = powf(1 - q, (float)K);
     n = 1.0f + n / (1.0f - n);
     const size_t smem = use_smem ? CI * sizeof(float) : 0;
-    if (K <= 10) sort_bwd_kernel<10><<<B, SORT_BWD_THREADS, smem, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
-    else sort_bwd_kernel<25><<<B, SORT_BWD_THREADS, smem, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
-    SNB_CUDA(launched());
+    auto go = [&](auto kern, int threads) {
+        kern<<<B, threads, smem, st>>>(g, pos, B, CO, CI, K, q, n, gx, gw, use_smem);
+        return launched();
+    };
+    const int sms = sm_count(), last = B % (2 * sms);        // rows in the last wave of CTAs of 512 threads
+    if (CO <= 256 || (K <= 10 && B > sms && last > 0 && last <= sms))
+        SNB_CUDA(K <= 10 ? go(sort_bwd_kernel<10, 256>, 256) : go(sort_bwd_kernel<25, 256>, 256));
+    else if (B > sms)
+        SNB_CUDA(K <= 10 ? go(sort_bwd_kernel<10, 512>, 512) : go(sort_bwd_kernel<25, 512>, 512));
+    else
+        SNB_CUDA(K <= 10 ? go(sort_bwd_kernel<10, 1024>, 1024) : go(sort_bwd_kernel<25, 1024>, 1024));
     return SNB_OK;
 }
 

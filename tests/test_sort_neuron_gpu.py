@@ -96,3 +96,22 @@ def test_autograd_function_and_model_eval():
     # the certified margin is an upper bound of the clean margin
     clean = logits - torch.gather(logits, 1, t.view(-1, 1))
     assert (margin * (2 * 0.01) + 1e-5 >= clean.scatter(1, t.view(-1, 1), 0)).all()
+
+
+# outputs around 256, rows around one and two CTAs per SM (148 SMs) and one and a half waves of two, rows in global memory
+@pytest.mark.parametrize("K", [3, 10, 11, 25])
+@pytest.mark.parametrize("B,CI,CO", [(149, 60, 256), (148, 60, 257), (149, 60, 257), (296, 30, 300), (297, 30, 300), (444, 30, 300),
+                                     (445, 30, 300), (33, 12289, 257), (150, 12289, 40)])
+def test_backward_by_rows_and_outputs(B, CI, CO, K):
+    from sortnet_b200 import norm_dist_cuda as C
+    rng = np.random.default_rng(B + CO)
+    pos = rng.integers(0, CI, (K, B, CO)).astype(np.uint32) | (rng.integers(0, 2, (K, B, CO)).astype(np.uint32) << 31)
+    pos = pos.view(np.int32)
+    g = rng.standard_normal((B, CO)).astype(np.float32)
+    gx_o, gw_o = oracle.sort_backward(g, pos, CI, 0.8, K)
+    P = dev(pos).unsqueeze(-1).contiguous()
+    gx, gx2 = (torch.full((B, CI, 1), float("nan"), device="cuda") for _ in range(2))
+    gw = torch.full((CO, CI), float("nan"), device="cuda")
+    C.sort_neuron_backward_input_weight(col3(g), P, gx, gw, 1, 0.8, K)
+    C.sort_neuron_backward_input(col3(g), P, gx2, 1, 0.8, K)
+    assert rel(host(gx), gx_o) < 1e-5 and rel(gw.cpu().numpy(), gw_o) < 1e-5 and rel(host(gx2), gx_o) < 1e-5
