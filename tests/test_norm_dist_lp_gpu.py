@@ -203,3 +203,44 @@ def test_wide_layers_vs_oracle(p, masked):
     assert rel(gx, gx_o) < TOL and rel(gw, gw_o) < TOL
     gx2, _ = run_bwd(g, x, w, y, p, ci, co, weight=False)
     assert rel(gx2, gx_o) < TOL
+
+
+@pytest.mark.parametrize("p", [1.0, 2.0, 3.0, 4.0, 5.0, 6.0, 7.0, 8.0])
+@pytest.mark.parametrize("B,CI,CO", [(33, 130, 9), (64, 128, 40)])
+def test_whole_p_with_nan_and_infinities(p, B, CI, CO):
+    """What the multiply chains make of them: max(NaN, FLT_MIN) = FLT_MIN in the forward; in the backward the oracle's infinities
+    and NaN, and for p = 1 a sign that is -1 where t >= 0 does not hold."""
+    rng = np.random.default_rng(int(p) + CI)
+    x, g = rng.random((B, CI), dtype=np.float32), rng.standard_normal((B, CO)).astype(np.float32)
+    w = rng.standard_normal((CO, CI)).astype(np.float32)
+    y = run_fwd(x, w, p)
+    x[1, 5], x[B - 1, CI - 1], x[7, 0], x[3, 4], x[3, 9], w[CO // 2, 64] = np.nan, np.inf, -np.inf, np.inf, np.nan, np.nan
+    y_o = oracle.norm_dist_forward(x, w, p)
+    y_o = np.where(np.isnan(y_o), np.float64(np.finfo(np.float32).tiny) ** (1 / p), y_o)
+    got, finite = run_fwd(x, w, p), np.isfinite(y_o)
+    assert np.array_equal(got[~finite], y_o[~finite]) and rel_each(got[finite], y_o[finite]) < TOL
+    if p == 1:                                               # a value far below, resp. above, has that sign
+        x_o, w_o = np.where(np.isnan(x), np.float32(-1e30), x), np.where(np.isnan(w), np.float32(1e30), w)
+    else:
+        x_o, w_o = x, w
+    want = oracle.norm_dist_backward(g, x_o, w_o, y, p)
+    for a, b in zip(run_bwd(g, x, w, y, p), want):
+        finite = np.isfinite(b)
+        assert np.array_equal(a[~finite], b[~finite].astype(np.float32), equal_nan=True) and rel(a[finite], b[finite]) < TOL
+    assert p == 1 or not np.isfinite(want[0]).all()
+
+
+@pytest.mark.parametrize("p", [1.0, 2.0, 8.0])
+def test_whole_p_with_one_tile_per_cta(p):
+    """As many tiles of 32 x 128 outputs as a whole number of waves: one launch, which takes the root itself."""
+    from sortnet_b200 import norm_dist_cuda as C
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, CI, CO = 12 * 32, 17, sms * 128                       # twelve tiles per SM: a multiple for 1, 2, 3, 4, 6 CTAs per SM
+    rng = np.random.default_rng(int(p))
+    x = rng.random((B, CI), dtype=np.float32)
+    w = rng.standard_normal((CO, CI)).astype(np.float32)
+    before = C.launch_count
+    y = run_fwd(x, w, p)
+    assert C.launch_count == before + 1
+    for b in (0, 160, B - 32):
+        assert rel_each(y[b:b + 32], oracle.norm_dist_forward(x[b:b + 32], w, p)) < TOL
