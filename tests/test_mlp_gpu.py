@@ -174,3 +174,72 @@ def test_other_threads_run_while_a_pass_is_issued(what):
         thread.join()
     assert ended - began > 0.05, "no call had to wait"
     assert sum(began < s < ended for s in ticks) > 100 * (ended - began)
+
+
+@pytest.mark.parametrize("flat", [False, True])
+def test_training_pass_of_many_sub_batches(flat):
+    """More sub-batches than the mean shift holds the sums of in shared memory (64).  A gradient entry is a sum over up to 2085 rows:
+    in fp32 2084 * 2^-24 = 1.2e-4 of the magnitudes at worst; against 64 bits the layers' atomics are off by 1.8e-5 of the largest
+    entry here, the whole pass by 1.5e-6.  Bar: 4e-5."""
+    a, b = nets(4, 130, (1, 12, 12), 10, 0.8, std=0.02 if flat else 1.0)
+    x = torch.rand(2085, 144, device="cuda")
+    t = torch.randint(0, 10, (2085,), device="cuda")
+    masks = a.draw_masks(2085, x.device)
+    assert a._plan(masks).applies(2085)
+    out = []
+    for net, run in ((a, lambda f: f()), (b, layer_by_layer)):
+        at = x.clone().requires_grad_()
+        loss = run(lambda: net.mixture_loss(at, t, 0.05, masks=masks))
+        grads = run(lambda: torch.autograd.grad(loss, [at, *net.parameters()]))
+        out.append((loss, grads, [l.mean_shift.running_mean for l in net.fc_dist[:-1]]))
+    (loss, grads, means), (loss_b, grads_b, means_b) = out
+    assert abs(float(loss) - float(loss_b)) <= 2e-6 * max(1.0, abs(float(loss_b)))
+    assert all(rel(p.cpu().numpy(), q.cpu().numpy()) < 4e-5 for p, q in zip(grads, grads_b))
+    assert all(torch.equal(p, q) for p, q in zip(means, means_b))
+
+
+@pytest.mark.parametrize("what", ["train", "sort"])
+def test_passes_with_new_weights_follow_one_another(what):
+    """The same for training passes with masks and for sort neurons: the kernels of a pass start while those before them end, and so
+    do a pass and its backward.  Values bit-identical, gradients 1e-5 of the largest entry."""
+    a, b = nets(4, 700, (3, 17, 17), 10, 0.8)
+    x = torch.rand(70, 867, device="cuda")
+    t = torch.randint(0, 10, (70,), device="cuda")
+    masks = a.draw_masks(70, x.device)
+    if what == "sort":
+        a.eval(), b.eval()
+        assert a._plan(None, sort_eval=True).applies(70)
+    else:
+        assert a._plan(masks).applies(70)
+
+    def step(net, to):
+        with torch.no_grad():
+            for l in net.fc_dist:
+                l.weight.mul_(1.01)
+            to.mul_(0.99)
+            if what == "sort":
+                return list(net(to, t, 0.02, up=1.0, down=0.0)), []
+        at = to.detach().requires_grad_()
+        loss = net.mixture_loss(at, t, 0.05, masks=masks)
+        grads = torch.autograd.grad(loss, [at, *net.parameters()])
+        return [l.mean_shift.running_mean.clone() for l in net.fc_dist[:-1]], [loss.detach(), *grads]
+
+    u, v = x.clone(), x.clone()
+    got = [step(a, u) for _ in range(3)]
+    want = [layer_by_layer(lambda: step(b, v)) for _ in range(3)]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        got.append(step(a, u))
+    torch.cuda.current_stream().wait_stream(stream)
+    want.append(layer_by_layer(lambda: step(b, v)))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        last = step(a, u)
+    for _ in range(4):
+        graph.replay()
+        got.append([[o.clone() for o in part] for part in last])
+        want.append(layer_by_layer(lambda: step(b, v)))
+    for (same, near), (same_b, near_b) in zip(got, want):
+        assert all(torch.equal(p, q) for p, q in zip(same, same_b)) and len(same) == len(same_b)
+        assert all(rel(p.cpu().numpy(), q.cpu().numpy()) < 1e-5 for p, q in zip(near, near_b)) and len(near) == len(near_b)
