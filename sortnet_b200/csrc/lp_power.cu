@@ -10,7 +10,8 @@
 // the backward.  Everything is done on pairs of values (sub / mul / fma .f32x2: two operations per issued instruction, at the
 // pipe's full rate), which leaves half of the issue slots for loads and addresses.  B200, 512 x 5120 x 5120, scalar kernels with four
 // lanes per column -> these: p = 8 forward 1.74 -> 1.61 ms, backward 4.46 -> 3.56; p = 2 0.99 -> 0.95, 2.94 -> 2.14; p = 5 backward
-// 3.88 -> 3.3.  The backward keeps the pipe 78 % busy (7 operations per term: 2.6 ms); the reductions into grad_w are 4 % of it.
+// 3.88 -> 3.3.  Cycles in which the pipe is busy at p = 8 (256 x 3840 x 5120): forward 91 %, backward 76 % (7 operations per term: 2.6 ms
+// of the 3.56 above; the reductions into grad_w are 4 % of it).
 #include <float.h>
 #include "launch.h"
 #include "lp_dense.h"
@@ -356,6 +357,10 @@ cudaError_t resident(long long* slots) {
 // end one after the other and leave the last ones alone on their SM (512 x 2048 x 2048 backward: 3.0 of 4 warps per scheduler);
 // several shares per slot keep the slots filled to the end (512 x 5120 x 5120, p = 8: backward 3.81 -> 3.56 ms, forward
 // 1.67 -> 1.61).  Not below `least` units, where loading and storing a share's operands counts, and whole multiples only.
+// Where that leaves one share per slot, p = 8, forward and backward, scalar kernels -> these: 33 x 784 x 500 13.1 -> 10.8 and 21.0 -> 19.7 us, 67 x 1000 x
+// 1000 28.3 -> 21.6 and 46.9 -> 43.0, 200 x 1503 x 777 63 -> 51 and 102 -> 89, 16 x 5120 x 5120 117 -> 113 and 311 -> 268.  Slower: 128 x 5120 x 200 with lists
+// of three quarters, forward 29.7 -> 30.9 (p = 3 26.7 -> 28.8): up to three steps of 128 outputs one after the other instead of two of 256.  Fewer shares, all
+// equal, give 30.3 there and 30.6 instead of 32.5 at 200 x 1503 x 777 with lists, but 55 instead of 51 without.
 unsigned shares(long long units, long long slots, int most, int least) {
     long long per_slot = units / (slots * least);
     per_slot = per_slot < 1 ? 1 : per_slot < most ? per_slot : most;

@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(FT + 64 * R) prune_filter(const PruneArgs a) {
     const int steps = (p.W_CO + R - 1) / R;
     const float nan = __int_as_float(0x7fc00000);
     if (tid < 2 * R) n_found[tid / R][tid % R] = 0;
-    // In a whole-net call the kernel before this one has nothing to do with W, whose first rows are fetched while it ends.
+    // In a whole-net call the kernel before this one has nothing to do with W, whose first rows are fetched while it ends.  Nor may any
+    // kernel that still runs then: what wrote W before the call has ended, as the call's prune_prep is an ordinary launch.
     const bool ahead = p.xt && !p.ci;
     if (!ahead) after_previous();
     if (p.ci && (a.counters[GENERAL] & LIST_TWICE)) return;  // no list will be walked
