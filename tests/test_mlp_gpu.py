@@ -179,8 +179,8 @@ def test_other_threads_run_while_a_pass_is_issued(what):
 @pytest.mark.parametrize("flat", [False, True])
 def test_training_pass_of_many_sub_batches(flat):
     """More sub-batches than the mean shift holds the sums of in shared memory (64).  A gradient entry is a sum over up to 2085 rows:
-    in fp32 2084 * 2^-24 = 1.2e-4 of the magnitudes at worst; against 64 bits the layers' atomics are off by 1.8e-5 of the largest
-    entry here, the whole pass by 1.5e-6.  Bar: 4e-5."""
+    in fp32 2084 * 2^-24 = 1.2e-4 of the magnitudes at worst, which is the bar.  Against 64 bits the layers' atomics are off by up
+    to 2.5e-5 of the largest entry at this size, the whole pass by 1.5e-6."""
     a, b = nets(4, 130, (1, 12, 12), 10, 0.8, std=0.02 if flat else 1.0)
     x = torch.rand(2085, 144, device="cuda")
     t = torch.randint(0, 10, (2085,), device="cuda")
@@ -194,7 +194,7 @@ def test_training_pass_of_many_sub_batches(flat):
         out.append((loss, grads, [l.mean_shift.running_mean for l in net.fc_dist[:-1]]))
     (loss, grads, means), (loss_b, grads_b, means_b) = out
     assert abs(float(loss) - float(loss_b)) <= 2e-6 * max(1.0, abs(float(loss_b)))
-    assert all(rel(p.cpu().numpy(), q.cpu().numpy()) < 4e-5 for p, q in zip(grads, grads_b))
+    assert all(rel(p.cpu().numpy(), q.cpu().numpy()) < 1.2e-4 for p, q in zip(grads, grads_b))
     assert all(torch.equal(p, q) for p, q in zip(means, means_b))
 
 
