@@ -541,7 +541,7 @@ def lp_blocks(job):
             tl = profiled_pass(job, 2, bounds=False)
             _, roof, _, _ = roofline_blocks(tl, job.cfg["width"], ("snb_norm_dist_forward_ws", "snb_norm_dist_backward_ws"))
             roof = {"p": 31.6, "forward": roof["snb_norm_dist_forward_ws"], "backward": roof["snb_norm_dist_backward_ws"],
-                    "note": "evaluated are the terms that can matter; the special-function unit bounds those (75 % busy, "
+                    "note": "evaluated are the terms that can matter; the special-function unit bounds those (82 to 90 % busy, "
                             "profiles/lp_skip_kernels.md).  The forward's time includes the maxima that supply the normaliser"}
     job.model.set_p(INF)
     return out, roof
