@@ -671,7 +671,7 @@ def mlp_train_forward(plan, x, targets, eps, clip, lam, scale):
         for w, _, _, _, kept, _, _ in plan.keep:
             if kept is not None and not check_index_lists(kept, w.size(0), "mask"):
                 raise RuntimeError("mask is not in ascending order")
-    return plan.native.train_forward(x, targets, eps, clip, lam, scale)
+    return plan.native.train_forward(x, targets, float(eps), float(clip), float(lam), float(scale))
 
 
 def mlp_train_backward(plan, B, grad_loss, saved, grad_w, grad_bias, grad_x):

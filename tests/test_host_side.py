@@ -149,6 +149,18 @@ def test_whole_net_calls_refuse_other_targets():
                 call()
 
 
+def test_whole_net_calls_take_numbers_as_float_takes_them():
+    from fractions import Fraction
+    from sortnet_b200 import norm_dist_cuda as C
+    plan = C.MlpPlan([[torch.rand(3, 8), torch.zeros(3), None, 0.0, None, 1, 0.0]])
+    x, t = torch.rand(4, 8), torch.tensor([0, 1, 2, 0])
+    for eps in (0.1, 1, "0.1", Fraction(1, 10), torch.tensor(0.1), torch.tensor([0.1])):
+        with pytest.raises(RuntimeError, match="(?i)cuda"):  # gets as far as the device, which is none
+            C.mlp_train_forward(plan, x, t, eps, 1.0, 0.1, 1.0)
+    with pytest.raises(ValueError, match="one element"):
+        C.mlp_train_forward(plan, x, t, torch.rand(2), 1.0, 0.1, 1.0)
+
+
 def test_whole_net_plan_takes_only_what_the_kernels_read():
     """Anything else is left to the layers, which refuse it or know what to do with it."""
     from sortnet_b200 import norm_dist_cuda as C
