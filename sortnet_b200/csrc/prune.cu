@@ -1215,16 +1215,16 @@ cudaError_t run_sort_walk(const PruneArgs& a, cudaStream_t st) {
 }
 
 // 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves of what
-// fits (four CTAs per SM up to ten values, two above: registers) they take eight.  Up to ten values: 128 x 5120 x 5120 with positions,
-// 640 CTAs of 32: 111 us with 32, 99 with 8; 512 rows for point and box, 2560 CTAs: 211 with 32, 222 with 8.  More, with positions, by 32 / 8
-// outputs: 32 x 2048 x 2048 143 / 68 us at K = 17, 128 x 5120 x 5120 536 / 546, 512 x 5120 x 5120 1332 / 1476; past K = 21 the positions of
-// 32 outputs leave room for one CTA: K = 25 at 200 x 2048 x 3000 701 / 577.
+// fits (four CTAs per SM; two with positions of more than ten values: registers) they take eight.  Ten values: 128 x 5120 x 5120 with positions,
+// 640 CTAs of 32: 111 us with 32, 99 with 8; 512 rows for point and box, 2560 CTAs: 211 with 32, 222 with 8.  More values, by 32 / 8 outputs: alone,
+// K = 17, 512 x 2048 x 2048 (1024 CTAs of 32) 252 / 230; with positions, K = 17, 32 x 2048 x 2048 143 / 68, 128 x 5120 x 5120 536 / 546, 512 x 2048 x 2048
+// 545 / 576, 512 x 5120 x 5120 1332 / 1476; past K = 21 the positions of 32 outputs leave room for one CTA: K = 25, 300 x 2048 x 4000 1069 / 776.
 template <int NX, int KMAX, bool POS>
 cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     int redo = 0;
     cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
     if (e != cudaSuccess) return e;
-    constexpr int FIT = KMAX <= 10 ? 4 : 2;
+    constexpr int FIT = POS && KMAX > 10 ? 2 : 4;
     const bool room = FIT * (sort_walk_smem<NX, POS, 32>(a.p.K) + 1152) <= 228 * 1024;       // an SM's; 1 KB per CTA is taken, and its own few words
     if (!room || (long long)grid.x * grid.y < 3ll * FIT * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
     else e = run_sort_walk<NX, KMAX, POS, 32>(a, st);
