@@ -144,3 +144,36 @@ def test_gradient_all_reduce_refuses_parameters_with_sinks():
     FlatAdamW(model)
     with pytest.raises(ValueError, match="FlatAdamW"):
         GradientAllReduce(model.parameters())
+
+
+@pytest.mark.parametrize("n", [4, 1020, 1024, 1028, 2044, 2048, 2052, 6148])
+@pytest.mark.parametrize("parts", [0, 1, 3])
+def test_adamw_kernels_at_block_edges(n, parts):
+    """The update (parts 0) and its form with partial gradients around the values that a CTA takes (2048 and 1024), against float64; what lies
+    behind the buffers stays as it is."""
+    import ctypes
+    from sortnet_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    w, m, v, out = (torch.randn(n + 8, device="cuda", generator=gen) for _ in range(4))
+    v.abs_()
+    g = [torch.randn(n + 8, device="cuda", generator=gen) for _ in range(max(parts, 1))]
+    before = [t.clone() for t in (w, m, v, out)]
+    lr, b1, b2, eps, wd, step, scale = 0.02, 0.9, 0.99, 1e-6, 0.01, 3, 0.5
+    G = scale * sum(t.double() for t in g)
+    M, V = b1 * m.double() + (1 - b1) * G, b2 * v.double() + (1 - b2) * G * G
+    W = w.double() * (1 - lr * wd) - lr / (1 - b1 ** step) * M / (V.sqrt() / (1 - b2 ** step) ** 0.5 + eps)
+    st = torch.cuda.current_stream().cuda_stream
+    if parts == 0:
+        rc = _lib.load().snb_adamw_step(w.data_ptr(), g[0].data_ptr(), m.data_ptr(), v.data_ptr(), n, lr, b1, b2, eps, wd, step, scale, st)
+        out = w
+    else:
+        ptrs = (ctypes.c_void_p * parts)(*[t.data_ptr() for t in g])
+        rc = _lib.load().snb_adamw_reduce_step(w.data_ptr(), out.data_ptr(), ptrs, parts, m.data_ptr(), v.data_ptr(), n, lr, b1, b2, eps, wd,
+                                               step, scale, st)
+        assert torch.equal(w, before[0])
+    _lib.check(rc, "adamw")
+    # a handful of fp32 operations of 2^-24 each on values of size 1
+    for got, want in ((out, W), (m, M), (v, V)):
+        assert ((got.double() - want)[:n].abs() <= 2e-6 * want[:n].abs().clamp(min=1)).all()
+    for got, old in zip((out, m, v), (before[0] if parts == 0 else before[3], before[1], before[2])):
+        assert torch.equal(got[n:], old[n:])
