@@ -498,6 +498,21 @@ struct TopList {
         if (high) merge<KMAX>();
         else merge<HALF>();
     }
+    // The first eight values, none of them NaN or negative: 19 compare-and-swaps (Batcher's odd-even merge sort).
+    __device__ __forceinline__ void start8(float (&e)[8]) {
+        auto order = [&](int i, int j) {                     // ascending
+            const float lo = fminf(e[i], e[j]);
+            e[j] = fmaxf(e[i], e[j]), e[i] = lo;
+        };
+        order(0, 1), order(2, 3), order(4, 5), order(6, 7);
+        order(0, 2), order(1, 3), order(4, 6), order(5, 7);
+        order(1, 2), order(5, 6);
+        order(0, 4), order(1, 5), order(2, 6), order(3, 7);
+        order(2, 4), order(3, 5);
+        order(1, 2), order(3, 4), order(5, 6);
+#pragma unroll
+        for (int s = 0; s < KMAX; s++) v[s] = s < KMAX - 8 ? 0.f : e[s < KMAX - 8 ? 0 : s - (KMAX - 8)];
+    }
     // v[KMAX - K], as a minimum over an ascending tail: an index that is not a constant would move the list to local memory
     __device__ __forceinline__ float kth(int K) const {
         if (K == KMAX) return v[0];
@@ -533,26 +548,6 @@ struct SortState {
             const float t1 = w - v[NX - 2], t2 = v[NX - 1] - w;
             top[NX - 2].add(fmaxf(-t1, -t2));
             top[NX - 1].add(fmaxf(t1, t2));
-        }
-    }
-    // four columns
-    __device__ __forceinline__ void add4(const float (&v)[4][NX], const float (&w)[4]) {
-        float e[4];
-        if (NX != 2) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) e[k] = fmaxf(fabsf(v[k][0] - w[k]), 0.f);        // NaN -> 0
-            top[0].add4(e[0], e[1], e[2], e[3]);
-        }
-        if (NX >= 2) {
-            float u[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float t1 = w[k] - v[k][NX - 2], t2 = v[k][NX - 1] - w[k];
-                e[k] = max3(-t1, -t2, 0.f);
-                u[k] = max3(t1, t2, 0.f);
-            }
-            top[NX - 2].add4(e[0], e[1], e[2], e[3]);
-            top[NX - 1].add4(u[0], u[1], u[2], u[3]);
         }
     }
     __device__ __forceinline__ float worst(int K) const {
@@ -645,20 +640,20 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
     float* outs[NV];
     if (NX != 2) outs[0] = p.y;
     if (NX >= 2) outs[NV - 2] = p.yl, outs[NV - 1] = p.yu;
-    const int no = n0 + lane;
-    const bool here = lane < SLOTS && no < p.CO, kept = here && (!p.keep || p.keep[(size_t)s * p.CO + no]);
+    const int col = tid % SLOTS, no = n0 + col;
+    const bool here = no < p.CO, kept = here && (!p.keep || p.keep[(size_t)s * p.CO + no]);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int r = warp + 8 * k, b = s * 32 + r;
+    for (int k = 0; k < SLOTS / 8; k++) {
+        const int r = tid / SLOTS + 256 / SLOTS * k, b = s * 32 + r;
         if (b >= p.B || !here) continue;
         const size_t o = (size_t)b * p.CO + no;
 #pragma unroll
         for (int t = 0; t < NV; t++)
-            if (outs[t]) outs[t][o] = shifted<NV>(p, tile[t][r][lane], no);
-        if (NW == 1 && NX == 1 && p.pos) p.pos[o] = kept ? __float_as_int(tile[NV][r][lane]) : (int)SNB_NO_GRAD_ID;
+            if (outs[t]) outs[t][o] = shifted<NV>(p, tile[t][r][col], no);
+        if (NW == 1 && NX == 1 && p.pos) p.pos[o] = kept ? __float_as_int(tile[NV][r][col]) : (int)SNB_NO_GRAD_ID;
         if (NW == 2) {
-            p.posl[o] = __float_as_int(tile[NV][r][lane]);
-            p.posu[o] = __float_as_int(tile[NV + NW - 1][r][lane]);
+            p.posl[o] = __float_as_int(tile[NV][r][col]);
+            p.posu[o] = __float_as_int(tile[NV + NW - 1][r][col]);
         }
     }
     if (p.yt || p.post) {
@@ -672,10 +667,10 @@ __device__ __forceinline__ void emit_tile(const PruneProblem& p, float (*tile)[3
             emit_chain<NV>(p, s, n0 + slot, v, NW > 0 ? __float_as_uint(tile[NW > 0 ? NV : 0][lane][slot]) : 0u, !((again >> slot) & 1u));
         }
     }
-    if (p.part && warp == 0 && here) {
+    if (p.part && tid < SLOTS && here) {
         float sum = 0.f;
         const int rows = min(32, p.B - s * 32);
-        for (int r = 0; r < rows; r++) sum += tile[0][r][lane];
+        for (int r = 0; r < rows; r++) sum += tile[0][r][col];
         p.part[(size_t)s * p.CO + no] = kept ? sum : 0.f;
     }
 }
@@ -742,9 +737,6 @@ __device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, in
 // Bound by the latency of the two dependent loads (list, column) and by the columns' traffic from L2.
 // TRACK keeps, per row, the step that set the maximum; the word is made at the end from the step's columns.  A
 // later step that only equals the maximum (rare) sends the lane over the list once more for the lowest position.
-// Chain form (training: words; evaluation: point and box): written from the registers, so that no warp waits for the CTA's longest list; the last
-// warp adds the row sums up.  512 x 5120 x 5120, as the profiler has it, the end of the filter included: 53.0 -> 49.5 us with words, 50.7 -> 45.1 for point and
-// box, whose seven layers took 496 and now 460 us.
 template <int NX, bool TRACK>
 __global__ void __launch_bounds__(256, NX == 1 && !TRACK ? 6 : NX == 2 && TRACK ? 3 : 4) prune_max(const __grid_constant__ PruneArgs a) {
     constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
@@ -988,118 +980,298 @@ __device__ __noinline__ void ordered_positions(const int2* entries, int cnt, con
         if (k < K) words[k][lane][slot] = __uint_as_float(pl.word[KMAX - 1 - k]);
 }
 
-// The sort neuron over the same lists, one warp per output, lane = row; POS: the K positions too.  Bound by the
-// issue rate of the insertion chains.  With the values known, a second walk collects the columns that reach a row's K-th value, in
-// the order of the list; there are K of them, and the rank of one is the number of larger values in the row's list, of equal
-// values the later column first.  Only where more columns share the K-th value than there is room for does the order of
-// insertion decide (ordered_positions).  Ranking each hit where it is met, in a tile that all lanes wait for: 114 us per
-// 128 x 5120 x 5120 layer against 99.
-template <int NX, int KMAX, bool POS, int SLOTS>
-__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : POS ? 2 : 1) prune_sort(const __grid_constant__ PruneArgs a) {
+// What may enter a row's list waits in shared memory until a row has four of them, and only then are the lists touched: after the first eight entries a row takes
+// one in five, but some row of the warp takes one of nearly every step.  512 x 5120 x 3000, K = 17: values 370 -> 291 us, boxes
+// 800 -> 525; K = 10: values 147 -> 131.  Boxes, and points with boxes, of up to ten values are inserted as they come: three tests and a store per column
+// cost what they save (box 512 x 2048 x 2000 109 us as they come, 121 queued).  With positions of up to ten values the queue is a log of (value,
+// column) that the ranking reads; of more, it lies where the ranking's values come later.
+template <int NX, int KMAX, bool POS>
+struct SortQueue {
+    static constexpr bool LOG = POS && KMAX <= 10;
+    static constexpr bool USED = POS || NX == 1 || KMAX > 10;
+    static constexpr int DEPTH = LOG ? 16 : USED ? 8 : 0;
+    static constexpr int WIDTH = NX == 3 ? 4 : NX;           // floats of an entry: the values of all tensors side by side
+};
+constexpr int SORT_SLOTS = 8;           // outputs of a CTA of prune_sort
+template <int NX, int KMAX, bool POS>
+constexpr int sort_walk_smem(int K) {
+    using Q = SortQueue<NX, KMAX, POS>;
+    const int tile = (NX + (POS ? K : 0)) * 32 * (SORT_SLOTS + 1), found = POS ? 8 * K * 32 : 0;
+    const int queue = POS && !Q::LOG ? 0 : 8 * Q::DEPTH * Q::WIDTH * 32;
+    return (tile + found + queue) * (int)sizeof(float) + (Q::LOG ? 8 * Q::DEPTH * 32 * (int)sizeof(unsigned short) : 0);
+}
+// Without a branch: a row's values of a column go to the end of its queue if one of them beats the least of its list.
+__device__ __forceinline__ void push_above(unsigned& end, const float (&v)[1], const float (&least)[1]) {
+    asm volatile("{\n .reg .pred p;\n setp.gt.f32 p, %1, %2;\n @p st.shared.f32 [%0], %1;\n @p add.u32 %0, %0, 128;\n}"
+                 : "+r"(end) : "f"(v[0]), "f"(least[0]) : "memory");
+}
+__device__ __forceinline__ void push_above(unsigned& end, const float (&v)[2], const float (&least)[2]) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.gt.f32 p, %1, %3;\n setp.gt.or.f32 p, %2, %4, p;\n @p st.shared.v2.f32 [%0], {%1, %2};\n"
+        " @p add.u32 %0, %0, 256;\n}"
+        : "+r"(end) : "f"(v[0]), "f"(v[1]), "f"(least[0]), "f"(least[1]) : "memory");
+}
+__device__ __forceinline__ void push_above(unsigned& end, const float (&v)[3], const float (&least)[3]) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.gt.f32 p, %1, %4;\n setp.gt.or.f32 p, %2, %5, p;\n setp.gt.or.f32 p, %3, %6, p;\n"
+        " @p st.shared.v4.f32 [%0], {%1, %2, %3, %3};\n @p add.u32 %0, %0, 512;\n}"
+        : "+r"(end) : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(least[0]), "f"(least[1]), "f"(least[2]) : "memory");
+}
+// An entry of the queue, which is empty (zero) then.
+__device__ __forceinline__ void take_entry(unsigned at, float (&v)[1]) {
+    asm volatile("ld.shared.f32 %0, [%1];\n st.shared.f32 [%1], %2;" : "=&f"(v[0]) : "r"(at), "f"(0.f) : "memory");
+}
+__device__ __forceinline__ void take_entry(unsigned at, float (&v)[2]) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n st.shared.v2.f32 [%2], {%3, %3};" : "=&f"(v[0]), "=&f"(v[1]) : "r"(at), "f"(0.f) : "memory");
+}
+__device__ __forceinline__ void take_entry(unsigned at, float (&v)[3]) {
+    float none;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n st.shared.v4.f32 [%4], {%5, %5, %5, %5};"
+                 : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(none) : "r"(at), "f"(0.f) : "memory");
+}
+// The same for a value and its column, if the value's size is at least `least`.
+__device__ __forceinline__ void push_pair(unsigned& end, unsigned& column_end, float v, int column, float least) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .f32 d;\n abs.f32 d, %2;\n setp.ge.f32 p, d, %4;\n @p st.shared.f32 [%0], %2;\n @p st.shared.u16 [%1], %3;\n"
+        " @p add.u32 %0, %0, 128;\n @p add.u32 %1, %1, 64;\n}"
+        : "+r"(end), "+r"(column_end) : "f"(v), "h"((unsigned short)column), "f"(least) : "memory");
+}
+// A column that reaches a row's K-th value: its size and its word, as long as there is room.
+__device__ __forceinline__ void push_hit(int& hits, unsigned& at, unsigned& word_at, float v, int column, float least, int K, unsigned word_stride) {
+    asm volatile(
+        "{\n .reg .pred p, r;\n .reg .f32 d;\n .reg .b32 w;\n abs.f32 d, %3;\n setp.ge.f32 p, d, %5;\n setp.gt.and.f32 p, d, 0f00000000, p;\n"
+        " setp.lt.and.s32 r, %0, %6, p;\n mov.b32 w, %3;\n and.b32 w, w, 0x80000000;\n or.b32 w, w, %4;\n"
+        " @r st.shared.f32 [%1], d;\n @r st.shared.b32 [%2], w;\n @r add.u32 %1, %1, 128;\n @r add.u32 %2, %2, %7;\n @p add.s32 %0, %0, 1;\n}"
+        : "+r"(hits), "+r"(at), "+r"(word_at) : "f"(v), "r"(column), "f"(least), "r"(K), "r"(word_stride) : "memory");
+}
+__device__ __forceinline__ float shared_f32(unsigned at) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ int shared_u16(unsigned at) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// The sort neuron over the same lists, one warp per output, lane = row; POS: the K positions too.  Bound by the issue of minima and maxima
+// (half-rate pipe, 73 % busy).  The first eight entries of the list (largest upper bounds) start a row's list, by sorting; the others are inserted four
+// at a time.  In the chain form a warp writes its output and leaves, without a tile.  Point and box of 512 x 5120 x 5120: 287 -> 243 us.
+// POS: with the values known, the columns that reach a row's K-th value are collected, from the first entries and the log of what was
+// queued (from a second walk where the log ran over, and for more than ten values); there are K of them, and the rank of one is the
+// number of larger values in the row's list, of equal values the later column first.  Only where more columns share the K-th value than there is room for does the
+// order of insertion decide (ordered_positions).  128 x 5120 x 5120, K = 10: 107 -> 86 us; always with a second walk, and
+// each word stored for eight of 32 lanes: 107.
+template <int NX, int KMAX, bool POS>
+__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 2) prune_sort(const __grid_constant__ PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
-    constexpr int WALK = STEP;                               // entries per step: all insertion chains of a step are unrolled
-    constexpr int LD = SLOTS + 1;
+    constexpr int LD = SORT_SLOTS + 1;
+    constexpr bool LOG = SortQueue<NX, KMAX, POS>::LOG, QUEUED = SortQueue<NX, KMAX, POS>::USED;
+    constexpr int DEPTH = SortQueue<NX, KMAX, POS>::DEPTH, FLUSH = 3;
+    constexpr int WIDTH = SortQueue<NX, KMAX, POS>::WIDTH;
+    constexpr unsigned ROW = WIDTH * 32 * sizeof(float);     // bytes from one queued entry to the next
     extern __shared__ __align__(16) unsigned char dyn[];
     float(*tile)[32][LD] = reinterpret_cast<float(*)[32][LD]>(dyn);   // [NX] values, then [K] words
     float* const found = reinterpret_cast<float*>(dyn) + (NX + (POS ? a.p.K : 0)) * 32 * LD;  // POS: [8 warps][K][32]
-    __shared__ unsigned failed;
+    __shared__ unsigned failed, arrived;
     const PruneProblem& p = a.p;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int s = blockIdx.y, n0 = blockIdx.x * SLOTS, C = p.W_CI, K = p.K;
+    const int s = blockIdx.y, n0 = blockIdx.x * SORT_SLOTS, C = p.W_CI, K = p.K;
     const bool live = s * 32 + lane < p.B;
     const float* xt = a.xt + (size_t)s * C * NX * 32 + lane;
+    // queue [8 warps][DEPTH][32 rows][WIDTH], columns [8 warps][DEPTH][32]
+    const unsigned found_at = smem_u32(found), queues = POS && !LOG ? found_at : found_at + (POS ? 8 * K * 128 : 0);
+    const unsigned queue = queues + (POS && !LOG ? warp * K * 128 : warp * DEPTH * ROW) + lane * WIDTH * 4;
+    const unsigned columns = queues + 8 * DEPTH * ROW + warp * DEPTH * 64 + lane * 2;
+    const int fill = max(8, (K + 3) / 4 * 4);                // LOG: entries that are not logged
     after_previous();
     let_next();
     if (dense_mode(a)) {
-        if (!POS) dense_prepare<NX>(a, s, n0, 0, SLOTS);     // positions: sort_positions_if reads the rows as they came
+        if (!POS) dense_prepare<NX>(a, s, n0, 0, SORT_SLOTS);     // positions: sort_positions_if reads the rows as they came
         return;
     }
-    if (tid == 0) failed = 0u;
+    const bool chain = !POS && !p.y && !p.yl && !p.yu && !p.part;   // written from here: no warp waits for the others
+    if (tid == 0) failed = arrived = 0u;
     __syncthreads();
-#pragma unroll 1
-    for (int i = 0; i < SLOTS / 8; i++) {
-        const int slot = warp * (SLOTS / 8) + i, j = n0 + slot;
-        if (j >= p.CO) break;
+    const int slot = warp, j = n0 + slot;
+    if (j < p.CO) {
+        if (QUEUED && !LOG) {
+            float none[NX];
+#pragma unroll
+            for (int q = 0; q < DEPTH; q++) take_entry(queue + q * ROW, none);
+        }
         const int cnt = a.cnt[j];
         const float tau = a.tau[j];
         const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
         const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
-        SortState<NX, KMAX> st;
-        st.init();
-        int k = 0;                                           // entries seen
-        float w[WALK], v[WALK][NX];
-        auto fetch = [&](int at, float (&wv)[WALK], float (&xv)[WALK][NX]) {
+        TopList<KMAX> top[NX];
+        float reach[NX];                                     // the K-th value when the list was last touched
+        unsigned end = queue;                                // of what is queued
+        unsigned merged = queue;                             // LOG: of what of it is in the list
+        unsigned column_end = columns;
+        bool lost = false;                                   // LOG: it ran over
 #pragma unroll
-            for (int e = 0; e < WALK / 2; e++) {
-                const int4 two = list[at / 2 + e];
-                wv[2 * e] = __int_as_float(two.y);
-                wv[2 * e + 1] = __int_as_float(two.w);
-#pragma unroll
-                for (int t = 0; t < NX; t++) {
-                    xv[2 * e][t] = xt[((size_t)two.x * NX + t) * 32];
-                    xv[2 * e + 1][t] = xt[((size_t)two.z * NX + t) * 32];
-                }
+        for (int t = 0; t < NX; t++) top[t].init(), reach[t] = 0.f;
+        // Row values of one column: x - w or |x - w|, lower, upper.
+        auto values = [&](const float (&x)[NX], float w, float (&e)[NX]) {
+            if (NX != 2) e[0] = LOG ? x[0] - w : fabsf(x[0] - w);
+            if (NX >= 2) {
+                const float t1 = w - x[NX - 2], t2 = x[NX - 1] - w;
+                e[NX - 2] = fmaxf(-t1, -t2);
+                e[NX - 1] = fmaxf(t1, t2);
             }
         };
-        // With one tensor the walk waits for its loads: the columns of a step come while the step before is entered.
-        if (NX == 1 && cnt > 0) fetch(0, w, v);
-        for (; k < cnt; k += WALK) {
-            if (k >= K) {
-                const float left = ub[k / STEP];
-                if (__all_sync(0xffffffffu, !live || st.worst(K) > left)) break;
+        float w[STEP], v[STEP][NX];
+        int c[STEP];
+        int4 two[STEP / 2];
+        auto entries = [&](int at) {
+#pragma unroll
+            for (int e = 0; e < STEP / 2; e++) two[e] = list[at / 2 + e];
+        };
+        auto fetch = [&]() {
+#pragma unroll
+            for (int e = 0; e < STEP; e++) {
+                c[e] = e % 2 ? two[e / 2].z : two[e / 2].x;
+                w[e] = __int_as_float(e % 2 ? two[e / 2].w : two[e / 2].y);
+#pragma unroll
+                for (int t = 0; t < NX; t++) v[e][t] = xt[((size_t)c[e] * NX + t) * 32];
             }
-            if (NX == 1) {
-                float w0[WALK], v0[WALK][NX];
+        };
+        int k = 0;                                           // entries seen
+        if (cnt > 0) {
+            float left = 0.f;
+            {
+                float first[NX][8];
 #pragma unroll
-                for (int e = 0; e < WALK; e++) {
-                    w0[e] = w[e];
+                for (int h = 0; h < 2; h++) {
+                    entries(4 * h);
+                    fetch();
 #pragma unroll
-                    for (int t = 0; t < NX; t++) v0[e][t] = v[e][t];
+                    for (int q = 0; q < STEP; q++) {
+                        float e[NX];
+                        values(v[q], w[q], e);
+#pragma unroll
+                        for (int t = 0; t < NX; t++) first[t][4 * h + q] = fmaxf(t == 0 && LOG ? fabsf(e[t]) : e[t], 0.f);   // NaN -> 0
+                    }
                 }
-                if (k + WALK < cnt) fetch(k + WALK, w, v);
-                st.add4(v0, w0);
-            } else {
-                fetch(k, w, v);
-                st.add4(v, w);
+#pragma unroll
+                for (int t = 0; t < NX; t++) top[t].start8(first[t]), reach[t] = top[t].kth(K);
+            }
+            k = 8;
+            if (!QUEUED) {
+                for (; k < cnt; k += STEP) {
+                    left = ub[k / STEP];
+                    float least = top[0].kth(K);
+#pragma unroll
+                    for (int t = 1; t < NX; t++) least = fminf(least, top[t].kth(K));
+                    if (__all_sync(0xffffffffu, !live || least > left)) break;
+                    entries(k);
+                    fetch();
+                    float e[STEP][NX];
+#pragma unroll
+                    for (int q = 0; q < STEP; q++) {
+                        values(v[q], w[q], e[q]);
+#pragma unroll
+                        for (int t = 0; t < NX; t++) e[q][t] = fmaxf(e[q][t], 0.f);     // NaN -> 0
+                    }
+#pragma unroll
+                    for (int t = 0; t < NX; t++) top[t].add4(e[0][t], e[1][t], e[2][t], e[3][t]);
+                }
+#pragma unroll
+                for (int t = 0; t < NX; t++) reach[t] = top[t].kth(K);
+            }
+            if (QUEUED && k < cnt) left = ub[k / STEP];
+            if (QUEUED && NX < 3 && k < cnt) entries(k);
+            while (QUEUED) {
+                float least = reach[0];
+#pragma unroll
+                for (int t = 1; t < NX; t++) least = fminf(least, reach[t]);
+                const bool over = k >= cnt || __all_sync(0xffffffffu, !live || least > left);
+                if (!over) {
+                    if (NX == 3) entries(k);                 // registers
+                    fetch();
+                    k += STEP;
+                    if (NX < 3 && k < cnt) entries(k);
+                    if (k < cnt) left = ub[k / STEP];
+#pragma unroll
+                    for (int q = 0; q < STEP; q++) {
+                        float e[NX];
+                        values(v[q], w[q], e);
+                        if (LOG) push_pair(end, column_end, e[0], c[q], reach[0]);
+                        else push_above(end, e, reach);
+                    }
+                }
+                const bool full = LOG && __any_sync(0xffffffffu, end > queue + (DEPTH - 4) * ROW);
+                if (over || full || (LOG && k <= fill) || __any_sync(0xffffffffu, end > merged + FLUSH * ROW)) {
+                    for (unsigned r = merged; __any_sync(0xffffffffu, r < end); r += 4 * ROW) {
+                        float e[4][NX];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (LOG) {
+                                const float queued = shared_f32(r + q * ROW);   // past the end: whatever follows in shared memory
+                                e[q][0] = r + q * ROW < end ? fabsf(queued) : 0.f;
+                            } else {
+                                take_entry(r + q * ROW, e[q]);
+#pragma unroll
+                                for (int t = 0; t < NX; t++) e[q][t] = fmaxf(e[q][t], 0.f);     // NaN -> 0
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < NX; t++) top[t].add4(e[0][t], e[1][t], e[2][t], e[3][t]);
+                    }
+#pragma unroll
+                    for (int t = 0; t < NX; t++) reach[t] = top[t].kth(K);
+                    if (LOG) {
+                        merged = end;
+                        if (k <= fill || (full && !over)) {  // a new log
+                            lost = lost || k > fill;
+                            end = merged = queue;
+                            column_end = columns;
+                        }
+                    } else {
+                        end = queue;
+                    }
+                }
+                if (over) break;
             }
         }
-        const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || st.worst(K) >= tau);
-        if (!good && lane == 0) atomicOr(&failed, 1u << slot);
+        float worst = reach[0];
 #pragma unroll
-        for (int t = 0; t < NX; t++) tile[t][lane][slot] = st.result(t, K, p.q);
+        for (int t = 1; t < NX; t++) worst = fminf(worst, reach[t]);
+        const bool good = cnt >= 0 && __all_sync(0xffffffffu, !live || worst >= tau);
+        if (!good && lane == 0) atomicOr(&failed, 1u << slot);
+        float result[NX];
+#pragma unroll
+        for (int t = 0; t < NX; t++) result[t] = top[t].combine(K, p.q, SNB_EPS);
+        if (chain) emit_chain<NX>(p, s, j, result, 0u, good);
+        else
+#pragma unroll
+            for (int t = 0; t < NX; t++) tile[t][lane][slot] = result[t];
         if (POS && good) {
-            const float least = st.top[0].kth(K);
-            float* mine = found + warp * K * 32 + lane;   // this row's values in the order of the walk; their words in the tile
+            const float least = reach[0];
+            float* mine = found + warp * K * 32 + lane;      // this row's values in the order of the walk; their words in the tile
             int hits = 0;
             bool twice = false;
 #pragma unroll
-            for (int r = 1; r < KMAX; r++)
-                twice = twice || (r > KMAX - K && st.top[0].v[r] > 0.f && st.top[0].v[r] == st.top[0].v[r - 1]);
+            for (int r = 1; r < KMAX; r++) twice = twice || (r > KMAX - K && top[0].v[r] > 0.f && top[0].v[r] == top[0].v[r - 1]);
+            unsigned at = smem_u32(mine), word_at = smem_u32(&tile[NX][lane][slot]);
             // Entries past k have smaller upper bounds than every row's K-th value: none of them is a hit.
-            for (int k2 = 0; k2 < k; k2 += PAD) {
-                int c[PAD];
-                float w[PAD], v[PAD];
+            const int again = LOG && !lost ? min(fill, k) : k;
+            for (int k2 = 0; k2 < again; k2 += STEP) {
+                entries(k2);
+                fetch();
 #pragma unroll
-                for (int e = 0; e < PAD / 2; e++) {
-                    const int4 two = list[k2 / 2 + e];
-                    c[2 * e] = two.x;
-                    w[2 * e] = __int_as_float(two.y);
-                    c[2 * e + 1] = two.z;
-                    w[2 * e + 1] = __int_as_float(two.w);
-                    v[2 * e] = xt[(size_t)two.x * 32];
-                    v[2 * e + 1] = xt[(size_t)two.z * 32];
-                }
+                for (int q = 0; q < STEP; q++) push_hit(hits, at, word_at, v[q][0] - w[q], c[q], least, K, 32 * LD * 4);
+            }
+            if (LOG && !lost) {
+                unsigned cr = columns;
+                for (unsigned r = queue; __any_sync(0xffffffffu, r < end); r += 4 * ROW, cr += 4 * 64)
 #pragma unroll
-                for (int e = 0; e < PAD; e++) {
-                    const float t = v[e] - w[e], d = fabsf(t);
-                    if (d >= least && d > 0.f) {
-                        if (hits < K) {
-                            mine[hits * 32] = d;
-                            tile[NX + hits][lane][slot] = __uint_as_float((uint32_t)c[e] | (t >= 0.f ? 0u : SNB_SIGN_BIT));
-                        }
-                        hits++;
+                    for (int q = 0; q < 4; q++) {
+                        const float queued = shared_f32(r + q * ROW);
+                        push_hit(hits, at, word_at, r + q * ROW < end ? queued : 0.f, shared_u16(cr + q * 64), least, K, 32 * LD * 4);
                     }
-                }
             }
             const bool crowded = hits > K;
             uint32_t word[KMAX];
@@ -1112,7 +1284,7 @@ __global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : POS ? 2 : 1) prune_sort(
                 const float d = i < hits ? mine[i * 32] : -1.f;
                 int rank = 0;
 #pragma unroll
-                for (int r = 0; r < KMAX; r++) rank += st.top[0].v[r] > d;
+                for (int r = 0; r < KMAX; r++) rank += top[0].v[r] > d;
                 if (twice)                                   // of equal values, the later column comes first
 #pragma unroll
                     for (int r = 0; r < KMAX; r++)
@@ -1123,19 +1295,21 @@ __global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : POS ? 2 : 1) prune_sort(
                 ordered_positions<KMAX, LD>(a.cand + (size_t)j * a.lcap, cnt, xt, live ? least : 0.f, K, tile + NX, slot);
         }
     }
-    __syncthreads();
-    emit_tile<NX, NX, 0, SLOTS>(p, tile, s, n0, failed);
-    if (POS) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int r = warp + 8 * k, b = s * 32 + r, n = n0 + lane;
-            if (b >= p.B || n >= p.CO || lane >= SLOTS) continue;
-            for (int t = 0; t < K; t++) {
-                const uint32_t word = __float_as_uint(tile[NX + t][r][lane]);
-                p.pos[((size_t)t * p.B + b) * p.CO + n] = word == EMPTY ? 0 : (int)word;   // fewer than K values above 0
-            }
+    if (chain) {
+        if (last_warp(&arrived) && lane == 0) {
+            const unsigned mask = *(volatile unsigned*)&failed;
+            if (mask) a.fail[atomicAdd(a.counters + FAILED, 1u)] = make_int4(s, n0, (int)mask, 0);
         }
+        return;
     }
+    __syncthreads();
+    emit_tile<NX, NX, 0, SORT_SLOTS>(p, tile, s, n0, failed);
+    const int col = tid % SORT_SLOTS, r = tid / SORT_SLOTS, b = s * 32 + r, n = n0 + col;
+    if (POS && b < p.B && n < p.CO)
+        for (int t = 0; t < K; t++) {
+            const uint32_t word = __float_as_uint(tile[NX + t][r][col]);
+            p.pos[((size_t)t * p.B + b) * p.CO + n] = word == EMPTY ? 0 : (int)word;       // fewer than K values above 0
+        }
     if (tid == 0 && failed) a.fail[atomicAdd(a.counters + FAILED, 1u)] = make_int4(s, n0, (int)failed, 0);
 }
 
@@ -1270,32 +1444,16 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
 }
 
-template <int NX, bool POS, int SLOTS>
-constexpr int sort_walk_smem(int K) {
-    return ((NX + (POS ? K : 0)) * 32 * (SLOTS + 1) + (POS ? 8 * K * 32 : 0)) * (int)sizeof(float);
-}
-template <int NX, int KMAX, bool POS, int SLOTS>
-cudaError_t run_sort_walk(const PruneArgs& a, cudaStream_t st) {
-    const cudaError_t e = allow_smem<prune_sort<NX, KMAX, POS, SLOTS>, sort_walk_smem<NX, POS, SLOTS>(KMAX)>();
-    if (e != cudaSuccess) return e;
-    return launch_next(prune_sort<NX, KMAX, POS, SLOTS>, dim3((a.p.CO + SLOTS - 1) / SLOTS, a.S), 256,
-                       sort_walk_smem<NX, POS, SLOTS>(a.p.K), st, a);
-}
-
-// 32 outputs per CTA write whole lines.  Few CTAs, though, end in a wave that leaves most of the device idle: below three waves of what
-// fits (four CTAs per SM; two with positions of more than ten values: registers) they take eight.  Ten values: 128 x 5120 x 5120 with positions,
-// 640 CTAs of 32: 111 us with 32, 99 with 8; 512 rows for point and box, 2560 CTAs: 211 with 32, 222 with 8.  More values, by 32 / 8 outputs: alone,
-// K = 17, 512 x 2048 x 2048 (1024 CTAs of 32) 252 / 230; with positions, K = 17, 32 x 2048 x 2048 143 / 68, 128 x 5120 x 5120 536 / 546, 512 x 2048 x 2048
-// 545 / 576, 512 x 5120 x 5120 1332 / 1476; past K = 21 the positions of 32 outputs leave room for one CTA: K = 25, 300 x 2048 x 4000 1069 / 776.
+// Eight outputs per CTA, a warp each.  With 32, four one after the other per warp, a few long CTAs end last: 8 / 32 outputs, values of K = 10
+// 512 x 2048 x 2000 79.6 / 89.5 us, 512 x 5120 x 5120 215 / 225, K = 17 485 / 562; boxes of K = 10 119 / 127 and 333 / 332, K = 17 321 / 339 and
+// 872 / 908, chained points and boxes of K = 10 243 / 249; positions of K = 11 64 x 1024 x 2048 53 / 88, 512 x 5120 x 5120 842 / 852.
 template <int NX, int KMAX, bool POS>
-cudaError_t run_sort(const PruneArgs& a, dim3 grid, cudaStream_t st) {
+cudaError_t run_sort(const PruneArgs& a, cudaStream_t st) {
     int redo = 0;
     cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
+    if (e == cudaSuccess) e = allow_smem<prune_sort<NX, KMAX, POS>, sort_walk_smem<NX, KMAX, POS>(KMAX)>();
     if (e != cudaSuccess) return e;
-    constexpr int FIT = POS && KMAX > 10 ? 2 : 4;
-    const bool room = FIT * (sort_walk_smem<NX, POS, 32>(a.p.K) + 1152) <= 228 * 1024;       // an SM's; 1 KB per CTA is taken, and its own few words
-    if (!room || (long long)grid.x * grid.y < 3ll * FIT * sm_count()) e = run_sort_walk<NX, KMAX, POS, 8>(a, st);
-    else e = run_sort_walk<NX, KMAX, POS, 32>(a, st);
+    e = launch_next(prune_sort<NX, KMAX, POS>, dim3((a.p.CO + SORT_SLOTS - 1) / SORT_SLOTS, a.S), 256, sort_walk_smem<NX, KMAX, POS>(a.p.K), st, a);
     if (e != cudaSuccess) return e;
     if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;
     return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
@@ -1349,11 +1507,11 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
         return run_max<3, false>(a, grid, st);
     }
     if (p.K <= 10) {
-        if (a.NX == 1) return p.pos ? run_sort<1, 10, true>(a, grid, st) : run_sort<1, 10, false>(a, grid, st);
-        return a.NX == 2 ? run_sort<2, 10, false>(a, grid, st) : run_sort<3, 10, false>(a, grid, st);
+        if (a.NX == 1) return p.pos ? run_sort<1, 10, true>(a, st) : run_sort<1, 10, false>(a, st);
+        return a.NX == 2 ? run_sort<2, 10, false>(a, st) : run_sort<3, 10, false>(a, st);
     }
-    if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, grid, st) : run_sort<1, 25, false>(a, grid, st);
-    return a.NX == 2 ? run_sort<2, 25, false>(a, grid, st) : run_sort<3, 25, false>(a, grid, st);
+    if (a.NX == 1) return p.pos ? run_sort<1, 25, true>(a, st) : run_sort<1, 25, false>(a, st);
+    return a.NX == 2 ? run_sort<2, 25, false>(a, st) : run_sort<3, 25, false>(a, st);
 }
 
 }  // namespace snb

@@ -207,6 +207,47 @@ def test_sort_neuron_of_many_values_around_the_split_of_outputs(off, kind, K):
     assert torch.equal(pos, want) and torch.equal(y, v) and rel(host(y), host(z)) < 2e-6
 
 
+@pytest.mark.parametrize("K", [2, 8, 9, 10, 11, 25])
+@pytest.mark.parametrize("kind", ["rising", "few", "few and NaN"])
+def test_sort_neuron_queues(K, kind):
+    """Rows whose values rise along the list, so that every entry enters and is merged in its turn (the log of positions runs over), and
+    lists around the entries that start a row's list (8) and a step (4).  Values, positions and bounds against the dense kernels."""
+    from sortnet_b200 import _lib, norm_dist_cuda as C
+    B, CI, CO, q = 70, 140, 1100, 0.8
+    rng = np.random.default_rng(K)
+    x, w = rng.random((B, CI), dtype=np.float32), rng.standard_normal((CO, CI)).astype(np.float32)
+    if kind == "rising":
+        # every column spans [0, 1]; its largest bound is 4 - c / 1000, while rows 2, 34 and 66 see 3 + c / 1000
+        x[:] = 0.0
+        x[1::32] = 1.0
+        x[2::32] = 0.002 * np.arange(CI)
+        w[:] = -3.0 + 0.001 * np.arange(CI) + 1e-5 * rng.random((CO, CI))
+    else:
+        # a handful of columns with far weights, K and more of them in turn
+        x *= 0.01
+        w *= 0.01
+        for j in range(CO):
+            w[j, rng.permutation(CI)[:K + j % 7]] += 5.0
+        if kind == "few and NaN":
+            x[40, 3], w[5, 100], x[7] = np.nan, np.nan, np.nan
+    X, W = col3(x.astype(np.float32)), dev(w.astype(np.float32))
+    st = torch.cuda.current_stream().cuda_stream
+    y, v, z = (torch.empty(B, CO, 1, device="cuda") for _ in range(3))
+    pos, want = (torch.empty(K, B, CO, 1, device="cuda", dtype=torch.int32) for _ in range(2))
+    C.sort_neuron_forward(X, W, y, pos, 1, q, K)
+    C.sort_neuron_forward_nograd(X, W, v, 1, q, K)
+    _lib.check(_lib.load().snb_sort_neuron_forward(X.data_ptr(), W.data_ptr(), B, CO, CI, 1, 1, z.data_ptr(), want.data_ptr(), q, K, st), "sort")
+    assert torch.equal(pos, want) and torch.equal(y, v) and torch.allclose(y, z, rtol=2e-6, atol=0)
+    if "NaN" in kind:
+        return                                              # dense bounds move their lists on NaN
+    XL, XU = X - 0.03, X + 0.03
+    yl, yu, zl, zu = (torch.empty_like(y) for _ in range(4))
+    C.bound_sort_neuron_forward(XL, XU, W, yl, yu, 1, q, K)
+    _lib.check(_lib.load().snb_bound_sort_neuron_forward(XL.data_ptr(), XU.data_ptr(), W.data_ptr(), B, CO, CI, 1, 1, zl.data_ptr(), zu.data_ptr(),
+                                                         q, K, st), "bounds")
+    assert torch.allclose(yl, zl, rtol=2e-6, atol=0) and torch.allclose(yu, zu, rtol=2e-6, atol=0)
+
+
 def test_positions_of_25_values_where_some_lists_overflow():
     """Outputs that the walk leaves to prune_redo, among others that it does not: the positions of all are the dense kernel's."""
     from sortnet_b200 import _lib, norm_dist_cuda as C
