@@ -590,13 +590,32 @@ struct Area {
     }
 };
 
-size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a) {
+// The maxima by the pruned evaluation (prune.cuh), which reads W once for all sub-batches, where skip_maxima does so for each: it pays from so many
+// weights on that it need not read again.  Forward at p = 1000, skip_maxima / pruned: 512 x 5120 x 5120 876 / 476 us, 512 x 784 x 5120 198 / 144,
+// 64 x 5120 x 5120 144 / 113, 512 x 784 x 1000 (12 M weights not read again) 56.5 / 52.2, 67 x 5120 x 1000 (10 M) 53.9 / 54.1, 67 x 784 x 2000
+// (3 M) 33.7 / 42.0.  With lists of three quarters the pruned form reads all of W and has more to prepare: 512 x 5120 x 5120 (221 M) 516 / 342,
+// 512 x 784 x 5120 (34 M) 131.6 / 127.4, 64 x 5120 x 5120 (15 M) 101 / 117.  One sub-batch gains nothing: 24 x 5120 x 5120 84 / 90.
+PruneProblem maxima_problem(const LpProblem& q, float* mt) {
+    PruneProblem m;
+    m.x = q.x, m.w = q.w, m.ci = q.ci, m.co = q.co;
+    m.B = q.B, m.CO = q.CO, m.CI = q.CI, m.W_CO = q.W_CO, m.W_CI = q.W_CI;
+    m.yt = mt;
+    return m;
+}
+bool maxima_pruned(const LpProblem& q) {
+    const long long again = (long long)((q.B + 31) / 32 - 1) * q.CO * q.CI;
+    return again >= (q.ci ? 32ll << 20 : 10ll << 20) && prune_applies(maxima_problem(q, nullptr));
+}
+
+size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, char** prune = nullptr) {
     const size_t S = (q.B + 31) / 32;
     Area at{base};
     float* xt = at.take<float>(S * q.CI * 32);
     float2* range = at.take<float2>(S * q.CI);
     float* mt = at.take<float>(S * q.CO * 32);
     float* sum = at.take<float>(S * q.CO * 32);
+    char* scratch = at.take<char>(maxima_pruned(q) ? prune_workspace_bytes(maxima_problem(q, mt)) : 0);
+    if (prune) *prune = scratch;
     if (a) {
         a->w = q.w, a->ci = q.ci, a->co = q.co, a->xt = xt, a->range = range, a->mt = mt, a->sum = sum;
         a->sl = slabs((int)S, q.CI, q.CO, 128, 12);
@@ -635,13 +654,17 @@ size_t lp_skip_backward_bytes(const LpProblem& q) { return backward_applies(q) ?
 
 cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, cudaStream_t st) {
     ForwardArgs a{};
-    forward_layout(q, static_cast<char*>(ws), &a);
+    char* prune = nullptr;
+    forward_layout(q, static_cast<char*>(ws), &a, &prune);
     const int S = (q.B + 31) / 32, smem = slab_bytes(a.sl, 128, 12);
+    const bool pruned = maxima_pruned(q);
     cudaError_t e = cudaSuccess;
     // maxima and sums lie side by side
-    if (a.sl.chunks > 1 && (e = cudaMemsetAsync(a.mt, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - (char*)a.mt, st)) != cudaSuccess) return e;
+    char* const zeroed = reinterpret_cast<char*>(pruned ? a.sum : a.mt);
+    if (a.sl.chunks > 1 && (e = cudaMemsetAsync(zeroed, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - zeroed, st)) != cudaSuccess) return e;
+    if (pruned && (e = prune_forward(maxima_problem(q, a.mt), prune, st)) != cudaSuccess) return e;
     skip_columns<<<dim3((q.CI + 63) / 64, S), 256, 0, st>>>(q.x, q.B, q.CI, const_cast<float*>(a.xt), const_cast<float2*>(a.range));
-    if ((e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
+    if (!pruned && (e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
     if ((e = launch<skip_forward>(a, smem, st)) != cudaSuccess) return e;
     skip_finish<<<dim3((q.CO + 63) / 64, S), 256, 0, st>>>(a.sum, a.mt, q.B, q.CO, q.p, y);
     return launched(2);

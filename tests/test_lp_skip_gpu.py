@@ -92,6 +92,33 @@ def test_against_float64(B, CI, CO, keep, p):
     assert near(gx2, gx) < 1e-6                                     # sums in another order
 
 
+# two, ten and three sub-batches on both sides of the 10 M weights (32 M with lists) that are not read again
+@pytest.mark.parametrize("B,CI,CO,keep", [(33, 3260, 3220, 1.0), (33, 3200, 3220, 1.0), (290, 1103, 1100, 1.0), (96, 5120, 4600, 0.9), (96, 4700, 4200, 0.9)])
+@pytest.mark.parametrize("kind", ["plain", "no numbers", "wide"])
+@pytest.mark.parametrize("p", [31.6, 1000.0])
+def test_maxima_of_many_sub_batches(B, CI, CO, keep, kind, p):
+    """The forward where the maxima come from the pruned evaluation: values of the first, a middle and the last row against float64."""
+    x, w, g, ci, co = inputs(B, CI, CO, keep, B + CI, spread=30.0 if kind == "wide" else 1.0)
+    if kind == "wide":
+        w *= 0.01                                                   # no list holds the columns that matter
+    if kind == "no numbers":
+        x[1, 17], x[B - 2, 5], w[7, 100], w[8, 101] = float("nan"), float("inf"), float("nan"), -float("inf")
+    y, _, _ = calls(x, w, g, ci, co, p)
+    dense, _, _ = calls(x, w, g, ci, co, p, sparse=False)
+    # from p = 48 on the dense kernel passes over whole batches of terms, NaN among them
+    assert torch.equal(dense.isfinite(), y.isfinite()) if p < 48 else bool((dense.isfinite() | ~y.isfinite()).all())
+    ok = dense.isfinite() & y.isfinite()
+    assert torch.allclose(dense[ok], y[ok], rtol=TOL, atol=0)
+    for b in (0, B // 2, B - 1):
+        cols = ci[b // 32].long() if ci is not None else slice(None)
+        outs = co[b // 32].long() if co is not None else slice(None)
+        a = (x[b][None, :] - w[outs][:, cols]).abs().double()
+        m = a.amax(1).clamp(min=1e-10)
+        y_o = m * ((a / m[:, None]).pow(p).sum(1) + (1e-10 / m).pow(p)).pow(1 / p)
+        ok = y_o.isfinite() & y[b].isfinite()
+        assert float(((y[b].double() - y_o).abs() / y_o)[ok].max()) < TOL
+
+
 def test_data_that_cannot_be_skipped():
     """Inputs spread far wider than the weights: nearly every pair passes the test."""
     x, w, g, ci, co = inputs(64, 1400, 800, 1.0, 5, spread=50.0)
