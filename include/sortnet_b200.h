@@ -323,6 +323,16 @@ int snb_mean_shift_stats(const float* x, const int* index, int B, int C, int C_f
 int snb_mean_shift_apply(const float* x, const float* mean, const int* index, int B, int C,
                          float* y, void* stream);
 
+/* The mean shift over rows and positions: x [B, G kept, hw] with lists index [S, G, kept] of within-group channels, ascending
+ * (NULL: all channels, then channels == G kept).  mean [channels] (0 for never-kept ones), y = x minus its channel's mean,
+ * optional running mean as above.  The sums alone, and x plus its channel's entry of v (a bias, and the bias gradient).
+ * Replace core/models/bound_basic_module.py:123-157 and core/models/norm_dist.py:102-103 for [B, C, HW]. */
+int snb_plane_shift(const float* x, const int* index, int B, int G, int kept, int hw, int channels, float* mean,
+                    float* running_mean, float momentum, float* y, void* stream);
+int snb_plane_sum(const float* x, const int* index, int B, int G, int kept, int hw, int channels, float* sum, void* stream);
+int snb_plane_add(const float* x, const int* index, int B, int G, int kept, int hw, int channels, const float* v, float* y,
+                  void* stream);
+
 /* ---- mask sampling ---------------------------------------------------------------------------- */
 
 /* out [lists, count] int32: for each list an independent, uniformly random subset of

@@ -61,6 +61,9 @@ SIGNATURES = {
     "snb_certified_fraction": [_P, _P, _P, _I, _I, _P, _P, _P],
     "snb_unfold": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "snb_fold": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "snb_plane_shift": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _F, _P, _P],
+    "snb_plane_sum": [_P, _P, _I, _I, _I, _I, _I, _P, _P],
+    "snb_plane_add": [_P, _P, _I, _I, _I, _I, _I, _P, _P, _P],
     "snb_plane_index": [_P, _I, _I, _I, _I, _I, _P, _P],
     # the three *_bytes return size_t
     "snb_mlp_applies": [_P, _I, _I],

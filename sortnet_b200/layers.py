@@ -106,34 +106,59 @@ class _UnfoldF(torch.autograd.Function):
 
 class _MeanShiftPlaneF(torch.autograd.Function):
     """The centring of _MeanShiftTrainF for x [B, C, HW] and grouped index lists
-    (core/models/bound_basic_module.py:125-139: the mean runs over rows and positions).  The
-    statistics kernel sees the (channel, position) plane as one long channel axis; every
-    position of a channel has the same row count, so the channel mean is the plain average of
-    its per-position means."""
+    (core/models/bound_basic_module.py:125-139: the mean runs over rows and positions), one launch per direction."""
 
     @staticmethod
-    def forward(ctx, x, plane_index, channels):
-        B, hw = x.size(0), x.size(-1)
-        flat = x.contiguous().view(B, -1, 1)
-        per_pos = torch.empty(channels * hw, device=x.device, dtype=torch.float32)
-        _C.mean_shift_stats(flat, plane_index, per_pos, None, 0.0)
-        mean = per_pos.view(channels, hw).mean(dim=1)
-        y = torch.empty_like(flat)
-        _C.mean_shift_apply(flat, _per_position(mean, hw), plane_index, y)
-        ctx.plane_index, ctx.channels = plane_index, channels
+    def forward(ctx, x, index, running_mean, momentum):
+        x = x.contiguous()
+        mean, y = torch.empty_like(running_mean), torch.empty_like(x)
+        _C.plane_shift(x, index, running_mean.numel(), mean, y, running_mean, momentum)
+        ctx.index, ctx.channels = index, running_mean.numel()
         ctx.mark_non_differentiable(mean)
-        return y.view(x.shape), mean
+        return y, mean
 
     @staticmethod
     def backward(ctx, grad_y, _grad_mean):
-        B, hw = grad_y.size(0), grad_y.size(-1)
-        flat = grad_y.contiguous().view(B, -1, 1)
-        per_pos = torch.empty(ctx.channels * hw, device=grad_y.device, dtype=torch.float32)
-        _C.mean_shift_stats(flat, ctx.plane_index, per_pos, None, 0.0)
-        gmean = per_pos.view(ctx.channels, hw).mean(dim=1)
-        grad_x = torch.empty_like(flat)
-        _C.mean_shift_apply(flat, _per_position(gmean, hw), ctx.plane_index, grad_x)
-        return grad_x.view(grad_y.shape), None, None
+        grad_y = grad_y.contiguous()
+        gmean, grad_x = torch.empty(ctx.channels, device=grad_y.device, dtype=torch.float32), torch.empty_like(grad_y)
+        _C.plane_shift(grad_y, ctx.index, ctx.channels, gmean, grad_x)
+        return grad_x, None, None, None
+
+
+class _PlaneAddF(torch.autograd.Function):
+    """x [B, C, HW] plus the entry of vec [channels] of every channel."""
+
+    @staticmethod
+    def forward(ctx, x, vec, index):
+        ctx.index, ctx.channels = index, vec.numel()
+        return _C.plane_add(x.contiguous(), index, vec.contiguous())
+
+    @staticmethod
+    def backward(ctx, grad):
+        need_x, need_vec = ctx.needs_input_grad[:2]
+        return grad if need_x else None, _PlaneSumF.apply(grad, ctx.index, ctx.channels) if need_vec else None, None
+
+
+class _PlaneSumF(torch.autograd.Function):
+    """The transpose of adding vec: sums per channel."""
+
+    @staticmethod
+    def forward(ctx, x, index, channels):
+        ctx.index, ctx.shape = index, x.shape
+        return _C.plane_sum(x.contiguous(), index, channels)
+
+    @staticmethod
+    def backward(ctx, grad):
+        zeros = torch.zeros(ctx.shape, device=grad.device, dtype=grad.dtype)
+        return _PlaneAddF.apply(zeros, grad, ctx.index), None, None
+
+
+def _add_per_channel(z, vec, index):
+    """z [B, C, HW] plus vec [channels], gathered by the kept channels of each row's sub-batch."""
+    plain = z.is_cuda and z.dtype == vec.dtype == torch.float32 and z.device == vec.device and not ops.tracing() and not ops.forward_mode()
+    if plain and (index is None or (index.dtype == torch.int32 and index.is_contiguous())) and torch._C._functorch.peek_interpreter_stack() is None:
+        return _PlaneAddF.apply(z, vec, index)
+    return z + MeanShiftDropout._gathered(vec, index, z.size(0)).unsqueeze(-1)
 
 
 class _MeanShiftTrainF(torch.autograd.Function):
@@ -183,13 +208,10 @@ class MeanShiftDropout(nn.Module):
         some = x if x is not None else lower
         hw = some.size(-1)
         plane = hw != 1 or (index is not None and index.size(1) != 1)
-        kernel_index = _plane_index(index, self.out_channels, hw) if plane else index
         if self.training:
             assert x is not None, "training needs the activations"
             if plane:
-                x, mean = _MeanShiftPlaneF.apply(x, kernel_index, self.out_channels)
-                with torch.no_grad():
-                    self.running_mean.mul_(1 - self.momentum).add_(mean, alpha=self.momentum)
+                x, mean = _MeanShiftPlaneF.apply(x, index, self.running_mean, self.momentum)
             else:
                 x, mean = _MeanShiftTrainF.apply(x, index, self.running_mean, self.momentum)
             if self.bias is not None:
@@ -199,8 +221,8 @@ class MeanShiftDropout(nn.Module):
         else:
             mean = self.running_mean if self.bias is None else self.running_mean - self.bias.detach()
             x_done, todo = None, (x, lower, upper)
-        if plane:
-            mean = _per_position(mean, hw)
+        if plane and any(z is not None for z in todo):
+            mean, kernel_index = _per_position(mean, hw), _plane_index(index, self.out_channels, hw)
         outs = []
         for z in todo:
             if z is None:
@@ -382,8 +404,7 @@ class NormDistConv(nn.Module):
         if self.mean_shift is not None:
             x3, l3, u3 = self.mean_shift(x3, l3, u3, index=mask_out)
         if self.bias is not None:
-            b = MeanShiftDropout._gathered(self.bias, mask_out, some.size(0)).unsqueeze(-1)
-            x3, l3, u3 = (None if z is None else z + b for z in (x3, l3, u3))
+            x3, l3, u3 = (None if z is None else _add_per_channel(z, self.bias, mask_out) for z in (x3, l3, u3))
         return tuple(None if z is None else z.view(z.size(0), -1, h, w) for z in (x3, l3, u3))
 
     def extra_repr(self):

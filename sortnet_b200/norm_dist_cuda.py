@@ -476,6 +476,54 @@ def mean_shift_apply(x, mean, index, y):
           _ptr(x), _ptr(mean), _ptr(index), B, C, _ptr(y))
 
 
+def _plane(x, index, channels):
+    """(B, G, kept, hw) of x [B, G kept, hw] with lists index [S, G, kept] (None: all channels)."""
+    _check(x, "x")
+    if x.dim() != 3:
+        raise RuntimeError("x must have shape [B, C, HW]")
+    B, C, hw = x.shape
+    G, kept = (1, C) if index is None else (index.size(1), index.size(2))
+    if index is not None:
+        _check(index, "index", torch.int32)
+        if tuple(index.shape) != ((B + _SUB_BATCH - 1) // _SUB_BATCH, G, C // max(G, 1)) or G * kept != C:
+            raise RuntimeError("index must have shape [sub-batches, groups, C / groups]")
+    elif C != channels:
+        raise RuntimeError("x must have all channels when there is no index")
+    return B, G, kept, hw
+
+
+def plane_shift(x, index, channels, mean, y, running_mean=None, momentum=0.1):
+    """y = x minus the mean of its channel over the rows that kept it and all positions, mean [channels] (output),
+    optional running-mean update.  x, y [B, C, HW]; index [S, G, C / G] or None."""
+    B, G, kept, hw = _plane(x, index, channels)
+    _check(mean, "mean"); _check(y, "y")
+    if running_mean is not None:
+        _check(running_mean, "running_mean")
+    if y.shape != x.shape or mean.numel() != channels or (running_mean is not None and running_mean.numel() != channels):
+        raise RuntimeError("shape mismatch")
+    dev = _same_device(x, index, mean, y, running_mean)
+    _call(dev, x, "snb_plane_shift", (B, channels), x.data_ptr(), _ptr(index), B, G, kept, hw, channels, mean.data_ptr(),
+          _ptr(running_mean), float(momentum), y.data_ptr())
+
+
+def plane_sum(x, index, channels):
+    """Sums of x [B, C, HW] per channel -> [channels]."""
+    B, G, kept, hw = _plane(x, index, channels)
+    out = torch.empty(channels, device=x.device, dtype=torch.float32)
+    _call(_same_device(x, index), x, "snb_plane_sum", (B, channels), x.data_ptr(), _ptr(index), B, G, kept, hw, channels, out.data_ptr())
+    return out
+
+
+def plane_add(x, index, v):
+    """x [B, C, HW] plus the entry of v [channels] of every channel."""
+    B, G, kept, hw = _plane(x, index, v.numel())
+    _check(v, "v")
+    y = torch.empty_like(x)
+    _call(_same_device(x, index, v), x, "snb_plane_add", (B, v.numel()), x.data_ptr(), _ptr(index), B, G, kept, hw, v.numel(), v.data_ptr(),
+          y.data_ptr())
+    return y
+
+
 def sample_mask_into(out, channels, seed):
     """out [S, G, count] int32 CUDA tensor -> S * G independent sorted subsets of range(channels)."""
     _check(out, "out", torch.int32)

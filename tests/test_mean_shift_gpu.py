@@ -53,3 +53,31 @@ def test_in_place_apply_and_eval():
     X = col3(x)
     C.mean_shift_apply(X, dev(rm), None, X)
     assert rel(host(X), x - rm[None]) < 1e-6
+
+
+@pytest.mark.parametrize("B,G,C,kept,hw", [(1, 1, 8, 8, 1), (33, 1, 9, 5, 4), (70, 3, 30, 7, 9), (64, 2, 1000, 400, 1), (1100, 1, 40, 30, 2),
+                                           (31, 1, 7, 7, 33)])
+def test_plane_shift(B, G, C, kept, hw):
+    """Mean shift, per-channel add and per-channel sums over rows and positions against float64."""
+    from sortnet_b200 import norm_dist_cuda as NC
+    gen = torch.Generator(device="cuda").manual_seed(B + hw)
+    S, per, masked = (B + 31) // 32, C // G, kept * G < C
+    index = None
+    if masked:
+        index = torch.rand(S, G, per, device="cuda", generator=gen).argsort(-1)[..., :kept].sort(-1)[0].int().contiguous()
+        glob = (index.long() + torch.arange(G, device="cuda").view(1, G, 1) * per).reshape(S, -1)
+    else:
+        kept, glob = per, torch.arange(C, device="cuda").expand(S, C)
+    chan = glob[torch.arange(B, device="cuda") // 32]
+    x = torch.randn(B, G * kept, hw, device="cuda", generator=gen) + 3
+    sums = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), x.double().sum(-1).reshape(-1))
+    rows = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), torch.full((chan.numel(),), float(hw), dtype=torch.float64, device="cuda"))
+    mean_o = torch.where(rows > 0, sums / rows.clamp(min=1), 0.0)
+    mean, y, run = torch.empty(C, device="cuda"), torch.empty_like(x), torch.ones(C, device="cuda")
+    NC.plane_shift(x, index, C, mean, y, run, 0.1)
+    # sums of up to 35 200 values of size 3 in 32 lanes: 1100 roundings of 2^-24 of the sum at most, far fewer in earnest
+    assert (mean.double() - mean_o).abs().max() <= 1e-5 and torch.equal(y, x - mean[chan].unsqueeze(-1))
+    assert (run.double() - (0.9 + 0.1 * mean_o)).abs().max() <= 2e-6
+    assert ((NC.plane_sum(x, index, C).double() - sums).abs() <= 1e-5 * sums.abs().clamp(min=1)).all()
+    v = torch.randn(C, device="cuda", generator=gen)
+    assert torch.equal(NC.plane_add(x, index, v), x + v[chan].unsqueeze(-1))
