@@ -3,7 +3,8 @@
 // steps at about four times the host time (a small layer's forward, backward and bounds: 310 us per pass against
 // kernels of 30 us); they stay for what needs Python: gradient sinks, the profile, index-list validation.
 // Also the layer table, the mask lists and the calls of a whole-net pass (a training pass of six layers on small images issued in 650 us
-// through ctypes, 490 us here, against 360 us of kernels).
+// through ctypes, 490 us here, against 360 us of kernels), and what a convolution does around its distance (patches, mean shift and
+// bias over positions: a forward and backward of two convolutions issued in 740 us by Python functions, 503 here).
 //
 // The library is reached through function pointers (init), so this module links against PyTorch only.
 
@@ -55,6 +56,11 @@ struct Api {
     decltype(&snb_mlp_backward_scratch_bytes) mlp_backward_bytes;
     decltype(&snb_mlp_train_forward) mlp_forward;
     decltype(&snb_mlp_train_backward) mlp_backward;
+    decltype(&snb_unfold) unfold;
+    decltype(&snb_fold) fold;
+    decltype(&snb_plane_shift) plane_shift;
+    decltype(&snb_plane_sum) plane_sum;
+    decltype(&snb_plane_add) plane_add;
     decltype(&snb_status_string) status_string;
     decltype(&snb_last_cuda_error) last_cuda_error;
 } api;
@@ -99,6 +105,11 @@ void init(const std::string& path, py::object error_class) {
     get(api.mlp_backward_bytes, "snb_mlp_backward_scratch_bytes");
     get(api.mlp_forward, "snb_mlp_train_forward");
     get(api.mlp_backward, "snb_mlp_train_backward");
+    get(api.unfold, "snb_unfold");
+    get(api.fold, "snb_fold");
+    get(api.plane_shift, "snb_plane_shift");
+    get(api.plane_sum, "snb_plane_sum");
+    get(api.plane_add, "snb_plane_add");
     get(api.status_string, "snb_status_string");
     get(api.last_cuda_error, "snb_last_cuda_error");
 }
@@ -393,6 +404,142 @@ std::tuple<Tensor, Tensor> bound_sort_neuron(const Tensor& xl, const Tensor& xu,
     return {yl, yu};
 }
 
+// ---- around the operators of a convolution -----------------------------------------------------------
+struct UnfoldFn : public torch::autograd::Function<UnfoldFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& given, int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t dil) {
+        const Tensor x = given.contiguous();
+        check(x, "x");
+        TORCH_CHECK(x.dim() == 4, "x must have shape [B, C, H, W]");
+        const int64_t B = x.size(0), C = x.size(1), H = x.size(2), W = x.size(3);
+        auto places = [&](int64_t n, int64_t k) {            // rounded down, as Python divides
+            const int64_t room = n + 2 * pad - dil * (k - 1) - 1;
+            TORCH_CHECK(stride > 0, "stride must be positive");
+            return std::max<int64_t>(room < 0 ? 0 : room / stride + 1, 0);
+        };
+        Call call(x);
+        Tensor out = at::empty({B, C * kh * kw, places(H, kh) * places(W, kw)}, x.options());
+        done(api.unfold(x.data_ptr<float>(), B, C, H, W, kh, kw, stride, pad, dil, out.data_ptr<float>(), call.stream), "unfold");
+        ctx->saved_data["args"] = std::vector<int64_t>{B, C, H, W, kh, kw, stride, pad, dil};
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(6);
+        if (!grads[0].defined() || !ctx->needs_input_grad(0)) return out;
+        const auto a = ctx->saved_data["args"].toIntVector();
+        const Tensor g = grads[0].contiguous();
+        check(g, "g");
+        Call call(g);
+        out[0] = at::empty({a[0], a[1], a[2], a[3]}, g.options());
+        done(api.fold(g.data_ptr<float>(), a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], out[0].data_ptr<float>(), call.stream),
+             "fold");
+        return out;
+    }
+};
+
+// x [B, G kept, HW] with lists [S, G, kept]: (groups, kept channels per group).
+std::pair<int, int> check_plane(const Tensor& x, const optional<Tensor>& index, int64_t channels) {
+    check(x, "x");
+    TORCH_CHECK(x.dim() == 3, "x must have shape [B, C, HW]");
+    if (!index.has_value()) {
+        TORCH_CHECK(x.size(1) == channels, "x must have all channels when there is no index");
+        return {1, (int)channels};
+    }
+    check(*index, "index", at::kInt);
+    TORCH_CHECK(index->dim() == 3 && index->device() == x.device() && index->size(0) == (x.size(0) + 31) / 32 &&
+                    index->size(1) * index->size(2) == x.size(1), "index must have shape [sub-batches, groups, C / groups]");
+    return {(int)index->size(1), (int)index->size(2)};
+}
+Tensor plane_shift(const Tensor& x, const optional<Tensor>& index, const Tensor& mean, const optional<Tensor>& running_mean, double momentum) {
+    const auto [G, kept] = check_plane(x, index, mean.numel());
+    Call call(x);
+    Tensor y = at::empty_like(x);
+    done(api.plane_shift(x.data_ptr<float>(), list_ptr(index), x.size(0), G, kept, x.size(2), mean.numel(), mean.data_ptr<float>(),
+                         running_mean.has_value() ? running_mean->data_ptr<float>() : nullptr, (float)momentum, y.data_ptr<float>(),
+                         call.stream), "plane_shift");
+    return y;
+}
+struct PlaneShiftFn : public torch::autograd::Function<PlaneShiftFn> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& given, const optional<Tensor>& index, const Tensor& running_mean,
+                                 double momentum) {
+        const Tensor x = given.contiguous();
+        check(running_mean, "running_mean");
+        TORCH_CHECK(running_mean.device() == x.device(), "all tensors must be on the same device");
+        Tensor mean = at::empty_like(running_mean), y = plane_shift(x, index, mean, running_mean, momentum);
+        if (index.has_value()) ctx->saved_data["index"] = *index;
+        ctx->saved_data["channels"] = running_mean.numel();
+        ctx->mark_non_differentiable({mean});
+        return {y, mean};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(4);
+        if (!grads[0].defined() || !ctx->needs_input_grad(0)) return out;
+        optional<Tensor> index;
+        if (ctx->saved_data.count("index")) index = ctx->saved_data["index"].toTensor();
+        const Tensor g = grads[0].contiguous();
+        Tensor mean = at::empty({ctx->saved_data["channels"].toInt()}, g.options());
+        out[0] = plane_shift(g, index, mean, c10::nullopt, 0.0);
+        return out;
+    }
+};
+
+struct PlaneSumFn;
+struct PlaneAddFn : public torch::autograd::Function<PlaneAddFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& given, const Tensor& values, const optional<Tensor>& index) {
+        const Tensor x = given.contiguous(), v = values.contiguous();
+        check(v, "v");
+        TORCH_CHECK(v.device() == x.device(), "all tensors must be on the same device");
+        const auto [G, kept] = check_plane(x, index, v.numel());
+        Call call(x);
+        Tensor y = at::empty_like(x);
+        done(api.plane_add(x.data_ptr<float>(), list_ptr(index), x.size(0), G, kept, x.size(2), v.numel(), v.data_ptr<float>(),
+                           y.data_ptr<float>(), call.stream), "plane_add");
+        if (index.has_value()) ctx->saved_data["index"] = *index;
+        ctx->saved_data["channels"] = v.numel();
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads);
+};
+// The transpose of adding v: sums per channel.
+struct PlaneSumFn : public torch::autograd::Function<PlaneSumFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& given, const optional<Tensor>& index, int64_t channels) {
+        const Tensor x = given.contiguous();
+        const auto [G, kept] = check_plane(x, index, channels);
+        Call call(x);
+        Tensor sum = at::empty({channels}, x.options());
+        done(api.plane_sum(x.data_ptr<float>(), list_ptr(index), x.size(0), G, kept, x.size(2), channels, sum.data_ptr<float>(), call.stream),
+             "plane_sum");
+        if (index.has_value()) ctx->saved_data["index"] = *index;
+        ctx->saved_data["shape"] = x.sizes().vec();
+        return sum;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(3);
+        if (!grads[0].defined()) return out;
+        optional<Tensor> index;
+        if (ctx->saved_data.count("index")) index = ctx->saved_data["index"].toTensor();
+        out[0] = PlaneAddFn::apply(at::zeros(ctx->saved_data["shape"].toIntVector(), grads[0].options()), grads[0], index);
+        return out;
+    }
+};
+variable_list PlaneAddFn::backward(AutogradContext* ctx, variable_list grads) {
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    optional<Tensor> index;
+    if (ctx->saved_data.count("index")) index = ctx->saved_data["index"].toTensor();
+    if (ctx->needs_input_grad(0)) out[0] = grads[0];
+    if (ctx->needs_input_grad(1)) out[1] = PlaneSumFn::apply(grads[0], index, ctx->saved_data["channels"].toInt());
+    return out;
+}
+
+Tensor unfold(const Tensor& x, int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t dil) {
+    return UnfoldFn::apply(x, kh, kw, stride, pad, dil);
+}
+std::tuple<Tensor, Tensor> mean_shift(const Tensor& x, const optional<Tensor>& index, const Tensor& running_mean, double momentum) {
+    auto out = PlaneShiftFn::apply(x, index, running_mean, momentum);
+    return {out[0], out[1]};
+}
+Tensor add_per_channel(const Tensor& x, const Tensor& v, const optional<Tensor>& index) { return PlaneAddFn::apply(x, v, index); }
+
 // ---- whole nets ------------------------------------------------------------------------------------
 // The layer table of one call, with the tensors it points to.  Row: (weight, bias, running mean, momentum, kept list [S, 1, count],
 // K, q) per layer.
@@ -509,6 +656,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sort_neuron", &sort_neuron);
     m.def("bound_inf_dist", &bound_inf_dist);
     m.def("bound_sort_neuron", &bound_sort_neuron);
+    m.def("unfold", &unfold);
+    m.def("mean_shift", &mean_shift);
+    m.def("add_per_channel", &add_per_channel);
     // A call that issues a whole pass takes long, and as long as the device does once the launch queue is full: other Python
     // threads run meanwhile.  None of the three touches a Python object.
     using Unlocked = py::call_guard<py::gil_scoped_release>;

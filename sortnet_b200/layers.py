@@ -24,6 +24,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules import module as _module
 
+from . import _lib
 from . import norm_dist_cuda as _C
 from . import ops
 
@@ -43,6 +44,10 @@ def sample_mask(batch, groups, channel, q, device, count=None):
     writes all lists; on the CPU the lists are made with PyTorch ops the way the reference does."""
     device = torch.device(device)
     if device.type == "cuda":
+        if count is None and isinstance(q, float) and _C._timeline is None and channel > 0:
+            # the same numbers from the host generator, counted and drawn in native code
+            uniform, seed = torch.rand(channel), torch.randint(0, 2 ** 62, (1,))
+            return _lib.ops().draw_lists(uniform, seed, [channel], [q], batch * groups, device)[0].view(batch, groups, -1)
         if count is None:
             count = int((torch.rand(channel) < q).sum())
         count = min(max(int(count), 1), channel)
@@ -153,11 +158,16 @@ class _PlaneSumF(torch.autograd.Function):
         return _PlaneAddF.apply(zeros, grad, ctx.index), None, None
 
 
+def _native():
+    """Whether the native forms of the autograd functions above are taken: not where they would not be seen or the profile wants each call."""
+    return _C._timeline is None and not ops.tracing() and not ops.forward_mode()
+
+
 def _add_per_channel(z, vec, index):
     """z [B, C, HW] plus vec [channels], gathered by the kept channels of each row's sub-batch."""
     plain = z.is_cuda and z.dtype == vec.dtype == torch.float32 and z.device == vec.device and not ops.tracing() and not ops.forward_mode()
     if plain and (index is None or (index.dtype == torch.int32 and index.is_contiguous())) and torch._C._functorch.peek_interpreter_stack() is None:
-        return _PlaneAddF.apply(z, vec, index)
+        return (_lib.ops().add_per_channel if _native() else _PlaneAddF.apply)(z, vec, index)
     return z + MeanShiftDropout._gathered(vec, index, z.size(0)).unsqueeze(-1)
 
 
@@ -211,7 +221,7 @@ class MeanShiftDropout(nn.Module):
         if self.training:
             assert x is not None, "training needs the activations"
             if plane:
-                x, mean = _MeanShiftPlaneF.apply(x, index, self.running_mean, self.momentum)
+                x, mean = (_lib.ops().mean_shift if _native() else _MeanShiftPlaneF.apply)(x, index, self.running_mean, self.momentum)
             else:
                 x, mean = _MeanShiftTrainF.apply(x, index, self.running_mean, self.momentum)
             if self.bias is not None:
@@ -381,6 +391,8 @@ class NormDistConv(nn.Module):
         if self.kernel_size == (1, 1) and self.stride == 1 and self.padding == 0:
             return z.reshape(z.size(0), z.size(1), -1).contiguous()
         if z.is_cuda and z.dtype == torch.float32 and all(isinstance(v, int) for v in (self.dilation, self.padding, self.stride)):
+            if _native():
+                return _lib.ops().unfold(z, *self.kernel_size, self.stride, self.padding, self.dilation)
             return _UnfoldF.apply(z, self.kernel_size, self.stride, self.padding, self.dilation)
         return F.unfold(z, self.kernel_size, self.dilation, self.padding, self.stride).contiguous()
 

@@ -93,3 +93,43 @@ def test_mean_shift_plane_matches_per_channel_mean():
     gy = torch.randn_like(y)
     y.backward(gy)
     assert rel(x.grad.cpu().numpy(), (gy - gy.mean(dim=(0, 2), keepdim=True)).cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("B,G,C,kept,hw", [(1, 1, 5, 5, 1), (33, 1, 9, 4, 4), (70, 3, 30, 7, 9)])
+def test_native_glue_is_the_python_one(B, G, C, kept, hw):
+    """Mean shift and per-channel add in native code: values and gradients of the Python functions, second order of the add included."""
+    from sortnet_b200 import layers, _lib
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    S, per = (B + 31) // 32, C // G
+    index = None if kept == per else torch.rand(S, G, per, device="cuda", generator=gen).argsort(-1)[..., :kept].sort(-1)[0].int().contiguous()
+    x = torch.randn(hw, G * kept, B, device="cuda", generator=gen).permute(2, 1, 0).requires_grad_()       # not contiguous
+    v = torch.randn(C, device="cuda", generator=gen).requires_grad_()
+    g = torch.randn(B, G * kept, hw, device="cuda", generator=gen)
+    got = []
+    for shift, add in ((_lib.ops().mean_shift, _lib.ops().add_per_channel), (layers._MeanShiftPlaneF.apply, layers._PlaneAddF.apply)):
+        run = torch.ones(C, device="cuda")
+        y, mean = shift(x, index, run, 0.1)
+        z = add(y, v, index)
+        gx, gv = torch.autograd.grad(z, (x, v), g)
+        second, = torch.autograd.grad(torch.autograd.grad((add(x, v, index) ** 3).sum(), v, create_graph=True)[0].sum(), v)
+        assert not mean.requires_grad
+        got.append((y, mean, run, z, gx, gv, second))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    rows = torch.arange(B, device="cuda") // 32
+    chan = torch.arange(C, device="cuda").expand(B, C) if index is None else layers._global_index(index, C)[rows]
+    want = 6 * torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), (x + v[chan].unsqueeze(-1)).double().sum(-1).reshape(-1))
+    assert (got[0][-1].double() - want).abs().max() <= 1e-4 * want.abs().max().clamp(min=1)                # fp32 sums of up to 630 values
+
+
+@pytest.mark.parametrize("S,G,channel,q", [(1, 1, 7, 0.5), (4, 1, 1024, 0.75), (3, 3, 341, 0.9), (2, 1, 40, 0.0)])
+def test_sample_mask_draws_what_it_did(S, G, channel, q):
+    """The lists of the seeds and counts that the host generator gives, one kernel call as before."""
+    from sortnet_b200 import layers, norm_dist_cuda as C
+    torch.manual_seed(7)
+    got, after = layers.sample_mask(S, G, channel, q, "cuda"), torch.rand(1)
+    torch.manual_seed(7)
+    count = min(max(int((torch.rand(channel) < q).sum()), 1), channel)
+    seed = int(torch.randint(0, 2 ** 62, (1,)))
+    want = torch.empty(S, G, count, dtype=torch.int32, device="cuda")
+    C.sample_mask_into(want, channel, seed)
+    assert torch.equal(got, want) and got.is_contiguous() and torch.equal(after, torch.rand(1))
