@@ -32,6 +32,21 @@ inline cudaError_t allow_smem() {
 }
 constexpr int MOST_SMEM = 227 * 1024;        // what a CTA of sm_100a may have
 
+// Asks that the SM's memory be divided for KERN as CTAS of its CTAs with BYTES of shared memory each need it, the rest being its L1 (once per device, as
+// above).  Without that an SM stays as the kernel before left it, and in a chain that is what a filter with 217 KB of stages wants: the
+// list walks behind it, which live on L1, took 50 instead of 43 us per layer of a training pass.
+template <auto KERN, int CTAS, int BYTES>
+inline cudaError_t prefer_l1() {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (done[dev & 63].load(std::memory_order_acquire)) return cudaSuccess;
+    constexpr int room = CTAS * (BYTES + 1024), all = 228 * 1024, share = room >= all ? 100 : (100 * room + all - 1) / all;
+    const cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributePreferredSharedMemoryCarveout, share);
+    if (e == cudaSuccess) done[dev & 63].store(true, std::memory_order_release);
+    return e;
+}
+
 // Launches KERN so that its CTAs may be set up while the kernel before it in the stream ends.  Every thread of it calls after_previous()
 // (common.cuh) before it touches what that kernel writes or may still read.  For chains of kernels of 10 to 40 us, where 2 to 3 us from
 // the end of one to the first loads of the next count: interval bounds of seven layers (24 launches) 540 -> 500 us, a training pass of

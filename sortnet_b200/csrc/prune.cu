@@ -738,7 +738,9 @@ __device__ __noinline__ void dense_prepare(const PruneArgs& a, int s, int n0, in
 // TRACK keeps, per row, the step that set the maximum; the word is made at the end from the step's columns.  A
 // later step that only equals the maximum (rare) sends the lane over the list once more for the lowest position.
 template <int NX, bool TRACK>
-__global__ void __launch_bounds__(256, NX == 1 && !TRACK ? 6 : NX == 2 && TRACK ? 3 : 4) prune_max(const __grid_constant__ PruneArgs a) {
+constexpr int WALK_CTAS = NX == 1 && !TRACK ? 6 : NX == 2 && TRACK ? 3 : 4;
+template <int NX, bool TRACK>
+__global__ void __launch_bounds__(256, WALK_CTAS<NX, TRACK>) prune_max(const __grid_constant__ PruneArgs a) {
     constexpr int NV = NX == 3 ? 3 : NX;                     // values per row: |x - w|, lower, upper
     constexpr int WORDS = TRACK ? NX : 0;
     __shared__ float tile[NV + WORDS][32][33];
@@ -993,6 +995,8 @@ struct SortQueue {
     static constexpr int WIDTH = NX == 3 ? 4 : NX;           // floats of an entry: the values of all tensors side by side
 };
 constexpr int SORT_SLOTS = 8;           // outputs of a CTA of prune_sort
+template <int KMAX>
+constexpr int SORT_CTAS = KMAX <= 10 ? 4 : 2;
 template <int NX, int KMAX, bool POS>
 constexpr int sort_walk_smem(int K) {
     using Q = SortQueue<NX, KMAX, POS>;
@@ -1064,7 +1068,7 @@ __device__ __forceinline__ int shared_u16(unsigned at) {
 // order of insertion decide (ordered_positions).  128 x 5120 x 5120, K = 10: 107 -> 86 us; always with a second walk, and
 // each word stored for eight of 32 lanes: 107.
 template <int NX, int KMAX, bool POS>
-__global__ void __launch_bounds__(256, KMAX <= 10 ? 4 : 2) prune_sort(const __grid_constant__ PruneArgs a) {
+__global__ void __launch_bounds__(256, SORT_CTAS<KMAX>) prune_sort(const __grid_constant__ PruneArgs a) {
     constexpr uint32_t EMPTY = 0xffffffffu;
     constexpr int LD = SORT_SLOTS + 1;
     constexpr bool LOG = SortQueue<NX, KMAX, POS>::LOG, QUEUED = SortQueue<NX, KMAX, POS>::USED;
@@ -1440,6 +1444,8 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     int redo = 0;
     if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
+    constexpr int tile = (TRACK ? 2 : 1) * NX * 32 * 33 * (int)sizeof(float);
+    if ((e = prefer_l1<prune_max<NX, TRACK>, WALK_CTAS<NX, TRACK>, tile>()) != cudaSuccess) return e;
     if ((e = launch_next(prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
     return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
 }
@@ -1453,6 +1459,8 @@ cudaError_t run_sort(const PruneArgs& a, cudaStream_t st) {
     cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
     if (e == cudaSuccess) e = allow_smem<prune_sort<NX, KMAX, POS>, sort_walk_smem<NX, KMAX, POS>(KMAX)>();
     if (e != cudaSuccess) return e;
+    constexpr int most = sort_walk_smem<NX, KMAX, POS>(KMAX);
+    if ((e = prefer_l1<prune_sort<NX, KMAX, POS>, SORT_CTAS<KMAX>, most>()) != cudaSuccess) return e;
     e = launch_next(prune_sort<NX, KMAX, POS>, dim3((a.p.CO + SORT_SLOTS - 1) / SORT_SLOTS, a.S), 256, sort_walk_smem<NX, KMAX, POS>(a.p.K), st, a);
     if (e != cudaSuccess) return e;
     if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;
