@@ -52,6 +52,20 @@ def test_distance_and_words(B, CI, CO, kind):
     assert np.array_equal(host(yn), y_o)
 
 
+# widths on both sides of the filter's forms, copied by fours and by ones; fewer rows than CTAs, and many steps per CTA
+@pytest.mark.parametrize("B,CI,CO", [(32, 2048, 200), (33, 2050, 200), (31, 3072, 150), (31, 3073, 150), (32, 4096, 120), (32, 4097, 120),
+                                     (32, 5501, 100), (32, 6144, 90), (32, 8193, 60), (32, 300, 4001), (32, 132, 9001)])
+@pytest.mark.parametrize("kind", ["normal", "ties", "mixed"])
+def test_filter_forms(B, CI, CO, kind):
+    from sortnet_b200 import norm_dist_cuda as C
+    assert uses_pruning(1, 1, 1, B, CO, CI, CO, CI, 0)
+    x, w = operands(kind, np.random.default_rng(CI), B, CI, CO)
+    y_o, pos_o = oracle.inf_dist_forward(x, w)
+    y, pos = torch.full((B, CO, 1), 7.0, device="cuda"), torch.full((B, CO, 1), 7, device="cuda", dtype=torch.int32)
+    C.inf_dist_forward(col3(x), dev(w), y, pos, 1)
+    assert np.array_equal(host(y), y_o) and np.array_equal(host(pos), pos_o)
+
+
 @pytest.mark.parametrize("B,CI,CO,keep", [(70, 1024, 1100, 0.9), (160, 1030, 460, 0.7), (33, 2049, 1900, 0.5),
                                           (96, 5120, 200, 0.95)])
 @pytest.mark.parametrize("which", ["both", "ci", "co"])
