@@ -755,10 +755,14 @@ __global__ void __launch_bounds__(256, WALK_CTAS<NX, TRACK>) prune_max(const __g
     let_next();
     const unsigned overflowed = load_now(a.counters + OVERFLOWED), general = p.ci ? load_now(a.counters + GENERAL) : 0u;
     const int j = n < p.CO ? (p.co ? p.co[(size_t)s * p.CO + n] : n) : 0;
-    const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
-    const int cnt = wanted ? a.cnt[j] : 0;
-    const float tau = a.tau[j];
+    // What the walk starts from comes together, not one after the other: the head of a list that is not there (or not wanted) is memory all the
+    // same, and not looked at.  Seven layers of points and boxes 460 -> 443 us.
     const int4* list = reinterpret_cast<const int4*>(a.cand + (size_t)j * a.lcap);
+    const int listed = a.cnt[j];
+    int4 e01 = list[0], e23 = list[1];
+    const float tau = a.tau[j];
+    const bool wanted = n < p.CO && (!p.keep || p.keep[(size_t)s * p.CO + j]);
+    const int cnt = wanted ? listed : 0;
     const float* ub = a.ub + (size_t)j * (a.lcap / STEP);
     const int live = min(4, p.B - s * 32 - 4 * l);           // rows of this lane that exist (may be <= 0)
 
@@ -790,10 +794,8 @@ __global__ void __launch_bounds__(256, WALK_CTAS<NX, TRACK>) prune_max(const __g
         }
     };
     bool active = cnt > 0;
-    int4 e01 = make_int4(0, 0, 0, 0), e23 = e01;
     float left = 0.f;
     int walked = 0;
-    if (active) e01 = list[0], e23 = list[1];
     // looked at only here, so that it is on its way together with the head of the list
     if ((general & LIST_TWICE) || prune_gives_up(overflowed, p.W_CO)) {
         dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
