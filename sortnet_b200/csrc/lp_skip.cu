@@ -191,11 +191,14 @@ struct ForwardArgs {
     Slabs sl;
     int B, CO, CI, W_CI;
     float p, cut;
+    const unsigned* pruned;     // skip_maxima: counters of the evaluation that may have left the layer, or null
+    int W_CO;
 };
 
 // The maxima M.  Per warp: an output; the threshold is the largest lower bound |w - mid| - rad of a column so far, and the
 // columns that can still exceed it are evaluated.  Bound by the scan of W.
 __global__ void __launch_bounds__(THREADS, 1) skip_maxima(const ForwardArgs a) {
+    if (a.pruned && !prune_left(a.pruned, a.ci != nullptr, a.W_CO)) return;
     extern __shared__ __align__(16) unsigned char dyn[];
     const int padded = up_to(a.sl.chunk, SCAN);
     float* xs = reinterpret_cast<float*>(dyn);                              // [chunk + 1][32]; the last row is zero
@@ -590,21 +593,23 @@ struct Area {
     }
 };
 
-// The maxima by the pruned evaluation (prune.cuh), which reads W once for all sub-batches, where skip_maxima does so for each: it pays from so many
-// weights on that it need not read again.  Forward at p = 1000, skip_maxima / pruned: 512 x 5120 x 5120 876 / 476 us, 512 x 784 x 5120 198 / 144,
-// 64 x 5120 x 5120 144 / 113, 512 x 784 x 1000 (12 M weights not read again) 56.5 / 52.2, 67 x 5120 x 1000 (10 M) 53.9 / 54.1, 67 x 784 x 2000
-// (3 M) 33.7 / 42.0.  With lists of three quarters the pruned form reads all of W and has more to prepare: 512 x 5120 x 5120 (221 M) 516 / 342,
-// 512 x 784 x 5120 (34 M) 131.6 / 127.4, 64 x 5120 x 5120 (15 M) 101 / 117.  One sub-batch gains nothing: 24 x 5120 x 5120 84 / 90.
+// The maxima by the pruned evaluation (prune.cuh), which reads W once for all sub-batches, where skip_maxima does so for each: from so many weights on
+// that it need not read again.  Forward at p = 1000, skip_maxima / pruned, inputs in [0, 1]: 512 x 5120 x 5120 899 / 502 us, 512 x 784 x 5120
+// (60 M weights not read again) 225 / 170; with lists of three quarters, for which the pruned form reads all of W and has more to prepare,
+// 512 x 5120 x 5120 (221 M) 516 / 342, 512 x 784 x 5120 (34 M) 131.6 / 127.4, 64 x 5120 x 5120 (15 M) 101 / 117.  A layer that cannot be pruned is left to
+// skip_maxima, after a filter in vain: inputs N(0, 0.35) 1054 / 1105 and 259 / 284.  At 64 x 5120 x 5120 (26 M) that would be 195 / 232 for a gain
+// of 175 / 140: not taken.
 PruneProblem maxima_problem(const LpProblem& q, float* mt) {
     PruneProblem m;
     m.x = q.x, m.w = q.w, m.ci = q.ci, m.co = q.co;
     m.B = q.B, m.CO = q.CO, m.CI = q.CI, m.W_CO = q.W_CO, m.W_CI = q.W_CI;
     m.yt = mt;
+    m.leave = true;
     return m;
 }
 bool maxima_pruned(const LpProblem& q) {
     const long long again = (long long)((q.B + 31) / 32 - 1) * q.CO * q.CI;
-    return again >= (q.ci ? 32ll << 20 : 10ll << 20) && prune_applies(maxima_problem(q, nullptr));
+    return again >= 32ll << 20 && prune_applies(maxima_problem(q, nullptr));
 }
 
 size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, char** prune = nullptr) {
@@ -619,7 +624,7 @@ size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, char** pru
     if (a) {
         a->w = q.w, a->ci = q.ci, a->co = q.co, a->xt = xt, a->range = range, a->mt = mt, a->sum = sum;
         a->sl = slabs((int)S, q.CI, q.CO, 128, 12);
-        a->B = q.B, a->CO = q.CO, a->CI = q.CI, a->W_CI = q.W_CI;
+        a->B = q.B, a->CO = q.CO, a->CI = q.CI, a->W_CI = q.W_CI, a->W_CO = q.W_CO;
         // what is left out changes y by less than CI cut^p / p = 2^-27 of it
         a->p = q.p, a->cut = fminf(exp2f(-(27.0f + log2f((float)q.CI / q.p)) / q.p), CUT_MOST);
     }
@@ -660,11 +665,13 @@ cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, cudaStream_t
     const bool pruned = maxima_pruned(q);
     cudaError_t e = cudaSuccess;
     // maxima and sums lie side by side
-    char* const zeroed = reinterpret_cast<char*>(pruned ? a.sum : a.mt);
-    if (a.sl.chunks > 1 && (e = cudaMemsetAsync(zeroed, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - zeroed, st)) != cudaSuccess) return e;
-    if (pruned && (e = prune_forward(maxima_problem(q, a.mt), prune, st)) != cudaSuccess) return e;
+    if (a.sl.chunks > 1 && (e = cudaMemsetAsync(a.mt, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - (char*)a.mt, st)) != cudaSuccess) return e;
+    if (pruned) {
+        if ((e = prune_forward(maxima_problem(q, a.mt), prune, st)) != cudaSuccess) return e;
+        a.pruned = reinterpret_cast<const unsigned*>(prune);
+    }
     skip_columns<<<dim3((q.CI + 63) / 64, S), 256, 0, st>>>(q.x, q.B, q.CI, const_cast<float*>(a.xt), const_cast<float2*>(a.range));
-    if (!pruned && (e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
+    if ((e = launch<skip_maxima>(a, smem, st)) != cudaSuccess) return e;
     if ((e = launch<skip_forward>(a, smem, st)) != cudaSuccess) return e;
     skip_finish<<<dim3((q.CO + 63) / 64, S), 256, 0, st>>>(a.sum, a.mt, q.B, q.CO, q.p, y);
     return launched(2);

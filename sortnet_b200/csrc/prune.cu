@@ -36,14 +36,7 @@ struct PruneArgs {
     unsigned* tile_done;            // [S][blocks of 128 outputs] k-tiles merged
 };
 
-// Outputs left over by the walks; rows of W whose list overflowed; what the column lists are not: in ascending order, or (the
-// transposed input has one place per column) without an entry that comes twice.
-enum { FAILED = 0, OVERFLOWED = 1, GENERAL = 2 };
-constexpr unsigned LIST_ORDER = 1u, LIST_TWICE = 2u;
-
-__device__ __forceinline__ bool dense_mode(const PruneArgs& a) {
-    return (a.p.ci && (a.counters[GENERAL] & LIST_TWICE)) || prune_gives_up(a.counters[OVERFLOWED], a.p.W_CO);
-}
+__device__ __forceinline__ bool dense_mode(const PruneArgs& a) { return prune_left(a.counters, a.p.ci != nullptr, a.p.W_CO); }
 
 // A load that stays where it is written.
 __device__ __forceinline__ unsigned load_now(const unsigned* p) {
@@ -798,7 +791,7 @@ __global__ void __launch_bounds__(256, WALK_CTAS<NX, TRACK>) prune_max(const __g
     int walked = 0;
     // looked at only here, so that it is on its way together with the head of the list
     if ((general & LIST_TWICE) || prune_gives_up(overflowed, p.W_CO)) {
-        dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
+        if (!p.leave) dense_prepare<NX>(a, s, n0, TRACK ? 8 : 4);
         return;
     }
     if (tid == 0) failed = arrived = 0u;

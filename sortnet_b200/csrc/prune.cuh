@@ -64,6 +64,7 @@ struct PruneProblem {
     const float* bias = nullptr;
     unsigned* counters = nullptr;       // four zeroed counters of the caller's, or null: those in the workspace
     const int* kept_list = nullptr;     // [S][kept] kept columns: the first one is the position of an output at its floor
+    bool leave = false;                 // maxima: a layer that would be evaluated as a whole is left to the caller (prune_left)
 };
 
 // Transposes x (or x and the box [max(x - eps, down), min(x + eps, up)], or given box ends) to the chain form.
@@ -95,6 +96,15 @@ __device__ __forceinline__ float decode(unsigned e) {   // 0 -> NaN
 // Above 1 / 32 of overflowed lists the layer is evaluated as a whole: one output by itself costs about 12 times its part
 // of the whole (512 x 5120 x 5120 with positions).
 __host__ __device__ __forceinline__ bool prune_gives_up(unsigned overflowed, int W_CO) { return (long long)overflowed * 32 > W_CO; }
+
+// What the counters of a problem count, at the start of its workspace (unless they are the caller's): outputs left over by the walks; rows of W whose list
+// overflowed; what the column lists are not: in ascending order, or (the transposed input has one place per column) without an entry that
+// comes twice.
+enum { FAILED = 0, OVERFLOWED = 1, GENERAL = 2 };
+constexpr unsigned LIST_ORDER = 1u, LIST_TWICE = 2u;
+__device__ __forceinline__ bool prune_left(const unsigned* counters, bool column_lists, int W_CO) {
+    return (column_lists && (counters[GENERAL] & LIST_TWICE)) || prune_gives_up(counters[OVERFLOWED], W_CO);
+}
 
 // y and pos of a sort neuron by the kernels of sort_neuron.cu if the layer is to be evaluated as a whole, nothing otherwise.
 cudaError_t sort_positions_if(const PruneProblem& p, const unsigned* overflowed, cudaStream_t st);

@@ -558,6 +558,7 @@ __global__ void __launch_bounds__(REDO_THREADS, 2) prune_redo_max(const __grid_c
     after_previous();
     let_next();
     if (dense_mode(a)) {
+        if (a.p.leave) return;
         const DenseLayer d(a);
         if constexpr (NX != 2) {
             if (a.p.co || a.p.ci || a.p.out_list || a.S == 1) dense_point<NX, TRACK, 1>(a, d, redo_smem);

@@ -92,8 +92,8 @@ def test_against_float64(B, CI, CO, keep, p):
     assert near(gx2, gx) < 1e-6                                     # sums in another order
 
 
-# two, ten and three sub-batches on both sides of the 10 M weights (32 M with lists) that are not read again
-@pytest.mark.parametrize("B,CI,CO,keep", [(33, 3260, 3220, 1.0), (33, 3200, 3220, 1.0), (290, 1103, 1100, 1.0), (96, 5120, 4600, 0.9), (96, 4700, 4200, 0.9)])
+# two, ten and three sub-batches on both sides of the 32 M weights that are not read again; slabs of one and more chunks
+@pytest.mark.parametrize("B,CI,CO,keep", [(33, 5900, 5800, 1.0), (33, 5700, 5800, 1.0), (290, 2003, 1900, 1.0), (1100, 1003, 1100, 1.0), (96, 5120, 4600, 0.9), (96, 4700, 4200, 0.9)])
 @pytest.mark.parametrize("kind", ["plain", "no numbers", "wide"])
 @pytest.mark.parametrize("p", [31.6, 1000.0])
 def test_maxima_of_many_sub_batches(B, CI, CO, keep, kind, p):
