@@ -32,36 +32,37 @@ inline cudaError_t allow_smem() {
 }
 constexpr int MOST_SMEM = 227 * 1024;        // what a CTA of sm_100a may have
 
-// Asks that the SM's memory be divided for KERN as CTAS of its CTAs with BYTES of shared memory each need it, the rest being its L1 (once per device, as
-// above).  Without that an SM stays as the kernel before left it, and in a chain that is what a filter with 217 KB of stages wants: the
-// list walks behind it, which live on L1, took 50 instead of 43 us per layer of a training pass.
-template <auto KERN, int CTAS, int BYTES>
-inline cudaError_t prefer_l1() {
-    static std::atomic<bool> done[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (done[dev & 63].load(std::memory_order_acquire)) return cudaSuccess;
-    constexpr int room = CTAS * (BYTES + 1024), all = 228 * 1024, share = room >= all ? 100 : (100 * room + all - 1) / all;
-    const cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributePreferredSharedMemoryCarveout, share);
-    if (e == cudaSuccess) done[dev & 63].store(true, std::memory_order_release);
-    return e;
-}
-
 // Launches KERN so that its CTAs may be set up while the kernel before it in the stream ends.  Every thread of it calls after_previous()
 // (common.cuh) before it touches what that kernel writes or may still read.  For chains of kernels of 10 to 40 us, where 2 to 3 us from
 // the end of one to the first loads of the next count: interval bounds of seven layers (24 launches) 540 -> 500 us, a training pass of
 // six 777 -> 765 us, sort neurons with gradients 995 -> 953 us.
+// share: percent of an SM's memory that shared memory should have, the rest being L1 (l1_share below); negative: as the kernel before left it.
 template <typename... Params, typename... Args>
-inline cudaError_t launch_next(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args) {
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_next_with(int share, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attributes[1].val.sharedMemCarveout = share > 0 ? (unsigned)share : 0u;
     cudaLaunchConfig_t config = {};
     config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem, config.stream = st;
-    config.attrs = &attribute, config.numAttrs = 1;
+    config.attrs = attributes, config.numAttrs = share < 0 ? 1 : 2;
     const cudaError_t e = cudaLaunchKernelEx(&config, kern, static_cast<Params>(args)...);
     const cudaError_t last = launched();                     // takes a failed launch's error away, so that no later call reports it
     return e != cudaSuccess ? e : last;
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_next(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args) {
+    return launch_next_with(-1, kern, grid, block, smem, st, args...);
+}
+
+// The share with which `ctas` CTAs of `bytes` of shared memory fit an SM and the rest is L1, for a grid of `grid` CTAs.  Left alone, an SM stays as the
+// kernel before wanted it, and in a chain that is a filter with its stages: the list walks behind it, which live on L1, took 50 instead of
+// 43 us per layer of a training pass.  A grid of less than a CTA per SM is left alone: it has little to gain, and dividing the memory anew
+// takes its while (four layers of 28 rows and 832 outputs 95 us, with all of them divided 98).
+inline int l1_share(int ctas, int bytes, long long grid) {
+    const int room = ctas * (bytes + 1024), all = 228 * 1024;
+    return grid < sm_count() ? -1 : room >= all ? 100 : (100 * room + all - 1) / all;
 }
 
 // Values with positions of small problems by one launch of a warp per row and four outputs, instead of tiles, partial results and a

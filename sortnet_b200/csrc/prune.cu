@@ -1407,11 +1407,11 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     cudaError_t e = allow_smem<KERN, bytes(LONG_LIST)>();
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    if ((e = prefer_l1<KERN, FIT, bytes(LONG_LIST)>()) != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, threads, smem);
     if (e != cudaSuccess) return e;
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
-    return launch_next(KERN, steps < slots ? steps : slots, threads, smem, st, a);
+    const int grid = steps < slots ? steps : slots;
+    return launch_next_with(l1_share(FIT, bytes(LONG_LIST), grid), KERN, grid, threads, smem, st, a);
 }
 
 template <bool VEC>
@@ -1445,8 +1445,8 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     int redo = 0;
     if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
     constexpr int tile = (TRACK ? 2 : 1) * NX * 32 * 33 * (int)sizeof(float);
-    if ((e = prefer_l1<prune_max<NX, TRACK>, WALK_CTAS<NX, TRACK>, tile>()) != cudaSuccess) return e;
-    if ((e = launch_next(prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
+    const int share = l1_share(WALK_CTAS<NX, TRACK>, tile, (long long)grid.x * grid.y);
+    if ((e = launch_next_with(share, prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
     return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
 }
 
@@ -1459,9 +1459,9 @@ cudaError_t run_sort(const PruneArgs& a, cudaStream_t st) {
     cudaError_t e = redo_grid<prune_redo_sort<NX, KMAX, POS>>(256, 0, &redo);
     if (e == cudaSuccess) e = allow_smem<prune_sort<NX, KMAX, POS>, sort_walk_smem<NX, KMAX, POS>(KMAX)>();
     if (e != cudaSuccess) return e;
-    constexpr int most = sort_walk_smem<NX, KMAX, POS>(KMAX);
-    if ((e = prefer_l1<prune_sort<NX, KMAX, POS>, SORT_CTAS<KMAX>, most>()) != cudaSuccess) return e;
-    e = launch_next(prune_sort<NX, KMAX, POS>, dim3((a.p.CO + SORT_SLOTS - 1) / SORT_SLOTS, a.S), 256, sort_walk_smem<NX, KMAX, POS>(a.p.K), st, a);
+    const dim3 grid((a.p.CO + SORT_SLOTS - 1) / SORT_SLOTS, a.S);
+    const int smem = sort_walk_smem<NX, KMAX, POS>(a.p.K), share = l1_share(SORT_CTAS<KMAX>, smem, (long long)grid.x * grid.y);
+    e = launch_next_with(share, prune_sort<NX, KMAX, POS>, grid, 256, smem, st, a);
     if (e != cudaSuccess) return e;
     if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;
     return sort_positions_if(a.p, a.counters + OVERFLOWED, st);
