@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) mean_shift_apply_kernel(const float* __re
 // The same over rows and positions of x [B, n, HW] (n kept channels of G groups, lists of within-group channels): a warp per channel, which
 // walks the channel's HW neighbouring floats of every row that kept it twice, for the sum and for the result; the second time they come from L1
 // or L2.  The slot of the channel in 32 sub-batches' lists is searched for by 32 lanes at once.  SHIFT: the mean into `out`, x minus it into y;
-// otherwise the sums alone.  Bound by latency: 128 x 1024 x 4 with lists 7.9 us, against 8.2 + 3.2 for the same plane as 4096 channels and six
+// otherwise the sums alone.  Bound by latency: 128 x 1024 x 4 with lists 8.4 us, against 8.2 + 3.2 for the same plane as 4096 channels and six
 // launches for its lists, the average over positions, its expansion and the running mean; a forward and backward of two convolutions, which
 // the host issues, 1050 -> 740 us (58 -> 39 launches).
 template <bool SHIFT>
@@ -120,15 +120,14 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
             }
         }
     };
-    float sum = 0.f, cnt = 0.f;
+    double sum = 0.;                                         // a lane's chain grows with rows x HW: in fp32 its rounding showed (1.4e-7 -> 1.6e-7 of the mean)
+    float cnt = 0.f;
     int first = -1;                                          // the slots of the first 32 sub-batches
     for (int s0 = 0; s0 < S; s0 += 32) {
         const int mine = s0 + lane < S ? slot_in(s0 + lane) : -1;
         if (s0 == 0) first = mine;
         if (mine >= 0) cnt += (float)(min(SNB_SUB_BATCH, B - (s0 + lane) * SNB_SUB_BATCH) * HW);
-        float part = 0.f;
-        walk(s0, mine, [&](size_t o) { part += x[o]; });
-        sum += part;
+        walk(s0, mine, [&](size_t o) { sum += (double)x[o]; });
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -136,10 +135,10 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
         cnt += __shfl_xor_sync(0xffffffffu, cnt, d);
     }
     if (!SHIFT) {
-        if (lane == 0) out[c] = sum;
+        if (lane == 0) out[c] = (float)sum;
         return;
     }
-    const float m = sum / fmaxf(cnt, 1e-10f);
+    const float m = (float)(sum / fmaxf(cnt, 1e-10f));
     if (lane == 0) {
         out[c] = m;
         if (running_mean) running_mean[c] = running_mean[c] * (1.0f - momentum) + momentum * m;
