@@ -1087,11 +1087,11 @@ __global__ void __launch_bounds__(256, SORT_CTAS<KMAX>) prune_sort(const __grid_
     const unsigned columns = queues + 8 * DEPTH * ROW + warp * DEPTH * 64 + lane * 2;
     const int fill = max(8, (K + 3) / 4 * 4);                // LOG: entries that are not logged
     after_previous();
-    let_next();
-    if (dense_mode(a)) {
+    if (dense_mode(a)) {                                     // no CTA of the next kernel before the last of these: its few hundred long ones spread evenly then
         if (!POS) dense_prepare<NX>(a, s, n0, 0, SORT_SLOTS);     // positions: sort_positions_if reads the rows as they came
         return;
     }
+    let_next();
     const bool chain = !POS && !p.y && !p.yl && !p.yu && !p.part;   // written from here: no warp waits for the others
     if (tid == 0) failed = arrived = 0u;
     __syncthreads();
