@@ -325,7 +325,8 @@ int snb_mean_shift_apply(const float* x, const float* mean, const int* index, in
 
 /* The mean shift over rows and positions: x [B, G kept, hw] with lists index [S, G, kept] of within-group channels, ascending
  * (NULL: all channels, then channels == G kept).  mean [channels] (0 for never-kept ones), y = x minus its channel's mean,
- * optional running mean as above.  The sums alone, and x plus its channel's entry of v (a bias, and the bias gradient).
+ * optional running mean as above.  x plus its channel's entry of v, and the sums alone (a bias, and its gradient): these two for lists in
+ * any order, that may name a channel twice.
  * Replace core/models/bound_basic_module.py:123-157 and core/models/norm_dist.py:102-103 for [B, C, HW]. */
 int snb_plane_shift(const float* x, const int* index, int B, int G, int kept, int hw, int channels, float* mean,
                     float* running_mean, float momentum, float* y, void* stream);

@@ -96,28 +96,35 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
     const int lane = threadIdx.x & 31, c = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (c >= C) return;
     const int S = (B + SNB_SUB_BATCH - 1) / SNB_SUB_BATCH, per = C / G, g = c / per, inside = c % per, n = G * kept;
-    auto slot_in = [&](int s) {
-        if (!index) return c;
+    // Place of channel `want` in list g of sub-batch s: that of the first entry that is not smaller, if the list ascends.
+    auto place = [&](int s, int g, int want) {
         const int* list = index + ((size_t)s * G + g) * kept;
         int lo = 0, hi = kept;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (list[mid] < inside) lo = mid + 1;
+            if (list[mid] < want) lo = mid + 1;
             else hi = mid;
         }
-        return lo < kept && list[lo] == inside ? g * kept + lo : -1;
+        return lo;
     };
-    // body(offset of the element) for this lane's elements of the channel
-    auto walk = [&](int s0, int mine, auto&& body) {
+    auto slot_in = [&](int s) {
+        if (!index) return c;
+        const int at = place(s, g, inside);
+        return at < kept && index[((size_t)s * G + g) * kept + at] == inside ? g * kept + at : -1;
+    };
+    // body(offset of the element) for this lane's elements of slot `slot` of sub-batch s
+    auto walk = [&](int s, int slot, auto&& body) {
+        const int b0 = s * SNB_SUB_BATCH, items = min(SNB_SUB_BATCH, B - b0) * HW;
+#pragma unroll 4
+        for (int i = lane; i < items; i += 32) {
+            const int b = i / HW;
+            body(((size_t)(b0 + b) * n + slot) * HW + (i - b * HW));
+        }
+    };
+    auto walk_all = [&](int s0, int mine, auto&& body) {
         for (int t = 0; t < min(32, S - s0); t++) {
             const int slot = __shfl_sync(0xffffffffu, mine, t);
-            if (slot < 0) continue;
-            const int b0 = (s0 + t) * SNB_SUB_BATCH, items = min(SNB_SUB_BATCH, B - b0) * HW;
-#pragma unroll 4
-            for (int i = lane; i < items; i += 32) {
-                const int b = i / HW;
-                body(((size_t)(b0 + b) * n + slot) * HW + (i - b * HW));
-            }
+            if (slot >= 0) walk(s0 + t, slot, body);
         }
     };
     double sum = 0.;                                         // a lane's chain grows with rows x HW: in fp32 its rounding showed (1.4e-7 -> 1.6e-7 of the mean)
@@ -127,7 +134,7 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
         const int mine = s0 + lane < S ? slot_in(s0 + lane) : -1;
         if (s0 == 0) first = mine;
         if (mine >= 0) cnt += (float)(min(SNB_SUB_BATCH, B - (s0 + lane) * SNB_SUB_BATCH) * HW);
-        walk(s0, mine, [&](size_t o) { sum += (double)x[o]; });
+        walk_all(s0, mine, [&](size_t o) { sum += (double)x[o]; });
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -135,7 +142,25 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
         cnt += __shfl_xor_sync(0xffffffffu, cnt, d);
     }
     if (!SHIFT) {
-        if (lane == 0) out[c] = (float)sum;
+        if (lane == 0 && !index) out[c] = (float)sum;
+        else if (lane == 0 && cnt > 0.f) atomicAdd(out + c, (float)sum);
+        if (!index || c >= n) return;
+        // The warp also looks whether slot c of every list was found by its channel's warp.  In a list that does not ascend, or names a channel twice, some
+        // are not: their sums are added here.  Lists that ascend end in one addition to zero per channel.
+        const int gj = c / kept;
+        for (int s0 = 0; s0 < S; s0 += 32) {
+            const int s = s0 + lane, entry = s < S ? index[(size_t)s * n + c] : -1;
+            unsigned lost = __ballot_sync(0xffffffffu, entry >= 0 && entry < per && place(s, gj, entry) != c - gj * kept);
+            for (; lost; lost &= lost - 1) {
+                const int t = __ffs(lost) - 1;
+                double part = 0.;
+                walk(s0 + t, c, [&](size_t o) { part += (double)x[o]; });
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+                const int channel = gj * per + __shfl_sync(0xffffffffu, entry, t);
+                if (lane == 0) atomicAdd(out + channel, (float)part);
+            }
+        }
         return;
     }
     const float m = (float)(sum / fmaxf(cnt, 1e-10f));
@@ -145,7 +170,7 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
     }
     for (int s0 = 0; s0 < S; s0 += 32) {
         const int mine = s0 == 0 ? first : s0 + lane < S ? slot_in(s0 + lane) : -1;
-        walk(s0, mine, [&](size_t o) { y[o] = x[o] - m; });
+        walk_all(s0, mine, [&](size_t o) { y[o] = x[o] - m; });
     }
 }
 
@@ -208,6 +233,7 @@ extern "C" int snb_plane_sum(const float* x, const int* index, int B, int G, int
     if (!x || !sum) return SNB_ERR_NULL_POINTER;
     const int rc = check_plane(B, G, kept, hw, channels, index != nullptr);
     if (rc) return rc;
+    if (index) SNB_CUDA(cudaMemsetAsync(sum, 0, sizeof(float) * channels, (cudaStream_t)stream));
     plane_shift_kernel<false><<<(channels + 7) / 8, 256, 0, (cudaStream_t)stream>>>(x, index, B, G, kept, hw, channels, sum, nullptr, 0.f,
                                                                                     nullptr);
     SNB_CUDA(launched());

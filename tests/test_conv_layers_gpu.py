@@ -133,3 +133,31 @@ def test_sample_mask_draws_what_it_did(S, G, channel, q):
     want = torch.empty(S, G, count, dtype=torch.int32, device="cuda")
     C.sample_mask_into(want, channel, seed)
     assert torch.equal(got, want) and got.is_contiguous() and torch.equal(after, torch.rand(1))
+
+
+@pytest.mark.parametrize("G,repeat", [(1, False), (1, True), (3, False), (3, True)])
+def test_bias_gradient_of_lists_in_any_order(G, repeat):
+    """Output masks that do not ascend and, with `repeat`, name a channel twice: values, bias, input and weight gradients of a layer without mean shift against
+    the same in PyTorch's indexing and 64 bits."""
+    from sortnet_b200.layers import NormDistConv
+    B, ci, co, side, kept = 70, 12, 30, 3, 7
+    S, per = (B + 31) // 32, co // G
+    gen = torch.Generator(device="cuda").manual_seed(G)
+    lists = torch.rand(S, G, per, device="cuda", generator=gen).argsort(-1)[..., :kept].int()
+    if repeat:
+        lists[:, :, 3], lists[1, :, 5] = lists[:, :, 0], lists[1, :, 0]
+    lists = lists.contiguous()
+    layer = NormDistConv(ci, co, 1, groups=G, bias=True, mean_shift=False, dropout=0.5).cuda().train()
+    with torch.no_grad():
+        layer.bias.normal_(generator=gen)
+    x = torch.rand(B, ci, side, side, device="cuda", generator=gen).requires_grad_()
+    y = layer(x, mask_out=lists)[0]
+    gy = torch.randn(y.shape, device="cuda", generator=gen) + 1
+    gx, gw, gb = torch.autograd.grad(y, (x, layer.weight, layer.bias), gy)
+    xo, wo, bo = (t.detach().double().requires_grad_() for t in (x, layer.weight, layer.bias))
+    chan = (lists.long() + torch.arange(G, device="cuda").view(1, G, 1) * per)[torch.arange(B, device="cuda") // 32]          # [B, G, kept]
+    dist = (xo.view(B, G, 1, ci // G, -1) - wo[chan].unsqueeze(-1)).abs().amax(3) + bo[chan].unsqueeze(-1)
+    want = torch.autograd.grad(dist.reshape(y.shape), (xo, wo, bo), gy.double())
+    assert rel(y.detach().cpu().numpy(), dist.reshape(y.shape).detach().cpu().numpy()) < 1e-6
+    for got, exact, tol in zip((gx, gw, gb), want, (1e-5, 1e-5, 1e-6)):  # the bias sums in 64 bits up to a few additions of 2^-24
+        assert rel(got.cpu().numpy(), exact.cpu().numpy()) < tol
