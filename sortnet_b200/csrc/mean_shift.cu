@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
         }
         return lo;
     };
-    auto slot_in = [&](int s) {
-        if (!index) return c;
+    auto slot_in = [&](int s, int g, int inside) {
+        if (!index) return inside;
         const int at = place(s, g, inside);
         return at < kept && index[((size_t)s * G + g) * kept + at] == inside ? g * kept + at : -1;
     };
@@ -127,30 +127,42 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
             if (slot >= 0) walk(s0 + t, slot, body);
         }
     };
-    double sum = 0.;                                         // a lane's chain grows with rows x HW: in fp32 its rounding showed (1.4e-7 -> 1.6e-7 of the mean)
-    float cnt = 0.f;
     int first = -1;                                          // the slots of the first 32 sub-batches
-    for (int s0 = 0; s0 < S; s0 += 32) {
-        const int mine = s0 + lane < S ? slot_in(s0 + lane) : -1;
-        if (s0 == 0) first = mine;
-        if (mine >= 0) cnt += (float)(min(SNB_SUB_BATCH, B - (s0 + lane) * SNB_SUB_BATCH) * HW);
-        walk_all(s0, mine, [&](size_t o) { sum += (double)x[o]; });
-    }
+    float cnt;
+    // Sum and number of the elements of a channel.
+    auto total = [&](int g, int inside) {
+        double sum = 0.;                                     // a lane's chain grows with rows x HW: in fp32 its rounding showed (1.4e-7 -> 1.6e-7 of the mean)
+        cnt = 0.f;
+        for (int s0 = 0; s0 < S; s0 += 32) {
+            const int mine = s0 + lane < S ? slot_in(s0 + lane, g, inside) : -1;
+            if (s0 == 0) first = mine;
+            if (mine >= 0) cnt += (float)(min(SNB_SUB_BATCH, B - (s0 + lane) * SNB_SUB_BATCH) * HW);
+            walk_all(s0, mine, [&](size_t o) { sum += (double)x[o]; });
+        }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, d);
-    }
+        for (int d = 16; d > 0; d >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            cnt += __shfl_xor_sync(0xffffffffu, cnt, d);
+        }
+        return sum;
+    };
+    // Whether slot c of the list of sub-batch s0 + lane was found by its channel's warp (`entry`: the channel).  In a list that does not ascend, or names a
+    // channel twice, some are not.
+    const int gj = c / kept;
+    auto lost_in = [&](int s0, int& entry) {
+        const int s = s0 + lane;
+        entry = s < S ? index[(size_t)s * n + c] : -1;
+        return __ballot_sync(0xffffffffu, entry >= 0 && entry < per && place(s, gj, entry) != c - gj * kept);
+    };
+    const double sum = total(g, inside);
     if (!SHIFT) {
         if (lane == 0 && !index) out[c] = (float)sum;
         else if (lane == 0 && cnt > 0.f) atomicAdd(out + c, (float)sum);
         if (!index || c >= n) return;
-        // The warp also looks whether slot c of every list was found by its channel's warp.  In a list that does not ascend, or names a channel twice, some
-        // are not: their sums are added here.  Lists that ascend end in one addition to zero per channel.
-        const int gj = c / kept;
+        // What was not found is added here.  Lists that ascend end in one addition to zero per channel.
         for (int s0 = 0; s0 < S; s0 += 32) {
-            const int s = s0 + lane, entry = s < S ? index[(size_t)s * n + c] : -1;
-            unsigned lost = __ballot_sync(0xffffffffu, entry >= 0 && entry < per && place(s, gj, entry) != c - gj * kept);
+            int entry;
+            unsigned lost = lost_in(s0, entry);
             for (; lost; lost &= lost - 1) {
                 const int t = __ffs(lost) - 1;
                 double part = 0.;
@@ -169,8 +181,20 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
         if (running_mean) running_mean[c] = running_mean[c] * (1.0f - momentum) + momentum * m;
     }
     for (int s0 = 0; s0 < S; s0 += 32) {
-        const int mine = s0 == 0 ? first : s0 + lane < S ? slot_in(s0 + lane) : -1;
+        const int mine = s0 == 0 ? first : s0 + lane < S ? slot_in(s0 + lane, g, inside) : -1;
         walk_all(s0, mine, [&](size_t o) { y[o] = x[o] - m; });
+    }
+    if (!index || c >= n) return;
+    // The lists are to ascend; where one does not, what was not found is left out of the means, but every element of y is written.
+    for (int s0 = 0; s0 < S; s0 += 32) {
+        int entry;
+        unsigned lost = lost_in(s0, entry);
+        for (; lost; lost &= lost - 1) {
+            const int t = __ffs(lost) - 1;
+            const double its = total(gj, __shfl_sync(0xffffffffu, entry, t));
+            const float mean = (float)(its / fmaxf(cnt, 1e-10f));
+            walk(s0 + t, c, [&](size_t o) { y[o] = x[o] - mean; });
+        }
     }
 }
 

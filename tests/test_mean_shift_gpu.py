@@ -81,3 +81,19 @@ def test_plane_shift(B, G, C, kept, hw):
     assert ((NC.plane_sum(x, index, C).double() - sums).abs() <= 1e-5 * sums.abs().clamp(min=1)).all()
     v = torch.randn(C, device="cuda", generator=gen)
     assert torch.equal(NC.plane_add(x, index, v), x + v[chan].unsqueeze(-1))
+
+
+@pytest.mark.parametrize("B,G,per,kept,hw", [(70, 3, 10, 7, 9), (33, 1, 40, 40, 4), (1100, 1, 12, 5, 2)])
+def test_plane_shift_writes_every_element(B, G, per, kept, hw):
+    """Lists are to ascend; those that do not, or name a channel twice, leave no element of y unwritten: each is x minus the mean that its channel got."""
+    from sortnet_b200 import norm_dist_cuda as NC
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    S, C = (B + 31) // 32, G * per
+    index = torch.rand(S, G, per, device="cuda", generator=gen).argsort(-1)[..., :kept].int()
+    index[1:, :, 3] = index[1:, :, 0]
+    index = index.contiguous()
+    chan = (index.long() + torch.arange(G, device="cuda").view(1, G, 1) * per).reshape(S, -1)[torch.arange(B, device="cuda") // 32]
+    x = torch.randn(B, G * kept, hw, device="cuda", generator=gen)
+    mean, y = torch.empty(C, device="cuda"), torch.full_like(x, float("nan"))
+    NC.plane_shift(x, index, C, mean, y)
+    assert torch.equal(y, x - mean[chan].unsqueeze(-1))
