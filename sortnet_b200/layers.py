@@ -44,14 +44,14 @@ def sample_mask(batch, groups, channel, q, device, count=None):
     writes all lists; on the CPU the lists are made with PyTorch ops the way the reference does."""
     device = torch.device(device)
     if device.type == "cuda":
-        if count is None and isinstance(q, float) and _C._timeline is None and channel > 0:
-            # the same numbers from the host generator, counted and drawn in native code
-            uniform, seed = torch.rand(channel), torch.randint(0, 2 ** 62, (1,))
-            return _lib.ops().draw_lists(uniform, seed, [channel], [q], batch * groups, device)[0].view(batch, groups, -1)
-        if count is None:
-            count = int((torch.rand(channel) < q).sum())
-        count = min(max(int(count), 1), channel)
-        seed = int(torch.randint(0, 2 ** 62, (1,)))
+        uniform = torch.rand(channel) if count is None else None
+        seed = torch.randint(0, 2 ** 62, (1,))
+        if uniform is not None and isinstance(q, float) and channel > 0:
+            drawn = _C.draw_lists(uniform, seed, [channel], [q], batch * groups, device)     # counted and drawn in native code
+            if drawn is not None:
+                return drawn[0].view(batch, groups, -1)
+        count = min(max(int((uniform < q).sum() if uniform is not None else count), 1), channel)
+        seed = int(seed)
         out = torch.empty(batch, groups, count, dtype=torch.int32, device=device)
         _C.sample_mask_into(out, channel, seed)
         return out

@@ -176,3 +176,24 @@ def test_debug_mode_validates_index_lists_before_the_kernels(monkeypatch):
     unsorted = torch.tensor([[[2, 0, 4]]], dtype=torch.int32, device="cuda")
     with pytest.raises(RuntimeError, match="ascending"):
         C.inf_dist_forward_sorted(x, w, y, pos, unsorted, co)
+
+
+@pytest.mark.parametrize("S,G,channel,q", [(1, 1, 7, 0.5), (4, 3, 341, 0.9), (2, 1, 40, 0.0)])
+@pytest.mark.parametrize("device,dtype", [("cuda", torch.float32), ("cpu", torch.float64), ("cuda", torch.float64)])
+def test_sample_mask_under_other_defaults(S, G, channel, q, device, dtype):
+    """Whatever the default device and dtype give `torch.rand` for the count, the lists are those of that count and the next seed."""
+    from sortnet_b200 import layers, norm_dist_cuda as C
+    was = torch.get_default_dtype()
+    torch.set_default_dtype(dtype)
+    try:
+        with torch.device(device):
+            torch.manual_seed(7)
+            got = layers.sample_mask(S, G, channel, q, "cuda")
+            torch.manual_seed(7)
+            count = min(max(int((torch.rand(channel) < q).sum()), 1), channel)
+            seed = int(torch.randint(0, 2 ** 62, (1,)))
+    finally:
+        torch.set_default_dtype(was)
+    want = torch.empty(S, G, count, dtype=torch.int32, device="cuda")
+    C.sample_mask_into(want, channel, seed)
+    assert torch.equal(got, want) and got.dtype == torch.int32 and got.is_contiguous()
