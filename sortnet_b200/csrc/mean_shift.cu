@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) plane_shift_kernel(const float* __restric
     }
 }
 
-// y[b, j, :] = x[b, j, :] + v[channel j of b's list].  Bound by the traffic of x and y.
+// y[b, j, :] = x[b, j, :] + v[channel j of b's list] (NaN where the list holds no channel).  Bound by the traffic of x and y.
 __global__ void __launch_bounds__(256) plane_add_kernel(const float* __restrict__ x, const int* __restrict__ index, int G, int kept,
                                                         int HW, int C, const float* __restrict__ v, long long total, float* __restrict__ y) {
     const int n = G * kept, per = C / G;
@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(256) plane_add_kernel(const float* __restrict_
         const long long row = i / HW;
         const int j = (int)(row % n), g = j / kept;
         const int s = (int)(row / n) / SNB_SUB_BATCH;
-        y[i] = x[i] + v[index ? g * per + index[(size_t)s * n + j] : j];
+        const int inside = index ? index[(size_t)s * n + j] : j - g * kept;
+        y[i] = (unsigned)inside < (unsigned)per ? x[i] + v[g * per + inside] : __int_as_float(0x7fc00000);
     }
 }
 

@@ -159,8 +159,9 @@ class _PlaneSumF(torch.autograd.Function):
 
 
 def _native():
-    """Whether the native forms of the autograd functions above are taken: not where they would not be seen or the profile wants each call."""
-    return _C._timeline is None and not ops.tracing() and not ops.forward_mode()
+    """Whether the native forms of the autograd functions above are taken: not where they would not be seen, the profile wants each call
+    or index lists are to be validated."""
+    return _C._timeline is None and not _C.DEBUG_INDEX_CHECKS and not ops.tracing() and not ops.forward_mode()
 
 
 def _add_per_channel(z, vec, index):

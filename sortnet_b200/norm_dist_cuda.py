@@ -484,9 +484,7 @@ def _plane(x, index, channels):
     B, C, hw = x.shape
     G, kept = (1, C) if index is None else (index.size(1), index.size(2))
     if index is not None:
-        _check(index, "index", torch.int32)
-        if tuple(index.shape) != ((B + _SUB_BATCH - 1) // _SUB_BATCH, G, C // max(G, 1)) or G * kept != C:
-            raise RuntimeError("index must have shape [sub-batches, groups, C / groups]")
+        _check_opt_index(index, "index", (B + _SUB_BATCH - 1) // _SUB_BATCH, C, G, channels // max(G, 1))
     elif C != channels:
         raise RuntimeError("x must have all channels when there is no index")
     return B, G, kept, hw

@@ -161,3 +161,27 @@ def test_bias_gradient_of_lists_in_any_order(G, repeat):
     assert rel(y.detach().cpu().numpy(), dist.reshape(y.shape).detach().cpu().numpy()) < 1e-6
     for got, exact, tol in zip((gx, gw, gb), want, (1e-5, 1e-5, 1e-6)):  # the bias sums in 64 bits up to a few additions of 2^-24
         assert rel(got.cpu().numpy(), exact.cpu().numpy()) < tol
+
+
+@pytest.mark.parametrize("entry", [-1, 10])
+def test_lists_that_name_no_channel(entry, monkeypatch):
+    """Validated where that is asked for, by mean shift and bias alike; otherwise such an entry adds NaN and reads nothing."""
+    from sortnet_b200 import layers, norm_dist_cuda as C
+    index = torch.arange(7, device="cuda", dtype=torch.int32).repeat(3, 3, 1)
+    index[1, 2, 4] = entry
+    x, bias = torch.randn(70, 21, 4, device="cuda"), torch.randn(30, device="cuda", requires_grad=True)
+    y = layers._add_per_channel(x, bias, index)
+    bad = torch.zeros_like(x, dtype=torch.bool)
+    bad[32:64, 18] = True
+    assert torch.equal(y.isnan(), bad)
+    y.sum().backward()                                       # leaves the entry out
+    rows = 70.0 * 4 * torch.ones(3, 7, device="cuda")
+    rows[2, 4] -= 32 * 4
+    assert torch.equal(bias.grad.view(3, 10)[:, :7], rows) and not bias.grad.view(3, 10)[:, 7:].any()
+    monkeypatch.setattr(C, "DEBUG_INDEX_CHECKS", True)
+    shift = layers.MeanShiftDropout(30, affine=False).cuda().train()
+    for call in (lambda: layers._add_per_channel(x, bias, index), lambda: shift(x, index=index)):
+        with pytest.raises(RuntimeError, match="outside"):
+            call()
+    index[1, 2, 4] = 4
+    assert torch.isfinite(layers._add_per_channel(x, bias, index)).all() and torch.isfinite(shift(x, index=index)[0]).all()
