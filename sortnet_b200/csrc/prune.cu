@@ -1437,17 +1437,18 @@ cudaError_t redo_grid(int threads, int smem, int* grid) {
     return e;
 }
 
-template <int NX, bool TRACK>
+template <int NX, bool TRACK, bool LEAVE = false>
 cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     constexpr int smem = redo_max_smem<NX, TRACK>();
-    cudaError_t e = allow_smem<prune_redo_max<NX, TRACK>, smem>();
+    constexpr auto REDO = prune_redo_max<NX, TRACK, LEAVE>;
+    cudaError_t e = allow_smem<REDO, smem>();
     if (e != cudaSuccess) return e;
     int redo = 0;
-    if ((e = redo_grid<prune_redo_max<NX, TRACK>>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
+    if ((e = redo_grid<REDO>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
     constexpr int tile = (TRACK ? 2 : 1) * NX * 32 * 33 * (int)sizeof(float);
     const int share = l1_share(WALK_CTAS<NX, TRACK>, tile, (long long)grid.x * grid.y);
     if ((e = launch_next_with(share, prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
-    return launch_next(prune_redo_max<NX, TRACK>, redo, REDO_THREADS, smem, st, a);
+    return launch_next(REDO, redo, REDO_THREADS, smem, st, a);
 }
 
 // Eight outputs per CTA, a warp each.  With 32, four one after the other per warp, a few long CTAs end last: 8 / 32 outputs, values of K = 10
@@ -1510,6 +1511,7 @@ cudaError_t prune_forward(const PruneProblem& p, void* ws, cudaStream_t st) {
     const dim3 grid((p.CO + 31) / 32, a.S);
     if (p.K == 1) {
         const bool track = with_words(p);
+        if (p.leave) return run_max<1, false, true>(a, grid, st);
         if (a.NX == 1) return track ? run_max<1, true>(a, grid, st) : run_max<1, false>(a, grid, st);
         if (a.NX == 2) return track ? run_max<2, true>(a, grid, st) : run_max<2, false>(a, grid, st);
         return run_max<3, false>(a, grid, st);

@@ -64,7 +64,7 @@ struct PruneProblem {
     const float* bias = nullptr;
     unsigned* counters = nullptr;       // four zeroed counters of the caller's, or null: those in the workspace
     const int* kept_list = nullptr;     // [S][kept] kept columns: the first one is the position of an output at its floor
-    bool leave = false;                 // maxima: a layer that would be evaluated as a whole is left to the caller (prune_left)
+    bool leave = false;                 // maxima of points, no positions: a layer that would be evaluated as a whole is left to the caller (prune_left)
 };
 
 // Transposes x (or x and the box [max(x - eps, down), min(x + eps, up)], or given box ends) to the chain form.
