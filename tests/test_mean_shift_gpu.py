@@ -97,3 +97,45 @@ def test_plane_shift_writes_every_element(B, G, per, kept, hw):
     mean, y = torch.empty(C, device="cuda"), torch.full_like(x, float("nan"))
     NC.plane_shift(x, index, C, mean, y)
     assert torch.equal(y, x - mean[chan].unsqueeze(-1))
+
+
+# a warp per channel (with more than 32 sub-batches too), one CTA, clusters of 2, 4 and 8; more sub-batches than a CTA has threads; positions by four and by one
+@pytest.mark.parametrize("B,G,C,kept,hw", [(1100, 1, 2000, 1500, 1), (40, 1, 600, 500, 4), (40, 1, 64, 48, 32), (70, 3, 30, 7, 49), (200, 1, 64, 64, 100), (200, 1, 64, 48, 33),
+                                           (130, 1, 40, 30, 225), (128, 1, 16, 16, 1024), (128, 3, 15, 4, 1024), (8300, 2, 4, 1, 1), (300, 1, 3, 3, 401)])
+@pytest.mark.parametrize("lists", ["ascending", "any order", "misaligned"])
+def test_plane_kernels_of_every_form(B, G, C, kept, hw, lists):
+    """Mean shift, sums and add against float64; lists in any order and with repeated channels as far as they are taken."""
+    from sortnet_b200 import norm_dist_cuda as NC
+    gen = torch.Generator(device="cuda").manual_seed(B + hw)
+    S, per = (B + 31) // 32, C // G
+    index, chan = None, torch.arange(C, device="cuda").expand(B, C)
+    if kept * G < C:
+        index = torch.rand(S, G, per, device="cuda", generator=gen).argsort(-1)[..., :kept].int()
+        if lists == "any order":
+            index[::2, :, -1] = index[::2, :, 0]
+        else:
+            index = index.sort(-1)[0]
+        index = index.contiguous()
+        chan = (index.long() + torch.arange(G, device="cuda").view(1, G, 1) * per).reshape(S, -1)[torch.arange(B, device="cuda") // 32]
+    off = 1 if lists == "misaligned" else 0
+    def buffer():
+        return torch.full((off + chan.numel() * hw + 8,), 7.0, device="cuda")
+    def view(t):
+        return t[off:off + chan.numel() * hw].view(*chan.shape, hw)
+    x = view(buffer())
+    x.copy_(torch.randn(x.shape, device="cuda", generator=gen) + 1000)
+    rows = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), torch.full((chan.numel(),), float(hw), dtype=torch.float64, device="cuda"))
+    sums = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), x.double().sum(-1).reshape(-1))
+    y_all, mean, run = buffer(), torch.empty(C, device="cuda"), torch.ones(C, device="cuda")
+    y = view(y_all)
+    NC.plane_shift(x, index, C, mean, y, run, 0.1)
+    assert torch.equal(y, x - mean[chan].unsqueeze(-1)) and (y_all[off + y.numel():] == 7).all() and (y_all[:off] == 7).all()
+    if lists != "any order" or index is None:
+        want = torch.where(rows > 0, sums / rows.clamp(min=1), 0.0)
+        assert ((mean.double() - want).abs() <= 2 ** -23 * want.abs()).all()         # 64-bit sums: the result's rounding and a last digit
+        assert ((run.double() - (0.9 + 0.1 * want)).abs() <= 2 ** -22 * (0.9 + 0.1 * want.abs())).all()
+    # in any order up to three additions of parts per sub-batch
+    bound = 2 ** -23 if lists != "any order" else 2 ** -23 * (2 + 3 * S)
+    assert ((NC.plane_sum(x, index, C).double() - sums).abs() <= bound * sums.abs()).all()
+    v = torch.randn(C, device="cuda", generator=gen)
+    assert torch.equal(NC.plane_add(x, index, v), x + v[chan].unsqueeze(-1))
