@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(PLANE_THREADS) plane_add_kernel(const PlaneArg
 static int check_plane(int B, int G, int kept, int hw, int channels, bool lists) {
     if (B <= 0 || G <= 0 || kept <= 0 || hw <= 0 || channels < (long long)G * kept || channels % G || (!lists && channels != G * kept))
         return SNB_ERR_BAD_SHAPE;
-    return (long long)B * G * kept * hw >= (1ll << 31) ? SNB_ERR_TOO_LARGE : SNB_OK;
+    return SNB_OK;
 }
 
 template <bool SHIFT, bool WIDE, int V>

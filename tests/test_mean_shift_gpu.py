@@ -139,3 +139,24 @@ def test_plane_kernels_of_every_form(B, G, C, kept, hw, lists):
     assert ((NC.plane_sum(x, index, C).double() - sums).abs() <= bound * sums.abs()).all()
     v = torch.randn(C, device="cuda", generator=gen)
     assert torch.equal(NC.plane_add(x, index, v), x + v[chan].unsqueeze(-1))
+
+
+@pytest.mark.parametrize("lists", [False, True])
+def test_plane_kernels_past_31_bits(lists):
+    """More than 2^31 elements in all."""
+    from sortnet_b200 import norm_dist_cuda as NC
+    B, G, kept, hw = 33, 2, 2, (1 << 31) // (33 * 4) + 5
+    C = G * (3 if lists else 2)
+    index = torch.tensor([[[0, 2], [1, 2]], [[1, 2], [0, 1]]], dtype=torch.int32, device="cuda") if lists else None
+    chan = torch.tensor([[0, 2, 4, 5]] * 32 + [[1, 2, 3, 4]] if lists else [[0, 1, 2, 3]] * B, device="cuda")
+    x = torch.empty(B, G * kept, hw, device="cuda").uniform_(generator=torch.Generator(device="cuda").manual_seed(0))
+    sums = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), x.sum(-1, dtype=torch.float64).reshape(-1))
+    rows = torch.zeros(C, dtype=torch.float64, device="cuda").index_add_(0, chan.reshape(-1), torch.ones(chan.numel(), dtype=torch.float64, device="cuda"))
+    assert ((NC.plane_sum(x, index, C).double() - sums).abs() <= 2 ** -23 * sums).all()
+    v = torch.randn(C, device="cuda")
+    y = NC.plane_add(x, index, v)
+    assert all(torch.equal(y[b, j], x[b, j] + v[chan[b, j]]) for b in range(B) for j in range(G * kept))
+    mean = torch.empty(C, device="cuda")
+    NC.plane_shift(x, index, C, mean, y.fill_(7.0))
+    assert ((mean.double() - sums / (rows * hw)).abs() <= 2 ** -23).all()
+    assert all(torch.equal(y[b, j], x[b, j] - mean[chan[b, j]]) for b in range(B) for j in range(G * kept))
