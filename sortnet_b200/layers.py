@@ -222,7 +222,13 @@ class MeanShiftDropout(nn.Module):
         if self.training:
             assert x is not None, "training needs the activations"
             if plane:
-                x, mean = (_lib.ops().mean_shift if _native() else _MeanShiftPlaneF.apply)(x, index, self.running_mean, self.momentum)
+                run = self.running_mean
+                plain = run.dtype == torch.float32 and run.is_contiguous() and run.device == x.device      # what the kernel updates
+                kept = run if plain else torch.zeros(self.out_channels, device=x.device, dtype=torch.float32)
+                x, mean = (_lib.ops().mean_shift if _native() else _MeanShiftPlaneF.apply)(x, index, kept, self.momentum)
+                if not plain:
+                    with torch.no_grad():
+                        run.mul_(1 - self.momentum).add_(mean, alpha=self.momentum)
             else:
                 x, mean = _MeanShiftTrainF.apply(x, index, self.running_mean, self.momentum)
             if self.bias is not None:

@@ -185,3 +185,16 @@ def test_lists_that_name_no_channel(entry, monkeypatch):
             call()
     index[1, 2, 4] = 4
     assert torch.isfinite(layers._add_per_channel(x, bias, index)).all() and torch.isfinite(shift(x, index=index)[0]).all()
+
+
+@pytest.mark.parametrize("kind", ["double", "strided"])
+def test_running_mean_of_another_layout(kind):
+    """A running mean that the kernel cannot update is updated in PyTorch."""
+    from sortnet_b200.layers import MeanShiftDropout
+    x = torch.randn(40, 6, 9, device="cuda")
+    want, got = (MeanShiftDropout(6, affine=False).cuda().train() for _ in range(2))
+    got.running_mean = torch.zeros(6, device="cuda", dtype=torch.float64) if kind == "double" else torch.zeros(12, device="cuda")[::2]
+    for _ in range(2):
+        y, z = want(x)[0], got(x)[0]
+        assert torch.equal(y, z) and torch.allclose(want.running_mean.double(), got.running_mean.double(), rtol=1e-6, atol=1e-8)
+    assert got.running_mean.dtype == (torch.float64 if kind == "double" else torch.float32)
