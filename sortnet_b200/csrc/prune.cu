@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(FT + 32 * NB * R, FIT) prune_filter(const Prun
                         if (lane < TOP) top[buf][r][warp * TOP + lane] = kept & ~31u;
                     }
                 }
+                __syncwarp();                                // the barriers are for whole warps: here and below lanes come out of branches of their own
                 bar_arrive(BAR_TOP + buf, ALL);
             }
             if (!first) {
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(FT + 32 * NB * R, FIT) prune_filter(const Prun
                         at++;
                     }
                 }
+                __syncwarp();
                 bar_arrive(BAR_FULL + last, ALL);
                 const int next = step + (STAGES - 1) * (int)gridDim.x;
                 if (next < steps) fetch(next, before);
