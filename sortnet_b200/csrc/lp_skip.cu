@@ -596,9 +596,12 @@ struct Area {
 // The maxima by the pruned evaluation (prune.cuh), which reads W once for all sub-batches, where skip_maxima does so for each: from so many weights on
 // that it need not read again.  Forward at p = 1000, skip_maxima / pruned, inputs in [0, 1]: 512 x 5120 x 5120 899 / 502 us, 512 x 784 x 5120
 // (60 M weights not read again) 225 / 170; with lists of three quarters, for which the pruned form reads all of W and has more to prepare,
-// 512 x 5120 x 5120 (221 M) 516 / 342, 512 x 784 x 5120 (34 M) 131.6 / 127.4, 64 x 5120 x 5120 (15 M) 101 / 117.  A layer that cannot be pruned is left to
-// skip_maxima, after a filter in vain: inputs N(0, 0.35) 1054 / 1105 and 259 / 284.  At 64 x 5120 x 5120 (26 M) that would be 195 / 232 for a gain
-// of 175 / 140: not taken.
+// 512 x 5120 x 5120 (221 M) 516 / 342, 512 x 784 x 5120 (34 M) 131.6 / 127.4, 64 x 5120 x 5120 (15 M) 101 / 117.  What it reads and the scan would not is to
+// be two thirds of that at most (M not read again, M more: us): CO x CI of W_CO x W_CI 512 x 5120 of 5120 x 5120, 512 rows (38, 22: 130 / 119), 4096 x 4096 of 8192 x
+// 8192, 256 rows (112, 48: 335 / 295), 128 rows (48, 48: 185 / 214), 1000 x 3300, 512 rows (47, 61: 231 / 253), 2000 x 6000 of 12288 x 12288, 512 rows (172, 133:
+// 622 / 725), 128 rows (34, 133: 187 / 290).  A layer that cannot be pruned is left to
+// skip_maxima, after a filter in vain: inputs N(0, 0.35) 1030 / 1078 and 237 / 261, with lists 609 / 669 and 157 / 204.  At 64 x 5120 x 5120 (26 M) that would be 195 / 232
+// for a gain of 175 / 140: not taken.
 PruneProblem maxima_problem(const LpProblem& q, float* mt) {
     PruneProblem m;
     m.x = q.x, m.w = q.w, m.ci = q.ci, m.co = q.co;
@@ -609,7 +612,8 @@ PruneProblem maxima_problem(const LpProblem& q, float* mt) {
 }
 bool maxima_pruned(const LpProblem& q) {
     const long long again = (long long)((q.B + 31) / 32 - 1) * q.CO * q.CI;
-    return again >= 32ll << 20 && prune_applies(maxima_problem(q, nullptr));
+    const long long more = (long long)q.W_CO * q.W_CI - (long long)q.CO * q.CI;
+    return again >= 32ll << 20 && 2 * again >= 3 * more && prune_applies(maxima_problem(q, nullptr));
 }
 
 size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, char** prune = nullptr) {

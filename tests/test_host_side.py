@@ -306,3 +306,25 @@ def test_shard_bounds_tile_the_flat_buffer():
             for (lo, hi), (lo2, _) in zip(edges, edges[1:]):
                 assert hi == lo2 and lo <= hi
             assert all(lo % 4 == 0 and hi % 4 == 0 for lo, hi in edges)
+
+
+def up256(n):
+    return (n + 255) // 256 * 256
+
+
+def sparse_forward_bytes(B, CO, CI):
+    """Scratch of the sparse l-p forward itself: transposed inputs and their ranges, maxima and sums."""
+    S = (B + 31) // 32
+    return up256(S * CI * 128) + up256(S * CI * 8) + 2 * up256(S * CO * 128)
+
+
+# sub-batches read W again often enough, and the pruned form does not read much more of it than they do
+@pytest.mark.parametrize("B,CO,CI,W_CO,W_CI,pruned", [(512, 5120, 5120, 5120, 5120, True), (64, 5120, 5120, 5120, 5120, False), (96, 5120, 5120, 5120, 5120, True),
+                                                      (512, 3840, 3840, 5120, 5120, True), (512, 512, 5120, 5120, 5120, True), (256, 4096, 4096, 8192, 8192, True),
+                                                      (128, 4096, 4096, 8192, 8192, False), (512, 1000, 3300, 8192, 8192, False), (128, 2000, 6000, 12288, 12288, False),
+                                                      (512, 2000, 6000, 12288, 12288, False)])
+def test_maxima_of_the_sparse_forward_by_pruning(built_lib, B, CO, CI, W_CO, W_CI, pruned):
+    from sortnet_b200 import _lib
+    need = _lib.load().snb_norm_dist_scratch_bytes(0, B, CO, CI, W_CO, W_CI, 1000.0, int(CI < W_CI))
+    own = sparse_forward_bytes(B, CO, CI)
+    assert need > own if pruned else need == own
