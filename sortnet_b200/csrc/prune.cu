@@ -1371,9 +1371,10 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
     char* cand = take(sizeof(int2) * J * lcap);
     char* fail = take(sizeof(int4) * S * ((p.CO + 31) / 32) * (p.K > 1 ? 4 : 1));      // prune_sort: down to eight outputs per CTA
     const size_t ldr = (C + 3) / 4 * 4;
-    char* xr = take(sizeof(float) * NX * S * 32 * ldr);
-    char* partial = take(p.K > 1 ? 0 : (with_words(p) ? 8 : 4) * NX * S * p.CO * 32);
-    char* tile_done = take(p.K > 1 ? 0 : sizeof(unsigned) * S * ((p.CO + 127) / 128));
+    const bool whole = !p.leave;                             // evaluated as a whole here, should it come to that
+    char* xr = take(whole ? sizeof(float) * NX * S * 32 * ldr : 0);
+    char* partial = take(p.K > 1 || !whole ? 0 : (with_words(p) ? 8 : 4) * NX * S * p.CO * 32);
+    char* tile_done = take(p.K > 1 || !whole ? 0 : sizeof(unsigned) * S * ((p.CO + 127) / 128));
     if (a) {
         a->ldr = (int)ldr;
         a->xr = reinterpret_cast<float*>(xr);

@@ -328,3 +328,14 @@ def test_maxima_of_the_sparse_forward_by_pruning(built_lib, B, CO, CI, W_CO, W_C
     need = _lib.load().snb_norm_dist_scratch_bytes(0, B, CO, CI, W_CO, W_CI, 1000.0, int(CI < W_CI))
     own = sparse_forward_bytes(B, CO, CI)
     assert need > own if pruned else need == own
+
+
+@pytest.mark.parametrize("B,CO,CI,W_CO,W_CI", [(512, 5120, 5120, 5120, 5120), (1024, 3840, 3840, 5120, 5120), (4096, 1500, 1001, 1500, 1001)])
+def test_scratch_of_pruned_maxima(built_lib, B, CO, CI, W_CO, W_CI):
+    """What the pruned form of this layer takes, without what only an evaluation as a whole needs: rows side by side, partial results, counters of tiles."""
+    from sortnet_b200 import _lib
+    lib = _lib.load()
+    S, lists = (B + 31) // 32, int(CI < W_CI)
+    whole = lib.snb_prune_scratch_bytes(1, 1, 0, B, CO, CI, W_CO, W_CI, lists)
+    unused = up256(4 * S * 32 * ((W_CI + 3) // 4 * 4)) + up256(4 * S * CO * 32) + up256(4 * S * ((CO + 127) // 128))
+    assert lib.snb_norm_dist_scratch_bytes(0, B, CO, CI, W_CO, W_CI, 1000.0, lists) == sparse_forward_bytes(B, CO, CI) + up256(whole - unused)
