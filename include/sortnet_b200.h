@@ -243,8 +243,9 @@ int snb_norm_dist_backward_input_weight(const float* grad_output, const float* x
  * the forward, terms that together stay below 2^-27 of the result (each below 2^-27 p / CI of the largest) and, in the
  * backward, terms below 2^-40 of the largest possible.  snb_norm_dist_scratch_bytes: bytes for
  * snb_norm_dist_forward_ws (backward = 0; never less than snb_norm_dist_forward_workspace_bytes) or snb_norm_dist_backward_ws
- * (backward = 1; 0: the call needs none); column_lists = 1 when w_index_ci is given (the answer does not depend on it
- * today).  16-byte aligned, any content on entry.  With less workspace, or NULL, the dense kernels run.  No counterpart in the reference. */
+ * (backward = 1; 0: the call needs none); column_lists = 1 when w_index_ci is given.  16-byte aligned, any content on entry.  With less
+ * workspace, down to 256 (ceil(B/32) CI + ceil(B/32) CO + 4) bytes, a forward of many sub-batches scans for its maxima; with less still, or
+ * NULL, the dense kernels run.  No counterpart in the reference. */
 size_t snb_norm_dist_scratch_bytes(int backward, int B, int CO, int CI, int W_CO, int W_CI, float p, int column_lists);
 int snb_norm_dist_backward_ws(const float* grad_output, const float* x, const float* w, const float* y, int B, int CO, int CI,
                               int G, int HW, float* grad_input, float* grad_weight, float p, const int* w_index_ci,

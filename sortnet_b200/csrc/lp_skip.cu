@@ -616,14 +616,15 @@ bool maxima_pruned(const LpProblem& q) {
     return again >= 32ll << 20 && 2 * again >= 3 * more && prune_applies(maxima_problem(q, nullptr));
 }
 
-size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, char** prune = nullptr) {
+// pruned: with the pruned evaluation's scratch, at the end.
+size_t forward_layout(const LpProblem& q, char* base, ForwardArgs* a, bool pruned, char** prune = nullptr) {
     const size_t S = (q.B + 31) / 32;
     Area at{base};
     float* xt = at.take<float>(S * q.CI * 32);
     float2* range = at.take<float2>(S * q.CI);
     float* mt = at.take<float>(S * q.CO * 32);
     float* sum = at.take<float>(S * q.CO * 32);
-    char* scratch = at.take<char>(maxima_pruned(q) ? prune_workspace_bytes(maxima_problem(q, mt)) : 0);
+    char* scratch = at.take<char>(pruned ? prune_workspace_bytes(maxima_problem(q, mt)) : 0);
     if (prune) *prune = scratch;
     if (a) {
         a->w = q.w, a->ci = q.ci, a->co = q.co, a->xt = xt, a->range = range, a->mt = mt, a->sum = sum;
@@ -656,17 +657,18 @@ size_t backward_layout(const LpProblem& q, char* base, BackwardArgs* a) {
 }  // namespace
 
 size_t lp_skip_forward_bytes(const LpProblem& q) {
-    return forward_applies(q) ? forward_layout(q, nullptr, nullptr) : 0;
+    return forward_applies(q) ? forward_layout(q, nullptr, nullptr, maxima_pruned(q)) : 0;
 }
+size_t lp_skip_forward_least_bytes(const LpProblem& q) { return forward_applies(q) ? forward_layout(q, nullptr, nullptr, false) : 0; }
 
 size_t lp_skip_backward_bytes(const LpProblem& q) { return backward_applies(q) ? backward_layout(q, nullptr, nullptr) : 0; }
 
-cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, cudaStream_t st) {
+cudaError_t lp_skip_forward(const LpProblem& q, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
     ForwardArgs a{};
     char* prune = nullptr;
-    forward_layout(q, static_cast<char*>(ws), &a, &prune);
+    const bool pruned = maxima_pruned(q) && ws_bytes >= lp_skip_forward_bytes(q);
+    forward_layout(q, static_cast<char*>(ws), &a, pruned, &prune);
     const int S = (q.B + 31) / 32, smem = slab_bytes(a.sl, 128, 12);
-    const bool pruned = maxima_pruned(q);
     cudaError_t e = cudaSuccess;
     // maxima and sums lie side by side
     if (a.sl.chunks > 1 && (e = cudaMemsetAsync(a.mt, 0, (char*)(a.sum + (size_t)S * q.CO * 32) - (char*)a.mt, st)) != cudaSuccess) return e;

@@ -492,9 +492,9 @@ static int lp_forward_impl(const float* x, const float* w, int B, int CO, int CI
     LpFwdParams q{x, w, y, nullptr, w_index_ci, w_index_co, B, CO, CI, W_CI, p, 0};
     if (p > 10.0f) {
         const LpProblem sparse{x, w, w_index_ci, w_index_co, B, CO, CI, W_CO, W_CI, p};
-        const size_t need = lp_skip_forward_bytes(sparse);
-        if (ws && need && ws_bytes >= need) {
-            SNB_CUDA(lp_skip_forward(sparse, y, ws, st));
+        const size_t least = lp_skip_forward_least_bytes(sparse);
+        if (ws && least && ws_bytes >= least) {
+            SNB_CUDA(lp_skip_forward(sparse, y, ws, ws_bytes, st));
             return SNB_OK;
         }
         float* scratch = ws && ws_bytes >= sizeof(float) * (size_t)B * CO ? static_cast<float*>(ws) : nullptr;

@@ -191,3 +191,26 @@ def test_huge_finite_p(p, shape, narrow):
     dense, _, _ = calls(x, w, g, ci, co, p, sparse=False)
     top = (x[:, None, :] - w[None]).abs().amax(-1)
     assert near(y, dense) < 1e-6 and float(((y - top).abs() / top).max()) < 1e-5
+
+
+def test_forward_with_scratch_between_the_forms():
+    """Scratch for the sparse form but not for pruned maxima, as it was asked for before there were such: the scan's maxima, which are the same
+    numbers, and so the same result; a byte less and the dense kernels run."""
+    from sortnet_b200 import _lib
+    lib = _lib.load()
+    B, CI, CO, p = 1100, 1003, 1100, 200.0                          # one chunk of columns: sums in a fixed order
+    x, w, _, _, _ = inputs(B, CI, CO, 1.0, 3)
+    up256 = lambda n: (n + 255) // 256 * 256
+    S = (B + 31) // 32
+    least, full = up256(S * CI * 128) + up256(S * CI * 8) + 2 * up256(S * CO * 128), lib.snb_norm_dist_scratch_bytes(0, B, CO, CI, CO, CI, p, 0)
+    assert full > least
+    ys = []
+    for nbytes in (full, full - 1, least, least - 1):
+        ws = torch.full((nbytes + 16,), 0xff, dtype=torch.uint8, device="cuda")
+        y = torch.full((B, CO), float("nan"), device="cuda")
+        _lib.check(lib.snb_norm_dist_forward_ws(x.data_ptr(), w.data_ptr(), B, CO, CI, 1, 1, y.data_ptr(), p, None, None, CO, CI, ws.data_ptr(), nbytes,
+                                                torch.cuda.current_stream().cuda_stream), "forward")
+        assert (ws[nbytes:] == 0xff).all()
+        ys.append(y)
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+    assert not torch.equal(ys[0], ys[3]) and torch.allclose(ys[0], ys[3], rtol=TOL, atol=0)
