@@ -547,12 +547,6 @@ struct SortState {
             top[NX - 1].add(fmaxf(t1, t2));
         }
     }
-    __device__ __forceinline__ float worst(int K) const {
-        float m = top[0].kth(K);
-#pragma unroll
-        for (int t = 1; t < NX; t++) m = fminf(m, top[t].kth(K));
-        return m;
-    }
     // the lower bound's list holds the mirrored values: -combine(-1e-10, -v) = combine(1e-10, v)
     __device__ __forceinline__ float result(int t, int K, float q) const { return top[t].combine(K, q, SNB_EPS); }
 };
@@ -1399,7 +1393,8 @@ size_t layout(const PruneProblem& p, char* base, PruneArgs* a) {
     return off;
 }
 
-// Persistent grid: as many CTAs as fit (the shared memory of the stages limits them to two per SM for wide rows).
+// Persistent grid: as many CTAs as fit.  FIT, for which the registers are allotted: one CTA of 512 filter threads, two where the stages of wide rows leave no room for
+// more, three otherwise.
 template <int R, int NIT, int FT, int STAGES, int NB, bool VEC, int FIT = FT == 512 ? 1 : NIT >= 4 ? 2 : 3>
 cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     constexpr auto bytes = [](int lcap) {
