@@ -1415,7 +1415,11 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
 template <bool VEC>
 cudaError_t filter(const PruneArgs& a, cudaStream_t st) {
     const int C = a.p.W_CI;
-    if (C <= 1024) return launch_filter<2, 1, 256, 3, 3, VEC>(a, st);
+    // Narrow rows take two per step, for which three list buffers are too few where lists are long (us at 5120 rows, cold, rank 1 / 10; before: sweeps behind a barrier each,
+    // four rows per step): 512 columns 12.5 / 22.7 with three, 12.3 / 18.1 with four, before 13.4 / 20.2; 1024 columns 14.0 / 23.7, 14.0 / 19.5, before 15.2 / 21.4; one
+    // row per step 13.7 / 16.6 and 14.9 / 19.1.  Wider ones, one row per step, before -> now: 1500 18.1 -> 17.0 / 25.6 -> 21.4, 2048 19.1 -> 17.5 / 26.5 -> 22.1, 3000 22.0 ->
+    // 20.5 / 30.1 -> 25.8, 4000 26.3 -> 26.4 / 34.3 -> 30.3.
+    if (C <= 1024) return launch_filter<2, 1, 256, 3, 4, VEC>(a, st);
     if (C <= 2048) return launch_filter<1, 2, 256, 3, 4, VEC>(a, st);
     if (C <= 3072) return launch_filter<1, 3, 256, 3, 4, VEC>(a, st);
     if (C <= 4096) return launch_filter<1, 4, 256, 3, 4, VEC>(a, st);
