@@ -1424,8 +1424,10 @@ cudaError_t filter(const PruneArgs& a, cudaStream_t st) {
     if (C <= 3072) return launch_filter<1, 3, 256, 3, 4, VEC>(a, st);
     if (C <= 4096) return launch_filter<1, 4, 256, 3, 4, VEC>(a, st);
     if (C <= 5120) return launch_filter<1, 5, 256, 3, 4, VEC>(a, st);
-    // Rows that are copied by single floats: 16 warps of fewer columns each, 3000 x 6001 30.8 us against 34.2; by fours two CTAs, 3000 x 6000 23.4 against 27.3.
-    if (C <= 6144) return VEC ? launch_filter<1, 6, 256, 3, 4, true>(a, st) : launch_filter<1, 3, 512, 3, 4, false>(a, st);
+    // Copied by single floats three list buffers are better than four, and than 16 warps of fewer columns each (which let the walk start late, too): 3000 x 6001,
+    // cold, rank 1 / 10, 30.3 / 35.6 us against 34.1 / 41.4 and 30.3 / 36.3; values with positions of 67 rows, W in L2, 40.6 against 40.8 and 43.5 in all.  By fours 3000 x 6000
+    // 23.4 with four buffers, 27.3 with 16 warps.
+    if (C <= 6144) return VEC ? launch_filter<1, 6, 256, 3, 4, true>(a, st) : launch_filter<1, 6, 256, 3, 3, false>(a, st);
     if (C <= 8192) return launch_filter<1, 4, 512, 3, 4, VEC>(a, st);
     return launch_filter<1, 6, 512, 3, 4, VEC>(a, st);
 }
