@@ -58,11 +58,11 @@ inline cudaError_t launch_next(void (*kern)(Params...), dim3 grid, dim3 block, s
 
 // The share with which `ctas` CTAs of `bytes` of shared memory fit an SM and the rest is L1, for a grid of `grid` CTAs.  Left alone, an SM stays as the
 // kernel before wanted it, and in a chain that is a filter with its stages: the list walks behind it, which live on L1, took 50 instead of
-// 43 us per layer of a training pass.  A grid of less than a CTA per SM is left alone: it has little to gain, and dividing the memory anew
-// takes its while (four layers of 28 rows and 832 outputs 95 us, with all of them divided 98).
-inline int l1_share(int ctas, int bytes, long long grid) {
+// 43 us per layer of a training pass.  A grid of less than `from` CTAs per SM is left alone: it has little to gain, and dividing the memory anew
+// takes 1 to 2 us (four layers of 28 rows and 832 outputs 95 us, with all of them divided 98).
+inline int l1_share(int ctas, int bytes, long long grid, float from) {
     const int room = ctas * (bytes + 1024), all = 228 * 1024;
-    return grid < sm_count() ? -1 : room >= all ? 100 : (100 * room + all - 1) / all;
+    return (float)grid < from * (float)sm_count() ? -1 : room >= all ? 100 : (100 * room + all - 1) / all;
 }
 
 // Values with positions of small problems by one launch of a warp per row and four outputs, instead of tiles, partial results and a

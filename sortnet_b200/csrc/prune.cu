@@ -1409,7 +1409,10 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
     const int grid = steps < slots ? steps : slots;
-    return launch_next_with(l1_share(FIT, bytes(LONG_LIST), grid), KERN, grid, threads, smem, st, a);
+    // Long lists: all for shared memory (32 x 1024 x 1024, ten and seventeen values 20.0 and 25.7 us, left alone 21.5 and 34.0).  Short ones leave the division as it is, and the
+    // walk behind them has what they do not use (positions of 200 x 1024 x 1024 17.6 us, else 18.6; boxes of 67 x 300 x 700 with positions 19.1, else 21.9).
+    const int share = a.m > 2 ? l1_share(FIT, bytes(LONG_LIST), grid, 1) : -1;
+    return launch_next_with(share, KERN, grid, threads, smem, st, a);
 }
 
 template <bool VEC>
@@ -1450,7 +1453,12 @@ cudaError_t run_max(const PruneArgs& a, dim3 grid, cudaStream_t st) {
     int redo = 0;
     if ((e = redo_grid<REDO>(REDO_THREADS, smem, &redo)) != cudaSuccess) return e;
     constexpr int tile = (TRACK ? 2 : 1) * NX * 32 * 33 * (int)sizeof(float);
-    const int share = l1_share(WALK_CTAS<NX, TRACK>, tile, (long long)grid.x * grid.y);
+    // By CTAs, divided / left alone.  Points with positions: 441 (200 x 2048 x 2000) 23.2 / 21.8 us, 480 (67 x 5120 x 5120) 42.4 / 42.2, 512 (512 x 1024 x 1024) 19.7 / 20.7,
+    // 2560 72.2 / 72.9, masked 84.4 / 86.8; boxes with positions: 189 (67 x 2048 x 2000) 27.8 / 25.9, 224 24.8 / 24.8, 352 (512 x 300 x 700) 24.8 / 25.9, 480 49.9 / 52.2, 2560
+    // 115 / 119; values: 512 19.6 / 18.9, 1008 (512 x 2048 x 2000) 27.9 / 26.9, 1120 47.7 / 47.8, 2560 (512 x 5120 x 5120) 58.8 / 60.1.  Boxes and points with boxes without
+    // positions gain nothing (seven layers of 2560 441 / 439).
+    constexpr float from = TRACK ? (NX == 1 ? 3.4f : 2) : 12;
+    const int share = TRACK || NX == 1 ? l1_share(WALK_CTAS<NX, TRACK>, tile, (long long)grid.x * grid.y, from) : -1;
     if ((e = launch_next_with(share, prune_max<NX, TRACK>, grid, 256, 0, st, a)) != cudaSuccess) return e;
     return launch_next(REDO, redo, REDO_THREADS, smem, st, a);
 }
@@ -1465,7 +1473,11 @@ cudaError_t run_sort(const PruneArgs& a, cudaStream_t st) {
     if (e == cudaSuccess) e = allow_smem<prune_sort<NX, KMAX, POS>, sort_walk_smem<NX, KMAX, POS>(KMAX)>();
     if (e != cudaSuccess) return e;
     const dim3 grid((a.p.CO + SORT_SLOTS - 1) / SORT_SLOTS, a.S);
-    const int smem = sort_walk_smem<NX, KMAX, POS>(a.p.K), share = l1_share(SORT_CTAS<KMAX>, smem, (long long)grid.x * grid.y);
+    // By CTAs, divided / left alone: values of K = 10 250 (32 x 2048 x 2000) 27.9 / 25.8 us, 384 23.7 / 22.2, 750 32.0 / 31.9, 10240 202.5 / 202.9; boxes 384 30.9 / 29.0, 616 31.7 /
+    // 32.9, 10240 315.5 / 319.5; points and boxes of five layers 1125 / 1138.  Positions of more than ten values, whose walks are long: 188 (32 x 9000 x 1500) 216 / 224, 264 49.7 / 50.6,
+    // 10240 1109 / 1142.
+    const int smem = sort_walk_smem<NX, KMAX, POS>(a.p.K);
+    const int share = l1_share(SORT_CTAS<KMAX>, smem, (long long)grid.x * grid.y, POS && KMAX > 10 ? 1 : 3.4f);
     e = launch_next_with(share, prune_sort<NX, KMAX, POS>, grid, 256, smem, st, a);
     if (e != cudaSuccess) return e;
     if ((e = launch_next(prune_redo_sort<NX, KMAX, POS>, redo, 256, 0, st, a)) != cudaSuccess || !POS) return e;
