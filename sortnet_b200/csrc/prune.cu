@@ -1410,7 +1410,7 @@ cudaError_t launch_filter(const PruneArgs& a, cudaStream_t st) {
     const int steps = (a.p.W_CO + R - 1) / R, slots = sm_count() * (per_sm > 0 ? per_sm : 1);
     const int grid = steps < slots ? steps : slots;
     // Long lists: all for shared memory (32 x 1024 x 1024, ten and seventeen values 20.0 and 25.7 us, left alone 21.5 and 34.0).  Short ones leave the division as it is, and the
-    // walk behind them has what they do not use (positions of 200 x 1024 x 1024 17.6 us, else 18.6; boxes of 67 x 300 x 700 with positions 19.1, else 21.9).
+    // walk behind them has what they do not use (boxes with positions of 67 x 300 x 700 19.1 us, else 21.9; of 67 x 1024 x 1024 20.6, else 21.9).
     const int share = a.m > 2 ? l1_share(FIT, bytes(LONG_LIST), grid, 1) : -1;
     return launch_next_with(share, KERN, grid, threads, smem, st, a);
 }
